@@ -111,3 +111,40 @@ def test_engine_sampled_generation_graph_equals_eager():
     assert torch.equal(a.cpu(), b.cpu())
     c = InferenceEngine(model, max_batch=3, max_seq=64, page=16).generate(prompts, 12, params, seed=12)
     assert not torch.equal(a.cpu(), c.cpu())
+
+
+@pytest.mark.parametrize("vocab", [5, 8192, 8193, 100003, 128256, 393221])
+def test_equal_logits_take_ties_in_id_order_on_every_row_split(vocab):
+    """All weights equal: the draw is the floor(u * V)-th id, wherever the row is cut (one CTA, eight CTAs with a slice
+    in shared memory, a slice too long for it); a row with one id masked shifts every id behind it by one."""
+    rows = 5
+    lg = torch.zeros(rows, vocab)
+    hole = vocab // 3
+    lg[rows - 1, hole] = float("-inf")
+    s = DeviceSampler(SamplingParams(temperature=1.0), rows, vocab, range(50, 50 + rows), "cuda")
+    got = s.sample(lg.cuda()).cpu().tolist()
+    w = 2 ** 32 - 1
+    for b in range(rows):
+        n = vocab - (b == rows - 1)
+        z = n * w
+        t = min(int(SamplerRng(50 + b).next_uniform() * float(z)), z - 1)
+        want = t // w
+        if b == rows - 1 and want >= hole:
+            want += 1
+        assert got[b] == want
+
+
+@pytest.mark.parametrize("vocab", [1, 37, 8191, 20001])
+def test_odd_rows_and_penalties_match_the_float64_policy(vocab):
+    """Odd lengths (unaligned rows), a window with repeats, top-k and top-p together: only a draw within rounding of a
+    CDF boundary may differ from the float64 statement."""
+    rows = 32
+    params = SamplingParams(temperature=0.8, top_k=40, top_p=0.9, repetition_penalty=1.3, repetition_window=8)
+    lg = _logits(rows, vocab, 21)
+    hist = torch.randint(0, vocab, (rows, 12), generator=torch.Generator().manual_seed(3))
+    hist[:, 9] = hist[:, 7]
+    dev = DeviceSampler(params, rows, vocab, range(rows), "cuda", history_len=16)
+    dev.set_history(hist)
+    got = dev.sample(lg.cuda()).cpu().tolist()
+    same = sum(got[b] == _exact_pick(lg[b], params, hist[b].tolist(), SamplerRng(b).next_uniform()) for b in range(rows))
+    assert same >= rows - 1
