@@ -220,3 +220,14 @@ def test_driver_smoke_entry_runs_training_decode_and_batched_decode():
     bf16 and int8 weights (the weight-streaming GEMM and its W8A8 form)."""
     import __graft_entry__ as entry
     entry.smoke()
+
+
+@pytest.mark.parametrize("K,N", [(1, 8), (7, 24), (8, 2048), (65, 4104), (9, 20), (33, 13)])
+def test_dequantize_is_the_rounded_product(K, N):
+    """Whole 8-byte words (one thread per eight columns, eight rows at a time) and rows that are not: the same bits as
+    bf16(code * scale)."""
+    g = torch.Generator(device="cuda").manual_seed(K + N)
+    q = torch.randint(-128, 128, (K, N), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    scale = torch.rand(N, generator=g, device="cuda") * 0.01 + 1e-4
+    want = (q.float() * scale[None, :]).to(BF)
+    assert torch.equal(D.QuantWeight(q, scale).dequantize(), want)
