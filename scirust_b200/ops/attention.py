@@ -22,7 +22,7 @@ _lib.register("sb_attention_bwd", [_lib.vp, _lib.vp, _lib.vp, _lib.vp, _lib.vp, 
                                    _lib.i32, _lib.i32, _lib.i32, _lib.i32, _lib.i32, _lib.i32, _lib.f32,
                                    _lib.i32, _lib.vp, _lib.vp])
 
-# Head dimension 64 runs the kernel with two query tiles per CTA (output accumulator kept in tensor memory,
+# The forward pass runs the kernel with two query tiles per CTA (output accumulator kept in tensor memory,
 # rescaled only when a row maximum grows by more than 2^8); SB_ATT_FWD=single selects the one-tile kernel.
 FWD_TWO_TILES = os.environ.get("SB_ATT_FWD", "pair") != "single"
 
@@ -69,7 +69,7 @@ def attention_fwd(qkv, B, S, H, Hkv, dh, causal=True, scale=None, want_lse=True)
         raise ValueError("qkv must be a 2-D bf16 matrix with unit inner stride")
     out = _lib.empty((B * S, H * dh), torch.bfloat16, qkv.device)
     lse = _lib.empty((B, H, S), torch.float32, qkv.device) if want_lse else None
-    entry = "sb_attention_fwd_pp" if (FWD_TWO_TILES and dh == 64) else "sb_attention_fwd"
+    entry = "sb_attention_fwd_pp" if FWD_TWO_TILES else "sb_attention_fwd"
     _lib.call(entry, qkv.data_ptr(), out.data_ptr(), _lib.ptr(lse), B, S, H, Hkv, dh, qkv.stride(0),
               out.stride(0), float(scale), int(causal), _lib.status_word(qkv.device).data_ptr(), _lib.stream())
     _g.launch_count += 1

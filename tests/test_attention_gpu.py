@@ -71,3 +71,27 @@ def test_backward(B, S, H, Hkv, dh, causal, spill, monkeypatch):
     assert err < 3e-2 * max(1.0, ref.abs().max().item()), err
     d2 = A.attention_bwd(qkv, o, lse, do, B, S, H, Hkv, dh, causal=causal)
     assert torch.equal(d, d2)
+
+
+@pytest.mark.parametrize("B,S,H,Hkv", [(1, 1, 1, 1), (2, 127, 2, 1), (1, 129, 2, 2), (3, 256, 4, 1), (1, 257, 2, 1),
+                                       (2, 1000, 4, 2), (1, 2048, 8, 2)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_forward_two_tiles_head_dimension_128(B, S, H, Hkv, causal, monkeypatch):
+    """Tile edges of the two-tile kernel at 128 (second tile empty, one row, full; K in two stages, V in half tiles)
+    against the dense statement and, with growing keys (the accumulator is rescaled), the one-tile kernel: both keep P in
+    bf16 (2^-8 of each term), so they agree to 2^-7 of the largest value."""
+    dh = 128
+    qkv = _qkv(B, S, H, Hkv, dh, seed=S).float().reshape(B, S, H + 2 * Hkv, dh)
+    qkv[:, :, H:H + Hkv] *= (1.0 + 4.0 * torch.arange(S, device="cuda") / S).reshape(1, S, 1, 1)
+    qkv = qkv.reshape(B * S, -1).to(torch.bfloat16)
+    monkeypatch.setattr(A, "FWD_TWO_TILES", True)
+    o, lse = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal)
+    again, _ = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal)
+    monkeypatch.setattr(A, "FWD_TWO_TILES", False)
+    o1, lse1 = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal)
+    _lib.check_status()
+    o_ref, lse_ref = A.attention_ref(qkv, B, S, H, Hkv, dh, causal=causal)
+    assert torch.equal(o, again)
+    assert (o.float() - o_ref).abs().max().item() < 3e-2
+    assert (lse - lse_ref).abs().max().item() < 2e-2
+    assert (o.float() - o1.float()).abs().max().item() <= 2 ** -7 * o_ref.abs().max().item()
