@@ -281,8 +281,8 @@ def sumsq(g, out=None, accumulate=False):
             out.copy_(out + s if accumulate else s)
             return out
         return s
-    if out is None:
-        out = torch.zeros(1, dtype=torch.float32, device=g.device)
+    if out is None:      # every call writes it; only an accumulating one reads it first
+        out = torch.zeros(1, dtype=torch.float32, device=g.device) if accumulate else _lib.empty(1, torch.float32, g.device)
     part = _lib.empty((n + 4095) // 4096, torch.float32, g.device)
     _lib.call("sb_sumsq", g.data_ptr(), n, int(g.dtype == BF), part.data_ptr(), out.data_ptr(), int(accumulate),
               _lib.stream())

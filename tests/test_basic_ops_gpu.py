@@ -138,3 +138,17 @@ def test_deferred_status_raises_collective_timeout_one_poll_late():
     assert int(st.item()) == 0
     ds.poll()
     ds.poll()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [1, 4095, 4096, 4097, 32768 + 5, 1000003])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_sumsq_edges(dtype, n, offset):
+    """Whole and partial blocks of 4096, 16-byte aligned buffers and others, against float64: fp32 sums of up to 4096 + n / 4096
+    terms in a tree, 1e-5 relative; accumulation adds to what is there."""
+    g = _r((n + offset,), n).cuda().to(dtype)[offset:]
+    want = g.double().square().sum().item()
+    out = ops.sumsq(g)
+    assert abs(out.item() - want) <= 1e-5 * want
+    ops.sumsq(g, out=out, accumulate=True)
+    assert abs(out.item() - 2 * want) <= 2e-5 * want
