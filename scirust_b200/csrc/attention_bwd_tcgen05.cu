@@ -118,20 +118,26 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 }
 
 // --------------------------------------------------------------------------- dK / dV
-// Pipeline (DH == 64): the bf16 P^T / dS^T tiles are double-buffered in shared memory, so the MMA
-// warp issues the score products of iteration t+1 *before* the gradient products of iteration t;
-// the softmax warps then work on t+1 while the tensor cores finish t. With DH == 128 shared
-// memory only fits single buffers and the two groups are issued in program order.
+// Pipeline: scores and dP have barriers of their own, so the exponentials of iteration t+1 (which need the scores only)
+// run under the gradient products of iteration t, and dS follows when dP arrives. Order of the tensor work:
+//   S(t+1) | dV(t) += P(t)^T dO(t) | dK(t) += dS(t)^T Q(t) | dP(t+1)
+// S(t+1) needs Q(t+1), so Q has two stages; dO(t) is free after dV(t), two products before dP(t+1) needs its successor,
+// so at head dimension 128, where shared memory holds seven 32 KB tiles (K, V, 2 Q, dO, P, dS), one stage is enough.
+// P is single: dV(t) has read it (dv_done) long before the exponentials of t+1 are stored. Until then the two score
+// products of an iteration were one group, which the softmax warps waited for as a whole, and at 128 the loads,
+// the scores, the softmax and the gradient products of an iteration ran one after another: 2 x 2048 tokens of 32 heads,
+// causal, 241 us then and 176 us so (head dimension 64, 8 x 2048 tokens of 16 heads: 301 and 303 us).
 template <int DH>
 struct DkvCfg {
-  static constexpr bool PDB = (DH == 64);             // double-buffer P^T / dS^T
-  static constexpr int NPB = PDB ? 2 : 1;
-  static constexpr int QS = (DH == 64) ? 2 : 1;       // (Q, dO) ring stages
+  static constexpr int QS = 2;                        // Q stages
+  static constexpr int OS = (DH == 64) ? 2 : 1;       // dO stages
+  static constexpr int NDS = (DH == 64) ? 2 : 1;      // dS buffers (a bulk store may still read the older one)
   static constexpr int T_BYTES = BT * DH * 2;         // one [128 x DH] tile
   static constexpr int PT_BYTES = BT * BT * 2;
-  static constexpr int TILE_BYTES = 2 * T_BYTES + QS * 2 * T_BYTES + NPB * 2 * PT_BYTES;
-  static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 128;
-  static constexpr int TMEM_COLS = 512;  // S^T 128 | dP^T 128 | dK DH | dV DH
+  static constexpr int TILE_BYTES = (2 + QS + OS) * T_BYTES + (1 + NDS) * PT_BYTES;
+  static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 256;
+  static constexpr int TMEM_COLS = 512;  // S 128 | dP 128 | dK DH | dV DH
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 };
 
 template <int DH>
@@ -145,16 +151,21 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
   uint8_t* sK = smem;
   uint8_t* sV = sK + Cfg::T_BYTES;
   uint8_t* sQ = sV + Cfg::T_BYTES;                 // QS stages
-  uint8_t* sdO = sQ + Cfg::QS * Cfg::T_BYTES;      // QS stages
-  uint8_t* sPT = sdO + Cfg::QS * Cfg::T_BYTES;     // NPB buffers
-  uint8_t* sdST = sPT + Cfg::NPB * Cfg::PT_BYTES;  // NPB buffers
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sdST + Cfg::NPB * Cfg::PT_BYTES);
+  uint8_t* sdO = sQ + Cfg::QS * Cfg::T_BYTES;      // OS stages
+  uint8_t* sPT = sdO + Cfg::OS * Cfg::T_BYTES;
+  uint8_t* sdST = sPT + Cfg::PT_BYTES;             // NDS buffers
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sdST + Cfg::NDS * Cfg::PT_BYTES);
   uint64_t* kv_full = bars;
-  uint64_t* q_full = bars + 1;            // QS
-  uint64_t* q_empty = q_full + Cfg::QS;   // QS
-  uint64_t* st_full = q_empty + Cfg::QS;
-  uint64_t* p_full = st_full + 1;
-  uint64_t* done = p_full + 1;
+  uint64_t* q_full = bars + 1;             // QS
+  uint64_t* q_empty = q_full + Cfg::QS;    // QS
+  uint64_t* do_full = q_empty + Cfg::QS;   // OS
+  uint64_t* do_empty = do_full + Cfg::OS;  // OS
+  uint64_t* s_full = do_empty + Cfg::OS;   // scores of t are in tensor memory
+  uint64_t* dp_full = s_full + 1;          // dP of t is; every earlier product has completed and dS may be rewritten
+  uint64_t* p_full = dp_full + 1;          // P of t is in shared memory (8 warp arrivals), the scores have been read
+  uint64_t* ds_full = p_full + 1;          // dS of t is, dP has been read
+  uint64_t* dv_done = ds_full + 1;         // dV(t) has read P
+  uint64_t* done = dv_done + 1;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -173,8 +184,12 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int s = 0; s < Cfg::QS; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
-    mbar_init(st_full, 1);
+    for (int s = 0; s < Cfg::OS; ++s) { mbar_init(&do_full[s], 1); mbar_init(&do_empty[s], 1); }
+    mbar_init(s_full, 1);
+    mbar_init(dp_full, 1);
     mbar_init(p_full, 8);  // one arrival per softmax warp
+    mbar_init(ds_full, 8);
+    mbar_init(dv_done, 1);
     mbar_init(done, 1);
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -197,21 +212,25 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
         tma_load_2d(sK + c * (BT * 128), &tm_qkv, kv_full, (p.H + kvh) * DH + c * 64, row_base + kv0);
         tma_load_2d(sV + c * (BT * 128), &tm_qkv, kv_full, (p.H + p.Hkv + kvh) * DH + c * 64, row_base + kv0);
       }
-      int st = 0;
-      uint32_t ph = 0;
+      int qs = 0, os = 0;
+      uint32_t qph = 0, oph = 0;
       for (int t = 0; t < n_iter; ++t) {
         const int head = kvh * group + t / n_qt;
         const int qt = qt_first + t % n_qt;
-        if (!mbar_wait(&q_empty[st], ph ^ 1, p.status, ST_TIMEOUT_EMPTY)) break;
-        mbar_arrive_expect_tx(&q_full[st], 2 * Cfg::T_BYTES);
+        if (!mbar_wait(&q_empty[qs], qph ^ 1, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_arrive_expect_tx(&q_full[qs], Cfg::T_BYTES);
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-          tma_load_2d(sQ + st * Cfg::T_BYTES + c * (BT * 128), &tm_qkv, &q_full[st], head * DH + c * 64,
+        for (int c = 0; c < NCH; ++c)
+          tma_load_2d(sQ + qs * Cfg::T_BYTES + c * (BT * 128), &tm_qkv, &q_full[qs], head * DH + c * 64,
                       row_base + qt * BT);
-          tma_load_2d(sdO + st * Cfg::T_BYTES + c * (BT * 128), &tm_do, &q_full[st], head * DH + c * 64,
+        if (++qs == Cfg::QS) { qs = 0; qph ^= 1; }
+        if (!mbar_wait(&do_empty[os], oph ^ 1, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_arrive_expect_tx(&do_full[os], Cfg::T_BYTES);
+#pragma unroll
+        for (int c = 0; c < NCH; ++c)
+          tma_load_2d(sdO + os * Cfg::T_BYTES + c * (BT * 128), &tm_do, &do_full[os], head * DH + c * 64,
                       row_base + qt * BT);
-        }
-        if (++st == Cfg::QS) { st = 0; ph ^= 1; }
+        if (++os == Cfg::OS) { os = 0; oph ^= 1; }
       }
     }
   } else if (warp == 1) {
@@ -219,74 +238,69 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
       constexpr uint32_t idesc_s = make_idesc_bf16(BT, BT, false, false);   // [q x kv], both K-major
       constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, true, true);     // [kv x dh] = A^T B, both MN-major
       bool ok = mbar_wait(kv_full, 0, p.status, ST_TIMEOUT_FULL);
-      int st_s = 0;          // stage / phase of the next score issue
-      uint32_t ph_s = 0;
-      int st_g = 0;          // stage of the next gradient issue
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV);
-      auto issue_scores = [&]() -> bool {
-        if (!mbar_wait(&q_full[st_s], ph_s, p.status, ST_TIMEOUT_FULL)) return false;
+      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aPT = smem_u32(sPT);
+      int qn = 0, on = 0;            // stage and phase of the next score / dP product
+      uint32_t qn_ph = 0, on_ph = 0;
+      int qg = 0, og = 0;            // stage of the next dK / dV product
+      // D = A B^T over DH, both K-major
+      auto score_product = [&](uint32_t d, uint32_t a, uint32_t b) {
+#pragma unroll
+        for (int k = 0; k < DH / 16; ++k) {
+          const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
+          umma_bf16_ss(d, make_smem_desc(a + off, 16, 1024), make_smem_desc(b + off, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
+        }
+      };
+      // D += A^T B over the 128 query rows, 16 at a time in both operands
+      auto grad_product = [&](uint32_t d, uint32_t a, uint32_t b, bool acc) {
+#pragma unroll
+        for (int k = 0; k < BT / 16; ++k)
+          umma_bf16_ss(d, make_smem_desc(a + k * (16 * 128), BT * 128, 1024),
+                       make_smem_desc(b + k * (16 * 128), BT * 128, 1024), idesc_g, (acc || k > 0) ? 1u : 0u);
+      };
+      auto issue_s = [&]() -> bool {
+        if (!mbar_wait(&q_full[qn], qn_ph, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        const uint32_t bQ = smem_u32(sQ + st_s * Cfg::T_BYTES), bdO = smem_u32(sdO + st_s * Cfg::T_BYTES);
-#pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
-          const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
-          umma_bf16_ss(tm_ST, make_smem_desc(bQ + off, 16, 1024), make_smem_desc(aK + off, 16, 1024), idesc_s,
-                       k > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
-          const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
-          umma_bf16_ss(tm_dPT, make_smem_desc(bdO + off, 16, 1024), make_smem_desc(aV + off, 16, 1024), idesc_s,
-                       k > 0 ? 1u : 0u);
-        }
-        umma_commit(st_full);
-        if (++st_s == Cfg::QS) { st_s = 0; ph_s ^= 1; }
+        score_product(tm_ST, smem_u32(sQ + qn * Cfg::T_BYTES), aK);
+        umma_commit(s_full);
+        if (++qn == Cfg::QS) { qn = 0; qn_ph ^= 1; }
         return true;
       };
-      auto issue_grads = [&](int t) {
-        const int pb = Cfg::PDB ? (t & 1) : 0;
-        const uint32_t aPT = smem_u32(sPT + pb * Cfg::PT_BYTES), adST = smem_u32(sdST + pb * Cfg::PT_BYTES);
-        const uint32_t bQ = smem_u32(sQ + st_g * Cfg::T_BYTES), bdO = smem_u32(sdO + st_g * Cfg::T_BYTES);
-#pragma unroll
-        for (int k = 0; k < BT / 16; ++k) {   // k walks 16 query rows at a time in both operands
-          umma_bf16_ss(tm_dV, make_smem_desc(aPT + k * (16 * 128), BT * 128, 1024),
-                       make_smem_desc(bdO + k * (16 * 128), BT * 128, 1024), idesc_g, (t > 0 || k > 0) ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < BT / 16; ++k) {
-          umma_bf16_ss(tm_dK, make_smem_desc(adST + k * (16 * 128), BT * 128, 1024),
-                       make_smem_desc(bQ + k * (16 * 128), BT * 128, 1024), idesc_g, (t > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(&q_empty[st_g]);
-        if (++st_g == Cfg::QS) st_g = 0;
+      auto issue_dp = [&]() -> bool {
+        if (!mbar_wait(&do_full[on], on_ph, p.status, ST_TIMEOUT_FULL)) return false;
+        tc_fence_after();
+        // dp_full lets the softmax warps write the next dS buffer: its last bulk store must have been read out
+        if (p.spill_ds) tma_store_wait_read<Cfg::NDS - 1>();
+        score_product(tm_dPT, smem_u32(sdO + on * Cfg::T_BYTES), aV);
+        umma_commit(dp_full);
+        if (++on == Cfg::OS) { on = 0; on_ph ^= 1; }
+        return true;
       };
-      if (ok && n_iter > 0) ok = issue_scores();
+      if (n_iter > 0) ok = ok && issue_s() && issue_dp();
       for (int t = 0; t < n_iter && ok; ++t) {
+        const bool more = t + 1 < n_iter;
         if (!mbar_wait(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
         tc_fence_after();
-        // scores of t+1 first (double-buffered P^T / dS^T): the softmax warps wait for nothing else, and the
-        // commit of these scores also covers the gradient MMAs of t-1, which is what lets the softmax warps
-        // reuse the P^T / dS^T buffer of parity (t+1)&1
-        // (the dS store of t-1 has long been read out of its buffer; the wait only makes that certain before the
-        // scores whose completion lets the softmax warps write that buffer again)
-        if (p.spill_ds) tma_store_wait_read<0>();
-        if (Cfg::PDB && t + 1 < n_iter) ok = issue_scores();
+        if (more && !issue_s()) { ok = false; break; }
+        grad_product(tm_dV, aPT, smem_u32(sdO + og * Cfg::T_BYTES), t > 0);
+        umma_commit(dv_done);
+        umma_commit(&do_empty[og]);
+        if (++og == Cfg::OS) og = 0;
+        if (!mbar_wait(ds_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
+        tc_fence_after();
+        const uint8_t* ds = sdST + (Cfg::NDS == 2 ? (t & 1) : 0) * Cfg::PT_BYTES;
         if (p.spill_ds) {
           // the finished dS tile (bf16, [q rows][kv], scale included) also goes to global memory, where
-          // the dQ kernel streams it back instead of recomputing scores; the bulk store reads shared
-          // memory asynchronously, so it must have been read out before this buffer is written again
+          // the dQ kernel streams it back instead of recomputing scores
           const int head = kvh * group + t / n_qt;
           const int qt = qt_first + t % n_qt;
-          const uint8_t* src = sdST + (Cfg::PDB ? (t & 1) : 0) * Cfg::PT_BYTES;
-          tma_store_3d(&tm_ds, src, kv0, qt * BT, b * p.H + head);
-          tma_store_3d(&tm_ds, src + BT * 128, kv0 + 64, qt * BT, b * p.H + head);
+          tma_store_3d(&tm_ds, ds, kv0, qt * BT, b * p.H + head);
+          tma_store_3d(&tm_ds, ds + BT * 128, kv0 + 64, qt * BT, b * p.H + head);
           tma_store_commit();
         }
-        issue_grads(t);
-        if (!Cfg::PDB) {
-          if (p.spill_ds) tma_store_wait_read<0>();   // single dS buffer: read out before it is rewritten
-          if (t + 1 < n_iter) ok = issue_scores();
-        }
+        grad_product(tm_dK, smem_u32(ds), smem_u32(sQ + qg * Cfg::T_BYTES), t > 0);
+        umma_commit(&q_empty[qg]);
+        if (++qg == Cfg::QS) qg = 0;
+        if (more && !issue_dp()) { ok = false; break; }
       }
       if (ok) umma_commit(done);
       if (p.spill_ds) tma_store_wait<0>();   // the stores are complete before the CTA retires
@@ -298,7 +312,6 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
     const int r = q * 32 + lane;    // row inside the tile == TMEM lane (query row in the loop, kv row at the end)
     const int kv_idx = kv0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    const float delta_scale = p.scale;
     bool ok = true;
     for (int t = 0; t < n_iter; ++t) {
       const int head = kvh * group + t / n_qt;
@@ -306,31 +319,64 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
       const int q0 = qt * BT;
       const int q_idx = q0 + r;
       const float2 sd = __ldg(p.stats + (static_cast<size_t>(b) * p.H + head) * p.S + min(q_idx, p.S - 1));
-      const int pb = Cfg::PDB ? (t & 1) : 0;
-      uint8_t* pt_buf = sPT + pb * Cfg::PT_BYTES;
-      uint8_t* dst_buf = sdST + pb * Cfg::PT_BYTES;
+      uint8_t* dst_buf = sdST + (Cfg::NDS == 2 ? (t & 1) : 0) * Cfg::PT_BYTES;
       // last visible kv column of this query row inside the tile (-1: row is past the sequence end)
       const bool diag = p.causal && qt == kt;
       int lim = min(diag ? r : BT - 1, p.S - 1 - kv0);
       if (q_idx >= p.S) lim = -1;
       const bool need_mask = diag || (q0 + BT > p.S) || (kv0 + BT > p.S);
-      if (!mbar_wait(st_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait(s_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
+      // P = 2^(s * sl2 - lse2), kept in fp32 registers for dS
+      uint32_t pv[64];
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) tmem_ld_32x32(tm_ST + lane_off + (half * 2 + cc) * 32, pv + cc * 32);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 64; i += 2) {
+        fma2(pv[i], pv[i + 1], p.scale_log2, -sd.x);
+        pv[i] = __float_as_uint(fast_exp2(__uint_as_float(pv[i])));
+        pv[i + 1] = __float_as_uint(fast_exp2(__uint_as_float(pv[i + 1])));
+      }
       if (need_mask) {
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc)
-          bwd_chunk<true, true>(tm_ST, tm_dPT, lane_off, half * 2 + cc, r, lim, p.scale_log2, sd.x,
-                                sd.y * delta_scale, p.scale, pt_buf, dst_buf);
-      } else {
+        for (int i = 0; i < 64; ++i)
+          if (half * 64 + i > lim) pv[i] = 0u;
+      }
+      if (t > 0 && !mbar_wait(dv_done, (t - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc)
-          bwd_chunk<false, true>(tm_ST, tm_dPT, lane_off, half * 2 + cc, r, lim, p.scale_log2, sd.x,
-                                 sd.y * delta_scale, p.scale, pt_buf, dst_buf);
+      for (int cc = 0; cc < 2; ++cc) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2)
+          pk[i >> 1] = pack_bf16x2(__uint_as_float(pv[cc * 32 + i]), __uint_as_float(pv[cc * 32 + i + 1]));
+        store_row32_sw128(sPT, r, half * 2 + cc, pk);
       }
       tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
+      // dS = P * (dP * scale - delta * scale)
+      if (!mbar_wait(dp_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      tc_fence_after();
+      const float neg_delta = -sd.y * p.scale;
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) {
+        uint32_t dv[32], dk[16];
+        tmem_ld_32x32(tm_dPT + lane_off + (half * 2 + cc) * 32, dv);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          fma2(dv[i], dv[i + 1], p.scale, neg_delta);
+          mul2(dv[i], dv[i + 1], __uint_as_float(pv[cc * 32 + i]), __uint_as_float(pv[cc * 32 + i + 1]));
+          dk[i >> 1] = pack_bf16x2(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1]));
+        }
+        store_row32_sw128(dst_buf, r, half * 2 + cc, dk);
+      }
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_full);
     }
     if (ok && mbar_wait(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();

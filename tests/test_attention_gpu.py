@@ -95,3 +95,19 @@ def test_forward_two_tiles_head_dimension_128(B, S, H, Hkv, causal, monkeypatch)
     assert (o.float() - o_ref).abs().max().item() < 3e-2
     assert (lse - lse_ref).abs().max().item() < 2e-2
     assert (o.float() - o1.float()).abs().max().item() <= 2 ** -7 * o_ref.abs().max().item()
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,dh", [(1, 1, 1, 1, 128), (1, 129, 4, 1, 128), (2, 640, 8, 2, 128), (1, 640, 6, 2, 64),
+                                          (3, 255, 2, 2, 64)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_backward_pipeline_edges(B, S, H, Hkv, dh, causal):
+    """One iteration, an odd and an even number, several heads per kv head: the dK / dV pipeline with its single P buffer
+    (and, at 128, single dO and dS) against the fp32 statement, twice with the same bits."""
+    qkv = _qkv(B, S, H, Hkv, dh, seed=7)
+    do = torch.randn(B * S, H * dh, generator=torch.Generator(device="cuda").manual_seed(8), device="cuda").to(torch.bfloat16)
+    o, lse = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal)
+    d = A.attention_bwd(qkv, o, lse, do, B, S, H, Hkv, dh, causal=causal)
+    assert torch.equal(d, A.attention_bwd(qkv, o, lse, do, B, S, H, Hkv, dh, causal=causal))
+    _lib.check_status()
+    ref = A.attention_bwd_ref(qkv, do, B, S, H, Hkv, dh, causal=causal)
+    assert (d.float() - ref).abs().max().item() < 3e-2 * max(1.0, ref.abs().max().item())
