@@ -15,9 +15,10 @@
 // CTA per row the passes over global memory set the pace, whatever the number of rows. A row is spread over the
 // shared memory of a cluster instead: eight CTAs hold 64 KB each, a pass takes 16 words per thread, and the CTAs
 // exchange only their 256-bin histograms (distributed shared memory, one cluster barrier per radix level, two
-// histogram buffers in turn). The bin scan runs in every warp by shuffles instead of in one thread, the number of
+// histogram buffers in turn). The bin scan runs in one warp by shuffles instead of in one thread, the number of
 // ties falls out of the last level, and the second walk starts from the first walk's top-level histogram. 16 rows of
-// 128256 logits, top-k 50, top-p 0.95: 418 us with one CTA per row, 147 us so.
+// 128256 logits, top-k 50, top-p 0.95: 418 us with one CTA per row, 78 us so (147 us while all 32 warps scanned the bins
+// of every level, eight neighbours to a lane and so sixteen lanes to a bank).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -58,10 +59,17 @@ struct SampHist {
   };
 };
 
+// The bins of a level over the cluster: a lane scans eight neighbours, so bin d lies at d + d / 8 (a stride of nine words
+// between lanes; eight would put 16 lanes on one bank).
+constexpr int SAMP_BINS = 256 + 32;
+__device__ __forceinline__ int samp_bin(int d) { return d + (d >> 3); }
+
 struct SampShared {
   SampHist h[2];
-  unsigned long long tot_cnt[256], tot_sum[256];   // of the level being scanned, over the cluster
-  unsigned long long top_cnt[256], top_sum[256];   // level 0 of the first walk
+  unsigned long long tot_cnt[SAMP_BINS], tot_sum[SAMP_BINS];   // of the level being scanned, over the cluster
+  unsigned long long top_cnt[SAMP_BINS], top_sum[SAMP_BINS];   // level 0 of the first walk
+  int cut_d;                                       // result of the scan
+  unsigned long long cut_cnt, cut_sum, in_cnt, in_sum;
   unsigned long long total;                        // this CTA's weight sum
   float vmax;                                      // this CTA's maximum (greedy: the value at vid)
   int vid;
@@ -101,11 +109,10 @@ __device__ __forceinline__ void hist_add(SampHist& h, int d, uint32_t c, unsigne
   else atomicAdd(&h.sum[d], s);
 }
 
-// Sums the cluster's histograms into tot_cnt / tot_sum and clears the buffer of the next level. `all_cnt` / `all_sum`
-// are the totals over the 256 bins, from which bin 0 follows (its elements, usually the most, are never counted).
+// Sums the cluster's histograms into tot_cnt / tot_sum (bin 0, usually the fullest, is not counted: the scan gets it from
+// the totals) and clears the buffer of the next level.
 template <bool SMEM>
-__device__ void combine(cg::cluster_group& cl, SampShared& s, int buf, unsigned long long all_cnt,
-                        unsigned long long all_sum) {
+__device__ void combine(cg::cluster_group& cl, SampShared& s, int buf) {
   cl.sync();
   const int t = threadIdx.x;
   if (t < 256) {
@@ -120,8 +127,8 @@ __device__ void combine(cg::cluster_group& cl, SampShared& s, int buf, unsigned 
         else v += h->sum[t];
       }
     }
-    s.tot_cnt[t] = c;
-    s.tot_sum[t] = v;
+    s.tot_cnt[samp_bin(t)] = c;
+    s.tot_sum[samp_bin(t)] = v;
   } else if (t < 512) {
     // every CTA has read this buffer's previous level before it arrived at the barrier above
     SampHist& h = s.h[buf ^ 1];
@@ -129,57 +136,51 @@ __device__ void combine(cg::cluster_group& cl, SampShared& s, int buf, unsigned 
     h.sum[t - 256] = 0;
   }
   __syncthreads();
-  if (t < 32) {
-    unsigned long long c = 0, v = 0;
-    for (int i = t; i < 256; i += 32) if (i) { c += s.tot_cnt[i]; v += s.tot_sum[i]; }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      c += __shfl_xor_sync(0xffffffffu, c, o);
-      v += __shfl_xor_sync(0xffffffffu, v, o);
-    }
-    if (t == 0) { s.tot_cnt[0] = all_cnt - c; s.tot_sum[0] = all_sum - v; }
-  }
-  __syncthreads();
 }
 
-struct Cut { int d; unsigned long long cnt, sum; };   // chosen digit; counts and sums of everything ranked above it
-
 // The first digit, from 255 down, where the running count reaches limit_count or the running sum reaches target
-// (passes it when `strict`); digit 0 when none above does. Every warp scans all 256 bins (8 per lane).
-__device__ Cut scan_bins(const unsigned long long* cnt, const unsigned long long* sum, unsigned long long cnt_before,
-                         unsigned long long sum_before, unsigned long long limit_count, unsigned long long target,
-                         bool strict) {
-  const int lane = threadIdx.x & 31;
-  const int hi = 255 - 8 * lane;                 // this lane's bins: hi, hi - 1, ... hi - 7
-  unsigned long long c8 = 0, s8 = 0;
+// (passes it when `strict`); digit 0 when none above does. Warp 0 scans, eight bins per lane, all loads first; the
+// digit, the counts and sums of everything above it and its own go to s.cut_* and s.in_*. in_cnt / in_sum: totals over
+// the 256 bins.
+__device__ void scan_bins(SampShared& s, const unsigned long long* cnt, const unsigned long long* sum,
+                          unsigned long long in_cnt, unsigned long long in_sum, unsigned long long cnt_before,
+                          unsigned long long sum_before, unsigned long long limit_count, unsigned long long target,
+                          bool strict) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const int hi = 255 - 8 * lane;                 // this lane's bins: hi, hi - 1, ... hi - 7
+    unsigned long long cb[8], sb_[8], c8 = 0, s8 = 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) { c8 += cnt[hi - i]; s8 += sum[hi - i]; }
-  unsigned long long c = c8, v = s8;             // inclusive over lanes
+    for (int i = 0; i < 8; ++i) { cb[i] = cnt[samp_bin(hi - i)]; sb_[i] = sum[samp_bin(hi - i)]; }
+    if (lane == 31) cb[7] = sb_[7] = 0;            // bin 0 is set below
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long pc = __shfl_up_sync(0xffffffffu, c, o), ps = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) { c += pc; v += ps; }
-  }
-  c += cnt_before - c8;
-  v += sum_before - s8;                          // before this lane's first bin
-  Cut k;
-  k.d = 0; k.cnt = c; k.sum = v;
-  bool found = false;
+    for (int i = 0; i < 8; ++i) { c8 += cb[i]; s8 += sb_[i]; }
+    unsigned long long c = c8, v = s8;             // inclusive over lanes
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int d = hi - i;
-    const unsigned long long cd = cnt[d], ci = c + cd, si = v + sum[d];
-    if (!found && ((cd != 0 && (ci >= limit_count || (strict ? si > target : si >= target))) || d == 0)) {
-      found = true;
-      k.d = d; k.cnt = c; k.sum = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long pc = __shfl_up_sync(0xffffffffu, c, o), ps = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) { c += pc; v += ps; }
     }
-    c = ci; v = si;
+    if (lane == 31) { cb[7] = in_cnt - c; sb_[7] = in_sum - v; }
+    c += cnt_before - c8;
+    v += sum_before - s8;                          // before this lane's first bin
+    int d = 0;
+    unsigned long long kc = c, ks = v, kic = 0, kis = 0;
+    bool found = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const unsigned long long ci = c + cb[i], si = v + sb_[i];
+      if (!found && ((cb[i] != 0 && (ci >= limit_count || (strict ? si > target : si >= target))) || hi - i == 0)) {
+        found = true;
+        d = hi - i; kc = c; ks = v; kic = cb[i]; kis = sb_[i];
+      }
+      c = ci; v = si;
+    }
+    if (lane == __ffs(__ballot_sync(0xffffffffu, found)) - 1) {     // lane 31 always finds bin 0
+      s.cut_d = d; s.cut_cnt = kc; s.cut_sum = ks; s.in_cnt = kic; s.in_sum = kis;
+    }
   }
-  const int src = __ffs(__ballot_sync(0xffffffffu, found)) - 1;   // lane 31 always finds bin 0
-  k.d = __shfl_sync(0xffffffffu, k.d, src);
-  k.cnt = __shfl_sync(0xffffffffu, k.cnt, src);
-  k.sum = __shfl_sync(0xffffffffu, k.sum, src);
-  return k;
+  __syncthreads();
 }
 
 struct Walk {                   // result of one ranked walk
@@ -223,21 +224,21 @@ __device__ Walk ranked_walk(cg::cluster_group& cl, SampShared& s, const Row<SMEM
         }
       });
       if (c_run) hist_add<SMEM>(h, cur, c_run, s_run, lo, hi);
-      combine<SMEM>(cl, s, buf, in_cnt, in_sum);
+      combine<SMEM>(cl, s, buf);
       buf ^= 1;
-      if (level == 0 && threadIdx.x < 256) {
+      if (level == 0 && threadIdx.x < SAMP_BINS) {
         s.top_cnt[threadIdx.x] = s.tot_cnt[threadIdx.x];
         s.top_sum[threadIdx.x] = s.tot_sum[threadIdx.x];
       }
     }
-    const Cut k = scan_bins(tc, ts, cnt_before, sum_before, limit_count, target, strict);
-    prefix |= static_cast<uint32_t>(k.d) << shift;
-    in_cnt = tc[k.d];
-    in_sum = ts[k.d];
-    cnt_before = k.cnt;
-    sum_before = k.sum;
+    scan_bins(s, tc, ts, in_cnt, in_sum, cnt_before, sum_before, limit_count, target, strict);
+    prefix |= static_cast<uint32_t>(s.cut_d) << shift;
+    in_cnt = s.in_cnt;
+    in_sum = s.in_sum;
+    cnt_before = s.cut_cnt;
+    sum_before = s.cut_sum;
+    __syncthreads();                               // all have read the cut
   }
-  __syncthreads();
   // all elements with weight == prefix are tied; they are taken in id order
   const unsigned long long v = prefix;
   Walk out;
