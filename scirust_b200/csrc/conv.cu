@@ -42,25 +42,42 @@ __global__ void im2col_nhwc_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfl
   col[idx] = v;
 }
 
-// The same gather, eight channels (16 bytes) per thread, for C a multiple of 8 (every layer but an RGB stem): one
-// index decomposition per 16-byte word instead of per element, and 16-byte loads and stores.
-__global__ void im2col_nhwc_vec8_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, int B, int H, int W,
-                                        int C8, int KH, int KW, int stride, int pad, int OH, int OW, int Kp8) {
-  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t total = static_cast<size_t>(B) * OH * OW * Kp8;
+// Division of a 31-bit value by a launch constant: one multiply-high and a shift (the magic number rounds up, exact for
+// n < 2^31). The index arithmetic below would otherwise spend several hundred instructions per 16-byte word on
+// 64-bit divisions.
+struct FastDiv {
+  uint32_t d, mul, sh;
+  __host__ explicit FastDiv(int div) : d(static_cast<uint32_t>(div)), mul(0), sh(0) {
+    if (d <= 1) return;
+    while ((1u << sh) < d) ++sh;                       // ceil(log2 d)
+    mul = static_cast<uint32_t>(((1ull << (31 + sh)) + d - 1) / d);
+    --sh;
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return d <= 1 ? n : __umulhi(n, mul) >> sh; }
+  __device__ __forceinline__ uint32_t divmod(uint32_t n, uint32_t& r) const {
+    const uint32_t q = div(n);
+    r = n - q * d;
+    return q;
+  }
+};
+
+// The same gather, eight channels (16 bytes) per thread, for C a multiple of 8 (every layer but an RGB stem): bound by
+// the bytes of the patch matrix it writes (86 us with 64-bit divisions for 128 x 32 x 32 x 64, 3 x 3).
+__global__ void __launch_bounds__(256)
+im2col_nhwc_vec8_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, uint32_t total, int H, int W, int C8,
+                        int taps8, int stride, int pad, FastDiv by_kp8, FastDiv by_ow, FastDiv by_oh, FastDiv by_c8,
+                        FastDiv by_kw) {
+  const uint32_t idx = blockIdx.x * 256u + threadIdx.x;
   if (idx >= total) return;
-  const int k8 = static_cast<int>(idx % Kp8);
-  const size_t row = idx / Kp8;
-  const int ow = static_cast<int>(row % OW);
-  const int oh = static_cast<int>((row / OW) % OH);
-  const int b = static_cast<int>(row / (static_cast<size_t>(OW) * OH));
+  uint32_t k8, ow, oh, c8, kw;
+  const uint32_t row = by_kp8.divmod(idx, k8);
+  const uint32_t b = by_oh.divmod(by_ow.divmod(row, ow), oh);
   uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  if (k8 < KH * KW * C8) {
-    const int c8 = k8 % C8;
-    const int kw = (k8 / C8) % KW;
-    const int kh = k8 / (C8 * KW);
-    const int ih = oh * stride - pad + kh, iw = ow * stride - pad + kw;
-    if (ih >= 0 && ih < H && iw >= 0 && iw < W) v = __ldg(x + ((static_cast<size_t>(b) * H + ih) * W + iw) * C8 + c8);
+  if (k8 < static_cast<uint32_t>(taps8)) {
+    const uint32_t kh = by_kw.divmod(by_c8.divmod(k8, c8), kw);
+    const int ih = static_cast<int>(oh) * stride - pad + static_cast<int>(kh);
+    const int iw = static_cast<int>(ow) * stride - pad + static_cast<int>(kw);
+    if (ih >= 0 && ih < H && iw >= 0 && iw < W) v = __ldg(x + (static_cast<size_t>(b * H + ih) * W + iw) * C8 + c8);
   }
   col[idx] = v;
 }
@@ -72,28 +89,29 @@ __device__ __forceinline__ uint32_t conv_pack(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// col2im, eight channels per thread; the taps are added in the same ascending (kh, kw) order as the scalar kernel
-__global__ void col2im_nhwc_vec8_kernel(const uint4* __restrict__ dcol, uint4* __restrict__ dx, int B, int H, int W,
-                                        int C8, int KH, int KW, int stride, int pad, int OH, int OW, int Kp8) {
-  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t total = static_cast<size_t>(B) * H * W * C8;
+// col2im, eight channels per thread; the taps are added in the same ascending (kh, kw) order as the scalar kernel.
+// STRIDE 1 and 2 are compiled in (0: any), so that the tap test needs no division.
+template <int STRIDE>
+__global__ void __launch_bounds__(256)
+col2im_nhwc_vec8_kernel(const uint4* __restrict__ dcol, uint4* __restrict__ dx, uint32_t total, int C8, int KH, int KW,
+                        int stride_, int pad, int OH, int OW, int Kp8, FastDiv by_c8, FastDiv by_w, FastDiv by_h) {
+  const uint32_t idx = blockIdx.x * 256u + threadIdx.x;
   if (idx >= total) return;
-  const int c8 = static_cast<int>(idx % C8);
-  const int iw = static_cast<int>((idx / C8) % W);
-  const int ih = static_cast<int>((idx / (static_cast<size_t>(C8) * W)) % H);
-  const int b = static_cast<int>(idx / (static_cast<size_t>(C8) * W * H));
+  const int stride = STRIDE ? STRIDE : stride_;
+  uint32_t c8, iw, ih;
+  const uint32_t b = by_h.divmod(by_w.divmod(by_c8.divmod(idx, c8), iw), ih);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int kh = 0; kh < KH; ++kh) {
-    const int th = ih + pad - kh;
+    const int th = static_cast<int>(ih) + pad - kh;
     if (th < 0 || th % stride) continue;
     const int oh = th / stride;
     if (oh >= OH) continue;
     for (int kw = 0; kw < KW; ++kw) {
-      const int tw = iw + pad - kw;
+      const int tw = static_cast<int>(iw) + pad - kw;
       if (tw < 0 || tw % stride) continue;
       const int ow = tw / stride;
       if (ow >= OW) continue;
-      const uint4 v = __ldg(dcol + ((static_cast<size_t>(b) * OH + oh) * OW + ow) * Kp8 + (kh * KW + kw) * C8 + c8);
+      const uint4 v = __ldg(dcol + (static_cast<size_t>(b * OH + oh) * OW + ow) * Kp8 + (kh * KW + kw) * C8 + c8);
       acc[0] += conv_bf_lo(v.x); acc[1] += conv_bf_hi(v.x); acc[2] += conv_bf_lo(v.y); acc[3] += conv_bf_hi(v.y);
       acc[4] += conv_bf_lo(v.z); acc[5] += conv_bf_hi(v.z); acc[6] += conv_bf_lo(v.w); acc[7] += conv_bf_hi(v.w);
     }
@@ -187,14 +205,17 @@ __global__ void maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const u
 // Column statistics of a [rows, C] matrix in two fixed-order stages.
 // stage 1: partial[chunk][0][c] = sum x, partial[chunk][1][c] = sum x*y (y = x for variance, or a
 // second matrix for the backward dot products). 256 rows per chunk, rows visited in order.
+// `mask` (optional): rows of a count only where mask > 0 (the ReLU that followed the forward pass).
 __global__ void colstats_partial_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
-                                        float* __restrict__ partial, int rows, int C) {
+                                        const __nv_bfloat16* __restrict__ mask, float* __restrict__ partial, int rows,
+                                        int C) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const int r0 = blockIdx.y * 256, r1 = min(rows, r0 + 256);
   float s1 = 0.f, s2 = 0.f;
   for (int r = r0; r < r1; ++r) {
-    const float x = __bfloat162float(a[static_cast<size_t>(r) * C + c]);
+    float x = __bfloat162float(a[static_cast<size_t>(r) * C + c]);
+    if (mask && !(__bfloat162float(mask[static_cast<size_t>(r) * C + c]) > 0.f)) x = 0.f;
     const float y = __bfloat162float(b[static_cast<size_t>(r) * C + c]);
     s1 += x;
     s2 += x * y;
@@ -202,17 +223,159 @@ __global__ void colstats_partial_kernel(const __nv_bfloat16* __restrict__ a, con
   partial[(static_cast<size_t>(blockIdx.y) * 2 + 0) * C + c] = s1;
   partial[(static_cast<size_t>(blockIdx.y) * 2 + 1) * C + c] = s2;
 }
-__global__ void colstats_finish_kernel(const float* __restrict__ partial, int chunks, int C, float* __restrict__ s1,
-                                       float* __restrict__ s2) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  float a = 0.f, b = 0.f;
-  for (int k = 0; k < chunks; ++k) {
-    a += partial[(static_cast<size_t>(k) * 2 + 0) * C + c];
-    b += partial[(static_cast<size_t>(k) * 2 + 1) * C + c];
+__device__ __forceinline__ void conv_unpack8(const uint4& v, float (&f)[8]) {
+  f[0] = conv_bf_lo(v.x); f[1] = conv_bf_hi(v.x); f[2] = conv_bf_lo(v.y); f[3] = conv_bf_hi(v.y);
+  f[4] = conv_bf_lo(v.z); f[5] = conv_bf_hi(v.z); f[6] = conv_bf_lo(v.w); f[7] = conv_bf_hi(v.w);
+}
+__device__ __forceinline__ uint4 conv_pack8(const float (&f)[8]) {
+  return make_uint4(conv_pack(f[0], f[1]), conv_pack(f[2], f[3]), conv_pack(f[4], f[5]), conv_pack(f[6], f[7]));
+}
+// a word of eight bf16 values where the same word of y is positive, else zero
+__device__ __forceinline__ uint4 conv_relu_mask8(uint4 g, const uint4& y) {
+  float f[8], m[8];
+  conv_unpack8(g, f);
+  conv_unpack8(y, m);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = m[j] > 0.f ? f[j] : 0.f;
+  return conv_pack8(f);
+}
+
+// Stage 1 of the backward sums for C a multiple of 8: bound by the bytes of the matrices. A block takes 64 columns (8 words of 16 bytes)
+// of a chunk of 256 rows, 32 row lanes of 8 rows each, all loads of a thread in flight; lanes, then warps are added in
+// a fixed order. The one-column-per-thread kernel above walks its 256 rows in one dependent chain of 2-byte loads: 39 us
+// for 131072 x 64, 8 us here.
+template <bool MASK>
+__global__ void __launch_bounds__(256)
+colstats_vec8_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, const uint4* __restrict__ mask,
+                     float* __restrict__ partial, int rows, int C8) {
+  __shared__ float s_sum[8][8][16];                 // [warp][column word][sum x: 8 | sum xy: 8]
+  const int cw = threadIdx.x & 7, rl = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c8 = blockIdx.x * 8 + cw;
+  const int r0 = blockIdx.y * 256 + rl;
+  float s1[8], s2[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) s1[j] = s2[j] = 0.f;
+  if (c8 < C8) {
+    uint4 va[8], vb[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = r0 + i * 32;
+      va[i] = vb[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (r < rows) {
+        const size_t at = static_cast<size_t>(r) * C8 + c8;
+        va[i] = __ldg(a + at);
+        vb[i] = __ldg(b + at);
+        if (MASK) va[i] = conv_relu_mask8(va[i], __ldg(mask + at));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float x[8], y[8];
+      conv_unpack8(va[i], x);
+      conv_unpack8(vb[i], y);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { s1[j] += x[j]; s2[j] += x[j] * y[j]; }
+    }
   }
-  s1[c] = a;
-  s2[c] = b;
+#pragma unroll
+  for (int o = 8; o < 32; o <<= 1) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      s1[j] += __shfl_xor_sync(0xffffffffu, s1[j], o);
+      s2[j] += __shfl_xor_sync(0xffffffffu, s2[j], o);
+    }
+  }
+  if (lane < 8) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { s_sum[warp][cw][j] = s1[j]; s_sum[warp][cw][8 + j] = s2[j]; }
+  }
+  __syncthreads();
+  if (threadIdx.x < 128) {
+    const int w = threadIdx.x >> 4, e = threadIdx.x & 15;      // column word, (sum, column in the word)
+    float v = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v += s_sum[i][w][e];
+    const int c = (blockIdx.x * 8 + w) * 8 + (e & 7);
+    if (c < C8 * 8) partial[(static_cast<size_t>(blockIdx.y) * 2 + (e >> 3)) * (C8 * 8) + c] = v;
+  }
+}
+
+// Stage 1 of the FORWARD statistics for even C, in the order of the kernel at the top: a column's 256 rows of a chunk in
+// one chain. Mean and variance decide on which side of zero a normalised value falls, and with it the ReLU mask, so the
+// order of these sums is kept to the bit; the loads are what is rearranged (a thread owns two columns and has 32 rows in
+// flight, a warp reads 128 contiguous bytes per row): 39 -> 10 us for 131072 x 64.
+__global__ void __launch_bounds__(128)
+colstats_chain_kernel(const uint32_t* __restrict__ a, float* __restrict__ partial, int rows, int C2) {
+  const int c2 = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int chunk = blockIdx.y * 4 + (threadIdx.x >> 5);
+  const int r0 = chunk * 256, r1 = min(rows, r0 + 256);
+  if (c2 >= C2 || r0 >= rows) return;
+  const uint32_t* p = a + static_cast<size_t>(r0) * C2 + c2;
+  float s1l = 0.f, s2l = 0.f, s1h = 0.f, s2h = 0.f;
+  int r = r0;
+  for (; r + 32 <= r1; r += 32, p += static_cast<size_t>(32) * C2) {
+    uint32_t v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __ldg(p + static_cast<size_t>(i) * C2);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const float x = conv_bf_lo(v[i]), y = conv_bf_hi(v[i]);
+      s1l += x;
+      s2l += x * x;
+      s1h += y;
+      s2h += y * y;
+    }
+  }
+  for (; r < r1; ++r, p += C2) {
+    const uint32_t v = __ldg(p);
+    const float x = conv_bf_lo(v), y = conv_bf_hi(v);
+    s1l += x;
+    s2l += x * x;
+    s1h += y;
+    s2h += y * y;
+  }
+  float* o = partial + static_cast<size_t>(chunk) * 4 * C2 + 2 * c2;    // [chunk][sum x | sum xx][C]
+  o[0] = s1l;
+  o[1] = s1h;
+  o[2 * C2] = s2l;
+  o[2 * C2 + 1] = s2h;
+}
+
+// Stage 2, chunks in ascending order: 32 columns per block. All threads bring 64 chunks at a time into shared memory
+// (the next 64 on their way meanwhile); the additions of a column, which are one chain, then run at shared-memory speed
+// instead of at a memory latency every few chunks (512 chunks: 28 -> 7 us).
+constexpr int CF_CHUNKS = 64;
+__global__ void __launch_bounds__(256)
+colstats_finish_kernel(const float* __restrict__ partial, int chunks, int C, float* __restrict__ s1,
+                       float* __restrict__ s2) {
+  __shared__ float s[CF_CHUNKS * 64];                    // [chunk][sum x: 32 | sum xy: 32]
+  constexpr int PER = CF_CHUNKS * 64 / 256;
+  const int e = threadIdx.x & 63, row0 = threadIdx.x >> 6;   // this thread's element of a chunk; its chunks row0 + 4 i
+  const int c = blockIdx.x * 32 + (e & 31);
+  const float* src = partial + static_cast<size_t>(e >> 5) * C + c;
+  float v[PER];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int k = k0 + row0 + 4 * i;
+      v[i] = (k < chunks && c < C) ? __ldg(src + static_cast<size_t>(k) * 2 * C) : 0.f;
+    }
+  };
+  fetch(0);
+  float acc = 0.f;
+  for (int k0 = 0; k0 < chunks; k0 += CF_CHUNKS) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; ++i) s[(row0 + 4 * i) * 64 + e] = v[i];
+    __syncthreads();
+    if (k0 + CF_CHUNKS < chunks) fetch(k0 + CF_CHUNKS);
+    if (threadIdx.x < 64) {
+      const int n = min(CF_CHUNKS, chunks - k0);
+#pragma unroll 16
+      for (int k = 0; k < n; ++k) acc += s[k * 64 + e];
+    }
+  }
+  if (threadIdx.x < 64 && c < C) (e < 32 ? s1 : s2)[c] = acc;
 }
 
 // BatchNorm forward (training): from column sums, mean/var (biased for normalisation), update
@@ -244,6 +407,32 @@ __global__ void bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float
   if (relu) v = fmaxf(v, 0.f);
   y[i] = __float2bfloat16_rn(v);
 }
+// Eight channels (16 bytes) per thread, for C a multiple of 8: bound by bytes, the per-channel values come from L1.
+__device__ __forceinline__ void conv_load8(const float* __restrict__ p, float (&f)[8]) {
+  const float4 u = __ldg(reinterpret_cast<const float4*>(p)), v = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  f[0] = u.x; f[1] = u.y; f[2] = u.z; f[3] = u.w; f[4] = v.x; f[5] = v.y; f[6] = v.z; f[7] = v.w;
+}
+__global__ void __launch_bounds__(256)
+bn_apply_vec8_kernel(const uint4* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ inv_std,
+                     const float* __restrict__ gamma, const float* __restrict__ beta, uint4* __restrict__ y,
+                     uint32_t total, FastDiv by_c8, int relu) {
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= total) return;
+  uint32_t c8;
+  by_c8.divmod(i, c8);
+  float v[8], m[8], s[8], g[8], b[8];
+  conv_unpack8(__ldg(x + i), v);
+  conv_load8(mean + c8 * 8, m);
+  conv_load8(inv_std + c8 * 8, s);
+  conv_load8(gamma + c8 * 8, g);
+  conv_load8(beta + c8 * 8, b);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    v[j] = (v[j] - m[j]) * s[j] * g[j] + b[j];
+    if (relu) v[j] = fmaxf(v[j], 0.f);
+  }
+  y[i] = conv_pack8(v);
+}
 // BatchNorm backward. With xhat = (x-mean)*inv_std, g = dy (already masked by ReLU when fused):
 //   dbeta = sum g, dgamma = sum g*xhat, dx = gamma*inv_std/n * (n*g - dbeta - xhat*dgamma)
 // sums come from colstats (a = g, b = x): sum g and sum g*x; dgamma = (sum g*x - mean*sum g)*inv_std.
@@ -258,15 +447,46 @@ __global__ void bn_bwd_finish_kernel(const float* __restrict__ sum_g, const floa
 __global__ void bn_bwd_dx_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ x,
                                  const float* __restrict__ mean, const float* __restrict__ inv_std,
                                  const float* __restrict__ gamma, const float* __restrict__ dgamma,
-                                 const float* __restrict__ dbeta, __nv_bfloat16* __restrict__ dx, size_t total,
-                                 int C, int rows) {
+                                 const float* __restrict__ dbeta, const __nv_bfloat16* __restrict__ mask,
+                                 __nv_bfloat16* __restrict__ dx, size_t total, int C, int rows) {
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int c = static_cast<int>(i % C);
   const float n = static_cast<float>(rows);
   const float xhat = (__bfloat162float(x[i]) - mean[c]) * inv_std[c];
-  const float v = gamma[c] * inv_std[c] / n * (n * __bfloat162float(g[i]) - dbeta[c] - xhat * dgamma[c]);
+  float gi = __bfloat162float(g[i]);
+  if (mask && !(__bfloat162float(mask[i]) > 0.f)) gi = 0.f;
+  const float v = gamma[c] * inv_std[c] / n * (n * gi - dbeta[c] - xhat * dgamma[c]);
   dx[i] = __float2bfloat16_rn(v);
+}
+template <bool MASK>
+__global__ void __launch_bounds__(256)
+bn_bwd_dx_vec8_kernel(const uint4* __restrict__ g, const uint4* __restrict__ x, const float* __restrict__ mean,
+                      const float* __restrict__ inv_std, const float* __restrict__ gamma,
+                      const float* __restrict__ dgamma, const float* __restrict__ dbeta,
+                      const uint4* __restrict__ mask, uint4* __restrict__ dx, uint32_t total, FastDiv by_c8, int rows) {
+  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= total) return;
+  uint32_t c8;
+  by_c8.divmod(i, c8);
+  const float n = static_cast<float>(rows);
+  uint4 gw = __ldg(g + i);
+  const uint4 xw = __ldg(x + i);
+  if (MASK) gw = conv_relu_mask8(gw, __ldg(mask + i));
+  float gi[8], xi[8], m[8], s[8], ga[8], dg[8], db[8];
+  conv_unpack8(gw, gi);
+  conv_unpack8(xw, xi);
+  conv_load8(mean + c8 * 8, m);
+  conv_load8(inv_std + c8 * 8, s);
+  conv_load8(gamma + c8 * 8, ga);
+  conv_load8(dgamma + c8 * 8, dg);
+  conv_load8(dbeta + c8 * 8, db);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float xhat = (xi[j] - m[j]) * s[j];
+    gi[j] = ga[j] * s[j] / n * (n * gi[j] - db[j] - xhat * dg[j]);
+  }
+  dx[i] = conv_pack8(gi);
 }
 // g = dy * (y > 0)
 __global__ void relu_mask_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ y,
@@ -290,15 +510,20 @@ __global__ void bias_act_kernel(const __nv_bfloat16* __restrict__ x, const float
 using namespace sb;
 #define STREAM static_cast<cudaStream_t>(stream)
 #define CHECK_LAUNCH() return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH
+static inline bool conv_al16(const void* a, const void* b, const void* c = nullptr, const void* d = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
+           reinterpret_cast<uintptr_t>(d)) & 15) == 0;
+}
 static inline unsigned nblk(size_t n) { return static_cast<unsigned>((n + 255) / 256); }
 
 extern "C" int sb_im2col_nhwc(const void* x, void* col, int B, int H, int W, int C, int KH, int KW, int stride,
                               int pad, int OH, int OW, int Kp, void* stream) {
   if (B <= 0 || Kp < KH * KW * C || (Kp & 7)) return SB_ERR_ARG;
   const size_t total = static_cast<size_t>(B) * OH * OW * Kp;
-  if ((C & 7) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(col)) & 15) == 0) {
-    im2col_nhwc_vec8_kernel<<<nblk(total / 8), 256, 0, STREAM>>>(static_cast<const uint4*>(x), static_cast<uint4*>(col),
-                                                                 B, H, W, C / 8, KH, KW, stride, pad, OH, OW, Kp / 8);
+  if ((C & 7) == 0 && total / 8 <= 0x7fffff00u && conv_al16(x, col)) {
+    im2col_nhwc_vec8_kernel<<<nblk(total / 8), 256, 0, STREAM>>>(
+        static_cast<const uint4*>(x), static_cast<uint4*>(col), static_cast<uint32_t>(total / 8), H, W, C / 8,
+        KH * KW * (C / 8), stride, pad, FastDiv(Kp / 8), FastDiv(OW), FastDiv(OH), FastDiv(C / 8), FastDiv(KW));
     CHECK_LAUNCH();
   }
   im2col_nhwc_kernel<<<nblk(total), 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x),
@@ -310,10 +535,11 @@ extern "C" int sb_col2im_nhwc(const void* dcol, void* dx, int B, int H, int W, i
                               int pad, int OH, int OW, int Kp, void* stream) {
   if (B <= 0 || Kp < KH * KW * C) return SB_ERR_ARG;
   const size_t total = static_cast<size_t>(B) * H * W * C;
-  if ((C & 7) == 0 && (Kp & 7) == 0 && ((reinterpret_cast<uintptr_t>(dcol) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0) {
-    col2im_nhwc_vec8_kernel<<<nblk(total / 8), 256, 0, STREAM>>>(static_cast<const uint4*>(dcol),
-                                                                 static_cast<uint4*>(dx), B, H, W, C / 8, KH, KW,
-                                                                 stride, pad, OH, OW, Kp / 8);
+  if ((C & 7) == 0 && (Kp & 7) == 0 && total / 8 <= 0x7fffff00u && conv_al16(dcol, dx)) {
+    auto kern = stride == 1 ? col2im_nhwc_vec8_kernel<1> : stride == 2 ? col2im_nhwc_vec8_kernel<2> : col2im_nhwc_vec8_kernel<0>;
+    kern<<<nblk(total / 8), 256, 0, STREAM>>>(static_cast<const uint4*>(dcol), static_cast<uint4*>(dx),
+                                              static_cast<uint32_t>(total / 8), C / 8, KH, KW, stride, pad, OH, OW,
+                                              Kp / 8, FastDiv(C / 8), FastDiv(W), FastDiv(H));
     CHECK_LAUNCH();
   }
   col2im_nhwc_kernel<<<nblk(total), 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(dcol),
@@ -339,16 +565,28 @@ extern "C" int sb_maxpool_bwd(const void* dy, const void* arg, void* dx, int B, 
                                                       static_cast<__nv_bfloat16*>(dx), B, H, W, C, k, stride, OH, OW);
   CHECK_LAUNCH();
 }
+// s1 = column sums of a, s2 = of a * b; `mask` (optional, same shape): elements of a count where mask > 0.
 // partial: 2 * ceil(rows/256) * C floats
-extern "C" int sb_colstats(const void* a, const void* b, float* partial, float* s1, float* s2, int rows, int C,
-                           void* stream) {
+extern "C" int sb_colstats_masked(const void* a, const void* b, const void* mask, float* partial, float* s1, float* s2,
+                                  int rows, int C, void* stream) {
   if (rows <= 0 || C <= 0) return SB_ERR_ARG;
   const int chunks = (rows + 255) / 256;
-  dim3 grid((C + 127) / 128, chunks);
-  colstats_partial_kernel<<<grid, 128, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(a),
-                                                    static_cast<const __nv_bfloat16*>(b), partial, rows, C);
+  if (a == b && !mask && (C & 1) == 0 && (reinterpret_cast<uintptr_t>(a) & 3) == 0 && (chunks + 3) / 4 <= 65535) {
+    colstats_chain_kernel<<<dim3((C / 2 + 31) / 32, (chunks + 3) / 4), 128, 0, STREAM>>>(static_cast<const uint32_t*>(a),
+                                                                                        partial, rows, C / 2);
+  } else if ((C & 7) == 0 && chunks <= 65535 && conv_al16(a, b, mask)) {
+    const dim3 grid((C / 8 + 7) / 8, chunks);
+    auto kern = mask ? colstats_vec8_kernel<true> : colstats_vec8_kernel<false>;
+    kern<<<grid, 256, 0, STREAM>>>(static_cast<const uint4*>(a), static_cast<const uint4*>(b),
+                                   static_cast<const uint4*>(mask), partial, rows, C / 8);
+  } else {
+    dim3 grid((C + 127) / 128, chunks);
+    colstats_partial_kernel<<<grid, 128, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(a),
+                                                      static_cast<const __nv_bfloat16*>(b),
+                                                      static_cast<const __nv_bfloat16*>(mask), partial, rows, C);
+  }
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
-  colstats_finish_kernel<<<(C + 127) / 128, 128, 0, STREAM>>>(partial, chunks, C, s1, s2);
+  colstats_finish_kernel<<<(C + 31) / 32, 256, 0, STREAM>>>(partial, chunks, C, s1, s2);
   CHECK_LAUNCH();
 }
 extern "C" int sb_bn_fwd(const void* x, const float* sum, const float* sumsq, const float* gamma, const float* beta,
@@ -361,21 +599,47 @@ extern "C" int sb_bn_fwd(const void* x, const float* sum, const float* sumsq, co
     if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   }
   const size_t total = static_cast<size_t>(rows) * C;
+  if ((C & 7) == 0 && total / 8 <= 0x7fffff00u && conv_al16(x, y) && conv_al16(mean, inv_std, gamma, beta)) {
+    bn_apply_vec8_kernel<<<nblk(total / 8), 256, 0, STREAM>>>(static_cast<const uint4*>(x), mean, inv_std, gamma, beta,
+                                                              static_cast<uint4*>(y), static_cast<uint32_t>(total / 8),
+                                                              FastDiv(C / 8), relu);
+    CHECK_LAUNCH();
+  }
   bn_apply_kernel<<<nblk(total), 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x), mean, inv_std, gamma, beta,
                                                    static_cast<__nv_bfloat16*>(y), total, C, relu);
   CHECK_LAUNCH();
 }
-extern "C" int sb_bn_bwd(const void* g, const void* x, const float* sum_g, const float* sum_gx, const float* mean,
-                         const float* inv_std, const float* gamma, float* dgamma, float* dbeta, void* dx, int rows,
-                         int C, void* stream) {
+// mask (optional): the forward output after a fused ReLU; g counts where it is positive (sum_g, sum_gx likewise).
+extern "C" int sb_bn_bwd_masked(const void* g, const void* x, const float* sum_g, const float* sum_gx,
+                                const float* mean, const float* inv_std, const float* gamma, float* dgamma,
+                                float* dbeta, const void* mask, void* dx, int rows, int C, void* stream) {
   if (rows <= 0 || C <= 0) return SB_ERR_ARG;
   bn_bwd_finish_kernel<<<(C + 127) / 128, 128, 0, STREAM>>>(sum_g, sum_gx, mean, inv_std, C, dgamma, dbeta);
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   const size_t total = static_cast<size_t>(rows) * C;
+  if ((C & 7) == 0 && total / 8 <= 0x7fffff00u && conv_al16(g, x, dx, mask) && conv_al16(mean, inv_std, gamma) &&
+      conv_al16(dgamma, dbeta)) {
+    auto kern = mask ? bn_bwd_dx_vec8_kernel<true> : bn_bwd_dx_vec8_kernel<false>;
+    kern<<<nblk(total / 8), 256, 0, STREAM>>>(static_cast<const uint4*>(g), static_cast<const uint4*>(x), mean, inv_std,
+                                              gamma, dgamma, dbeta, static_cast<const uint4*>(mask),
+                                              static_cast<uint4*>(dx), static_cast<uint32_t>(total / 8),
+                                              FastDiv(C / 8), rows);
+    CHECK_LAUNCH();
+  }
   bn_bwd_dx_kernel<<<nblk(total), 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(g),
                                                     static_cast<const __nv_bfloat16*>(x), mean, inv_std, gamma,
-                                                    dgamma, dbeta, static_cast<__nv_bfloat16*>(dx), total, C, rows);
+                                                    dgamma, dbeta, static_cast<const __nv_bfloat16*>(mask),
+                                                    static_cast<__nv_bfloat16*>(dx), total, C, rows);
   CHECK_LAUNCH();
+}
+extern "C" int sb_colstats(const void* a, const void* b, float* partial, float* s1, float* s2, int rows, int C,
+                           void* stream) {
+  return sb_colstats_masked(a, b, nullptr, partial, s1, s2, rows, C, stream);
+}
+extern "C" int sb_bn_bwd(const void* g, const void* x, const float* sum_g, const float* sum_gx, const float* mean,
+                         const float* inv_std, const float* gamma, float* dgamma, float* dbeta, void* dx, int rows,
+                         int C, void* stream) {
+  return sb_bn_bwd_masked(g, x, sum_g, sum_gx, mean, inv_std, gamma, dgamma, dbeta, nullptr, dx, rows, C, stream);
 }
 extern "C" int sb_relu_mask(const void* dy, const void* y, void* g, size_t total, void* stream) {
   if (total == 0) return SB_ERR_ARG;

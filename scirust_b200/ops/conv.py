@@ -19,10 +19,9 @@ _lib.register("sb_im2col_nhwc", [vp, vp] + [i32] * 11 + [vp])
 _lib.register("sb_col2im_nhwc", [vp, vp] + [i32] * 11 + [vp])
 _lib.register("sb_maxpool_fwd", [vp, vp, vp] + [i32] * 8 + [vp])
 _lib.register("sb_maxpool_bwd", [vp, vp, vp] + [i32] * 8 + [vp])
-_lib.register("sb_colstats", [vp, vp, vp, vp, vp, i32, i32, vp])
+_lib.register("sb_colstats_masked", [vp, vp, vp, vp, vp, vp, i32, i32, vp])
 _lib.register("sb_bn_fwd", [vp] * 10 + [i32, i32, f32, f32, i32, i32, vp])
-_lib.register("sb_bn_bwd", [vp] * 10 + [i32, i32, vp])
-_lib.register("sb_relu_mask", [vp, vp, vp, sz, vp])
+_lib.register("sb_bn_bwd_masked", [vp] * 11 + [i32, i32, vp])
 _lib.register("sb_bias_act", [vp, vp, vp, sz, i32, i32, vp])
 
 
@@ -142,12 +141,13 @@ def maxpool2d(x, geom: ConvGeom, k: int, stride: int):
     return _MaxPool.apply(x.contiguous(), geom, k, stride), og
 
 
-def _colstats(a, b):
+def _colstats(a, b, mask=None):
+    """Column sums of ``a`` and of ``a * b``; with ``mask`` only the elements of ``a`` where it is positive count."""
     rows, C = a.shape
     part = torch.empty(2 * ((rows + 255) // 256) * C, dtype=torch.float32, device=a.device)
     s1 = _lib.empty(C, torch.float32, a.device)
     s2 = _lib.empty(C, torch.float32, a.device)
-    _lib.call("sb_colstats", a.data_ptr(), b.data_ptr(), part.data_ptr(), s1.data_ptr(), s2.data_ptr(), rows, C,
+    _lib.call("sb_colstats_masked", a.data_ptr(), b.data_ptr(), _lib.ptr(mask), part.data_ptr(), s1.data_ptr(), s2.data_ptr(), rows, C,
               _lib.stream())
     G.launch_count += 2
     return s1, s2
@@ -180,18 +180,15 @@ class _BatchNorm(torch.autograd.Function):
         x, y, gamma, mean, inv = ctx.saved_tensors
         rows, C = x.shape
         dy = dy.contiguous()
-        g = dy
-        if ctx.relu:
-            g = torch.empty_like(dy)
-            _lib.call("sb_relu_mask", dy.data_ptr(), y.data_ptr(), g.data_ptr(), dy.numel(), _lib.stream())
-        sg, sgx = _colstats(g, x)
+        mask = y if ctx.relu else None                  # the ReLU's mask is applied where dy is read
+        sg, sgx = _colstats(dy, x, mask)
         dgamma = _lib.empty(C, torch.float32, x.device)
         dbeta = _lib.empty(C, torch.float32, x.device)
         dx = torch.empty_like(x)
-        _lib.call("sb_bn_bwd", g.data_ptr(), x.data_ptr(), sg.data_ptr(), sgx.data_ptr(), mean.data_ptr(),
-                  inv.data_ptr(), gamma.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), dx.data_ptr(), rows, C,
-                  _lib.stream())
-        G.launch_count += 3
+        _lib.call("sb_bn_bwd_masked", dy.data_ptr(), x.data_ptr(), sg.data_ptr(), sgx.data_ptr(), mean.data_ptr(),
+                  inv.data_ptr(), gamma.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), _lib.ptr(mask), dx.data_ptr(),
+                  rows, C, _lib.stream())
+        G.launch_count += 2
         return dx, dgamma, dbeta, None, None, None, None, None, None
 
 

@@ -96,3 +96,30 @@ def test_cnn_models_train_on_gpu():
             losses.append(float(loss.detach()))
         _lib.check_status()
         assert losses[-1] < losses[0], losses
+
+
+@pytest.mark.parametrize("rows,C_", [(1, 8), (255, 72), (257, 64), (1000, 200), (300, 12), (2050, 520)])
+@pytest.mark.parametrize("relu", [False, True])
+def test_batchnorm_row_and_column_edges(rows, C_, relu):
+    """Chunks of 256 rows, blocks of 64 columns, channels in whole 16-byte words or not, with the ReLU mask folded into
+    the backward sums: against the fp32 statement. Sums of n fp32 terms: n * 2^-24 relative at most; the results are
+    rounded to bf16 (2^-8)."""
+    g = torch.Generator(device="cuda").manual_seed(rows + C_)
+    x = torch.randn(rows, C_, generator=g, device="cuda").to(BF)
+    dy = torch.randn(rows, C_, generator=g, device="cuda").to(BF)
+    gamma, beta = torch.rand(C_, generator=g, device="cuda") + 0.5, torch.randn(C_, generator=g, device="cuda")
+    xi, gi, bi = x.clone().requires_grad_(True), gamma.clone().requires_grad_(True), beta.clone().requires_grad_(True)
+    rm, rv = torch.zeros(C_, device="cuda"), torch.ones(C_, device="cuda")
+    y = C.batchnorm(xi, gi, bi, rm, rv, relu=relu)
+    y.backward(dy)
+    # the mask is taken from the kernel's own output, so that a rounding near zero does not flip it
+    xr, gr, br = x.float().requires_grad_(True), gamma.clone().requires_grad_(True), beta.clone().requires_grad_(True)
+    mean, var = xr.mean(0), xr.var(0, unbiased=False)
+    yr = (xr - mean) * torch.rsqrt(var + 1e-5) * gr + br
+    yr.backward(dy.float() * (y > 0) if relu else dy.float())
+    _close(y, torch.relu(yr) if relu else yr, 1e-2)
+    if rows > 1:
+        _close(xi.grad, xr.grad, 1e-2)
+    _close(gi.grad, gr.grad, 1e-2)
+    _close(bi.grad, br.grad, 1e-2)
+    _close(rm, 0.1 * mean, 1e-4)
