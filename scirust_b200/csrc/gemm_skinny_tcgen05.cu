@@ -206,27 +206,49 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   if (warp == 1) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
 }
 
-// C[m, n] = bf16(sum over splits in split order (+ scales) + R[m, n])
+// C[m, n] = bf16(sum over splits in split order (+ scales) + R[m, n]). Four columns (16 bytes of every partial) per thread
+// with up to eight splits' loads in flight: the partials lie in L2, and a column per thread with one load after another
+// was bound by its latency. 64 rows of the three split products of an 8B layer: 4.9 -> 2.8 us each.
 template <bool I8>
-__global__ void skinny_reduce_kernel(const void* __restrict__ part, int splits, int rows, int N,
-                                     const float* __restrict__ sx, const float* __restrict__ sw,
-                                     const __nv_bfloat16* __restrict__ R, int ldr, __nv_bfloat16* __restrict__ C,
-                                     int ldc) {
-  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t mn = static_cast<size_t>(rows) * N;
-  if (i >= mn) return;
-  const int m = static_cast<int>(i / N), n = static_cast<int>(i - static_cast<size_t>(m) * N);
-  float v;
-  if constexpr (I8) {
-    int acc = 0;
-    for (int s = 0; s < splits; ++s) acc += static_cast<const int*>(part)[s * mn + i];
-    v = __fmul_rn(static_cast<float>(acc), __fmul_rn(sx[m], sw[n]));
-  } else {
-    v = static_cast<const float*>(part)[i];
-    for (int s = 1; s < splits; ++s) v += static_cast<const float*>(part)[s * mn + i];
+__global__ void __launch_bounds__(128)
+skinny_reduce_kernel(const uint32_t* __restrict__ part, int splits, int rows, int N4, const float* __restrict__ sx,
+                     const float* __restrict__ sw, const __nv_bfloat16* __restrict__ R, int ldr,
+                     __nv_bfloat16* __restrict__ C, int ldc) {
+  const bool wide = (reinterpret_cast<uintptr_t>(part) & 15) == 0;     // a caller's workspace may start anywhere
+  const int n4 = blockIdx.x * 128 + threadIdx.x, m = blockIdx.y;
+  if (n4 >= N4) return;
+  const size_t plane = static_cast<size_t>(rows) * N4, at = static_cast<size_t>(m) * N4 + n4;
+  float f[4] = {0.f, 0.f, 0.f, 0.f};
+  int acc[4] = {0, 0, 0, 0};
+  for (int s0 = 0; s0 < splits; s0 += 8) {
+    uint4 v[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x)
+      if (s0 + x < splits) {
+        const uint32_t* p = part + ((s0 + x) * plane + at) * 4;
+        v[x] = wide ? *reinterpret_cast<const uint4*>(p) : make_uint4(p[0], p[1], p[2], p[3]);
+      }
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      if (s0 + x < splits) {
+        const uint32_t w[4] = {v[x].x, v[x].y, v[x].z, v[x].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if constexpr (I8) acc[e] += static_cast<int>(w[e]);
+          else f[e] = s0 + x == 0 ? __uint_as_float(w[e]) : f[e] + __uint_as_float(w[e]);
+        }
+      }
+    }
   }
-  if (R) v += __bfloat162float(R[static_cast<size_t>(m) * ldr + n]);
-  C[static_cast<size_t>(m) * ldc + n] = __float2bfloat16_rn(v);
+  const int n = n4 * 4;
+  __nv_bfloat16* c = C + static_cast<size_t>(m) * ldc + n;
+  const __nv_bfloat16* r = R ? R + static_cast<size_t>(m) * ldr + n : nullptr;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if constexpr (I8) f[e] = __fmul_rn(static_cast<float>(acc[e]), __fmul_rn(sx[m], sw[n + e]));
+    if (r) f[e] += __bfloat162float(r[e]);
+    c[e] = __float2bfloat16_rn(f[e]);
+  }
 }
 
 template <int RB, bool I8>
@@ -298,14 +320,10 @@ extern "C" int sb_gemm_skinny(const void* X, int ldx, const void* W, int ldw, vo
 #undef SB_SKINNY
   if (rc) return rc;
   if (splits > 1) {
-    const size_t mn = static_cast<size_t>(rows) * N;
-    const unsigned blocks = static_cast<unsigned>((mn + 255) / 256);
-    if (is_i8) skinny_reduce_kernel<true><<<blocks, 256, 0, stream>>>(workspace, splits, rows, N, sx, sw,
-                                                                     static_cast<const __nv_bfloat16*>(R), ldr,
-                                                                     static_cast<__nv_bfloat16*>(C), ldc);
-    else skinny_reduce_kernel<false><<<blocks, 256, 0, stream>>>(workspace, splits, rows, N, nullptr, nullptr,
-                                                                 static_cast<const __nv_bfloat16*>(R), ldr,
-                                                                 static_cast<__nv_bfloat16*>(C), ldc);
+    const dim3 grid_r((N / 4 + 127) / 128, rows);          // N is a multiple of 8
+    auto kern = is_i8 ? skinny_reduce_kernel<true> : skinny_reduce_kernel<false>;
+    kern<<<grid_r, 128, 0, stream>>>(static_cast<const uint32_t*>(workspace), splits, rows, N / 4, sx, sw,
+                                     static_cast<const __nv_bfloat16*>(R), ldr, static_cast<__nv_bfloat16*>(C), ldc);
     if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   }
   return 0;

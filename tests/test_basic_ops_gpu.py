@@ -152,3 +152,24 @@ def test_sumsq_edges(dtype, n, offset):
     assert abs(out.item() - want) <= 1e-5 * want
     ops.sumsq(g, out=out, accumulate=True)
     assert abs(out.item() - 2 * want) <= 2e-5 * want
+
+
+@pytest.mark.parametrize("cols", [8, 1024, 2056, 8192, 9000])
+def test_rmsnorm_few_rows_are_the_bits_of_many(cols):
+    """A CTA per row up to 1184 rows, a warp per row beyond: the same association, so the same bits; rows longer than
+    what a thread keeps are read again."""
+    x, w = _r((1185, cols), 1).cuda(), _r((cols,), 2).cuda()
+    many, inv_many = ops.rmsnorm_fwd(x, w)
+    few, inv_few = ops.rmsnorm_fwd(x[:7], w)
+    assert torch.equal(few, many[:7]) and torch.equal(inv_few, inv_many[:7])
+
+
+@pytest.mark.parametrize("M,K", [(1, 8), (3, 4096), (2, 16384), (2, 16392), (5, 24)])
+def test_quantize_rows_edges(M, K):
+    """Rows that fit a CTA's registers and rows that do not, a zero row: the host statement bit for bit."""
+    from scirust_b200.ops import decode
+    x = _r((M, K), K).cuda()
+    x[0] = 0
+    q, s = decode.quantize_rows(x)
+    qc, sc = decode.quantize_rows(x.cpu())
+    assert torch.equal(s.cpu(), sc) and torch.equal(q.cpu(), qc)
