@@ -173,3 +173,24 @@ def test_quantize_rows_edges(M, K):
     q, s = decode.quantize_rows(x)
     qc, sc = decode.quantize_rows(x.cpu())
     assert torch.equal(s.cpu(), sc) and torch.equal(q.cpu(), qc)
+
+
+@pytest.mark.parametrize("cols", [8, 4096, 32760, 32768, 32776])
+def test_cross_entropy_row_kept_in_registers(cols):
+    """Both sides of the 32768-column line, ignored and clamped targets, the gradient over the logits or beside them: the
+    loss does not depend on where the gradient goes, and a repeated call gives the same bits."""
+    rows = 37
+    lg = _r((rows, cols), 11).cuda() * 3
+    lg[4] = float("-inf")
+    lg[4, 5] = 1.0
+    tg = torch.randint(0, cols, (rows,), generator=torch.Generator().manual_seed(1)).cuda()
+    tg[0], tg[1], tg[4] = -1, cols + 7, 5
+    loss, d = ops.ce_fwd_bwd(lg.clone(), tg, 0.25, in_place=False)
+    loss_only = ops.ce_loss_only(lg, tg)
+    inp = lg.clone()
+    loss2, d2 = ops.ce_fwd_bwd(inp, tg, 0.25)
+    assert d2.data_ptr() == inp.data_ptr()
+    assert torch.equal(loss, loss2) and torch.equal(d, d2) and torch.equal(loss, loss_only)
+    want_loss, want = ops.ce_fwd_bwd(lg.cpu(), tg.cpu(), 0.25, in_place=False)
+    assert (loss.cpu() - want_loss).abs().max().item() <= 2e-5 * max(1.0, want_loss.abs().max().item())
+    assert (d.cpu().float() - want.float()).abs().max().item() <= 0.25 * 2 ** -8
