@@ -45,6 +45,23 @@ struct GemmCfg {
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
 };
 
+// Convolution operands without a patch matrix. The patches of an NHWC tensor [B, H, W, C] are 4-D TMA boxes of 64 channels
+// x a row tile of output pixels, shifted by the filter tap; pixels outside the image arrive as zeros, a stride is the
+// map's element stride. Needs C % 64 == 0 and output rows that tile 128 (64 for the weight gradient) pixels. Bound by the
+// operand tiles that come out of L2 (each pixel nine times); the patch matrix would cross memory five times per
+// convolution. 128 x 32 x 32 x 64 -> 64, 3 x 3: gather + GEMM 133 -> 32 us forward, 61 -> 40 us weight gradient, GEMM +
+// scatter 129 -> 33 us input gradient, whose tap sums now stay in fp32.
+//   CONV_FPROP  A = patches of x [pixels, taps * C],  B = packed weights [oc, taps * C]
+//   CONV_WGRAD  A = dy [pixels, oc] (transposed),     B = patches of x
+//   CONV_DGRAD  A = patches of dy, taps mirrored (stride 1), B = packed weights read as [oc, C] per tap
+enum { CONV_NONE = 0, CONV_FPROP = 1, CONV_WGRAD = 2, CONV_DGRAD = 3 };
+struct ConvTile {
+  int cb;              // 64-channel blocks per tap of the tensor that is patched
+  int C;               // channels of x (DGRAD: columns of one tap in the packed weights)
+  int KW, stride, pad; // filter width (a square filter), stride and padding of the convolution
+  int ow, ohw;         // output pixels per row and per image of the pixel grid that is walked
+};
+
 struct GemmParams {
   int M, N, K;
   int splits;          // explicit split-K factor (1 = none)
@@ -56,9 +73,21 @@ struct GemmParams {
   int* status;
   BalancedSched sched;   // balanced schedule (splits == 1 only); see gemm_sched.cuh
   float* partials;       // scratch slots of the balanced schedule: dense fp32 [BM, BN] blocks
+  ConvTile conv;
 };
 
-template <int BN, bool A_MN, bool B_MN>
+// Patch box of output pixels [pix, pix + box) at k-block / column block `blk` (tap-major, 64 channels each).
+template <int CONV>
+__device__ __forceinline__ void conv_load_patch(void* dst, const CUtensorMap* m, uint64_t* bar, const ConvTile& cv,
+                                                int pix, int blk) {
+  const int tap = blk / cv.cb, c0 = (blk - tap * cv.cb) * 64;
+  const int kh = tap / cv.KW, kw = tap - kh * cv.KW;
+  const int b0 = pix / cv.ohw, oh0 = (pix - b0 * cv.ohw) / cv.ow;
+  if constexpr (CONV == CONV_DGRAD) tma_load_4d(dst, m, bar, c0, cv.pad - kw, oh0 + cv.pad - kh, b0);
+  else tma_load_4d(dst, m, bar, c0, kw - cv.pad, oh0 * cv.stride + kh - cv.pad, b0);
+}
+
+template <int BN, bool A_MN, bool B_MN, int CONV = CONV_NONE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const GemmParams p) {
@@ -123,14 +152,28 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           uint8_t* sa = tiles + stage * Cfg::STAGE_BYTES;
           uint8_t* sb_ = sa + Cfg::A_BYTES;
           mbar_arrive_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
-          if constexpr (!A_MN) {
+          if constexpr (CONV == CONV_FPROP || CONV == CONV_DGRAD) {
+            conv_load_patch<CONV>(sa, &tmap_a, &full_bar[stage], p.conv, m_idx * BM, kb);
+          } else if constexpr (!A_MN) {
             tma_load_2d(sa, &tmap_a, &full_bar[stage], kb * BK, m_idx * BM);
           } else {
 #pragma unroll
             for (int c = 0; c < BM / 64; ++c)
               tma_load_2d(sa + c * (64 * BK * 2), &tmap_a, &full_bar[stage], m_idx * BM + c * 64, kb * BK);
           }
-          if constexpr (!B_MN) {
+          if constexpr (CONV == CONV_WGRAD) {
+            const int last = p.N / 64 - 1;            // columns past N are dropped by the epilogue: any block will do
+#pragma unroll
+            for (int c = 0; c < BN / 64; ++c)
+              conv_load_patch<CONV>(sb_ + c * (64 * BK * 2), &tmap_b, &full_bar[stage], p.conv, kb * BK,
+                                    min(n_idx * (BN / 64) + c, last));
+          } else if constexpr (CONV == CONV_DGRAD) {
+            const int tap = kb / p.conv.cb;
+#pragma unroll
+            for (int c = 0; c < BN / 64; ++c)
+              tma_load_2d(sb_ + c * (64 * BK * 2), &tmap_b, &full_bar[stage], tap * p.conv.C + n_idx * BN + c * 64,
+                          (kb - tap * p.conv.cb) * 64);
+          } else if constexpr (!B_MN) {
             tma_load_2d(sb_, &tmap_b, &full_bar[stage], kb * BK, n_idx * BN);
           } else {
 #pragma unroll
@@ -369,6 +412,35 @@ int make_tmap_2d_u16_plain(CUtensorMap* out, const void* base, uint64_t inner, u
   return r == CUDA_SUCCESS ? 0 : SB_ERR_DRIVER;
 }
 
+// Patches of an NHWC tensor [B, H, W, C]: boxes of 64 channels x `box` output pixels (ow per row, whole rows, whole
+// images when an image is smaller than the box) at element stride `stride`. 0 when the shape does not tile.
+static int make_tmap_patches(CUtensorMap* out, const void* base, int B, int H, int W, int C, int ow, int oh, int stride,
+                             int box) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return SB_ERR_DRIVER;
+  if (reinterpret_cast<uintptr_t>(base) & 15) return SB_ERR_ALIGN;
+  if (ow > box || box % ow || (C & 63)) return SB_ERR_ARG;
+  int rows = box / ow, images = 1;
+  if (rows > oh) {
+    if (rows % oh) return SB_ERR_ARG;
+    images = rows / oh;
+    rows = oh;
+  } else if (oh % rows) {
+    return SB_ERR_ARG;
+  }
+  const cuuint64_t c = static_cast<cuuint64_t>(C);
+  cuuint64_t dims[4] = {c, static_cast<cuuint64_t>(W), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(B)};
+  cuuint64_t strides[3] = {c * 2, c * 2 * W, c * 2 * W * H};
+  cuuint32_t bx[4] = {64, static_cast<cuuint32_t>((ow - 1) * stride + 1), static_cast<cuuint32_t>((rows - 1) * stride + 1),
+                      static_cast<cuuint32_t>(images)};
+  cuuint32_t es[4] = {1, static_cast<cuuint32_t>(stride), static_cast<cuuint32_t>(stride), 1};
+  if (bx[1] > 256 || bx[2] > 256 || stride > 8) return SB_ERR_ARG;
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, bx, es,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : SB_ERR_DRIVER;
+}
+
 static int g_num_sms = 0;
 int num_sms() {
   if (!g_num_sms) {
@@ -379,11 +451,11 @@ int num_sms() {
   return g_num_sms;
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, int CONV = CONV_NONE>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
                        cudaStream_t stream) {
   using Cfg = GemmCfg<BN>;
-  auto kern = gemm_bf16_kernel<BN, A_MN, B_MN>;
+  auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, CONV>;
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess)
@@ -481,6 +553,78 @@ extern "C" int sb_gemm_bf16(const void* A, const void* B, void* C, const void* R
     splitk_reduce_kernel<<<blocks, threads, 0, stream>>>(static_cast<const float*>(workspace), splits, mn, N,
                                                          static_cast<__nv_bfloat16*>(C), ldc,
                                                          static_cast<const __nv_bfloat16*>(R), ldr);
+    if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
+  }
+  return 0;
+}
+
+// One product of an NHWC convolution (square k x k filter) without a patch matrix; the packed weights are [oc, k*k*C] in
+// (kh, kw, c) order, C % 64 == 0, oc % 64 == 0.
+//   mode 1: out = y [B*OH*OW, oc]   from a = x, b = weights
+//   mode 2: out = dw [oc, k*k*C]    from a = dy [B*OH*OW, oc], b = x
+//   mode 3: out = dx [B*H*W, C]     from a = dy, b = weights; stride 1
+// splits > 1: split-K over `workspace` (splits * rows * columns of out, floats). Shapes whose pixel rows do not tile 128
+// (mode 2: 64) pixels are refused with SB_ERR_ARG.
+extern "C" int sb_conv_gemm(int mode, const void* a, const void* b, void* out, int B, int H, int W, int C, int oc, int k,
+                            int stride, int pad, int OH, int OW, int splits, void* workspace, int* status,
+                            void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (mode < 1 || mode > 3 || B <= 0 || C <= 0 || oc <= 0 || (C & 63) || (oc & 63) || k < 1 || stride < 1 || pad < 0 || !status)
+    return SB_ERR_ARG;
+  if (OH != (H + 2 * pad - k) / stride + 1 || OW != (W + 2 * pad - k) / stride + 1 || OH < 1 || OW < 1) return SB_ERR_ARG;
+  if (mode == 3 && stride != 1) return SB_ERR_ARG;
+  if (reinterpret_cast<uintptr_t>(out) & 15) return SB_ERR_ALIGN;
+  const int taps = k * k, kp = taps * C;
+  const long long pix_o = static_cast<long long>(B) * OH * OW, pix_i = static_cast<long long>(B) * H * W;
+  if (pix_o >= (1ll << 31) || pix_i >= (1ll << 31)) return SB_ERR_TOO_LARGE;
+  GemmParams p;
+  p.M = mode == 2 ? oc : static_cast<int>(mode == 1 ? pix_o : pix_i);
+  p.N = mode == 1 ? oc : mode == 2 ? kp : C;
+  p.K = mode == 1 ? kp : mode == 2 ? static_cast<int>(pix_o) : taps * oc;
+  const int num_kb = (p.K + BK - 1) / BK;
+  if (splits < 1) splits = 1;
+  if (splits > num_kb) splits = num_kb;
+  p.kb_per_split = (num_kb + splits - 1) / splits;
+  splits = (num_kb + p.kb_per_split - 1) / p.kb_per_split;
+  if (splits > 1 && !workspace) return SB_ERR_ARG;
+  const int bn = p.N <= 128 ? 128 : 256;
+  p.splits = splits;
+  p.C = splits > 1 ? workspace : out;
+  p.ldc = p.N;
+  p.R = nullptr; p.ldr = 0;
+  p.status = status;
+  p.partials = nullptr;
+  p.sched.dp_tiles = p.sched.sk_tiles = p.sched.sk_workers = p.sched.sk_slots = 0;
+  p.conv.C = C; p.conv.KW = k; p.conv.stride = stride; p.conv.pad = pad;
+  p.conv.cb = (mode == 3 ? oc : C) / 64;
+  p.conv.ow = mode == 3 ? W : OW;
+  p.conv.ohw = mode == 3 ? H * W : OH * OW;
+  CUtensorMap ta, tb;
+  int rc;
+  if (mode == 1) {
+    rc = make_tmap_patches(&ta, a, B, H, W, C, OW, OH, stride, BM);
+    if (!rc) rc = make_tmap_2d_bf16(&tb, b, kp, oc, kp, BK, bn);
+  } else if (mode == 2) {
+    rc = make_tmap_2d_bf16(&ta, a, oc, pix_o, oc, 64, BK);
+    if (!rc) rc = make_tmap_patches(&tb, b, B, H, W, C, OW, OH, stride, BK);
+  } else {
+    rc = make_tmap_patches(&ta, a, B, OH, OW, oc, W, H, 1, BM);
+    if (!rc) rc = make_tmap_2d_bf16(&tb, b, kp, oc, kp, 64, BK);
+  }
+  if (rc) return rc;
+  const long long tiles = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + bn - 1) / bn) * splits;
+  const int grid = tiles < num_sms() ? static_cast<int>(tiles) : num_sms();
+  if (mode == 1) rc = bn == 128 ? launch_gemm<128, false, false, CONV_FPROP>(ta, tb, p, grid, stream)
+                                : launch_gemm<256, false, false, CONV_FPROP>(ta, tb, p, grid, stream);
+  else if (mode == 2) rc = bn == 128 ? launch_gemm<128, true, true, CONV_WGRAD>(ta, tb, p, grid, stream)
+                                     : launch_gemm<256, true, true, CONV_WGRAD>(ta, tb, p, grid, stream);
+  else rc = bn == 128 ? launch_gemm<128, false, true, CONV_DGRAD>(ta, tb, p, grid, stream)
+                      : launch_gemm<256, false, true, CONV_DGRAD>(ta, tb, p, grid, stream);
+  if (rc) return rc;
+  if (splits > 1) {
+    const size_t mn = static_cast<size_t>(p.M) * p.N;
+    splitk_reduce_kernel<<<static_cast<unsigned>((mn / 4 + 255) / 256), 256, 0, stream>>>(
+        static_cast<const float*>(workspace), splits, mn, p.N, static_cast<__nv_bfloat16*>(out), p.N, nullptr, 0);
     if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   }
   return 0;

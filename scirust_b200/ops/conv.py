@@ -1,6 +1,6 @@
-"""Convolutional ops on NHWC bf16 activations (csrc/conv.cu + the tcgen05 GEMM): explicit-GEMM
-convolution (im2col -> GEMM, col2im for the input gradient, transposed GEMM for the weight
-gradient), max pooling, BatchNorm2d with optional fused ReLU. Activations are ``[B*H*W, C]``
+"""Convolutional ops on NHWC bf16 activations (csrc/conv.cu + the tcgen05 GEMM): convolution as implicit
+GEMMs whose patch operand is fetched by TMA (forward, weight gradient, stride-1 input gradient), or with an explicit
+patch matrix where the shape does not tile (im2col -> GEMM, col2im for the input gradient), max pooling, BatchNorm2d with optional fused ReLU. Activations are ``[B*H*W, C]``
 matrices; ``ConvGeom`` carries the spatial shape. CPU tensors run the fp32 PyTorch statement
 (``torch.nn.functional``), which is also the oracle of the GPU tests."""
 from __future__ import annotations
@@ -65,11 +65,51 @@ def unpack_conv_weight(wp: torch.Tensor, in_c: int, k: int) -> torch.Tensor:
     return wp[:, : k * k * in_c].reshape(oc, k, k, in_c).permute(0, 3, 1, 2).reshape(oc, in_c * k * k)
 
 
+_lib.register("sb_conv_gemm", [i32, vp, vp, vp] + [i32] * 11 + [vp, vp, vp])
+_FPROP, _WGRAD, _DGRAD = 1, 2, 3
+
+
+def _rows_tile(oh: int, ow: int, box: int) -> bool:
+    """Whether ``box`` consecutive pixels of an oh x ow grid are whole rows of one image or whole images."""
+    if ow > box or box % ow:
+        return False
+    rows = box // ow
+    return oh % rows == 0 if rows <= oh else rows % oh == 0
+
+
+def implicit_ok(geom: ConvGeom, oc: int, k: int, stride: int, pad: int) -> bool:
+    """Whether a convolution runs without a patch matrix (csrc/gemm_tcgen05.cu: ``sb_conv_gemm``): channels in whole
+    64-wide blocks and output rows that tile the 128-pixel operand (and the weight gradient's 64-pixel one). Others
+    (an RGB stem, odd image sizes) gather their patches first."""
+    oh, ow = (geom.H + 2 * pad - k) // stride + 1, (geom.W + 2 * pad - k) // stride + 1
+    return (geom.C % 64 == 0 and oc % 64 == 0 and stride <= 8 and _rows_tile(oh, ow, 128) and _rows_tile(oh, ow, 64)
+            and (ow - 1) * stride < 256 and (128 // ow - 1) * stride < 256)
+
+
+def _conv_gemm(mode, a, b, geom, oc, k, stride, pad, OH, OW):
+    pix_o, pix_i, kp = geom.B * OH * OW, geom.rows, k * k * geom.C
+    M, N, K = {_FPROP: (pix_o, oc, kp), _WGRAD: (oc, kp, pix_o), _DGRAD: (pix_i, geom.C, k * k * oc)}[mode]
+    out = _lib.empty((M, N), BF, a.device)
+    # one wave of work items, at least eight 64-deep k-blocks each (a weight gradient has K = pixels and few tiles)
+    tiles = ((M + 127) // 128) * ((N + 255) // 256)
+    splits = max(1, min(G.num_sms(a.device) // tiles, (K + 63) // 64 // 8, 64))
+    ws = G._workspace(splits * M * N, a.device) if splits > 1 else None
+    _lib.call("sb_conv_gemm", mode, a.data_ptr(), b.data_ptr(), out.data_ptr(), geom.B, geom.H, geom.W, geom.C, oc, k,
+              stride, pad, OH, OW, splits, _lib.ptr(ws), _lib.status_word(a.device).data_ptr(), _lib.stream())
+    G.launch_count += 2 if splits > 1 else 1
+    return out
+
+
 class _Conv(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, wp, geom, k, stride, pad):
         B, H, W, C = geom.B, geom.H, geom.W, geom.C
         OH, OW = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
+        ctx.meta = (geom, k, stride, pad, OH, OW)
+        ctx.implicit = implicit_ok(geom, wp.shape[0], k, stride, pad) and _tma_ok(x, wp, geom, k)
+        if ctx.implicit:
+            ctx.save_for_backward(x, wp)
+            return _conv_gemm(_FPROP, x, wp, geom, wp.shape[0], k, stride, pad, OH, OW)
         Kp = wp.shape[1]
         col = _lib.empty((B * OH * OW, Kp), BF, x.device)
         _lib.call("sb_im2col_nhwc", x.data_ptr(), col.data_ptr(), B, H, W, C, k, k, stride, pad, OH, OW, Kp,
@@ -77,24 +117,36 @@ class _Conv(torch.autograd.Function):
         G.launch_count += 1
         y = G.matmul_nt(col, wp)
         ctx.save_for_backward(col, wp)
-        ctx.meta = (geom, k, stride, pad, OH, OW)
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        col, wp = ctx.saved_tensors
+        col, wp = ctx.saved_tensors                           # col: the input itself when no patch matrix was made
         geom, k, stride, pad, OH, OW = ctx.meta
+        oc = wp.shape[0]
         dy = dy.contiguous()
+        implicit = ctx.implicit and dy.dtype == BF and dy.data_ptr() % 16 == 0
+        if ctx.implicit and not implicit:
+            raise ValueError("conv2d: the output gradient must be bf16 and 16-byte aligned")
         dx = dw = None
         if ctx.needs_input_grad[1]:
-            dw = G.matmul_tn(dy, col)                         # [oc, Kp] = dy^T col
+            dw = (_conv_gemm(_WGRAD, dy, col, geom, oc, k, stride, pad, OH, OW) if implicit
+                  else G.matmul_tn(dy, col))                  # [oc, Kp] = dy^T col
         if ctx.needs_input_grad[0]:
+            if implicit and stride == 1 and _rows_tile(geom.H, geom.W, 128):
+                return _conv_gemm(_DGRAD, dy, wp, geom, oc, k, stride, pad, OH, OW), dw, None, None, None, None
             dcol = G.matmul_nn(dy, wp)                        # [M, Kp]
             dx = _lib.empty((geom.rows, geom.C), BF, dy.device)
             _lib.call("sb_col2im_nhwc", dcol.data_ptr(), dx.data_ptr(), geom.B, geom.H, geom.W, geom.C, k, k, stride,
                       pad, OH, OW, wp.shape[1], _lib.stream())
             G.launch_count += 1
         return dx, dw, None, None, None, None
+
+
+def _tma_ok(x, wp, geom, k) -> bool:
+    """Types, shapes and 16-byte bases of the operands as the tensor maps need them; others take the patch matrix."""
+    return (x.dtype == BF and wp.dtype == BF and wp.is_contiguous() and x.data_ptr() % 16 == 0
+            and wp.data_ptr() % 16 == 0 and wp.shape[1] == k * k * geom.C and x.numel() == geom.rows * geom.C)
 
 
 def conv2d(x, wp, geom: ConvGeom, k: int, stride: int = 1, pad: int = 0):

@@ -123,3 +123,34 @@ def test_batchnorm_row_and_column_edges(rows, C_, relu):
     _close(gi.grad, gr.grad, 1e-2)
     _close(bi.grad, br.grad, 1e-2)
     _close(rm, 0.1 * mean, 1e-4)
+
+
+@pytest.mark.parametrize("B,Cin,H,W,Cout,k,stride,pad", [
+    (3, 64, 16, 16, 64, 3, 1, 1),       # whole rows of one image per 128-pixel tile, both gradients implicit
+    (5, 128, 4, 4, 64, 3, 1, 1),        # eight images per tile, a batch that ends inside one
+    (1, 64, 64, 32, 192, 1, 1, 0),      # 1 x 1, three column blocks
+    (1, 64, 8, 8, 128, 5, 1, 2),        # a halo wider than one pixel
+    (2, 128, 32, 16, 64, 3, 2, 1),      # strided: forward and weight gradient implicit, input gradient through col2im
+])
+def test_conv_without_patch_matrix_matches_patch_matrix(B, Cin, H, W, Cout, k, stride, pad, monkeypatch):
+    """The implicit products against the explicit ones on the same inputs: the same bf16 operands and fp32 sums in
+    another order, so they agree to a rounding of the result (2^-8) plus the fp32 sums (K * 2^-24 of the terms' norm);
+    the explicit input gradient also rounds each of the k * k tap sums to bf16."""
+    geom = C.ConvGeom(B, H, W, Cin)
+    assert C.implicit_ok(geom, Cout, k, stride, pad)
+    g = torch.Generator(device="cuda").manual_seed(Cin + k)
+    x = torch.randn(geom.rows, Cin, generator=g, device="cuda").to(BF)
+    w = (torch.randn(Cout, k * k * Cin, generator=g, device="cuda") * 0.1).to(BF)
+    got = []
+    for implicit in (True, False):
+        if not implicit:
+            monkeypatch.setattr(C, "implicit_ok", lambda *a: False)
+        xi, wi = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+        y, og = C.conv2d(xi, wi, geom, k, stride, pad)
+        dy = torch.randn(y.shape, generator=torch.Generator(device="cuda").manual_seed(5), device="cuda").to(BF)
+        y.backward(dy)
+        got.append((y.detach(), xi.grad, wi.grad))
+    _lib.check_status()
+    for a, b, taps in zip(got[0], got[1], (1, k * k, 1)):
+        lim = b.float().abs().max().item() * 2 ** -8 * (1 + taps ** 0.5)
+        assert (a.float() - b.float()).abs().max().item() <= lim
