@@ -162,7 +162,9 @@ def check_canaries() -> None:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device, without building a ``torch.cuda.Stream`` object (an op asks
+    for it two or three times: the launch and the keys of its workspaces)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def check(rc: int, what: str) -> None:
@@ -180,6 +182,9 @@ _status_words: dict[int, torch.Tensor] = {}
 
 def status_word(device=None) -> torch.Tensor:
     """Per-device int32 word that kernels with bounded waits write an error code into."""
+    w = _status_words.get(getattr(device, "index", None))
+    if w is not None:
+        return w
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     w = _status_words.get(key)

@@ -183,17 +183,17 @@ def gemv(x, w, residual=None, out=None, out_f32=None, splits=None, rms_weight=No
     splits = max(splits, (K + 4095) // 4096)
     ws = _gemv_workspace(4096 + splits * min(M, grp) * N, x.device)
     st = _lib.status_word(x.device)
+    # row groups are addressed by offsets: a decode step is one group, and slicing its tensors costs more than the launch
+    xp, xs = x.data_ptr(), x.stride(0)
+    rp, rs = (residual.data_ptr(), residual.stride(0)) if residual is not None else (None, 0)
+    op, os_ = (out.data_ptr(), out.stride(0)) if out is not None else (None, 0)
+    fp, fs = (out_f32.data_ptr(), out_f32.stride(0)) if out_f32 is not None else (None, 0)
+    pro = 1 if rms_weight is not None else (2 if swiglu else 0)
     for m0 in range(0, M, grp):
-        mb = min(grp, M - m0)
-        xs = x[m0:m0 + mb]
-        _lib.call("sb_gemv", xs.data_ptr(), xs.stride(0), wm.data_ptr(), wm.stride(0),
-                  w.scale.data_ptr() if quant else None,
-                  residual[m0:m0 + mb].data_ptr() if residual is not None else None,
-                  residual.stride(0) if residual is not None else 0,
-                  out[m0:m0 + mb].data_ptr() if out is not None else None, out.stride(0) if out is not None else 0,
-                  out_f32[m0:m0 + mb].data_ptr() if out_f32 is not None else None, mb, N, K, int(quant), splits,
-                  ws.data_ptr(), 1 if rms_weight is not None else (2 if swiglu else 0), _lib.ptr(rms_weight),
-                  float(eps), st.data_ptr(), _lib.stream())
+        _lib.call("sb_gemv", xp + m0 * xs * 2, xs, wm.data_ptr(), wm.stride(0), w.scale.data_ptr() if quant else None,
+                  rp + m0 * rs * 2 if rp else None, rs, op + m0 * os_ * 2 if op else None, os_,
+                  fp + m0 * fs * 4 if fp else None, min(grp, M - m0), N, K, int(quant), splits, ws.data_ptr(), pro,
+                  _lib.ptr(rms_weight), float(eps), st.data_ptr(), _lib.stream())
         _g.launch_count += 1
     return out if out is not None else out_f32
 
