@@ -71,6 +71,7 @@ int sb_gemv_argmax(const void* X, int ldx, const void* W, int ldw, const float* 
 int sb_kv_append(const void* qkv, int ld, int H, int Hkv, int dh, void* pool, const int* block_table, int max_blocks, int page, const int* seq_of, const int* pos, int n_tok, void* stream);
 int sb_rope_kv_append(void* qkv, int ld, int H, int Hkv, int dh, const float* cos_t, const float* sin_t, void* pool, const int* block_table, int max_blocks, int page, const int* seq_of, const int* pos, int n_tok, void* stream);
 int sb_decode_attention(const void* q, int ldq, const void* pool, const int* block_table, int max_blocks, int page, const int* seq_len, int B, int H, int Hkv, int dh, int n_splits, float scale, float* part_o, float* part_ml, unsigned int* counters, void* out, int ldo, void* stream);
+int sb_decode_attention_stream(const void* q, int ldq, const void* pool, int n_blocks, const int* block_table, int max_blocks, int page, const int* seq_len, int B, int H, int Hkv, int dh, int max_tiles, float scale, float* part, unsigned int* counters, void* out, int ldo, int* status, void* stream);
 int sb_argmax(const float* logits, int rows, int V, float* pval, int* pidx, int64_t* out_tokens, int64_t* generated, int gen_stride, int step, void* stream);
 int sb_quantize_per_channel(const void* W, int K, int N, int ldw, float* scale, void* Q, void* stream);
 int sb_dequantize(const void* Q, const float* scale, int K, int N, void* W, void* stream);

@@ -1449,6 +1449,397 @@ decode_attn_kernel(const __grid_constant__ DecodeAttnParams p) {
 }
 
 // ---------------------------------------------------------------------------
+// The same attention with the whole grid as one stream of KV tiles (pages of 8, 16, 32 or a multiple of 64 positions).
+//
+// Bound by the KV bytes. The kernel above starts (kv head, sequence, split) CTAs of two 64-position stages: 96 KB in
+// flight per SM, a split count that depends on the batch only, and a last wave that is mostly empty (16 sequences: 640
+// CTAs over 444 places). Here one CTA per SM holds four to six 32 KB stages that a
+// producer warp fills with 128-byte-swizzled TMA boxes, and the 64-position tiles of all (sequence, kv head) jobs, laid
+// end to end, are dealt out in equal contiguous ranges, so lengths may be as ragged as they like. A job that ends up in
+// several CTAs is merged by the last of them to finish, pieces in tile order (a counter, no data atomics): the
+// summation tree depends on the lengths and the grid only.
+// Two groups of four consumer warps take the tiles of a piece in turn (one group alone needs 1650 cycles for a tile that
+// memory delivers in 1400); warp w of a group owns positions [16w, 16w + 16), as above.
+// Head dimension 128 only: at 64 the tiles are half the bytes for the same consumer work, and the kernel above is as fast
+// or faster up to 64 x 2048 positions (36.9 us against 37.1). Where the line lies at 128, with figures: ops/decode.py,
+// _stream_wins. 64 sequences of 1536-2048 positions, 8 kv heads: 108.5 us above (4.3 TB/s), 87.5 us here (5.4 TB/s).
+// ---------------------------------------------------------------------------
+constexpr int DST_THREADS = 288;         // warps 0-7 consume (two groups of four, every other tile each), warp 8 produces
+constexpr int DST_STAGES_MAX = 10;
+constexpr int DST_MAX_B = 1024;          // sequences whose tile offsets fit the shared prefix table
+
+struct DecodeStreamParams {
+  const __nv_bfloat16* q; int ldq;
+  const int* block_table; int max_blocks, page;
+  const int* seq_len;
+  int B, H, Hkv;
+  float scale_log2;
+  float* part;             // [2 * grid][16][DH + 2]: partial O, then (max, sum) per row
+  __nv_bfloat16* out; int ldo;
+  unsigned int* counters;  // [B * Hkv], zero between calls
+  int* status;
+  int stages;
+};
+
+template <int DH>
+struct DstCfg {
+  static constexpr int NCH = DH / 64;
+  static constexpr int TILE_BYTES = DEC_TK * DH * 2;         // K or V of one tile
+  // eight warps' partial results of the G live rows; what is left of shared memory holds stages
+  static constexpr int merge_floats(int G) { return 8 * G * (DH + 2); }
+  static constexpr int fixed_bytes(int G) { return merge_floats(G) * 4 + (DST_MAX_B + 1) * 4 + 2 * DST_STAGES_MAX * 8 + 1024 + 64; }
+  static constexpr int stages(int G) {
+    const int n = (226 * 1024 - fixed_bytes(G)) / (2 * TILE_BYTES);
+    return n < DST_STAGES_MAX ? n : DST_STAGES_MAX;
+  }
+  static constexpr int smem_bytes(int G) { return stages(G) * 2 * TILE_BYTES + fixed_bytes(G); }
+  static_assert(stages(16) >= 4, "a ring of at least four stages");
+};
+
+// Tiles of one sequence: an empty one keeps a tile without positions, whose job writes zeros.
+__device__ __forceinline__ int dst_tiles(int len) { return len > 0 ? (len + DEC_TK - 1) / DEC_TK : 1; }
+
+template <int DH>
+__global__ void __launch_bounds__(DST_THREADS, 1)
+decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ DecodeStreamParams p) {
+  using C = DstCfg<DH>;
+  constexpr int KS = DH / 16;                  // k-steps of Q K^T
+  constexpr int NB = DH / 8;                   // 8-wide output blocks of P V
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int H = p.H, Hkv = p.Hkv, G = H / Hkv, stages = p.stages;
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + stages * 2 * C::TILE_BYTES);
+  uint64_t* empty = full + DST_STAGES_MAX;
+  float* sm_o = reinterpret_cast<float*>(empty + DST_STAGES_MAX);                   // [8 warps][G rows][DH]
+  float* sm_ml = sm_o + 8 * G * DH;                                                 // [8 warps][G rows][2]
+  int* prefix = reinterpret_cast<int*>(sm_ml + 8 * G * 2);                          // [B + 1] tiles before sequence b
+  __shared__ int s_last;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    prefetch_tmap(&tmap);
+    for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+    fence_barrier_init();
+  }
+  pdl_wait();
+  if (warp == 0) {
+    int base = 0;
+    for (int b0 = 0; b0 < p.B; b0 += 32) {
+      const int n = b0 + lane < p.B ? dst_tiles(p.seq_len[b0 + lane]) : 0;
+      int inc = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (b0 + lane < p.B) prefix[b0 + lane] = base + inc - n;
+      base += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) prefix[p.B] = base;
+  }
+  __syncthreads();
+  // unit u = tile u - S of job (b, kvh), jobs in (b, kvh) order; this CTA takes units [u0, u1)
+  const long long T = static_cast<long long>(prefix[p.B]) * Hkv;
+  const long long grid = min(static_cast<long long>(gridDim.x), T);     // every CTA of the deal has a unit
+  if (blockIdx.x >= grid) return;
+  const long long u0 = blockIdx.x * T / grid, u1 = (blockIdx.x + 1) * T / grid;
+  int b_first = 0;
+  {
+    int lo = 0, hi = p.B - 1;                  // last sequence whose first unit is <= u0
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (static_cast<long long>(prefix[mid]) * Hkv <= u0) lo = mid; else hi = mid - 1;
+    }
+    b_first = lo;
+  }
+
+  if (warp == 8) {
+    // ------------------------------ producer ------------------------------
+    const int box = min(p.page, DEC_TK), nbx = DEC_TK / box;    // positions per TMA box, boxes per tile
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int b = b_first;
+    for (long long u = u0; u < u1 && ok; ++b) {
+      const int len = p.seq_len[b], nt = dst_tiles(len);
+      const long long s_b = static_cast<long long>(prefix[b]) * Hkv;
+      const long long e_b = min(u1, s_b + static_cast<long long>(nt) * Hkv);
+      const int* table = p.block_table + static_cast<size_t>(b) * p.max_blocks;
+      for (; u < e_b && ok;) {
+        const int kvh = static_cast<int>((u - s_b) / nt);
+        const int t_beg = static_cast<int>((u - s_b) - static_cast<long long>(kvh) * nt);
+        const int t_end = static_cast<int>(min(static_cast<long long>(nt), t_beg + (e_b - u)));
+        int blk_of_lane = 0;                   // block of box (fetched + lane) of this job
+        int fetched = -1000000;
+        for (int t = t_beg; t < t_end && ok; ++t) {
+          if (!mbar_wait(&empty[stage], phase ^ 1, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
+          const int bx0 = t * nbx;
+          if (bx0 + nbx > fetched + 32) {      // nbx divides 32: a tile's boxes are fetched together
+            fetched = bx0;
+            const int pos = (fetched + lane) * box;
+            blk_of_lane = pos < len ? table[pos / p.page] : 0;
+          }
+          const int live = max(0, min(nbx, (len - t * DEC_TK + box - 1) / box));   // boxes with a position < len
+          uint8_t* kt = ring + stage * 2 * C::TILE_BYTES;
+          if (lane == 0) mbar_arrive_expect_tx(&full[stage], live * box * DH * 2 * 2);
+          for (int x = 0; x < live; ++x) {
+            const int blk = __shfl_sync(0xffffffffu, blk_of_lane, bx0 + x - fetched);
+            if (lane == 0) {
+              const int row = (blk * 2 * Hkv + kvh) * p.page + (bx0 + x) * box % p.page;
+              const int vrow = row + Hkv * p.page;
+#pragma unroll
+              for (int c = 0; c < C::NCH; ++c) {
+                tma_load_2d(kt + c * (DEC_TK * 128) + x * box * 128, &tmap, &full[stage], c * 64, row);
+                tma_load_2d(kt + C::TILE_BYTES + c * (DEC_TK * 128) + x * box * 128, &tmap, &full[stage], c * 64, vrow);
+              }
+            }
+          }
+          __syncwarp();
+          if (++stage == stages) { stage = 0; phase ^= 1; }
+        }
+        u += t_end - t_beg;
+      }
+    }
+    return;
+  }
+
+  // ------------------------------ consumers -----------------------------
+  const int quad = lane >> 2, tq = lane & 3, mi = lane >> 3;
+  const int group = warp >> 2, pw = warp & 3;      // group 0 takes the even tiles of a piece, group 1 the odd ones
+  int stage = 0;
+  uint32_t phase = 0;
+  bool ok = true;
+  int b = b_first;
+  for (long long u = u0; u < u1;) {
+    const int len = p.seq_len[b], nt = dst_tiles(len);
+    const long long s_b = static_cast<long long>(prefix[b]) * Hkv;
+    if (u >= s_b + static_cast<long long>(nt) * Hkv) { ++b; continue; }
+    const int kvh = static_cast<int>((u - s_b) / nt);
+    const long long s_job = s_b + static_cast<long long>(kvh) * nt;
+    const int t_beg = static_cast<int>(u - s_job);
+    const int t_end = static_cast<int>(min(static_cast<long long>(nt), t_beg + (u1 - u)));
+
+    // Q as A fragments: row `quad` (and quad + 8) of the 16-row operand is query head kvh * G + row
+    uint32_t qa[KS][4];
+    {
+      const __nv_bfloat16* q_lo = p.q + static_cast<size_t>(b) * p.ldq + static_cast<size_t>(kvh * G + quad) * DH;
+      const __nv_bfloat16* q_hi = q_lo + 8 * DH;
+      const bool lo = quad < G, hi = quad + 8 < G;
+#pragma unroll
+      for (int ks = 0; ks < KS; ++ks) {
+        const int c = ks * 16 + tq * 2;
+        qa[ks][0] = lo ? *reinterpret_cast<const uint32_t*>(q_lo + c) : 0u;
+        qa[ks][1] = hi ? *reinterpret_cast<const uint32_t*>(q_hi + c) : 0u;
+        qa[ks][2] = lo ? *reinterpret_cast<const uint32_t*>(q_lo + c + 8) : 0u;
+        qa[ks][3] = hi ? *reinterpret_cast<const uint32_t*>(q_hi + c + 8) : 0u;
+      }
+    }
+    float m_lo = -1.0e30f, m_hi = -1.0e30f, l_lo = 0.f, l_hi = 0.f;
+    float o[NB][4];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
+
+    for (int t = t_beg; t < t_end; ++t) {
+      const int st = stage;
+      const uint32_t ph = phase;
+      if (++stage == stages) { stage = 0; phase ^= 1; }
+      // the other group's tiles are waited for too: a parity wait tells a stage's fill from its next one only as long as
+      // nobody is a whole fill ahead
+      if (ok && !mbar_wait(&full[st], ph, p.status, ST_TIMEOUT_FULL)) ok = false;
+      if (!ok || ((t - t_beg) & 1) != group) continue;
+      uint8_t* kp = ring + st * 2 * C::TILE_BYTES;
+      uint8_t* vp = kp + C::TILE_BYTES;
+      const uint32_t kt = smem_u32(kp), vt = smem_u32(vp);
+      const int valid = len - t * DEC_TK - pw * 16;        // positions of this warp's 16 that exist
+      if (valid < 16) {
+        // value rows past the end hold whatever the page holds (or an older tile): 0 * x must not meet NaN
+        for (int i = lane; i < 16 * C::NCH * 8; i += 32) {
+          const int r = i / (C::NCH * 8), x = i - r * (C::NCH * 8);
+          if (r >= valid)
+            *reinterpret_cast<uint4*>(vp + (x >> 3) * (DEC_TK * 128) + (pw * 16 + r) * 128 + (x & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_proxy_async_smem();              // the stage is refilled by TMA later
+        __syncwarp();
+      }
+      // ---- S = Q K^T for this warp's 16 positions (two 16x8 blocks) ----
+      float sacc[2][4];
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) { sacc[nb][0] = sacc[nb][1] = sacc[nb][2] = sacc[nb][3] = 0.f; }
+      {
+        const int r = pw * 16 + (mi >> 1) * 8 + (lane & 7);
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks) {
+          const int unit = ks * 2 + (mi & 1);
+          uint32_t r0, r1, r2, r3;
+          ldsm_x4(kt + (unit >> 3) * (DEC_TK * 128) + r * 128 + (((unit & 7) ^ (r & 7)) << 4), r0, r1, r2, r3);
+          mma_16816(sacc[0], qa[ks], r0, r1);
+          mma_16816(sacc[1], qa[ks], r2, r3);
+        }
+      }
+      // ---- online softmax on the fragments ----
+      float mx_lo = -1.0e30f, mx_hi = -1.0e30f;
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+        const int pos = nb * 8 + tq * 2;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const bool in = pos + e < valid;
+          sacc[nb][e] = in ? sacc[nb][e] * p.scale_log2 : -1.0e30f;
+          sacc[nb][2 + e] = in ? sacc[nb][2 + e] * p.scale_log2 : -1.0e30f;
+          mx_lo = fmaxf(mx_lo, sacc[nb][e]);
+          mx_hi = fmaxf(mx_hi, sacc[nb][2 + e]);
+        }
+      }
+      mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
+      mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
+      mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
+      mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
+      const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
+      const float al_lo = exp2f(m_lo - mn_lo), al_hi = exp2f(m_hi - mn_hi);
+      m_lo = mn_lo; m_hi = mn_hi;
+      uint32_t pa[4];
+      {
+        float pr[2][4];
+        float sum_lo = 0.f, sum_hi = 0.f;
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            // a masked score stays at -1e30: exp2 of (-1e30 - m) is 0 unless the row is empty so far,
+            // in which case m is -1e30 too and the position must still contribute nothing
+            pr[nb][e] = sacc[nb][e] > -1.0e29f ? exp2f(sacc[nb][e] - mn_lo) : 0.f;
+            pr[nb][2 + e] = sacc[nb][2 + e] > -1.0e29f ? exp2f(sacc[nb][2 + e] - mn_hi) : 0.f;
+            sum_lo += pr[nb][e];
+            sum_hi += pr[nb][2 + e];
+          }
+        }
+        l_lo = l_lo * al_lo + sum_lo;
+        l_hi = l_hi * al_hi + sum_hi;
+        pa[0] = dpack(pr[0][0], pr[0][1]);
+        pa[1] = dpack(pr[0][2], pr[0][3]);
+        pa[2] = dpack(pr[1][0], pr[1][1]);
+        pa[3] = dpack(pr[1][2], pr[1][3]);
+      }
+#pragma unroll
+      for (int j = 0; j < NB; ++j) { o[j][0] *= al_lo; o[j][1] *= al_lo; o[j][2] *= al_hi; o[j][3] *= al_hi; }
+      // ---- O += P V over this warp's 16 positions ----
+      {
+        const int r = pw * 16 + (mi & 1) * 8 + (lane & 7);
+#pragma unroll
+        for (int j = 0; j < NB; j += 2) {
+          const int unit = j + (mi >> 1);
+          uint32_t r0, r1, r2, r3;
+          ldsm_x4_t(vt + (unit >> 3) * (DEC_TK * 128) + r * 128 + (((unit & 7) ^ (r & 7)) << 4), r0, r1, r2, r3);
+          mma_16816(o[j], pa, r0, r1);
+          mma_16816(o[j + 1], pa, r2, r3);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[st]);
+    }
+
+    // ---- merge the eight warps in warp order ----
+    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
+    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
+    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
+    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      float* r_lo = sm_o + (warp * G + quad) * DH + j * 8 + tq * 2;
+      if (quad < G) *reinterpret_cast<float2*>(r_lo) = make_float2(o[j][0], o[j][1]);
+      if (quad + 8 < G) *reinterpret_cast<float2*>(r_lo + 8 * DH) = make_float2(o[j][2], o[j][3]);
+    }
+    if (tq == 0) {
+      if (quad < G) { sm_ml[(warp * G + quad) * 2] = m_lo; sm_ml[(warp * G + quad) * 2 + 1] = l_lo; }
+      if (quad + 8 < G) { sm_ml[(warp * G + quad + 8) * 2] = m_hi; sm_ml[(warp * G + quad + 8) * 2 + 1] = l_hi; }
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    const bool direct = t_beg == 0 && t_end == nt;
+    const int job = b * Hkv + kvh;
+    // CTAs that share this job: c is the owner of unit v when c * T / grid <= v < (c + 1) * T / grid
+    const int c_first = static_cast<int>(((s_job + 1) * grid - 1) / T);
+    const int c_last = static_cast<int>(((s_job + nt) * grid - 1) / T);
+    constexpr int SLOT = 16 * (DH + 2);
+    // a CTA's first piece goes to slot 2c, a later one (a job that starts inside its range) to 2c + 1
+    float* slot = p.part + static_cast<size_t>(2 * blockIdx.x + (u == u0 ? 0 : 1)) * SLOT;
+    for (int i = threadIdx.x; i < G * DH; i += 256) {
+      const int g = i / DH, d = i - g * DH;
+      float mt = -1.0e30f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) mt = fmaxf(mt, sm_ml[(w * G + g) * 2]);
+      float lt = 0.f, ot = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        const float wgt = exp2f(sm_ml[(w * G + g) * 2] - mt);
+        lt += sm_ml[(w * G + g) * 2 + 1] * wgt;
+        ot += sm_o[(w * G + g) * DH + d] * wgt;
+      }
+      if (direct) {
+        p.out[static_cast<size_t>(b) * p.ldo + (kvh * G + g) * DH + d] = __float2bfloat16_rn(lt > 0.f ? ot / lt : 0.f);
+      } else {
+        slot[g * DH + d] = ot;
+        if (d == 0) { slot[16 * DH + g * 2] = mt; slot[16 * DH + g * 2 + 1] = lt; }
+      }
+    }
+    if (!direct) {
+      __threadfence();
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (threadIdx.x == 0) {
+        const unsigned int prev = atomicAdd(p.counters + job, 1u);
+        s_last = (prev == static_cast<unsigned int>(c_last - c_first)) ? 1 : 0;
+        if (s_last) p.counters[job] = 0;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (s_last) {
+        __threadfence();
+        const int np = c_last - c_first + 1;
+        // the first sharing CTA's piece is its second slot unless its range starts with this job
+        const int first_odd = c_first * T / grid < s_job ? 1 : 0;
+        for (int i = threadIdx.x; i < G * DH; i += 256) {
+          const int g = i / DH, d = i - g * DH;
+          const float* base = p.part + static_cast<size_t>(2 * c_first) * SLOT;
+          float mt = -1.0e30f;
+          for (int s0 = 0; s0 < np; s0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+              const int s = s0 + x;
+              v[x] = s < np ? __ldcg(base + static_cast<size_t>(2 * s + (s == 0 ? first_odd : 0)) * SLOT + 16 * DH + g * 2) : -1.0e30f;
+            }
+#pragma unroll
+            for (int x = 0; x < 8; ++x) mt = fmaxf(mt, v[x]);
+          }
+          float lt = 0.f, ot = 0.f;
+          for (int s0 = 0; s0 < np; s0 += 8) {   // eight pieces' loads in flight, added in piece order
+            float vm[8], vl[8], vo[8];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+              const int s = s0 + x;
+              const float* sp = base + static_cast<size_t>(2 * s + (s == 0 ? first_odd : 0)) * SLOT;
+              vm[x] = s < np ? __ldcg(sp + 16 * DH + g * 2) : -1.0e30f;
+              vl[x] = s < np ? __ldcg(sp + 16 * DH + g * 2 + 1) : 0.f;
+              vo[x] = s < np ? __ldcg(sp + g * DH + d) : 0.f;
+            }
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+              if (s0 + x < np) {
+                const float wgt = exp2f(vm[x] - mt);
+                lt += vl[x] * wgt;
+                ot += vo[x] * wgt;
+              }
+            }
+          }
+          p.out[static_cast<size_t>(b) * p.ldo + (kvh * G + g) * DH + d] = __float2bfloat16_rn(lt > 0.f ? ot / lt : 0.f);
+        }
+      }
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");   // the merge buffers and s_last are free again
+    u += t_end - t_beg;
+  }
+  pdl_trigger();
+}
+
+// ---------------------------------------------------------------------------
 // Arg-max over logits rows with the rule of the reference's greedy loop (`best = row[0]; if v > best`,
 // scirust-cuda/src/decode.rs:107-114): a NaN in column 0 makes token 0 win outright; any other NaN is
 // skipped explicitly (`v != v`), never left to how a comparison with NaN folds; among equal maxima the
@@ -1639,6 +2030,7 @@ static int launch_gemv(const GemvParams& p, int splits, cudaStream_t s) {
 namespace sb {
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
                       uint32_t box_inner, uint32_t box_outer);   // gemm_tcgen05.cu (128-byte swizzle)
+int num_sms();
 }
 
 // bf16 weights: the tensor-core kernel. The staged slice of X takes 16 bytes per k for every 8 rows.
@@ -1867,6 +2259,49 @@ extern "C" int sb_decode_attention(const void* q, int ldq, const void* pool, con
   p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.counters = counters;
   dim3 grid(Hkv, B, n_splits);
   return dh == 64 ? launch_decode_attn<64>(p, grid, STREAM) : launch_decode_attn<128>(p, grid, STREAM);
+}
+
+template <int DH>
+static int launch_decode_stream(const CUtensorMap& tm, DecodeStreamParams p, int grid, cudaStream_t s) {
+  auto kern = decode_attn_stream_kernel<DH>;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess)
+      return SB_ERR_LAUNCH;
+    attr = true;
+  }
+  const int G = p.H / p.Hkv;
+  p.stages = DstCfg<DH>::stages(G);
+  return launch_dep(kern, dim3(grid), dim3(DST_THREADS), DstCfg<DH>::smem_bytes(G), s, tm, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+}
+
+// The same attention as one balanced stream of KV tiles. pool: n_blocks pages (n_blocks * 2 * Hkv * page < 2^31, base
+// 16-byte aligned), page 8, 16, 32 or a multiple of 64, B <= 1024, B * Hkv counters (zero before the first call, left
+// zero). max_tiles: an upper bound of the 64-position tiles of all (sequence, kv head) pairs, which only caps the grid.
+// part: 2 * (SMs) * 16 * (dh + 2) floats.
+extern "C" int sb_decode_attention_stream(const void* q, int ldq, const void* pool, int n_blocks,
+                                          const int* block_table, int max_blocks, int page, const int* seq_len, int B,
+                                          int H, int Hkv, int dh, int max_tiles, float scale, float* part,
+                                          unsigned int* counters, void* out, int ldo, int* status, void* stream) {
+  if (B <= 0 || B > DST_MAX_B || H <= 0 || Hkv <= 0 || (H % Hkv) || H / Hkv > 16 || dh != 128 ||
+      n_blocks < 1 || max_tiles < 1 || (ldq & 1) || !status)
+    return SB_ERR_ARG;
+  if (page != 8 && page != 16 && page != 32 && (page < 64 || page % 64)) return SB_ERR_ARG;
+  const uint64_t rows = static_cast<uint64_t>(n_blocks) * 2 * Hkv * page;
+  if (rows >= (1ull << 31)) return SB_ERR_TOO_LARGE;
+  CUtensorMap tm;
+  const int rc = make_tmap_2d_bf16(&tm, pool, dh, rows, dh, 64, page < DEC_TK ? page : DEC_TK);
+  if (rc) return rc;
+  DecodeStreamParams p;
+  p.q = static_cast<const __nv_bfloat16*>(q); p.ldq = ldq;
+  p.block_table = block_table; p.max_blocks = max_blocks; p.page = page; p.seq_len = seq_len;
+  p.B = B; p.H = H; p.Hkv = Hkv;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.part = part; p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.counters = counters; p.status = status;
+  // a CTA with less than two tiles has nothing to overlap; more CTAs than that only add pieces to merge
+  int grid = (max_tiles + 1) / 2;
+  if (grid > num_sms()) grid = num_sms();
+  return launch_decode_stream<128>(tm, p, grid, STREAM);
 }
 
 // logits: fp32 [rows, V]. pval/pidx: rows * ceil(V/4096) scratch. out_tokens: int64 [rows].

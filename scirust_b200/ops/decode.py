@@ -18,6 +18,8 @@ _lib.register("sb_rope_kv_append", [vp, i32, i32, i32, i32, vp, vp, vp, vp, i32,
 _lib.register("sb_kv_append", [vp, i32, i32, i32, i32, vp, vp, i32, i32, vp, vp, i32, vp])
 _lib.register("sb_decode_attention", [vp, i32, vp, vp, i32, i32, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp, i32,
                                       vp])
+_lib.register("sb_decode_attention_stream", [vp, i32, vp, i32, vp, i32, i32, vp, i32, i32, i32, i32, i32, f32, vp, vp, vp,
+                                             i32, vp, vp])
 _lib.register("sb_argmax", [vp, i32, i32, vp, vp, vp, vp, i32, i32, vp])
 _lib.register("sb_quantize_per_channel", [vp, i32, i32, i32, vp, vp, vp])
 _lib.register("sb_dequantize", [vp, vp, i32, i32, vp, vp])
@@ -466,14 +468,44 @@ def decode_attention_ref(q, pool, block_table, page, seq_len, H, Hkv, dh, scale=
     return out
 
 
+def _stream_wins(L, tiles, device) -> bool:
+    """Where the balanced stream beats the split kernel, by the 64-position tiles per SM of the batch. Measured at 32 / 8
+    heads (us, split against stream): 1 x 2048 15.4 / 13.2, 1 x 8192 43.4 / 20.6, 4 x 2048 23.9 / 18.2, 16 x 512 20.8 / 17.5,
+    16 x 2304 41.1 / 33.3, 64 x 2048 108.5 / 87.5; but 4 x 1024 14.3 / 19.7, 16 x 256 12.6 / 15.8, 64 x 128 14.5 / 22.0: its
+    start and the merge of many short pieces need six tiles per SM, or long sequences (where the split kernel's 64 splits
+    and its last wave bind), to pay."""
+    per_sm = tiles / _g.num_sms(device)
+    return L >= 256 and per_sm >= (1.5 if L >= 2048 else 6.0)
+
+
+def _stream_ok(pool, page, B, H, Hkv, dh) -> bool:
+    """Whether the balanced streaming kernel takes this cache: page sizes whose tiles are whole TMA boxes, tensor-map
+    coordinates within 31 bits, counters and the offset table of its shared memory large enough."""
+    return (B <= 1024 and B * Hkv <= 2048 and H // Hkv <= 16 and dh == 128 and pool.is_contiguous()
+            and (page in (8, 16, 32) or (page >= 64 and page % 64 == 0)) and pool.data_ptr() % 16 == 0
+            and pool.shape[0] * 2 * Hkv * page < 1 << 31)
+
+
 def decode_attention(q, pool, block_table, page, seq_len, H, Hkv, dh, scale=None, n_splits=None, max_len=None):
     """Single-query GQA attention of each sequence over its paged KV. q: [B, >= H*dh] (RoPE'd)."""
     scale = 1.0 / math.sqrt(dh) if scale is None else scale
     B = q.shape[0]
     if not q.is_cuda:
         return decode_attention_ref(q, pool, block_table, page, seq_len, H, Hkv, dh, scale).to(BF)
+    L = max_len if max_len is not None else block_table.shape[1] * page
+    tiles = B * Hkv * max(1, (L + 63) // 64)
+    if n_splits is None and _stream_wins(L, tiles, q.device) and _stream_ok(pool, page, B, H, Hkv, dh):
+        # the tiles of the whole batch dealt out evenly over the SMs; an explicit split count keeps the kernel below
+        part = _workspace(2 * _g.num_sms(q.device) * 16 * (dh + 2), q.device)
+        ctr = _gemv_workspace(4096, q.device)
+        out = _lib.empty((B, H * dh), BF, q.device)
+        _lib.call("sb_decode_attention_stream", q.data_ptr(), q.stride(0), pool.data_ptr(), pool.shape[0],
+                  block_table.data_ptr(), block_table.shape[1], page, seq_len.data_ptr(), B, H, Hkv, dh,
+                  tiles, float(scale), part.data_ptr(), ctr.data_ptr() + 2048 * 4,
+                  out.data_ptr(), out.stride(0), _lib.status_word(q.device).data_ptr(), _lib.stream())
+        _g.launch_count += 1
+        return out
     if n_splits is None:
-        L = max_len if max_len is not None else block_table.shape[1] * page
         # about four 128-thread CTAs per SM, at least two 64-position tiles per split
         n_splits = max(1, min(64, (148 * 4 + B * Hkv - 1) // max(1, B * Hkv), (L + 127) // 128))
     ws = _workspace(B * H * n_splits * (dh + 2), q.device)

@@ -231,3 +231,36 @@ def test_dequantize_is_the_rounded_product(K, N):
     scale = torch.rand(N, generator=g, device="cuda") * 0.01 + 1e-4
     want = (q.float() * scale[None, :]).to(BF)
     assert torch.equal(D.QuantWeight(q, scale).dequantize(), want)
+
+
+@pytest.mark.parametrize("dh,H,Hkv", [(128, 32, 8), (128, 16, 1), (128, 3, 3), (128, 8, 1)])
+@pytest.mark.parametrize("page", [8, 16, 32, 64, 192])
+def test_paged_decode_attention_stream(dh, H, Hkv, page, monkeypatch):
+    """The balanced tile stream (no explicit split count): ragged lengths around the 64-position tile, an empty and a
+    one-position sequence, jobs inside one CTA and across many, several page sizes; positions past the end and pages of
+    nobody hold NaN and must not be seen."""
+    monkeypatch.setattr(D, "_stream_wins", lambda *a: True)
+    for lens in ([0, 1, 63, 64, 65, 700], [1500], [200] * 40):
+        B, longest = len(lens), max(lens)
+        max_blocks = (longest + page - 1) // page
+        n_blocks = B * max_blocks + 3
+        pool = torch.full((n_blocks, 2, Hkv, page, dh), float("nan"), dtype=BF, device="cuda")
+        table = torch.randperm(n_blocks, generator=torch.Generator().manual_seed(page))[:B * max_blocks].int()
+        table = table.reshape(B, max_blocks).cuda()
+        ld = (H + 2 * Hkv) * dh
+        for b, L in enumerate(lens):
+            if L:
+                D.kv_append(_r((L, ld), 10 + b), H, Hkv, dh, pool, table, page,
+                            torch.full((L,), b, dtype=torch.int32, device="cuda"),
+                            torch.arange(L, dtype=torch.int32, device="cuda"))
+        ln = torch.tensor(lens, dtype=torch.int32, device="cuda")
+        q = _r((B, ld), 20)
+        out = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, max_len=longest)
+        ref = D.decode_attention_ref(q, pool.nan_to_num(0.0), table, page, ln.clamp(min=1), H, Hkv, dh)
+        ref[ln == 0] = 0.0
+        assert (out.float() - ref).abs().max().item() < 2e-2
+        assert torch.equal(out, D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, max_len=longest))
+        one = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, n_splits=1)
+        assert (out.float() - one.float()).abs().max().item() < 2e-2
+    from scirust_b200.ops import _lib
+    _lib.check_status(torch.device("cuda"))
