@@ -2,7 +2,7 @@
 (conv 1->32->64 3x3 + ReLU + 2x2 max-pool -> Linear 128 -> 10; docs/MNIST.md:27-34) and a
 CIFAR-shaped ResNet-18 (3x3 stem, channels 64/128/256/512, BatchNorm, ReLU, global average pool,
 FC; scirust-core/src/nn/vision.rs:65-72). Parameters are fp32 masters; compute runs in bf16 through
-``ops.conv`` (im2col + tcgen05 GEMM, BatchNorm and pooling kernels) on CUDA and through
+``ops.conv`` (tcgen05 convolution products, BatchNorm and pooling kernels) on CUDA and through
 ``torch.nn.functional`` on CPU. Convolution weights are kept in the packed ``[out_c, pad8(k*k*in_c)]``
 layout; ``state_dict_ref`` converts back to the reference's ``(out_c, in_c*k*k)``."""
 from __future__ import annotations
