@@ -1518,7 +1518,7 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap);
-    for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+    for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 8); }
     fence_barrier_init();
   }
   pdl_wait();
@@ -1643,10 +1643,15 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
       const int st = stage;
       const uint32_t ph = phase;
       if (++stage == stages) { stage = 0; phase ^= 1; }
-      // the other group's tiles are waited for too: a parity wait tells a stage's fill from its next one only as long as
-      // nobody is a whole fill ahead
+      // All eight warps wait for and release every tile, the other group's too: a parity wait tells one fill of a stage from
+      // the next only while no warp is a whole fill ahead (it would pass on the previous fill) or behind (it would wait
+      // for the fill after next, which in turn waits for it).
       if (ok && !mbar_wait(&full[st], ph, p.status, ST_TIMEOUT_FULL)) ok = false;
-      if (!ok || ((t - t_beg) & 1) != group) continue;
+      if (!ok) continue;
+      if (((t - t_beg) & 1) != group) {
+        if (lane == 0) mbar_arrive(&empty[st]);
+        continue;
+      }
       uint8_t* kp = ring + st * 2 * C::TILE_BYTES;
       uint8_t* vp = kp + C::TILE_BYTES;
       const uint32_t kt = smem_u32(kp), vt = smem_u32(vp);

@@ -264,3 +264,21 @@ def test_paged_decode_attention_stream(dh, H, Hkv, page, monkeypatch):
         assert (out.float() - one.float()).abs().max().item() < 2e-2
     from scirust_b200.ops import _lib
     _lib.check_status(torch.device("cuda"))
+
+
+def test_decode_attention_stream_repeats_under_load(monkeypatch):
+    """The ring of the streamed attention refills a stage only after all eight consumer warps have passed its fill: many
+    repetitions over long sequences give the same bits, and no bounded wait runs out."""
+    monkeypatch.setattr(D, "_stream_wins", lambda *a: True)
+    B, L, H, Hkv, dh, page = 48, 1600, 32, 8, 128, 64
+    nb = L // page
+    pool = _r((B * nb, 2, Hkv, page, dh), 1)
+    table = torch.randperm(B * nb, generator=torch.Generator().manual_seed(2)).int().reshape(B, nb).cuda()
+    ln = torch.randint(L // 2, L + 1, (B,), generator=torch.Generator().manual_seed(3)).int().cuda()
+    q = _r((B, (H + 2 * Hkv) * dh), 4)
+    first = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, max_len=L)
+    for _ in range(300):
+        last = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, max_len=L)
+    assert torch.equal(first, last)
+    from scirust_b200.ops import _lib
+    _lib.check_status(torch.device("cuda"))
