@@ -26,6 +26,16 @@ _lib.register("sb_attention_bwd", [_lib.vp, _lib.vp, _lib.vp, _lib.vp, _lib.vp, 
 # rescaled only when a row maximum grows by more than 2^8); SB_ATT_FWD=single selects the one-tile kernel.
 FWD_TWO_TILES = os.environ.get("SB_ATT_FWD", "pair") != "single"
 
+
+def _two_tiles_win(B, S, H, device) -> bool:
+    """Where the two-tile kernel is the faster one: when its CTAs outnumber the SMs. Below that every CTA runs by itself, and
+    an iteration over one kv block for one tile (2.4 us at head dimension 128) beats one for two (3.0 us). Measured, one
+    tile against two, us: dh 128, 32 heads 1 x 512 13.8 / 16.3, 1 x 1024 (128 CTAs) 26.6 / 27.2, 1 x 1500 (192) 51.9 / 36.7,
+    3 x 2048 238 / 153; dh 64, 16 heads 1 x 512 11.4 / 13.9, 2 x 512 11.6 / 14.0, 3 x 1000 (192) 24.8 / 23.9,
+    1 x 4096 88.6 / 70.8."""
+    return B * H * ((S + 255) // 256) > _g.num_sms(device)
+
+
 # The backward pass spills its dS tiles (bf16 [B*H, S, S]) to a scratch buffer so that dQ is a streamed
 # product instead of a second pass over scores and exponentials; above this size it recomputes instead.
 DS_SCRATCH_LIMIT_BYTES = int(os.environ.get("SB_ATT_DS_SCRATCH_MB", "4096")) << 20
@@ -69,7 +79,7 @@ def attention_fwd(qkv, B, S, H, Hkv, dh, causal=True, scale=None, want_lse=True)
         raise ValueError("qkv must be a 2-D bf16 matrix with unit inner stride")
     out = _lib.empty((B * S, H * dh), torch.bfloat16, qkv.device)
     lse = _lib.empty((B, H, S), torch.float32, qkv.device) if want_lse else None
-    entry = "sb_attention_fwd_pp" if FWD_TWO_TILES else "sb_attention_fwd"
+    entry = "sb_attention_fwd_pp" if FWD_TWO_TILES and _two_tiles_win(B, S, H, qkv.device) else "sb_attention_fwd"
     _lib.call(entry, qkv.data_ptr(), out.data_ptr(), _lib.ptr(lse), B, S, H, Hkv, dh, qkv.stride(0),
               out.stride(0), float(scale), int(causal), _lib.status_word(qkv.device).data_ptr(), _lib.stream())
     _g.launch_count += 1

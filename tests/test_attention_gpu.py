@@ -85,6 +85,7 @@ def test_forward_two_tiles_head_dimension_128(B, S, H, Hkv, causal, monkeypatch)
     qkv[:, :, H:H + Hkv] *= (1.0 + 4.0 * torch.arange(S, device="cuda") / S).reshape(1, S, 1, 1)
     qkv = qkv.reshape(B * S, -1).to(torch.bfloat16)
     monkeypatch.setattr(A, "FWD_TWO_TILES", True)
+    monkeypatch.setattr(A, "_two_tiles_win", lambda *a: True)
     o, lse = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal)
     again, _ = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal)
     monkeypatch.setattr(A, "FWD_TWO_TILES", False)
