@@ -138,7 +138,12 @@ def _auto_splits(N, K, cols, M=1, quant=False):
     kernel's 64 KB: 16 bytes per k (8 rows of 16-bit values) in the tensor-core kernels, (K / splits) rows x
     {1,2,4,8} floats in the FMA kernels that SB_GEMV_FMA=1 selects."""
     ctas = (N + cols - 1) // cols
-    s = max(1, min(148 * 2 // max(ctas, 1), K // 64))
+    # at least 128 rows of k per split, and at most 18 of them with int8 weights: the finish reads one partial per split, and
+    # past that it costs more than the shorter stream saves (us, one row: bf16 2816 x 1024 at 44 splits 8.0, at 22 6.9; int8
+    # 4096 x 4096 at 37 14.4, at 18 12.4; five rows: bf16 2816 x 1024 20.7 / 14.0, int8 4096 x 6144 at 24 29.4, at 12 23.5)
+    s = max(1, min(148 * 2 // max(ctas, 1), K // 128))
+    if quant:
+        s = min(s, 18)
     if ctas > 148 * 2 and not quant:
         # several waves of column blocks (an LM head): eight k-splits keep more CTAs streaming at once and shorten
         # the tail (4096 x 128256: 213 us with one split, 176 us with eight)
