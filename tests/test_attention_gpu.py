@@ -76,11 +76,11 @@ def test_backward(B, S, H, Hkv, dh, causal, spill, monkeypatch):
 @pytest.mark.parametrize("B,S,H,Hkv", [(1, 1, 1, 1), (2, 127, 2, 1), (1, 129, 2, 2), (3, 256, 4, 1), (1, 257, 2, 1),
                                        (2, 1000, 4, 2), (1, 2048, 8, 2)])
 @pytest.mark.parametrize("causal", [True, False])
-def test_forward_two_tiles_head_dimension_128(B, S, H, Hkv, causal, monkeypatch):
-    """Tile edges of the two-tile kernel at 128 (second tile empty, one row, full; K in two stages, V in half tiles)
+@pytest.mark.parametrize("dh", [64, 128])
+def test_forward_two_tiles_at_tile_edges(B, S, H, Hkv, causal, dh, monkeypatch):
+    """Tile edges of the two-tile kernel (second tile empty, one row, full; at 128 K in two stages, V in half tiles)
     against the dense statement and, with growing keys (the accumulator is rescaled), the one-tile kernel: both keep P in
     bf16 (2^-8 of each term), so they agree to 2^-7 of the largest value."""
-    dh = 128
     qkv = _qkv(B, S, H, Hkv, dh, seed=S).float().reshape(B, S, H + 2 * Hkv, dh)
     qkv[:, :, H:H + Hkv] *= (1.0 + 4.0 * torch.arange(S, device="cuda") / S).reshape(1, S, 1, 1)
     qkv = qkv.reshape(B * S, -1).to(torch.bfloat16)
