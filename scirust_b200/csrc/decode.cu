@@ -1800,41 +1800,63 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
         const int np = c_last - c_first + 1;
         // the first sharing CTA's piece is its second slot unless its range starts with this job
         const int first_odd = c_first * T / grid < s_job ? 1 : 0;
-        for (int i = threadIdx.x; i < G * DH; i += 256) {
-          const int g = i / DH, d = i - g * DH;
-          const float* base = p.part + static_cast<size_t>(2 * c_first) * SLOT;
-          float mt = -1.0e30f;
-          for (int s0 = 0; s0 < np; s0 += 8) {
-            float v[8];
+        const float* base = p.part + static_cast<size_t>(2 * c_first) * SLOT;
+        auto piece = [&](int s) { return base + static_cast<size_t>(2 * s + (s == 0 ? first_odd : 0)) * SLOT; };
+        // a piece's (max, sum) of every row first, all loads at once; a warp then turns a row's maxima into weights, and the
+        // sums take 16-byte loads (a job of 1 x 2048 positions has 16 pieces: 14.0 -> 10.7 us for the whole kernel)
+        float* w_m = sm_o;                             // [np][G] maxima, then weights
+        float* w_l = sm_o + np * G;                    // [np][G] sums; row g's total ends up in w_l[g]
+        for (int i = threadIdx.x; i < np * G; i += 256) {
+          const int s = i / G, g = i - s * G;
+          const float2 ml = __ldcg(reinterpret_cast<const float2*>(piece(s) + 16 * DH + g * 2));
+          w_m[i] = ml.x;
+          w_l[i] = ml.y;
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        for (int g = warp; g < G; g += 8) {
+          float mt = -1.0e30f, lt = 0.f;
+          for (int s = lane; s < np; s += 32) mt = fmaxf(mt, w_m[s * G + g]);
 #pragma unroll
-            for (int x = 0; x < 8; ++x) {
-              const int s = s0 + x;
-              v[x] = s < np ? __ldcg(base + static_cast<size_t>(2 * s + (s == 0 ? first_odd : 0)) * SLOT + 16 * DH + g * 2) : -1.0e30f;
-            }
-#pragma unroll
-            for (int x = 0; x < 8; ++x) mt = fmaxf(mt, v[x]);
+          for (int o2 = 16; o2 > 0; o2 >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o2));
+          for (int s = lane; s < np; s += 32) {
+            const float wgt = exp2f(w_m[s * G + g] - mt);
+            w_m[s * G + g] = wgt;
+            lt += w_l[s * G + g] * wgt;
           }
-          float lt = 0.f, ot = 0.f;
-          for (int s0 = 0; s0 < np; s0 += 8) {   // eight pieces' loads in flight, added in piece order
-            float vm[8], vl[8], vo[8];
 #pragma unroll
-            for (int x = 0; x < 8; ++x) {
-              const int s = s0 + x;
-              const float* sp = base + static_cast<size_t>(2 * s + (s == 0 ? first_odd : 0)) * SLOT;
-              vm[x] = s < np ? __ldcg(sp + 16 * DH + g * 2) : -1.0e30f;
-              vl[x] = s < np ? __ldcg(sp + 16 * DH + g * 2 + 1) : 0.f;
-              vo[x] = s < np ? __ldcg(sp + g * DH + d) : 0.f;
-            }
+          for (int o2 = 16; o2 > 0; o2 >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o2);
+          __syncwarp();
+          if (lane == 0) w_l[g] = lt;                  // row g of piece 0, read by this warp only
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        for (int i = threadIdx.x; i < G * (DH / 4); i += 256) {
+          const int g = i / (DH / 4), d = (i - g * (DH / 4)) * 4;
+          float4 ot = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int s0 = 0; s0 < np; s0 += 4) {   // four pieces' loads in flight, added in piece order
+            float4 vo[4];
 #pragma unroll
-            for (int x = 0; x < 8; ++x) {
+            for (int x = 0; x < 4; ++x)
+              if (s0 + x < np) vo[x] = __ldcg(reinterpret_cast<const float4*>(piece(s0 + x) + g * DH + d));
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
               if (s0 + x < np) {
-                const float wgt = exp2f(vm[x] - mt);
-                lt += vl[x] * wgt;
-                ot += vo[x] * wgt;
+                const float wgt = w_m[(s0 + x) * G + g];
+                ot.x += vo[x].x * wgt; ot.y += vo[x].y * wgt; ot.z += vo[x].z * wgt; ot.w += vo[x].w * wgt;
               }
             }
           }
-          p.out[static_cast<size_t>(b) * p.ldo + (kvh * G + g) * DH + d] = __float2bfloat16_rn(lt > 0.f ? ot / lt : 0.f);
+          const float lt = w_l[g], inv = lt > 0.f ? 1.f : 0.f;
+          const float dn = lt > 0.f ? lt : 1.f;
+          uint2 pk;
+          pk.x = dpack(ot.x / dn * inv, ot.y / dn * inv);
+          pk.y = dpack(ot.z / dn * inv, ot.w / dn * inv);
+          __nv_bfloat16* dst = p.out + static_cast<size_t>(b) * p.ldo + (kvh * G + g) * DH + d;
+          if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) *reinterpret_cast<uint2*>(dst) = pk;
+          else {
+            uint16_t* d16 = reinterpret_cast<uint16_t*>(dst);
+            d16[0] = static_cast<uint16_t>(pk.x); d16[1] = static_cast<uint16_t>(pk.x >> 16);
+            d16[2] = static_cast<uint16_t>(pk.y); d16[3] = static_cast<uint16_t>(pk.y >> 16);
+          }
         }
       }
     }

@@ -475,8 +475,8 @@ def decode_attention_ref(q, pool, block_table, page, seq_len, H, Hkv, dh, scale=
 
 def _stream_wins(L, tiles, device) -> bool:
     """Where the balanced stream beats the split kernel, by the 64-position tiles per SM of the batch. Measured at 32 / 8
-    heads (us, split against stream): 1 x 2048 15.4 / 13.2, 1 x 8192 43.4 / 20.6, 4 x 2048 23.9 / 18.2, 16 x 512 20.8 / 17.5,
-    16 x 2304 41.1 / 33.3, 64 x 2048 108.5 / 87.5; but 4 x 1024 14.3 / 19.7, 16 x 256 12.6 / 15.8, 64 x 128 14.5 / 22.0: its
+    heads (us, split against stream): 1 x 2048 15.2 / 10.7, 1 x 8192 44.2 / 18.8, 4 x 2048 21.8 / 17.8, 16 x 512 20.9 / 18.1,
+    16 x 2304 41.6 / 33.9, 64 x 2048 103.2 / 87.6; but 4 x 1024 14.3 / 16.0, 16 x 256 12.6 / 16.0, 64 x 128 14.5 / 22.5: its
     start and the merge of many short pieces need six tiles per SM, or long sequences (where the split kernel's 64 splits
     and its last wave bind), to pay."""
     per_sm = tiles / _g.num_sms(device)
