@@ -118,7 +118,256 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 }
 
 // --------------------------------------------------------------------------- dK / dV
-// Pipeline: scores and dP have barriers of their own, so the exponentials of iteration t+1 (which need the scores only)
+// Pipeline (DH == 64): the bf16 P^T / dS^T tiles are double-buffered in shared memory, so the MMA
+// warp issues the score products of iteration t+1 *before* the gradient products of iteration t;
+// the softmax warps then work on t+1 while the tensor cores finish t. With DH == 128 shared
+// memory only fits single buffers and the two groups are issued in program order.
+template <int DH>
+struct DkvCfg {
+  static constexpr bool PDB = (DH == 64);             // double-buffer P^T / dS^T
+  static constexpr int NPB = PDB ? 2 : 1;
+  static constexpr int QS = (DH == 64) ? 2 : 1;       // (Q, dO) ring stages
+  static constexpr int T_BYTES = BT * DH * 2;         // one [128 x DH] tile
+  static constexpr int PT_BYTES = BT * BT * 2;
+  static constexpr int TILE_BYTES = 2 * T_BYTES + QS * 2 * T_BYTES + NPB * 2 * PT_BYTES;
+  static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 128;
+  static constexpr int TMEM_COLS = 512;  // S^T 128 | dP^T 128 | dK DH | dV DH
+};
+
+template <int DH>
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
+                         const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
+  using Cfg = DkvCfg<DH>;
+  constexpr int NCH = DH / 64;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sK = smem;
+  uint8_t* sV = sK + Cfg::T_BYTES;
+  uint8_t* sQ = sV + Cfg::T_BYTES;                 // QS stages
+  uint8_t* sdO = sQ + Cfg::QS * Cfg::T_BYTES;      // QS stages
+  uint8_t* sPT = sdO + Cfg::QS * Cfg::T_BYTES;     // NPB buffers
+  uint8_t* sdST = sPT + Cfg::NPB * Cfg::PT_BYTES;  // NPB buffers
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sdST + Cfg::NPB * Cfg::PT_BYTES);
+  uint64_t* kv_full = bars;
+  uint64_t* q_full = bars + 1;            // QS
+  uint64_t* q_empty = q_full + Cfg::QS;   // QS
+  uint64_t* st_full = q_empty + Cfg::QS;
+  uint64_t* p_full = st_full + 1;
+  uint64_t* done = p_full + 1;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_t = (p.S + BT - 1) / BT;
+  // The kv tile is the slowest grid index: CTAs are handed out in block-id order, so all the long tiles
+  // (causal: small kt, up to 4x16 query tiles) start first and the short ones fill the tail.
+  const int kt = blockIdx.z;  // kv tile
+  const int kvh = blockIdx.x, b = blockIdx.y;
+  const int group = p.H / p.Hkv;
+  const int kv0 = kt * BT;
+  const int row_base = b * p.S;
+  const int qt_first = p.causal ? kt : 0;
+  const int n_qt = n_t - qt_first;
+  const int n_iter = group * n_qt;  // iteration t -> head kvh*group + t / n_qt, q tile qt_first + t % n_qt
+
+  if (threadIdx.x == 0) {
+    mbar_init(kv_full, 1);
+    for (int s = 0; s < Cfg::QS; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
+    mbar_init(st_full, 1);
+    mbar_init(p_full, 8);  // one arrival per softmax warp
+    mbar_init(done, 1);
+    fence_barrier_init();
+    fence_proxy_async_smem();
+  }
+  if (warp == 0 && lane == 0) { prefetch_tmap(&tm_qkv); prefetch_tmap(&tm_do); }
+  if (warp == 1) { tmem_alloc(tmem_holder, Cfg::TMEM_COLS); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  // S and dP are [query x kv] (TMEM lane = query row, as in the dQ kernel); their bf16 images P and dS
+  // are stored [q rows][kv] and consumed as MN-major A operands (A^T) by the dV / dK products.
+  const uint32_t tm_ST = tmem_base, tm_dPT = tmem_base + 128, tm_dK = tmem_base + 256, tm_dV = tmem_base + 256 + DH;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      mbar_arrive_expect_tx(kv_full, 2 * Cfg::T_BYTES);
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        tma_load_2d(sK + c * (BT * 128), &tm_qkv, kv_full, (p.H + kvh) * DH + c * 64, row_base + kv0);
+        tma_load_2d(sV + c * (BT * 128), &tm_qkv, kv_full, (p.H + p.Hkv + kvh) * DH + c * 64, row_base + kv0);
+      }
+      int st = 0;
+      uint32_t ph = 0;
+      for (int t = 0; t < n_iter; ++t) {
+        const int head = kvh * group + t / n_qt;
+        const int qt = qt_first + t % n_qt;
+        if (!mbar_wait(&q_empty[st], ph ^ 1, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_arrive_expect_tx(&q_full[st], 2 * Cfg::T_BYTES);
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) {
+          tma_load_2d(sQ + st * Cfg::T_BYTES + c * (BT * 128), &tm_qkv, &q_full[st], head * DH + c * 64,
+                      row_base + qt * BT);
+          tma_load_2d(sdO + st * Cfg::T_BYTES + c * (BT * 128), &tm_do, &q_full[st], head * DH + c * 64,
+                      row_base + qt * BT);
+        }
+        if (++st == Cfg::QS) { st = 0; ph ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = make_idesc_bf16(BT, BT, false, false);   // [q x kv], both K-major
+      constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, true, true);     // [kv x dh] = A^T B, both MN-major
+      bool ok = mbar_wait(kv_full, 0, p.status, ST_TIMEOUT_FULL);
+      int st_s = 0;          // stage / phase of the next score issue
+      uint32_t ph_s = 0;
+      int st_g = 0;          // stage of the next gradient issue
+      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV);
+      auto issue_scores = [&]() -> bool {
+        if (!mbar_wait(&q_full[st_s], ph_s, p.status, ST_TIMEOUT_FULL)) return false;
+        tc_fence_after();
+        const uint32_t bQ = smem_u32(sQ + st_s * Cfg::T_BYTES), bdO = smem_u32(sdO + st_s * Cfg::T_BYTES);
+#pragma unroll
+        for (int k = 0; k < DH / 16; ++k) {
+          const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
+          umma_bf16_ss(tm_ST, make_smem_desc(bQ + off, 16, 1024), make_smem_desc(aK + off, 16, 1024), idesc_s,
+                       k > 0 ? 1u : 0u);
+        }
+#pragma unroll
+        for (int k = 0; k < DH / 16; ++k) {
+          const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
+          umma_bf16_ss(tm_dPT, make_smem_desc(bdO + off, 16, 1024), make_smem_desc(aV + off, 16, 1024), idesc_s,
+                       k > 0 ? 1u : 0u);
+        }
+        umma_commit(st_full);
+        if (++st_s == Cfg::QS) { st_s = 0; ph_s ^= 1; }
+        return true;
+      };
+      auto issue_grads = [&](int t) {
+        const int pb = Cfg::PDB ? (t & 1) : 0;
+        const uint32_t aPT = smem_u32(sPT + pb * Cfg::PT_BYTES), adST = smem_u32(sdST + pb * Cfg::PT_BYTES);
+        const uint32_t bQ = smem_u32(sQ + st_g * Cfg::T_BYTES), bdO = smem_u32(sdO + st_g * Cfg::T_BYTES);
+#pragma unroll
+        for (int k = 0; k < BT / 16; ++k) {   // k walks 16 query rows at a time in both operands
+          umma_bf16_ss(tm_dV, make_smem_desc(aPT + k * (16 * 128), BT * 128, 1024),
+                       make_smem_desc(bdO + k * (16 * 128), BT * 128, 1024), idesc_g, (t > 0 || k > 0) ? 1u : 0u);
+        }
+#pragma unroll
+        for (int k = 0; k < BT / 16; ++k) {
+          umma_bf16_ss(tm_dK, make_smem_desc(adST + k * (16 * 128), BT * 128, 1024),
+                       make_smem_desc(bQ + k * (16 * 128), BT * 128, 1024), idesc_g, (t > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit(&q_empty[st_g]);
+        if (++st_g == Cfg::QS) st_g = 0;
+      };
+      if (ok && n_iter > 0) ok = issue_scores();
+      for (int t = 0; t < n_iter && ok; ++t) {
+        if (!mbar_wait(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
+        tc_fence_after();
+        // scores of t+1 first (double-buffered P^T / dS^T): the softmax warps wait for nothing else, and the
+        // commit of these scores also covers the gradient MMAs of t-1, which is what lets the softmax warps
+        // reuse the P^T / dS^T buffer of parity (t+1)&1
+        // (the dS store of t-1 has long been read out of its buffer; the wait only makes that certain before the
+        // scores whose completion lets the softmax warps write that buffer again)
+        if (p.spill_ds) tma_store_wait_read<0>();
+        if (Cfg::PDB && t + 1 < n_iter) ok = issue_scores();
+        if (p.spill_ds) {
+          // the finished dS tile (bf16, [q rows][kv], scale included) also goes to global memory, where
+          // the dQ kernel streams it back instead of recomputing scores; the bulk store reads shared
+          // memory asynchronously, so it must have been read out before this buffer is written again
+          const int head = kvh * group + t / n_qt;
+          const int qt = qt_first + t % n_qt;
+          const uint8_t* src = sdST + (Cfg::PDB ? (t & 1) : 0) * Cfg::PT_BYTES;
+          tma_store_3d(&tm_ds, src, kv0, qt * BT, b * p.H + head);
+          tma_store_3d(&tm_ds, src + BT * 128, kv0 + 64, qt * BT, b * p.H + head);
+          tma_store_commit();
+        }
+        issue_grads(t);
+        if (!Cfg::PDB) {
+          if (p.spill_ds) tma_store_wait_read<0>();   // single dS buffer: read out before it is rewritten
+          if (t + 1 < n_iter) ok = issue_scores();
+        }
+      }
+      if (ok) umma_commit(done);
+      if (p.spill_ds) tma_store_wait<0>();   // the stores are complete before the CTA retires
+    }
+  } else {
+    const int sw = warp - 2;        // 0..7
+    const int q = warp & 3;         // TMEM lane quarter
+    const int half = sw >> 2;       // which 64 kv columns of the tile this warp handles
+    const int r = q * 32 + lane;    // row inside the tile == TMEM lane (query row in the loop, kv row at the end)
+    const int kv_idx = kv0 + r;
+    const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
+    const float delta_scale = p.scale;
+    bool ok = true;
+    for (int t = 0; t < n_iter; ++t) {
+      const int head = kvh * group + t / n_qt;
+      const int qt = qt_first + t % n_qt;
+      const int q0 = qt * BT;
+      const int q_idx = q0 + r;
+      const float2 sd = __ldg(p.stats + (static_cast<size_t>(b) * p.H + head) * p.S + min(q_idx, p.S - 1));
+      const int pb = Cfg::PDB ? (t & 1) : 0;
+      uint8_t* pt_buf = sPT + pb * Cfg::PT_BYTES;
+      uint8_t* dst_buf = sdST + pb * Cfg::PT_BYTES;
+      // last visible kv column of this query row inside the tile (-1: row is past the sequence end)
+      const bool diag = p.causal && qt == kt;
+      int lim = min(diag ? r : BT - 1, p.S - 1 - kv0);
+      if (q_idx >= p.S) lim = -1;
+      const bool need_mask = diag || (q0 + BT > p.S) || (kv0 + BT > p.S);
+      if (!mbar_wait(st_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      tc_fence_after();
+      if (need_mask) {
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc)
+          bwd_chunk<true, true>(tm_ST, tm_dPT, lane_off, half * 2 + cc, r, lim, p.scale_log2, sd.x,
+                                sd.y * delta_scale, p.scale, pt_buf, dst_buf);
+      } else {
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc)
+          bwd_chunk<false, true>(tm_ST, tm_dPT, lane_off, half * 2 + cc, r, lim, p.scale_log2, sd.x,
+                                 sd.y * delta_scale, p.scale, pt_buf, dst_buf);
+      }
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+    }
+    if (ok && mbar_wait(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
+      tc_fence_after();
+      constexpr int CPW = DH / 64;  // 32-column chunks per warp and matrix
+#pragma unroll 1
+      for (int which = 0; which < 2; ++which) {
+        const uint32_t src = which == 0 ? tm_dK : tm_dV;
+        const int col0 = (which == 0 ? (p.H + kvh) : (p.H + p.Hkv + kvh)) * DH;
+#pragma unroll 1
+        for (int cc = 0; cc < CPW; ++cc) {
+          const int c = half * CPW + cc;
+          uint32_t v[32];
+          tmem_ld_32x32(src + lane_off + c * 32, v);
+          tmem_ld_wait();
+          if (kv_idx < p.S) {
+            __nv_bfloat16* dst = p.dqkv + static_cast<size_t>(row_base + kv_idx) * p.ld_dqkv + col0 + c * 32;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              uint4 w;
+              w.x = pack_bf16x2(__uint_as_float(v[u * 8 + 0]), __uint_as_float(v[u * 8 + 1]));
+              w.y = pack_bf16x2(__uint_as_float(v[u * 8 + 2]), __uint_as_float(v[u * 8 + 3]));
+              w.z = pack_bf16x2(__uint_as_float(v[u * 8 + 4]), __uint_as_float(v[u * 8 + 5]));
+              w.w = pack_bf16x2(__uint_as_float(v[u * 8 + 6]), __uint_as_float(v[u * 8 + 7]));
+              *reinterpret_cast<uint4*>(dst + u * 8) = w;
+            }
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+}
+
+// Pipeline at head dimension 128: scores and dP have barriers of their own, so the exponentials of iteration t+1 (which need the scores only)
 // run under the gradient products of iteration t, and dS follows when dP arrives. Order of the tensor work:
 //   S(t+1) | dV(t) += P(t)^T dO(t) | dK(t) += dS(t)^T Q(t) | dP(t+1)
 // S(t+1) needs Q(t+1), so Q has two stages; dO(t) is free after dV(t), two products before dP(t+1) needs its successor,
@@ -126,9 +375,10 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 // P is single: dV(t) has read it (dv_done) long before the exponentials of t+1 are stored. Until then the two score
 // products of an iteration were one group, which the softmax warps waited for as a whole, and at 128 the loads,
 // the scores, the softmax and the gradient products of an iteration ran one after another: 2 x 2048 tokens of 32 heads,
-// causal, 241 us then and 176 us so (head dimension 64, 8 x 2048 tokens of 16 heads: 301 and 303 us).
+// causal, 241 us then and 176 us so. At 64 the kernel above stays: its scores of t+1 and dP are one group ahead of the gradient
+// products, and forward and backward of 2 x 700 tokens of 16 heads take 85.8 us with it, 86.9 with this one.
 template <int DH>
-struct DkvCfg {
+struct DkvSplitCfg {
   static constexpr int QS = 2;                        // Q stages
   static constexpr int OS = (DH == 64) ? 2 : 1;       // dO stages
   static constexpr int NDS = (DH == 64) ? 2 : 1;      // dS buffers (a bulk store may still read the older one)
@@ -142,9 +392,9 @@ struct DkvCfg {
 
 template <int DH>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
-attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
+attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                          const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
-  using Cfg = DkvCfg<DH>;
+  using Cfg = DkvSplitCfg<DH>;
   constexpr int NCH = DH / 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -749,12 +999,14 @@ attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
 template <int DH>
 static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& td, const CUtensorMap& tds, const BwdParams& p,
                       cudaStream_t stream) {
-  auto k1 = attention_bwd_dkv_kernel<DH>;
+  constexpr int DKV_SMEM = DH == 64 ? DkvCfg<64>::SMEM_BYTES : DkvSplitCfg<128>::SMEM_BYTES;
+  void (*k1)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const BwdParams);
+  if constexpr (DH == 64) k1 = attention_bwd_dkv_kernel<64>; else k1 = attention_bwd_dkv_split_kernel<128>;
   auto k2 = attention_bwd_dq_kernel<DH>;
   auto k3 = attention_bwd_dq_stream_kernel<DH>;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvCfg<DH>::SMEM_BYTES) !=
+    if (cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, DKV_SMEM) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<DH>::SMEM_BYTES) != cudaSuccess ||
         cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, DqsCfg<DH>::SMEM_BYTES) != cudaSuccess)
@@ -762,7 +1014,7 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& td, const CUtens
     attr_set = true;
   }
   const int n_t = (p.S + BT - 1) / BT;
-  k1<<<dim3(p.Hkv, p.B, n_t), BWD_THREADS, DkvCfg<DH>::SMEM_BYTES, stream>>>(tq, td, tds, p);
+  k1<<<dim3(p.Hkv, p.B, n_t), BWD_THREADS, DKV_SMEM, stream>>>(tq, td, tds, p);
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   if (p.spill_ds) k3<<<dim3(p.H, p.B, n_t), BWD_THREADS, DqsCfg<DH>::SMEM_BYTES, stream>>>(tq, tds, p);
   else k2<<<dim3(p.H, p.B, n_t), BWD_THREADS, DqCfg<DH>::SMEM_BYTES, stream>>>(tq, td, p);
