@@ -653,6 +653,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
               *reinterpret_cast<uint4*>(dst + u * 8) = w;
             }
           }
+          __syncwarp();   // rows past the end have skipped the stores; the next tensor-memory load needs the whole warp
         }
       }
     }

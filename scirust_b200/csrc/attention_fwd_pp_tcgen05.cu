@@ -390,16 +390,18 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
 #pragma unroll
         for (int c = 0; c < 2; ++c) tmem_ld_32x32(tm_O + c0 + c * 32, o + c * 32);
         tmem_ld_wait();
-        if (q_idx >= p.S) continue;
+        if (q_idx < p.S) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint4 w;
-          w.x = pack_bf16x2(__uint_as_float(o[c * 8 + 0]) * inv_l, __uint_as_float(o[c * 8 + 1]) * inv_l);
-          w.y = pack_bf16x2(__uint_as_float(o[c * 8 + 2]) * inv_l, __uint_as_float(o[c * 8 + 3]) * inv_l);
-          w.z = pack_bf16x2(__uint_as_float(o[c * 8 + 4]) * inv_l, __uint_as_float(o[c * 8 + 5]) * inv_l);
-          w.w = pack_bf16x2(__uint_as_float(o[c * 8 + 6]) * inv_l, __uint_as_float(o[c * 8 + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(orow + c0 + c * 8) = w;
+          for (int c = 0; c < 8; ++c) {
+            uint4 w;
+            w.x = pack_bf16x2(__uint_as_float(o[c * 8 + 0]) * inv_l, __uint_as_float(o[c * 8 + 1]) * inv_l);
+            w.y = pack_bf16x2(__uint_as_float(o[c * 8 + 2]) * inv_l, __uint_as_float(o[c * 8 + 3]) * inv_l);
+            w.z = pack_bf16x2(__uint_as_float(o[c * 8 + 4]) * inv_l, __uint_as_float(o[c * 8 + 5]) * inv_l);
+            w.w = pack_bf16x2(__uint_as_float(o[c * 8 + 6]) * inv_l, __uint_as_float(o[c * 8 + 7]) * inv_l);
+            *reinterpret_cast<uint4*>(orow + c0 + c * 8) = w;
+          }
         }
+        __syncwarp();   // rows past the end have skipped the stores; the next tensor-memory load needs the whole warp
       }
       if (q_idx < p.S) {
         if (p.lse) p.lse[(static_cast<size_t>(b) * p.H + head) * p.S + q_idx] = m_ref * 0.6931471805599453f + logf(l);
