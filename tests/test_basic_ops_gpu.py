@@ -191,6 +191,49 @@ def test_cross_entropy_row_kept_in_registers(cols):
     loss2, d2 = ops.ce_fwd_bwd(inp, tg, 0.25)
     assert d2.data_ptr() == inp.data_ptr()
     assert torch.equal(loss, loss2) and torch.equal(d, d2) and torch.equal(loss, loss_only)
-    want_loss, want = ops.ce_fwd_bwd(lg.cpu(), tg.cpu(), 0.25, in_place=False)
-    assert (loss.cpu() - want_loss).abs().max().item() <= 2e-5 * max(1.0, want_loss.abs().max().item())
-    assert (d.cpu().float() - want.float()).abs().max().item() <= 0.25 * 2 ** -8
+    _check_cross_entropy(lg, tg, 0.25, loss, d)
+
+
+def _check_cross_entropy(lg, tg, scale, loss, d):
+    """Against the float64 statement. The loss: exponentials to 2^-21, sums of positive terms and a difference rounded to
+    fp32, 1e-5 in all. The gradient is rounded to bf16 (2^-9) after a probability good to 1e-5 (2^-8 covers both; the
+    target's entry p - 1 carries p's absolute error; results below 1e-36 may be flushed), so a row's sum is zero to 2^-9 of
+    the sum of magnitudes, 2 * scale."""
+    x, cols = lg.double(), lg.shape[1]
+    ignored = tg < 0
+    at = tg.clamp(0, cols - 1)[:, None]
+    p = torch.softmax(x, -1)
+    # the target's loss relative to the maximum: the difference of two large logits is exact, their logsumexp is not
+    m = x.max(-1, keepdim=True).values
+    want_loss = (torch.exp(x - m).sum(-1).log() - (x.gather(1, at) - m)[:, 0]).masked_fill(ignored, 0.0)
+    want = p.scatter_add(1, at, -torch.ones_like(at, dtype=torch.float64)) * scale
+    want[ignored] = 0.0
+    lim = 2 ** -8 * want.abs() + 1e-36
+    lim.scatter_add_(1, at, torch.full_like(at, 1e-5 * scale, dtype=torch.float64))
+    assert ((loss.double() - want_loss).abs() <= 1e-5 * want_loss.abs().clamp(min=1.0)).all()
+    assert ((d.double() - want).abs() <= lim).all()
+    assert (d.double().sum(-1).abs() <= 2 ** -8 * 2 * scale).all()
+    assert (d[ignored] == 0).all()
+
+
+@pytest.mark.parametrize("cols", [8, 4096, 32768, 32776])
+def test_cross_entropy_of_large_logits(cols):
+    """Rows far from zero, down to the type's lowest value, on both sides of the 32768-column line: the result depends on
+    the distances from the row's maximum, whatever the offset. Each row holds its offset and values up to three bf16 steps
+    below it. Ignored rows give zeros, also where the logits are not numbers."""
+    offsets = [0.0, 1e3, -1e3, 1e5, -1e7, 1e9, -1e30, 2.5e38, -3.0e38, torch.finfo(torch.bfloat16).min]
+    g = torch.Generator().manual_seed(cols)
+    base = torch.tensor(offsets).to(torch.bfloat16)[:, None].expand(-1, cols)
+    steps = torch.randint(0, 4, base.shape, generator=g) * (base[:, :1].float().abs() * 2 ** -8).clamp(min=1.0)
+    lg = (base.float() - steps).clamp(min=torch.finfo(torch.bfloat16).min).to(torch.bfloat16)
+    lg[:, 3] = base[:, 3]
+    lg = torch.cat((lg, lg, torch.full((2, cols), float("nan"), dtype=torch.bfloat16))).cuda()
+    lg[-1] = float("-inf")
+    n = len(offsets)
+    tg = torch.randint(0, cols, (2 * n + 2,), generator=g)
+    tg[:n:2], tg[n:] = 3, -1
+    tg = tg.cuda()
+    loss, d = ops.ce_fwd_bwd(lg.clone(), tg, 0.25, in_place=False)
+    assert (loss[n:] == 0).all() and (d[n:] == 0).all()
+    _check_cross_entropy(lg[:n], tg[:n], 0.25, loss[:n], d[:n])
+    assert torch.equal(loss, ops.ce_loss_only(lg, tg))
