@@ -20,10 +20,9 @@ CASES = [(1, 128, 1, 1, 64), (2, 256, 4, 2, 64), (1, 1000, 4, 1, 64), (2, 2048, 
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("two_tiles", [True, False])
 def test_forward(B, S, H, Hkv, dh, causal, two_tiles, monkeypatch):
-    # two_tiles: the head-dimension-64 kernel with two query tiles per CTA; otherwise the one-tile kernel
-    if dh != 64 and two_tiles:
-        pytest.skip("the two-tile kernel covers head dimension 64")
+    # two_tiles: the kernel with two query tiles per CTA, also where the rule on sizes would not choose it
     monkeypatch.setattr(A, "FWD_TWO_TILES", two_tiles)
+    monkeypatch.setattr(A, "_two_tiles_win", lambda *a: True)
     qkv = _qkv(B, S, H, Hkv, dh)
     o, lse = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal)
     _lib.check_status()
@@ -39,6 +38,7 @@ def test_forward_growing_maxima(causal, monkeypatch):
     # keys grow along the sequence, so row maxima rise by more than 2^8 from block to block and the
     # output accumulator in tensor memory is rescaled many times
     monkeypatch.setattr(A, "FWD_TWO_TILES", True)
+    monkeypatch.setattr(A, "_two_tiles_win", lambda *a: True)
     B, S, H, Hkv, dh = 2, 1024, 4, 2, 64
     qkv = _qkv(B, S, H, Hkv, dh, seed=5).float().reshape(B, S, H + 2 * Hkv, dh)
     ramp = (1.0 + 6.0 * torch.arange(S, device="cuda") / S).reshape(1, S, 1, 1)
@@ -112,3 +112,27 @@ def test_backward_pipeline_edges(B, S, H, Hkv, dh, causal):
     _lib.check_status()
     ref = A.attention_bwd_ref(qkv, do, B, S, H, Hkv, dh, causal=causal)
     assert (d.float() - ref).abs().max().item() < 3e-2 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("causal,scale", [(True, 1.0), (True, 2.0), (False, 3.0)])
+def test_two_tiles_at_128_are_as_exact_as_one(causal, scale, monkeypatch):
+    """Against float64, on scores of growing spread: the two-tile kernel refers P to the running maximum, as the one-tile
+    kernel does, so the largest weight of a row is exactly 1 in bf16 in both. What is left between them is the order of
+    the fp32 sums, far below the 2^-9 of P and of the output: a thousandth of the error, where a reference that lags the
+    maximum costs 2 % (unit scores) to 20 %."""
+    B, S, H, Hkv, dh = 1, 1500, 4, 1, 128
+    qkv = _qkv(B, S, H, Hkv, dh, seed=21).float()
+    qkv[:, :(H + Hkv) * dh] *= scale
+    qkv = qkv.to(torch.bfloat16)
+    x = qkv.double().reshape(S, H + 2 * Hkv, dh)
+    sc = torch.einsum("qhd,kd->hqk", x[:, :H], x[:, H]) / dh ** 0.5
+    if causal:
+        sc = sc.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref = torch.einsum("hqk,kd->qhd", torch.softmax(sc, -1), x[:, H + Hkv]).reshape(S, H * dh)
+    err = []
+    for two in (False, True):
+        monkeypatch.setattr(A, "_two_tiles_win", lambda *a: two)
+        o, _ = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal)
+        err.append(((o.double() - ref).norm() / ref.norm()).item())
+    _lib.check_status()
+    assert err[1] <= err[0] * 1.001, err
