@@ -27,13 +27,28 @@ _lib.register("sb_attention_bwd", [_lib.vp, _lib.vp, _lib.vp, _lib.vp, _lib.vp, 
 FWD_TWO_TILES = os.environ.get("SB_ATT_FWD", "pair") != "single"
 
 
-def _two_tiles_win(B, S, H, device) -> bool:
-    """Where the two-tile kernel is the faster one: when its CTAs outnumber the SMs. Below that every CTA runs by itself, and
-    an iteration over one kv block for one tile (2.4 us at head dimension 128) beats one for two (3.0 us). Measured, one
-    tile against two, us: dh 128, 32 heads 1 x 512 13.8 / 16.3, 1 x 1024 (128 CTAs) 26.6 / 27.2, 1 x 1500 (192) 51.9 / 36.7,
-    3 x 2048 238 / 153; dh 64, 16 heads 1 x 512 11.4 / 13.9, 2 x 512 11.6 / 14.0, 3 x 1000 (192) 24.8 / 23.9,
-    1 x 4096 88.6 / 70.8."""
-    return B * H * ((S + 255) // 256) > _g.num_sms(device)
+def _two_tiles_win(B, S, H, dh, causal, device) -> bool:
+    """Where the two-tile kernel is the faster one, by the CTAs that each of the two starts.
+
+    Head dimension 128 (one CTA per SM in both): a CTA of two tiles takes about 1.7 times as long as one of a single
+    tile, so while its grid fits the GPU at once one tile wins, and beyond that it must save waves: sequences of up to
+    256 rows need more than 1.5 times fewer, up to 384 (the second CTA of a head has one tile) 1.5 times, longer ones
+    always do. Causal, 32 heads, us, one tile against two: 1 x 1000 (128 CTAs) 26.3 / 27.7, 1 x 1300 (192) 45.3 / 35.0,
+    2 x 1000 51.4 / 39.5, 9 x 256 29.5 / 25.6, but 6 x 256 21.6 / 24.3, 3 x 333 17.9 / 22.4, 5 x 333 30.9 / 33.2.
+
+    Head dimension 64 (two CTAs per SM with one tile, one with two), 16 heads: while the two-tile grid fits the GPU at
+    once one tile is faster for causal sequences, but past 512 rows for an even number of tiles only (the longest tile
+    of an odd number runs alone in its CTA): 1 x 512 11.5 / 13.6, 2 x 1000 21.1 / 21.6, but 3 x 600 14.8 / 14.3; without
+    the mask up to 384 rows only: 3 x 333 9.9 / 11.9, but 2 x 1000 24.4 / 22.0."""
+    sms, tiles = _g.num_sms(device), (S + 127) // 128
+    one, two = B * H * tiles, B * H * ((S + 255) // 256)
+    if dh == 64:
+        fewer = (S <= 512 or tiles % 2 == 0) if causal else S <= 384
+        return two > sms or not fewer
+    if two <= sms or S <= 128:
+        return False
+    one, two = -(-one // sms), -(-two // sms)          # waves
+    return S > 384 or (2 * one >= 3 * two if S > 256 else 2 * one > 3 * two)
 
 
 # The backward pass spills its dS tiles (bf16 [B*H, S, S]) to a scratch buffer so that dQ is a streamed
@@ -79,7 +94,7 @@ def attention_fwd(qkv, B, S, H, Hkv, dh, causal=True, scale=None, want_lse=True)
         raise ValueError("qkv must be a 2-D bf16 matrix with unit inner stride")
     out = _lib.empty((B * S, H * dh), torch.bfloat16, qkv.device)
     lse = _lib.empty((B, H, S), torch.float32, qkv.device) if want_lse else None
-    entry = "sb_attention_fwd_pp" if FWD_TWO_TILES and _two_tiles_win(B, S, H, qkv.device) else "sb_attention_fwd"
+    entry = "sb_attention_fwd_pp" if FWD_TWO_TILES and _two_tiles_win(B, S, H, dh, causal, qkv.device) else "sb_attention_fwd"
     _lib.call(entry, qkv.data_ptr(), out.data_ptr(), _lib.ptr(lse), B, S, H, Hkv, dh, qkv.stride(0),
               out.stride(0), float(scale), int(causal), _lib.status_word(qkv.device).data_ptr(), _lib.stream())
     _g.launch_count += 1
