@@ -224,7 +224,7 @@ class InferenceEngine:
             logits.copy_(ops.matmul_nn(hn, self.head_t).float())
 
     # ------------------------------------------------------------------ decode
-    def _decode_body(self, B: int, max_len: int, greedy: bool = False):
+    def _decode_body(self, B: int, max_len: int, greedy: bool = False, stream: bool | None = None):
         cfg, cache = self.cfg, self.cache
         H, Hkv, dh = self.H, self.Hkv, cfg.head_dim
         seq_of = self._seq_of[:B]
@@ -241,7 +241,7 @@ class InferenceEngine:
             D.rope_kv_append(qkv, H, Hkv, dh, self.cos, self.sin, cache.pools[li], cache.block_table, cache.page,
                              seq_of, pos)
             a = D.decode_attention(qkv, cache.pools[li], cache.block_table, cache.page, self._len_plus1[:B], H, Hkv,
-                                   dh, max_len=max_len)
+                                   dh, max_len=max_len, stream=stream)
             x = self._proj_out(a, l["wo"], x, site="attn")
             if small:
                 gu = D.gemv(x, l["wgu"], rms_weight=l["rms2"], eps=cfg.eps)
@@ -263,10 +263,10 @@ class InferenceEngine:
         D.gemv_argmax(x, self.head_t, out_tokens=self.tokens[:B], rms_weight=self.rms_final, eps=self.cfg.eps,
                       logits=logits, generated=self._generated, step=0)
 
-    def _step_eager(self, B, max_len, sampler=None, want_logits=False):
+    def _step_eager(self, B, max_len, sampler=None, want_logits=False, stream=None):
         torch.add(self.cache.seq_len[:B], 1, out=self._len_plus1[:B])
         with D.dependent_launch(self.dev.type == "cuda"):
-            done = self._decode_body(B, max_len, greedy=sampler is None and not want_logits)
+            done = self._decode_body(B, max_len, greedy=sampler is None and not want_logits, stream=stream)
         if done:
             pass
         elif sampler is None:
@@ -275,6 +275,17 @@ class InferenceEngine:
             sampler.sample(self.logits[:B], out_tokens=self.tokens[:B])
             sampler.push(self.tokens[:B])
         self.cache.seq_len[:B] += 1
+
+    def _streams(self, B: int, held: int) -> bool:
+        """Which of the two decode-attention kernels suits ``B`` sequences of ``held`` positions (the cap that they may grow
+        to does not count: the first part of a long generation is short)."""
+        return (self.dev.type == "cuda"
+                and D._stream_wins(held, B * self.Hkv, self.H // self.Hkv, self.cache.page, self.dev))
+
+    # A generation that crosses the line between the two kernels captures its step anew (two or three milliseconds for eight
+    # layers), unless it ends within this many steps. 64 prompts of 128 tokens, 1800 new ones, eight layers of 4096: 2755 ms
+    # so, 2903 with the split kernel to the end.
+    RECAPTURE_STEPS = 64
 
     def generate(self, prompts: torch.Tensor, max_new: int, params: SamplingParams | None = None, seed: int = 0,
                  stop_on_zero: bool = False):
@@ -310,25 +321,47 @@ class InferenceEngine:
             sampler.push(self.tokens[:B])
         out[:, 0] = self.tokens[:B]
         max_len = P + max_new
+        stream = self._streams(B, P + 1)
+
+        def crosses(i):
+            return max_new - i >= self.RECAPTURE_STEPS and self._streams(B, P + i) != stream
+
         if self.use_graph and max_new > 2:
             # one eager step on the capture stream warms every workspace (they are kept per stream, and nothing may be
             # allocated or cleared inside the capture), then the step is captured once and replayed
-            g = torch.cuda.CUDAGraph()
             s = torch.cuda.Stream(device=self.dev)
-            s.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(s):
-                self._step_eager(B, max_len, sampler)
-                out[:, 1] = self.tokens[:B]
-                with torch.cuda.graph(g, stream=s):
-                    self._step_eager(B, max_len, sampler)
-            torch.cuda.current_stream().wait_stream(s)
+            graphs = []                        # an earlier one may still be running when the next is captured
+
+            def capture(i):
+                g = torch.cuda.CUDAGraph()
+                s.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(s):
+                    self._step_eager(B, max_len, sampler, stream=stream)
+                    out[:, i] = self.tokens[:B]
+                    if graphs:                 # in the middle of a generation, without torch.cuda.graph's collection and cache flush
+                        g.capture_begin()
+                        self._step_eager(B, max_len, sampler, stream=stream)
+                        g.capture_end()
+                    else:
+                        with torch.cuda.graph(g, stream=s):
+                            self._step_eager(B, max_len, sampler, stream=stream)
+                graphs.append(g)
+                torch.cuda.current_stream().wait_stream(s)
+
+            capture(1)
             # capture only records; run the recorded step for positions 2 .. max_new-1
             for i in range(2, max_new):
-                g.replay()
+                if crosses(i):
+                    stream = not stream
+                    capture(i)
+                    continue
+                graphs[-1].replay()
                 out[:, i] = self.tokens[:B]
         else:
             for i in range(1, max_new):
-                self._step_eager(B, max_len, sampler)
+                if crosses(i):
+                    stream = not stream
+                self._step_eager(B, max_len, sampler, stream=stream)
                 out[:, i] = self.tokens[:B]
         _lib.check_status(self.dev) if self.dev.type == "cuda" else None
         return out
@@ -354,7 +387,7 @@ def teacher_forced_logits(engine: "InferenceEngine", prompts: torch.Tensor, toke
     tok = tokens.to(engine.dev)
     for i in range(n):
         engine.tokens[:B] = tok[:, i]
-        engine._step_eager(B, P + n + 1, want_logits=True)
+        engine._step_eager(B, P + n + 1, want_logits=True, stream=engine._streams(B, P + i + 1))
         out.append(engine.logits[:B].float().clone())
     return torch.stack(out, 1)
 

@@ -473,14 +473,25 @@ def decode_attention_ref(q, pool, block_table, page, seq_len, H, Hkv, dh, scale=
     return out
 
 
-def _stream_wins(L, tiles, device) -> bool:
-    """Where the balanced stream beats the split kernel, by the 64-position tiles per SM of the batch. Measured at 32 / 8
-    heads (us, split against stream): 1 x 2048 15.2 / 10.7, 1 x 8192 44.2 / 18.8, 4 x 2048 21.8 / 17.8, 16 x 512 20.9 / 18.1,
-    16 x 2304 41.6 / 33.9, 64 x 2048 103.2 / 87.6; but 4 x 1024 14.3 / 16.0, 16 x 256 12.6 / 16.0, 64 x 128 14.5 / 22.5: its
-    start and the merge of many short pieces need six tiles per SM, or long sequences (where the split kernel's 64 splits
-    and its last wave bind), to pay."""
-    per_sm = tiles / _g.num_sms(device)
-    return L >= 256 and per_sm >= (1.5 if L >= 2048 else 6.0)
+def _stream_wins(L, jobs, G, page, device) -> bool:
+    """Where the balanced stream beats the split kernel, for ``jobs`` (sequence, kv head) pairs that hold about ``L`` positions,
+    ``G`` query heads per kv head. us, split against stream.
+
+    Four query heads and more, pages of 64 and more (32 / 8 heads): 1 x 2048 14.1 / 10.1, 1 x 8192 43.8 / 16.7, 4 x 2048
+    22.4 / 16.5, 16 x 512 18.9 / 16.6, 16 x 2304 40.2 / 32.3, 64 x 256 31.3 / 29.5, 64 x 2048 107.0 / 88.6; but 4 x 1024
+    13.3 / 14.3, 16 x 256 11.9 / 14.2, 64 x 128 13.0 / 21.0: its start and the merge of many short pieces need six tiles of
+    64 positions per SM, or long sequences (where the split kernel's 64 splits and its last wave bind), to pay.
+    Smaller pages make smaller copies, one thread issues them: 32 positions win by less (64 x 2048 105.7 / 106.6), 16 only
+    while a batch is small (1 x 8192 43.5 / 20.0, 4 x 2048 23.7 / 22.3; 16 x 2304 41.5 / 49.8), 8 lose (64 x 2048 110 / 250).
+    With fewer query heads per kv head the split kernel is bound by memory sooner and the merge weighs more: two and three want
+    512 positions (16 / 8 heads, 32 x 256 17.1 / 17.7, 16 x 512 16.4 / 15.5), one long sequences and few jobs (32 / 32 heads
+    16 x 2304 105.5 / 89.6, 4 x 512 14.5 / 15.2, 64 x 1024 156.9 / 166.4)."""
+    per_sm = jobs * max(1, (L + 63) // 64) / _g.num_sms(device)
+    if G < 4:
+        return page >= 64 and per_sm >= 6.0 and (L >= 512 if G > 1 else L >= 2048 and jobs <= 512)
+    if page < 32:
+        return page == 16 and L >= 2048 and 1.5 <= per_sm <= 7.0
+    return L >= 256 and per_sm >= (1.5 if L >= 2048 else 6.0) and (page >= 64 or per_sm <= 60.0)
 
 
 def _stream_ok(pool, page, B, H, Hkv, dh) -> bool:
@@ -491,16 +502,21 @@ def _stream_ok(pool, page, B, H, Hkv, dh) -> bool:
             and pool.shape[0] * 2 * Hkv * page < 1 << 31)
 
 
-def decode_attention(q, pool, block_table, page, seq_len, H, Hkv, dh, scale=None, n_splits=None, max_len=None):
-    """Single-query GQA attention of each sequence over its paged KV. q: [B, >= H*dh] (RoPE'd)."""
+def decode_attention(q, pool, block_table, page, seq_len, H, Hkv, dh, scale=None, n_splits=None, max_len=None, stream=None):
+    """Single-query GQA attention of each sequence over its paged KV. q: [B, >= H*dh] (RoPE'd). ``max_len`` bounds the
+    lengths. The lengths themselves are on the device, so which kernel runs is the caller's knowledge: ``stream`` says it
+    (``_stream_wins`` of what the cache holds; a captured step keeps the choice), by default ``max_len`` is taken for what the
+    cache holds, and without either the split kernel runs. An explicit ``n_splits`` means the split kernel too."""
     scale = 1.0 / math.sqrt(dh) if scale is None else scale
     B = q.shape[0]
     if not q.is_cuda:
         return decode_attention_ref(q, pool, block_table, page, seq_len, H, Hkv, dh, scale).to(BF)
     L = max_len if max_len is not None else block_table.shape[1] * page
     tiles = B * Hkv * max(1, (L + 63) // 64)
-    if n_splits is None and _stream_wins(L, tiles, q.device) and _stream_ok(pool, page, B, H, Hkv, dh):
-        # the tiles of the whole batch dealt out evenly over the SMs; an explicit split count keeps the kernel below
+    if stream is None:
+        stream = max_len is not None and _stream_wins(L, B * Hkv, H // Hkv, page, q.device)
+    if n_splits is None and stream and _stream_ok(pool, page, B, H, Hkv, dh):
+        # the tiles of the whole batch dealt out evenly over the SMs
         part = _workspace(2 * _g.num_sms(q.device) * 16 * (dh + 2), q.device)
         ctr = _gemv_workspace(4096, q.device)
         out = _lib.empty((B, H * dh), BF, q.device)

@@ -2,7 +2,7 @@
 sides were timed, with the side that was faster (or, within 2 %, the one that was there first)."""
 import pytest
 
-from scirust_b200.ops import attention as A, gemm as G
+from scirust_b200.ops import attention as A, decode as D, gemm as G
 
 
 @pytest.fixture(autouse=True)
@@ -24,3 +24,19 @@ def _sms(monkeypatch):
 ])
 def test_attention_forward_tiles(B, S, H, dh, causal, two):
     assert A._two_tiles_win(B, S, H, dh, causal, None) is two
+
+
+@pytest.mark.parametrize("B,L,H,Hkv,page,stream", [
+    (1, 2048, 32, 8, 64, True), (4, 2048, 32, 8, 128, True), (16, 512, 32, 8, 64, True), (64, 256, 32, 8, 64, True),
+    (64, 2048, 32, 8, 64, True), (16, 2304, 32, 2, 64, True), (1, 8192, 16, 2, 64, True),
+    (1, 1024, 32, 8, 64, False), (4, 1024, 32, 8, 64, False), (16, 256, 32, 8, 64, False), (64, 128, 32, 8, 64, False),
+    # small pages: one thread issues a copy per page
+    (16, 2304, 32, 8, 32, True), (64, 2048, 32, 8, 32, False), (1, 8192, 32, 8, 16, True), (4, 2048, 32, 8, 16, True),
+    (16, 512, 32, 8, 16, False), (64, 2048, 32, 8, 16, False), (1, 2048, 32, 8, 8, False), (64, 2048, 32, 8, 8, False),
+    # few query heads per kv head
+    (1, 2048, 8, 8, 64, False), (1, 4096, 8, 8, 64, False), (1, 8192, 8, 8, 64, True), (64, 512, 8, 8, 64, False),
+    (64, 2048, 8, 8, 64, True), (32, 256, 32, 32, 64, False), (64, 1024, 32, 32, 64, False), (16, 2304, 32, 32, 64, True),
+    (2, 2048, 16, 8, 64, False), (16, 512, 16, 8, 64, True), (32, 256, 16, 8, 64, False), (16, 1024, 24, 8, 32, False),
+])
+def test_streamed_decode_attention(B, L, H, Hkv, page, stream):
+    assert D._stream_wins(L, B * Hkv, H // Hkv, page, None) is stream

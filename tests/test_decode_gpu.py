@@ -282,3 +282,32 @@ def test_decode_attention_stream_repeats_under_load(monkeypatch):
     assert torch.equal(first, last)
     from scirust_b200.ops import _lib
     _lib.check_status(torch.device("cuda"))
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_generation_chooses_attention_by_what_the_cache_holds(graph, monkeypatch):
+    """The engine asks for the streamed kernel once the sequences are long enough, whatever they may grow to: a generation
+    that crosses the line runs the split kernel before it and the stream after it, replayed or not, and one that ends soon
+    after the line keeps its kernel."""
+    torch.manual_seed(0)
+    model = GQADecoder(SciAgentConfig(512, 512, 2, 4, 1, 512, 256, 1e4), device="cuda")
+    prompts = torch.randint(0, 512, (3, 20), generator=torch.Generator().manual_seed(1))
+    monkeypatch.setattr(D, "_stream_wins", lambda L, *a: L >= 30)
+    asked = []
+    real = D.decode_attention
+    monkeypatch.setattr(D, "decode_attention", lambda *a, **k: (asked.append(k["stream"]), real(*a, **k))[1])
+    out = {}
+    for recapture in (8, 100):
+        eng = InferenceEngine(model, max_batch=3, max_seq=128, page=64, use_graph=graph)
+        eng.RECAPTURE_STEPS = recapture
+        asked.clear()
+        out[recapture] = eng.generate(prompts, 40).cpu()
+        # two layers a step; a graph runs each kernel eagerly once and records it once
+        per = {False: 4, True: 4} if graph else {False: 9 * 2, True: 30 * 2}
+        want = per if recapture == 8 else {False: 4 if graph else 39 * 2, True: 0}
+        assert {r: asked.count(r) for r in (False, True)} == want
+    a = InferenceEngine(model, max_batch=3, max_seq=128, page=64, use_graph=not graph)
+    a.RECAPTURE_STEPS = 8
+    assert torch.equal(a.generate(prompts, 40).cpu(), out[8])
+    assert (out[8] == out[100]).float().mean().item() > 0.5      # the kernels differ by roundings, which may flip a near-tie
+
