@@ -1845,11 +1845,9 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
               }
             }
           }
-          const float lt = w_l[g], inv = lt > 0.f ? 1.f : 0.f;
-          const float dn = lt > 0.f ? lt : 1.f;
-          uint2 pk;
-          pk.x = dpack(ot.x / dn * inv, ot.y / dn * inv);
-          pk.y = dpack(ot.z / dn * inv, ot.w / dn * inv);
+          const float lt = w_l[g];
+          uint2 pk = make_uint2(0u, 0u);             // no weight: zeros, whatever the values held
+          if (lt > 0.f) pk = make_uint2(dpack(ot.x / lt, ot.y / lt), dpack(ot.z / lt, ot.w / lt));
           __nv_bfloat16* dst = p.out + static_cast<size_t>(b) * p.ldo + (kvh * G + g) * DH + d;
           if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) *reinterpret_cast<uint2*>(dst) = pk;
           else {

@@ -311,3 +311,20 @@ def test_generation_chooses_attention_by_what_the_cache_holds(graph, monkeypatch
     assert torch.equal(a.generate(prompts, 40).cpu(), out[8])
     assert (out[8] == out[100]).float().mean().item() > 0.5      # the kernels differ by roundings, which may flip a near-tie
 
+
+def test_decode_attention_stream_without_weight_is_zero():
+    """A sequence whose scores are all NaN has no weight: zeros, as from the split kernel, also where its values are NaN
+    and its tiles are spread over many CTAs."""
+    H, Hkv, dh, page = 8, 2, 128, 64
+    lens = [1500, 40, 300]
+    nb = (max(lens) + page - 1) // page
+    pool = _r((3 * nb, 2, Hkv, page, dh), 1)
+    table = torch.arange(3 * nb, dtype=torch.int32, device="cuda").reshape(3, nb)
+    pool[table[0].long()] = float("nan")
+    pool[table[1].long()] = float("nan")
+    ln = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q = _r((3, (H + 2 * Hkv) * dh), 2)
+    out = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, stream=True)
+    one = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, stream=False)
+    assert (one[:2] == 0).all() and (out[:2] == 0).all()
+    assert (out[2].float() - one[2].float()).abs().max().item() < 2e-2
