@@ -245,21 +245,23 @@ __global__ void quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int ld
   }
 }
 
-// The same quantiser, one CTA per row, eight elements (16 bytes) per thread and step: the row is read once from
-// memory (rows up to 16384 stay in registers, all loads in flight; 16 rows of 4096: 3.6 -> 3.0 us), the maximum is combined
-// through shared memory.
-constexpr int QR_THREADS = 512, QR_KEEP = 4;
-__global__ void __launch_bounds__(QR_THREADS)
+// The same quantiser, one CTA per row, eight elements (16 bytes) per thread and step: the row is read once from memory,
+// the maximum is combined through shared memory. KEEP words a thread stay in registers, all loads in flight; what lies
+// beyond them is read again from L1 / L2. Rows of 8192 and more are bound by those loads (16 rows of 14336: 5.6 us with
+// 256 threads and nothing kept, 4.5 with 512 threads and four words); for shorter ones and for many rows the
+// unrolled words only cost the threads that have none (1024 rows of 1024: 3.2 and 7.0 us, 4096 of 8192: 42.7 and 47.5).
+template <int THREADS, int KEEP>
+__global__ void __launch_bounds__(THREADS)
 quantize_rows_vec8_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int8_t* __restrict__ q, int ldq,
                           float* __restrict__ sx, int K) {
-  __shared__ float s_max[QR_THREADS / 32];
+  __shared__ float s_max[THREADS / 32];
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * ldx);
   const int n8 = K >> 3;
-  uint4 kept[QR_KEEP];
+  uint4 kept[KEEP ? KEEP : 1];
 #pragma unroll
-  for (int j = 0; j < QR_KEEP; ++j) {
-    const int i = threadIdx.x + j * QR_THREADS;
+  for (int j = 0; j < KEEP; ++j) {
+    const int i = threadIdx.x + j * THREADS;
     kept[j] = i < n8 ? xr[i] : make_uint4(0u, 0u, 0u, 0u);
   }
   float amax = 0.f;
@@ -268,15 +270,15 @@ quantize_rows_vec8_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int8_t* 
     amax = fmaxf(amax, fmaxf(fmaxf(fabsf(bf16_lo(v.z)), fabsf(bf16_hi(v.z))), fmaxf(fabsf(bf16_lo(v.w)), fabsf(bf16_hi(v.w)))));
   };
 #pragma unroll
-  for (int j = 0; j < QR_KEEP; ++j) widen(kept[j]);
-  for (int i = threadIdx.x + QR_KEEP * QR_THREADS; i < n8; i += QR_THREADS) widen(xr[i]);
+  for (int j = 0; j < KEEP; ++j) widen(kept[j]);
+  for (int i = threadIdx.x + KEEP * THREADS; i < n8; i += THREADS) widen(xr[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   if (lane == 0) s_max[warp] = amax;
   __syncthreads();
   amax = s_max[0];
 #pragma unroll
-  for (int w = 1; w < QR_THREADS / 32; ++w) amax = fmaxf(amax, s_max[w]);
+  for (int w = 1; w < THREADS / 32; ++w) amax = fmaxf(amax, s_max[w]);
   const float s = amax == 0.f ? 1.f : amax / 127.f;
   if (threadIdx.x == 0) sx[row] = s;
   uint2* qr = reinterpret_cast<uint2*>(q + static_cast<size_t>(row) * ldq);
@@ -294,11 +296,11 @@ quantize_rows_vec8_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int8_t* 
     qr[i] = make_uint2(w[0], w[1]);
   };
 #pragma unroll
-  for (int j = 0; j < QR_KEEP; ++j) {
-    const int i = threadIdx.x + j * QR_THREADS;
+  for (int j = 0; j < KEEP; ++j) {
+    const int i = threadIdx.x + j * THREADS;
     if (i < n8) quantise(i, kept[j]);
   }
-  for (int i = threadIdx.x + QR_KEEP * QR_THREADS; i < n8; i += QR_THREADS) quantise(i, xr[i]);
+  for (int i = threadIdx.x + KEEP * THREADS; i < n8; i += THREADS) quantise(i, xr[i]);
 }
 
 }  // namespace sb
@@ -312,8 +314,9 @@ extern "C" int sb_quantize_rows(const void* x, int ldx, void* xq, int ldq, float
   if (M <= 0 || K <= 0 || ldq < K) return SB_ERR_ARG;
   if ((K & 7) == 0 && (ldx & 7) == 0 && (ldq & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(xq) & 7) == 0) {
-    quantize_rows_vec8_kernel<<<M, QR_THREADS, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x), ldx,
-                                                     static_cast<int8_t*>(xq), ldq, sx, K);
+    const bool keep = K >= 8192 && M <= 1024;
+    auto kern = keep ? quantize_rows_vec8_kernel<512, 4> : quantize_rows_vec8_kernel<256, 0>;
+    kern<<<M, keep ? 512 : 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x), ldx, static_cast<int8_t*>(xq), ldq, sx, K);
     return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
   }
   quantize_rows_kernel<<<(M + 7) / 8, 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x), ldx,

@@ -164,7 +164,7 @@ def test_rmsnorm_few_rows_are_the_bits_of_many(cols):
     assert torch.equal(few, many[:7]) and torch.equal(inv_few, inv_many[:7])
 
 
-@pytest.mark.parametrize("M,K", [(1, 8), (3, 4096), (2, 16384), (2, 16392), (5, 24)])
+@pytest.mark.parametrize("M,K", [(1, 8), (3, 4096), (3, 8184), (3, 8192), (1025, 8192), (2, 16384), (2, 16392), (5, 24)])
 def test_quantize_rows_edges(M, K):
     """Rows that fit a CTA's registers and rows that do not, a zero row: the host statement bit for bit."""
     from scirust_b200.ops import decode
