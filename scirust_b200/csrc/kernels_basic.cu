@@ -912,12 +912,15 @@ using namespace sb;
 #define CHECK_LAUNCH() return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH
 static inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-constexpr int RMS_FEW_ROWS = 1184;    // eight CTAs of 256 threads on every SM: beyond it a row per warp fills the GPU
+// A CTA per row while all of them fit the GPU at once (eight of 256 threads on each SM) and the rows are long enough to give
+// most of its threads a word: us, a row per warp against a CTA per row, 1184 rows of 2816 4.6 / 3.8, 512 of 1024 2.5 / 2.1,
+// 296 of 256 1.94 / 1.85, but 768 of 1024 2.6 / 2.8, 1184 of 2048 3.5 / 3.6, 1024 of 256 2.1 / 3.0.
+static inline bool rms_few_rows(int rows, int cols) { return rows <= 296 || (rows <= 1184 && 2 * rows <= cols); }
 extern "C" int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* inv_rms, int rows, int cols, int ldx,
                               int ldy, float eps, void* stream) {
   if (rows <= 0 || cols <= 0 || (cols & 7) || (ldx & 7) || (ldy & 7)) return SB_ERR_ARG;
   if (!al16(x) || !al16(w) || !al16(y)) return SB_ERR_ALIGN;
-  if (rows <= RMS_FEW_ROWS) {
+  if (rms_few_rows(rows, cols)) {
     rmsnorm_fwd_row_kernel<<<rows, 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x),
                                                      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
                                                      inv_rms, cols, ldx, ldy, eps);

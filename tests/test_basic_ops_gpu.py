@@ -154,14 +154,15 @@ def test_sumsq_edges(dtype, n, offset):
     assert abs(out.item() - 2 * want) <= 2e-5 * want
 
 
-@pytest.mark.parametrize("cols", [8, 1024, 2056, 8192, 9000])
+@pytest.mark.parametrize("cols", [8, 600, 1024, 2056, 8192, 9000])
 def test_rmsnorm_few_rows_are_the_bits_of_many(cols):
-    """A CTA per row up to 1184 rows, a warp per row beyond: the same association, so the same bits; rows longer than
-    what a thread keeps are read again."""
+    """A CTA per row for few rows (up to 296, or up to 1184 of twice as many columns), a warp per row beyond: the same
+    association, so the same bits on both sides of every line; rows longer than what a thread keeps are read again."""
     x, w = _r((1185, cols), 1).cuda(), _r((cols,), 2).cuda()
     many, inv_many = ops.rmsnorm_fwd(x, w)
-    few, inv_few = ops.rmsnorm_fwd(x[:7], w)
-    assert torch.equal(few, many[:7]) and torch.equal(inv_few, inv_many[:7])
+    for n in (7, 296, 297, min(1184, cols // 2)):
+        few, inv_few = ops.rmsnorm_fwd(x[:n], w)
+        assert torch.equal(few, many[:n]) and torch.equal(inv_few, inv_many[:n])
 
 
 @pytest.mark.parametrize("M,K", [(1, 8), (3, 4096), (3, 8184), (3, 8192), (1025, 8192), (2, 16384), (2, 16392), (5, 24)])
