@@ -98,7 +98,7 @@ def test_cnn_models_train_on_gpu():
         assert losses[-1] < losses[0], losses
 
 
-@pytest.mark.parametrize("rows,C_", [(1, 8), (255, 72), (257, 64), (1000, 200), (300, 12), (2050, 520)])
+@pytest.mark.parametrize("rows,C_", [(1, 8), (255, 72), (257, 64), (1000, 200), (300, 12), (523, 13), (2050, 520)])
 @pytest.mark.parametrize("relu", [False, True])
 def test_batchnorm_row_and_column_edges(rows, C_, relu):
     """Chunks of 256 rows, blocks of 64 columns, channels in whole 16-byte words or not, with the ReLU mask folded into
