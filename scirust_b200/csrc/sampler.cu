@@ -71,10 +71,8 @@ struct SampShared {
   int cut_d;                                       // result of the scan
   unsigned long long cut_cnt, cut_sum, in_cnt, in_sum;
   unsigned long long total;                        // this CTA's weight sum
-  float vmax;                                      // this CTA's maximum (greedy: the value at vid)
-  int vid;
+  float vmax;                                      // this CTA's maximum
   float red[SAMP_THREADS / 32];
-  int red_i[SAMP_THREADS / 32];
   unsigned long long red_u[SAMP_THREADS / 32];
   int64_t tok[SAMP_MAX_WINDOW];
 };
@@ -259,7 +257,7 @@ __device__ Walk ranked_walk(cg::cluster_group& cl, SampShared& s, const Row<SMEM
 }
 
 template <bool SMEM>
-__global__ void __launch_bounds__(SAMP_THREADS)
+__global__ void __launch_bounds__(SAMP_THREADS, 1)
 sample_rows_kernel(const SampleParams p) {
   extern __shared__ __align__(16) uint32_t slice_smem[];
   __shared__ SampShared s;
@@ -321,135 +319,100 @@ sample_rows_kernel(const SampleParams p) {
   __syncthreads();
 
   int token = -1;              // known to the thread that writes it out
-  if (p.temperature <= 0.f) {
-    // greedy: first maximum, a NaN never wins against a number
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int j = t; j < row.n; j += SAMP_THREADS) {
-      float v = wf[j];
-      v = v != v ? -INFINITY : v;          // a NaN never beats a number
-      if (bi == 0x7fffffff || v > best) { best = v; bi = row.base + j; }
-    }
+  float mx = -INFINITY;
+  for (int j = t; j < row.n; j += SAMP_THREADS) mx = fmaxf(mx, wf[j]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob > best || (!(best > ob) && oi < bi)) { best = ob; bi = oi; }
-    }
-    if (lane == 0) { s.red[warp] = best; s.red_i[warp] = bi; }
-    __syncthreads();
-    if (t == 0) {
-      for (int i = 1; i < SAMP_THREADS / 32; ++i)
-        if (s.red[i] > best || (!(best > s.red[i]) && s.red_i[i] < bi)) { best = s.red[i]; bi = s.red_i[i]; }
-      s.vmax = best;
-      s.vid = bi;
-    }
-    cl.sync();
-    if (rank == 0 && t == 0) {
-      for (int r = 1; r < nr; ++r) {
-        const float ob = *cl.map_shared_rank(&s.vmax, r);
-        const int oi = *cl.map_shared_rank(&s.vid, r);
-        if (ob > best || (!(best > ob) && oi < bi)) { best = ob; bi = oi; }
-      }
-      // the host rule starts from element 0, so a NaN there is never displaced
-      token = (bi == 0x7fffffff || wf[0] != wf[0]) ? 0 : bi;
-    }
-  } else {
-    float mx = -INFINITY;
-    for (int j = t; j < row.n; j += SAMP_THREADS) mx = fmaxf(mx, wf[j]);
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) s.red[warp] = mx;
+  __syncthreads();
+  if (warp == 0) {
+    mx = s.red[lane];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) s.red[warp] = mx;
-    __syncthreads();
-    if (warp == 0) {
-      mx = s.red[lane];
+    if (lane == 0) s.vmax = mx;
+  }
+  cl.sync();
+  mx = s.vmax;
+  for (int r = 0; r < nr; ++r) mx = fmaxf(mx, *cl.map_shared_rank(&s.vmax, r));
+  // fixed-point weights and their total
+  unsigned long long local = 0;
+  const float inv_t = 1.0f / p.temperature;
+  for (int j = t; j < row.n; j += SAMP_THREADS) {
+    const float e = expf((wf[j] - mx) * inv_t);              // in [0, 1]
+    const float f = e * 4294967296.0f;
+    const uint32_t q = f >= 4294967040.0f ? 0xffffffffu : static_cast<uint32_t>(f);
+    row.w[j] = q;
+    local += q;
+  }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      if (lane == 0) s.vmax = mx;
-    }
-    cl.sync();
-    mx = s.vmax;
-    for (int r = 0; r < nr; ++r) mx = fmaxf(mx, *cl.map_shared_rank(&s.vmax, r));
-    // fixed-point weights and their total
-    unsigned long long local = 0;
-    const float inv_t = 1.0f / p.temperature;
-    for (int j = t; j < row.n; j += SAMP_THREADS) {
-      const float e = expf((wf[j] - mx) * inv_t);              // in [0, 1]
-      const float f = e * 4294967296.0f;
-      const uint32_t q = f >= 4294967040.0f ? 0xffffffffu : static_cast<uint32_t>(f);
-      row.w[j] = q;
-      local += q;
-    }
+  for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
+  if (lane == 0) s.red_u[warp] = local;
+  __syncthreads();
+  if (warp == 0) {
+    local = s.red_u[lane];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-    if (lane == 0) s.red_u[warp] = local;
-    __syncthreads();
-    if (warp == 0) {
-      local = s.red_u[lane];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-      if (lane == 0) s.total = local;
+    if (lane == 0) s.total = local;
+  }
+  cl.sync();
+  unsigned long long z = 0;
+  for (int r = 0; r < nr; ++r) z += *cl.map_shared_rank(&s.total, r);
+  // kept set: first min(top_k, V) ranks, cut where the cumulative probability reaches top_p
+  const unsigned long long n_all = static_cast<unsigned long long>(V);
+  const unsigned long long limit = (p.top_k > 0 && p.top_k < V) ? static_cast<unsigned long long>(p.top_k) : n_all;
+  unsigned long long zz = z;
+  int buf = 0;
+  bool have_top = false;
+  if (limit < n_all || p.top_p < 1.0f) {
+    unsigned long long tp = ~0ull;   // unreachable sum: only the count stops the walk
+    if (p.top_p < 1.0f) {
+      const double d = static_cast<double>(p.top_p) * static_cast<double>(z);
+      tp = d <= 1.0 ? 1ull : static_cast<unsigned long long>(ceil(d));
     }
-    cl.sync();
-    unsigned long long z = 0;
-    for (int r = 0; r < nr; ++r) z += *cl.map_shared_rank(&s.total, r);
-    // kept set: first min(top_k, V) ranks, cut where the cumulative probability reaches top_p
-    const unsigned long long n_all = static_cast<unsigned long long>(V);
-    const unsigned long long limit = (p.top_k > 0 && p.top_k < V) ? static_cast<unsigned long long>(p.top_k) : n_all;
-    unsigned long long zz = z;
-    int buf = 0;
-    bool have_top = false;
-    if (limit < n_all || p.top_p < 1.0f) {
-      unsigned long long tp = ~0ull;   // unreachable sum: only the count stops the walk
-      if (p.top_p < 1.0f) {
-        const double d = static_cast<double>(p.top_p) * static_cast<double>(z);
-        tp = d <= 1.0 ? 1ull : static_cast<unsigned long long>(ceil(d));
-      }
-      zz = ranked_walk<SMEM>(cl, s, row, buf, false, n_all, z, limit, tp, false).sum;
-      have_top = true;
-    }
-    // one uniform draw; every thread computes it, one stores the state after all have read it
-    uint64_t st = p.rng_state[row_id];
-    st ^= st << 13; st ^= st >> 7; st ^= st << 17;
-    const float u = static_cast<float>(static_cast<double>(st >> 11) / 9007199254740992.0);
-    unsigned long long target = static_cast<unsigned long long>(static_cast<double>(u) * static_cast<double>(zz));
-    if (zz > 0 && target >= zz) target = zz - 1;
-    const Walk wk = ranked_walk<SMEM>(cl, s, row, buf, have_top, n_all, z, n_all, target, true);
-    cl.sync();
-    if (rank == 0 && t == 0) p.rng_state[row_id] = st;
-    if (wk.ties == 1) {
-      row.each([&](int j, uint32_t v) { if (v == wk.weight) token = row.base + j; });
-    } else {
-      // id of the take-th smallest id among the ties: radix-select on the id (three 8-bit levels)
-      unsigned long long k = wk.take - 1;   // 0-based index among ties
-      uint32_t id_prefix = 0;
+    zz = ranked_walk<SMEM>(cl, s, row, buf, false, n_all, z, limit, tp, false).sum;
+    have_top = true;
+  }
+  // one uniform draw; every thread computes it, one stores the state after all have read it
+  uint64_t st = p.rng_state[row_id];
+  st ^= st << 13; st ^= st >> 7; st ^= st << 17;
+  const float u = static_cast<float>(static_cast<double>(st >> 11) / 9007199254740992.0);
+  unsigned long long target = static_cast<unsigned long long>(static_cast<double>(u) * static_cast<double>(zz));
+  if (zz > 0 && target >= zz) target = zz - 1;
+  const Walk wk = ranked_walk<SMEM>(cl, s, row, buf, have_top, n_all, z, n_all, target, true);
+  cl.sync();
+  if (rank == 0 && t == 0) p.rng_state[row_id] = st;
+  if (wk.ties == 1) {
+    row.each([&](int j, uint32_t v) { if (v == wk.weight) token = row.base + j; });
+  } else {
+    // id of the take-th smallest id among the ties: radix-select on the id (three 8-bit levels)
+    unsigned long long k = wk.take - 1;   // 0-based index among ties
+    uint32_t id_prefix = 0;
 #pragma unroll 1
-      for (int level = 0; level < 3; ++level) {
-        const int shift = 16 - 8 * level;
-        const uint32_t mask_hi = level == 0 ? 0u : (0xffffffffu << (shift + 8));
-        row.each([&](int j, uint32_t v) {
-          const uint32_t id = static_cast<uint32_t>(row.base + j);
-          if (v == wk.weight && (id & mask_hi) == id_prefix) atomicAdd(&s.h[buf].cnt[(id >> shift) & 0xff], 1u);
-        });
-        cl.sync();
-        if (t < 256) {
-          unsigned long long c = 0;
-          for (int r = 0; r < nr; ++r) c += cl.map_shared_rank(&s.h[buf], r)->cnt[t];
-          s.tot_cnt[t] = c;
-        } else if (t < 512) {
-          s.h[buf ^ 1].cnt[t - 256] = 0;
-        }
-        buf ^= 1;
-        __syncthreads();
-        int d = 0;
-        for (; d < 255; ++d) {
-          if (k < s.tot_cnt[d]) break;
-          k -= s.tot_cnt[d];
-        }
-        id_prefix |= static_cast<uint32_t>(d) << shift;
+    for (int level = 0; level < 3; ++level) {
+      const int shift = 16 - 8 * level;
+      const uint32_t mask_hi = level == 0 ? 0u : (0xffffffffu << (shift + 8));
+      row.each([&](int j, uint32_t v) {
+        const uint32_t id = static_cast<uint32_t>(row.base + j);
+        if (v == wk.weight && (id & mask_hi) == id_prefix) atomicAdd(&s.h[buf].cnt[(id >> shift) & 0xff], 1u);
+      });
+      cl.sync();
+      if (t < 256) {
+        unsigned long long c = 0;
+        for (int r = 0; r < nr; ++r) c += cl.map_shared_rank(&s.h[buf], r)->cnt[t];
+        s.tot_cnt[t] = c;
+      } else if (t < 512) {
+        s.h[buf ^ 1].cnt[t - 256] = 0;
       }
-      if (rank == 0 && t == 0) token = static_cast<int>(id_prefix);
+      buf ^= 1;
+      __syncthreads();
+      int d = 0;
+      for (; d < 255; ++d) {
+        if (k < s.tot_cnt[d]) break;
+        k -= s.tot_cnt[d];
+      }
+      id_prefix |= static_cast<uint32_t>(d) << shift;
     }
+    if (rank == 0 && t == 0) token = static_cast<int>(id_prefix);
   }
   if (token >= 0) {
     p.out_tokens[row_id] = token;
@@ -458,19 +421,144 @@ sample_rows_kernel(const SampleParams p) {
   cl.sync();   // no CTA leaves while another may still read its shared memory
 }
 
-template <bool SMEM>
-static int launch_sample(const SampleParams& p, int rows, int cluster, cudaStream_t stream) {
-  auto kern = sample_rows_kernel<SMEM>;
-  const size_t smem = SMEM ? static_cast<size_t>(p.slice) * 4 : 0;
-  static bool attr = false;
-  if (SMEM && !attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMP_SLICE_WORDS * 4) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr = true;
+// Greedy rows (T <= 0) need one pass: the logits are read once, straight from memory, by as many CTAs of a cluster as leave
+// each at least 4096 words and the grid within the GPU (a cluster of eight for every row from 8193 words on took 18.6 us
+// for 64 rows of 9000, where one CTA per row takes 5.2). The ids of the penalty's window are worked out first, one thread
+// each, and skipped by the pass: it looks an id up only where its logit would win, in a bitmap of the slice (of
+// its low 16 bits, and then the window itself, for slices longer than that).
+constexpr int SAMP_BITMAP = 65536;
+constexpr int SAMP_SMALL_V = 2048, SAMP_SMALL_THREADS = 256;   // a small block starts sooner; it has a thread per id of the window
+static_assert(SAMP_SMALL_THREADS >= SAMP_MAX_WINDOW, "a thread per id of the window");
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
+greedy_rows_kernel(const SampleParams p) {
+  __shared__ __align__(16) int tok[SAMP_MAX_WINDOW];          // -1: no id of this row
+  __shared__ uint32_t bitmap[SAMP_BITMAP / 32];
+  __shared__ float red[THREADS / 32];
+  __shared__ int red_i[THREADS / 32];
+  __shared__ float vmax;
+  __shared__ int vid;
+  cg::cluster_group cl = cg::this_cluster();
+  const int nr = cl.num_blocks(), rank = cl.block_rank();
+  const int row_id = blockIdx.x / nr;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const float* x = p.logits + static_cast<size_t>(row_id) * p.ld;
+  const int base = rank * p.slice, n = max(0, min(p.slice, p.V - base));
+  const float x0 = rank == 0 && t == 0 ? x[0] : 0.f;     // asked for now, looked at in the end
+  // the larger value, the lower id among equals; a NaN never wins against a number
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  auto better = [](float ob, int oi, float b, int i) { return ob > b || (!(b > ob) && oi < i); };
+  auto number = [](float v) { return v != v ? -INFINITY : v; };
+  int n_win = 0;
+  if (p.rep_penalty > 1.0f && p.recent && p.n_recent) {
+    const int nrec = p.n_recent[row_id];
+    n_win = min(min(nrec, p.rep_window), SAMP_MAX_WINDOW);
+    const int64_t* rec = p.recent + static_cast<size_t>(row_id) * p.recent_ld + (nrec - n_win);
+    for (int j = t; j < (min(n, SAMP_BITMAP) + 31) / 32; j += THREADS) bitmap[j] = 0;
+    if (t < SAMP_MAX_WINDOW) {
+      const int64_t id = t < n_win ? rec[t] : -1;
+      tok[t] = id >= 0 && id < p.V ? static_cast<int>(id) : -1;
+    }
+    __syncthreads();
+    const int tk = t < n_win ? tok[t] : -1, at = tk - base;
+    if (tk >= 0 && at >= 0 && at < n) {
+      const uint32_t bit = static_cast<uint32_t>(at) & (SAMP_BITMAP - 1);
+      atomicOr(&bitmap[bit >> 5], 1u << (bit & 31));
+      // every occurrence in the window applies the penalty once more; the first occurrence's thread applies them all
+      int before = 0, times = 0;
+      for (int k = 0; k < n_win; k += 4) {
+        const int4 o = *reinterpret_cast<const int4*>(tok + k);
+        times += (o.x == tk) + (o.y == tk) + (o.z == tk) + (o.w == tk);
+        before += (o.x == tk && k < t) + (o.y == tk && k + 1 < t) + (o.z == tk && k + 2 < t) + (o.w == tk && k + 3 < t);
+      }
+      if (before == 0) {
+        float l = x[tk];
+        for (int k = 0; k < times; ++k) l = l > 0.f ? l / p.rep_penalty : l * p.rep_penalty;
+        best = number(l);
+        bi = tk;
+      }
+    }
+    __syncthreads();
   }
+
+  auto visit = [&](int j, float v) {
+    v = number(v);
+    if (!better(v, base + j, best, bi)) return;
+    if (n_win > 0) {
+      const uint32_t bit = static_cast<uint32_t>(j) & (SAMP_BITMAP - 1);
+      if (bitmap[bit >> 5] >> (bit & 31) & 1u) {
+        bool in = n <= SAMP_BITMAP;
+        for (int k = 0; k < n_win && !in; ++k) in = tok[k] == base + j;
+        if (in) return;
+      }
+    }
+    best = v;
+    bi = base + j;
+  };
+  const float* xs = x + min(base, p.V);
+  int done = 0;
+  if ((reinterpret_cast<uintptr_t>(xs) & 15) == 0) {
+    const int n4 = n >> 2;
+    constexpr int U = 4;                       // 16-byte loads in flight
+    for (int j0 = t; j0 < n4; j0 += U * THREADS) {
+      float4 a[U];
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        const int j = j0 + i * THREADS;
+        a[i] = j < n4 ? __ldg(reinterpret_cast<const float4*>(xs) + j) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      }
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        const int j = j0 + i * THREADS;
+        if (j >= n4 || fmaxf(fmaxf(a[i].x, a[i].y), fmaxf(a[i].z, a[i].w)) < best) continue;
+        visit(4 * j, a[i].x); visit(4 * j + 1, a[i].y); visit(4 * j + 2, a[i].z); visit(4 * j + 3, a[i].w);
+      }
+    }
+    done = 4 * n4;
+  }
+#pragma unroll 4
+  for (int j = done + t; j < n; j += THREADS) visit(j, xs[j]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
+  }
+  if (lane == 0) { red[warp] = best; red_i[warp] = bi; }
+  __syncthreads();
+  if (warp == 0) {
+    best = lane < THREADS / 32 ? red[lane] : -INFINITY;
+    bi = lane < THREADS / 32 ? red_i[lane] : 0x7fffffff;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
+    }
+    if (lane == 0) { vmax = best; vid = bi; }
+  }
+  if (nr > 1) cl.sync();
+  if (rank == 0 && t == 0) {
+    for (int r = 1; r < nr; ++r) {
+      const float ob = *cl.map_shared_rank(&vmax, r);
+      const int oi = *cl.map_shared_rank(&vid, r);
+      if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
+    }
+    // the host rule starts from element 0, so a NaN there is never displaced
+    const int token = (bi == 0x7fffffff || x0 != x0) ? 0 : bi;
+    p.out_tokens[row_id] = token;
+    if (p.generated) p.generated[static_cast<size_t>(row_id) * p.gen_stride + p.step] = token;
+  }
+  if (nr > 1) cl.sync();   // no CTA leaves while another may still read its shared memory
+}
+
+static int launch_clusters(void (*kern)(const SampleParams), const SampleParams& p, int rows, int cluster, int threads,
+                           size_t smem, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(rows) * cluster);
-  cfg.blockDim = dim3(SAMP_THREADS);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute at[1];
@@ -479,8 +567,34 @@ static int launch_sample(const SampleParams& p, int rows, int cluster, cudaStrea
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;      // a plain launch is a cluster of one
   return cudaLaunchKernelEx(&cfg, kern, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+}
+
+int num_sms();   // gemm_tcgen05.cu
+
+static int launch_greedy(SampleParams p, int rows, cudaStream_t stream) {
+  // a cluster's CTAs lie in one part of the GPU: sixteen clusters of eight do not run at once (16 rows of 128256: 12.9 us, in
+  // clusters of four 7.7), so those fill three quarters of the SMs at most
+  int cluster = 1;
+  while (cluster < SAMP_CLUSTER && p.V / (2 * cluster) >= 4096 &&
+         rows * 2 * cluster <= (cluster < 4 ? num_sms() : num_sms() * 3 / 4)) cluster *= 2;
+  p.slice = ((p.V + cluster - 1) / cluster + 3) / 4 * 4;
+  if (p.V <= SAMP_SMALL_V)
+    return launch_clusters(greedy_rows_kernel<SAMP_SMALL_THREADS>, p, rows, cluster, SAMP_SMALL_THREADS, 0, stream);
+  return launch_clusters(greedy_rows_kernel<SAMP_THREADS>, p, rows, cluster, SAMP_THREADS, 0, stream);
+}
+
+template <bool SMEM>
+static int launch_sample(const SampleParams& p, int rows, int cluster, cudaStream_t stream) {
+  auto kern = sample_rows_kernel<SMEM>;
+  static bool attr = false;
+  if (SMEM && !attr) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMP_SLICE_WORDS * 4) != cudaSuccess)
+      return SB_ERR_LAUNCH;
+    attr = true;
+  }
+  return launch_clusters(kern, p, rows, cluster, SAMP_THREADS, SMEM ? static_cast<size_t>(p.slice) * 4 : 0, stream);
 }
 
 }  // namespace sb
@@ -501,8 +615,9 @@ extern "C" int sb_sample_rows(const float* logits, int ld, int rows, int V, floa
   p.rep_penalty = rep_penalty; p.rep_window = rep_window; p.recent = recent; p.recent_ld = recent_ld;
   p.n_recent = n_recent; p.rng_state = rng_state; p.out_tokens = out_tokens; p.generated = generated;
   p.gen_stride = gen_stride; p.step = step; p.work = work;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (temperature <= 0.f) return launch_greedy(p, rows, st);
   const int cluster = V <= SAMP_SINGLE_MAX_V ? 1 : SAMP_CLUSTER;
   p.slice = ((V + cluster - 1) / cluster + 3) / 4 * 4;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   return p.slice <= SAMP_SLICE_WORDS ? launch_sample<true>(p, rows, cluster, st) : launch_sample<false>(p, rows, cluster, st);
 }

@@ -148,3 +148,46 @@ def test_odd_rows_and_penalties_match_the_float64_policy(vocab):
     got = dev.sample(lg.cuda()).cpu().tolist()
     same = sum(got[b] == _exact_pick(lg[b], params, hist[b].tolist(), SamplerRng(b).next_uniform()) for b in range(rows))
     assert same >= rows - 1
+
+
+def _greedy_pick(row, recent, penalty):
+    """First maximum of the penalised row; a NaN never beats a number, but one in column 0 is never displaced."""
+    v, p = row.clone(), torch.tensor(penalty, dtype=torch.float32)
+    for t in recent:
+        if 0 <= t < len(v):
+            v[t] = v[t] / p if v[t] > 0 else v[t] * p
+    if v[0] != v[0]:
+        return 0
+    v = v.masked_fill(v != v, float("-inf"))
+    return int((v == v.max()).nonzero()[0])
+
+
+@pytest.mark.parametrize("vocab", [1, 3, 2047, 2049, 4097, 8191, 16384, 16389, 100003, 600001])
+@pytest.mark.parametrize("rows", [1, 20, 64])
+@pytest.mark.parametrize("penalty", [1.0, 1.5])
+def test_greedy_rows_on_every_split(vocab, rows, penalty):
+    """One CTA per row and clusters of two to eight, rows at any alignment: ties at the first and last element of a slice, NaN in
+    column 0 and elsewhere, rows of -inf only, and windows that repeat the winner or share its bit of the bitmap."""
+    wide = torch.randn(rows, vocab + 3, generator=torch.Generator().manual_seed(vocab)).cuda()
+    lg = wide[:, :vocab]
+    hist = torch.randint(0, vocab, (rows, 16), generator=torch.Generator().manual_seed(2))
+    for b in range(rows):
+        top = int(lg[b].argmax())
+        hist[b, 3] = hist[b, 9] = top
+        hist[b, 5] = (top + 65536) % vocab
+        cut = ((vocab + 3) // 4 + 3) // 4 * 4
+        if b % 5 == 1:
+            lg[b, vocab - 1] = lg[b, min(cut, vocab - 1)] = lg[b, max(min(cut, vocab) - 1, 0)] = 9.0
+        if b % 5 == 2:
+            lg[b, vocab // 2:] = float("nan")
+        if b % 5 == 3:
+            lg[b] = float("-inf")
+        if b % 5 == 4:
+            lg[b, 0] = float("nan")
+    s = DeviceSampler(SamplingParams(temperature=0.0, repetition_penalty=penalty, repetition_window=12), rows, vocab,
+                      range(rows), "cuda", history_len=16)
+    s.set_history(hist)
+    got = s.sample(lg).cpu().tolist()
+    host = lg.cpu()
+    want = [_greedy_pick(host[b], hist[b, 4:].tolist() if penalty > 1 else [], penalty) for b in range(rows)]
+    assert got == want
