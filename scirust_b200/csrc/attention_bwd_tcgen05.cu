@@ -14,6 +14,7 @@
 // P is recomputed from the saved log-sum-exp; dS = P * (dP - delta) * scale.
 #include "sm100_ptx.cuh"
 #include "api.h"
+#include "per_device.h"
 
 namespace sb {
 
@@ -1005,15 +1006,10 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& td, const CUtens
   if constexpr (DH == 64) k1 = attention_bwd_dkv_kernel<64>; else k1 = attention_bwd_dkv_split_kernel<128>;
   auto k2 = attention_bwd_dq_kernel<DH>;
   auto k3 = attention_bwd_dq_stream_kernel<DH>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, DKV_SMEM) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, DqCfg<DH>::SMEM_BYTES) != cudaSuccess ||
-        cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, DqsCfg<DH>::SMEM_BYTES) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr_set = true;
-  }
+  static PerDeviceOnce a1, a2, a3;
+  if (allow_smem(a1, k1, DKV_SMEM, SB_ERR_LAUNCH) || allow_smem(a2, k2, DqCfg<DH>::SMEM_BYTES, SB_ERR_LAUNCH) ||
+      allow_smem(a3, k3, DqsCfg<DH>::SMEM_BYTES, SB_ERR_LAUNCH))
+    return SB_ERR_LAUNCH;
   const int n_t = (p.S + BT - 1) / BT;
   k1<<<dim3(p.Hkv, p.B, n_t), BWD_THREADS, DKV_SMEM, stream>>>(tq, td, tds, p);
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;

@@ -42,6 +42,7 @@
 // Warps: 0 TMA producer, 1 MMA issuer, 2-5 softmax of tile 0, 6-9 softmax of tile 1.
 #include "sm100_ptx.cuh"
 #include "api.h"
+#include "per_device.h"
 
 namespace sb {
 
@@ -431,12 +432,8 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
 template <int DH>
 static int launch(const CUtensorMap& tm, const CUtensorMap& tv, const Params& p, cudaStream_t stream) {
   auto kern = attention_fwd_pp_kernel<DH>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<DH>::SMEM_BYTES) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr_set = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, kern, Cfg<DH>::SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   dim3 grid(p.H, p.B, (p.S + 2 * BM - 1) / (2 * BM));
   kern<<<grid, THREADS, Cfg<DH>::SMEM_BYTES, stream>>>(tm, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;

@@ -15,6 +15,7 @@
 // CTA = (128-query tile, head, batch); 6 warps: 0 TMA producer, 1 MMA issuer, 2-5 softmax.
 #include "sm100_ptx.cuh"
 #include "api.h"
+#include "per_device.h"
 
 namespace sb {
 
@@ -290,12 +291,8 @@ template <int DH>
 static int launch_att_fwd(const CUtensorMap& tm, const AttParams& p, cudaStream_t stream) {
   using Cfg = AttCfg<DH>;
   auto kern = attention_fwd_kernel<DH>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr_set = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, kern, Cfg::SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   dim3 grid(p.H, p.B, (p.S + ATT_BM - 1) / ATT_BM);
   kern<<<grid, ATT_THREADS, Cfg::SMEM_BYTES, stream>>>(tm, p);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;

@@ -13,6 +13,7 @@
 #include <math.h>
 #include <stdint.h>
 #include "api.h"
+#include "per_device.h"
 #include <cuda_fp16.h>
 #include <cstdlib>
 #include "sm100_ptx.cuh"
@@ -2256,11 +2257,8 @@ static int launch_decode_attn(const DecodeAttnParams& p, dim3 grid, cudaStream_t
   constexpr int SMEM = 2 * 2 * DEC_TK * (DH * 2 + 16);   // also covers the merge buffers (4*16*(DH+2) floats)
   static_assert(SMEM >= 4 * 16 * (DH + 2) * 4, "merge buffers must fit in the tile ring");
   auto kern = decode_attn_kernel<DH>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return SB_ERR_LAUNCH;
-    attr = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, kern, SMEM, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   return launch_dep(kern, grid, dim3(128), SMEM, s, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
@@ -2289,12 +2287,8 @@ extern "C" int sb_decode_attention(const void* q, int ldq, const void* pool, con
 template <int DH>
 static int launch_decode_stream(const CUtensorMap& tm, DecodeStreamParams p, int grid, cudaStream_t s) {
   auto kern = decode_attn_stream_kernel<DH>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, kern, 227 * 1024 - 1024, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   const int G = p.H / p.Hkv;
   p.stages = DstCfg<DH>::stages(G);
   return launch_dep(kern, dim3(grid), dim3(DST_THREADS), DstCfg<DH>::smem_bytes(G), s, tm, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;

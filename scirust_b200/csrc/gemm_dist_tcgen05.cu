@@ -35,6 +35,7 @@
 // stops touching peer memory and falls through to its teardown.
 #include "sm100_ptx.cuh"
 #include "api.h"
+#include "per_device.h"
 
 namespace sb {
 
@@ -492,12 +493,8 @@ template <int BN, bool A_MN, bool B_MN>
 static int launch_dist(const DistMaps& maps, const DistParams& p, int grid, cudaStream_t stream) {
   using Cfg = DistCfg<BN>;
   auto kern = gemm_dist_kernel<BN, A_MN, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr_set = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, kern, Cfg::SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   kern<<<grid, DIST_THREADS, Cfg::SMEM_BYTES, stream>>>(maps, p);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }

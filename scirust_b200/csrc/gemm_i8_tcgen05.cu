@@ -14,6 +14,7 @@
 // by i8_splitk_reduce_kernel, which applies the scales.
 #include "sm100_ptx.cuh"
 #include "api.h"
+#include "per_device.h"
 
 namespace sb {
 
@@ -348,12 +349,8 @@ extern "C" int sb_gemm_i8(const void* xq, int ldq, const float* sx, const void* 
   I8Params p;
   p.M = M; p.N = N; p.K = K; p.splits = splits; p.kb_per_split = kbps;
   p.C = splits == 1 ? C : workspace; p.ldc = ldc; p.R = R; p.ldr = ldr; p.sx = sx; p.sw = sw; p.status = status;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(gemm_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM_BYTES) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, gemm_i8_kernel, I8_SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   const int mt = (M + I8_BM - 1) / I8_BM, nt = (N + I8_BN - 1) / I8_BN;
   const int total = mt * nt * splits;
   const int grid = total < num_sms() ? total : num_sms();

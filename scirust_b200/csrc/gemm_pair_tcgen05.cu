@@ -18,6 +18,7 @@
 #include <cstdlib>
 #include "sm100_ptx.cuh"
 #include "api.h"
+#include "per_device.h"
 #include "gemm_sched.cuh"
 
 namespace sb {
@@ -735,12 +736,8 @@ template <bool A_MN, bool B_MN>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int grid, cudaStream_t stream,
                   const CUtensorMap* ta_own = nullptr, const CUtensorMap* tc = nullptr, const TmapSet* trs = nullptr) {
   auto kern = gemm_pair_kernel<A_MN, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr_set = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, kern, SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(THREADS);

@@ -17,6 +17,7 @@
 // Warps: 0 TMA, 1 MMA, 2-5 epilogue (one per TMEM lane quarter).
 #include "sm100_ptx.cuh"
 #include "api.h"
+#include "per_device.h"
 
 namespace sb {
 
@@ -256,12 +257,8 @@ static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const Ski
                          cudaStream_t stream) {
   using Cfg = SkinnyCfg<RB>;
   auto kern = gemm_skinny_kernel<RB, I8>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, kern, Cfg::SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   kern<<<grid, SK_THREADS, Cfg::SMEM_BYTES, stream>>>(tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }

@@ -13,6 +13,7 @@
 // reduced in split order by w8_splitk_reduce_kernel (scale applied there).
 #include "sm100_ptx.cuh"
 #include "api.h"
+#include "per_device.h"
 
 namespace sb {
 
@@ -309,12 +310,8 @@ extern "C" int sb_gemm_w8(const void* A, const void* Q, const float* scale, void
   p.ldr = ldr;
   p.scale = scale;
   p.status = status;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_w8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W8_SMEM_BYTES) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr_set = true;
-  }
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, gemm_w8_kernel, W8_SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   const int tiles = ((M + WBM - 1) / WBM) * ((N + WBN - 1) / WBN) * splits;
   const int grid = tiles < num_sms() ? tiles : num_sms();
   gemm_w8_kernel<<<grid, W8_THREADS, W8_SMEM_BYTES, stream>>>(ta, tq, p);

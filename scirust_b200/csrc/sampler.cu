@@ -24,6 +24,7 @@
 #include <math.h>
 #include <stdint.h>
 #include "api.h"
+#include "per_device.h"
 
 namespace sb {
 
@@ -588,12 +589,8 @@ static int launch_greedy(SampleParams p, int rows, cudaStream_t stream) {
 template <bool SMEM>
 static int launch_sample(const SampleParams& p, int rows, int cluster, cudaStream_t stream) {
   auto kern = sample_rows_kernel<SMEM>;
-  static bool attr = false;
-  if (SMEM && !attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMP_SLICE_WORDS * 4) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr = true;
-  }
+  static PerDeviceOnce attr;
+  if (SMEM && allow_smem(attr, kern, SAMP_SLICE_WORDS * 4, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   return launch_clusters(kern, p, rows, cluster, SAMP_THREADS, SMEM ? static_cast<size_t>(p.slice) * 4 : 0, stream);
 }
 

@@ -1,5 +1,8 @@
 """Rules that choose between two kernels by sizes, on the CPU, for a GPU of 148 SMs: each line is a shape at which both
 sides were timed, with the side that was faster (or, within 2 %, the one that was there first)."""
+import subprocess
+from pathlib import Path
+
 import pytest
 
 from scirust_b200.ops import attention as A, decode as D, gemm as G
@@ -40,3 +43,27 @@ def test_attention_forward_tiles(B, S, H, dh, causal, two):
 ])
 def test_streamed_decode_attention(B, L, H, Hkv, page, stream):
     assert D._stream_wins(L, B * Hkv, H // Hkv, page, None) is stream
+
+
+def test_kernel_attributes_are_set_for_every_device(tmp_path):
+    """The helper of the launchers, with a counting stand-in for the CUDA call: once per device, again after a failure, and
+    every time for device numbers beyond its mask."""
+    src = tmp_path / "once.cpp"
+    src.write_text('''
+        #include "per_device.h"
+        #include <cstdio>
+        #include <initializer_list>
+        int main() {
+          static sb::PerDeviceOnce once;
+          int calls[128] = {}, rc = 0;
+          auto set = [&](int d, int r) { return once(d, [&] { ++calls[d]; return r; }); };
+          for (int i = 0; i < 3; ++i) for (int d : {0, 1, 63}) rc |= set(d, 0);
+          int failed = set(2, -7) == -7 && set(2, -7) == -7;
+          rc |= set(2, 0) | set(2, -7);                      // set by now: not called again
+          rc |= set(64, 0) | set(64, 0);
+          std::printf("%d %d %d %d %d %d %d", rc, failed, calls[0], calls[1], calls[63], calls[2], calls[64]);
+        }''')
+    csrc = Path(__file__).resolve().parent.parent / "scirust_b200" / "csrc"
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", str(csrc), str(src), "-o", str(tmp_path / "once")], check=True)
+    out = subprocess.run([str(tmp_path / "once")], check=True, capture_output=True, text=True).stdout
+    assert out == "0 1 1 1 1 3 2"
