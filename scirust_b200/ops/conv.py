@@ -65,7 +65,7 @@ def unpack_conv_weight(wp: torch.Tensor, in_c: int, k: int) -> torch.Tensor:
     return wp[:, : k * k * in_c].reshape(oc, k, k, in_c).permute(0, 3, 1, 2).reshape(oc, in_c * k * k)
 
 
-_lib.register("sb_conv_gemm", [i32, vp, vp, vp] + [i32] * 11 + [vp, vp, vp])
+_lib.register("sb_conv_gemm", [i32, vp, vp, vp, vp] + [i32] * 11 + [vp, vp, vp])
 _FPROP, _WGRAD, _DGRAD = 1, 2, 3
 
 
@@ -86,7 +86,7 @@ def implicit_ok(geom: ConvGeom, oc: int, k: int, stride: int, pad: int) -> bool:
             and (ow - 1) * stride < 256 and (128 // ow - 1) * stride < 256)
 
 
-def _conv_gemm(mode, a, b, geom, oc, k, stride, pad, OH, OW):
+def _conv_gemm(mode, a, b, geom, oc, k, stride, pad, OH, OW, keep=None):
     pix_o, pix_i, kp = geom.B * OH * OW, geom.rows, k * k * geom.C
     M, N, K = {_FPROP: (pix_o, oc, kp), _WGRAD: (oc, kp, pix_o), _DGRAD: (pix_i, geom.C, k * k * oc)}[mode]
     out = _lib.empty((M, N), BF, a.device)
@@ -94,22 +94,25 @@ def _conv_gemm(mode, a, b, geom, oc, k, stride, pad, OH, OW):
     tiles = ((M + 127) // 128) * ((N + 255) // 256)
     splits = max(1, min(G.num_sms(a.device) // tiles, (K + 63) // 64 // 8, 64))
     ws = G._workspace(splits * M * N, a.device) if splits > 1 else None
-    _lib.call("sb_conv_gemm", mode, a.data_ptr(), b.data_ptr(), out.data_ptr(), geom.B, geom.H, geom.W, geom.C, oc, k,
-              stride, pad, OH, OW, splits, _lib.ptr(ws), _lib.status_word(a.device).data_ptr(), _lib.stream())
+    _lib.call("sb_conv_gemm", mode, a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(keep), geom.B, geom.H, geom.W,
+              geom.C, oc, k, stride, pad, OH, OW, splits, _lib.ptr(ws), _lib.status_word(a.device).data_ptr(), _lib.stream())
     G.launch_count += 2 if splits > 1 else 1
     return out
 
 
 class _Conv(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, wp, geom, k, stride, pad):
+    def forward(ctx, x, wp, geom, k, stride, pad, want_dw):
         B, H, W, C = geom.B, geom.H, geom.W, geom.C
         OH, OW = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
         ctx.meta = (geom, k, stride, pad, OH, OW)
         ctx.implicit = implicit_ok(geom, wp.shape[0], k, stride, pad) and _tma_ok(x, wp, geom, k)
         if ctx.implicit:
-            ctx.save_for_backward(x, wp)
-            return _conv_gemm(_FPROP, x, wp, geom, wp.shape[0], k, stride, pad, OH, OW)
+            # a copy, as the patch matrix is one: the caller's tensor may be written before the backward pass, also by
+            # kernels that its version counter does not see (128 x 32 x 32 x 64: 7 us, where the patch matrix took 86)
+            keep = _lib.empty(x.shape, BF, x.device) if want_dw else None
+            ctx.save_for_backward(keep, wp)
+            return _conv_gemm(_FPROP, x, wp, geom, wp.shape[0], k, stride, pad, OH, OW, keep)
         Kp = wp.shape[1]
         col = _lib.empty((B * OH * OW, Kp), BF, x.device)
         _lib.call("sb_im2col_nhwc", x.data_ptr(), col.data_ptr(), B, H, W, C, k, k, stride, pad, OH, OW, Kp,
@@ -121,7 +124,7 @@ class _Conv(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        col, wp = ctx.saved_tensors                           # col: the input itself when no patch matrix was made
+        col, wp = ctx.saved_tensors                           # col: a copy of the input when no patch matrix was made
         geom, k, stride, pad, OH, OW = ctx.meta
         oc = wp.shape[0]
         dy = dy.contiguous()
@@ -134,13 +137,13 @@ class _Conv(torch.autograd.Function):
                   else G.matmul_tn(dy, col))                  # [oc, Kp] = dy^T col
         if ctx.needs_input_grad[0]:
             if implicit and stride == 1 and _rows_tile(geom.H, geom.W, 128):
-                return _conv_gemm(_DGRAD, dy, wp, geom, oc, k, stride, pad, OH, OW), dw, None, None, None, None
+                return _conv_gemm(_DGRAD, dy, wp, geom, oc, k, stride, pad, OH, OW), dw, None, None, None, None, None
             dcol = G.matmul_nn(dy, wp)                        # [M, Kp]
             dx = _lib.empty((geom.rows, geom.C), BF, dy.device)
             _lib.call("sb_col2im_nhwc", dcol.data_ptr(), dx.data_ptr(), geom.B, geom.H, geom.W, geom.C, k, k, stride,
                       pad, OH, OW, wp.shape[1], _lib.stream())
             G.launch_count += 1
-        return dx, dw, None, None, None, None
+        return dx, dw, None, None, None, None, None
 
 
 def _tma_ok(x, wp, geom, k) -> bool:
@@ -157,7 +160,8 @@ def conv2d(x, wp, geom: ConvGeom, k: int, stride: int = 1, pad: int = 0):
         w4 = wp[:, : k * k * geom.C].reshape(wp.shape[0], k, k, geom.C).permute(0, 3, 1, 2)
         y4 = F.conv2d(rows_to_nchw(x.float(), geom), w4.float(), stride=stride, padding=pad)
         return nchw_to_rows(y4.to(x.dtype))[0], og
-    return _Conv.apply(x.contiguous(), wp, geom, k, stride, pad), og
+    want_dw = torch.is_grad_enabled() and wp.requires_grad
+    return _Conv.apply(x.contiguous(), wp, geom, k, stride, pad, want_dw), og
 
 
 class _MaxPool(torch.autograd.Function):

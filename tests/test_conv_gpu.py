@@ -154,3 +154,24 @@ def test_conv_without_patch_matrix_matches_patch_matrix(B, Cin, H, W, Cout, k, s
     for a, b, taps in zip(got[0], got[1], (1, k * k, 1)):
         lim = b.float().abs().max().item() * 2 ** -8 * (1 + taps ** 0.5)
         assert (a.float() - b.float()).abs().max().item() <= lim
+
+
+def test_conv_input_may_be_written_before_the_backward_pass():
+    """Without a patch matrix the input itself is read for the weight gradient, from a copy: a write in place, seen by the
+    version counter or not, changes neither gradient. Without a weight gradient nothing of the input is kept."""
+    geom = C.ConvGeom(2, 16, 16, 64)
+    assert C.implicit_ok(geom, 64, 3, 1, 1)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x0 = torch.randn(geom.rows, 64, generator=g, device="cuda").to(BF)
+    w = (torch.randn(64, 9 * 64, generator=g, device="cuda") * 0.1).to(BF).requires_grad_(True)
+    dy = torch.randn(geom.rows, 64, generator=g, device="cuda").to(BF)
+    want = torch.autograd.grad(C.conv2d(x0.clone(), w, geom, 3, 1, 1)[0], w, dy)[0]
+    for write in (lambda x: x.zero_(), lambda x: x.data.fill_(float("nan"))):
+        x = x0.clone()
+        y, _ = C.conv2d(x, w, geom, 3, 1, 1)
+        write(x)
+        assert torch.equal(torch.autograd.grad(y, w, dy)[0], want)
+    x, frozen = x0.clone().requires_grad_(True), w.detach()
+    y, _ = C.conv2d(x, frozen, geom, 3, 1, 1)
+    x.data.fill_(float("nan"))
+    assert torch.isfinite(torch.autograd.grad(y, x, dy)[0].float()).all()
