@@ -71,7 +71,7 @@ _FPROP, _WGRAD, _DGRAD = 1, 2, 3
 
 def _rows_tile(oh: int, ow: int, box: int) -> bool:
     """Whether ``box`` consecutive pixels of an oh x ow grid are whole rows of one image or whole images."""
-    if ow > box or box % ow:
+    if oh < 1 or ow < 1 or ow > box or box % ow:
         return False
     rows = box // ow
     return oh % rows == 0 if rows <= oh else rows % oh == 0
@@ -80,9 +80,9 @@ def _rows_tile(oh: int, ow: int, box: int) -> bool:
 def implicit_ok(geom: ConvGeom, oc: int, k: int, stride: int, pad: int) -> bool:
     """Whether a convolution runs without a patch matrix (csrc/gemm_tcgen05.cu: ``sb_conv_gemm``): channels in whole
     64-wide blocks and output rows that tile the 128-pixel operand (and the weight gradient's 64-pixel one). Others
-    (an RGB stem, odd image sizes) gather their patches first."""
+    (an RGB stem, odd image sizes) gather their patches first, and so do those without a pixel, which the native call refuses."""
     oh, ow = (geom.H + 2 * pad - k) // stride + 1, (geom.W + 2 * pad - k) // stride + 1
-    return (geom.C % 64 == 0 and oc % 64 == 0 and stride <= 8 and _rows_tile(oh, ow, 128) and _rows_tile(oh, ow, 64)
+    return (geom.B > 0 and geom.C % 64 == 0 and oc % 64 == 0 and stride <= 8 and _rows_tile(oh, ow, 128) and _rows_tile(oh, ow, 64)
             and (ow - 1) * stride < 256 and (128 // ow - 1) * stride < 256)
 
 

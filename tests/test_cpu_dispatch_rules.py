@@ -5,7 +5,7 @@ from pathlib import Path
 
 import pytest
 
-from scirust_b200.ops import attention as A, decode as D, gemm as G
+from scirust_b200.ops import attention as A, conv as C, decode as D, gemm as G
 
 
 @pytest.fixture(autouse=True)
@@ -67,3 +67,14 @@ def test_kernel_attributes_are_set_for_every_device(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", str(csrc), str(src), "-o", str(tmp_path / "once")], check=True)
     out = subprocess.run([str(tmp_path / "once")], check=True, capture_output=True, text=True).stdout
     assert out == "0 1 1 1 1 3 2"
+
+
+@pytest.mark.parametrize("B,H,W,Cin,oc,k,stride,pad,implicit", [
+    (128, 32, 32, 64, 64, 3, 1, 1, True), (5, 4, 4, 128, 64, 3, 1, 1, True), (2, 32, 16, 128, 64, 3, 2, 1, True),
+    (1, 224, 224, 64, 64, 3, 1, 1, False), (4, 28, 28, 64, 64, 3, 1, 1, False), (8, 32, 32, 3, 64, 3, 1, 1, False),
+    # no output pixel, no image: the patch path, whose native call reports the error
+    (1, 2, 2, 64, 64, 3, 1, 0, False), (1, 8, 2, 64, 64, 3, 1, 0, False), (1, 1, 8, 64, 64, 3, 2, 0, False),
+    (0, 32, 32, 64, 64, 3, 1, 1, False),
+])
+def test_convolution_without_patch_matrix(B, H, W, Cin, oc, k, stride, pad, implicit):
+    assert C.implicit_ok(C.ConvGeom(B, H, W, Cin), oc, k, stride, pad) is implicit
