@@ -119,15 +119,14 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 }
 
 // --------------------------------------------------------------------------- dK / dV
-// Pipeline (DH == 64): the bf16 P^T / dS^T tiles are double-buffered in shared memory, so the MMA
+// Pipeline at head dimension 64: the bf16 P^T / dS^T tiles are double-buffered in shared memory, so the MMA
 // warp issues the score products of iteration t+1 *before* the gradient products of iteration t;
-// the softmax warps then work on t+1 while the tensor cores finish t. With DH == 128 shared
-// memory only fits single buffers and the two groups are issued in program order.
-template <int DH>
+// the softmax warps then work on t+1 while the tensor cores finish t. At 128 shared memory fits single
+// buffers only: the kernel below this one.
 struct DkvCfg {
-  static constexpr bool PDB = (DH == 64);             // double-buffer P^T / dS^T
-  static constexpr int NPB = PDB ? 2 : 1;
-  static constexpr int QS = (DH == 64) ? 2 : 1;       // (Q, dO) ring stages
+  static constexpr int DH = 64;
+  static constexpr int NPB = 2;                       // P^T / dS^T buffers
+  static constexpr int QS = 2;                        // (Q, dO) ring stages
   static constexpr int T_BYTES = BT * DH * 2;         // one [128 x DH] tile
   static constexpr int PT_BYTES = BT * BT * 2;
   static constexpr int TILE_BYTES = 2 * T_BYTES + QS * 2 * T_BYTES + NPB * 2 * PT_BYTES;
@@ -135,12 +134,11 @@ struct DkvCfg {
   static constexpr int TMEM_COLS = 512;  // S^T 128 | dP^T 128 | dK DH | dV DH
 };
 
-template <int DH>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                          const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
-  using Cfg = DkvCfg<DH>;
-  constexpr int NCH = DH / 64;
+  using Cfg = DkvCfg;
+  constexpr int DH = Cfg::DH, NCH = DH / 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
@@ -245,7 +243,7 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
         return true;
       };
       auto issue_grads = [&](int t) {
-        const int pb = Cfg::PDB ? (t & 1) : 0;
+        const int pb = t & 1;
         const uint32_t aPT = smem_u32(sPT + pb * Cfg::PT_BYTES), adST = smem_u32(sdST + pb * Cfg::PT_BYTES);
         const uint32_t bQ = smem_u32(sQ + st_g * Cfg::T_BYTES), bdO = smem_u32(sdO + st_g * Cfg::T_BYTES);
 #pragma unroll
@@ -271,23 +269,19 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
         // (the dS store of t-1 has long been read out of its buffer; the wait only makes that certain before the
         // scores whose completion lets the softmax warps write that buffer again)
         if (p.spill_ds) tma_store_wait_read<0>();
-        if (Cfg::PDB && t + 1 < n_iter) ok = issue_scores();
+        if (t + 1 < n_iter) ok = issue_scores();
         if (p.spill_ds) {
           // the finished dS tile (bf16, [q rows][kv], scale included) also goes to global memory, where
           // the dQ kernel streams it back instead of recomputing scores; the bulk store reads shared
           // memory asynchronously, so it must have been read out before this buffer is written again
           const int head = kvh * group + t / n_qt;
           const int qt = qt_first + t % n_qt;
-          const uint8_t* src = sdST + (Cfg::PDB ? (t & 1) : 0) * Cfg::PT_BYTES;
+          const uint8_t* src = sdST + (t & 1) * Cfg::PT_BYTES;
           tma_store_3d(&tm_ds, src, kv0, qt * BT, b * p.H + head);
           tma_store_3d(&tm_ds, src + BT * 128, kv0 + 64, qt * BT, b * p.H + head);
           tma_store_commit();
         }
         issue_grads(t);
-        if (!Cfg::PDB) {
-          if (p.spill_ds) tma_store_wait_read<0>();   // single dS buffer: read out before it is rewritten
-          if (t + 1 < n_iter) ok = issue_scores();
-        }
       }
       if (ok) umma_commit(done);
       if (p.spill_ds) tma_store_wait<0>();   // the stores are complete before the CTA retires
@@ -307,7 +301,7 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
       const int q0 = qt * BT;
       const int q_idx = q0 + r;
       const float2 sd = __ldg(p.stats + (static_cast<size_t>(b) * p.H + head) * p.S + min(q_idx, p.S - 1));
-      const int pb = Cfg::PDB ? (t & 1) : 0;
+      const int pb = t & 1;
       uint8_t* pt_buf = sPT + pb * Cfg::PT_BYTES;
       uint8_t* dst_buf = sdST + pb * Cfg::PT_BYTES;
       // last visible kv column of this query row inside the tile (-1: row is past the sequence end)
@@ -368,50 +362,47 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
   if (warp == 1) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
 }
 
-// Pipeline at head dimension 128: scores and dP have barriers of their own, so the exponentials of iteration t+1 (which need the scores only)
-// run under the gradient products of iteration t, and dS follows when dP arrives. Order of the tensor work:
+// Pipeline at head dimension 128: scores and dP have barriers of their own, so the exponentials of iteration t+1 (which need
+// the scores only) run under the gradient products of iteration t, and dS follows when dP arrives. Order of the tensor work:
 //   S(t+1) | dV(t) += P(t)^T dO(t) | dK(t) += dS(t)^T Q(t) | dP(t+1)
 // S(t+1) needs Q(t+1), so Q has two stages; dO(t) is free after dV(t), two products before dP(t+1) needs its successor,
-// so at head dimension 128, where shared memory holds seven 32 KB tiles (K, V, 2 Q, dO, P, dS), one stage is enough.
+// so one stage is enough where shared memory holds seven 32 KB tiles (K, V, 2 Q, dO, P, dS).
 // P is single: dV(t) has read it (dv_done) long before the exponentials of t+1 are stored. Until then the two score
 // products of an iteration were one group, which the softmax warps waited for as a whole, and at 128 the loads,
 // the scores, the softmax and the gradient products of an iteration ran one after another: 2 x 2048 tokens of 32 heads,
 // causal, 241 us then and 176 us so. At 64 the kernel above stays: its scores of t+1 and dP are one group ahead of the gradient
 // products, and forward and backward of 2 x 700 tokens of 16 heads take 85.8 us with it, 86.9 with this one.
-template <int DH>
 struct DkvSplitCfg {
-  static constexpr int QS = 2;                        // Q stages
-  static constexpr int OS = (DH == 64) ? 2 : 1;       // dO stages
-  static constexpr int NDS = (DH == 64) ? 2 : 1;      // dS buffers (a bulk store may still read the older one)
+  static constexpr int DH = 128;
+  static constexpr int QS = 2;                        // Q stages; dO, P and dS have one
   static constexpr int T_BYTES = BT * DH * 2;         // one [128 x DH] tile
   static constexpr int PT_BYTES = BT * BT * 2;
-  static constexpr int TILE_BYTES = (2 + QS + OS) * T_BYTES + (1 + NDS) * PT_BYTES;
+  static constexpr int TILE_BYTES = (2 + QS + 1) * T_BYTES + 2 * PT_BYTES;
   static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 256;
   static constexpr int TMEM_COLS = 512;  // S 128 | dP 128 | dK DH | dV DH
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 };
 
-template <int DH>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
-                         const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
-  using Cfg = DkvSplitCfg<DH>;
-  constexpr int NCH = DH / 64;
+                               const __grid_constant__ CUtensorMap tm_ds, const BwdParams p) {
+  using Cfg = DkvSplitCfg;
+  constexpr int DH = Cfg::DH, NCH = DH / 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + Cfg::T_BYTES;
   uint8_t* sQ = sV + Cfg::T_BYTES;                 // QS stages
-  uint8_t* sdO = sQ + Cfg::QS * Cfg::T_BYTES;      // OS stages
-  uint8_t* sPT = sdO + Cfg::OS * Cfg::T_BYTES;
-  uint8_t* sdST = sPT + Cfg::PT_BYTES;             // NDS buffers
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sdST + Cfg::NDS * Cfg::PT_BYTES);
+  uint8_t* sdO = sQ + Cfg::QS * Cfg::T_BYTES;
+  uint8_t* sPT = sdO + Cfg::T_BYTES;
+  uint8_t* sdST = sPT + Cfg::PT_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sdST + Cfg::PT_BYTES);
   uint64_t* kv_full = bars;
   uint64_t* q_full = bars + 1;             // QS
   uint64_t* q_empty = q_full + Cfg::QS;    // QS
-  uint64_t* do_full = q_empty + Cfg::QS;   // OS
-  uint64_t* do_empty = do_full + Cfg::OS;  // OS
-  uint64_t* s_full = do_empty + Cfg::OS;   // scores of t are in tensor memory
+  uint64_t* do_full = q_empty + Cfg::QS;
+  uint64_t* do_empty = do_full + 1;
+  uint64_t* s_full = do_empty + 1;         // scores of t are in tensor memory
   uint64_t* dp_full = s_full + 1;          // dP of t is; every earlier product has completed and dS may be rewritten
   uint64_t* p_full = dp_full + 1;          // P of t is in shared memory (8 warp arrivals), the scores have been read
   uint64_t* ds_full = p_full + 1;          // dS of t is, dP has been read
@@ -435,7 +426,8 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int s = 0; s < Cfg::QS; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
-    for (int s = 0; s < Cfg::OS; ++s) { mbar_init(&do_full[s], 1); mbar_init(&do_empty[s], 1); }
+    mbar_init(do_full, 1);
+    mbar_init(do_empty, 1);
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
     mbar_init(p_full, 8);  // one arrival per softmax warp
@@ -463,8 +455,8 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
         tma_load_2d(sK + c * (BT * 128), &tm_qkv, kv_full, (p.H + kvh) * DH + c * 64, row_base + kv0);
         tma_load_2d(sV + c * (BT * 128), &tm_qkv, kv_full, (p.H + p.Hkv + kvh) * DH + c * 64, row_base + kv0);
       }
-      int qs = 0, os = 0;
-      uint32_t qph = 0, oph = 0;
+      int qs = 0;
+      uint32_t qph = 0;
       for (int t = 0; t < n_iter; ++t) {
         const int head = kvh * group + t / n_qt;
         const int qt = qt_first + t % n_qt;
@@ -475,13 +467,11 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
           tma_load_2d(sQ + qs * Cfg::T_BYTES + c * (BT * 128), &tm_qkv, &q_full[qs], head * DH + c * 64,
                       row_base + qt * BT);
         if (++qs == Cfg::QS) { qs = 0; qph ^= 1; }
-        if (!mbar_wait(&do_empty[os], oph ^ 1, p.status, ST_TIMEOUT_EMPTY)) break;
-        mbar_arrive_expect_tx(&do_full[os], Cfg::T_BYTES);
+        if (!mbar_wait(do_empty, (t & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY)) break;
+        mbar_arrive_expect_tx(do_full, Cfg::T_BYTES);
 #pragma unroll
         for (int c = 0; c < NCH; ++c)
-          tma_load_2d(sdO + os * Cfg::T_BYTES + c * (BT * 128), &tm_do, &do_full[os], head * DH + c * 64,
-                      row_base + qt * BT);
-        if (++os == Cfg::OS) { os = 0; oph ^= 1; }
+          tma_load_2d(sdO + c * (BT * 128), &tm_do, do_full, head * DH + c * 64, row_base + qt * BT);
       }
     }
   } else if (warp == 1) {
@@ -489,10 +479,10 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
       constexpr uint32_t idesc_s = make_idesc_bf16(BT, BT, false, false);   // [q x kv], both K-major
       constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, true, true);     // [kv x dh] = A^T B, both MN-major
       bool ok = mbar_wait(kv_full, 0, p.status, ST_TIMEOUT_FULL);
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aPT = smem_u32(sPT);
-      int qn = 0, on = 0;            // stage and phase of the next score / dP product
-      uint32_t qn_ph = 0, on_ph = 0;
-      int qg = 0, og = 0;            // stage of the next dK / dV product
+      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), adO = smem_u32(sdO), aPT = smem_u32(sPT), adS = smem_u32(sdST);
+      int qn = 0;                    // Q stage and phase of the next score product
+      uint32_t qn_ph = 0;
+      int qg = 0;                    // Q stage of the next dK product
       // D = A B^T over DH, both K-major
       auto score_product = [&](uint32_t d, uint32_t a, uint32_t b) {
 #pragma unroll
@@ -516,42 +506,39 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
         if (++qn == Cfg::QS) { qn = 0; qn_ph ^= 1; }
         return true;
       };
-      auto issue_dp = [&]() -> bool {
-        if (!mbar_wait(&do_full[on], on_ph, p.status, ST_TIMEOUT_FULL)) return false;
+      auto issue_dp = [&](int t) -> bool {
+        if (!mbar_wait(do_full, t & 1, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        // dp_full lets the softmax warps write the next dS buffer: its last bulk store must have been read out
-        if (p.spill_ds) tma_store_wait_read<Cfg::NDS - 1>();
-        score_product(tm_dPT, smem_u32(sdO + on * Cfg::T_BYTES), aV);
+        // dp_full lets the softmax warps write dS again: its last bulk store must have been read out
+        if (p.spill_ds) tma_store_wait_read<0>();
+        score_product(tm_dPT, adO, aV);
         umma_commit(dp_full);
-        if (++on == Cfg::OS) { on = 0; on_ph ^= 1; }
         return true;
       };
-      if (n_iter > 0) ok = ok && issue_s() && issue_dp();
+      if (n_iter > 0) ok = ok && issue_s() && issue_dp(0);
       for (int t = 0; t < n_iter && ok; ++t) {
         const bool more = t + 1 < n_iter;
         if (!mbar_wait(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
         tc_fence_after();
         if (more && !issue_s()) { ok = false; break; }
-        grad_product(tm_dV, aPT, smem_u32(sdO + og * Cfg::T_BYTES), t > 0);
+        grad_product(tm_dV, aPT, adO, t > 0);
         umma_commit(dv_done);
-        umma_commit(&do_empty[og]);
-        if (++og == Cfg::OS) og = 0;
+        umma_commit(do_empty);
         if (!mbar_wait(ds_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
         tc_fence_after();
-        const uint8_t* ds = sdST + (Cfg::NDS == 2 ? (t & 1) : 0) * Cfg::PT_BYTES;
         if (p.spill_ds) {
           // the finished dS tile (bf16, [q rows][kv], scale included) also goes to global memory, where
           // the dQ kernel streams it back instead of recomputing scores
           const int head = kvh * group + t / n_qt;
           const int qt = qt_first + t % n_qt;
-          tma_store_3d(&tm_ds, ds, kv0, qt * BT, b * p.H + head);
-          tma_store_3d(&tm_ds, ds + BT * 128, kv0 + 64, qt * BT, b * p.H + head);
+          tma_store_3d(&tm_ds, sdST, kv0, qt * BT, b * p.H + head);
+          tma_store_3d(&tm_ds, sdST + BT * 128, kv0 + 64, qt * BT, b * p.H + head);
           tma_store_commit();
         }
-        grad_product(tm_dK, smem_u32(ds), smem_u32(sQ + qg * Cfg::T_BYTES), t > 0);
+        grad_product(tm_dK, adS, smem_u32(sQ + qg * Cfg::T_BYTES), t > 0);
         umma_commit(&q_empty[qg]);
         if (++qg == Cfg::QS) qg = 0;
-        if (more && !issue_dp()) { ok = false; break; }
+        if (more && !issue_dp(t + 1)) { ok = false; break; }
       }
       if (ok) umma_commit(done);
       if (p.spill_ds) tma_store_wait<0>();   // the stores are complete before the CTA retires
@@ -570,7 +557,6 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
       const int q0 = qt * BT;
       const int q_idx = q0 + r;
       const float2 sd = __ldg(p.stats + (static_cast<size_t>(b) * p.H + head) * p.S + min(q_idx, p.S - 1));
-      uint8_t* dst_buf = sdST + (Cfg::NDS == 2 ? (t & 1) : 0) * Cfg::PT_BYTES;
       // last visible kv column of this query row inside the tile (-1: row is past the sequence end)
       const bool diag = p.causal && qt == kt;
       int lim = min(diag ? r : BT - 1, p.S - 1 - kv0);
@@ -622,7 +608,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
           mul2(dv[i], dv[i + 1], __uint_as_float(pv[cc * 32 + i]), __uint_as_float(pv[cc * 32 + i + 1]));
           dk[i >> 1] = pack_bf16x2(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1]));
         }
-        store_row32_sw128(dst_buf, r, half * 2 + cc, dk);
+        store_row32_sw128(sdST, r, half * 2 + cc, dk);
       }
       tc_fence_before();
       fence_proxy_async_smem();
@@ -1001,9 +987,8 @@ attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
 template <int DH>
 static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& td, const CUtensorMap& tds, const BwdParams& p,
                       cudaStream_t stream) {
-  constexpr int DKV_SMEM = DH == 64 ? DkvCfg<64>::SMEM_BYTES : DkvSplitCfg<128>::SMEM_BYTES;
-  void (*k1)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const BwdParams);
-  if constexpr (DH == 64) k1 = attention_bwd_dkv_kernel<64>; else k1 = attention_bwd_dkv_split_kernel<128>;
+  constexpr int DKV_SMEM = DH == 64 ? DkvCfg::SMEM_BYTES : DkvSplitCfg::SMEM_BYTES;
+  auto k1 = DH == 64 ? attention_bwd_dkv_kernel : attention_bwd_dkv_split_kernel;
   auto k2 = attention_bwd_dq_kernel<DH>;
   auto k3 = attention_bwd_dq_stream_kernel<DH>;
   static PerDeviceOnce a1, a2, a3;

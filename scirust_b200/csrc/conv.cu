@@ -42,8 +42,9 @@ __global__ void im2col_nhwc_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfl
   col[idx] = v;
 }
 
-// Division of a 31-bit value by a launch constant: one multiply-high and a shift (the magic number rounds up, exact for
-// n < 2^31). The index arithmetic below would otherwise spend several hundred instructions per 16-byte word on
+// Division of a 31-bit value by a launch constant: one multiply-high and a shift, after Granlund and Montgomery, "Division by
+// invariant integers using multiplication" (PLDI 1994): the multiplier 2^(31 + l) / d, l = ceil(log2 d), rounded up, is exact for
+// n < 2^31. The index arithmetic below would otherwise spend several hundred instructions per 16-byte word on
 // 64-bit divisions.
 struct FastDiv {
   uint32_t d, mul, sh;
@@ -648,6 +649,7 @@ extern "C" int sb_bn_bwd_masked(const void* g, const void* x, const float* sum_g
                                                     static_cast<__nv_bfloat16*>(dx), total, C, rows);
   CHECK_LAUNCH();
 }
+// The forms without a mask: entry points of their own in the C ABI.
 extern "C" int sb_colstats(const void* a, const void* b, float* partial, float* s1, float* s2, int rows, int C,
                            void* stream) {
   return sb_colstats_masked(a, b, nullptr, partial, s1, s2, rows, C, stream);

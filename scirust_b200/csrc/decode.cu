@@ -1466,7 +1466,7 @@ decode_attn_kernel(const __grid_constant__ DecodeAttnParams p) {
 // _stream_wins. 64 sequences of 1536-2048 positions, 8 kv heads: 108.5 us above (4.3 TB/s), 87.5 us here (5.4 TB/s).
 // ---------------------------------------------------------------------------
 constexpr int DST_THREADS = 288;         // warps 0-7 consume (two groups of four, every other tile each), warp 8 produces
-constexpr int DST_STAGES_MAX = 10;
+constexpr int DST_STAGES_MAX = 6;        // one query head per kv head; sixteen leave room for four
 constexpr int DST_MAX_B = 1024;          // sequences whose tile offsets fit the shared prefix table
 
 struct DecodeStreamParams {
@@ -1482,8 +1482,8 @@ struct DecodeStreamParams {
   int stages;
 };
 
-template <int DH>
 struct DstCfg {
+  static constexpr int DH = 128;
   static constexpr int NCH = DH / 64;
   static constexpr int TILE_BYTES = DEC_TK * DH * 2;         // K or V of one tile
   // eight warps' partial results of the G live rows; what is left of shared memory holds stages
@@ -1494,16 +1494,16 @@ struct DstCfg {
     return n < DST_STAGES_MAX ? n : DST_STAGES_MAX;
   }
   static constexpr int smem_bytes(int G) { return stages(G) * 2 * TILE_BYTES + fixed_bytes(G); }
-  static_assert(stages(16) >= 4, "a ring of at least four stages");
 };
+static_assert(DstCfg::stages(16) >= 4 && DstCfg::stages(1) == DST_STAGES_MAX, "a ring of four to six stages");
 
 // Tiles of one sequence: an empty one keeps a tile without positions, whose job writes zeros.
 __device__ __forceinline__ int dst_tiles(int len) { return len > 0 ? (len + DEC_TK - 1) / DEC_TK : 1; }
 
-template <int DH>
 __global__ void __launch_bounds__(DST_THREADS, 1)
 decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ DecodeStreamParams p) {
-  using C = DstCfg<DH>;
+  using C = DstCfg;
+  constexpr int DH = C::DH;
   constexpr int KS = DH / 16;                  // k-steps of Q K^T
   constexpr int NB = DH / 8;                   // 8-wide output blocks of P V
   extern __shared__ uint8_t smem_raw[];
@@ -2284,14 +2284,13 @@ extern "C" int sb_decode_attention(const void* q, int ldq, const void* pool, con
   return dh == 64 ? launch_decode_attn<64>(p, grid, STREAM) : launch_decode_attn<128>(p, grid, STREAM);
 }
 
-template <int DH>
 static int launch_decode_stream(const CUtensorMap& tm, DecodeStreamParams p, int grid, cudaStream_t s) {
-  auto kern = decode_attn_stream_kernel<DH>;
   static PerDeviceOnce attr;
-  if (allow_smem(attr, kern, 227 * 1024 - 1024, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
+  if (allow_smem(attr, decode_attn_stream_kernel, 227 * 1024 - 1024, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   const int G = p.H / p.Hkv;
-  p.stages = DstCfg<DH>::stages(G);
-  return launch_dep(kern, dim3(grid), dim3(DST_THREADS), DstCfg<DH>::smem_bytes(G), s, tm, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+  p.stages = DstCfg::stages(G);
+  return launch_dep(decode_attn_stream_kernel, dim3(grid), dim3(DST_THREADS), DstCfg::smem_bytes(G), s, tm, p) == cudaSuccess
+             ? 0 : SB_ERR_LAUNCH;
 }
 
 // The same attention as one balanced stream of KV tiles. pool: n_blocks pages (n_blocks * 2 * Hkv * page < 2^31, base
@@ -2302,7 +2301,7 @@ extern "C" int sb_decode_attention_stream(const void* q, int ldq, const void* po
                                           const int* block_table, int max_blocks, int page, const int* seq_len, int B,
                                           int H, int Hkv, int dh, int max_tiles, float scale, float* part,
                                           unsigned int* counters, void* out, int ldo, int* status, void* stream) {
-  if (B <= 0 || B > DST_MAX_B || H <= 0 || Hkv <= 0 || (H % Hkv) || H / Hkv > 16 || dh != 128 ||
+  if (B <= 0 || B > DST_MAX_B || H <= 0 || Hkv <= 0 || (H % Hkv) || H / Hkv > 16 || dh != DstCfg::DH ||
       n_blocks < 1 || max_tiles < 1 || (ldq & 1) || !status)
     return SB_ERR_ARG;
   if (page != 8 && page != 16 && page != 32 && (page < 64 || page % 64)) return SB_ERR_ARG;
@@ -2320,7 +2319,7 @@ extern "C" int sb_decode_attention_stream(const void* q, int ldq, const void* po
   // a CTA with less than two tiles has nothing to overlap; more CTAs than that only add pieces to merge
   int grid = (max_tiles + 1) / 2;
   if (grid > num_sms()) grid = num_sms();
-  return launch_decode_stream<128>(tm, p, grid, STREAM);
+  return launch_decode_stream(tm, p, grid, STREAM);
 }
 
 // logits: fp32 [rows, V]. pval/pidx: rows * ceil(V/4096) scratch. out_tokens: int64 [rows].
