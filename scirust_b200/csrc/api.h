@@ -95,7 +95,8 @@ int sb_gemm_skinny(const void* X, int ldx, const void* W, int ldw, void* C, int 
 // gemm_tcgen05.cu
 size_t sb_gemm_balanced_workspace_floats();
 int sb_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, int splits, void* workspace, int bn, int* status, void* stream_);
-int sb_conv_gemm(int mode, const void* a, const void* b, void* out, void* keep, int B, int H, int W, int C, int oc, int k, int stride, int pad, int OH, int OW, int splits, void* workspace, int* status, void* stream_);
+int sb_conv_gemm(int mode, const void* a, const void* b, void* out, int B, int H, int W, int C, int oc, int k, int stride, int pad, int OH, int OW, int splits, void* workspace, int* status, void* stream_);
+int sb_conv_fprop_keep(const void* x, const void* w, void* y, void* keep, int B, int H, int W, int C, int oc, int k, int stride, int pad, int OH, int OW, int splits, void* workspace, int* status, void* stream_);
 
 // gemm_w8_tcgen05.cu
 int sb_gemm_w8(const void* A, const void* Q, const float* scale, void* C, const void* R, int M, int N, int K, int lda, int ldq, int ldc, int ldr, int splits, void* workspace, int* status, void* stream_);

@@ -561,15 +561,14 @@ extern "C" int sb_gemm_bf16(const void* A, const void* B, void* C, const void* R
 //   mode 2: out = dw [oc, k*k*C]    from a = dy [B*OH*OW, oc], b = x
 //   mode 3: out = dx [B*H*W, C]     from a = dy, b = weights; stride 1
 // splits > 1: split-K over `workspace` (splits * rows * columns of out, floats). Shapes whose pixel rows do not tile 128
-// (mode 2: 64) pixels are refused with SB_ERR_ARG. keep (mode 1, optional): gets a copy of x for the weight gradient.
-extern "C" int sb_conv_gemm(int mode, const void* a, const void* b, void* out, void* keep, int B, int H, int W, int C, int oc, int k,
-                            int stride, int pad, int OH, int OW, int splits, void* workspace, int* status,
-                            void* stream_) {
+// (mode 2: 64) pixels are refused with SB_ERR_ARG. keep (mode 1, optional): gets a copy of x.
+static int conv_gemm(int mode, const void* a, const void* b, void* out, void* keep, int B, int H, int W, int C, int oc, int k,
+                     int stride, int pad, int OH, int OW, int splits, void* workspace, int* status, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (mode < 1 || mode > 3 || B <= 0 || C <= 0 || oc <= 0 || (C & 63) || (oc & 63) || k < 1 || stride < 1 || pad < 0 || !status)
     return SB_ERR_ARG;
   if (OH != (H + 2 * pad - k) / stride + 1 || OW != (W + 2 * pad - k) / stride + 1 || OH < 1 || OW < 1) return SB_ERR_ARG;
-  if ((mode == 3 && stride != 1) || (keep && mode != 1)) return SB_ERR_ARG;
+  if (mode == 3 && stride != 1) return SB_ERR_ARG;
   if (reinterpret_cast<uintptr_t>(out) & 15) return SB_ERR_ALIGN;
   const int taps = k * k, kp = taps * C;
   const long long pix_o = static_cast<long long>(B) * OH * OW, pix_i = static_cast<long long>(B) * H * W;
@@ -627,4 +626,18 @@ extern "C" int sb_conv_gemm(int mode, const void* a, const void* b, void* out, v
     if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   }
   return 0;
+}
+
+extern "C" int sb_conv_gemm(int mode, const void* a, const void* b, void* out, int B, int H, int W, int C, int oc, int k,
+                            int stride, int pad, int OH, int OW, int splits, void* workspace, int* status,
+                            void* stream_) {
+  return conv_gemm(mode, a, b, out, nullptr, B, H, W, C, oc, k, stride, pad, OH, OW, splits, workspace, status, stream_);
+}
+
+// Mode 1 with a copy of x into keep [B*H*W, C], for a weight gradient that is taken later.
+extern "C" int sb_conv_fprop_keep(const void* x, const void* w, void* y, void* keep, int B, int H, int W, int C, int oc, int k,
+                                  int stride, int pad, int OH, int OW, int splits, void* workspace, int* status,
+                                  void* stream_) {
+  if (!keep) return SB_ERR_ARG;
+  return conv_gemm(1, x, w, y, keep, B, H, W, C, oc, k, stride, pad, OH, OW, splits, workspace, status, stream_);
 }

@@ -65,7 +65,8 @@ def unpack_conv_weight(wp: torch.Tensor, in_c: int, k: int) -> torch.Tensor:
     return wp[:, : k * k * in_c].reshape(oc, k, k, in_c).permute(0, 3, 1, 2).reshape(oc, in_c * k * k)
 
 
-_lib.register("sb_conv_gemm", [i32, vp, vp, vp, vp] + [i32] * 11 + [vp, vp, vp])
+_lib.register("sb_conv_gemm", [i32, vp, vp, vp] + [i32] * 11 + [vp, vp, vp])
+_lib.register("sb_conv_fprop_keep", [vp, vp, vp, vp] + [i32] * 11 + [vp, vp, vp])
 _FPROP, _WGRAD, _DGRAD = 1, 2, 3
 
 
@@ -94,8 +95,12 @@ def _conv_gemm(mode, a, b, geom, oc, k, stride, pad, OH, OW, keep=None):
     tiles = ((M + 127) // 128) * ((N + 255) // 256)
     splits = max(1, min(G.num_sms(a.device) // tiles, (K + 63) // 64 // 8, 64))
     ws = G._workspace(splits * M * N, a.device) if splits > 1 else None
-    _lib.call("sb_conv_gemm", mode, a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(keep), geom.B, geom.H, geom.W,
-              geom.C, oc, k, stride, pad, OH, OW, splits, _lib.ptr(ws), _lib.status_word(a.device).data_ptr(), _lib.stream())
+    rest = (geom.B, geom.H, geom.W, geom.C, oc, k, stride, pad, OH, OW, splits, _lib.ptr(ws),
+            _lib.status_word(a.device).data_ptr(), _lib.stream())
+    if keep is None:
+        _lib.call("sb_conv_gemm", mode, a.data_ptr(), b.data_ptr(), out.data_ptr(), *rest)
+    else:
+        _lib.call("sb_conv_fprop_keep", a.data_ptr(), b.data_ptr(), out.data_ptr(), keep.data_ptr(), *rest)
     G.launch_count += 2 if splits > 1 else 1
     return out
 
