@@ -138,12 +138,18 @@ def _auto_splits(N, K, cols, M=1, quant=False):
     kernel's 64 KB: 16 bytes per k (8 rows of 16-bit values) in the tensor-core kernels, (K / splits) rows x
     {1,2,4,8} floats in the FMA kernels that SB_GEMV_FMA=1 selects."""
     ctas = (N + cols - 1) // cols
-    # at least 128 rows of k per split, and at most 18 of them with int8 weights: the finish reads one partial per split, and
-    # past that it costs more than the shorter stream saves (us, one row: bf16 2816 x 1024 at 44 splits 8.0, at 22 6.9; int8
-    # 4096 x 4096 at 37 14.4, at 18 12.4; five rows: bf16 2816 x 1024 20.7 / 14.0, int8 4096 x 6144 at 24 29.4, at 12 23.5)
-    s = max(1, min(148 * 2 // max(ctas, 1), K // 128))
+    # at least 128 rows of k per split: the finish reads one partial per split, row and column, and past that it costs more than
+    # the shorter stream saves (us, one row: bf16 2816 x 1024 at 44 splits 8.0, at 22 6.9; five rows 20.7 / 14.0). One row has
+    # the cheapest finish: below 2048 rows of k it takes 96 a split, and up to eight splits of 64 (512 x 2048 int8 at 4 splits
+    # 7.6, at 8 7.2; 1376 x 1024 at 10 8.8, at 14 8.6).
+    rows = K // (96 if M == 1 and K < 2048 else 128)
+    s = max(1, min(148 * 2 // max(ctas, 1), max(rows, min(8, K // 64)) if M == 1 else rows))
     if quant:
-        s = min(s, 18)
+        # int8 columns come 512 to a CTA, so narrow matrices would get many splits: 18 is where the finish outweighs them for one
+        # row and up to 16384 rows of k (4096 x 4096 at 37 14.4, at 18 12.4; 14336 x 3584 at 18 19.1, at 36 19.2; eight rows
+        # 4096 x 1024 at 64 65, at 18 26); beyond that a split of 18 is a long stream by itself, and one row takes 640 of k at
+        # least (28672 x 256 at 18 25.5, at 48 14.4; 28672 x 2048 28.7 / 23.5, x 3584 at 18 30.2, at 42 25.7)
+        s = min(s, K // 640 if M == 1 and K > 16384 else 18)
     if ctas > 148 * 2 and not quant:
         # several waves of column blocks (an LM head): eight k-splits keep more CTAs streaming at once and shorten
         # the tail (4096 x 128256: 213 us with one split, 176 us with eight)

@@ -78,3 +78,13 @@ def test_kernel_attributes_are_set_for_every_device(tmp_path):
 ])
 def test_convolution_without_patch_matrix(B, H, W, Cin, oc, k, stride, pad, implicit):
     assert C.implicit_ok(C.ConvGeom(B, H, W, Cin), oc, k, stride, pad) is implicit
+
+
+@pytest.mark.parametrize("K,N,M,quant,splits", [
+    (4096, 4096, 1, True, 18), (14336, 4096, 1, True, 18), (28672, 2048, 1, True, 44), (28672, 3584, 1, True, 42),
+    (28672, 2048, 8, True, 18), (512, 2048, 1, True, 8), (512, 2048, 8, True, 4), (1376, 1024, 1, True, 14),
+    (2816, 1024, 1, False, 22), (1024, 1024, 1, False, 10), (4096, 6144, 1, False, 12), (64, 256, 1, False, 1),
+    (4096, 128256, 1, False, 8), (73728, 256, 8, True, 18), (98304, 256, 8, True, 24),
+])
+def test_splits_of_the_weight_stream(K, N, M, quant, splits):
+    assert D._auto_splits(N, K, 512 if quant else 256, M, quant) == splits
