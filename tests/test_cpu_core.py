@@ -22,7 +22,8 @@ from scirust_b200.numerics import reproducible as R
 # golden files of the reference implementation: a checkout beside this repository, or SCIRUST_REFERENCE_DIR
 REF = os.environ.get("SCIRUST_REFERENCE_DIR") or os.path.normpath(
     os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "..", "reference"))
-need_ref = pytest.mark.skipif(not os.path.isdir(REF), reason="reference tree not mounted")
+SHIPPED = f"{REF}/scirust-sciagent/checkpoints/small-20M/final/model.safetensors"
+need_ref = pytest.mark.skipif(not os.path.isfile(SHIPPED), reason="reference tree not mounted")
 
 
 # ------------------------------------------------------------------ RNG
@@ -67,7 +68,7 @@ def test_safetensors_layout_and_errors():
 
 @need_ref
 def test_safetensors_roundtrip_of_shipped_checkpoint_is_byte_identical():
-    raw = open(f"{REF}/scirust-sciagent/checkpoints/small-20M/final/model.safetensors", "rb").read()
+    raw = open(SHIPPED, "rb").read()
     sd = ST.deserialize(raw)
     assert len(sd) == 38 and tuple(sd["sciagent.embed.weight"].shape) == (8192, 128)
     assert ST.serialize([(k, sd[k]) for k in ST.header_order(raw)]) == raw

@@ -120,7 +120,8 @@ def test_warmup_cosine_schedule():
     assert s.lr_at(60) == pytest.approx(0.55, abs=1e-6) and s.lr_at(500) == pytest.approx(0.1)
 
 
-@pytest.mark.skipif(not os.path.isdir(REF), reason="reference tree not mounted")
+@pytest.mark.skipif(not os.path.isfile(f"{REF}/scirust-sciagent/checkpoints/small-20M/final/model.safetensors"),
+                    reason="reference tree not mounted")
 def test_shipped_reference_checkpoint_predicts_source_text():
     from scirust_b200.tokenizer import BpeTokenizer
     m, meta = CK.load_sciagent_checkpoint(f"{REF}/scirust-sciagent/checkpoints/small-20M/final")
