@@ -36,8 +36,8 @@
 // stages; V is a ring of two half tiles of 64 kv rows, because the products consume V row by row: the first half is
 // free again before the second tile's P V ends, and its successor lands while the next scores run. With three
 // whole-tile slots for K and V together, every block would wait about a load latency for its K. Against the one-tile
-// kernel (scores, softmax and P V of a block one after another): 5000 tokens, 32 heads, causal 422 -> 266 us (486 ->
-// 772 TFLOP/s), 2 x 2048 tokens 164 -> 110 us.
+// kernel (scores, softmax and P V of a block one after another): 5000 tokens, 32 heads, causal 422 -> 278 us (486 ->
+// 737 TFLOP/s), 2 x 2048 tokens 164 -> 108 us.
 //
 // Warps: 0 TMA producer, 1 MMA issuer, 2-5 softmax of tile 0, 6-9 softmax of tile 1.
 #include "sm100_ptx.cuh"
