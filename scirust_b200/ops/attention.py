@@ -22,8 +22,8 @@ _lib.register("sb_attention_bwd", [_lib.vp, _lib.vp, _lib.vp, _lib.vp, _lib.vp, 
                                    _lib.i32, _lib.i32, _lib.i32, _lib.i32, _lib.i32, _lib.i32, _lib.f32,
                                    _lib.i32, _lib.vp, _lib.vp])
 
-# The forward pass runs the kernel with two query tiles per CTA (output accumulator kept in tensor memory,
-# rescaled only when a row maximum grows by more than 2^8); SB_ATT_FWD=single selects the one-tile kernel.
+# The forward pass has a kernel with two query tiles per CTA, whose output accumulator stays in tensor memory, and one with one;
+# sizes choose (_two_tiles_win). SB_ATT_FWD=single selects the one-tile kernel throughout.
 FWD_TWO_TILES = os.environ.get("SB_ATT_FWD", "pair") != "single"
 
 
