@@ -24,6 +24,7 @@
 // main loop of tile i+1. K is walked in a fixed order, so results are bitwise
 // repeatable; split-K writes fp32 partials that a second kernel adds in split order.
 #include <stdio.h>
+#include <algorithm>
 #include "sm100_ptx.cuh"
 #include "api.h"
 #include "per_device.h"
@@ -555,6 +556,20 @@ extern "C" int sb_gemm_bf16(const void* A, const void* B, void* C, const void* R
   return 0;
 }
 
+// A plain copy of 16-byte words, four in flight per thread: as a kernel it costs the host half of what cudaMemcpyAsync does.
+__global__ void __launch_bounds__(256) copy_words_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t words) {
+  const size_t step = static_cast<size_t>(gridDim.x) * 1024;
+  for (size_t i = static_cast<size_t>(blockIdx.x) * 1024 + threadIdx.x; i < words; i += step) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * 256 < words) v[u] = __ldg(src + i + u * 256);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * 256 < words) dst[i + u * 256] = v[u];
+  }
+}
+
 // One product of an NHWC convolution (square k x k filter) without a patch matrix; the packed weights are [oc, k*k*C] in
 // (kh, kw, c) order, C % 64 == 0, oc % 64 == 0.
 //   mode 1: out = y [B*OH*OW, oc]   from a = x, b = weights
@@ -569,7 +584,7 @@ static int conv_gemm(int mode, const void* a, const void* b, void* out, void* ke
     return SB_ERR_ARG;
   if (OH != (H + 2 * pad - k) / stride + 1 || OW != (W + 2 * pad - k) / stride + 1 || OH < 1 || OW < 1) return SB_ERR_ARG;
   if (mode == 3 && stride != 1) return SB_ERR_ARG;
-  if (reinterpret_cast<uintptr_t>(out) & 15) return SB_ERR_ALIGN;
+  if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(keep)) & 15) return SB_ERR_ALIGN;
   const int taps = k * k, kp = taps * C;
   const long long pix_o = static_cast<long long>(B) * OH * OW, pix_i = static_cast<long long>(B) * H * W;
   if (pix_o >= (1ll << 31) || pix_i >= (1ll << 31)) return SB_ERR_TOO_LARGE;
@@ -608,8 +623,12 @@ static int conv_gemm(int mode, const void* a, const void* b, void* out, void* ke
     if (!rc) rc = make_tmap_2d_bf16(&tb, b, kp, oc, kp, 64, BK);
   }
   if (rc) return rc;
-  if (keep && cudaMemcpyAsync(keep, a, static_cast<size_t>(pix_i) * C * 2, cudaMemcpyDeviceToDevice, stream) != cudaSuccess)
-    return SB_ERR_LAUNCH;
+  if (keep) {
+    const size_t words = static_cast<size_t>(pix_i) * C / 8;
+    copy_words_kernel<<<static_cast<unsigned>(std::min<size_t>((words + 1023) / 1024, 8 * num_sms())), 256, 0, stream>>>(
+        static_cast<const uint4*>(a), static_cast<uint4*>(keep), words);
+    if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
+  }
   const long long tiles = static_cast<long long>((p.M + BM - 1) / BM) * ((p.N + bn - 1) / bn) * splits;
   const int grid = tiles < num_sms() ? static_cast<int>(tiles) : num_sms();
   if (mode == 1) rc = bn == 128 ? launch_gemm<128, false, false, CONV_FPROP>(ta, tb, p, grid, stream)

@@ -115,7 +115,7 @@ class _Conv(torch.autograd.Function):
         if ctx.implicit:
             # a copy, as the patch matrix is one: the caller's tensor may be written before the backward pass, also by
             # kernels that its version counter does not see (128 x 32 x 32 x 64: 7 us, where the patch matrix took 86)
-            keep = _lib.empty(x.shape, BF, x.device) if want_dw else None
+            keep = torch.empty_like(x) if want_dw else None
             ctx.save_for_backward(keep, wp)
             return _conv_gemm(_FPROP, x, wp, geom, wp.shape[0], k, stride, pad, OH, OW, keep)
         Kp = wp.shape[1]
