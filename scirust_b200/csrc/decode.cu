@@ -18,6 +18,7 @@
 #include <cstdlib>
 #include "sm100_ptx.cuh"
 #include "peer_sync.cuh"
+#include "dependent.cuh"
 
 namespace sb {
 
@@ -27,15 +28,6 @@ __device__ __forceinline__ uint32_t dpack(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-
-// Programmatic dependent launch: a kernel launched with the stream-serialization attribute may start
-// while its predecessor in the stream is still draining. Work that does not depend on the
-// predecessor (weight prefetch, barrier set-up) runs at once; pdl_wait() returns when the predecessor
-// has completed and its writes are visible, and must precede every read of its results and every
-// global write. pdl_trigger() tells the scheduler that this CTA no longer minds dependents being
-// co-scheduled. Both are no-ops in a kernel launched without the attribute.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // GEMV / skinny GEMM: Y[M,N] = f(X)[M,K] * W[K,N] (* scale[n]) (+ R), M <= MB <= 8, W streamed once.
@@ -298,6 +290,7 @@ gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
     fence_barrier_init();
   }
   __syncthreads();
+  if (p.coll.W <= 1 && p.amax.W <= 1) pdl_trigger();   // a kernel that waits for its peers keeps the GPU to itself
 
   float acc[MB][VEC];
 #pragma unroll
@@ -309,6 +302,7 @@ gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
     // ------------------------------ producer ------------------------------
     // the map is over 16-bit words: x = byte offset of the CTA's columns / 2 (a multiple of 256)
     const int x0 = col0 * ESZ / 2;
+    pdl_wait();
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
       if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
@@ -319,7 +313,6 @@ gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
       }
       __syncwarp();
     }
-    pdl_wait();   // this warp writes results below
   } else {
     // ------------------------------ consumers -----------------------------
     pdl_wait();   // X, the residual and the workspace belong to the previous kernel until here
@@ -438,10 +431,6 @@ gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
   // every tile has been consumed (or a wait gave up and no copy is read any more): reuse the ring
   // for the cross-warp reduction, one output row at a time, warps added in warp order
   __syncthreads();
-  // the weight stream of this CTA is done: the next kernel in the stream may be co-scheduled, so that
-  // its weight prefetch overlaps this kernel's reduction tail. (Triggering at kernel start instead
-  // was measured slower: 3.84 against 3.68 ms per Llama-3-8B-shape token without any overlap.)
-  pdl_trigger();
   float* buf = reinterpret_cast<float*>(tiles);  // [8 warps][32 lanes][VEC]
   const bool direct = gridDim.y == 1;
 #pragma unroll
@@ -549,6 +538,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     fence_barrier_init();
   }
   __syncthreads();
+  if (p.coll.W <= 1 && p.amax.W <= 1) pdl_trigger();   // a kernel that waits for its peers keeps the GPU to itself
 
   float acc[2][MBLK][4];
 #pragma unroll
@@ -561,6 +551,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 
   if (warp == 8) {
     // ------------------------------ producer ------------------------------
+    pdl_wait();
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
       if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
@@ -574,7 +565,6 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       }
       __syncwarp();
     }
-    pdl_wait();
   } else {
     // ------------------------------ consumers -----------------------------
     pdl_wait();   // X, the residual and the workspace belong to the previous kernel until here
@@ -722,7 +712,6 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     }
   }
   __syncthreads();
-  pdl_trigger();
   const bool direct = gridDim.y == 1;
   const bool coll = p.coll.W > 1;
   const bool amax = p.amax.out_tokens != nullptr;
@@ -837,6 +826,7 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     fence_barrier_init();
   }
   __syncthreads();
+  if (p.coll.W <= 1 && p.amax.W <= 1) pdl_trigger();   // a kernel that waits for its peers keeps the GPU to itself
 
   float acc[4][MBLK][4];
 #pragma unroll
@@ -849,6 +839,7 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 
   if (warp == 8) {
     // ------------------------------ producer ------------------------------
+    pdl_wait();
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
       if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
@@ -862,7 +853,6 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
       __syncwarp();
     }
-    pdl_wait();
   } else {
     // ------------------------------ consumers -----------------------------
     pdl_wait();   // X, the residual and the workspace belong to the previous kernel until here
@@ -1027,7 +1017,6 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
   }
   __syncthreads();
-  pdl_trigger();
   const bool direct = gridDim.y == 1;
   const bool coll = p.coll.W > 1;
   const bool amax = p.amax.out_tokens != nullptr;
@@ -1128,14 +1117,13 @@ __global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, 
 // Decode-step fusion of RoPE and the cache append: rotates the q and k heads of each new token in
 // place (interleaved pairs, head-local frequency, position pos[t]) and writes the rotated k and the
 // v heads into the paged pool. One block per token.
-__global__ void rope_kv_append_kernel(__nv_bfloat16* __restrict__ qkv, int ld, int H, int Hkv, int dh,
-                                      const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                      __nv_bfloat16* __restrict__ pool, const int* __restrict__ block_table,
-                                      int max_blocks, int page, const int* __restrict__ seq_of,
-                                      const int* __restrict__ pos, int n_tok) {
+__global__ void rope_kv_append_kernel(__nv_bfloat16* qkv, int ld, int H, int Hkv, int dh, const float* cos_t,
+                                      const float* sin_t, __nv_bfloat16* pool, const int* block_table, int max_blocks,
+                                      int page, const int* seq_of, const int* pos, int n_tok) {
   // grid = (n_tok, H + 2*Hkv): one CTA per head of one token, one thread per (even, odd) pair
   const int t = blockIdx.x, head = blockIdx.y;
   if (t >= n_tok) return;
+  pdl_trigger();
   pdl_wait();
   const int b = seq_of[t], p = pos[t];
   const int half = dh >> 1;
@@ -1222,6 +1210,7 @@ decode_attn_kernel(const __grid_constant__ DecodeAttnParams p) {
   const int H = p.H, Hkv = p.Hkv, G = H / Hkv, n_splits = p.n_splits;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int quad = lane >> 2, tq = lane & 3;
+  pdl_trigger();
   pdl_wait();
   const int L = p.seq_len[b];
   const int per_split = ((L + n_splits - 1) / n_splits + DEC_TK - 1) / DEC_TK * DEC_TK;
@@ -1356,7 +1345,6 @@ decode_attn_kernel(const __grid_constant__ DecodeAttnParams p) {
   }
   cp_async_wait<0>();
   __syncthreads();
-  pdl_trigger();   // the output projection may start prefetching its weights
 
   // ---- merge the four warps in warp order ----
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
@@ -1522,6 +1510,7 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
     for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 8); }
     fence_barrier_init();
   }
+  pdl_trigger();
   pdl_wait();
   if (warp == 0) {
     int base = 0;
@@ -1862,7 +1851,6 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
     asm volatile("bar.sync 1, 256;" ::: "memory");   // the merge buffers and s_last are free again
     u += t_end - t_beg;
   }
-  pdl_trigger();
 }
 
 // ---------------------------------------------------------------------------
@@ -1993,24 +1981,10 @@ using namespace sb;
 #define STREAM static_cast<cudaStream_t>(stream)
 #define CHECK_LAUNCH() return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH
 
-static bool g_pdl = false;
+static bool g_pdl = true;
+bool sb::dependent_launches() { return g_pdl; }
 
-// Launch with (or without) the programmatic-stream-serialization attribute.
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_dep(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                              Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = g_pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
-}
-
-// Switches programmatic dependent launch of the decode-path kernels (GEMV, RoPE+append,
-// flash-decode) on or off for this process; off by default.
+// Switches programmatic dependent launch of the decode-path kernels off (0) or on again for this process.
 extern "C" int sb_set_pdl(int on) { g_pdl = on != 0; return 0; }
 
 namespace sb {

@@ -15,6 +15,7 @@
 #include "sm100_ptx.cuh"
 #include "api.h"
 #include "per_device.h"
+#include "dependent.cuh"
 
 namespace sb {
 
@@ -253,8 +254,9 @@ __global__ void quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int ld
 // unrolled words only cost the threads that have none (1024 rows of 1024: 3.2 and 7.0 us, 4096 of 8192: 42.7 and 47.5).
 template <int THREADS, int KEEP>
 __global__ void __launch_bounds__(THREADS)
-quantize_rows_vec8_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int8_t* __restrict__ q, int ldq,
-                          float* __restrict__ sx, int K) {
+quantize_rows_vec8_kernel(const __nv_bfloat16* x, int ldx, int8_t* q, int ldq, float* sx, int K) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float s_max[THREADS / 32];
   const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * ldx);
@@ -317,8 +319,8 @@ extern "C" int sb_quantize_rows(const void* x, int ldx, void* xq, int ldq, float
       (reinterpret_cast<uintptr_t>(xq) & 7) == 0) {
     const bool keep = K >= 8192 && M <= 1024;
     auto kern = keep ? quantize_rows_vec8_kernel<512, 4> : quantize_rows_vec8_kernel<256, 0>;
-    kern<<<M, keep ? 512 : 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x), ldx, static_cast<int8_t*>(xq), ldq, sx, K);
-    return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+    return launch_dep(kern, dim3(M), dim3(keep ? 512 : 256), 0, STREAM, static_cast<const __nv_bfloat16*>(x), ldx,
+                      static_cast<int8_t*>(xq), ldq, sx, K) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
   }
   quantize_rows_kernel<<<(M + 7) / 8, 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x), ldx,
                                                         static_cast<int8_t*>(xq), ldq, sx, M, K);

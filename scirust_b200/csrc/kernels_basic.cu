@@ -15,6 +15,8 @@
 #include <stdint.h>
 #include "api.h"
 
+#include "dependent.cuh"
+
 namespace sb {
 
 __device__ __forceinline__ float bflo(uint32_t v) { return __uint_as_float(v << 16); }
@@ -91,9 +93,10 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
 // row pays its loads one after another. Warp a computes accumulator a of the kernel above and the eight are added in
 // index order, so the results are the same bits. 64 rows of 4096: 7.2 us above, 2.3 us here.
 __global__ void __launch_bounds__(256)
-rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                       __nv_bfloat16* __restrict__ y, float* __restrict__ inv_rms, int cols, int ldx, int ldy,
-                       float eps) {
+rmsnorm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y, float* inv_rms, int cols,
+                       int ldx, int ldy, float eps) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float s_acc[8][32];
   const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const __nv_bfloat16* xr = x + static_cast<size_t>(row) * ldx;
@@ -105,7 +108,7 @@ rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16*
     const int c = threadIdx.x * 8 + i * 2048;
     if (c < cols) {
       kept[i] = *reinterpret_cast<const uint4*>(xr + c);
-      kw[i] = __ldg(reinterpret_cast<const uint4*>(w + c));
+      kw[i] = *reinterpret_cast<const uint4*>(w + c);
     }
   }
 #pragma unroll
@@ -340,8 +343,9 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, int ld, int rows, int
 // ---------------------------------------------------------------------------
 // SwiGLU over a fused [gate | up] activation: gu is [rows, 2*ff], h is [rows, ff].
 // ---------------------------------------------------------------------------
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, int rows,
-                                  int ff) {
+__global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* h, int rows, int ff) {
+  pdl_trigger();
+  pdl_wait();
   const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int per_row = ff >> 3;
   if (idx >= static_cast<size_t>(rows) * per_row) return;
@@ -932,10 +936,9 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* inv_
   if (rows <= 0 || cols <= 0 || (cols & 7) || (ldx & 7) || (ldy & 7)) return SB_ERR_ARG;
   if (!al16(x) || !al16(w) || !al16(y)) return SB_ERR_ALIGN;
   if (rms_few_rows(rows, cols)) {
-    rmsnorm_fwd_row_kernel<<<rows, 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x),
-                                                     static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
-                                                     inv_rms, cols, ldx, ldy, eps);
-    CHECK_LAUNCH();
+    return launch_dep(rmsnorm_fwd_row_kernel, dim3(rows), dim3(256), 0, STREAM, static_cast<const __nv_bfloat16*>(x),
+                      static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y), inv_rms, cols, ldx, ldy,
+                      eps) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
   }
   const int wpb = 4;
   rmsnorm_fwd_kernel<<<(rows + wpb - 1) / wpb, wpb * 32, 0, STREAM>>>(
@@ -991,9 +994,9 @@ extern "C" int sb_rope(void* x, int ld, int rows, int n_heads, int dh, int seq_l
 extern "C" int sb_swiglu_fwd(const void* gu, void* h, int rows, int ff, void* stream) {
   if (rows <= 0 || (ff & 7) || !al16(gu) || !al16(h)) return SB_ERR_ARG;
   const size_t total = static_cast<size_t>(rows) * (ff >> 3);
-  swiglu_fwd_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, STREAM>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), rows, ff);
-  CHECK_LAUNCH();
+  return launch_dep(swiglu_fwd_kernel, dim3(static_cast<unsigned>((total + 255) / 256)), dim3(256), 0, STREAM,
+                    static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(h), rows, ff) == cudaSuccess
+             ? 0 : SB_ERR_LAUNCH;
 }
 extern "C" int sb_swiglu_bwd(const void* gu, const void* dh, void* dgu, int rows, int ff, void* stream) {
   if (rows <= 0 || (ff & 7) || !al16(gu) || !al16(dh) || !al16(dgu)) return SB_ERR_ARG;

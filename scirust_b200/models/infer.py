@@ -265,8 +265,7 @@ class InferenceEngine:
 
     def _step_eager(self, B, max_len, sampler=None, want_logits=False, stream=None):
         torch.add(self.cache.seq_len[:B], 1, out=self._len_plus1[:B])
-        with D.dependent_launch(self.dev.type == "cuda"):
-            done = self._decode_body(B, max_len, greedy=sampler is None and not want_logits, stream=stream)
+        done = self._decode_body(B, max_len, greedy=sampler is None and not want_logits, stream=stream)
         if done:
             pass
         elif sampler is None:

@@ -42,24 +42,18 @@ _lib.register("sb_set_pdl", [i32])
 
 
 class dependent_launch:
-    """Context manager: launch the decode-path kernels (GEMV, RoPE+append, flash-decode) inside the
-    block with programmatic dependent launch, so each kernel's weight prefetch overlaps the tail of
-    its predecessor. Only for call chains whose weights are not produced by the preceding kernel.
-    Off unless ``SB_PDL=1``: with the 64 KB weight ring (three CTAs per SM) the early-scheduled
-    dependents measured slower than plain stream order (4.85 against 3.69 ms per token at
-    Llama-3-8B shape); with the earlier 96 KB ring it gained 5 %."""
+    """Context manager of earlier versions, kept for its callers; it does nothing. The decode-path kernels are launched with
+    programmatic dependent launch wherever they run: a kernel's CTAs start while its predecessor drains and read nothing
+    before it has completed, so the order that a program sees is plain stream order (csrc/dependent.cuh). A decoder layer of
+    Llama-3-8B shape, replayed from a graph: one row 110.8 -> 104.4 us, 16 int8 rows 127.5 -> 119.2, 64 rows 223 -> 215."""
 
     def __init__(self, enabled: bool = True):
-        self.enabled = enabled and os.environ.get("SB_PDL", "0") == "1"
+        self.enabled = enabled
 
     def __enter__(self):
-        if self.enabled:
-            _lib.call("sb_set_pdl", 1)
         return self
 
     def __exit__(self, *exc):
-        if self.enabled:
-            _lib.call("sb_set_pdl", 0)
         return False
 
 

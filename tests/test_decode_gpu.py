@@ -4,6 +4,7 @@ import torch
 
 from scirust_b200.models import GQADecoder, SciAgentConfig
 from scirust_b200.models.infer import InferenceEngine, reference_generate
+from scirust_b200 import ops
 from scirust_b200.ops import _lib, decode as D
 
 pytestmark = pytest.mark.gpu
@@ -118,7 +119,6 @@ def test_lm_head_fused_with_argmax_equals_gemv_then_argmax(quant, M, K, N, split
         assert torch.equal(torch.isnan(lg2), nan) and torch.equal(lg2[~nan], lg[~nan])
     if not quant:
         assert got.tolist() == [0] * M
-    from scirust_b200.ops import _lib
     _lib.check_status(torch.device("cuda"))
 
 
@@ -175,7 +175,6 @@ def test_w8a8_gemm_on_integer_tensor_cores_is_exact(M, K, N, splits):
     assert torch.equal(again, got)                        # split-K adds integers: same bits
     full = x.float() @ w.float() + r.float()
     assert (got.float() - full).abs().max().item() <= 0.04 * full.abs().max().item()
-    from scirust_b200.ops import _lib
     _lib.check_status(torch.device("cuda"))
 
 
@@ -211,7 +210,6 @@ def test_skinny_weight_streaming_gemm_matches_reference(quant, M, K, N, splits):
         assert torch.equal(D.matmul_skinny(x, w, residual=r, splits=splits), got)
         plain = D.matmul_skinny(x, w, splits=1)
         assert (plain.float() - x.float() @ w.float()).abs().max().item() <= 0.02 * max(1.0, (x.float() @ w.float()).abs().max().item())
-    from scirust_b200.ops import _lib
     _lib.check_status(torch.device("cuda"))
 
 
@@ -262,7 +260,6 @@ def test_paged_decode_attention_stream(dh, H, Hkv, page, monkeypatch):
         assert torch.equal(out, D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, max_len=longest))
         one = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, n_splits=1)
         assert (out.float() - one.float()).abs().max().item() < 2e-2
-    from scirust_b200.ops import _lib
     _lib.check_status(torch.device("cuda"))
 
 
@@ -280,7 +277,6 @@ def test_decode_attention_stream_repeats_under_load(monkeypatch):
     for _ in range(300):
         last = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, max_len=L)
     assert torch.equal(first, last)
-    from scirust_b200.ops import _lib
     _lib.check_status(torch.device("cuda"))
 
 
@@ -328,3 +324,42 @@ def test_decode_attention_stream_without_weight_is_zero():
     one = D.decode_attention(q, pool, table, page, ln, H, Hkv, dh, stream=False)
     assert (one[:2] == 0).all() and (out[:2] == 0).all()
     assert (out[2].float() - one[2].float()).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("rows,quant", [(1, False), (8, True), (9, False), (33, True), (64, False)])
+def test_dependent_launches_read_what_their_predecessor_wrote(rows, quant):
+    """Chains of decode kernels whose inputs AND weights the kernel right before them has just written give, launch for
+    launch, the bits of plain stream order."""
+    K, N = 1024, 1536
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    gain = torch.ones(K, dtype=torch.bfloat16, device="cuda")
+    xs = [torch.randn(rows, K, generator=g, device="cuda").to(torch.bfloat16) for _ in range(4)]
+    ws = [(torch.randn(K, N, generator=g, device="cuda") * 0.05).to(torch.bfloat16) for _ in range(4)]
+    qs = [D.quantize_per_channel(w) for w in ws]
+    for q in qs:
+        q.transposed()
+
+    def chain():
+        w = D.QuantWeight(qs[0].q.clone(), qs[0].scale.clone()) if quant else ws[0].clone()
+        if quant:
+            w.transposed()
+        out = []
+        for i in range(12):
+            x = ops.rmsnorm_fwd(xs[i % 4], gain, 1e-5, want_inv=False)[0]
+            if quant:
+                w.scale.copy_(qs[i % 4].scale)
+                w.q.copy_(qs[i % 4].q)
+                w.transposed().copy_(qs[i % 4].transposed())
+            else:
+                w.copy_(ws[i % 4])
+            y = D.gemv(x, w, rms_weight=gain) if rows <= 8 else D.matmul_skinny(x, w)
+            out.append(ops.swiglu_fwd(y))
+        return torch.stack(out)
+
+    got = chain()
+    _lib.call("sb_set_pdl", 0)
+    try:
+        want = chain()
+    finally:
+        _lib.call("sb_set_pdl", 1)
+    assert torch.equal(got, want)
