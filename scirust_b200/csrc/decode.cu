@@ -265,6 +265,55 @@ __device__ __forceinline__ void gemv_coll_finish(const GemvParams& p, uint32_t e
   }
 }
 
+// Four finished values of row m, columns gc .. gc + 3.
+__device__ __forceinline__ void gemv_store4(const GemvParams& p, int m, int gc, float4 v) {
+  if (p.scale) { v.x *= p.scale[gc]; v.y *= p.scale[gc + 1]; v.z *= p.scale[gc + 2]; v.w *= p.scale[gc + 3]; }
+  if (p.R) {
+    const __nv_bfloat16* r = p.R + static_cast<size_t>(m) * p.ldr + gc;
+    v.x += __bfloat162float(r[0]); v.y += __bfloat162float(r[1]);
+    v.z += __bfloat162float(r[2]); v.w += __bfloat162float(r[3]);
+  }
+  if (p.out) {
+    __nv_bfloat16* o = p.out + static_cast<size_t>(m) * p.ldo + gc;
+    if ((reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+      *reinterpret_cast<uint2*>(o) = make_uint2(dpack(v.x, v.y), dpack(v.z, v.w));
+    } else {
+      o[0] = __float2bfloat16_rn(v.x); o[1] = __float2bfloat16_rn(v.y);
+      o[2] = __float2bfloat16_rn(v.z); o[3] = __float2bfloat16_rn(v.w);
+    }
+  }
+  if (p.out_f32) {
+    float* o = p.out_f32 + static_cast<size_t>(m) * p.N + gc;
+    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+  }
+}
+
+// Split-K finish inside a cluster: its CTAs are the splits of one column block, each holds its partial sums in shared
+// memory ([M][COLS] floats at `vals`), and CTA r adds columns [r COLS / c, (r + 1) COLS / c) of all c in split order, the
+// order of the finish through memory. That one costs a store, a fence, a counter and dependent loads from L2 after the
+// stream has ended, with one CTA adding for all (us, through memory / here, at the splits that suit each: one row
+// 1024 x 1536 5.6 / 3.8, 4096 x 4096 11.0 / 9.1, 14336 x 4096 23.5 / 21.9; eight rows 11.0 / 4.0, 20.9 / 10.4, 37.6 / 24.6).
+template <int COLS>
+__device__ __forceinline__ void gemv_cluster_finish(const GemvParams& p, float* vals, int col0) {
+  const int c = gridDim.y, rank = blockIdx.y;
+  cluster_sync_all();
+  const int q0 = rank * (COLS / 4) / c, nq = (rank + 1) * (COLS / 4) / c - q0;
+  const uint32_t base = smem_u32(vals);
+  for (int i = threadIdx.x; i < p.M * nq; i += GEMV_THREADS) {
+    const int m = i / nq, col = (q0 + i - m * nq) * 4;
+    if (col0 + col >= p.N) continue;             // N is a multiple of 8
+    const uint32_t at = base + (m * COLS + col) * 4;
+    float4 v[8], sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) if (r < c) v[r] = ld_cluster_f4(mapa_shared(at, r));
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < c) { sum.x += v[r].x; sum.y += v[r].y; sum.z += v[r].z; sum.w += v[r].w; }
+    gemv_store4(p, m, col0 + col, sum);
+  }
+  cluster_sync_all();                            // nobody leaves while its sums are being read
+}
+
 template <int MB, bool INT8>
 __global__ void __launch_bounds__(GEMV_THREADS)
 gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ GemvParams p) {
@@ -514,10 +563,13 @@ __device__ __forceinline__ void gemv_mma_16816(float (&c)[4], const uint32_t (&a
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int MBLK>   // blocks of 8 activation rows: 1, 2 or 4 (M <= 8 * MBLK)
+// MBLK: blocks of 8 activation rows, 1, 2 or 4 (M <= 8 * MBLK); a warp owns 16 NB columns; CLUSTER: the splits of a column
+// block are a cluster and finish in shared memory
+template <int MBLK, int NB, bool CLUSTER>
 __global__ void __launch_bounds__(GEMV_THREADS)
 gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ GemvParams p) {
-  constexpr int COLS = 256;
+  constexpr int COLS = 128 * NB;
+  constexpr int KT = 64 / NB;    // rows of a 16 KB tile
   constexpr int XR = 8 * MBLK;   // 32-bit words per k pair in the staged activations
   extern __shared__ __align__(1024) uint8_t smem_mma[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_mma) + 1023) & ~uintptr_t(1023));
@@ -530,7 +582,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   const int col0 = blockIdx.x * COLS;
   const int k0 = blockIdx.y * p.k_per_split;            // a multiple of 32
   const int k1 = min(K, k0 + p.k_per_split);
-  const int ntiles = (k1 - k0 + GEMV_KT - 1) / GEMV_KT;
+  const int ntiles = (k1 - k0 + KT - 1) / KT;
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_w);
@@ -540,9 +592,9 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   __syncthreads();
   if (p.coll.W <= 1 && p.amax.W <= 1) pdl_trigger();   // a kernel that waits for its peers keeps the GPU to itself
 
-  float acc[2][MBLK][4];
+  float acc[NB][MBLK][4];
 #pragma unroll
-  for (int nb = 0; nb < 2; ++nb)
+  for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
     for (int mb = 0; mb < MBLK; ++mb)
 #pragma unroll
@@ -559,9 +611,9 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         // rows past K and columns past N arrive as zeros and still count towards the byte total
         mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          tma_load_2d(tiles + s * GEMV_TILE_BYTES + c * (GEMV_KT * 128), &tmap_w, &full[s], col0 + c * 64,
-                      k0 + t * GEMV_KT);
+        for (int c = 0; c < 2 * NB; ++c)
+          tma_load_2d(tiles + s * GEMV_TILE_BYTES + c * (KT * 128), &tmap_w, &full[s], col0 + c * 64,
+                      k0 + t * KT);
       }
       __syncwarp();
     }
@@ -619,7 +671,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     // written (lanes of the other rows feed zeros to the MMA below); k past the split's range is zero, since a
     // weight row past K is zero too and 0 * x must not meet garbage
     uint32_t* xs_w = reinterpret_cast<uint32_t*>(xs);
-    const int n_pairs = ntiles * GEMV_KT / 2;
+    const int n_pairs = ntiles * KT / 2;
     const bool vec_ok = ((p.ldx & 7) == 0) && ((K & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.X) & 15) == 0) &&
                         (p.prologue != PRO_RMSNORM || (reinterpret_cast<uintptr_t>(p.norm_w) & 15) == 0);
     if (vec_ok && M > 1) {   // a single row is staged faster by the pair loop below (3.40 against 4.07 ms per decode step)
@@ -681,15 +733,16 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     const uint32_t* xs32 = reinterpret_cast<const uint32_t*>(xs);
     // ldmatrix lane address: matrix mi = lane / 8 -> (k group = mi / 2, n half = mi % 2), row lane % 8
     const int mi = lane >> 3, lr = lane & 7;
-    const int sub = warp >> 1;                          // which 64-column box holds this warp's columns
-    const uint32_t tiles_u32 = smem_u32(tiles) + sub * (GEMV_KT * 128);
+    const int sub = warp * NB >> 2;                     // which 64-column box holds this warp's columns
+    const uint32_t tiles_u32 = smem_u32(tiles) + sub * (KT * 128);
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
       if (!mbar_wait(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
       const uint32_t tbase = tiles_u32 + s * GEMV_TILE_BYTES;
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        const int kp = (t * GEMV_KT + ks * 16) >> 1;      // index of the first bf16 pair of this k-step
+      for (int ks = 0; ks < KT / 16; ++ks) {
+        if (KT > 32 && t * KT + ks * 16 >= k1 - k0) break;   // the rest of the tile belongs to the next split
+        const int kp = (t * KT + ks * 16) >> 1;      // index of the first bf16 pair of this k-step
         uint32_t b0[MBLK], b1[MBLK];
 #pragma unroll
         for (int mb = 0; mb < MBLK; ++mb) {
@@ -699,8 +752,8 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         }
         const int r = ks * 16 + (mi >> 1) * 8 + lr;       // k row inside the tile
 #pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-          const int chunk = (warp & 1) * 4 + nb * 2 + (mi & 1);   // 16-byte chunk of the 128-byte row
+        for (int nb = 0; nb < NB; ++nb) {
+          const int chunk = (warp * NB & 3) * 2 + nb * 2 + (mi & 1);   // 16-byte chunk of the 128-byte row
           uint32_t a[4];
           gemv_ldsm_x4_t(tbase + r * 128 + ((chunk ^ (r & 7)) << 4), a);
 #pragma unroll
@@ -719,18 +772,20 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   // the epoch word is advanced only after every finishing CTA of this call has read it
   const uint32_t epoch = coll ? *reinterpret_cast<volatile uint32_t*>(p.coll.epoch_word) + 1u : 0u;
   if (warp < 8) {
-    // accumulator (nb, mb, j): column col0 + 32 warp + 16 nb + g + 8 (j / 2), row 8 mb + 2 tq + (j & 1)
+    // accumulator (nb, mb, j): column col0 + 16 (NB warp + nb) + g + 8 (j / 2), row 8 mb + 2 tq + (j & 1)
 #pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
+    for (int nb = 0; nb < NB; ++nb) {
 #pragma unroll
       for (int mb = 0; mb < MBLK; ++mb) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int gc = col0 + warp * 32 + nb * 16 + g + (j >> 1) * 8;
+          const int gc = col0 + (warp * NB + nb) * 16 + g + (j >> 1) * 8;
           const int m = mb * 8 + tq * 2 + (j & 1);
           if (m < M && gc < N) {
             float sum = acc[nb][mb][j];
-            if (direct) {
+            if constexpr (CLUSTER) {
+              vals[m * COLS + (gc - col0)] = sum;
+            } else if (direct) {
               if (coll) { gemv_coll_push(p, epoch, m, gc, sum); continue; }
               if (p.R) sum += __bfloat162float(p.R[static_cast<size_t>(m) * p.ldr + gc]);
               if (p.out) p.out[static_cast<size_t>(m) * p.ldo + gc] = __float2bfloat16_rn(sum);
@@ -744,6 +799,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       }
     }
   }
+  if constexpr (CLUSTER) { gemv_cluster_finish<COLS>(p, vals, col0); return; }
   if (direct) {
     if (coll) gemv_coll_finish(p, epoch, col0, min(COLS, N - col0), &s_last);
     else if (amax) gemv_argmax_tail(p, vals, COLS, col0, min(COLS, N - col0), &s_last);
@@ -802,9 +858,11 @@ __device__ __forceinline__ void gemv_mma_16816_f16(float (&c)[4], const uint32_t
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+template <int NP, bool CLUSTER>   // a warp owns 32 NP columns
 __global__ void __launch_bounds__(GEMV_THREADS)
 gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ GemvParams p) {
-  constexpr int COLS = 512;      // int8 columns per CTA: 512 bytes of every weight row
+  constexpr int COLS = 256 * NP;   // int8 columns per CTA: 512 or 256 bytes of every weight row
+  constexpr int KT = 64 / NP;      // rows of a 16 KB tile
   constexpr int MBLK = 1;
   constexpr int XR = 8;          // 32-bit words (fp16 pairs) per k pair in the staged activations
   extern __shared__ __align__(1024) uint8_t smem_mma[];
@@ -818,7 +876,7 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const int col0 = blockIdx.x * COLS;
   const int k0 = blockIdx.y * p.k_per_split;            // a multiple of 32
   const int k1 = min(K, k0 + p.k_per_split);
-  const int ntiles = (k1 - k0 + GEMV_KT - 1) / GEMV_KT;
+  const int ntiles = (k1 - k0 + KT - 1) / KT;
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_w);
@@ -828,9 +886,9 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   __syncthreads();
   if (p.coll.W <= 1 && p.amax.W <= 1) pdl_trigger();   // a kernel that waits for its peers keeps the GPU to itself
 
-  float acc[4][MBLK][4];
+  float acc[2 * NP][MBLK][4];
 #pragma unroll
-  for (int nb = 0; nb < 4; ++nb)
+  for (int nb = 0; nb < 2 * NP; ++nb)
 #pragma unroll
     for (int mb = 0; mb < MBLK; ++mb)
 #pragma unroll
@@ -847,9 +905,9 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         // rows past K and columns past N arrive as zeros and still count towards the byte total
         mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          tma_load_2d(tiles + s * GEMV_TILE_BYTES + c * (GEMV_KT * 128), &tmap_w, &full[s], col0 / 2 + c * 64,
-                      k0 + t * GEMV_KT);   // the map is over 16-bit words: 64 words = 128 int8 columns
+        for (int c = 0; c < 2 * NP; ++c)
+          tma_load_2d(tiles + s * GEMV_TILE_BYTES + c * (KT * 128), &tmap_w, &full[s], col0 / 2 + c * 64,
+                      k0 + t * KT);   // the map is over 16-bit words: 64 words = 128 int8 columns
       }
       __syncwarp();
     }
@@ -908,7 +966,7 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // written (lanes of the other rows feed zeros to the MMA below); k past the split's range is zero, since a
     // weight row past K is zero too and 0 * x must not meet garbage
     uint32_t* xs_w = reinterpret_cast<uint32_t*>(xs);
-    const int n_pairs = ntiles * GEMV_KT / 2;
+    const int n_pairs = ntiles * KT / 2;
     const bool vec_ok = ((p.ldx & 7) == 0) && ((K & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.X) & 15) == 0) &&
                         (p.prologue != PRO_RMSNORM || (reinterpret_cast<uintptr_t>(p.norm_w) & 15) == 0);
     if (vec_ok && M > 1) {   // a single row is staged faster by the pair loop below (3.40 against 4.07 ms per decode step)
@@ -973,23 +1031,24 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // bytes {W[2tq][2g], W[2tq][2g+1], W[2tq+1][2g], W[2tq+1][2g+1]}; the even column feeds MMA row g, the odd one
     // row g + 8 (the epilogue maps rows back to columns).
     const int mi = lane >> 3, lr = lane & 7;
-    const int sub = warp >> 1;                          // which 128-column box holds this warp's 64 columns
-    const uint32_t tiles_u32 = smem_u32(tiles) + sub * (GEMV_KT * 128);
+    const int sub = warp * NP >> 2;                     // which 128-column box holds this warp's columns
+    const uint32_t tiles_u32 = smem_u32(tiles) + sub * (KT * 128);
     const __half2 bias = __floats2half2_rn(1152.f, 1152.f);   // 1024 (the magic exponent) + 128 (the sign flip)
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
       if (!mbar_wait(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
       const uint32_t tbase = tiles_u32 + s * GEMV_TILE_BYTES;
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        const int kp = (t * GEMV_KT + ks * 16) >> 1;      // index of the first fp16 pair of this k-step
+      for (int ks = 0; ks < KT / 16; ++ks) {
+        if (KT > 32 && t * KT + ks * 16 >= k1 - k0) break;   // the rest of the tile belongs to the next split
+        const int kp = (t * KT + ks * 16) >> 1;      // index of the first fp16 pair of this k-step
         const bool live = g < M;
         const uint32_t b0 = live ? xs32[(kp + tq) * XR + g] : 0u;
         const uint32_t b1 = live ? xs32[(kp + 4 + tq) * XR + g] : 0u;
         const int r = ks * 16 + (mi & 1) * 8 + lr;        // k row inside the tile
 #pragma unroll
-        for (int pr = 0; pr < 2; ++pr) {                  // two n blocks of 16 columns per ldmatrix.x4
-          const int chunk = (warp & 1) * 4 + pr * 2 + (mi >> 1);   // 16-byte chunk = 16 int8 columns
+        for (int pr = 0; pr < NP; ++pr) {                  // two n blocks of 16 columns per ldmatrix.x4
+          const int chunk = (warp * NP & 3) * 2 + pr * 2 + (mi >> 1);   // 16-byte chunk = 16 int8 columns
           uint32_t raw[4];
           gemv_ldsm_x4_t(tbase + r * 128 + ((chunk ^ (r & 7)) << 4), raw);
 #pragma unroll
@@ -1024,16 +1083,18 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   // the epoch word is advanced only after every finishing CTA of this call has read it
   const uint32_t epoch = coll ? *reinterpret_cast<volatile uint32_t*>(p.coll.epoch_word) + 1u : 0u;
   if (warp < 8) {
-    // accumulator (nb, j): column col0 + 64 warp + 16 nb + 2 g + (j / 2), row 2 tq + (j & 1)
+    // accumulator (nb, j): column col0 + 32 NP warp + 16 nb + 2 g + (j / 2), row 2 tq + (j & 1)
 #pragma unroll
-    for (int nb = 0; nb < 4; ++nb) {
+    for (int nb = 0; nb < 2 * NP; ++nb) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int gc = col0 + warp * 64 + nb * 16 + 2 * g + (j >> 1);
+        const int gc = col0 + warp * (32 * NP) + nb * 16 + 2 * g + (j >> 1);
         const int m = tq * 2 + (j & 1);
         if (m < M && gc < N) {
           float sum = acc[nb][0][j];
-          if (direct) {
+          if constexpr (CLUSTER) {
+            vals[m * COLS + (gc - col0)] = sum;
+          } else if (direct) {
             sum *= p.scale[gc];
             if (coll) { gemv_coll_push(p, epoch, m, gc, sum); continue; }
             if (p.R) sum += __bfloat162float(p.R[static_cast<size_t>(m) * p.ldr + gc]);
@@ -1047,6 +1108,7 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
     }
   }
+  if constexpr (CLUSTER) { gemv_cluster_finish<COLS>(p, vals, col0); return; }
   if (direct) {
     if (coll) gemv_coll_finish(p, epoch, col0, min(COLS, N - col0), &s_last);
     else if (amax) gemv_argmax_tail(p, vals, COLS, col0, min(COLS, N - col0), &s_last);
@@ -2033,53 +2095,31 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
 int num_sms();
 }
 
-// bf16 weights: the tensor-core kernel. The staged slice of X takes 16 bytes per k for every 8 rows.
-template <int MBLK>
-static int launch_gemv_mma_mb(const GemvParams& p, int splits, cudaStream_t s) {
-  dim3 grid((p.N + 255) / 256, splits);
-  const int kn_pad = (p.k_per_split + GEMV_KT - 1) / GEMV_KT * GEMV_KT;
-  const size_t xs_bytes = static_cast<size_t>(kn_pad) * 16 * MBLK;
-  if (xs_bytes > static_cast<size_t>(GEMV_MAX_XS_BYTES)) return SB_ERR_ARG;
-  // the RMSNorm prologue borrows the X staging area for M * 8 * 32 partial sums; 1 KB for the ring's alignment
-  const size_t borrow = static_cast<size_t>(8 * MBLK) * 1024;
-  const size_t smem = static_cast<size_t>(GEMV_STAGES) * GEMV_TILE_BYTES + (xs_bytes > borrow ? xs_bytes : borrow) + 1024;
-  CUtensorMap tm;
-  const int rc = make_tmap_2d_bf16(&tm, p.W, static_cast<uint64_t>(p.N), p.K, static_cast<uint64_t>(p.ldw), 64, GEMV_KT);
-  if (rc) return rc;
-  auto kern = gemv_mma_kernel<MBLK>;
-  static size_t attr = 0;
-  if (smem > attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr = smem;
-  }
-  return launch_dep(kern, grid, dim3(GEMV_THREADS), smem, s, tm, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
-}
-// int8 weights on the tensor-core kernel: the tensor map is over 16-bit words (two int8 columns each).
-static int launch_gemv_mma_i8(const GemvParams& p, int splits, cudaStream_t s) {
-  dim3 grid((p.N + 511) / 512, splits);
-  const int kn_pad = (p.k_per_split + GEMV_KT - 1) / GEMV_KT * GEMV_KT;
+// The tensor-core kernels. ESZ 2: bf16 weights, 1: int8 (the tensor map is over 16-bit words, two int8 columns each);
+// W2 = 2: 512 bytes of every weight row per CTA, 1: 256. The staged slice of X takes 16 bytes per k. Only one block of 8
+// rows is shipped: with two or four blocks the kernel is bound by the mma.sync rate, not by memory (117 MB of weights:
+// 33 us at 8 rows, 58 us at 16, 111 us at 32), and the tcgen05 GEMM is faster there.
+template <int ESZ, int W2, bool CLUSTER>
+static int launch_gemv_mma(const GemvParams& p, int splits, cudaStream_t s) {
+  constexpr int KT = 64 / W2, COLS = 256 * W2 / ESZ;
+  const int kn_pad = (p.k_per_split + KT - 1) / KT * KT;
   const size_t xs_bytes = static_cast<size_t>(kn_pad) * 16;
   if (xs_bytes > static_cast<size_t>(GEMV_MAX_XS_BYTES)) return SB_ERR_ARG;
+  if (ESZ == 1 && ((p.N & 1) || (p.ldw & 1))) return SB_ERR_ARG;
+  // the RMSNorm prologue borrows the X staging area for M * 8 * 32 partial sums; 1 KB for the ring's alignment
   const size_t smem = static_cast<size_t>(GEMV_STAGES) * GEMV_TILE_BYTES + (xs_bytes > 8192 ? xs_bytes : 8192) + 1024;
-  if ((p.N & 1) || (p.ldw & 1)) return SB_ERR_ARG;
   CUtensorMap tm;
-  const int rc = make_tmap_2d_bf16(&tm, p.W, static_cast<uint64_t>(p.N) / 2, p.K, static_cast<uint64_t>(p.ldw) / 2, 64, GEMV_KT);
+  const int rc = make_tmap_2d_bf16(&tm, p.W, static_cast<uint64_t>(p.N) * ESZ / 2, p.K,
+                                   static_cast<uint64_t>(p.ldw) * ESZ / 2, 64, KT);
   if (rc) return rc;
-  auto kern = gemv_mma_i8_kernel;
-  static size_t attr = 0;
-  if (smem > attr) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-      return SB_ERR_LAUNCH;
-    attr = smem;
-  }
-  return launch_dep(kern, grid, dim3(GEMV_THREADS), smem, s, tm, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
-}
-
-// Only one block of 8 rows is shipped: with two or four blocks the kernel is bound by the mma.sync rate, not by
-// memory (117 MB of weights: 33 us at 8 rows, 58 us at 16, 111 us at 32), and the tcgen05 GEMM is faster there.
-static int launch_gemv_mma(const GemvParams& p, int splits, cudaStream_t s) {
-  return launch_gemv_mma_mb<1>(p, splits, s);
+  void (*kern)(const CUtensorMap, const GemvParams);
+  if constexpr (ESZ == 2) kern = gemv_mma_kernel<1, W2, CLUSTER>; else kern = gemv_mma_i8_kernel<W2, CLUSTER>;
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, kern, GEMV_STAGES * GEMV_TILE_BYTES + GEMV_MAX_XS_BYTES + 1024, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
+  const dim3 grid((p.N + COLS - 1) / COLS, splits);
+  const bool waits_for_peers = p.coll.W > 1 || p.amax.W > 1;
+  return launch_dep_cluster(kern, grid, dim3(GEMV_THREADS), smem, s, CLUSTER ? splits : 1, !waits_for_peers, tm, p) ==
+                 cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
 // Y[M,N] = f(X)[M,K] * W[K,N] (* scale[n]) (+ R). M <= 8 per call (callers loop over row groups).
@@ -2162,7 +2202,18 @@ static int gemv_impl(const void* X, int ldx, const void* W, int ldw, const float
       }
     }
   }
-  if (mma) return is_int8 ? launch_gemv_mma_i8(p, splits, STREAM) : launch_gemv_mma(p, splits, STREAM);
+  if (mma) {
+    // Up to eight splits finish inside a cluster, unless the grid runs in many waves (clusters are placed one by one:
+    // 4096 x 128256, eight splits: 160 us through memory, 174 in clusters) or one CTA has to hold the finished block, as
+    // the fused tails want it. Half the columns per CTA where the grid would leave SMs without one.
+    const int blocks = (N + cols - 1) / cols;
+    if (!ca && !aa && splits > 1 && splits <= 8 && blocks * splits <= 4 * num_sms()) {
+      if (blocks * splits > num_sms())
+        return is_int8 ? launch_gemv_mma<1, 2, true>(p, splits, STREAM) : launch_gemv_mma<2, 2, true>(p, splits, STREAM);
+      return is_int8 ? launch_gemv_mma<1, 1, true>(p, splits, STREAM) : launch_gemv_mma<2, 1, true>(p, splits, STREAM);
+    }
+    return is_int8 ? launch_gemv_mma<1, 2, false>(p, splits, STREAM) : launch_gemv_mma<2, 2, false>(p, splits, STREAM);
+  }
   return is_int8 ? launch_gemv<true>(p, splits, STREAM) : launch_gemv<false>(p, splits, STREAM);
 }
 

@@ -32,16 +32,30 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int c0, in
 
 bool dependent_launches();   // decode.cu: sb_set_pdl
 
+// `dependent` false: plain stream order. cluster_y > 1: clusters of that many CTAs along the grid's y.
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_dep(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+static cudaError_t launch_dep_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                      int cluster_y, bool dependent, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (dependent && dependent_launches()) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster_y > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = 1; at[n].val.clusterDim.y = cluster_y; at[n++].val.clusterDim.z = 1;
+  }
   cfg.attrs = at;
-  cfg.numAttrs = dependent_launches() ? 1 : 0;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_dep(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  return launch_dep_cluster(kern, grid, block, smem, s, 1, true, args...);
 }
 
 }  // namespace sb

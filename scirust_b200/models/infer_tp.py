@@ -122,7 +122,7 @@ class TPInferenceEngine(InferenceEngine):
             full = coll.source(site, (self._small_rows, d), torch.float32, device=x.device)
             if M <= D.gemv_max_rows(w):
                 src = full[:M]
-                D.gemv(a, w, out_f32=src, swiglu=swiglu)
+                D.gemv(a, w, out_f32=src, swiglu=swiglu, splits=D.allreduce_splits(w, M))   # the fused product's sums
             else:
                 src = full.view(-1).view(BF)[:M * d].view(M, d)     # same base address, bf16 partial
                 if swiglu:

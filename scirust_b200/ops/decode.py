@@ -155,6 +155,21 @@ def _auto_splits(N, K, cols, M=1, quant=False):
     return max(s, (K + lim - 1) // lim)
 
 
+def _gemv_splits(N, K, cols, M=1, quant=False):
+    """k-splits of ``gemv`` and ``gemv_argmax``. Up to eight splits of a column block run as one thread-block cluster and
+    finish in shared memory (csrc/decode.cu), which beats more of them that finish through memory (us, before / eight splits:
+    one row 4096 x 4096 11.0 / 9.1; eight rows 20.9 / 10.4, int8 14336 x 4096 44.4 / 23.0) as long as the staged slice of X
+    leaves room for two CTAs per SM: 28672 x 2048 at eight 51, at 37 27."""
+    s = _auto_splits(N, K, cols, M, quant)
+    if os.environ.get("SB_GEMV_FMA") == "1":
+        return s
+    if K <= 16384:
+        s = min(s, 8)
+        if (N + cols - 1) // cols > 148:          # several CTAs per SM, so at most 32 KB of staged X each: int8 4096 x 128256
+            s = max(s, (K + 2047) // 2048)        # at one split 114 us, at two 92
+    return s
+
+
 def gemv(x, w, residual=None, out=None, out_f32=None, splits=None, rms_weight=None, eps=1e-5, swiglu=False):
     """y[M,N] = f(x)[M,K] @ W (+ residual) for small M, streaming W once. ``w`` is a bf16 ``[K, N]``
     matrix or a ``QuantWeight``. Rows are processed in groups of 8. ``rms_weight`` fuses the RMSNorm of
@@ -186,7 +201,7 @@ def gemv(x, w, residual=None, out=None, out_f32=None, splits=None, rms_weight=No
         out = _lib.empty((M, N), BF, x.device)
     grp = 8                                   # rows per call
     if splits is None:
-        splits = _auto_splits(N, K, 512 if quant else 256, min(M, grp), quant)
+        splits = _gemv_splits(N, K, 512 if quant else 256, min(M, grp), quant)
     splits = max(splits, (K + 4095) // 4096)
     ws = _gemv_workspace(4096 + splits * min(M, grp) * N, x.device)
     st = _lib.status_word(x.device)
@@ -209,6 +224,13 @@ _lib.register("sb_gemv_allreduce", [vp, i32, vp, i32, vp, vp, i32, vp, i32, i32,
                                     vp, vp, vp, vp, i32, i32, i32, i32, vp, vp])
 
 
+def allreduce_splits(w, M):
+    """k-splits of ``gemv_allreduce``: a ``gemv`` of as many splits has the same partial sums, bit for bit."""
+    K, N = w.shape
+    quant = isinstance(w, QuantWeight)
+    return _auto_splits(N, K, 512 if quant else 256, M, quant)
+
+
 def gemv_allreduce(x, w, chan, residual=None, out=None, splits=None, swiglu=False):
     """out[M,N] = residual + sum over the ranks of ``chan`` of f(x_r)[M,K_r] @ W_r, M <= 8, in ONE launch per rank:
     the row-parallel product of tensor-parallel decoding with its all-reduce done by the CTAs that finish each block
@@ -223,7 +245,7 @@ def gemv_allreduce(x, w, chan, residual=None, out=None, splits=None, swiglu=Fals
     if out is None:
         out = _lib.empty((M, N), BF, x.device)
     if splits is None:
-        splits = _auto_splits(N, K, 512 if quant else 256, M, quant)
+        splits = allreduce_splits(w, M)
     splits = max(splits, (K + 4095) // 4096)
     ws = _gemv_workspace(4096 + splits * M * N, x.device)
     st = _lib.status_word(x.device)
@@ -265,7 +287,7 @@ def gemv_argmax(x, w, out_tokens=None, rms_weight=None, eps=1e-5, logits=None, c
     if out_tokens is None:
         out_tokens = _lib.empty(M, torch.int64, x.device)
     if splits is None:
-        splits = _auto_splits(N, K, 512 if quant else 256, M, quant)
+        splits = _gemv_splits(N, K, 512 if quant else 256, M, quant)
     splits = max(splits, (K + 4095) // 4096)
     ws = _gemv_workspace(4096 + splits * M * N, x.device)
     key = (str(x.device), _lib.stream())
