@@ -19,6 +19,12 @@
 // ties falls out of the last level, and the second walk starts from the first walk's top-level histogram. 16 rows of
 // 128256 logits, top-k 50, top-p 0.95: 418 us with one CTA per row, 78 us so (147 us while all 32 warps scanned the bins
 // of every level, eight neighbours to a lane and so sixteen lanes to a bank).
+//
+// Each of the ten levels that are left costs a barrier, an exchange and a scan, about 6 us, and mostly sorts out a few
+// dozen words. So when the first level, whose histogram is made by the pass that makes the weights, leaves no more than
+// SAMP_LIST words at or above the digit that the cut falls into, these go to one CTA, which ranks them and finishes alone
+// (a cut of top_k always ends there unless many weights are equal in their first digit; a nucleus of thousands does not).
+// Ranks, sums and ties are those of the walks. The same 16 rows: 27 us.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -36,6 +42,8 @@ constexpr int SAMP_CLUSTER = 8;                 // portable cluster size
 constexpr int SAMP_SLICE_WORDS = 48 * 1024;     // 192 KB of a CTA's shared memory; longer slices stay in `work`
 // Up to here one CTA holds the row: a cluster barrier costs more than a pass over so few words.
 constexpr int SAMP_SINGLE_MAX_V = 8192;
+// Words that one CTA finishes: a thread compares its word with all others, 512 x 512 comparisons take about 4 us.
+constexpr int SAMP_LIST = 512;
 
 struct SampleParams {
   const float* logits; int ld; int V;
@@ -68,7 +76,7 @@ __device__ __forceinline__ int samp_bin(int d) { return d + (d >> 3); }
 struct SampShared {
   SampHist h[2];
   unsigned long long tot_cnt[SAMP_BINS], tot_sum[SAMP_BINS];   // of the level being scanned, over the cluster
-  unsigned long long top_cnt[SAMP_BINS], top_sum[SAMP_BINS];   // level 0 of the first walk
+  unsigned long long top_cnt[SAMP_BINS], top_sum[SAMP_BINS];   // level 0
   int cut_d;                                       // result of the scan
   unsigned long long cut_cnt, cut_sum, in_cnt, in_sum;
   unsigned long long total;                        // this CTA's weight sum
@@ -76,6 +84,8 @@ struct SampShared {
   float red[SAMP_THREADS / 32];
   unsigned long long red_u[SAMP_THREADS / 32];
   int64_t tok[SAMP_MAX_WINDOW];
+  int n_list;                                      // rank 0's copy counts
+  unsigned long long list[SAMP_LIST], ranked[SAMP_LIST];   // weight << 32 | ~id: larger is earlier in the ranking
 };
 
 template <bool SMEM>
@@ -107,6 +117,24 @@ __device__ __forceinline__ void hist_add(SampHist& h, int d, uint32_t c, unsigne
   if constexpr (SMEM) { atomicAdd(&h.half.lo[d], lo); atomicAdd(&h.half.hi[d], hi); }
   else atomicAdd(&h.sum[d], s);
 }
+
+// A thread batches the run of equal digits it sees: near-uniform rows put everything into one bin. Digit 0 is not added.
+template <bool SMEM>
+struct RunOfDigits {
+  SampHist& h;
+  int cur = 0;
+  uint32_t c = 0, lo = 0, hi = 0;
+  unsigned long long s = 0;
+  __device__ __forceinline__ void flush() {
+    if (c) hist_add<SMEM>(h, cur, c, s, lo, hi);
+  }
+  __device__ __forceinline__ void add(int d, uint32_t v) {
+    if (d != cur) { flush(); cur = d; c = 0; s = 0; lo = 0; hi = 0; }
+    c += 1;
+    if constexpr (SMEM) { lo += v & 0xffffu; hi += v >> 16; }
+    else s += v;
+  }
+};
 
 // Sums the cluster's histograms into tot_cnt / tot_sum (bin 0, usually the fullest, is not counted: the scan gets it from
 // the totals) and clears the buffer of the next level.
@@ -192,7 +220,7 @@ struct Walk {                   // result of one ranked walk
 // first rank r where either r + 1 == limit_count, or the inclusive sum reaches `target`
 // (>= target, or > target when `strict`). `buf` is the histogram buffer to use next (clear on entry and on exit).
 template <bool SMEM>
-__device__ Walk ranked_walk(cg::cluster_group& cl, SampShared& s, const Row<SMEM>& row, int& buf, bool have_top,
+__device__ Walk ranked_walk(cg::cluster_group& cl, SampShared& s, const Row<SMEM>& row, int& buf,
                             unsigned long long n, unsigned long long z, unsigned long long limit_count,
                             unsigned long long target, bool strict) {
   uint32_t prefix = 0;
@@ -201,34 +229,19 @@ __device__ Walk ranked_walk(cg::cluster_group& cl, SampShared& s, const Row<SMEM
   for (int level = 0; level < 4; ++level) {
     const int shift = 24 - 8 * level;
     const unsigned long long *tc = s.tot_cnt, *ts = s.tot_sum;
-    if (level == 0 && have_top) {
+    if (level == 0) {
       tc = s.top_cnt; ts = s.top_sum;
     } else {
-      const uint32_t mask_hi = level == 0 ? 0u : (0xffffffffu << (shift + 8));
+      const uint32_t mask_hi = 0xffffffffu << (shift + 8);
       SampHist& h = s.h[buf];
-      // a thread batches the run of equal digits it sees: near-uniform rows put everything into one bin
-      int cur = 0;
-      uint32_t c_run = 0, lo = 0, hi = 0;
-      unsigned long long s_run = 0;
+      RunOfDigits<SMEM> run{h};
       row.each([&](int, uint32_t v) {
         const int d = (v >> shift) & 0xff;
-        if ((v & mask_hi) == prefix && d != 0) {
-          if (d != cur) {
-            if (c_run) hist_add<SMEM>(h, cur, c_run, s_run, lo, hi);
-            cur = d; c_run = 0; s_run = 0; lo = 0; hi = 0;
-          }
-          c_run += 1;
-          if constexpr (SMEM) { lo += v & 0xffffu; hi += v >> 16; }
-          else s_run += v;
-        }
+        if ((v & mask_hi) == prefix && d != 0) run.add(d, v);
       });
-      if (c_run) hist_add<SMEM>(h, cur, c_run, s_run, lo, hi);
+      run.flush();
       combine<SMEM>(cl, s, buf);
       buf ^= 1;
-      if (level == 0 && threadIdx.x < SAMP_BINS) {
-        s.top_cnt[threadIdx.x] = s.tot_cnt[threadIdx.x];
-        s.top_sum[threadIdx.x] = s.tot_sum[threadIdx.x];
-      }
     }
     scan_bins(s, tc, ts, in_cnt, in_sum, cnt_before, sum_before, limit_count, target, strict);
     prefix |= static_cast<uint32_t>(s.cut_d) << shift;
@@ -257,6 +270,59 @@ __device__ Walk ranked_walk(cg::cluster_group& cl, SampShared& s, const Row<SMEM
   return out;
 }
 
+// The cumulative probability's target in weight units, never below one.
+__device__ __forceinline__ unsigned long long nucleus_target(float top_p, unsigned long long z) {
+  const double d = static_cast<double>(top_p) * static_cast<double>(z);
+  return d <= 1.0 ? 1ull : static_cast<unsigned long long>(ceil(d));
+}
+// Where the draw falls in a kept sum of zz; advances the row's generator.
+__device__ __forceinline__ unsigned long long draw_target(uint64_t& st, unsigned long long zz) {
+  st ^= st << 13; st ^= st >> 7; st ^= st << 17;
+  const float u = static_cast<float>(static_cast<double>(st >> 11) / 9007199254740992.0);
+  unsigned long long target = static_cast<unsigned long long>(static_cast<double>(u) * static_cast<double>(zz));
+  if (zz > 0 && target >= zz) target = zz - 1;
+  return target;
+}
+
+// One CTA finishes the row: s.list holds every word down to the first digit of the cut (n of them, all above zero). The
+// kept set ends at the first rank r with r + 1 == limit or an inclusive sum of at least tp; the draw takes the first rank
+// whose inclusive sum is above its target. Returns the id to the thread that holds it, -1 to the others.
+__device__ int finish_list(SampShared& s, int n, unsigned long long limit, unsigned long long tp, bool cut,
+                           unsigned long long z, uint64_t& st) {
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (t < n) {
+    const unsigned long long mine = s.list[t];
+    int r = 0;
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) r += s.list[k] > mine;       // ids differ, so no two words are equal
+    s.ranked[r] = mine;
+  }
+  __syncthreads();
+  const unsigned long long key = t < n ? s.ranked[t] : 0;
+  unsigned long long sum = key >> 32;                        // inclusive over ranks
+  if (t < SAMP_LIST) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    if (lane == 31) s.red_u[warp] = sum;
+  }
+  __syncthreads();
+  if (t < SAMP_LIST) {
+    for (int k = 0; k < warp; ++k) sum += s.red_u[k];
+    const unsigned long long before = sum - (key >> 32);
+    // exactly one rank is the first to reach the limit or the sum
+    const unsigned long long place = static_cast<unsigned long long>(t) + 1;
+    if (t < n && (place == limit || sum >= tp) && place <= limit && before < tp) s.cut_sum = sum;
+  }
+  __syncthreads();
+  const unsigned long long zz = cut ? s.cut_sum : z;
+  const unsigned long long target = draw_target(st, zz);
+  const bool hit = t < n && sum > target && sum - (key >> 32) <= target;
+  return hit ? static_cast<int>(~static_cast<uint32_t>(key)) : -1;
+}
+
 template <bool SMEM>
 __global__ void __launch_bounds__(SAMP_THREADS, 1)
 sample_rows_kernel(const SampleParams p) {
@@ -275,21 +341,26 @@ sample_rows_kernel(const SampleParams p) {
 
   // ---- penalised copy of the slice ----
   const float* xs = x + min(row.base, V);
+  float mx = -INFINITY;
   if (SMEM && (reinterpret_cast<uintptr_t>(xs) & 15) == 0) {
     const int n4 = row.n >> 2;
 #pragma unroll 4
-    for (int j = t; j < n4; j += SAMP_THREADS)
-      reinterpret_cast<float4*>(wf)[j] = __ldg(reinterpret_cast<const float4*>(xs) + j);
+    for (int j = t; j < n4; j += SAMP_THREADS) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(xs) + j);
+      reinterpret_cast<float4*>(wf)[j] = a;
+      mx = fmaxf(fmaxf(mx, fmaxf(a.x, a.y)), fmaxf(a.z, a.w));
+    }
     const int j = 4 * n4 + t;
-    if (j < row.n) wf[j] = xs[j];
+    if (j < row.n) { wf[j] = xs[j]; mx = fmaxf(mx, xs[j]); }
   } else {
 #pragma unroll 4
-    for (int j = t; j < row.n; j += SAMP_THREADS) wf[j] = xs[j];
+    for (int j = t; j < row.n; j += SAMP_THREADS) { const float a = xs[j]; wf[j] = a; mx = fmaxf(mx, a); }
   }
   if (t < 512) {
     s.h[t >> 8].cnt[t & 255] = 0;
     s.h[t >> 8].sum[t & 255] = 0;
   }
+  if (t == 0) s.n_list = 0;
   int n_win = 0;
   if (p.rep_penalty > 1.0f && p.recent && p.n_recent) {
     const int n = p.n_recent[row_id];
@@ -320,8 +391,10 @@ sample_rows_kernel(const SampleParams p) {
   __syncthreads();
 
   int token = -1;              // known to the thread that writes it out
-  float mx = -INFINITY;
-  for (int j = t; j < row.n; j += SAMP_THREADS) mx = fmaxf(mx, wf[j]);
+  if (n_win > 0) {             // the penalty may have taken the maximum
+    mx = -INFINITY;
+    for (int j = t; j < row.n; j += SAMP_THREADS) mx = fmaxf(mx, wf[j]);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (lane == 0) s.red[warp] = mx;
@@ -335,15 +408,32 @@ sample_rows_kernel(const SampleParams p) {
   cl.sync();
   mx = s.vmax;
   for (int r = 0; r < nr; ++r) mx = fmaxf(mx, *cl.map_shared_rank(&s.vmax, r));
-  // fixed-point weights and their total
+  // fixed-point weights, their total and the first level's histogram
   unsigned long long local = 0;
   const float inv_t = 1.0f / p.temperature;
-  for (int j = t; j < row.n; j += SAMP_THREADS) {
-    const float e = expf((wf[j] - mx) * inv_t);              // in [0, 1]
-    const float f = e * 4294967296.0f;
-    const uint32_t q = f >= 4294967040.0f ? 0xffffffffu : static_cast<uint32_t>(f);
-    row.w[j] = q;
-    local += q;
+  {
+    RunOfDigits<SMEM> run{s.h[0]};
+    auto weigh = [&](float l) {
+      const float e = expf((l - mx) * inv_t);                // in [0, 1]
+      const float f = e * 4294967296.0f;
+      const uint32_t q = f >= 4294967040.0f ? 0xffffffffu : static_cast<uint32_t>(f);
+      local += q;
+      if (q >> 24) run.add(q >> 24, q);
+      return q;
+    };
+    if constexpr (SMEM) {
+      const int n4 = row.n >> 2;
+#pragma unroll 2
+      for (int j = t; j < n4; j += SAMP_THREADS) {
+        const float4 a = reinterpret_cast<const float4*>(wf)[j];
+        reinterpret_cast<uint4*>(row.w)[j] = make_uint4(weigh(a.x), weigh(a.y), weigh(a.z), weigh(a.w));
+      }
+      const int j = 4 * n4 + t;
+      if (j < row.n) row.w[j] = weigh(wf[j]);
+    } else {
+      for (int j = t; j < row.n; j += SAMP_THREADS) row.w[j] = weigh(wf[j]);
+    }
+    run.flush();
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
@@ -355,31 +445,48 @@ sample_rows_kernel(const SampleParams p) {
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
     if (lane == 0) s.total = local;
   }
-  cl.sync();
+  combine<SMEM>(cl, s, 0);
+  int buf = 1;
   unsigned long long z = 0;
   for (int r = 0; r < nr; ++r) z += *cl.map_shared_rank(&s.total, r);
+  if (t < SAMP_BINS) { s.top_cnt[t] = s.tot_cnt[t]; s.top_sum[t] = s.tot_sum[t]; }
   // kept set: first min(top_k, V) ranks, cut where the cumulative probability reaches top_p
   const unsigned long long n_all = static_cast<unsigned long long>(V);
   const unsigned long long limit = (p.top_k > 0 && p.top_k < V) ? static_cast<unsigned long long>(p.top_k) : n_all;
-  unsigned long long zz = z;
-  int buf = 0;
-  bool have_top = false;
-  if (limit < n_all || p.top_p < 1.0f) {
-    unsigned long long tp = ~0ull;   // unreachable sum: only the count stops the walk
-    if (p.top_p < 1.0f) {
-      const double d = static_cast<double>(p.top_p) * static_cast<double>(z);
-      tp = d <= 1.0 ? 1ull : static_cast<unsigned long long>(ceil(d));
-    }
-    zz = ranked_walk<SMEM>(cl, s, row, buf, false, n_all, z, limit, tp, false).sum;
-    have_top = true;
-  }
-  // one uniform draw; every thread computes it, one stores the state after all have read it
+  const bool cut = limit < n_all || p.top_p < 1.0f;
+  const unsigned long long tp = p.top_p < 1.0f ? nucleus_target(p.top_p, z) : ~0ull;   // ~0: only the count stops the walk
   uint64_t st = p.rng_state[row_id];
-  st ^= st << 13; st ^= st >> 7; st ^= st << 17;
-  const float u = static_cast<float>(static_cast<double>(st >> 11) / 9007199254740992.0);
-  unsigned long long target = static_cast<unsigned long long>(static_cast<double>(u) * static_cast<double>(zz));
-  if (zz > 0 && target >= zz) target = zz - 1;
-  const Walk wk = ranked_walk<SMEM>(cl, s, row, buf, have_top, n_all, z, n_all, target, true);
+  {
+    // the first level of the first walk: the cut's, or the draw's when everything is kept
+    uint64_t peek = st;
+    const unsigned long long target = cut ? tp : draw_target(peek, z);
+    scan_bins(s, s.tot_cnt, s.tot_sum, n_all, z, 0, 0, limit, target, !cut);
+    const uint32_t d0 = static_cast<uint32_t>(s.cut_d);
+    const unsigned long long n_up = s.cut_cnt + s.in_cnt;
+    if (d0 > 0 && n_up <= SAMP_LIST) {
+      SampShared* first = cl.map_shared_rank(&s, 0);
+      row.each([&](int j, uint32_t v) {
+        if (v >> 24 >= d0)
+          first->list[atomicAdd(&first->n_list, 1)] =
+              static_cast<unsigned long long>(v) << 32 | static_cast<uint32_t>(~static_cast<uint32_t>(row.base + j));
+      });
+      cl.sync();               // the list is whole; nobody reads another CTA's memory from here on
+      if (rank != 0) return;
+      token = finish_list(s, static_cast<int>(n_up), limit, tp, cut, z, st);
+      if (t == 0) p.rng_state[row_id] = st;
+      if (token >= 0) {
+        p.out_tokens[row_id] = token;
+        if (p.generated) p.generated[static_cast<size_t>(row_id) * p.gen_stride + p.step] = token;
+      }
+      return;
+    }
+    __syncthreads();           // all have read the cut
+  }
+  unsigned long long zz = z;
+  if (cut) zz = ranked_walk<SMEM>(cl, s, row, buf, n_all, z, limit, tp, false).sum;
+  // one uniform draw; every thread computes it, one stores the state after all have read it
+  const unsigned long long target = draw_target(st, zz);
+  const Walk wk = ranked_walk<SMEM>(cl, s, row, buf, n_all, z, n_all, target, true);
   cl.sync();
   if (rank == 0 && t == 0) p.rng_state[row_id] = st;
   if (wk.ties == 1) {

@@ -1,4 +1,6 @@
 """Device sampler (csrc/sampler.cu) against the host policy ``sample_row``."""
+import math
+
 import pytest
 import torch
 
@@ -191,3 +193,26 @@ def test_greedy_rows_on_every_split(vocab, rows, penalty):
     host = lg.cpu()
     want = [_greedy_pick(host[b], hist[b, 4:].tolist() if penalty > 1 else [], penalty) for b in range(rows)]
     assert got == want
+
+
+@pytest.mark.parametrize("vocab", [700, 8200, 128256, 393221])
+@pytest.mark.parametrize("ties", [1, 511, 512, 513, 640])
+@pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (0, 0.5), (1, 1.0), (512, 1.0), (600, 0.7)])
+def test_short_lists_and_walks_take_the_same_element(vocab, ties, top_k, top_p):
+    """`ties` ids share the largest weight and the rest are masked: up to 512 of them are finished as a list by one CTA, more
+    by the walks. The kept set is a prefix of the ids and the draw an exact integer statement either way."""
+    rows = 3
+    ids = torch.stack([torch.randperm(vocab, generator=torch.Generator().manual_seed(ties + b))[:ties].sort().values
+                       for b in range(rows)])
+    lg = torch.full((rows, vocab), float("-inf")).scatter_(1, ids, 0.0)
+    params = SamplingParams(temperature=1.0, top_k=top_k, top_p=top_p)
+    s = DeviceSampler(params, rows, vocab, range(7, 7 + rows), "cuda")
+    got = s.sample(lg.cuda()).cpu().tolist()
+    w = 2 ** 32 - 1
+    for b in range(rows):
+        kept = min(ties, top_k) if 0 < top_k < vocab else ties
+        if top_p < 1.0:                           # the first prefix whose weight reaches top_p of the total
+            kept = min(kept, -(-math.ceil(float(torch.tensor(top_p)) * float(ties * w)) // w))
+        z = kept * w
+        t = min(int(SamplerRng(7 + b).next_uniform() * float(z)), z - 1)
+        assert got[b] == int(ids[b, t // w])
