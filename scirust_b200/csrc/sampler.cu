@@ -261,7 +261,7 @@ __device__ Walk ranked_walk(cg::cluster_group& cl, SampShared& s, const Row<SMEM
   if (v > 0) {
     unsigned long long need;                            // ties needed for the sum criterion
     if (strict) need = target >= sum_before ? (target - sum_before) / v + 1 : 1;
-    else need = target > sum_before ? (target - sum_before + v - 1) / v : 1;
+    else need = target > sum_before ? (target - sum_before - 1) / v + 1 : 1;   // rounded up; target may be ~0
     if (need < take) take = need;
   }
   if (take < 1) take = 1;
