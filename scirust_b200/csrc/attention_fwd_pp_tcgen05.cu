@@ -9,8 +9,7 @@
 // stays below 2^8, far inside its range), which on real score distributions happens in the first blocks
 // only; at 128 by anything. There the reference is the running maximum itself, as in the one-tile kernel,
 // so the largest weight of a row is 1 and has no rounding; with the 2^8 margin the error against float64
-// was 2 % larger for unit scores and 20 % larger for scores of twice the spread. The rescales cost 5 %
-// (4096 tokens, 32 heads: 163.7 -> 172.8 us). The row sum uses the same reference point, so the final O / l
+// was 2 % larger for unit scores and 20 % larger for scores of twice the spread. The rescales cost 5 %. The row sum uses the same reference point, so the final O / l
 // and the log-sum-exp are exact regardless of when a rescale happened.
 //
 // Same interface, layout and semantics as the one-tile kernel (attention_fwd_tcgen05.cu): fused
@@ -22,24 +21,27 @@
 //
 // A softmax thread holds its whole 128-column score row in registers (one pass over tensor memory),
 // scales it with packed fp32 pairs (fma.rn.f32x2, add.rn.f32x2: half the issue slots of scalar
-// code) and takes the row maximum with three-input max. Cycle stamps taken inside the kernel put a kv
-// block of one tile at about 3500 cycles: 1500-1650 in the 128 exponentials with pack and store,
-// 400 in the row maximum, and about 1000 waiting for the tensor pipe (scores of the next block, P V
-// of the previous one), although the products themselves need only 256 + 436 cycles (a 128 x 128 x 16
-// tcgen05.mma takes 64 cycles, a 128 x 64 x 16 one 54.5: `bench_kernels umma`). Two variants that
-// looked right on paper measured slower and are not used: issuing the scores of block j+1 as soon
-// as block j sits in registers (the P V of block j then queued behind them), and taking every
-// fourth 2^x from a cubic polynomial on the FMA pipe (POLY_EVERY below; the softmax warps are short
-// of issue slots per warp, not of special-function throughput).
+// code) and takes the row maximum with three-input max. Its warps are the bottleneck: two of them share a
+// scheduler and its special-function unit, 1024 cycles for the 128 exponentials of a block each, while the
+// products of a block need 2 x 512 cycles at head dimension 128. So nothing else may stand in their way:
+//  - Every tile has an issuing warp of its own, and the scores of block j+1 are issued as soon as those of block j
+//    are in registers, so they are there when block j is done. With one issuer for both tiles the waits of one
+//    tile held up the other.
+//  - An issuing warp walks through its loop as a whole and one lane issues: descriptors and addresses stay in uniform
+//    registers. As the loop of a single thread a product cost it 70 to 150 cycles to issue, more than to run.
+//  - The exponentials, their sum and their bf16 pairs come before the wait for the previous P V, which runs meanwhile.
+//  - The mask is applied to the scores of the blocks that need one; as a select beside every exponential it
+//    cost all blocks a third of their instructions.
+// The softmax warpgroups take the registers that the issuing one does not need (setmaxnreg), so rows stay unspilled.
+// us before / now, causal, 32 heads of 128: 5000 tokens 262 / 209 (980 TFLOP/s), 4096 185 / 154, 2 x 2048 112 / 100;
+// 16 heads of 64: 8 x 2048 160 / 147.
 //
 // Head dimension 128: Q (64 KB), two P tiles (64 KB) and a K tile of 32 KB twice leave 32 KB for V. K gets two whole
 // stages; V is a ring of two half tiles of 64 kv rows, because the products consume V row by row: the first half is
 // free again before the second tile's P V ends, and its successor lands while the next scores run. With three
-// whole-tile slots for K and V together, every block would wait about a load latency for its K. Against the one-tile
-// kernel (scores, softmax and P V of a block one after another): 5000 tokens, 32 heads, causal 422 -> 278 us (486 ->
-// 737 TFLOP/s), 2 x 2048 tokens 164 -> 108 us.
+// whole-tile slots for K and V together, every block would wait about a load latency for its K.
 //
-// Warps: 0 TMA producer, 1 MMA issuer, 2-5 softmax of tile 0, 6-9 softmax of tile 1.
+// Warps: 0 TMA producer, 1 and 2 MMA issuers of tiles 0 and 1, 3 idle, 4-7 softmax of tile 0, 8-11 softmax of tile 1.
 #include "sm100_ptx.cuh"
 #include "api.h"
 #include "per_device.h"
@@ -53,7 +55,10 @@ namespace attpp {
 
 constexpr int BM = 128;        // query rows per tile
 constexpr int BN = 128;        // kv rows per block
-constexpr int THREADS = 320;
+constexpr int THREADS = 384;
+// Registers a thread: 168 at launch for all three warpgroups, shared out as 56 (producer, issuers) + 2 x 224 (softmax).
+constexpr int REGS_ISSUE = 56, REGS_SOFTMAX = 224;
+static_assert(REGS_ISSUE + 2 * REGS_SOFTMAX <= 3 * 168, "the shares draw on the registers of the launch");
 constexpr int P_BYTES = BM * BN * 2;
 constexpr int TMEM_COLS = 512;  // S0 [0,128) S1 [128,256) O0 [256,256+DH) O1 [256+DH,256+2DH)
 
@@ -84,24 +89,10 @@ struct Params {
   int* status;
 };
 
-constexpr int POLY_EVERY = 0;   // every POLY_EVERY-th element takes 2^x from the polynomial (0 = none)
-
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-// 2^x on the FMA pipe: n = round(x), f = x - n in [-0.5, 0.5], cubic minimax polynomial for 2^f,
-// n added to the exponent field. x is clamped at -126 (the result is then about 1e-38).
-__device__ __forceinline__ float ex2_poly(float x) {
-  x = fmaxf(x, -126.f);
-  const float magic = 12582912.f;            // 1.5 * 2^23: the sum holds round(x) in its low mantissa bits
-  const float xr = x + magic;
-  const float f = x - (xr - magic);
-  float pl = fmaf(0.0551716685295105f, f, 0.2426111251115799f);
-  pl = fmaf(pl, f, 0.6932609677314758f);
-  pl = fmaf(pl, f, 0.9999280571937561f);
-  return __int_as_float(__float_as_int(pl) + (__float_as_int(xr) << 23));
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
@@ -130,9 +121,10 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
   uint64_t* s_full = v_empty + VS;       // [2] scores of tile t are in tensor memory
   uint64_t* p_full = s_full + 2;         // [2] P of tile t is in shared memory (4 warp arrivals)
   uint64_t* pv_done = p_full + 2;        // [2] P V of tile t has completed
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(pv_done + 2);
+  uint64_t* s_free = pv_done + 2;        // [2] scores of tile t are in registers (4 warp arrivals)
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(s_free + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_pairs = (p.S + 2 * BM - 1) / (2 * BM);
   const int pair = n_pairs - 1 - blockIdx.z;  // slowest grid index: longest tiles first over the whole grid
   const int head = blockIdx.x, b = blockIdx.y;
@@ -157,9 +149,10 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
       mbar_init(&s_full[t], 1);
       mbar_init(&p_full[t], 4);
       mbar_init(&pv_done[t], 1);
+      mbar_init(&s_free[t], 4);
     }
-    for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
-    for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
+    for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 2); }   // one arrival per issuer
+    for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 2); }
     fence_barrier_init();
     fence_proxy_async_smem();
   }
@@ -171,8 +164,10 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
 
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_ISSUE));
   if (warp == 0) {
     // ------------------------------------ TMA producer ------------------------------------
     if (lane == 0) {
@@ -217,88 +212,74 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
         ok = ok && load_v(j);
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------------- MMA issuer -------------------------------------
-    if (lane == 0) {
+  } else if (warp == 1 || warp == 2) {
+    // ------------------------------------- MMA issuers -------------------------------------
+    {
+      // The whole warp walks through the loop, so that descriptors and addresses stay in uniform registers; one lane issues.
+      const bool leader = elect_one();
+      const int t = warp - 1;
+      const int n_t = nb[t];
       constexpr uint32_t idesc_s = make_idesc_bf16(BM, BN, false, false);
       constexpr uint32_t idesc_o = make_idesc_bf16(BM, DH, false, true);
+      const uint64_t dq = make_smem_desc(smem_u32(sQ + t * C::Q_BYTES), 16, 1024);
+      const uint64_t dp = make_smem_desc(smem_u32(sP + t * P_BYTES), 16, 1024);
       int ks = 0, vs = 0;
       uint32_t kph = 0, vph = 0;
-      bool ok = true;
-      for (int t = 0; t < 2 && ok; ++t)
-        if (nb[t] > 0) ok = mbar_wait(&q_full[t], 0, p.status, ST_TIMEOUT_FULL);
-      // S_t = Q_t K^T with K in ring slot `slot`
-      auto issue_s = [&](int t, int slot) {
-        const uint32_t aq = smem_u32(sQ + t * C::Q_BYTES), bk = smem_u32(sK + slot * C::K_BYTES);
-#pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
-          const uint32_t off = (k >> 2) * (BM * 128) + (k & 3) * 32;
-          umma_bf16_ss(tmem_base + t * BN, make_smem_desc(aq + off, 16, 1024), make_smem_desc(bk + off, 16, 1024),
-                       idesc_s, k > 0 ? 1u : 0u);
-        }
-        umma_commit(&s_full[t]);
-      };
-      // O_t (+)= P_t V, piece by piece of V starting at ring position (vs, vph); `first`: no other tile has waited for this
-      // V, `last`: none needs it. A wait costs the issuer its place even when it returns at once, and the softmax warps wait
-      // for pv_done, so it is committed ahead of the releases that only the producer waits for: head dimension 64, 16 heads,
-      // 3 x 2048 tokens, 66.4 us with a wait per tile and the releases first, 64.2 so.
-      auto issue_pv = [&](int t, bool acc, bool first, bool last) -> bool {
-        const uint32_t ap = smem_u32(sP + t * P_BYTES);
-        int slot = vs;
-        uint32_t ph = vph;
-#pragma unroll
-        for (int h = 0; h < C::VP; ++h) {
-          if (first) {
-            if (!mbar_wait(&v_full[slot], ph, p.status, ST_TIMEOUT_FULL)) return false;
+      bool ok = n_t == 0 || mbar_wait_warp(&q_full[t], 0, p.status, ST_TIMEOUT_FULL);
+      // Blocks that only the other tile sees are waited for and released all the same: a ring slot is free when both
+      // issuers have let go of it.
+      for (int j = 0; j <= n_blocks && ok; ++j) {
+        if (j < n_blocks) {                            // S = Q K^T of block j, as soon as the scores of j - 1 are in registers
+          if (!mbar_wait_warp(&k_full[ks], kph, p.status, ST_TIMEOUT_FULL)) break;
+          if (j < n_t) {
+            if (j > 0 && !mbar_wait_warp(&s_free[t], (j - 1) & 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
             tc_fence_after();
-          }
-          const uint32_t bv = smem_u32(sV + slot * C::V_BYTES);
+            const uint64_t dk = make_smem_desc(smem_u32(sK + ks * C::K_BYTES), 16, 1024);
 #pragma unroll
-          for (int k2 = 0; k2 < C::VROWS / 16; ++k2) {
-            const int k = h * (C::VROWS / 16) + k2;
-            const uint64_t adesc = make_smem_desc(ap + (k >> 2) * (BM * 128) + (k & 3) * 32, 16, 1024);
-            const uint64_t bdesc = make_smem_desc(bv + k2 * (16 * 128), C::VROWS * 128, 1024);
-            umma_bf16_ss(tmem_base + 2 * BN + t * DH, adesc, bdesc, idesc_o, (acc || k > 0) ? 1u : 0u);
+            for (int k = 0; k < DH / 16; ++k) {
+              const uint32_t off = (k >> 2) * (BM * 128) + (k & 3) * 32;
+              if (leader) umma_bf16_ss(tmem_base + t * BN, smem_desc_at(dq, off), smem_desc_at(dk, off),
+                           idesc_s, k > 0 ? 1u : 0u);
+            }
+            if (leader) umma_commit(&s_full[t]);
+            if (leader) umma_commit(&k_empty[ks]);
+          } else {
+            if (leader) mbar_arrive(&k_empty[ks]);
           }
-          if (h == C::VP - 1) umma_commit(&pv_done[t]);
-          if (last) umma_commit(&v_empty[slot]);
-          if (++slot == VS) { slot = 0; ph ^= 1; }
-        }
-        if (last) { vs = slot; vph = ph; }
-        return true;
-      };
-      if (ok && n_blocks > 0) {
-        ok = mbar_wait(&k_full[ks], kph, p.status, ST_TIMEOUT_FULL);
-        if (ok) {
-          tc_fence_after();
-          for (int t = 0; t < 2; ++t)
-            if (nb[t] > 0) issue_s(t, ks);
-          umma_commit(&k_empty[ks]);
           if (++ks == KS) { ks = 0; kph ^= 1; }
         }
-      }
-      for (int j = 0; j < n_blocks && ok; ++j) {
-        const bool have_next = j + 1 < n_blocks;
-        if (have_next && !mbar_wait(&k_full[ks], kph, p.status, ST_TIMEOUT_FULL)) break;
-        if (C::VP == 1 && !mbar_wait(&v_full[vs], vph, p.status, ST_TIMEOUT_FULL)) break;   // whole tiles: before P is there
-        for (int t = 0; t < 2; ++t) {
-          if (j >= nb[t]) continue;
-          const bool last = t == 1 || j >= nb[1];
-          if (!mbar_wait(&p_full[t], j & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
-          tc_fence_after();
-          if (j + 1 < nb[t]) issue_s(t, ks);   // scores first: the softmax warps of this tile can go on
-          if (KS == 2 && last && have_next) umma_commit(&k_empty[ks]);   // two stages: the producer waits for this one
-          ok = issue_pv(t, j > 0, C::VP > 1 && (t == 0 || j >= nb[0]), last);
-          if (!ok) break;
+        if (j > 0) {                                   // O (+)= P V of block j - 1
+          const int i = j - 1;
+#pragma unroll
+          for (int h = 0; h < C::VP && ok; ++h) {
+            ok = mbar_wait_warp(&v_full[vs], vph, p.status, ST_TIMEOUT_FULL);
+            if (ok && i < n_t) {
+              if (h == 0) ok = mbar_wait_warp(&p_full[t], i & 1, p.status, ST_TIMEOUT_MISC);
+              if (!ok) break;
+              tc_fence_after();
+              const uint64_t dv = make_smem_desc(smem_u32(sV + vs * C::V_BYTES), C::VROWS * 128, 1024);
+#pragma unroll
+              for (int k2 = 0; k2 < C::VROWS / 16; ++k2) {
+                const int k = h * (C::VROWS / 16) + k2;
+                if (leader)
+                  umma_bf16_ss(tmem_base + 2 * BN + t * DH, smem_desc_at(dp, (k >> 2) * (BM * 128) + (k & 3) * 32),
+                               smem_desc_at(dv, k2 * (16 * 128)), idesc_o, (i > 0 || k > 0) ? 1u : 0u);
+              }
+              if (h == C::VP - 1 && leader) umma_commit(&pv_done[t]);
+              if (leader) umma_commit(&v_empty[vs]);
+            } else if (ok) {
+              if (leader) mbar_arrive(&v_empty[vs]);
+            }
+            if (++vs == VS) { vs = 0; vph ^= 1; }
+          }
         }
-        if (KS > 2 && ok && have_next) umma_commit(&k_empty[ks]);
-        if (!ok) break;
-        if (have_next && ++ks == KS) { ks = 0; kph ^= 1; }
       }
     }
+  }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_SOFTMAX));
     // ------------------------------------ softmax warps ------------------------------------
-    const int t = (warp - 2) >> 2;
+    const int t = (warp >> 2) - 1;
     const int q = warp & 3;            // TMEM lane quarter this warp may read
     const int r = q * 32 + lane;       // row inside the tile == TMEM lane
     const int q_idx = q0 + t * BM + r; // position inside the sequence
@@ -318,75 +299,63 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
 #pragma unroll
       for (int c = 0; c < BN / 32; ++c) tmem_ld_32x32(tm_S + c * 32, v + c * 32);
       tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_free[t]);
       const int kv0 = j * BN;
       const bool need_mask = (p.causal && j == n_t - 1) || (kv0 + BN > p.S);
       const int lim = (p.causal ? min(q_idx, p.S - 1) : (p.S - 1)) - kv0;   // last visible column
       float m4[4] = {NEG, NEG, NEG, NEG};
       if (need_mask) {
+        // masked here and not among the exponentials, where every block would pay a compare and a select per score
 #pragma unroll
-        for (int i = 0; i < BN; i += 2)
-          m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], i > lim ? NEG : __uint_as_float(v[i]),
-                                  i + 1 > lim ? NEG : __uint_as_float(v[i + 1]));
-      } else {
+        for (int i = 0; i < BN; ++i)
+          if (i > lim) v[i] = 0xff800000u;             // -inf: 2^x is 0 whatever the row's reference
+      }
+      {
 #pragma unroll
         for (int i = 0; i < BN; i += 2)
           m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
       }
       const float m_blk = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2;
       const bool grow = m_blk > m_ref + C::RESCALE_GAP;   // always true in the first block
+      const float alpha = grow ? ex2(m_ref - m_blk) : 1.f;
+      if (grow) m_ref = m_blk;
+      // exponentials and their bf16 pairs, all in registers: P V of the previous block runs meanwhile
+      const float neg_m = -m_ref;
+      float sum4[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      uint32_t pk[BN / 2];
+#pragma unroll
+      for (int i = 0; i < BN; i += 2) {
+        fma2(v[i], v[i + 1], sl2, neg_m);
+        const float e0 = ex2(__uint_as_float(v[i]));
+        const float e1 = ex2(__uint_as_float(v[i + 1]));
+        add2(sum4[i & 6], sum4[(i & 6) + 1], __float_as_uint(e0), __float_as_uint(e1));
+        pk[i >> 1] = pack_bf16x2(e0, e1);
+      }
+      l = l * alpha + (((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) + ((sum4[4] + sum4[5]) + (sum4[6] + sum4[7])));
       if (j > 0) {
         // P V of the previous block has read the P tile and updated O
         if (!mbar_wait(&pv_done[t], (j - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
         if (__any_sync(0xffffffffu, grow)) {
           tc_fence_after();
-          const float alpha = grow ? ex2(m_ref - m_blk) : 1.f;
 #pragma unroll
-          for (int c = 0; c < DH / 16; ++c) {
-            uint32_t o[16];
-            tmem_ld_32x16(tm_O + c * 16, o);
+          for (int c = 0; c < DH / 32; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32(tm_O + c * 32, o);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; i += 2) mul2(o[i], o[i + 1], alpha, alpha);
-            tmem_st_32x16(tm_O + c * 16, o);
+            for (int i = 0; i < 32; i += 2) mul2(o[i], o[i + 1], alpha, alpha);
+            tmem_st_32x32(tm_O + c * 32, o);
           }
           tmem_st_wait();
-          l *= alpha;
         }
       }
-      if (grow) m_ref = m_blk;
-      // exponentials in place: every result lands in the register of its score, so all 128 are independent
-      const float neg_m = -m_ref;
 #pragma unroll
-      for (int i = 0; i < BN; i += 2) {
-        fma2(v[i], v[i + 1], sl2, neg_m);
-        float e0 = (POLY_EVERY > 0 && (i % (POLY_EVERY > 0 ? POLY_EVERY : 1)) == POLY_EVERY - 1)
-                       ? ex2_poly(__uint_as_float(v[i])) : ex2(__uint_as_float(v[i]));
-        float e1 = (POLY_EVERY > 0 && ((i + 1) % (POLY_EVERY > 0 ? POLY_EVERY : 1)) == POLY_EVERY - 1)
-                       ? ex2_poly(__uint_as_float(v[i + 1])) : ex2(__uint_as_float(v[i + 1]));
-        if (need_mask) {
-          if (i > lim) e0 = 0.f;
-          if (i + 1 > lim) e1 = 0.f;
-        }
-        v[i] = __float_as_uint(e0);
-        v[i + 1] = __float_as_uint(e1);
+      for (int c = 0; c < BN / 8; ++c) {               // 16-byte units of the swizzled row
+        uint8_t* prow = sPt + (c >> 3) * (BM * 128) + r * 128;
+        *reinterpret_cast<uint4*>(prow + (((c & 7) ^ (r & 7)) * 16)) = make_uint4(pk[c * 4], pk[c * 4 + 1], pk[c * 4 + 2], pk[c * 4 + 3]);
       }
-      float sum4[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int c = 0; c < BN / 16; ++c) {          // 16 columns = two 16-byte units of the swizzled row
-        uint32_t pk[8];
-#pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          add2(sum4[i & 6], sum4[(i & 6) + 1], v[c * 16 + i], v[c * 16 + i + 1]);
-          pk[i >> 1] = pack_bf16x2(__uint_as_float(v[c * 16 + i]), __uint_as_float(v[c * 16 + i + 1]));
-        }
-        uint8_t* prow = sPt + (c >> 2) * (BM * 128) + r * 128;
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int unit = ((c & 3) * 2 + u) ^ (r & 7);
-          *reinterpret_cast<uint4*>(prow + unit * 16) = make_uint4(pk[u * 4], pk[u * 4 + 1], pk[u * 4 + 2], pk[u * 4 + 3]);
-        }
-      }
-      l += ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) + ((sum4[4] + sum4[5]) + (sum4[6] + sum4[7]));
       tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();

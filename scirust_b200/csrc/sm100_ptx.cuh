@@ -103,6 +103,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   }
 }
 
+// The same for a whole converged warp; the result is the same in all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
+}
+
 // ---- TMA --------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -193,6 +198,11 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   d |= static_cast<uint64_t>(1) << 46;  // descriptor version for sm_100
   d |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
   return d;
+}
+
+// The descriptor of the same layout `bytes` further on (the address field does not carry inside shared memory).
+__device__ __forceinline__ uint64_t smem_desc_at(uint64_t desc, uint32_t bytes) {
+  return (desc & 0xffffffff00000000ull) | (static_cast<uint32_t>(desc) + (bytes >> 4));
 }
 
 // Instruction descriptor for kind::f16 with bf16 operands and fp32 accumulate.
