@@ -56,18 +56,17 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Element-wise core of both backward kernels for 32 score columns of one query row (thread = query
+// Element-wise core of the recomputing dQ kernel for 32 score columns of one query row (thread = query
 // row r, TMEM lane r): p = 2^(s*sl2 - lse2), dS = p * (dP*scale - delta*scale); columns beyond
-// `lim` are masked. Writes dS (and P when WRITE_P) as bf16 into the swizzled [q x kv] tiles.
-template <bool MASK, bool WRITE_P>
+// `lim` are masked. Writes dS as bf16 into the swizzled [q x kv] tile.
+template <bool MASK>
 __device__ __forceinline__ void bwd_chunk(uint32_t tm_S, uint32_t tm_dP, uint32_t lane_off, int c, int r, int lim,
-                                          float sl2, float lse2, float delta_s, float scale, uint8_t* p_buf,
-                                          uint8_t* ds_buf) {
+                                          float sl2, float lse2, float delta_s, float scale, uint8_t* ds_buf) {
   uint32_t sv[32], dv[32];
   tmem_ld_32x32(tm_S + lane_off + c * 32, sv);
   tmem_ld_32x32(tm_dP + lane_off + c * 32, dv);
   tmem_ld_wait();
-  uint32_t pk[16], dk[16];
+  uint32_t dk[16];
   const float neg_lse2 = -lse2, neg_delta = -delta_s;
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
@@ -81,10 +80,8 @@ __device__ __forceinline__ void bwd_chunk(uint32_t tm_S, uint32_t tm_dP, uint32_
       if (c * 32 + i + 1 > lim) p1 = 0.f;
     }
     mul2(dv[i], dv[i + 1], p0, p1);
-    if (WRITE_P) pk[i >> 1] = pack_bf16x2(p0, p1);
     dk[i >> 1] = pack_bf16x2(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1]));
   }
-  if (WRITE_P) store_row32_sw128(p_buf, r, c, pk);
   store_row32_sw128(ds_buf, r, c, dk);
 }
 
@@ -119,19 +116,24 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 }
 
 // --------------------------------------------------------------------------- dK / dV
-// Pipeline at head dimension 64: the bf16 P^T / dS^T tiles are double-buffered in shared memory, so the MMA
-// warp issues the score products of iteration t+1 *before* the gradient products of iteration t;
-// the softmax warps then work on t+1 while the tensor cores finish t. At 128 shared memory fits single
-// buffers only: the kernel below this one.
+// Pipeline at head dimension 64. A softmax thread takes its scores and dP into registers at once, so S and dP of iteration
+// t+1 follow while the exponentials of t run, and the gradient products of t while those of t+1 do: an iteration is as
+// long as its softmax. That takes three (Q, dO) stages, and P^T in one buffer to make room for them (dV(t-1) has read it
+// long before P(t) is ready); dS^T keeps two, since its bulk store reads it too. The issuing warp walks through its loop as
+// a whole with one lane issuing, so that descriptors stay in uniform registers: as a single thread it needed 1600 cycles
+// for the 16 gradient products, which run in 900. Until then the scores of t+1 waited for the whole softmax of t, then for a
+// stage, and then for the issuer, 3500 cycles an iteration: 8 x 2048 tokens of 16 heads, causal, the whole backward 449 us,
+// 397 now. At 128 shared memory has no room for this: the kernel below this one.
 struct DkvCfg {
   static constexpr int DH = 64;
-  static constexpr int NPB = 2;                       // P^T / dS^T buffers
-  static constexpr int QS = 2;                        // (Q, dO) ring stages
+  static constexpr int NPB = 2;                       // dS^T buffers
+  static constexpr int QS = 3;                        // (Q, dO) ring stages
   static constexpr int T_BYTES = BT * DH * 2;         // one [128 x DH] tile
   static constexpr int PT_BYTES = BT * BT * 2;
-  static constexpr int TILE_BYTES = 2 * T_BYTES + QS * 2 * T_BYTES + NPB * 2 * PT_BYTES;
+  static constexpr int TILE_BYTES = 2 * T_BYTES + QS * 2 * T_BYTES + (1 + NPB) * PT_BYTES;
   static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 128;
   static constexpr int TMEM_COLS = 512;  // S^T 128 | dP^T 128 | dK DH | dV DH
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
 };
 
 __global__ void __launch_bounds__(BWD_THREADS, 1)
@@ -145,18 +147,20 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
   uint8_t* sV = sK + Cfg::T_BYTES;
   uint8_t* sQ = sV + Cfg::T_BYTES;                 // QS stages
   uint8_t* sdO = sQ + Cfg::QS * Cfg::T_BYTES;      // QS stages
-  uint8_t* sPT = sdO + Cfg::QS * Cfg::T_BYTES;     // NPB buffers
-  uint8_t* sdST = sPT + Cfg::NPB * Cfg::PT_BYTES;  // NPB buffers
+  uint8_t* sPT = sdO + Cfg::QS * Cfg::T_BYTES;
+  uint8_t* sdST = sPT + Cfg::PT_BYTES;             // NPB buffers
   uint64_t* bars = reinterpret_cast<uint64_t*>(sdST + Cfg::NPB * Cfg::PT_BYTES);
   uint64_t* kv_full = bars;
   uint64_t* q_full = bars + 1;            // QS
   uint64_t* q_empty = q_full + Cfg::QS;   // QS
   uint64_t* st_full = q_empty + Cfg::QS;
-  uint64_t* p_full = st_full + 1;
-  uint64_t* done = p_full + 1;
+  uint64_t* st_free = st_full + 1;        // scores and dP of t are in registers (8 warp arrivals)
+  uint64_t* p_full = st_free + 1;
+  uint64_t* dv_done = p_full + 1;         // dV(t) has read P, and everything before it is done
+  uint64_t* done = dv_done + 1;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_t = (p.S + BT - 1) / BT;
   // The kv tile is the slowest grid index: CTAs are handed out in block-id order, so all the long tiles
   // (causal: small kt, up to 4x16 query tiles) start first and the short ones fill the tail.
@@ -174,6 +178,8 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
     for (int s = 0; s < Cfg::QS; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
     mbar_init(st_full, 1);
     mbar_init(p_full, 8);  // one arrival per softmax warp
+    mbar_init(st_free, 8);
+    mbar_init(dv_done, 1);
     mbar_init(done, 1);
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -183,7 +189,7 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
   // S and dP are [query x kv] (TMEM lane = query row, as in the dQ kernel); their bf16 images P and dS
   // are stored [q rows][kv] and consumed as MN-major A operands (A^T) by the dV / dK products.
   const uint32_t tm_ST = tmem_base, tm_dPT = tmem_base + 128, tm_dK = tmem_base + 256, tm_dV = tmem_base + 256 + DH;
@@ -214,78 +220,75 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(BT, BT, false, false);   // [q x kv], both K-major
-      constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, true, true);     // [kv x dh] = A^T B, both MN-major
-      bool ok = mbar_wait(kv_full, 0, p.status, ST_TIMEOUT_FULL);
-      int st_s = 0;          // stage / phase of the next score issue
-      uint32_t ph_s = 0;
-      int st_g = 0;          // stage of the next gradient issue
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV);
-      auto issue_scores = [&]() -> bool {
-        if (!mbar_wait(&q_full[st_s], ph_s, p.status, ST_TIMEOUT_FULL)) return false;
-        tc_fence_after();
-        const uint32_t bQ = smem_u32(sQ + st_s * Cfg::T_BYTES), bdO = smem_u32(sdO + st_s * Cfg::T_BYTES);
+    constexpr uint32_t idesc_s = make_idesc_bf16(BT, BT, false, false);   // [q x kv], both K-major
+    constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, true, true);     // [kv x dh] = A^T B, both MN-major
+    const bool leader = elect_one();
+    bool ok = mbar_wait_warp(kv_full, 0, p.status, ST_TIMEOUT_FULL);
+    int st_s = 0;          // stage / phase of the next score issue
+    uint32_t ph_s = 0;
+    int st_g = 0;          // stage of the next gradient issue
+    const uint64_t dK_ = make_smem_desc(smem_u32(sK), 16, 1024), dV_ = make_smem_desc(smem_u32(sV), 16, 1024);
+    const uint64_t dPT = make_smem_desc(smem_u32(sPT), BT * 128, 1024);
+    auto issue_scores = [&]() -> bool {
+      if (!mbar_wait_warp(&q_full[st_s], ph_s, p.status, ST_TIMEOUT_FULL)) return false;
+      tc_fence_after();
+      const uint64_t dQ = make_smem_desc(smem_u32(sQ + st_s * Cfg::T_BYTES), 16, 1024);
+      const uint64_t ddO = make_smem_desc(smem_u32(sdO + st_s * Cfg::T_BYTES), 16, 1024);
+      if (leader) {
 #pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
-          const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
-          umma_bf16_ss(tm_ST, make_smem_desc(bQ + off, 16, 1024), make_smem_desc(aK + off, 16, 1024), idesc_s,
-                       k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < DH / 16; ++k)
+          umma_bf16_ss(tm_ST, smem_desc_at(dQ, k * 32), smem_desc_at(dK_, k * 32), idesc_s, k > 0 ? 1u : 0u);
 #pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
-          const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
-          umma_bf16_ss(tm_dPT, make_smem_desc(bdO + off, 16, 1024), make_smem_desc(aV + off, 16, 1024), idesc_s,
-                       k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < DH / 16; ++k)
+          umma_bf16_ss(tm_dPT, smem_desc_at(ddO, k * 32), smem_desc_at(dV_, k * 32), idesc_s, k > 0 ? 1u : 0u);
         umma_commit(st_full);
-        if (++st_s == Cfg::QS) { st_s = 0; ph_s ^= 1; }
-        return true;
-      };
-      auto issue_grads = [&](int t) {
-        const int pb = t & 1;
-        const uint32_t aPT = smem_u32(sPT + pb * Cfg::PT_BYTES), adST = smem_u32(sdST + pb * Cfg::PT_BYTES);
-        const uint32_t bQ = smem_u32(sQ + st_g * Cfg::T_BYTES), bdO = smem_u32(sdO + st_g * Cfg::T_BYTES);
-#pragma unroll
-        for (int k = 0; k < BT / 16; ++k) {   // k walks 16 query rows at a time in both operands
-          umma_bf16_ss(tm_dV, make_smem_desc(aPT + k * (16 * 128), BT * 128, 1024),
-                       make_smem_desc(bdO + k * (16 * 128), BT * 128, 1024), idesc_g, (t > 0 || k > 0) ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < BT / 16; ++k) {
-          umma_bf16_ss(tm_dK, make_smem_desc(adST + k * (16 * 128), BT * 128, 1024),
-                       make_smem_desc(bQ + k * (16 * 128), BT * 128, 1024), idesc_g, (t > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(&q_empty[st_g]);
-        if (++st_g == Cfg::QS) st_g = 0;
-      };
-      if (ok && n_iter > 0) ok = issue_scores();
-      for (int t = 0; t < n_iter && ok; ++t) {
-        if (!mbar_wait(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
-        tc_fence_after();
-        // scores of t+1 first (double-buffered P^T / dS^T): the softmax warps wait for nothing else, and the
-        // commit of these scores also covers the gradient MMAs of t-1, which is what lets the softmax warps
-        // reuse the P^T / dS^T buffer of parity (t+1)&1
-        // (the dS store of t-1 has long been read out of its buffer; the wait only makes that certain before the
-        // scores whose completion lets the softmax warps write that buffer again)
-        if (p.spill_ds) tma_store_wait_read<0>();
-        if (t + 1 < n_iter) ok = issue_scores();
+      }
+      __syncwarp();
+      if (++st_s == Cfg::QS) { st_s = 0; ph_s ^= 1; }
+      return true;
+    };
+    if (ok && n_iter > 0) ok = issue_scores();
+    for (int t = 0; t < n_iter && ok; ++t) {
+      if (t + 1 < n_iter) {
+        if (!mbar_wait_warp(st_free, t & 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+        ok = issue_scores();
+        if (!ok) break;
+      }
+      if (!mbar_wait_warp(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
+      tc_fence_after();
+      const uint64_t ddS = make_smem_desc(smem_u32(sdST + (t & 1) * Cfg::PT_BYTES), BT * 128, 1024);
+      const uint64_t dQ = make_smem_desc(smem_u32(sQ + st_g * Cfg::T_BYTES), BT * 128, 1024);
+      const uint64_t ddO = make_smem_desc(smem_u32(sdO + st_g * Cfg::T_BYTES), BT * 128, 1024);
+      if (leader) {
         if (p.spill_ds) {
-          // the finished dS tile (bf16, [q rows][kv], scale included) also goes to global memory, where
-          // the dQ kernel streams it back instead of recomputing scores; the bulk store reads shared
-          // memory asynchronously, so it must have been read out before this buffer is written again
+          // the finished dS tile (bf16, [q rows][kv], scale included) also goes to global memory, where the dQ kernel
+          // streams it back instead of recomputing scores. The bulk store reads shared memory asynchronously: the one of
+          // t-1 must have been read out before dv_done(t), after which the softmax warps write that buffer again
           const int head = kvh * group + t / n_qt;
           const int qt = qt_first + t % n_qt;
           const uint8_t* src = sdST + (t & 1) * Cfg::PT_BYTES;
           tma_store_3d(&tm_ds, src, kv0, qt * BT, b * p.H + head);
           tma_store_3d(&tm_ds, src + BT * 128, kv0 + 64, qt * BT, b * p.H + head);
           tma_store_commit();
+          tma_store_wait_read<1>();
         }
-        issue_grads(t);
+#pragma unroll
+        for (int k = 0; k < BT / 16; ++k)   // k walks 16 query rows at a time in both operands
+          umma_bf16_ss(tm_dV, smem_desc_at(dPT, k * (16 * 128)), smem_desc_at(ddO, k * (16 * 128)), idesc_g,
+                       (t > 0 || k > 0) ? 1u : 0u);
+        umma_commit(dv_done);
+#pragma unroll
+        for (int k = 0; k < BT / 16; ++k)
+          umma_bf16_ss(tm_dK, smem_desc_at(ddS, k * (16 * 128)), smem_desc_at(dQ, k * (16 * 128)), idesc_g,
+                       (t > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&q_empty[st_g]);
       }
-      if (ok) umma_commit(done);
-      if (p.spill_ds) tma_store_wait<0>();   // the stores are complete before the CTA retires
+      __syncwarp();
+      if (++st_g == Cfg::QS) st_g = 0;
     }
+    if (ok && leader) umma_commit(done);
+    if (p.spill_ds && leader) tma_store_wait<0>();   // the stores are complete before the CTA retires
+    __syncwarp();
   } else {
     const int sw = warp - 2;        // 0..7
     const int q = warp & 3;         // TMEM lane quarter
@@ -293,7 +296,6 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
     const int r = q * 32 + lane;    // row inside the tile == TMEM lane (query row in the loop, kv row at the end)
     const int kv_idx = kv0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    const float delta_scale = p.scale;
     bool ok = true;
     for (int t = 0; t < n_iter; ++t) {
       const int head = kvh * group + t / n_qt;
@@ -301,9 +303,7 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
       const int q0 = qt * BT;
       const int q_idx = q0 + r;
       const float2 sd = __ldg(p.stats + (static_cast<size_t>(b) * p.H + head) * p.S + min(q_idx, p.S - 1));
-      const int pb = t & 1;
-      uint8_t* pt_buf = sPT + pb * Cfg::PT_BYTES;
-      uint8_t* dst_buf = sdST + pb * Cfg::PT_BYTES;
+      uint8_t* dst_buf = sdST + (t & 1) * Cfg::PT_BYTES;
       // last visible kv column of this query row inside the tile (-1: row is past the sequence end)
       const bool diag = p.causal && qt == kt;
       int lim = min(diag ? r : BT - 1, p.S - 1 - kv0);
@@ -311,16 +311,41 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
       const bool need_mask = diag || (q0 + BT > p.S) || (kv0 + BT > p.S);
       if (!mbar_wait(st_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
+      // P = 2^(s * sl2 - lse2), dS = P * (dP * scale - delta * scale)
+      uint32_t pv[64], dv[64];
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) tmem_ld_32x32(tm_ST + lane_off + (half * 2 + cc) * 32, pv + cc * 32);
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) tmem_ld_32x32(tm_dPT + lane_off + (half * 2 + cc) * 32, dv + cc * 32);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(st_free);
+      const float neg_delta = -sd.y * p.scale;
+#pragma unroll
+      for (int i = 0; i < 64; i += 2) {
+        fma2(pv[i], pv[i + 1], p.scale_log2, -sd.x);
+        pv[i] = __float_as_uint(fast_exp2(__uint_as_float(pv[i])));
+        pv[i + 1] = __float_as_uint(fast_exp2(__uint_as_float(pv[i + 1])));
+        fma2(dv[i], dv[i + 1], p.scale, neg_delta);
+      }
       if (need_mask) {
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc)
-          bwd_chunk<true, true>(tm_ST, tm_dPT, lane_off, half * 2 + cc, r, lim, p.scale_log2, sd.x,
-                                sd.y * delta_scale, p.scale, pt_buf, dst_buf);
-      } else {
+        for (int i = 0; i < 64; ++i)
+          if (half * 64 + i > lim) pv[i] = 0u;
+      }
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc)
-          bwd_chunk<false, true>(tm_ST, tm_dPT, lane_off, half * 2 + cc, r, lim, p.scale_log2, sd.x,
-                                 sd.y * delta_scale, p.scale, pt_buf, dst_buf);
+      for (int i = 0; i < 64; i += 2) {
+        mul2(dv[i], dv[i + 1], __uint_as_float(pv[i]), __uint_as_float(pv[i + 1]));
+        dv[i >> 1] = pack_bf16x2(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1]));
+        pv[i >> 1] = pack_bf16x2(__uint_as_float(pv[i]), __uint_as_float(pv[i + 1]));
+      }
+      // dV(t-1) has read P; the dS buffer of this parity was let go of before
+      if (t > 0 && !mbar_wait(dv_done, (t - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) {
+        store_row32_sw128(sPT, r, half * 2 + cc, pv + cc * 16);
+        store_row32_sw128(dst_buf, r, half * 2 + cc, dv + cc * 16);
       }
       tc_fence_before();
       fence_proxy_async_smem();
@@ -410,7 +435,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
   uint64_t* done = dv_done + 1;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_t = (p.S + BT - 1) / BT;
   // The kv tile is the slowest grid index: CTAs are handed out in block-id order, so all the long tiles
   // (causal: small kt, up to 4x16 query tiles) start first and the short ones fill the tail.
@@ -442,7 +467,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
   // S and dP are [query x kv] (TMEM lane = query row, as in the dQ kernel); their bf16 images P and dS
   // are stored [q rows][kv] and consumed as MN-major A operands (A^T) by the dV / dK products.
   const uint32_t tm_ST = tmem_base, tm_dPT = tmem_base + 128, tm_dK = tmem_base + 256, tm_dV = tmem_base + 256 + DH;
@@ -475,58 +500,63 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();       // the warp walks the loop as a whole, as at head dimension 64
       constexpr uint32_t idesc_s = make_idesc_bf16(BT, BT, false, false);   // [q x kv], both K-major
       constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, true, true);     // [kv x dh] = A^T B, both MN-major
-      bool ok = mbar_wait(kv_full, 0, p.status, ST_TIMEOUT_FULL);
+      bool ok = mbar_wait_warp(kv_full, 0, p.status, ST_TIMEOUT_FULL);
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), adO = smem_u32(sdO), aPT = smem_u32(sPT), adS = smem_u32(sdST);
       int qn = 0;                    // Q stage and phase of the next score product
       uint32_t qn_ph = 0;
       int qg = 0;                    // Q stage of the next dK product
       // D = A B^T over DH, both K-major
       auto score_product = [&](uint32_t d, uint32_t a, uint32_t b) {
+        const uint64_t da = make_smem_desc(a, 16, 1024), db = make_smem_desc(b, 16, 1024);
+        if (!leader) return;
 #pragma unroll
         for (int k = 0; k < DH / 16; ++k) {
           const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
-          umma_bf16_ss(d, make_smem_desc(a + off, 16, 1024), make_smem_desc(b + off, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
+          umma_bf16_ss(d, smem_desc_at(da, off), smem_desc_at(db, off), idesc_s, k > 0 ? 1u : 0u);
         }
       };
       // D += A^T B over the 128 query rows, 16 at a time in both operands
       auto grad_product = [&](uint32_t d, uint32_t a, uint32_t b, bool acc) {
+        const uint64_t da = make_smem_desc(a, BT * 128, 1024), db = make_smem_desc(b, BT * 128, 1024);
+        if (!leader) return;
 #pragma unroll
         for (int k = 0; k < BT / 16; ++k)
-          umma_bf16_ss(d, make_smem_desc(a + k * (16 * 128), BT * 128, 1024),
-                       make_smem_desc(b + k * (16 * 128), BT * 128, 1024), idesc_g, (acc || k > 0) ? 1u : 0u);
+          umma_bf16_ss(d, smem_desc_at(da, k * (16 * 128)), smem_desc_at(db, k * (16 * 128)), idesc_g, (acc || k > 0) ? 1u : 0u);
       };
       auto issue_s = [&]() -> bool {
-        if (!mbar_wait(&q_full[qn], qn_ph, p.status, ST_TIMEOUT_FULL)) return false;
+        if (!mbar_wait_warp(&q_full[qn], qn_ph, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
         score_product(tm_ST, smem_u32(sQ + qn * Cfg::T_BYTES), aK);
-        umma_commit(s_full);
+        if (leader) umma_commit(s_full);
         if (++qn == Cfg::QS) { qn = 0; qn_ph ^= 1; }
         return true;
       };
       auto issue_dp = [&](int t) -> bool {
-        if (!mbar_wait(do_full, t & 1, p.status, ST_TIMEOUT_FULL)) return false;
+        if (!mbar_wait_warp(do_full, t & 1, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
         // dp_full lets the softmax warps write dS again: its last bulk store must have been read out
-        if (p.spill_ds) tma_store_wait_read<0>();
+        if (p.spill_ds && leader) tma_store_wait_read<0>();
+        __syncwarp();
         score_product(tm_dPT, adO, aV);
-        umma_commit(dp_full);
+        if (leader) umma_commit(dp_full);
         return true;
       };
       if (n_iter > 0) ok = ok && issue_s() && issue_dp(0);
       for (int t = 0; t < n_iter && ok; ++t) {
         const bool more = t + 1 < n_iter;
-        if (!mbar_wait(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
+        if (!mbar_wait_warp(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
         tc_fence_after();
         if (more && !issue_s()) { ok = false; break; }
         grad_product(tm_dV, aPT, adO, t > 0);
-        umma_commit(dv_done);
-        umma_commit(do_empty);
-        if (!mbar_wait(ds_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
+        if (leader) umma_commit(dv_done);
+        if (leader) umma_commit(do_empty);
+        if (!mbar_wait_warp(ds_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
         tc_fence_after();
-        if (p.spill_ds) {
+        if (p.spill_ds && leader) {
           // the finished dS tile (bf16, [q rows][kv], scale included) also goes to global memory, where
           // the dQ kernel streams it back instead of recomputing scores
           const int head = kvh * group + t / n_qt;
@@ -536,12 +566,12 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
           tma_store_commit();
         }
         grad_product(tm_dK, adS, smem_u32(sQ + qg * Cfg::T_BYTES), t > 0);
-        umma_commit(&q_empty[qg]);
+        if (leader) umma_commit(&q_empty[qg]);
         if (++qg == Cfg::QS) qg = 0;
         if (more && !issue_dp(t + 1)) { ok = false; break; }
       }
-      if (ok) umma_commit(done);
-      if (p.spill_ds) tma_store_wait<0>();   // the stores are complete before the CTA retires
+      if (ok && leader) umma_commit(done);
+      if (p.spill_ds && leader) tma_store_wait<0>();   // the stores are complete before the CTA retires
     }
   } else {
     const int sw = warp - 2;        // 0..7
@@ -815,13 +845,13 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
       if (need_mask) {
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc)
-          bwd_chunk<true, false>(tm_S, tm_dP, lane_off, half * 2 + cc, r, lim, p.scale_log2, lse2, del * p.scale,
-                                 p.scale, nullptr, ds_buf);
+          bwd_chunk<true>(tm_S, tm_dP, lane_off, half * 2 + cc, r, lim, p.scale_log2, lse2, del * p.scale,
+                                 p.scale, ds_buf);
       } else {
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc)
-          bwd_chunk<false, false>(tm_S, tm_dP, lane_off, half * 2 + cc, r, lim, p.scale_log2, lse2, del * p.scale,
-                                  p.scale, nullptr, ds_buf);
+          bwd_chunk<false>(tm_S, tm_dP, lane_off, half * 2 + cc, r, lim, p.scale_log2, lse2, del * p.scale,
+                                  p.scale, ds_buf);
       }
       tc_fence_before();
       fence_proxy_async_smem();
