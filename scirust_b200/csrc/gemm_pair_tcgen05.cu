@@ -163,7 +163,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();          // 0 = leader, 1 = peer
   const bool leader = rank == 0;
@@ -217,7 +217,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   __syncthreads();
   cluster_sync_all();                 // both CTAs' barriers exist before anyone signals across
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
@@ -268,7 +268,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer (leader only) -------------------------------
-    if (leader && lane == 0) {
+    if (leader) {
+      // The whole warp walks through the loop and one lane issues: descriptors and addresses then stay in uniform registers.
+      // As the loop of a single thread a product took 70 to 150 cycles to issue, as long as a narrow one runs.
+      const bool issuer = elect_one();
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
@@ -279,26 +282,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       for (; ok && iter.next(sg); ++it) {
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+        if (!mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(tiles + stage * STAGE_BYTES);
-          const uint32_t sb_ = sa + A_BYTES;
+          const uint64_t da = make_smem_desc(sa, A_MN ? 64 * BK * 2 : 16, 1024);
+          const uint64_t db = make_smem_desc(sa + A_BYTES, B_MN ? 64 * BK * 2 : 16, 1024);
+          if (issuer) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t adesc = A_MN ? make_smem_desc(sa + k * (UMMA_K * 128), 64 * BK * 2, 1024)
-                                        : make_smem_desc(sa + k * (UMMA_K * 2), 16, 1024);
-            const uint64_t bdesc = B_MN ? make_smem_desc(sb_ + k * (UMMA_K * 128), 64 * BK * 2, 1024)
-                                        : make_smem_desc(sb_ + k * (UMMA_K * 2), 16, 1024);
-            umma_bf16_ss_pair(d_tmem, adesc, bdesc, idesc, (kb > sg.kb0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_bf16_ss_pair(d_tmem, smem_desc_at(da, k * (A_MN ? UMMA_K * 128 : UMMA_K * 2)),
+                                smem_desc_at(db, k * (B_MN ? UMMA_K * 128 : UMMA_K * 2)), idesc,
+                                (kb > sg.kb0 || k > 0) ? 1u : 0u);
+            umma_commit_pair(&empty_bar[stage], 3);   // frees the stage in both CTAs
           }
-          umma_commit_pair(&empty_bar[stage], 3);   // frees the stage in both CTAs
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit_pair(&tmem_full[acc], 3);
+        if (ok && issuer) umma_commit_pair(&tmem_full[acc], 3);
+        __syncwarp();
       }
     }
   } else if (warp >= 10) {

@@ -82,7 +82,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int nt = (p.N + SK_BM - 1) / SK_BM;
   const int num_kb = (p.K + BKE - 1) / BKE;
   const int items = nt * p.splits;
@@ -98,7 +98,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
   // Launched while the small kernels ahead of it (norm, quantiser, split sums) still run, a CTA brings as much of its
   // weights into L2 as its ring will hold. More takes the memory from the kernel ahead: a layer of 64 rows at Llama-3-8B
   // shape 218.4 us without, 214.2 with 8 k-blocks, 215.2 with 16, 225.2 with 64; 16 int8 rows 123.2 / 120.0 / 119.2 / 118.3.
@@ -146,7 +146,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      // The whole warp walks through the loop and one lane issues: descriptors and addresses then stay in uniform registers.
+      // As the loop of a single thread a product took 70 to 150 cycles to issue, as long as a narrow one runs.
+      const bool leader = elect_one();
       constexpr uint32_t idesc = skinny_idesc(I8, RB);
       int stage = 0;
       uint32_t phase = 0;
@@ -157,25 +160,25 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+        if (!mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_STRIDE;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES);
-          const uint32_t sb_ = sa + SK_A_BYTES;
+          const uint64_t da = make_smem_desc(sa, I8 ? 16 : 64 * 64 * 2, 1024), db = make_smem_desc(sa + SK_A_BYTES, 16, 1024);
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {               // four MMAs of 32 bytes of k each
-            const uint64_t adesc = I8 ? make_smem_desc(sa + k * 32, 16, 1024)
-                                      : make_smem_desc(sa + k * (16 * 128), 64 * 64 * 2, 1024);
-            const uint64_t bdesc = make_smem_desc(sb_ + k * 32, 16, 1024);
-            skinny_mma<I8>(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < 4; ++k)                 // four MMAs of 32 bytes of k each
+              skinny_mma<I8>(d_tmem, smem_desc_at(da, k * (I8 ? 32 : 16 * 128)), smem_desc_at(db, k * 32), idesc,
+                             (kb > kb0 || k > 0) ? 1u : 0u);
+            umma_commit(&empty_bar[stage]);
           }
-          umma_commit(&empty_bar[stage]);
           if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit(&tmem_full[acc]);
+        if (ok && leader) umma_commit(&tmem_full[acc]);
+        __syncwarp();
       }
     }
   } else {

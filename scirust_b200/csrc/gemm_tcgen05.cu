@@ -104,7 +104,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
 
   const int mt = (p.M + BM - 1) / BM;
@@ -135,7 +135,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -188,7 +188,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
-    if (lane == 0) {
+    {
+      // The whole warp walks through the loop and one lane issues: descriptors and addresses then stay in uniform registers.
+      // As the loop of a single thread a product took 70 to 150 cycles to issue, as long as a narrow one runs.
+      const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
@@ -200,26 +203,26 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int kb0 = sg.kb0, kb1 = sg.kb1;
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+        if (!mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES);
-          const uint32_t sb_ = sa + Cfg::A_BYTES;
+          const uint64_t da = make_smem_desc(sa, A_MN ? 64 * BK * 2 : 16, 1024);
+          const uint64_t db = make_smem_desc(sa + Cfg::A_BYTES, B_MN ? 64 * BK * 2 : 16, 1024);
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t adesc = A_MN ? make_smem_desc(sa + k * (UMMA_K * 128), 64 * BK * 2, 1024)
-                                        : make_smem_desc(sa + k * (UMMA_K * 2), 16, 1024);
-            const uint64_t bdesc = B_MN ? make_smem_desc(sb_ + k * (UMMA_K * 128), 64 * BK * 2, 1024)
-                                        : make_smem_desc(sb_ + k * (UMMA_K * 2), 16, 1024);
-            umma_bf16_ss(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_bf16_ss(d_tmem, smem_desc_at(da, k * (A_MN ? UMMA_K * 128 : UMMA_K * 2)),
+                           smem_desc_at(db, k * (B_MN ? UMMA_K * 128 : UMMA_K * 2)), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            umma_commit(&empty_bar[stage]);  // frees the stage once these MMAs have read it
           }
-          umma_commit(&empty_bar[stage]);  // frees the stage once these MMAs have read it
           if (++stage == Cfg::STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit(&tmem_full[acc]);
+        if (ok && leader) umma_commit(&tmem_full[acc]);
+        __syncwarp();
       }
     }
   } else {
