@@ -123,7 +123,7 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 // a whole with one lane issuing, so that descriptors stay in uniform registers: as a single thread it needed 1600 cycles
 // for the 16 gradient products, which run in 900. Until then the scores of t+1 waited for the whole softmax of t, then for a
 // stage, and then for the issuer, 3500 cycles an iteration: 8 x 2048 tokens of 16 heads, causal, the whole backward 449 us,
-// 397 now. At 128 shared memory has no room for this: the kernel below this one.
+// TIMES now. At 128 shared memory has no room for this: the kernel below this one.
 struct DkvCfg {
   static constexpr int DH = 64;
   static constexpr int NPB = 2;                       // dS^T buffers
@@ -395,8 +395,8 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
 // P is single: dV(t) has read it (dv_done) long before the exponentials of t+1 are stored. Until then the two score
 // products of an iteration were one group, which the softmax warps waited for as a whole, and at 128 the loads,
 // the scores, the softmax and the gradient products of an iteration ran one after another: 2 x 2048 tokens of 32 heads,
-// causal, 241 us then and 176 us so. At 64 the kernel above stays: its scores of t+1 and dP are one group ahead of the gradient
-// products, and forward and backward of 2 x 700 tokens of 16 heads take 85.8 us with it, 86.9 with this one.
+// causal, 241 us then and 176 us so. One thread issues here: a whole warp walking through the loop, which the kernel above gains
+// from, is level at 2 x 2048 tokens and loses 5 % at 1 x 2048.
 struct DkvSplitCfg {
   static constexpr int DH = 128;
   static constexpr int QS = 2;                        // Q stages; dO, P and dS have one
@@ -435,7 +435,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
   uint64_t* done = dv_done + 1;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
 
-  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_t = (p.S + BT - 1) / BT;
   // The kv tile is the slowest grid index: CTAs are handed out in block-id order, so all the long tiles
   // (causal: small kt, up to 4x16 query tiles) start first and the short ones fill the tail.
@@ -467,7 +467,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
   // S and dP are [query x kv] (TMEM lane = query row, as in the dQ kernel); their bf16 images P and dS
   // are stored [q rows][kv] and consumed as MN-major A operands (A^T) by the dV / dK products.
   const uint32_t tm_ST = tmem_base, tm_dPT = tmem_base + 128, tm_dK = tmem_base + 256, tm_dV = tmem_base + 256 + DH;
@@ -500,63 +500,58 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
       }
     }
   } else if (warp == 1) {
-    {
-      const bool leader = elect_one();       // the warp walks the loop as a whole, as at head dimension 64
+    if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(BT, BT, false, false);   // [q x kv], both K-major
       constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, true, true);     // [kv x dh] = A^T B, both MN-major
-      bool ok = mbar_wait_warp(kv_full, 0, p.status, ST_TIMEOUT_FULL);
+      bool ok = mbar_wait(kv_full, 0, p.status, ST_TIMEOUT_FULL);
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), adO = smem_u32(sdO), aPT = smem_u32(sPT), adS = smem_u32(sdST);
       int qn = 0;                    // Q stage and phase of the next score product
       uint32_t qn_ph = 0;
       int qg = 0;                    // Q stage of the next dK product
       // D = A B^T over DH, both K-major
       auto score_product = [&](uint32_t d, uint32_t a, uint32_t b) {
-        const uint64_t da = make_smem_desc(a, 16, 1024), db = make_smem_desc(b, 16, 1024);
-        if (!leader) return;
 #pragma unroll
         for (int k = 0; k < DH / 16; ++k) {
           const uint32_t off = (k >> 2) * (BT * 128) + (k & 3) * 32;
-          umma_bf16_ss(d, smem_desc_at(da, off), smem_desc_at(db, off), idesc_s, k > 0 ? 1u : 0u);
+          umma_bf16_ss(d, make_smem_desc(a + off, 16, 1024), make_smem_desc(b + off, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
         }
       };
       // D += A^T B over the 128 query rows, 16 at a time in both operands
       auto grad_product = [&](uint32_t d, uint32_t a, uint32_t b, bool acc) {
-        const uint64_t da = make_smem_desc(a, BT * 128, 1024), db = make_smem_desc(b, BT * 128, 1024);
-        if (!leader) return;
 #pragma unroll
         for (int k = 0; k < BT / 16; ++k)
-          umma_bf16_ss(d, smem_desc_at(da, k * (16 * 128)), smem_desc_at(db, k * (16 * 128)), idesc_g, (acc || k > 0) ? 1u : 0u);
+          umma_bf16_ss(d, make_smem_desc(a + k * (16 * 128), BT * 128, 1024),
+                       make_smem_desc(b + k * (16 * 128), BT * 128, 1024), idesc_g, (acc || k > 0) ? 1u : 0u);
       };
       auto issue_s = [&]() -> bool {
-        if (!mbar_wait_warp(&q_full[qn], qn_ph, p.status, ST_TIMEOUT_FULL)) return false;
+        if (!mbar_wait(&q_full[qn], qn_ph, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
         score_product(tm_ST, smem_u32(sQ + qn * Cfg::T_BYTES), aK);
-        if (leader) umma_commit(s_full);
+        umma_commit(s_full);
         if (++qn == Cfg::QS) { qn = 0; qn_ph ^= 1; }
         return true;
       };
       auto issue_dp = [&](int t) -> bool {
-        if (!mbar_wait_warp(do_full, t & 1, p.status, ST_TIMEOUT_FULL)) return false;
+        if (!mbar_wait(do_full, t & 1, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
         // dp_full lets the softmax warps write dS again: its last bulk store must have been read out
-        if (p.spill_ds && leader) tma_store_wait_read<0>();
-        __syncwarp();
+        if (p.spill_ds) tma_store_wait_read<0>();
         score_product(tm_dPT, adO, aV);
-        if (leader) umma_commit(dp_full);
+        umma_commit(dp_full);
         return true;
       };
       if (n_iter > 0) ok = ok && issue_s() && issue_dp(0);
       for (int t = 0; t < n_iter && ok; ++t) {
         const bool more = t + 1 < n_iter;
-        if (!mbar_wait_warp(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
+        if (!mbar_wait(p_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
         tc_fence_after();
         if (more && !issue_s()) { ok = false; break; }
         grad_product(tm_dV, aPT, adO, t > 0);
-        if (leader) umma_commit(dv_done);
-        if (leader) umma_commit(do_empty);
-        if (!mbar_wait_warp(ds_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
+        umma_commit(dv_done);
+        umma_commit(do_empty);
+        if (!mbar_wait(ds_full, t & 1, p.status, ST_TIMEOUT_MISC)) { ok = false; break; }
         tc_fence_after();
-        if (p.spill_ds && leader) {
+        if (p.spill_ds) {
           // the finished dS tile (bf16, [q rows][kv], scale included) also goes to global memory, where
           // the dQ kernel streams it back instead of recomputing scores
           const int head = kvh * group + t / n_qt;
@@ -566,12 +561,12 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
           tma_store_commit();
         }
         grad_product(tm_dK, adS, smem_u32(sQ + qg * Cfg::T_BYTES), t > 0);
-        if (leader) umma_commit(&q_empty[qg]);
+        umma_commit(&q_empty[qg]);
         if (++qg == Cfg::QS) qg = 0;
         if (more && !issue_dp(t + 1)) { ok = false; break; }
       }
-      if (ok && leader) umma_commit(done);
-      if (p.spill_ds && leader) tma_store_wait<0>();   // the stores are complete before the CTA retires
+      if (ok) umma_commit(done);
+      if (p.spill_ds) tma_store_wait<0>();   // the stores are complete before the CTA retires
     }
   } else {
     const int sw = warp - 2;        // 0..7
@@ -893,20 +888,25 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
 // When the dK/dV kernel has spilled its dS tiles (bf16 [B*H, S, S], scale included), dQ = dS K is a
 // plain streamed product: no scores, no exponentials. One CTA per (query tile, head, batch) walks the
 // kv tiles in ascending order through a TMA ring of (dS tile, K tile) pairs and accumulates in TMEM.
-// It is bound by the bytes of dS (half of S x S per head under the causal mask).
+// It is bound by the bytes of dS (half of S x S per head under the causal mask). A CTA's stream is short (16 tiles at 2048
+// tokens), so its start and its epilogue count: a stage holds half a kv tile, and two CTAs share an SM, one streaming while
+// the other starts or ends (8 x 2048 tokens of 16 heads of 64,
+// the whole backward 398 us with one CTA of twice the stages, 384 so).
 template <int DH>
 struct DqsCfg {
-  static constexpr int DS_BYTES = BT * BT * 2;
-  static constexpr int K_BYTES = BT * DH * 2;
+  static constexpr int KT = BT / 2;                      // kv rows per stage
+  static constexpr int DS_BYTES = BT * KT * 2;
+  static constexpr int K_BYTES = KT * DH * 2;
   static constexpr int STAGE_BYTES = DS_BYTES + K_BYTES;
   static constexpr int STAGES = (DH == 64) ? 4 : 3;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 128;
   static constexpr int TMEM_COLS = DH;
+  static_assert(2 * (SMEM_BYTES + 1024) <= 227 * 1024, "two CTAs per SM");
 };
 
 template <int DH>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
-attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_ds,
+__global__ void __launch_bounds__(BWD_THREADS, 2)
+attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_ds,
                                const BwdParams p) {
   using Cfg = DqsCfg<DH>;
   constexpr int NCH = DH / 64;
@@ -918,14 +918,14 @@ attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
   uint64_t* done = empty + Cfg::STAGES;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(done + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_t = (p.S + BT - 1) / BT;
   const int qt = n_t - 1 - blockIdx.z;   // slowest grid index: longest rows of tiles first over the whole grid
   const int head = blockIdx.x, b = blockIdx.y;
   const int kvh = head / (p.H / p.Hkv);
   const int q0 = qt * BT;
   const int row_base = b * p.S;
-  const int n_blocks = p.causal ? (qt + 1) : n_t;
+  const int n_blocks = 2 * (p.causal ? (qt + 1) : n_t);    // half tiles
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -933,12 +933,12 @@ attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
     fence_barrier_init();
     fence_proxy_async_smem();
   }
-  if (warp == 0 && lane == 0) { prefetch_tmap(&tm_qkv); prefetch_tmap(&tm_ds); }
+  if (warp == 0 && lane == 0) { prefetch_tmap(&tm_k); prefetch_tmap(&tm_ds); }
   if (warp == 1) { tmem_alloc(tmem_holder, Cfg::TMEM_COLS); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tm_dQ = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tm_dQ = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -949,35 +949,36 @@ attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
         uint8_t* sdS = smem + st * Cfg::STAGE_BYTES;
         uint8_t* sK = sdS + Cfg::DS_BYTES;
         mbar_arrive_expect_tx(&full[st], Cfg::STAGE_BYTES);
-        tma_load_3d(sdS, &tm_ds, &full[st], j * BT, q0, b * p.H + head);
-        tma_load_3d(sdS + BT * 128, &tm_ds, &full[st], j * BT + 64, q0, b * p.H + head);
+        tma_load_3d(sdS, &tm_ds, &full[st], j * Cfg::KT, q0, b * p.H + head);
 #pragma unroll
         for (int c = 0; c < NCH; ++c)
-          tma_load_2d(sK + c * (BT * 128), &tm_qkv, &full[st], (p.H + kvh) * DH + c * 64, row_base + j * BT);
+          tma_load_2d(sK + c * (Cfg::KT * 128), &tm_k, &full[st], (p.H + kvh) * DH + c * 64, row_base + j * Cfg::KT);
         if (++st == Cfg::STAGES) { st = 0; ph ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, false, true);
-      int st = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int j = 0; j < n_blocks && ok; ++j) {
-        if (!mbar_wait(&full[st], ph, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t adS = smem_u32(smem + st * Cfg::STAGE_BYTES), bK = adS + Cfg::DS_BYTES;
+    constexpr uint32_t idesc_g = make_idesc_bf16(BT, DH, false, true);
+    const bool leader = elect_one();
+    int st = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int j = 0; j < n_blocks && ok; ++j) {
+      ok = mbar_wait_warp(&full[st], ph, p.status, ST_TIMEOUT_FULL);
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t da = make_smem_desc(smem_u32(smem + st * Cfg::STAGE_BYTES), 16, 1024);
+      const uint64_t db = make_smem_desc(smem_u32(smem + st * Cfg::STAGE_BYTES + Cfg::DS_BYTES), Cfg::KT * 128, 1024);
+      if (leader) {
 #pragma unroll
-        for (int k = 0; k < BT / 16; ++k) {
-          const uint32_t aoff = (k >> 2) * (BT * 128) + (k & 3) * 32;
-          umma_bf16_ss(tm_dQ, make_smem_desc(adS + aoff, 16, 1024), make_smem_desc(bK + k * (16 * 128), BT * 128, 1024),
-                       idesc_g, (j > 0 || k > 0) ? 1u : 0u);
-        }
+        for (int k = 0; k < Cfg::KT / 16; ++k)
+          umma_bf16_ss(tm_dQ, smem_desc_at(da, k * 32), smem_desc_at(db, k * (16 * 128)), idesc_g, (j > 0 || k > 0) ? 1u : 0u);
         umma_commit(&empty[st]);
-        if (++st == Cfg::STAGES) { st = 0; ph ^= 1; }
       }
-      if (ok) umma_commit(done);
+      __syncwarp();
+      if (++st == Cfg::STAGES) { st = 0; ph ^= 1; }
     }
+    if (ok && leader) umma_commit(done);
+    __syncwarp();
   } else {
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
@@ -1005,6 +1006,7 @@ attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
             *reinterpret_cast<uint4*>(dst + u * 8) = w;
           }
         }
+        __syncwarp();   // rows past the end have skipped the stores; the next tensor-memory load needs the whole warp
       }
     }
   }
@@ -1015,7 +1017,7 @@ attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
 }
 
 template <int DH>
-static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& td, const CUtensorMap& tds, const BwdParams& p,
+static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& td, const CUtensorMap& tds, const BwdParams& p,
                       cudaStream_t stream) {
   constexpr int DKV_SMEM = DH == 64 ? DkvCfg::SMEM_BYTES : DkvSplitCfg::SMEM_BYTES;
   auto k1 = DH == 64 ? attention_bwd_dkv_kernel : attention_bwd_dkv_split_kernel;
@@ -1028,7 +1030,7 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& td, const CUtens
   const int n_t = (p.S + BT - 1) / BT;
   k1<<<dim3(p.Hkv, p.B, n_t), BWD_THREADS, DKV_SMEM, stream>>>(tq, td, tds, p);
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
-  if (p.spill_ds) k3<<<dim3(p.H, p.B, n_t), BWD_THREADS, DqsCfg<DH>::SMEM_BYTES, stream>>>(tq, tds, p);
+  if (p.spill_ds) k3<<<dim3(p.H, p.B, n_t), BWD_THREADS, DqsCfg<DH>::SMEM_BYTES, stream>>>(tk, tds, p);
   else k2<<<dim3(p.H, p.B, n_t), BWD_THREADS, DqCfg<DH>::SMEM_BYTES, stream>>>(tq, td, p);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
@@ -1053,8 +1055,10 @@ extern "C" int sb_attention_bwd(const void* qkv, const void* O, const float* lse
   if (B > 65535 || (S + 127) / 128 > 65535) return SB_ERR_TOO_LARGE;   // grid y / z limits
   if ((ld & 7) || (reinterpret_cast<uintptr_t>(dqkv) & 15)) return SB_ERR_ALIGN;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  CUtensorMap tq, td;
+  CUtensorMap tq, tk, td;
   int rc = make_tmap_2d_bf16(&tq, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(B) * S, ld, 64, 128);
+  if (rc) return rc;
+  rc = make_tmap_2d_bf16(&tk, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(B) * S, ld, 64, BT / 2);
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&td, dO, static_cast<uint64_t>(H) * dh, static_cast<uint64_t>(B) * S, ld_do, 64, 128);
   if (rc) return rc;
@@ -1085,5 +1089,5 @@ extern "C" int sb_attention_bwd(const void* qkv, const void* O, const float* lse
     rc = make_tmap_3d_bf16(&tds, ds_scratch, S, S, static_cast<uint64_t>(B) * H, sp, sp * S, 64, 128);
     if (rc) return rc;
   }
-  return dh == 64 ? launch_bwd<64>(tq, td, tds, p, stream) : launch_bwd<128>(tq, td, tds, p, stream);
+  return dh == 64 ? launch_bwd<64>(tq, tk, td, tds, p, stream) : launch_bwd<128>(tq, tk, td, tds, p, stream);
 }
