@@ -4,6 +4,8 @@ Outputs land in ``scirust_b200/lib/`` next to the sources so that a snapshot of 
 repository carries the binaries with it:
 
 * ``libscirust_b200_cuda.so``  - every ``csrc/*.cu`` (tcgen05 GEMM, attention, decode, comm ...)
+* ``sb_py_calls.so``           - ``csrc/py_calls.cc``: the C ABI's entry points as Python functions (left out where the
+  Python headers are missing; the calls then go through ctypes).
 * ``libscirust_b200_rt.so``    - every ``csrc/*.cpp`` (CPU runtime: fixed-order fp32 math,
   arena / paged-KV block allocators, TCP tree all-reduce, samplers); no CUDA dependency.
 
@@ -13,9 +15,11 @@ from __future__ import annotations
 
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -26,6 +30,7 @@ OBJ = LIB / "obj"
 
 CUDA_LIB = LIB / "libscirust_b200_cuda.so"
 RT_LIB = LIB / "libscirust_b200_rt.so"
+CALLS_LIB = LIB / "sb_py_calls.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -137,7 +142,6 @@ _DECL_RE = None
 def cuda_entry_points() -> list[tuple[str, str]]:
     """``(file name, declaration)`` of every ``extern "C"`` entry point defined in ``csrc/*.cu``: the C ABI of
     ``libscirust_b200_cuda.so``. Declarations are the definitions' signatures with the body cut off."""
-    import re
     global _DECL_RE
     if _DECL_RE is None:
         _DECL_RE = re.compile(r'^extern "C" ([^;{]*?\))\s*\{', re.S | re.M)
@@ -178,8 +182,31 @@ def write_api_header() -> bool:
     return True
 
 
+def build_calls(force: bool = False) -> Path | None:
+    include = Path(sysconfig.get_paths()["include"])
+    if not (include / "Python.h").exists():
+        return None
+    OBJ.mkdir(parents=True, exist_ok=True)
+    src, inc = CSRC / "py_calls.cc", OBJ / "py_calls.inc"
+    names = sorted({re.search(r"(sb_\w+)\(", decl).group(1) for _, decl in cuda_entry_points()})
+    table = "".join(f"SB_ENTRY({n})\n" for n in names)
+    if not inc.exists() or inc.read_text() != table:
+        inc.write_text(table)
+    flags = [*CXX_FLAGS, f"-I{include}", f"-I{CSRC}", f"-I{OBJ}"]
+    obj = OBJ / "py_calls.so"                 # the digest is kept beside it, as for the objects
+    deps = [CSRC / "api.h", inc]
+    if force or not CALLS_LIB.exists() or _stale(src, obj, deps, flags):
+        _run([os.environ.get("CXX", "g++"), "-shared", "-fPIC", *flags, "-o", str(obj), str(src), "-ldl"])
+        tmp = CALLS_LIB.with_suffix(".so.tmp")
+        shutil.copyfile(obj, tmp)
+        os.replace(tmp, CALLS_LIB)
+        _stamp(src, obj, deps, flags)
+    return CALLS_LIB
+
+
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_cuda(force=force, verbose=verbose)
+    build_calls(force=force)
     build_rt(force=force)
 
 

@@ -172,9 +172,42 @@ def check(rc: int, what: str) -> None:
         raise NativeError(f"{what}: {ERRORS.get(rc, rc)}")
 
 
+_calls: dict = {}           # entry point -> the function that ``call`` uses
+
+
+def _native_calls() -> dict:
+    """The entry points as functions of the extension module (csrc/py_calls.cc); empty where it is missing."""
+    import importlib.machinery
+    import importlib.util
+    path = _build.CALLS_LIB
+    if not path.exists():
+        return {}
+    loader = importlib.machinery.ExtensionFileLoader("sb_py_calls", str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("sb_py_calls", loader))
+    loader.exec_module(module)
+    return module.bind(str(_build.CUDA_LIB))
+
+
+def _bind(name: str):
+    lib = cuda()                                # loads the library
+    if not _calls:
+        _calls.update(_native_calls())
+    fn = _calls.get(name)
+    if fn is None:
+        fn = _calls[name] = getattr(lib, name)
+    return fn
+
+
 def call(name: str, *args) -> None:
-    fn = getattr(cuda(), name)
-    check(fn(*args), name)
+    fn = _calls.get(name) or _bind(name)
+    try:
+        rc = fn(*args)
+    except TypeError:
+        # arrays and references of ctypes are for ctypes, and so is an argument that neither takes
+        fn = _calls[name] = getattr(cuda(), name)
+        rc = fn(*args)
+    if rc:
+        check(rc, name)
 
 
 _status_words: dict[int, torch.Tensor] = {}

@@ -3,6 +3,7 @@ paged-KV append, split-KV GQA flash-decode, arg-max with device feedback, per-ch
 quantisation. CPU tensors take the fp32 PyTorch statement of the same arithmetic."""
 from __future__ import annotations
 
+import functools
 import math
 import os
 
@@ -26,11 +27,12 @@ _lib.register("sb_dequantize", [vp, vp, i32, i32, vp, vp])
 
 _lib.register("sb_gemm_w8", [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp])
 
+_GEMV_FMA = os.environ.get("SB_GEMV_FMA") == "1"      # as csrc/decode.cu, read once
 _ws: dict = {}
 
 
 def _workspace(n, device):
-    key = (str(device), _lib.stream())        # per stream: concurrent calls on two streams must not share scratch
+    key = (device, _lib.stream())             # per stream: concurrent calls on two streams must not share scratch
     w = _ws.get(key)
     if w is None or w.numel() < n:
         w = _lib.empty(max(n, 1 << 22), torch.float32, device)
@@ -63,7 +65,7 @@ _gemv_ws: dict = {}
 def _gemv_workspace(n, device):
     """Workspace of the GEMV: 4096 counter words (kept zero by the kernel) + split partials; one per (device,
     stream), so that GEMVs issued on two streams share neither counters nor partial sums."""
-    key = (str(device), _lib.stream())
+    key = (device, _lib.stream())
     w = _gemv_ws.get(key)
     if w is None or w.numel() < n:
         w = torch.zeros(max(n, 1 << 22), dtype=torch.float32, device=device)
@@ -149,19 +151,20 @@ def _auto_splits(N, K, cols, M=1, quant=False):
         # the tail (4096 x 128256: 213 us with one split, 176 us with eight)
         s = max(1, min(8, K // 512))
     lim = 4096                                # 16 bytes of staged X per k in the tensor-core kernels
-    if os.environ.get("SB_GEMV_FMA") == "1":
+    if _GEMV_FMA:
         mb = 1 if M <= 1 else 2 if M <= 2 else 4 if M <= 4 else 8
         lim = min(lim, 65536 // (4 * mb) // 8 * 8)
     return max(s, (K + lim - 1) // lim)
 
 
+@functools.lru_cache(maxsize=4096)       # a function of the sizes only; 3 us of a 10 us call
 def _gemv_splits(N, K, cols, M=1, quant=False):
     """k-splits of ``gemv`` and ``gemv_argmax``. Up to eight splits of a column block run as one thread-block cluster and
     finish in shared memory (csrc/decode.cu), which beats more of them that finish through memory (us, before / eight splits:
     one row 4096 x 4096 11.0 / 9.1; eight rows 20.9 / 10.4, int8 14336 x 4096 44.4 / 23.0) as long as the staged slice of X
     leaves room for two CTAs per SM: 28672 x 2048 at eight 51, at 37 27."""
     s = _auto_splits(N, K, cols, M, quant)
-    if os.environ.get("SB_GEMV_FMA") == "1":
+    if _GEMV_FMA:
         return s
     if K <= 16384:
         s = min(s, 8)
@@ -555,12 +558,11 @@ def decode_attention(q, pool, block_table, page, seq_len, H, Hkv, dh, scale=None
     ctr = _gemv_workspace(4096, q.device) if B * Hkv <= 2048 else None
     if ctr is None:
         raise ValueError("decode_attention: batch * kv_heads above 2048 is not supported")
-    part_o = ws[:B * H * n_splits * dh]
-    part_ml = ws[B * H * n_splits * dh:B * H * n_splits * (dh + 2)]
+    part_o = ws.data_ptr()                       # by offset: a slice costs as much as the launch
     out = _lib.empty((B, H * dh), BF, q.device)
     _lib.call("sb_decode_attention", q.data_ptr(), q.stride(0), pool.data_ptr(), block_table.data_ptr(),
               block_table.shape[1], page, seq_len.data_ptr(), B, H, Hkv, dh, n_splits, float(scale),
-              part_o.data_ptr(), part_ml.data_ptr(), ctr[2048:].data_ptr(), out.data_ptr(), out.stride(0),
+              part_o, part_o + B * H * n_splits * dh * 4, ctr.data_ptr() + 2048 * 4, out.data_ptr(), out.stride(0),
               _lib.stream())
     _g.launch_count += 1
     return out

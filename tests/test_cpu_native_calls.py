@@ -1,0 +1,49 @@
+"""The extension module that calls the C ABI (csrc/py_calls.cc) against ctypes; entry points that refuse their arguments return
+before they touch a device."""
+import ctypes
+
+import pytest
+
+from scirust_b200 import _build
+from scirust_b200.ops import _lib
+from scirust_b200.parallel import symm  # noqa: F401  (declares the entry points that take references)
+
+
+@pytest.fixture(scope="module")
+def calls():
+    _lib.cuda()
+    got = _lib._native_calls()
+    if not got:
+        pytest.skip("built without the Python headers")
+    return got
+
+
+def test_every_entry_point_is_there(calls):
+    import re
+    assert set(calls) == {re.search(r"(sb_\w+)\(", d).group(1) for _, d in _build.cuda_entry_points()}
+
+
+def test_arguments_and_results_are_those_of_ctypes(calls):
+    lib = _lib.cuda()
+    for name, args in (("sb_swiglu_fwd", (None, None, 0, 0, None)),                                   # bad argument
+                       ("sb_rmsnorm_fwd", (8, 16, 16, None, 1, 8, 8, 8, 1e-5, None)),                 # misaligned
+                       ("sb_attention_fwd_pp", (16, 16, None, 70000, 1, 1, 1, 64, 192, 64, 1, 1, 16, None))):   # too large
+        rc = calls[name](*args)
+        assert rc != 0 and rc == getattr(lib, name)(*args)
+        with pytest.raises(_lib.NativeError, match=_lib.ERRORS[rc]):
+            _lib.call(name, *args)
+
+
+def test_wrong_arguments_raise_type_error(calls):
+    fn = calls["sb_swiglu_fwd"]
+    for args in ((None, None, 0, 0), (None, None, 0, 0, None, None), (None, None, 0.5, 0, None), (None, None, None, 0, None),
+                 ("x", None, 0, 0, None)):
+        with pytest.raises(TypeError):
+            fn(*args)
+
+
+def test_ctypes_arrays_still_go_through_ctypes():
+    lib = _lib.cuda()
+    p, handle = ctypes.c_void_p(), (ctypes.c_char * lib.sb_ipc_handle_size())()
+    with pytest.raises(_lib.NativeError):                       # no such handle
+        _lib.call("sb_ipc_open", handle, ctypes.byref(p))
