@@ -2122,9 +2122,10 @@ static int launch_gemv_mma(const GemvParams& p, int splits, cudaStream_t s) {
   static PerDeviceOnce attr;
   if (allow_smem(attr, kern, GEMV_STAGES * GEMV_TILE_BYTES + GEMV_MAX_XS_BYTES + 1024, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   const dim3 grid((p.N + COLS - 1) / COLS, splits);
-  const bool waits_for_peers = p.coll.W > 1 || p.amax.W > 1;
-  return launch_dep_cluster(kern, grid, dim3(GEMV_THREADS), smem, s, CLUSTER ? splits : 1, !waits_for_peers, tm, p) ==
-                 cudaSuccess ? 0 : SB_ERR_LAUNCH;
+  // In plain stream order: two or three CTAs share an SM, and CTAs that are placed while the predecessor drains crowd the
+  // SMs that it leaves first, for the whole stream. The kernel after this one may start early (pdl_trigger).
+  return launch_dep_cluster(kern, grid, dim3(GEMV_THREADS), smem, s, CLUSTER ? splits : 1, false, tm, p) == cudaSuccess
+             ? 0 : SB_ERR_LAUNCH;
 }
 
 // Y[M,N] = f(X)[M,K] * W[K,N] (* scale[n]) (+ R). M <= 8 per call (callers loop over row groups).

@@ -363,3 +363,26 @@ def test_dependent_launches_read_what_their_predecessor_wrote(rows, quant):
     finally:
         _lib.call("sb_set_pdl", 1)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("M,K,N,splits", [(1, 1024, 264 + 8, 8), (8, 992, 1552, 8), (3, 4096, 4096, 8), (5, 200, 16, 3),
+                                          (1, 2816, 1024, 8), (8, 14336, 4096, 8), (2, 4096, 22016, 3), (7, 4096, 28672, 5)])
+def test_splits_that_finish_in_a_cluster_give_the_bits_of_the_finish_through_memory(quant, M, K, N, splits):
+    """Grids of narrow and of wide column blocks, ragged last blocks, k ranges that end inside a tile: the fused LM head keeps
+    the finish through memory, adds in the same order and so has the same logits; an output and a residual at odd addresses
+    give the bits of aligned ones."""
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N)
+    x = (torch.randn(M, K, generator=g, device="cuda") * 0.5).to(BF)
+    w = (torch.randn(K, N, generator=g, device="cuda") * 0.05).to(BF)
+    wt = D.quantize_per_channel(w) if quant else w
+    lg, lg2 = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    D.gemv(x, wt, out_f32=lg, splits=splits)
+    D.gemv_argmax(x, wt, logits=lg2, splits=splits)
+    assert torch.equal(lg, lg2)
+    ref = x.double() @ (wt.q.double() * wt.scale.double() if quant else w.double())
+    assert ((lg.double() - ref).norm() / ref.norm()).item() < 1e-5       # fp32 sums of exact products
+    r = torch.randn(M, N + 1, generator=g, device="cuda").to(BF)
+    wide = torch.empty(M, N + 3, dtype=BF, device="cuda")
+    D.gemv(x, wt, residual=r[:, 1:], out=wide[:, 1:N + 1], splits=splits)
+    assert torch.equal(wide[:, 1:N + 1], D.gemv(x, wt, residual=r[:, 1:].contiguous(), splits=splits))
