@@ -129,7 +129,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const AttParams p
   uint64_t* o_full = p_full + 1;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(o_full + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_qt = (p.S + ATT_BM - 1) / ATT_BM;
   const int qt = n_qt - 1 - blockIdx.z;  // slowest grid index: longest (most kv blocks) tiles first over the whole grid
   const int head = blockIdx.x, b = blockIdx.y;
@@ -159,7 +159,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const AttParams p
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
   const uint32_t tmem_S = tmem_base;
   const uint32_t tmem_O = tmem_base + 128;
 
@@ -188,41 +188,47 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const AttParams p
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      // the whole warp walks through the loop and one lane issues: descriptors stay in uniform registers
+      const bool leader = elect_one();
+      const uint64_t dq = make_smem_desc(smem_u32(sQ), 16, 1024), dp = make_smem_desc(smem_u32(sP), 16, 1024);
       constexpr uint32_t idesc_s = make_idesc_bf16(ATT_BM, ATT_BN, false, false);
       constexpr uint32_t idesc_o = make_idesc_bf16(ATT_BM, DH, false, true);
       int ks = 0, vs = 0;
       uint32_t kph = 0, vph = 0;
-      bool ok = mbar_wait(q_full, 0, p.status, ST_TIMEOUT_FULL);
+      bool ok = mbar_wait_warp(q_full, 0, p.status, ST_TIMEOUT_FULL);
       auto issue_s = [&]() -> bool {
-        if (!mbar_wait(&k_full[ks], kph, p.status, ST_TIMEOUT_FULL)) return false;
+        if (!mbar_wait_warp(&k_full[ks], kph, p.status, ST_TIMEOUT_FULL)) return false;
         tc_fence_after();
-        const uint32_t aq = smem_u32(sQ), bk = smem_u32(sK + ks * Cfg::KV_BYTES);
+        const uint64_t dk = make_smem_desc(smem_u32(sK + ks * Cfg::KV_BYTES), 16, 1024);
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < DH / 16; ++k) {
-          const uint32_t off = (k >> 2) * (ATT_BM * 128) + (k & 3) * 32;
-          umma_bf16_ss(tmem_S, make_smem_desc(aq + off, 16, 1024), make_smem_desc(bk + off, 16, 1024), idesc_s,
-                       k > 0 ? 1u : 0u);
+          for (int k = 0; k < DH / 16; ++k) {
+            const uint32_t off = (k >> 2) * (ATT_BM * 128) + (k & 3) * 32;
+            umma_bf16_ss(tmem_S, smem_desc_at(dq, off), smem_desc_at(dk, off), idesc_s, k > 0 ? 1u : 0u);
+          }
+          umma_commit(&k_empty[ks]);
+          umma_commit(s_full);
         }
-        umma_commit(&k_empty[ks]);
-        umma_commit(s_full);
+        __syncwarp();
         if (++ks == Cfg::KS) { ks = 0; kph ^= 1; }
         return true;
       };
       if (ok) ok = issue_s();
       for (int j = 0; j < n_blocks && ok; ++j) {
-        if (!mbar_wait(p_full, j & 1, p.status, ST_TIMEOUT_MISC)) break;
-        if (!mbar_wait(&v_full[vs], vph, p.status, ST_TIMEOUT_FULL)) break;
+        if (!mbar_wait_warp(p_full, j & 1, p.status, ST_TIMEOUT_MISC)) break;
+        if (!mbar_wait_warp(&v_full[vs], vph, p.status, ST_TIMEOUT_FULL)) break;
         tc_fence_after();
-        const uint32_t ap = smem_u32(sP), bv = smem_u32(sV + vs * Cfg::KV_BYTES);
+        const uint64_t dv = make_smem_desc(smem_u32(sV + vs * Cfg::KV_BYTES), ATT_BN * 128, 1024);
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < ATT_BN / 16; ++k) {
-          const uint64_t adesc = make_smem_desc(ap + (k >> 2) * (ATT_BM * 128) + (k & 3) * 32, 16, 1024);
-          const uint64_t bdesc = make_smem_desc(bv + k * (16 * 128), ATT_BN * 128, 1024);
-          umma_bf16_ss(tmem_O, adesc, bdesc, idesc_o, k > 0 ? 1u : 0u);
+          for (int k = 0; k < ATT_BN / 16; ++k)
+            umma_bf16_ss(tmem_O, smem_desc_at(dp, (k >> 2) * (ATT_BM * 128) + (k & 3) * 32), smem_desc_at(dv, k * (16 * 128)),
+                         idesc_o, k > 0 ? 1u : 0u);
+          umma_commit(&v_empty[vs]);
+          umma_commit(o_full);
         }
-        umma_commit(&v_empty[vs]);
-        umma_commit(o_full);
+        __syncwarp();
         if (++vs == Cfg::VS) { vs = 0; vph ^= 1; }
         if (j + 1 < n_blocks) ok = issue_s();
       }

@@ -73,7 +73,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int mt = (p.M + I8_BM - 1) / I8_BM, nt = (p.N + I8_BN - 1) / I8_BN;
   const int num_kb = (p.K + I8_BK - 1) / I8_BK;
   const int tiles_total = mt * nt * p.splits;
@@ -89,7 +89,7 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_holder);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(tmem_holder), 0);
 
   // work item t: split = t / (mt * nt), tile = t % (mt * nt), n index major so that CTAs next to one another share A
   if (warp == 0) {
@@ -115,7 +115,9 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      // the whole warp walks through the loop and one lane issues: descriptors stay in uniform registers
+      const bool leader = elect_one();
       constexpr uint32_t idesc = make_idesc_i8(I8_BM, I8_BN);
       int stage = 0;
       uint32_t phase = 0;
@@ -126,24 +128,25 @@ gemm_i8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
+        if (!mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * I8_BN;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(tiles + stage * I8_STAGE_BYTES);
-          const uint32_t sb_ = sa + I8_A_BYTES;
+          const uint64_t da = make_smem_desc(sa, 16, 1024), db = make_smem_desc(sa + I8_A_BYTES, 16, 1024);
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < I8_BK / I8_UMMA_K; ++k) {
-            const uint64_t adesc = make_smem_desc(sa + k * I8_UMMA_K, 16, 1024);
-            const uint64_t bdesc = make_smem_desc(sb_ + k * I8_UMMA_K, 16, 1024);
-            umma_i8_ss(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < I8_BK / I8_UMMA_K; ++k)
+              umma_i8_ss(d_tmem, smem_desc_at(da, k * I8_UMMA_K), smem_desc_at(db, k * I8_UMMA_K), idesc,
+                         (kb > kb0 || k > 0) ? 1u : 0u);
+            umma_commit(&empty_bar[stage]);
           }
-          umma_commit(&empty_bar[stage]);
           if (++stage == I8_STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit(&tmem_full[acc]);
+        if (ok && leader) umma_commit(&tmem_full[acc]);
+        __syncwarp();
       }
     }
   } else {
