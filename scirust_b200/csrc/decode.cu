@@ -35,21 +35,19 @@ __device__ __forceinline__ uint32_t dpack(float lo, float hi) {
 // and the k range of its split.
 //   warp 8      producer: streams the CTA's weight slab through a ring of STAGES tiles of 32 rows,
 //               one 16 KB TMA tile copy and one mbarrier per stage (copies of single 512-byte rows
-//               reached less than half of the memory bandwidth); it starts at once, because the
-//               weights do not depend on the previous kernel's output
+//               reached less than half of the memory bandwidth)
 //   warps 0-7   stage f(X) for the CTA's k range in shared memory (optionally fused RMSNorm or
 //               SwiGLU), then consume tiles: warp w takes rows w, w+8, w+16, w+24 of every tile, a
 //               lane holds VEC consecutive columns
 // Partials of the 8 warps are added in warp order in shared memory; split partials go to a
 // workspace and the LAST CTA of a column block (a counter, no data atomics) adds them in split
 // order and applies scale / residual: the summation tree depends only on (K, splits), and the
-// finishing pass needs no second launch.
+// finishing pass needs no second launch. (Up to eight splits of the tensor-core kernels below finish in a cluster.)
 // INT8: W is int8 with one fp32 scale per output column, applied after the sum.
 // ---------------------------------------------------------------------------
 constexpr int GEMV_KT = 32;          // rows per tile
 constexpr int GEMV_ROW_BYTES = 512;  // bytes of one weight row owned by a CTA
-constexpr int GEMV_STAGES = 4;   // 64 KB ring: three CTAs fit on an SM, so a dependent kernel's CTAs
-                                 // find room to prefetch their weights while this kernel still runs
+constexpr int GEMV_STAGES = 4;       // 64 KB ring: two or three CTAs fit on an SM
 constexpr int GEMV_TILE_BYTES = GEMV_KT * GEMV_ROW_BYTES;
 constexpr int GEMV_THREADS = 288;
 constexpr int GEMV_MAX_XS_BYTES = 64 * 1024;
