@@ -13,12 +13,16 @@
 //   int8 (I8 = true):  W8A8 of the reference's quantised linear layer (scirust-core/src/quantization.rs:150-190):
 //                      weights as the transposed codes [N, K], activations quantised per row; kind::i8, int32
 //                      accumulation (exact), one rescale by sx[m] * sw[n].
-// Split-K partials (fp32 / int32, [split][row][N]) are added in split order by skinny_reduce_kernel.
+// Split-K partials (fp32 / int32) are added in split order: inside a thread-block cluster, whose CTAs are the splits of one
+// column tile, where all these clusters are on the GPU at once (it holds 33 of four CTAs, 45 of three), else by
+// skinny_reduce_kernel from [split][row][N] in memory (us with that kernel / in the cluster: 4096 x 4096, 16 rows 10.4 / 9.1,
+// 64 rows 12.9 / 10.5, int8 13.3 / 11.9; 14336 x 4096, 64 rows 25.8 / 23.6).
 // Warps: 0 TMA, 1 MMA, 2-5 epilogue (one per TMEM lane quarter).
 #include "sm100_ptx.cuh"
 #include "api.h"
 #include "per_device.h"
 #include "dependent.cuh"
+#include <atomic>
 
 namespace sb {
 
@@ -28,6 +32,7 @@ int num_sms();
 
 constexpr int SK_BM = 128;          // output columns per tile (the MMA's M)
 constexpr int SK_THREADS = 192;
+constexpr int SK_MAX_CLUSTER = 6;   // splits that finish in a cluster
 constexpr int SK_A_BYTES = 16384;   // 128 columns x (64 bf16 | 128 int8) of k
 
 template <int RB>
@@ -67,7 +72,7 @@ __device__ __forceinline__ void skinny_mma(uint32_t d_tmem, uint64_t a_desc, uin
   }
 }
 
-template <int RB, bool I8>
+template <int RB, bool I8, bool CLUSTER>
 __global__ void __launch_bounds__(SK_THREADS, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const SkinnyParams p) {
@@ -85,7 +90,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int nt = (p.N + SK_BM - 1) / SK_BM;
   const int num_kb = (p.K + BKE - 1) / BKE;
+  // CLUSTER: grid (column tiles, splits), one item per CTA; else a CTA walks over items split-major
   const int items = nt * p.splits;
+  const int first = CLUSTER ? blockIdx.y * nt + blockIdx.x : blockIdx.x, step = CLUSTER ? items : gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -104,7 +111,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   // shape 218.4 us without, 214.2 with 8 k-blocks, 215.2 with 16, 225.2 with 64; 16 int8 rows 123.2 / 120.0 / 119.2 / 118.3.
   pdl_trigger();
   if (warp == 0 && lane == 0) {
-    const int split = blockIdx.x / nt, n_idx = blockIdx.x - split * nt;
+    const int split = first / nt, n_idx = first - split * nt;
     const int kb0 = split * p.kb_per_split, kb1 = min(min(num_kb, kb0 + p.kb_per_split), kb0 + Cfg::STAGES);
     for (int kb = kb0; kb < kb1; ++kb) {
       if constexpr (I8) {
@@ -123,7 +130,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+      for (int t = first; t < items && ok; t += step) {
         const int split = t / nt, n_idx = t - split * nt;
         const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -155,7 +162,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       uint32_t phase = 0;
       bool ok = true;
       int it = 0;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x, ++it) {
+      for (int t = first; t < items && ok; t += step, ++it) {
         const int split = t / nt;
         const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
         const int acc = it & 1;
@@ -185,7 +192,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const int q = warp & 3;                             // warps 2, 3, 4, 5 -> lane quarters 2, 3, 0, 1
     bool ok = true;
     int it = 0;
-    for (int t = blockIdx.x; t < items && ok; t += gridDim.x, ++it) {
+    for (int t = first; t < items && ok; t += step, ++it) {
       const int split = t / nt, n_idx = t - split * nt;
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
@@ -200,7 +207,12 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
         tmem_ld_wait();
-        if (col < p.N) {
+        if constexpr (CLUSTER) {                        // the ring is idle: every stage has been multiplied
+          uint32_t* vals = reinterpret_cast<uint32_t*>(tiles);
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (c * 32 + j < RB) vals[(c * 32 + j) * SK_BM + q * 32 + lane] = r[j];
+        } else if (col < p.N) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int m = c * 32 + j;
@@ -227,6 +239,66 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   __syncthreads();
   tc_fence_after();
   if (warp == 1) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  if constexpr (CLUSTER) {
+    // CTA r adds its share of the tile's (row, four columns) words over all splits, in split order
+    __syncwarp();
+    cluster_sync_all();
+    const int c = p.splits, rank = blockIdx.y;
+    const int words = p.rows * (SK_BM / 4), w1 = (rank + 1) * words / c;
+    int i = rank * words / c + threadIdx.x;             // SK_THREADS is a multiple of a row's 32 words: the columns stay
+    const int col4 = (i & (SK_BM / 4 - 1)) * 4, n = blockIdx.x * SK_BM + col4;
+    const bool live = n < p.N;                          // N is a multiple of 8
+    const __nv_bfloat16* R = static_cast<const __nv_bfloat16*>(p.R);
+    __nv_bfloat16* C = static_cast<__nv_bfloat16*>(p.C);
+    const bool wide = ((p.ldc | p.ldr) & 3) == 0 && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(R)) & 7) == 0;
+    float sw[4] = {0.f, 0.f, 0.f, 0.f};
+    if (I8 && live) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sw[e] = p.sw[n + e];
+    }
+    const uint32_t base = smem_u32(tiles) + col4 * 4;
+#pragma unroll 2
+    for (; live && i < w1; i += SK_THREADS) {
+      const int m = i / (SK_BM / 4);
+      float4 v[SK_MAX_CLUSTER];
+#pragma unroll
+      for (int s = 0; s < SK_MAX_CLUSTER; ++s)
+        if (s < c) v[s] = ld_cluster_f4(mapa_shared(base + m * SK_BM * 4, s));
+      float f[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+      if constexpr (I8) {
+        const float sx = p.sx[m];
+        int acc[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int s = 0; s < SK_MAX_CLUSTER; ++s)
+          if (s < c) {
+            acc[0] += __float_as_int(v[s].x); acc[1] += __float_as_int(v[s].y);
+            acc[2] += __float_as_int(v[s].z); acc[3] += __float_as_int(v[s].w);
+          }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) f[e] = __fmul_rn(static_cast<float>(acc[e]), __fmul_rn(sx, sw[e]));
+      } else {
+#pragma unroll
+        for (int s = 1; s < SK_MAX_CLUSTER; ++s)
+          if (s < c) { f[0] += v[s].x; f[1] += v[s].y; f[2] += v[s].z; f[3] += v[s].w; }
+      }
+      const __nv_bfloat16* res = R ? R + static_cast<size_t>(m) * p.ldr + n : nullptr;
+      __nv_bfloat16* out = C + static_cast<size_t>(m) * p.ldc + n;
+      if (wide) {
+        if (res) {
+          const uint2 w = *reinterpret_cast<const uint2*>(res);
+          f[0] += bf16_lo(w.x); f[1] += bf16_hi(w.x); f[2] += bf16_lo(w.y); f[3] += bf16_hi(w.y);
+        }
+        *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (res) f[e] += __bfloat162float(res[e]);
+          out[e] = __float2bfloat16_rn(f[e]);
+        }
+      }
+    }
+    cluster_sync_all();                                 // nobody leaves while its sums are being read
+  }
 }
 
 // C[m, n] = bf16(sum over splits in split order (+ scales) + R[m, n]). Four columns (16 bytes of every partial) per thread
@@ -275,14 +347,52 @@ skinny_reduce_kernel(const uint32_t* part, int splits, int rows, int N4, const f
   }
 }
 
+// Clusters of `c` CTAs that the current device holds at once; asked for once per device and size.
 template <int RB, bool I8>
-static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int grid,
+static int skinny_clusters(int c) {
+  auto kern = gemm_skinny_kernel<RB, I8, true>;
+  static std::atomic<int> known[64][SK_MAX_CLUSTER + 1] = {};      // count + 1
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return 0;
+  const bool keep = device >= 0 && device < 64;
+  if (keep) {
+    const int k = known[device][c].load(std::memory_order_relaxed);
+    if (k > 0) return k - 1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, c); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = SkinnyCfg<RB>::SMEM_BYTES;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = c; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+  if (keep) known[device][c].store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
+// in_cluster: set when the splits finish inside the kernel, p.C is then the output. `workspace` takes the partials otherwise.
+template <int RB, bool I8>
+static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, SkinnyParams p, void* workspace, bool* in_cluster,
                          cudaStream_t stream) {
   using Cfg = SkinnyCfg<RB>;
-  auto kern = gemm_skinny_kernel<RB, I8>;
-  static PerDeviceOnce attr;
+  const int nt = (p.N + SK_BM - 1) / SK_BM;
+  auto clustered = gemm_skinny_kernel<RB, I8, true>;
+  static PerDeviceOnce attr, attr_c;
+  *in_cluster = false;
+  if (p.splits > 1 && p.splits <= SK_MAX_CLUSTER) {
+    if (allow_smem(attr_c, clustered, Cfg::SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
+    *in_cluster = nt <= skinny_clusters<RB, I8>(p.splits);
+  }
+  if (*in_cluster)
+    return launch_dep_cluster(clustered, dim3(nt, p.splits), dim3(SK_THREADS), Cfg::SMEM_BYTES, stream, p.splits, true, tw, tx,
+                              p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+  auto kern = gemm_skinny_kernel<RB, I8, false>;
   if (allow_smem(attr, kern, Cfg::SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
-  return launch_dep(kern, dim3(grid), dim3(SK_THREADS), Cfg::SMEM_BYTES, stream, tw, tx, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+  if (p.splits > 1) p.C = workspace;
+  const int items = nt * p.splits;
+  return launch_dep(kern, dim3(items < num_sms() ? items : num_sms()), dim3(SK_THREADS), Cfg::SMEM_BYTES, stream, tw, tx, p) ==
+                 cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
 }  // namespace sb
@@ -294,7 +404,7 @@ using namespace sb;
 //   is_i8 == 1: X int8 [rows, ldx] with row scales sx, W int8 [N, K] (transposed codes, row pitch ldw, K % 16 == 0)
 //               with column scales sw.
 // Bases 16-byte aligned, pitches multiples of 16 bytes, N % 8 == 0. workspace: splits * rows * N 32-bit words, read
-// only when the k range is split (splits <= 0 lets the launcher fill the GPU: about one work item per SM).
+// only when the k range is split and its splits do not finish in a cluster (splits <= 0 lets the launcher fill the GPU: about one work item per SM).
 extern "C" int sb_gemm_skinny(const void* X, int ldx, const void* W, int ldw, void* C, int ldc, const void* R, int ldr,
                               int rows, int N, int K, int is_i8, const float* sx, const float* sw, int splits,
                               void* workspace, int* status, void* stream_) {
@@ -330,15 +440,15 @@ extern "C" int sb_gemm_skinny(const void* X, int ldx, const void* W, int ldw, vo
   if (rc) return rc;
   SkinnyParams p;
   p.rows = rows; p.N = N; p.K = K; p.splits = splits; p.kb_per_split = kbps;
-  p.C = splits > 1 ? workspace : C; p.ldc = ldc; p.R = R; p.ldr = ldr; p.sx = sx; p.sw = sw; p.status = status;
-  const int items = nt * splits;
-  const int grid = items < num_sms() ? items : num_sms();
-#define SB_SKINNY(RB_)                                                              \
-  rc = is_i8 ? launch_skinny<RB_, true>(tw, tx, p, grid, stream) : launch_skinny<RB_, false>(tw, tx, p, grid, stream)
+  p.C = C; p.ldc = ldc; p.R = R; p.ldr = ldr; p.sx = sx; p.sw = sw; p.status = status;
+  bool in_cluster = false;
+#define SB_SKINNY(RB_)                                                                            \
+  rc = is_i8 ? launch_skinny<RB_, true>(tw, tx, p, workspace, &in_cluster, stream)                \
+             : launch_skinny<RB_, false>(tw, tx, p, workspace, &in_cluster, stream)
   if (rb == 16) SB_SKINNY(16); else if (rb == 32) SB_SKINNY(32); else SB_SKINNY(64);
 #undef SB_SKINNY
   if (rc) return rc;
-  if (splits > 1) {
+  if (splits > 1 && !in_cluster) {
     const dim3 grid_r((N / 4 + 127) / 128, rows);          // N is a multiple of 8
     auto kern = is_i8 ? skinny_reduce_kernel<true> : skinny_reduce_kernel<false>;
     if (launch_dep(kern, grid_r, dim3(128), 0, stream, static_cast<const uint32_t*>(workspace), splits, rows, N / 4, sx, sw,

@@ -386,3 +386,25 @@ def test_splits_that_finish_in_a_cluster_give_the_bits_of_the_finish_through_mem
     wide = torch.empty(M, N + 3, dtype=BF, device="cuda")
     D.gemv(x, wt, residual=r[:, 1:], out=wide[:, 1:N + 1], splits=splits)
     assert torch.equal(wide[:, 1:N + 1], D.gemv(x, wt, residual=r[:, 1:].contiguous(), splits=splits))
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("M,K,N,splits", [(9, 1040, 8, 2), (33, 1040, 136, 3), (64, 4096, 4096, 4), (17, 2816, 1544, 5), (64, 4096, 1032, 6),
+                                          (48, 4096, 6144, 3)])
+def test_skinny_splits_in_a_cluster(quant, M, K, N, splits):
+    """Splits that finish inside a cluster (and 48 tiles of three, which do not all fit and finish through memory): int8 sums
+    are exact, so any split has the bits of none; bf16 sums against float64. Residual and output at odd addresses."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, generator=g, device="cuda").to(BF)
+    w = (torch.randn(K, N, generator=g, device="cuda") * 0.05).to(BF)
+    r = torch.randn(M, N + 1, generator=g, device="cuda").to(BF)[:, 1:]
+    wide = torch.zeros(M, N + 3, dtype=BF, device="cuda")
+    wt = D.quantize_per_channel(w) if quant else w
+    D.matmul_skinny(x, wt, residual=r, out=wide[:, 1:N + 1], splits=splits)
+    got = D.matmul_skinny(x, wt, residual=r.contiguous(), splits=splits)
+    assert torch.equal(wide[:, 1:N + 1], got) and not wide[:, 0].any() and not wide[:, N + 1:].any()
+    if quant:
+        assert torch.equal(got, D.matmul_skinny(x, wt, residual=r, splits=1))
+    else:
+        ref = x.double() @ w.double() + r.double()
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8      # one rounding to bf16
