@@ -123,7 +123,7 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 // a whole with one lane issuing, so that descriptors stay in uniform registers: as a single thread it needed 1600 cycles
 // for the 16 gradient products, which run in 900. Until then the scores of t+1 waited for the whole softmax of t, then for a
 // stage, and then for the issuer, 3500 cycles an iteration: 8 x 2048 tokens of 16 heads, causal, the whole backward 449 us,
-// TIMES now. At 128 shared memory has no room for this: the kernel below this one.
+// 384 now (with the dQ stream below). At 128 shared memory has no room for this: the kernel below this one.
 struct DkvCfg {
   static constexpr int DH = 64;
   static constexpr int NPB = 2;                       // dS^T buffers
