@@ -54,6 +54,23 @@ def test_forward_growing_maxima(causal, monkeypatch):
     assert (o.float() - o1.float()).abs().max().item() < 2e-2 and (lse - lse1).abs().max().item() < 1e-3
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,S,H,Hkv,dh", [(2, 300, 4, 2, 64), (1, 300, 2, 1, 128), (1, 513, 2, 2, 128)])
+@pytest.mark.parametrize("two_tiles", [True, False])
+def test_forward_takes_any_scale(two_tiles, B, S, H, Hkv, dh, causal, scale, monkeypatch):
+    # a masked weight is zero whatever the scale makes of its score: at zero every visible key weighs the same
+    monkeypatch.setattr(A, "FWD_TWO_TILES", two_tiles)
+    monkeypatch.setattr(A, "_two_tiles_win", lambda *a: True)
+    qkv = _qkv(B, S, H, Hkv, dh, seed=11)
+    o, lse = A.attention_fwd(qkv, B, S, H, Hkv, dh, causal=causal, scale=scale)
+    _lib.check_status()
+    o_ref, lse_ref = A.attention_ref(qkv, B, S, H, Hkv, dh, causal=causal, scale=scale)
+    # weights and output are rounded to bf16 once each (2^-9 of values of up to 5); sums are fp32
+    assert (o.float() - o_ref).abs().max().item() < 3e-2
+    assert (lse - lse_ref).abs().max().item() < 1e-3
+
+
 @pytest.mark.parametrize("B,S,H,Hkv,dh", CASES)
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("spill", [True, False])
