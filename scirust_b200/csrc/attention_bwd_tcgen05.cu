@@ -123,7 +123,7 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 // a whole with one lane issuing, so that descriptors stay in uniform registers: as a single thread it needed 1600 cycles
 // for the 16 gradient products, which run in 900. Until then the scores of t+1 waited for the whole softmax of t, then for a
 // stage, and then for the issuer, 3500 cycles an iteration: 8 x 2048 tokens of 16 heads, causal, the whole backward 449 us,
-// 384 now (with the dQ stream below). At 128 shared memory has no room for this: the kernel below this one.
+// 375 now (with the dQ stream below). At 128 shared memory has no room for this: the kernel below this one.
 struct DkvCfg {
   static constexpr int DH = 64;
   static constexpr int NPB = 2;                       // dS^T buffers
@@ -309,7 +309,7 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
       int lim = min(diag ? r : BT - 1, p.S - 1 - kv0);
       if (q_idx >= p.S) lim = -1;
       const bool need_mask = diag || (q0 + BT > p.S) || (kv0 + BT > p.S);
-      if (!mbar_wait(st_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(st_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       // P = 2^(s * sl2 - lse2), dS = P * (dP * scale - delta * scale)
       uint32_t pv[64], dv[64];
@@ -341,7 +341,7 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
         pv[i >> 1] = pack_bf16x2(__uint_as_float(pv[i]), __uint_as_float(pv[i + 1]));
       }
       // dV(t-1) has read P; the dS buffer of this parity was let go of before
-      if (t > 0 && !mbar_wait(dv_done, (t - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (t > 0 && !mbar_wait_warp(dv_done, (t - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc) {
         store_row32_sw128(sPT, r, half * 2 + cc, pv + cc * 16);
@@ -352,7 +352,7 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __gri
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
-    if (ok && mbar_wait(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
+    if (ok && mbar_wait_warp(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       constexpr int CPW = DH / 64;  // 32-column chunks per warp and matrix
 #pragma unroll 1
@@ -587,7 +587,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
       int lim = min(diag ? r : BT - 1, p.S - 1 - kv0);
       if (q_idx >= p.S) lim = -1;
       const bool need_mask = diag || (q0 + BT > p.S) || (kv0 + BT > p.S);
-      if (!mbar_wait(s_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       // P = 2^(s * sl2 - lse2), kept in fp32 registers for dS
       uint32_t pv[64];
@@ -605,7 +605,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
         for (int i = 0; i < 64; ++i)
           if (half * 64 + i > lim) pv[i] = 0u;
       }
-      if (t > 0 && !mbar_wait(dv_done, (t - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (t > 0 && !mbar_wait_warp(dv_done, (t - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc) {
         uint32_t pk[16];
@@ -619,7 +619,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
       // dS = P * (dP * scale - delta * scale)
-      if (!mbar_wait(dp_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(dp_full, t & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const float neg_delta = -sd.y * p.scale;
 #pragma unroll
@@ -640,7 +640,7 @@ attention_bwd_dkv_split_kernel(const __grid_constant__ CUtensorMap tm_qkv, const
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
     }
-    if (ok && mbar_wait(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
+    if (ok && mbar_wait_warp(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       constexpr int CPW = DH / 64;  // 32-column chunks per warp and matrix
 #pragma unroll 1
@@ -829,7 +829,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
     }
     bool ok = true;
     for (int j = 0; j < n_blocks; ++j) {
-      if (!mbar_wait(s_full, j & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, j & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const int kv0 = j * BT;
       const bool diag = p.causal && j == n_blocks - 1;
@@ -853,7 +853,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
-    if (ok && mbar_wait(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
+    if (ok && mbar_wait_warp(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       constexpr int CPW = DH / 64;
 #pragma unroll 1
@@ -985,7 +985,7 @@ attention_bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const _
     const int r = q * 32 + lane;
     const int q_idx = q0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    if (mbar_wait(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
+    if (mbar_wait_warp(done, 0, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
       constexpr int CPW = DH / 64;
 #pragma unroll 1

@@ -245,7 +245,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const AttParams p
     for (int i = 0; i < DH; ++i) o[i] = 0.f;
     bool ok = true;
     for (int j = 0; j < n_blocks; ++j) {
-      if (!mbar_wait(s_full, j & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, j & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const int kv0 = j * ATT_BN;
       const bool need_mask = (p.causal && j == n_blocks - 1) || (kv0 + ATT_BN > p.S);
@@ -259,7 +259,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const AttParams p
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
-      if (!mbar_wait(o_full, j & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(o_full, j & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll
       for (int c = 0; c < DH / 32; ++c) {

@@ -351,7 +351,7 @@ gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
     pdl_wait();
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
-      if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
+      if (t >= GEMV_STAGES && !mbar_wait_warp(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
       if (lane == 0) {
         // rows past K and columns past N arrive as zeros and still count towards the byte total
         mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
@@ -431,7 +431,7 @@ gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
     const bool active = lane * VEC < min(COLS, N - col0);
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
-      if (!mbar_wait(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
+      if (!mbar_wait_warp(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
       const int rows = min(GEMV_KT, k1 - (k0 + t * GEMV_KT));
       const uint8_t* tile = tiles + s * GEMV_TILE_BYTES;
       uint4 raw[4];
@@ -602,7 +602,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     pdl_wait();
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
-      if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
+      if (t >= GEMV_STAGES && !mbar_wait_warp(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
       if (lane == 0) {
         // rows past K and columns past N arrive as zeros and still count towards the byte total
         mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
@@ -733,7 +733,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     const uint32_t tiles_u32 = smem_u32(tiles) + sub * (KT * 128);
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
-      if (!mbar_wait(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
+      if (!mbar_wait_warp(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
       const uint32_t tbase = tiles_u32 + s * GEMV_TILE_BYTES;
 #pragma unroll
       for (int ks = 0; ks < KT / 16; ++ks) {
@@ -899,7 +899,7 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     pdl_wait();
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
-      if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
+      if (t >= GEMV_STAGES && !mbar_wait_warp(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
       if (lane == 0) {
         // rows past K and columns past N arrive as zeros and still count towards the byte total
         mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
@@ -1035,7 +1035,7 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const __half2 bias = __floats2half2_rn(1152.f, 1152.f);   // 1024 (the magic exponent) + 128 (the sign flip)
     for (int t = 0; t < ntiles; ++t) {
       const int s = t % GEMV_STAGES;
-      if (!mbar_wait(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
+      if (!mbar_wait_warp(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
       const uint32_t tbase = tiles_u32 + s * GEMV_TILE_BYTES;
 #pragma unroll
       for (int ks = 0; ks < KT / 16; ++ks) {
@@ -1627,7 +1627,7 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
         int blk_of_lane = 0;                   // block of box (fetched + lane) of this job
         int fetched = -1000000;
         for (int t = t_beg; t < t_end && ok; ++t) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
+          if (!mbar_wait_warp(&empty[stage], phase ^ 1, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
           const int bx0 = t * nbx;
           if (bx0 + nbx > fetched + 32) {      // nbx divides 32: a tile's boxes are fetched together
             fetched = bx0;
@@ -1701,7 +1701,7 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
       // All eight warps wait for and release every tile, the other group's too: a parity wait tells one fill of a stage from
       // the next only while no warp is a whole fill ahead (it would pass on the previous fill) or behind (it would wait
       // for the fill after next, which in turn waits for it).
-      if (ok && !mbar_wait(&full[st], ph, p.status, ST_TIMEOUT_FULL)) ok = false;
+      if (ok && !mbar_wait_warp(&full[st], ph, p.status, ST_TIMEOUT_FULL)) ok = false;
       if (!ok) continue;
       if (((t - t_beg) & 1) != group) {
         if (lane == 0) mbar_arrive(&empty[st]);

@@ -134,7 +134,7 @@ gemm_w8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const int kb0 = split * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
       for (int kb = kb0; kb < kb1; ++kb) {
         // the A tile lands on the same barrier; waiting here also covers the raw B tile
-        if (!mbar_wait(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) { ok = false; break; }
         const uint8_t* raw = smem + stage * W8_STAGE_BYTES + W8_A_BYTES;
         uint8_t* bt = smem + stage * W8_STAGE_BYTES + W8_A_BYTES + W8_RAW_BYTES;
 #pragma unroll 4
@@ -169,7 +169,7 @@ gemm_w8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const int rem = t - split * (mt * nt);
       const int n_idx = rem / mt, m_idx = rem - (rem / mt) * mt;
       const int acc = it & 1;
-      if (!mbar_wait(&tmem_full[acc], (it >> 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(&tmem_full[acc], (it >> 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const int row = m_idx * WBM + q * 32 + lane;
       const uint32_t taddr_row = tmem_base + acc * WBN + (static_cast<uint32_t>(q * 32) << 16);
