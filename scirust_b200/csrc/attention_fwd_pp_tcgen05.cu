@@ -335,7 +335,9 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
         add2(sum4[i & 6], sum4[(i & 6) + 1], __float_as_uint(e0), __float_as_uint(e1));
         pk[i >> 1] = pack_bf16x2(e0, e1);
       }
-      l = l * alpha + (((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) + ((sum4[4] + sum4[5]) + (sum4[6] + sum4[7])));
+      // Roundings are spelt out here and in the log-sum-exp: left to the compiler, what it contracts changes with the code around it.
+      const float row_sum = ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) + ((sum4[4] + sum4[5]) + (sum4[6] + sum4[7]));
+      l = __fadd_rn(__fmul_rn(l, alpha), row_sum);
       if (j > 0) {
         // P V of the previous block has read the P tile and updated O
         mbar_wait(&pv_done[t], (j - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL);
@@ -388,7 +390,8 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
         if (c0 + 64 < DH) __syncwarp();
       }
       if (q_idx < p.S) {
-        if (p.lse) p.lse[(static_cast<size_t>(b) * p.H + head) * p.S + q_idx] = m_ref * 0.6931471805599453f + logf(l);
+        if (p.lse)
+          p.lse[(static_cast<size_t>(b) * p.H + head) * p.S + q_idx] = __fmaf_rn(m_ref, 0.6931471805599453f, logf(l));
       }
     }
   }
