@@ -1,7 +1,7 @@
 // Calls from Python into libscirust_b200_cuda.so without ctypes: one typed function per entry point of the C ABI. A launch
 // of the decode path has about 20 arguments, which ctypes turns into as many objects (4.8 us); a conversion here is one
-// test and one read (0.5 us). Arguments are ints, None (a null pointer) and floats; anything else raises TypeError, and the
-// caller (ops/_lib.py) goes through ctypes instead. Built by _build.py; py_calls.inc lists the entry points.
+// test and one read (0.5 us). Arguments are ints, None (a null pointer), arrays of ctypes (their address) and floats; anything
+// else raises TypeError, and the caller (ops/_lib.py) makes that call through ctypes. Built by _build.py; py_calls.inc lists the entry points.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <dlfcn.h>
@@ -17,6 +17,19 @@ bool bad_arg(const char* want, PyObject* got) {
   return false;
 }
 
+PyTypeObject* ctypes_array = nullptr;            // _ctypes.Array
+
+bool is_array(PyObject* o) { return PyType_IsSubtype(Py_TYPE(o), ctypes_array); }
+
+// The address of a ctypes array; it stays where it is while the caller holds the array.
+void* array_address(PyObject* o) {
+  Py_buffer view;
+  if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE)) return nullptr;
+  void* at = view.buf;
+  PyBuffer_Release(&view);
+  return at;
+}
+
 template <class T>
 bool read_arg(PyObject* o, T& out) {
   if constexpr (std::is_floating_point_v<T>) {
@@ -24,7 +37,10 @@ bool read_arg(PyObject* o, T& out) {
     else if (PyLong_Check(o)) out = static_cast<T>(PyLong_AsDouble(o));
     else return bad_arg("a number", o);
   } else {
-    if (std::is_pointer_v<T> && o == Py_None) { out = T{}; return true; }
+    if constexpr (std::is_pointer_v<T>) {
+      if (o == Py_None) { out = T{}; return true; }
+      if (!PyLong_Check(o) && is_array(o)) { out = reinterpret_cast<T>(array_address(o)); return !PyErr_Occurred(); }
+    }
     if (!PyLong_Check(o)) return bad_arg(std::is_pointer_v<T> ? "an address or None" : "an integer", o);
     const unsigned long long v = PyLong_AsUnsignedLongLongMask(o);       // out of range: the low bits, as ctypes does
     if constexpr (std::is_pointer_v<T>) out = reinterpret_cast<T>(static_cast<uintptr_t>(v));
@@ -67,6 +83,14 @@ PyObject* invoke(R (*fn)(A...), PyObject* const* args, Py_ssize_t n) {
 PyObject* bind(PyObject*, PyObject* arg) {
   const char* path = PyUnicode_AsUTF8(arg);
   if (!path) return nullptr;
+  if (!ctypes_array) {
+    PyObject* ctypes = PyImport_ImportModule("_ctypes");
+    PyObject* array = ctypes ? PyObject_GetAttrString(ctypes, "Array") : nullptr;
+    Py_XDECREF(ctypes);
+    if (!array) return nullptr;
+    if (!PyType_Check(array)) { Py_DECREF(array); return PyErr_Format(PyExc_TypeError, "_ctypes.Array is not a type"); }
+    ctypes_array = reinterpret_cast<PyTypeObject*>(array);   // kept for the life of the process
+  }
   void* lib = dlopen(path, RTLD_NOW | RTLD_NOLOAD);
   if (!lib) return PyErr_Format(PyExc_OSError, "%s is not loaded", path);
   PyObject* out = PyDict_New();

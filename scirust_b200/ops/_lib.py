@@ -203,9 +203,8 @@ def call(name: str, *args) -> None:
     try:
         rc = fn(*args)
     except TypeError:
-        # arrays and references of ctypes are for ctypes, and so is an argument that neither takes
-        fn = _calls[name] = getattr(cuda(), name)
-        rc = fn(*args)
+        # references of ctypes, integers of NumPy, and what neither takes: for ctypes, this once
+        rc = getattr(cuda(), name)(*args)
     if rc:
         check(rc, name)
 

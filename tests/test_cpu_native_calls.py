@@ -2,6 +2,7 @@
 before they touch a device."""
 import ctypes
 
+import numpy as np
 import pytest
 
 from scirust_b200 import _build
@@ -47,3 +48,25 @@ def test_ctypes_arrays_still_go_through_ctypes():
     p, handle = ctypes.c_void_p(), (ctypes.c_char * lib.sb_ipc_handle_size())()
     with pytest.raises(_lib.NativeError):                       # no such handle
         _lib.call("sb_ipc_open", handle, ctypes.byref(p))
+
+
+def test_one_odd_argument_does_not_move_an_entry_point_to_ctypes(calls):
+    with pytest.raises(_lib.NativeError):
+        _lib.call("sb_swiglu_fwd", None, None, 0, 0, None)
+    fast = _lib._calls["sb_swiglu_fwd"]
+    assert not isinstance(fast, ctypes._CFuncPtr)
+    with pytest.raises((TypeError, ctypes.ArgumentError)):
+        _lib.call("sb_swiglu_fwd", None, None, 0.5, 0, None)
+    with pytest.raises(_lib.NativeError):
+        _lib.call("sb_swiglu_fwd", None, None, np.int32(0), 0, None)
+    assert _lib._calls["sb_swiglu_fwd"] is fast
+
+
+def test_arrays_of_ctypes_are_addresses(calls):
+    """The extension takes them as ctypes does; arrays of anything else stay refused."""
+    fn, lib = calls["sb_swiglu_fwd"], _lib.cuda()
+    arr = (ctypes.c_void_p * 4)(*range(4))
+    assert fn(arr, arr, 0, 8, None) == lib.sb_swiglu_fwd(arr, arr, 0, 8, None) != 0        # bad argument: no rows
+    for other in (np.zeros(4), bytearray(32), [1, 2]):
+        with pytest.raises(TypeError):
+            fn(other, None, 0, 0, None)
