@@ -4,8 +4,8 @@ Outputs land in ``scirust_b200/lib/`` next to the sources so that a snapshot of 
 repository carries the binaries with it:
 
 * ``libscirust_b200_cuda.so``  - every ``csrc/*.cu`` (tcgen05 GEMM, attention, decode, comm ...)
-* ``sb_py_calls.so``           - ``csrc/py_calls.cc``: the C ABI's entry points as Python functions (left out where the
-  Python headers are missing; the calls then go through ctypes).
+* ``sb_py_calls.<tag>.so``     - ``csrc/py_calls.cc``: the C ABI's entry points as Python functions of this interpreter (left
+  out where the Python headers are missing; the calls then go through ctypes).
 * ``libscirust_b200_rt.so``    - every ``csrc/*.cpp`` (CPU runtime: fixed-order fp32 math,
   arena / paged-KV block allocators, TCP tree all-reduce, samplers); no CUDA dependency.
 
@@ -30,7 +30,7 @@ OBJ = LIB / "obj"
 
 CUDA_LIB = LIB / "libscirust_b200_cuda.so"
 RT_LIB = LIB / "libscirust_b200_rt.so"
-CALLS_LIB = LIB / "sb_py_calls.so"
+CALLS_LIB = LIB / ("sb_py_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -182,9 +182,15 @@ def write_api_header() -> bool:
     return True
 
 
+def api_digest() -> str:
+    """Names the C ABI: a digest of ``csrc/api.h``, which the extension is compiled with and checked against when it is loaded."""
+    return hashlib.sha256((CSRC / "api.h").read_bytes()).hexdigest()
+
+
 def build_calls(force: bool = False) -> Path | None:
     include = Path(sysconfig.get_paths()["include"])
     if not (include / "Python.h").exists():
+        CALLS_LIB.unlink(missing_ok=True)     # of an earlier build
         return None
     OBJ.mkdir(parents=True, exist_ok=True)
     src, inc = CSRC / "py_calls.cc", OBJ / "py_calls.inc"
@@ -192,7 +198,7 @@ def build_calls(force: bool = False) -> Path | None:
     table = "".join(f"SB_ENTRY({n})\n" for n in names)
     if not inc.exists() or inc.read_text() != table:
         inc.write_text(table)
-    flags = [*CXX_FLAGS, f"-I{include}", f"-I{CSRC}", f"-I{OBJ}"]
+    flags = [*CXX_FLAGS, f"-I{include}", f"-I{CSRC}", f"-I{OBJ}", f'-DSB_API_DIGEST="{api_digest()}"']
     obj = OBJ / "py_calls.so"                 # the digest is kept beside it, as for the objects
     deps = [CSRC / "api.h", inc]
     if force or not CALLS_LIB.exists() or _stale(src, obj, deps, flags):
@@ -202,6 +208,12 @@ def build_calls(force: bool = False) -> Path | None:
         os.replace(tmp, CALLS_LIB)
         _stamp(src, obj, deps, flags)
     return CALLS_LIB
+
+
+def build_cuda_and_calls() -> None:
+    """What a first use builds: the CUDA library and the extension that calls it."""
+    build_cuda()
+    build_calls()
 
 
 def build_all(force: bool = False, verbose: bool = False) -> None:

@@ -1,7 +1,8 @@
 // Calls from Python into libscirust_b200_cuda.so without ctypes: one typed function per entry point of the C ABI. A launch
 // of the decode path has about 20 arguments, which ctypes turns into as many objects (4.8 us); a conversion here is one
 // test and one read (0.5 us). Arguments are ints, None (a null pointer), arrays of ctypes (their address) and floats; anything
-// else raises TypeError, and the caller (ops/_lib.py) makes that call through ctypes. Built by _build.py; py_calls.inc lists the entry points.
+// else raises TypeError, and the caller (ops/_lib.py) makes that call through ctypes. Built by _build.py;
+// py_calls.inc lists the entry points.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <dlfcn.h>
@@ -111,4 +112,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "sb_py_calls", nullptr, -1, methods
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_sb_py_calls() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit_sb_py_calls() {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "api_digest", SB_API_DIGEST) < 0) Py_CLEAR(m);   // of the api.h compiled in
+  return m;
+}

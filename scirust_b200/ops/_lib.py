@@ -72,7 +72,7 @@ def _load(path: Path, builder) -> C.CDLL:
 def cuda() -> C.CDLL:
     global _cuda
     if _cuda is None:
-        lib = _load(_build.CUDA_LIB, _build.build_cuda)
+        lib = _load(_build.CUDA_LIB, _build.build_cuda_and_calls)
         for name, sig in _CUDA_SIGS.items():
             if hasattr(lib, name):
                 fn = getattr(lib, name)
@@ -176,16 +176,22 @@ _calls: dict = {}           # entry point -> the function that ``call`` uses
 
 
 def _native_calls() -> dict:
-    """The entry points as functions of the extension module (csrc/py_calls.cc); empty where it is missing."""
+    """The entry points as functions of the extension module (csrc/py_calls.cc). Empty, so that calls go through ctypes, where
+    it is missing, does not load here, or was compiled with other declarations than those of ``csrc/api.h``."""
     import importlib.machinery
     import importlib.util
     path = _build.CALLS_LIB
     if not path.exists():
         return {}
     loader = importlib.machinery.ExtensionFileLoader("sb_py_calls", str(path))
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("sb_py_calls", loader))
-    loader.exec_module(module)
-    return module.bind(str(_build.CUDA_LIB))
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("sb_py_calls", loader))
+        loader.exec_module(module)
+        if getattr(module, "api_digest", None) != _build.api_digest():
+            return {}
+        return module.bind(str(_build.CUDA_LIB))
+    except (ImportError, OSError):
+        return {}
 
 
 def _bind(name: str):

@@ -70,3 +70,37 @@ def test_arrays_of_ctypes_are_addresses(calls):
     for other in (np.zeros(4), bytearray(32), [1, 2]):
         with pytest.raises(TypeError):
             fn(other, None, 0, 0, None)
+
+
+def test_an_extension_of_another_abi_or_interpreter_is_left_alone(calls, monkeypatch, tmp_path):
+    import sysconfig
+    assert _build.CALLS_LIB.name == "sb_py_calls" + sysconfig.get_config_var("EXT_SUFFIX")
+    with monkeypatch.context() as m:
+        m.setattr(_build, "api_digest", lambda: "of a changed api.h")
+        assert _lib._native_calls() == {}
+    broken = tmp_path / _build.CALLS_LIB.name
+    broken.write_bytes(b"not a shared library")
+    monkeypatch.setattr(_build, "CALLS_LIB", broken)
+    assert _lib._native_calls() == {}                           # and calls go through ctypes
+    monkeypatch.setattr(_lib, "_calls", {})
+    with pytest.raises(_lib.NativeError):
+        _lib.call("sb_swiglu_fwd", None, None, 0, 0, None)
+
+
+def test_an_extension_that_cannot_be_rebuilt_goes(monkeypatch, tmp_path):
+    old = tmp_path / "sb_py_calls.so"
+    old.touch()
+    monkeypatch.setattr(_build, "CALLS_LIB", old)
+    monkeypatch.setattr(_build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})      # no Python.h there
+    assert _build.build_calls() is None and not old.exists()
+
+
+def test_first_use_of_a_missing_library_builds_the_extension_too(monkeypatch, tmp_path):
+    built = []
+    monkeypatch.setattr(_build, "CUDA_LIB", tmp_path / "missing.so")
+    monkeypatch.setattr(_build, "build_cuda", lambda *a, **k: built.append("cuda"))
+    monkeypatch.setattr(_build, "build_calls", lambda *a, **k: built.append("calls"))
+    monkeypatch.setattr(_lib, "_cuda", None)
+    with pytest.raises(_lib.NativeError):                       # the builders here make nothing
+        _lib.cuda()
+    assert built == ["cuda", "calls"]
