@@ -371,6 +371,15 @@ static int skinny_clusters(int c) {
   return n;
 }
 
+// Whether the splits of `nt` column tiles finish inside the kernel; < 0: the launch cannot be prepared.
+template <int RB, bool I8>
+static int skinny_in_cluster(int nt, int splits) {
+  if (splits < 2 || splits > SK_MAX_CLUSTER) return 0;
+  static PerDeviceOnce attr;
+  if (allow_smem(attr, gemm_skinny_kernel<RB, I8, true>, SkinnyCfg<RB>::SMEM_BYTES, SB_ERR_LAUNCH)) return -1;
+  return nt <= skinny_clusters<RB, I8>(splits);
+}
+
 // in_cluster: set when the splits finish inside the kernel, p.C is then the output. `workspace` takes the partials otherwise.
 template <int RB, bool I8>
 static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, SkinnyParams p, void* workspace, bool* in_cluster,
@@ -378,12 +387,10 @@ static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, SkinnyPar
   using Cfg = SkinnyCfg<RB>;
   const int nt = (p.N + SK_BM - 1) / SK_BM;
   auto clustered = gemm_skinny_kernel<RB, I8, true>;
-  static PerDeviceOnce attr, attr_c;
-  *in_cluster = false;
-  if (p.splits > 1 && p.splits <= SK_MAX_CLUSTER) {
-    if (allow_smem(attr_c, clustered, Cfg::SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
-    *in_cluster = nt <= skinny_clusters<RB, I8>(p.splits);
-  }
+  static PerDeviceOnce attr;
+  const int fits = skinny_in_cluster<RB, I8>(nt, p.splits);
+  if (fits < 0) return SB_ERR_LAUNCH;
+  *in_cluster = fits > 0;
   if (*in_cluster)
     return launch_dep_cluster(clustered, dim3(nt, p.splits), dim3(SK_THREADS), Cfg::SMEM_BYTES, stream, p.splits, true, tw, tx,
                               p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
@@ -395,16 +402,46 @@ static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, SkinnyPar
                  cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
+// The number of k ranges that `splits` asks for (<= 0: one work item per SM), made whole; returns the k-blocks of a range.
+static int skinny_split(int N, int K, int is_i8, int* splits) {
+  const int bke = is_i8 ? 128 : 64;
+  const int num_kb = (K + bke - 1) / bke;
+  const int nt = (N + SK_BM - 1) / SK_BM;
+  int s = *splits;
+  if (s <= 0) {
+    s = num_sms() / nt;                             // one work item per SM, no second round
+    if (s < 1) s = 1;
+    const int max_splits = num_kb / 4 > 0 ? num_kb / 4 : 1;      // at least four k-blocks per item
+    if (s > max_splits) s = max_splits;
+  }
+  if (s > num_kb) s = num_kb;
+  const int kbps = (num_kb + s - 1) / s;
+  *splits = (num_kb + kbps - 1) / kbps;
+  return kbps;
+}
+
 }  // namespace sb
 
 using namespace sb;
+
+// Kernels that sb_gemm_skinny launches for these sizes on the current device: 1, or 2 where split sums are added from memory.
+extern "C" int sb_gemm_skinny_launches(int rows, int N, int K, int is_i8, int splits) {
+  if (rows <= 0 || rows > 64 || N <= 0 || K <= 0) return 0;
+  skinny_split(N, K, is_i8, &splits);
+  const int nt = (N + SK_BM - 1) / SK_BM;
+  const auto in_cluster = rows <= 16   ? (is_i8 ? skinny_in_cluster<16, true> : skinny_in_cluster<16, false>)
+                          : rows <= 32 ? (is_i8 ? skinny_in_cluster<32, true> : skinny_in_cluster<32, false>)
+                                       : (is_i8 ? skinny_in_cluster<64, true> : skinny_in_cluster<64, false>);
+  return splits > 1 && in_cluster(nt, splits) <= 0 ? 2 : 1;
+}
 
 // C[rows, N] (bf16) = X . W (+ R), rows <= 64.
 //   is_i8 == 0: X bf16 [rows, ldx], W bf16 [K, N] (row pitch ldw);
 //   is_i8 == 1: X int8 [rows, ldx] with row scales sx, W int8 [N, K] (transposed codes, row pitch ldw, K % 16 == 0)
 //               with column scales sw.
 // Bases 16-byte aligned, pitches multiples of 16 bytes, N % 8 == 0. workspace: splits * rows * N 32-bit words, read
-// only when the k range is split and its splits do not finish in a cluster (splits <= 0 lets the launcher fill the GPU: about one work item per SM).
+// only when the k range is split and its splits do not finish in a cluster (splits <= 0 lets the launcher fill the GPU: about one
+// work item per SM).
 extern "C" int sb_gemm_skinny(const void* X, int ldx, const void* W, int ldw, void* C, int ldc, const void* R, int ldr,
                               int rows, int N, int K, int is_i8, const float* sx, const float* sw, int splits,
                               void* workspace, int* status, void* stream_) {
@@ -412,18 +449,7 @@ extern "C" int sb_gemm_skinny(const void* X, int ldx, const void* W, int ldw, vo
   if (rows <= 0 || rows > 64 || N <= 0 || K <= 0 || (N & 7) || !status) return SB_ERR_ARG;
   if (is_i8 && (!sx || !sw || (K & 15) || (ldx & 15) || (ldw & 15))) return SB_ERR_ARG;
   if (!is_i8 && ((ldx & 7) || (ldw & 7))) return SB_ERR_ALIGN;
-  const int bke = is_i8 ? 128 : 64;
-  const int num_kb = (K + bke - 1) / bke;
-  const int nt = (N + SK_BM - 1) / SK_BM;
-  if (splits <= 0) {
-    splits = num_sms() / nt;                        // one work item per SM, no second round
-    if (splits < 1) splits = 1;
-    const int max_splits = num_kb / 4 > 0 ? num_kb / 4 : 1;      // at least four k-blocks per item
-    if (splits > max_splits) splits = max_splits;
-  }
-  if (splits > num_kb) splits = num_kb;
-  const int kbps = (num_kb + splits - 1) / splits;
-  splits = (num_kb + kbps - 1) / kbps;
+  const int kbps = skinny_split(N, K, is_i8, &splits);
   if (splits > 1 && !workspace) return SB_ERR_ARG;
   const int rb = rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
   CUtensorMap tw, tx;

@@ -311,6 +311,7 @@ def gemv_argmax(x, w, out_tokens=None, rms_weight=None, eps=1e-5, logits=None, c
 
 
 _lib.register("sb_gemm_skinny", [vp, i32, vp, i32, vp, i32, vp, i32, i32, i32, i32, i32, vp, vp, i32, vp, vp, vp])
+_lib.register("sb_gemm_skinny_launches", [i32, i32, i32, i32, i32])
 SKINNY_MAX_ROWS = 64
 
 
@@ -326,6 +327,11 @@ def skinny_ok(x, w) -> bool:
         return os.environ.get("SB_W8A8", "1") != "0" and K % 16 == 0 and N % 8 == 0
     K, N = w.shape
     return N % 8 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
+
+
+@functools.lru_cache(maxsize=4096)       # a function of the device and the sizes
+def _skinny_launches(device, rows, N, K, quant, splits):
+    return _lib.cuda().sb_gemm_skinny_launches(rows, N, K, int(quant), splits)
 
 
 def matmul_skinny(x, w, residual=None, out=None, splits=0):
@@ -355,7 +361,7 @@ def matmul_skinny(x, w, residual=None, out=None, splits=0):
     _lib.call("sb_gemm_skinny", *args, out.data_ptr(), out.stride(0), _lib.ptr(residual),
               residual.stride(0) if residual is not None else 0, M, N, K, int(quant), *scales,
               est, _lib.ptr(ws), _lib.status_word(x.device).data_ptr(), _lib.stream())
-    _g.launch_count += 2 if est > 1 else 1
+    _g.launch_count += _skinny_launches(x.device, M, N, K, quant, est) if est > 1 else 1
     return out
 
 

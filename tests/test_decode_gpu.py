@@ -5,7 +5,7 @@ import torch
 from scirust_b200.models import GQADecoder, SciAgentConfig
 from scirust_b200.models.infer import InferenceEngine, reference_generate
 from scirust_b200 import ops
-from scirust_b200.ops import _lib, decode as D
+from scirust_b200.ops import _lib, decode as D, gemm as _g
 
 pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
@@ -424,3 +424,19 @@ def test_sums_of_long_k_ranges_keep_the_precision_of_short_ones(quant, M, K, N):
     D.gemv(x, wt, out_f32=out)
     ref = x.double() @ (wt.q.double() * wt.scale.double() if quant else w.double())
     assert ((out.double() - ref).norm() / ref.norm()).item() < 2e-7
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("M,K,N,splits", [(16, 4096, 4096, 0), (64, 4096, 6144, 0), (33, 4096, 22016, 0), (9, 1024, 1536, 0),
+                                          (16, 2048, 1024, 7), (16, 100 * 16, 1024, 3)])
+def test_launches_of_the_weight_streaming_gemm_are_counted_as_they_are(quant, M, K, N, splits):
+    """Partial sums reach the workspace exactly where a second kernel adds them up."""
+    x, w = _r((M, K), 1), _r((K, N), 2)
+    w = D.quantize_per_channel(w) if quant else w
+    D.matmul_skinny(x, w, splits=splits)                       # the workspace and the transposed codes are there
+    ws = D._workspace(1, x.device)
+    ws.fill_(float("nan"))
+    before = _g.launch_count
+    D.matmul_skinny(x, w, splits=splits)
+    counted = _g.launch_count - before - (1 if quant else 0)   # the row quantiser is one
+    assert counted == (1 if ws.isnan().all() else 2)
