@@ -2064,10 +2064,11 @@ using namespace sb;
 #define STREAM static_cast<cudaStream_t>(stream)
 #define CHECK_LAUNCH() return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH
 
-static bool g_pdl = true;
+// Programmatic dependent launch of the decode-path kernels: on, unless the environment says SB_PDL=0.
+static bool g_pdl = [] { const char* e = getenv("SB_PDL"); return !(e && e[0] == '0'); }();
 bool sb::dependent_launches() { return g_pdl; }
 
-// Switches programmatic dependent launch of the decode-path kernels off (0) or on again for this process.
+// Switches it off (0) or on again for this process.
 extern "C" int sb_set_pdl(int on) { g_pdl = on != 0; return 0; }
 
 namespace sb {

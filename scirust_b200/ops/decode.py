@@ -43,22 +43,6 @@ def _workspace(n, device):
 _lib.register("sb_set_pdl", [i32])
 
 
-class dependent_launch:
-    """Context manager of earlier versions, kept for its callers; it does nothing. The decode-path kernels are launched with
-    programmatic dependent launch wherever they run: a kernel's CTAs start while its predecessor drains and read nothing
-    before it has completed, so the order that a program sees is plain stream order (csrc/dependent.cuh). A decoder layer of
-    Llama-3-8B shape, replayed from a graph: 16 int8 rows 127.5 -> 119.2 us, 64 rows 223 -> 215."""
-
-    def __init__(self, enabled: bool = True):
-        self.enabled = enabled
-
-    def __enter__(self):
-        return self
-
-    def __exit__(self, *exc):
-        return False
-
-
 _gemv_ws: dict = {}
 
 

@@ -104,3 +104,15 @@ def test_first_use_of_a_missing_library_builds_the_extension_too(monkeypatch, tm
     with pytest.raises(_lib.NativeError):                       # the builders here make nothing
         _lib.cuda()
     assert built == ["cuda", "calls"]
+
+
+@pytest.mark.parametrize("value,on", [(None, True), ("1", True), ("0", False)])
+def test_environment_switches_dependent_launches(value, on):
+    import os
+    import subprocess
+    import sys
+    env = {k: v for k, v in os.environ.items() if k != "SB_PDL"} | ({"SB_PDL": value} if value else {})
+    _lib.cuda()                                                 # is built
+    code = (f"import ctypes; f = ctypes.CDLL({str(_build.CUDA_LIB)!r})._ZN2sb18dependent_launchesEv; "
+            "f.restype = ctypes.c_bool; print(f())")
+    assert subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, check=True).stdout.strip() == str(on)
