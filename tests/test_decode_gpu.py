@@ -328,8 +328,8 @@ def test_decode_attention_stream_without_weight_is_zero():
 
 @pytest.mark.parametrize("rows,quant", [(1, False), (8, True), (9, False), (33, True), (64, False)])
 def test_dependent_launches_read_what_their_predecessor_wrote(rows, quant):
-    """Chains of decode kernels whose inputs AND weights the kernel right before them has just written give, launch for
-    launch, the bits of plain stream order."""
+    """A row norm, a product whose weights a copy has just written, and SwiGLU give, launch for launch, the bits of plain stream
+    order. (The copies are not launched dependently; the chains of the next test have none.)"""
     K, N = 1024, 1536
     g = torch.Generator(device="cuda").manual_seed(rows)
     gain = torch.ones(K, dtype=torch.bfloat16, device="cuda")
@@ -363,6 +363,70 @@ def test_dependent_launches_read_what_their_predecessor_wrote(rows, quant):
     finally:
         _lib.call("sb_set_pdl", 1)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("rows,quant,stream", [(1, False, False), (8, True, True), (9, False, True), (16, True, False),
+                                               (64, False, False), (64, True, True)])
+def test_chains_of_dependent_launches_give_the_bits_of_plain_stream_order(rows, quant, stream, graph):
+    """Decoder layers fed back into themselves, without any other kernel between: every kernel reads what the one right before it
+    has just written, at addresses that held another step's values before (product -> rotation and append -> attention -> product
+    -> norm -> product with split sums in memory -> SwiGLU -> product -> norm)."""
+    d, H, Hkv, dh, ff, page, past, steps = 1024, 8, 2, 128, 3072, 64, 300, 8
+    ws = [_r(s, 10 + i, 0.05) for i, s in enumerate([(d, (H + 2 * Hkv) * dh), (d, d), (d, 2 * ff), (ff, d)])]
+    if quant:
+        ws = [D.quantize_per_channel(w) for w in ws]
+        for w in ws:
+            w.transposed()
+    gain, x0 = _r((d,), 1) + 1, _r((rows, d), 2)
+    cos, sin = ops.rope_table(512, dh, 1e4, torch.device("cuda"))
+    nb = (past + steps + page - 1) // page
+    table = torch.arange(rows * nb, dtype=torch.int32, device="cuda").reshape(rows, nb)
+    pool0 = _r((rows * nb, 2, Hkv, page, dh), 3)
+    seq_of = torch.arange(rows, dtype=torch.int32, device="cuda")
+    pos = [torch.full((rows,), past + i, dtype=torch.int32, device="cuda") for i in range(steps)]
+    lens = [p + 1 for p in pos]
+    if rows > 8 and not quant:
+        assert D._skinny_launches(x0.device, rows, 2 * ff, d, False, 3) == 2       # clusters of three for 48 tiles do not fit
+
+    def linear(x, w):
+        return D.gemv(x, w) if rows <= 8 else D.matmul_skinny(x, w)
+
+    def chain():
+        pool, x, out = pool0.clone(), x0, []
+        for i in range(steps):
+            qkv = linear(x, ws[0])
+            D.rope_kv_append(qkv, H, Hkv, dh, cos, sin, pool, table, page, seq_of, pos[i])
+            a = D.decode_attention(qkv, pool, table, page, lens[i], H, Hkv, dh, stream=stream)
+            h = ops.rmsnorm_fwd(linear(a, ws[1]), gain, 1e-5, want_inv=False)[0]
+            x = ops.rmsnorm_fwd(linear(ops.swiglu_fwd(linear(h, ws[2])), ws[3]), gain, 1e-5, want_inv=False)[0]
+            out.append(x)
+        return torch.stack(out), pool
+
+    def run():
+        if not graph:
+            return chain()
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            chain()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=side):
+                out = chain()
+        torch.cuda.current_stream().wait_stream(side)
+        g.replay()
+        g.replay()
+        return [t.clone() for t in out]
+
+    got = run()
+    _lib.call("sb_set_pdl", 0)
+    try:
+        want = run()
+    finally:
+        _lib.call("sb_set_pdl", 1)
+    _lib.check_status()
+    assert got[0].isfinite().all() and len({bytes(t.view(torch.uint8).cpu().numpy().tobytes()) for t in got[0]}) == steps
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
 @pytest.mark.parametrize("quant", [False, True])
