@@ -19,6 +19,7 @@
 #include "sm100_ptx.cuh"
 #include "peer_sync.cuh"
 #include "dependent.cuh"
+#include <atomic>
 
 namespace sb {
 
@@ -2121,28 +2122,65 @@ int num_sms();
 // W2 = 2: 512 bytes of every weight row per CTA, 1: 256. The staged slice of X takes 16 bytes per k. Only one block of 8
 // rows is shipped: with two or four blocks the kernel is bound by the mma.sync rate, not by memory (117 MB of weights:
 // 33 us at 8 rows, 58 us at 16, 111 us at 32), and the tcgen05 GEMM is faster there.
+template <int ESZ, int W2>
+static size_t gemv_mma_smem(int k_per_split, size_t* xs_bytes) {
+  constexpr int KT = 64 / W2;
+  *xs_bytes = static_cast<size_t>((k_per_split + KT - 1) / KT * KT) * 16;
+  // the RMSNorm prologue borrows the X staging area for M * 8 * 32 partial sums; 1 KB for the ring's alignment
+  return static_cast<size_t>(GEMV_STAGES) * GEMV_TILE_BYTES + (*xs_bytes > 8192 ? *xs_bytes : 8192) + 1024;
+}
+
+template <int ESZ, int W2, bool CLUSTER>
+static auto gemv_mma_kern() {
+  if constexpr (ESZ == 2) return gemv_mma_kernel<1, W2, CLUSTER>; else return gemv_mma_i8_kernel<W2, CLUSTER>;
+}
+
+template <int ESZ, int W2, bool CLUSTER>
+static int gemv_mma_prepare() {
+  static PerDeviceOnce attr;
+  return allow_smem(attr, gemv_mma_kern<ESZ, W2, CLUSTER>(), GEMV_STAGES * GEMV_TILE_BYTES + GEMV_MAX_XS_BYTES + 1024, SB_ERR_LAUNCH);
+}
+
+// Clusters of `c` CTAs that the current device holds at once; asked for once per device, size and KB of shared memory.
+template <int ESZ, int W2>
+static int gemv_clusters(int c, int k_per_split) {
+  size_t xs = 0;
+  const size_t smem = gemv_mma_smem<ESZ, W2>(k_per_split, &xs);
+  static std::atomic<short> known[16][9][160] = {};                // count + 1
+  int device = 0;
+  if (c > 8 || xs > static_cast<size_t>(GEMV_MAX_XS_BYTES) || cudaGetDevice(&device) != cudaSuccess) return 0;
+  std::atomic<short>* keep = device >= 0 && device < 16 ? &known[device][c][smem >> 10] : nullptr;
+  if (keep && keep->load(std::memory_order_relaxed) > 0) return keep->load(std::memory_order_relaxed) - 1;
+  if (gemv_mma_prepare<ESZ, W2, true>()) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1, c); cfg.blockDim = dim3(GEMV_THREADS); cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = c; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, gemv_mma_kern<ESZ, W2, true>(), &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+  if (keep) keep->store(static_cast<short>(n + 1), std::memory_order_relaxed);
+  return n;
+}
+
 template <int ESZ, int W2, bool CLUSTER>
 static int launch_gemv_mma(const GemvParams& p, int splits, cudaStream_t s) {
   constexpr int KT = 64 / W2, COLS = 256 * W2 / ESZ;
-  const int kn_pad = (p.k_per_split + KT - 1) / KT * KT;
-  const size_t xs_bytes = static_cast<size_t>(kn_pad) * 16;
+  size_t xs_bytes = 0;
+  const size_t smem = gemv_mma_smem<ESZ, W2>(p.k_per_split, &xs_bytes);
   if (xs_bytes > static_cast<size_t>(GEMV_MAX_XS_BYTES)) return SB_ERR_ARG;
   if (ESZ == 1 && ((p.N & 1) || (p.ldw & 1))) return SB_ERR_ARG;
-  // the RMSNorm prologue borrows the X staging area for M * 8 * 32 partial sums; 1 KB for the ring's alignment
-  const size_t smem = static_cast<size_t>(GEMV_STAGES) * GEMV_TILE_BYTES + (xs_bytes > 8192 ? xs_bytes : 8192) + 1024;
   CUtensorMap tm;
   const int rc = make_tmap_2d_bf16(&tm, p.W, static_cast<uint64_t>(p.N) * ESZ / 2, p.K,
                                    static_cast<uint64_t>(p.ldw) * ESZ / 2, 64, KT);
   if (rc) return rc;
-  void (*kern)(const CUtensorMap, const GemvParams);
-  if constexpr (ESZ == 2) kern = gemv_mma_kernel<1, W2, CLUSTER>; else kern = gemv_mma_i8_kernel<W2, CLUSTER>;
-  static PerDeviceOnce attr;
-  if (allow_smem(attr, kern, GEMV_STAGES * GEMV_TILE_BYTES + GEMV_MAX_XS_BYTES + 1024, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
+  if (gemv_mma_prepare<ESZ, W2, CLUSTER>()) return SB_ERR_LAUNCH;
   const dim3 grid((p.N + COLS - 1) / COLS, splits);
   // In plain stream order: two or three CTAs share an SM, and CTAs that are placed while the predecessor drains crowd the
   // SMs that it leaves first, for the whole stream. The kernel after this one may start early (pdl_trigger).
-  return launch_dep_cluster(kern, grid, dim3(GEMV_THREADS), smem, s, CLUSTER ? splits : 1, false, tm, p) == cudaSuccess
-             ? 0 : SB_ERR_LAUNCH;
+  return launch_dep_cluster(gemv_mma_kern<ESZ, W2, CLUSTER>(), grid, dim3(GEMV_THREADS), smem, s, CLUSTER ? splits : 1, false, tm,
+                            p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
 // Y[M,N] = f(X)[M,K] * W[K,N] (* scale[n]) (+ R). M <= 8 per call (callers loop over row groups).
@@ -2226,14 +2264,21 @@ static int gemv_impl(const void* X, int ldx, const void* W, int ldw, const float
     }
   }
   if (mma) {
-    // Up to eight splits finish inside a cluster, unless the grid runs in many waves (clusters are placed one by one:
-    // 4096 x 128256, eight splits: 160 us through memory, 174 in clusters) or one CTA has to hold the finished block, as
-    // the fused tails want it. Half the columns per CTA where the grid would leave SMs without one.
-    const int blocks = (N + cols - 1) / cols;
-    if (!ca && !aa && splits > 1 && splits <= 8 && blocks * splits <= 4 * num_sms()) {
-      if (blocks * splits > num_sms())
+    // Up to eight splits finish inside a cluster, unless one CTA has to hold the finished block, as the fused tails want it, or the
+    // clusters are not all on the GPU at once (it holds 32 of eight): they are placed as a whole, and a second wave takes as
+    // long as the first. Us in clusters / through memory, bf16: one row 4096 x 9728 24.1 / 16.9, 4096 x 24576 50.4 / 35.0, eight
+    // rows 27.0 / 24.1, 56.3 / 43.7; int8, one row 4096 x 18432 24.5 / 19.1, four 1024 x 24576 14.2 / 17.5 but 4096 x 24576
+    // 32.3 / 29.6. The finish of five and more int8 rows costs more than the wave: eight rows 13.4 / 22.7 and 27.5 / 31.7.
+    // Half the columns per CTA where the grid would leave SMs without one, if those clusters fit too: one row of bf16
+    // 6144 x 4608, 36 of them, 19.3 us, with whole columns 14.0.
+    const int blocks = (N + cols - 1) / cols, halves = (N + cols / 2 - 1) / (cols / 2);
+    if (!ca && !aa && splits > 1 && splits <= 8) {
+      if (blocks * splits <= num_sms() &&
+          halves <= (is_int8 ? gemv_clusters<1, 1>(splits, kps) : gemv_clusters<2, 1>(splits, kps)))
+        return is_int8 ? launch_gemv_mma<1, 1, true>(p, splits, STREAM) : launch_gemv_mma<2, 1, true>(p, splits, STREAM);
+      if ((is_int8 && M > 4 && blocks * splits <= 4 * num_sms()) ||
+          blocks <= (is_int8 ? gemv_clusters<1, 2>(splits, kps) : gemv_clusters<2, 2>(splits, kps)))
         return is_int8 ? launch_gemv_mma<1, 2, true>(p, splits, STREAM) : launch_gemv_mma<2, 2, true>(p, splits, STREAM);
-      return is_int8 ? launch_gemv_mma<1, 1, true>(p, splits, STREAM) : launch_gemv_mma<2, 1, true>(p, splits, STREAM);
     }
     return is_int8 ? launch_gemv_mma<1, 2, false>(p, splits, STREAM) : launch_gemv_mma<2, 2, false>(p, splits, STREAM);
   }

@@ -431,7 +431,9 @@ def test_chains_of_dependent_launches_give_the_bits_of_plain_stream_order(rows, 
 
 @pytest.mark.parametrize("quant", [False, True])
 @pytest.mark.parametrize("M,K,N,splits", [(1, 1024, 264 + 8, 8), (8, 992, 1552, 8), (3, 4096, 4096, 8), (5, 200, 16, 3),
-                                          (1, 2816, 1024, 8), (8, 14336, 4096, 8), (2, 4096, 22016, 3), (7, 4096, 28672, 5)])
+                                          (1, 2816, 1024, 8), (8, 14336, 4096, 8), (2, 4096, 22016, 3), (7, 4096, 28672, 5),
+                                          # clusters of half blocks that do not fit at once, of whole blocks that do not
+                                          (1, 1024, 4608, 8), (2, 512, 9728, 8), (5, 512, 24576, 8)])
 def test_splits_that_finish_in_a_cluster_give_the_bits_of_the_finish_through_memory(quant, M, K, N, splits):
     """Grids of narrow and of wide column blocks, ragged last blocks, k ranges that end inside a tile: the fused LM head keeps
     the finish through memory, adds in the same order and so has the same logits; an output and a residual at odd addresses
