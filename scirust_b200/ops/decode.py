@@ -151,8 +151,18 @@ def _gemv_splits(N, K, cols, M=1, quant=False):
     if _GEMV_FMA:
         return s
     if K <= 16384:
+        ctas, halves = (N + cols - 1) // cols, (2 * N + cols - 1) // cols
+        # One row has the cheapest finish through memory, and where eight splits are about one CTA per SM, a long stream is faster
+        # as the two per SM of `_auto_splits`: narrow matrices, 17 to 20 (int8: 24) column blocks, and the 16 to 22 half blocks of
+        # int8, whose clusters do not fit at one CTA per SM. Us, eight splits / as many as before: bf16 14336 x 1024 14.3 / 12.5,
+        # x 2048 16.7 / 15.4, 8192 x 512 9.4 / 9.1, 9472 x 4608 20.5 / 18.5, 14336 x 5120 29.1 / 27.1; int8 14336 x 4096 24.0 / 20.7,
+        # 9472 x 4096 17.7 / 17.0, x 8704 27.3 / 22.4, x 12288 28.5 / 26.9, 6144 x 8704 18.7 / 16.9, 14336 x 4352 24.5 / 23.3; but
+        # bf16 11008 x 1024 11.8 / 12.2, 14336 x 4096 22.7 / 23.4, x 8192 38.9 / 40.2, int8 14336 x 3072 18.7 / 20.3.
+        if M == 1 and (K >= 6144 and 17 <= ctas <= 24 or K >= 9216 and halves == 16 or K >= 14336 and 17 <= halves <= 22 if quant else
+                       K >= 8192 and ctas <= 2 or K >= 12288 and ctas <= 10 or K >= 9216 and 17 <= ctas <= 20):
+            return s
         s = min(s, 8)
-        if (N + cols - 1) // cols > 148:          # several CTAs per SM, so at most 32 KB of staged X each: int8 4096 x 128256
+        if ctas > 148:                            # several CTAs per SM, so at most 32 KB of staged X each: int8 4096 x 128256
             s = max(s, (K + 2047) // 2048)        # at one split 114 us, at two 92
     return s
 

@@ -88,3 +88,17 @@ def test_convolution_without_patch_matrix(B, H, W, Cin, oc, k, stride, pad, impl
 ])
 def test_splits_of_the_weight_stream(K, N, M, quant, splits):
     assert D._auto_splits(N, K, 512 if quant else 256, M, quant) == splits
+
+
+@pytest.mark.parametrize("K,N,M,quant,splits", [
+    # up to eight finish in a cluster
+    (4096, 4096, 1, False, 8), (14336, 4096, 1, False, 8), (11008, 1024, 1, False, 8), (14336, 8192, 1, False, 8),
+    (14336, 3072, 1, True, 8), (14336, 3840, 1, True, 8), (4096, 8704, 1, True, 8), (8192, 4096, 1, True, 8), (14336, 2048, 2, False, 8),
+    (14336, 4096, 2, True, 8), (1024, 1536, 1, False, 8), (4096, 128256, 1, True, 2), (28672, 2048, 1, True, 44),
+    # one row, a long stream and about one CTA per SM with eight: as many as through memory
+    (14336, 1024, 1, False, 74), (14336, 2048, 1, False, 37), (8192, 512, 1, False, 64), (9472, 4608, 1, False, 16),
+    (14336, 5120, 1, False, 14), (14336, 4096, 1, True, 18), (9472, 4096, 1, True, 18), (9472, 8704, 1, True, 17),
+    (6144, 8704, 1, True, 17), (9472, 12288, 1, True, 12), (14336, 4352, 1, True, 18),
+])
+def test_splits_that_finish_in_a_cluster(K, N, M, quant, splits):
+    assert D._gemv_splits(N, K, 512 if quant else 256, M, quant) == splits
