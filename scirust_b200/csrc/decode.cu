@@ -350,16 +350,14 @@ gemv_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ 
     // the map is over 16-bit words: x = byte offset of the CTA's columns / 2 (a multiple of 256)
     const int x0 = col0 * ESZ / 2;
     pdl_wait();
-    for (int t = 0; t < ntiles; ++t) {
+    for (int t = 0; lane == 0 && t < ntiles; ++t) {     // one lane: a vote of the warp would delay every refill
       const int s = t % GEMV_STAGES;
-      if (t >= GEMV_STAGES && !mbar_wait_warp(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
-      if (lane == 0) {
-        // rows past K and columns past N arrive as zeros and still count towards the byte total
-        mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
-        tma_load_2d(tiles + s * GEMV_TILE_BYTES, &tmap_w, &full[s], x0, k0 + t * GEMV_KT);
-      }
-      __syncwarp();
+      if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
+      // rows past K and columns past N arrive as zeros and still count towards the byte total
+      mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
+      tma_load_2d(tiles + s * GEMV_TILE_BYTES, &tmap_w, &full[s], x0, k0 + t * GEMV_KT);
     }
+    __syncwarp();
   } else {
     // ------------------------------ consumers -----------------------------
     pdl_wait();   // X, the residual and the workspace belong to the previous kernel until here
@@ -617,19 +615,17 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   if (warp == 8) {
     // ------------------------------ producer ------------------------------
     pdl_wait();
-    for (int t = 0; t < ntiles; ++t) {
+    for (int t = 0; lane == 0 && t < ntiles; ++t) {     // one lane: a vote of the warp would delay every refill
       const int s = t % GEMV_STAGES;
-      if (t >= GEMV_STAGES && !mbar_wait_warp(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
-      if (lane == 0) {
-        // rows past K and columns past N arrive as zeros and still count towards the byte total
-        mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
+      if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
+      // rows past K and columns past N arrive as zeros and still count towards the byte total
+      mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < 2 * NB; ++c)
-          tma_load_2d(tiles + s * GEMV_TILE_BYTES + c * (KT * 128), &tmap_w, &full[s], col0 + c * 64,
-                      k0 + t * KT);
-      }
-      __syncwarp();
+      for (int c = 0; c < 2 * NB; ++c)
+        tma_load_2d(tiles + s * GEMV_TILE_BYTES + c * (KT * 128), &tmap_w, &full[s], col0 + c * 64,
+                    k0 + t * KT);
     }
+    __syncwarp();
   } else {
     // ------------------------------ consumers -----------------------------
     pdl_wait();   // X, the residual and the workspace belong to the previous kernel until here
@@ -915,19 +911,17 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   if (warp == 8) {
     // ------------------------------ producer ------------------------------
     pdl_wait();
-    for (int t = 0; t < ntiles; ++t) {
+    for (int t = 0; lane == 0 && t < ntiles; ++t) {     // one lane: a vote of the warp would delay every refill
       const int s = t % GEMV_STAGES;
-      if (t >= GEMV_STAGES && !mbar_wait_warp(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
-      if (lane == 0) {
-        // rows past K and columns past N arrive as zeros and still count towards the byte total
-        mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
+      if (t >= GEMV_STAGES && !mbar_wait(&empty[s], ((t / GEMV_STAGES) - 1) & 1, p.status, ST_TIMEOUT_EMPTY)) break;
+      // rows past K and columns past N arrive as zeros and still count towards the byte total
+      mbar_arrive_expect_tx(&full[s], GEMV_TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < 2 * NP; ++c)
-          tma_load_2d(tiles + s * GEMV_TILE_BYTES + c * (KT * 128), &tmap_w, &full[s], col0 / 2 + c * 64,
-                      k0 + t * KT);   // the map is over 16-bit words: 64 words = 128 int8 columns
-      }
-      __syncwarp();
+      for (int c = 0; c < 2 * NP; ++c)
+        tma_load_2d(tiles + s * GEMV_TILE_BYTES + c * (KT * 128), &tmap_w, &full[s], col0 / 2 + c * 64,
+                    k0 + t * KT);   // the map is over 16-bit words: 64 words = 128 int8 columns
     }
+    __syncwarp();
   } else {
     // ------------------------------ consumers -----------------------------
     pdl_wait();   // X, the residual and the workspace belong to the previous kernel until here
