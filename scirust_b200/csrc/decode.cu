@@ -562,8 +562,8 @@ __device__ __forceinline__ void gemv_mma_16816(float (&c)[4], const uint32_t (&a
 // The tensor core cuts its running sum off where fp32 addition rounds, so the error of a long k range grows with its length. After
 // GEMV_SUM_ROWS rows of k the accumulators are added to sums of rounded fp32 additions and start again, whatever the split: error
 // against 64 bits, one row, eight splits, without / with: 4096 x 4096 4.7e-7 / 1.4e-7, 14336 x 4096 1.8e-6 / 1.5e-7 (eighteen splits
-// without: 2.4e-7, 7.7e-7). Us without / with: a layer of Llama-3-8B
-// shape, one row 101.4 / 101.5; LM head 4096 x 128256 172 / 173, int8 101.7 / 103.3.
+// without: 2.4e-7, 7.7e-7). It costs nothing as a group of tiles whose
+// loop is unrolled: int8 4096 x 128256 at two splits 93.4 us as a test in every tile, 92.4 so, eight rows 4096 x 4096 11.1 / 10.7.
 constexpr int GEMV_SUM_ROWS = 128;
 template <int NB, int MBLK>
 __device__ __forceinline__ void gemv_add_clear(float (&total)[NB][MBLK][4], float (&acc)[NB][MBLK][4]) {
@@ -744,34 +744,40 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     const int mi = lane >> 3, lr = lane & 7;
     const int sub = warp * NB >> 2;                     // which 64-column box holds this warp's columns
     const uint32_t tiles_u32 = smem_u32(tiles) + sub * (KT * 128);
-    for (int t = 0; t < ntiles; ++t) {
-      const int s = t % GEMV_STAGES;
-      if (!mbar_wait_warp(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
-      const uint32_t tbase = tiles_u32 + s * GEMV_TILE_BYTES;
+    for (int t0 = 0; t0 < ntiles; t0 += GEMV_SUM_ROWS / KT) {
 #pragma unroll
-      for (int ks = 0; ks < KT / 16; ++ks) {
-        if (KT > 32 && t * KT + ks * 16 >= k1 - k0) break;   // the rest of the tile belongs to the next split
-        const int kp = (t * KT + ks * 16) >> 1;      // index of the first bf16 pair of this k-step
-        uint32_t b0[MBLK], b1[MBLK];
+      for (int i = 0; i < GEMV_SUM_ROWS / KT; ++i) {
+        const int t = t0 + i;
+        if (t >= ntiles) break;
+        const int s = t % GEMV_STAGES;
+        // a wait that gives up does not end the loop, in which the warp has to stay together; the status word says so
+        mbar_wait(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL);
+        const uint32_t tbase = tiles_u32 + s * GEMV_TILE_BYTES;
 #pragma unroll
-        for (int mb = 0; mb < MBLK; ++mb) {
-          const bool live = mb * 8 + g < M;
-          b0[mb] = live ? xs32[(kp + tq) * XR + mb * 8 + g] : 0u;
-          b1[mb] = live ? xs32[(kp + 4 + tq) * XR + mb * 8 + g] : 0u;
+        for (int ks = 0; ks < KT / 16; ++ks) {
+          if (KT > 32 && t * KT + ks * 16 >= k1 - k0) break;   // the rest of the tile belongs to the next split
+          const int kp = (t * KT + ks * 16) >> 1;      // index of the first bf16 pair of this k-step
+          uint32_t b0[MBLK], b1[MBLK];
+#pragma unroll
+          for (int mb = 0; mb < MBLK; ++mb) {
+            const bool live = mb * 8 + g < M;
+            b0[mb] = live ? xs32[(kp + tq) * XR + mb * 8 + g] : 0u;
+            b1[mb] = live ? xs32[(kp + 4 + tq) * XR + mb * 8 + g] : 0u;
+          }
+          const int r = ks * 16 + (mi >> 1) * 8 + lr;       // k row inside the tile
+#pragma unroll
+          for (int nb = 0; nb < NB; ++nb) {
+            const int chunk = (warp * NB & 3) * 2 + nb * 2 + (mi & 1);   // 16-byte chunk of the 128-byte row
+            uint32_t a[4];
+            gemv_ldsm_x4_t(tbase + r * 128 + ((chunk ^ (r & 7)) << 4), a);
+#pragma unroll
+            for (int mb = 0; mb < MBLK; ++mb) gemv_mma_16816(acc[nb][mb], a, b0[mb], b1[mb]);
+          }
         }
-        const int r = ks * 16 + (mi >> 1) * 8 + lr;       // k row inside the tile
-#pragma unroll
-        for (int nb = 0; nb < NB; ++nb) {
-          const int chunk = (warp * NB & 3) * 2 + nb * 2 + (mi & 1);   // 16-byte chunk of the 128-byte row
-          uint32_t a[4];
-          gemv_ldsm_x4_t(tbase + r * 128 + ((chunk ^ (r & 7)) << 4), a);
-#pragma unroll
-          for (int mb = 0; mb < MBLK; ++mb) gemv_mma_16816(acc[nb][mb], a, b0[mb], b1[mb]);
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
-      if ((t + 1) % (GEMV_SUM_ROWS / KT) == 0 || t + 1 == ntiles) gemv_add_clear(total, acc);
+      gemv_add_clear(total, acc);
     }
   }
   __syncthreads();
@@ -1045,46 +1051,51 @@ gemv_mma_i8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const int sub = warp * NP >> 2;                     // which 128-column box holds this warp's columns
     const uint32_t tiles_u32 = smem_u32(tiles) + sub * (KT * 128);
     const __half2 bias = __floats2half2_rn(1152.f, 1152.f);   // 1024 (the magic exponent) + 128 (the sign flip)
-    for (int t = 0; t < ntiles; ++t) {
-      const int s = t % GEMV_STAGES;
-      if (!mbar_wait_warp(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL)) break;
-      const uint32_t tbase = tiles_u32 + s * GEMV_TILE_BYTES;
+    for (int t0 = 0; t0 < ntiles; t0 += GEMV_SUM_ROWS / KT) {
 #pragma unroll
-      for (int ks = 0; ks < KT / 16; ++ks) {
-        if (KT > 32 && t * KT + ks * 16 >= k1 - k0) break;   // the rest of the tile belongs to the next split
-        const int kp = (t * KT + ks * 16) >> 1;      // index of the first fp16 pair of this k-step
-        const bool live = g < M;
-        const uint32_t b0 = live ? xs32[(kp + tq) * XR + g] : 0u;
-        const uint32_t b1 = live ? xs32[(kp + 4 + tq) * XR + g] : 0u;
-        const int r = ks * 16 + (mi & 1) * 8 + lr;        // k row inside the tile
+      for (int i = 0; i < GEMV_SUM_ROWS / KT; ++i) {
+        const int t = t0 + i;
+        if (t >= ntiles) break;
+        const int s = t % GEMV_STAGES;
+        mbar_wait(&full[s], (t / GEMV_STAGES) & 1, p.status, ST_TIMEOUT_FULL);
+        const uint32_t tbase = tiles_u32 + s * GEMV_TILE_BYTES;
 #pragma unroll
-        for (int pr = 0; pr < NP; ++pr) {                  // two n blocks of 16 columns per ldmatrix.x4
-          const int chunk = (warp * NP & 3) * 2 + pr * 2 + (mi >> 1);   // 16-byte chunk = 16 int8 columns
-          uint32_t raw[4];
-          gemv_ldsm_x4_t(tbase + r * 128 + ((chunk ^ (r & 7)) << 4), raw);
+        for (int ks = 0; ks < KT / 16; ++ks) {
+          if (KT > 32 && t * KT + ks * 16 >= k1 - k0) break;   // the rest of the tile belongs to the next split
+          const int kp = (t * KT + ks * 16) >> 1;      // index of the first fp16 pair of this k-step
+          const bool live = g < M;
+          const uint32_t b0 = live ? xs32[(kp + tq) * XR + g] : 0u;
+          const uint32_t b1 = live ? xs32[(kp + 4 + tq) * XR + g] : 0u;
+          const int r = ks * 16 + (mi & 1) * 8 + lr;        // k row inside the tile
 #pragma unroll
-          for (int q2 = 0; q2 < 2; ++q2) {
-            // int8 -> fp16 without the conversion pipe: flip the sign bit (value + 128 as an unsigned byte), drop the
-            // byte into the mantissa of 1024.0 and subtract 1152
-            const uint32_t u_lo = raw[q2 * 2] ^ 0x80808080u, u_hi = raw[q2 * 2 + 1] ^ 0x80808080u;
-            uint32_t a[4];
-            a[0] = __byte_perm(u_lo, 0x64646464u, 0x4240);   // row g     (even column), k 0-7
-            a[1] = __byte_perm(u_lo, 0x64646464u, 0x4341);   // row g + 8 (odd column),  k 0-7
-            a[2] = __byte_perm(u_hi, 0x64646464u, 0x4240);   // k 8-15
-            a[3] = __byte_perm(u_hi, 0x64646464u, 0x4341);
+          for (int pr = 0; pr < NP; ++pr) {                  // two n blocks of 16 columns per ldmatrix.x4
+            const int chunk = (warp * NP & 3) * 2 + pr * 2 + (mi >> 1);   // 16-byte chunk = 16 int8 columns
+            uint32_t raw[4];
+            gemv_ldsm_x4_t(tbase + r * 128 + ((chunk ^ (r & 7)) << 4), raw);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              __half2 h = *reinterpret_cast<__half2*>(&a[e]);
-              h = __hsub2(h, bias);
-              a[e] = *reinterpret_cast<uint32_t*>(&h);
+            for (int q2 = 0; q2 < 2; ++q2) {
+              // int8 -> fp16 without the conversion pipe: flip the sign bit (value + 128 as an unsigned byte), drop the
+              // byte into the mantissa of 1024.0 and subtract 1152
+              const uint32_t u_lo = raw[q2 * 2] ^ 0x80808080u, u_hi = raw[q2 * 2 + 1] ^ 0x80808080u;
+              uint32_t a[4];
+              a[0] = __byte_perm(u_lo, 0x64646464u, 0x4240);   // row g     (even column), k 0-7
+              a[1] = __byte_perm(u_lo, 0x64646464u, 0x4341);   // row g + 8 (odd column),  k 0-7
+              a[2] = __byte_perm(u_hi, 0x64646464u, 0x4240);   // k 8-15
+              a[3] = __byte_perm(u_hi, 0x64646464u, 0x4341);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                __half2 h = *reinterpret_cast<__half2*>(&a[e]);
+                h = __hsub2(h, bias);
+                a[e] = *reinterpret_cast<uint32_t*>(&h);
+              }
+              gemv_mma_16816_f16(acc[pr * 2 + q2][0], a, b0, b1);
             }
-            gemv_mma_16816_f16(acc[pr * 2 + q2][0], a, b0, b1);
           }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
-      if ((t + 1) % (GEMV_SUM_ROWS / KT) == 0 || t + 1 == ntiles) gemv_add_clear(total, acc);
+      gemv_add_clear(total, acc);
     }
   }
   __syncthreads();
