@@ -9,8 +9,8 @@
 // stays below 2^8, far inside its range), which on real score distributions happens in the first blocks
 // only; at 128 by anything. There the reference is the running maximum itself, as in the one-tile kernel,
 // so the largest weight of a row is 1 and has no rounding; with the 2^8 margin the error against float64
-// was 2 % larger for unit scores and 20 % larger for scores of twice the spread. The rescales cost 5 %. The row sum uses the same reference point, so the final O / l
-// and the log-sum-exp are exact regardless of when a rescale happened.
+// was 2 % larger for unit scores and 20 % larger for scores of twice the spread. The rescales cost 5 %. The row sum uses
+// the same reference point, so the final O / l and the log-sum-exp are exact regardless of when a rescale happened.
 //
 // Same interface, layout and semantics as the one-tile kernel (attention_fwd_tcgen05.cu): fused
 // activation matrix qkv [B*S, ld] = [q heads | k heads | v heads], scores scaled by 1/sqrt(dh),
@@ -21,9 +21,10 @@
 //
 // A softmax thread holds its whole 128-column score row in registers (one pass over tensor memory),
 // scales it with packed fp32 pairs (fma.rn.f32x2, add.rn.f32x2: half the issue slots of scalar
-// code) and takes the row maximum with three-input max. Its warps are the bottleneck: two of them share a
-// scheduler and its special-function unit, 1024 cycles for the 128 exponentials of a block each, while the
-// products of a block need 2 x 512 cycles at head dimension 128. So nothing else may stand in their way:
+// code) and takes the row maximum with three-input max. What bounds the kernel is the chain inside a tile: scores, maximum,
+// exponentials, P, P V. Two softmax warps share a scheduler, so the special-function unit needs 1024 cycles for a block of
+// both tiles, and so does the tensor pipe at head dimension 128; a block takes about twice that, and each of the two is
+// busy half of the time (profiles/attention_issue_and_softmax.md). Nothing else may lengthen the chain:
 //  - Every tile has an issuing warp of its own, and the scores of block j+1 are issued as soon as those of block j
 //    are in registers, so they are there when block j is done. With one issuer for both tiles the waits of one
 //    tile held up the other.
@@ -33,8 +34,8 @@
 //  - The mask is applied to the scores of the blocks that need one; as a select beside every exponential it
 //    cost all blocks a third of their instructions.
 // The softmax warpgroups take the registers that the issuing one does not need (setmaxnreg), so rows stay unspilled.
-// us before / now, causal, 32 heads of 128: 5000 tokens 262 / 209 (980 TFLOP/s), 4096 185 / 154, 2 x 2048 112 / 100;
-// 16 heads of 64: 8 x 2048 160 / 147.
+// us before all this / now, causal, 32 heads of 128, calls back to back on one input: 5000 tokens 262 / 206 (990 TFLOP/s; 237 and
+// 860 for a call among others on new inputs), 4096 185 / 154, 2 x 2048 112 / 96; 16 heads of 64: 8 x 2048 160 / 150.
 //
 // Head dimension 128: Q (64 KB), two P tiles (64 KB) and a K tile of 32 KB twice leave 32 KB for V. K gets two whole
 // stages; V is a ring of two half tiles of 64 kv rows, because the products consume V row by row: the first half is

@@ -15,8 +15,9 @@
 //                      accumulation (exact), one rescale by sx[m] * sw[n].
 // Split-K partials (fp32 / int32) are added in split order: inside a thread-block cluster, whose CTAs are the splits of one
 // column tile, where all these clusters are on the GPU at once (it holds 33 of four CTAs, 45 of three), else by
-// skinny_reduce_kernel from [split][row][N] in memory (us with that kernel / in the cluster: 4096 x 4096, 16 rows 10.4 / 9.1,
-// 64 rows 12.9 / 10.5, int8 13.3 / 11.9; 14336 x 4096, 64 rows 25.8 / 23.6).
+// skinny_reduce_kernel from [split][row][N] in memory. Us with that kernel / in the cluster, in a chain of dependent launches:
+// 4096 x 4096, 16 rows 8.6 / 8.2, 64 rows 11.1 / 9.2, int8 11.9 / 9.9; 14336 x 4096, 64 rows 24.5 / 22.0, int8 17.2 / 15.7; 1024 x
+// 1024, 64 int8 rows 8.0 / 7.4. The 48 tiles of a 6144-wide product in three splits are three too many for it.
 // Warps: 0 TMA, 1 MMA, 2-5 epilogue (one per TMEM lane quarter).
 #include "sm100_ptx.cuh"
 #include "api.h"

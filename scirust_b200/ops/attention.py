@@ -28,18 +28,21 @@ FWD_TWO_TILES = os.environ.get("SB_ATT_FWD", "pair") != "single"
 
 
 def _two_tiles_win(B, S, H, dh, causal, device) -> bool:
-    """Where the two-tile kernel is the faster one, by the CTAs that each of the two starts.
+    """Which of the two kernels runs, by the CTAs that each of them starts.
 
-    Head dimension 128 (one CTA per SM in both): a CTA of two tiles takes about 1.7 times as long as one of a single
-    tile, so while its grid fits the GPU at once one tile wins, and beyond that it must save waves: sequences of up to
-    256 rows need more than 1.5 times fewer, up to 384 (the second CTA of a head has one tile) 1.5 times, longer ones
-    always do. Causal, 32 heads, us, one tile against two: 1 x 1000 (128 CTAs) 26.3 / 27.7, 1 x 1300 (192) 45.3 / 35.0,
-    2 x 1000 51.4 / 39.5, 9 x 256 29.5 / 25.6, but 6 x 256 21.6 / 24.3, 3 x 333 17.9 / 22.4, 5 x 333 30.9 / 33.2.
+    Head dimension 128 (one CTA per SM in both): a CTA of two tiles took about 1.7 times as long as one of a single
+    tile when these lines were drawn, so while its grid fits the GPU at once one tile runs, and beyond that two must save
+    waves: sequences of up to 256 rows need more than 1.5 times fewer, up to 384 (the second CTA of a head has one tile)
+    1.5 times, longer ones always do. The two-tile kernel has become the faster by more since, and the lines lie too far
+    out by up to a third. Causal, 32 heads, us, one tile / two: taken as two 1 x 1300 43.0 / 29.2, 2 x 1000 49.2 / 32.8,
+    9 x 256 28.9 / 20.8; as one 1 x 128 6.5 / 6.7, 2 x 256 8.9 / 10.3, 3 x 333 17.4 / 18.7, and, where two would be faster,
+    1 x 1000 25.1 / 23.4, 2 x 512 18.9 / 15.3, 4 x 256 15.0 / 11.0, 5 x 333 30.1 / 27.6, 12 x 333 63.1 / 53.3.
 
     Head dimension 64 (two CTAs per SM with one tile, one with two), 16 heads: while the two-tile grid fits the GPU at
-    once one tile is faster for causal sequences, but past 512 rows for an even number of tiles only (the longest tile
-    of an odd number runs alone in its CTA): 1 x 512 11.5 / 13.6, 2 x 1000 21.1 / 21.6, but 3 x 600 14.8 / 14.3; without
-    the mask up to 384 rows only: 3 x 333 9.9 / 11.9, but 2 x 1000 24.4 / 22.0."""
+    once one tile runs for causal sequences, but past 512 rows for an even number of tiles only (the longest tile
+    of an odd number runs alone in its CTA): 1 x 512 10.7 / 11.6, 1 x 1000 17.8 / 18.8, but 3 x 600 13.9 / 12.2; without
+    the mask up to 384 rows only: 3 x 333 9.6 / 11.6, but 2 x 1000 22.2 / 21.2. Off the faster side by now: causal 3 x 333
+    9.1 / 8.1 (one runs), 16 x 100 7.4 / 10.3 (two run), without the mask 1 x 512 10.6 / 12.8 (two run)."""
     sms, tiles = _g.num_sms(device), (S + 127) // 128
     one, two = B * H * tiles, B * H * ((S + 255) // 256)
     if dh == 64:

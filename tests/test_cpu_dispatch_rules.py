@@ -1,5 +1,6 @@
 """Rules that choose between two kernels by sizes, on the CPU, for a GPU of 148 SMs: each line is a shape at which both
-sides were timed, with the side that was faster (or, within 2 %, the one that was there first)."""
+sides were timed, with the side that the rule takes: the faster one (or, within 2 %, the one that was there first) when the line
+was drawn. The attention forward's kernels have changed since its lines were; the rule's comment says where it is off."""
 import subprocess
 from pathlib import Path
 
