@@ -57,6 +57,8 @@ int sb_maxpool_fwd(const void* x, void* y, void* arg, int B, int H, int W, int C
 int sb_maxpool_bwd(const void* dy, const void* arg, void* dx, int B, int H, int W, int C, int k, int stride, int OH, int OW, void* stream);
 int sb_colstats_masked(const void* a, const void* b, const void* mask, float* partial, float* s1, float* s2, int rows, int C, void* stream);
 int sb_bn_fwd(const void* x, const float* sum, const float* sumsq, const float* gamma, const float* beta, float* mean, float* inv_std, float* run_mean, float* run_var, void* y, int rows, int C, float eps, float momentum, int relu, int training, void* stream);
+int sb_bn_layer_fwd(const void* x, float* partial, const float* gamma, const float* beta, float* mean, float* inv_std, float* run_mean, float* run_var, const void* res, void* y, int rows, int C, float eps, float momentum, int relu, void* stream);
+int sb_bn_layer_bwd(const void* dy, const void* x, const void* mask, void* g_out, float* partial, const float* mean, const float* inv_std, const float* gamma, float* dgamma, float* dbeta, void* dx, int rows, int C, void* stream);
 int sb_bn_bwd_masked(const void* g, const void* x, const float* sum_g, const float* sum_gx, const float* mean, const float* inv_std, const float* gamma, float* dgamma, float* dbeta, const void* mask, void* dx, int rows, int C, void* stream);
 int sb_colstats(const void* a, const void* b, float* partial, float* s1, float* s2, int rows, int C, void* stream);
 int sb_bn_bwd(const void* g, const void* x, const float* sum_g, const float* sum_gx, const float* mean, const float* inv_std, const float* gamma, float* dgamma, float* dbeta, void* dx, int rows, int C, void* stream);

@@ -247,24 +247,29 @@ __device__ __forceinline__ void conv_unpack8(const uint4& v, float (&f)[8]) {
 __device__ __forceinline__ uint4 conv_pack8(const float (&f)[8]) {
   return make_uint4(conv_pack(f[0], f[1]), conv_pack(f[2], f[3]), conv_pack(f[4], f[5]), conv_pack(f[6], f[7]));
 }
-// a word of eight bf16 values where the same word of y is positive, else zero
+// How the gradient of a ReLU is masked by the forward output y: where y is positive, or (after an added shortcut) where y is not
+// zero or below, so that a NaN in y lets the gradient through as torch's own ReLU does.
+enum : int { MASK_NONE = 0, MASK_POSITIVE = 1, MASK_NOT_BELOW = 2 };
+// a word of eight bf16 values where the mask of the same word of y holds, else zero
+template <int MASK>
 __device__ __forceinline__ uint4 conv_relu_mask8(uint4 g, const uint4& y) {
   float f[8], m[8];
   conv_unpack8(g, f);
   conv_unpack8(y, m);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) f[j] = m[j] > 0.f ? f[j] : 0.f;
+  for (int j = 0; j < 8; ++j) f[j] = (MASK == MASK_POSITIVE ? m[j] > 0.f : !(m[j] <= 0.f)) ? f[j] : 0.f;
   return conv_pack8(f);
 }
 
 // Stage 1 of the backward sums for C a multiple of 8: bound by the bytes of the matrices. A block takes 64 columns (8 words of 16 bytes)
-// of a chunk of 256 rows, 32 row lanes of 8 rows each, all loads of a thread in flight; lanes, then warps are added in
+// of a chunk of 256 rows, 32 row lanes of 8 rows each, four rows' loads of a thread in flight; lanes, then warps are added in
 // a fixed order. The one-column-per-thread kernel above walks its 256 rows in one dependent chain of 2-byte loads: 39 us
-// for 131072 x 64, 8 us here.
-template <bool MASK>
+// for 131072 x 64, 8 us here. MASK_NOT_BELOW also writes the masked gradient to g_out: it is the shortcut's gradient, and the input
+// gradient then reads it instead of dy and the mask.
+template <int MASK>
 __global__ void __launch_bounds__(256)
 colstats_vec8_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, const uint4* __restrict__ mask,
-                     float* __restrict__ partial, int rows, int C8) {
+                     uint4* __restrict__ g_out, float* __restrict__ partial, int rows, int C8) {
   __shared__ float s_sum[8][8][16];                 // [warp][column word][sum x: 8 | sum xy: 8]
   const int cw = threadIdx.x & 7, rl = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c8 = blockIdx.x * 8 + cw;
@@ -273,25 +278,34 @@ colstats_vec8_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, c
 #pragma unroll
   for (int j = 0; j < 8; ++j) s1[j] = s2[j] = 0.f;
   if (c8 < C8) {
-    uint4 va[8], vb[8];
+    constexpr int U = MASK ? 4 : 8;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = r0 + i * 32;
-      va[i] = vb[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (r < rows) {
-        const size_t at = static_cast<size_t>(r) * C8 + c8;
-        va[i] = __ldg(a + at);
-        vb[i] = __ldg(b + at);
-        if (MASK) va[i] = conv_relu_mask8(va[i], __ldg(mask + at));
+    for (int i0 = 0; i0 < 8; i0 += U) {
+      uint4 va[U], vb[U], vm[U];
+#pragma unroll
+      for (int i = 0; i < U; ++i) {
+        const int r = r0 + (i0 + i) * 32;
+        va[i] = vb[i] = vm[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (r < rows) {
+          const size_t at = static_cast<size_t>(r) * C8 + c8;
+          va[i] = __ldg(a + at);
+          vb[i] = __ldg(b + at);
+          if (MASK) vm[i] = __ldg(mask + at);
+        }
       }
-    }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float x[8], y[8];
-      conv_unpack8(va[i], x);
-      conv_unpack8(vb[i], y);
+      for (int i = 0; i < U; ++i) {
+        if (MASK) va[i] = conv_relu_mask8<MASK>(va[i], vm[i]);
+        if (MASK == MASK_NOT_BELOW) {
+          const int r = r0 + (i0 + i) * 32;
+          if (r < rows) g_out[static_cast<size_t>(r) * C8 + c8] = va[i];
+        }
+        float x[8], y[8];
+        conv_unpack8(va[i], x);
+        conv_unpack8(vb[i], y);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { s1[j] += x[j]; s2[j] += x[j] * y[j]; }
+        for (int j = 0; j < 8; ++j) { s1[j] += x[j]; s2[j] += x[j] * y[j]; }
+      }
     }
   }
 #pragma unroll
@@ -320,7 +334,7 @@ colstats_vec8_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b, c
 // Stage 1 of the FORWARD statistics for even C, in the order of the kernel at the top: a column's 256 rows of a chunk in
 // one chain. Mean and variance decide on which side of zero a normalised value falls, and with it the ReLU mask, so the
 // order of these sums is kept to the bit; the loads are what is rearranged (a thread owns two columns and has 32 rows in
-// flight, a warp reads 128 contiguous bytes per row): 39 -> 10 us for 131072 x 64.
+// flight, a warp reads 128 contiguous bytes per row): 39 -> 10 us for 131072 x 64; 64 in flight are level.
 __global__ void __launch_bounds__(128)
 colstats_chain_kernel(const uint32_t* __restrict__ a, float* __restrict__ partial, int rows, int C2) {
   const int c2 = blockIdx.x * 32 + (threadIdx.x & 31);
@@ -329,13 +343,14 @@ colstats_chain_kernel(const uint32_t* __restrict__ a, float* __restrict__ partia
   if (c2 >= C2 || r0 >= rows) return;
   const uint32_t* p = a + static_cast<size_t>(r0) * C2 + c2;
   float s1l = 0.f, s2l = 0.f, s1h = 0.f, s2h = 0.f;
+  constexpr int U = 32;
   int r = r0;
-  for (; r + 32 <= r1; r += 32, p += static_cast<size_t>(32) * C2) {
-    uint32_t v[32];
+  for (; r + U <= r1; r += U, p += static_cast<size_t>(U) * C2) {
+    uint32_t v[U];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __ldg(p + static_cast<size_t>(i) * C2);
+    for (int i = 0; i < U; ++i) v[i] = __ldg(p + static_cast<size_t>(i) * C2);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
+    for (int i = 0; i < U; ++i) {
       const float x = conv_bf_lo(v[i]), y = conv_bf_hi(v[i]);
       s1l += x;
       s2l += x * x;
@@ -358,45 +373,71 @@ colstats_chain_kernel(const uint32_t* __restrict__ a, float* __restrict__ partia
   o[2 * C2 + 1] = s2h;
 }
 
-// Stage 2, chunks in ascending order: 32 columns per block. All threads bring 64 chunks at a time into shared memory
-// (the next 64 on their way meanwhile); the additions of a column, which are one chain, then run at shared-memory speed
-// instead of at a memory latency every few chunks (512 chunks: 28 -> 7 us).
-constexpr int CF_CHUNKS = 64;
-__global__ void __launch_bounds__(256)
-colstats_finish_kernel(const float* __restrict__ partial, int chunks, int C, float* __restrict__ s1,
-                       float* __restrict__ s2) {
-  __shared__ float s[CF_CHUNKS * 64];                    // [chunk][sum x: 32 | sum xy: 32]
-  constexpr int PER = CF_CHUNKS * 64 / 256;
-  const int e = threadIdx.x & 63, row0 = threadIdx.x >> 6;   // this thread's element of a chunk; its chunks row0 + 4 i
-  const int c = blockIdx.x * 32 + (e & 31);
-  const float* src = partial + static_cast<size_t>(e >> 5) * C + c;
-  float v[PER];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int k = k0 + row0 + 4 * i;
-      v[i] = (k < chunks && c < C) ? __ldg(src + static_cast<size_t>(k) * 2 * C) : 0.f;
-    }
-  };
-  fetch(0);
+// Stage 2, chunks in ascending order, and what is made of a column's two sums: nothing (FIN_SUMS), mean, 1 / standard deviation and
+// the running statistics of a forward pass (FIN_FORWARD: biased variance to normalise, unbiased for the running one), or the gradients
+// of shift and scale (FIN_BACKWARD: dbeta = sum g, dgamma = sum g*xhat = (sum g*x - mean * sum g) * inv_std).
+// Eight columns per block, so that 512 chunks are on their way at once and then added, one chain a sum, at shared-memory speed: the
+// chain is what is left (131072 x 64: 5.3 us; 7.2 with 32 columns per block and 64 chunks at a time, and 1.7 to 2.6 for
+// what followed in a launch of its own).
+enum : int { FIN_SUMS = 0, FIN_FORWARD = 1, FIN_BACKWARD = 2 };
+struct BnFinish {
+  float *o1, *o2;               // FIN_SUMS: the sums; FIN_FORWARD: mean, inv_std; FIN_BACKWARD: dbeta, dgamma
+  float *run_mean, *run_var;    // FIN_FORWARD, optional
+  const float *mean, *inv_std;  // FIN_BACKWARD
+  int rows;
+  float eps, momentum;
+};
+constexpr int CF_COLS = 8, CF_CHUNKS = 512, CF_THREADS = 256;
+template <int WHAT>
+__global__ void __launch_bounds__(CF_THREADS)
+colstats_finish_kernel(const float* __restrict__ partial, int chunks, int C, const BnFinish f) {
+  __shared__ float s[CF_CHUNKS * 2 * CF_COLS];           // [chunk][sum x: 8 | sum xy: 8]
+  constexpr int STEP = CF_THREADS / (2 * CF_COLS), PER = CF_CHUNKS / STEP;
+  const int e = threadIdx.x % (2 * CF_COLS), row0 = threadIdx.x / (2 * CF_COLS);   // this thread's element of a chunk; its chunks row0 + STEP i
+  const int c = blockIdx.x * CF_COLS + e % CF_COLS;
+  const float* src = partial + static_cast<size_t>(e / CF_COLS) * C + c;
   float acc = 0.f;
   for (int k0 = 0; k0 < chunks; k0 += CF_CHUNKS) {
-    __syncthreads();
+    float v[PER];
 #pragma unroll
-    for (int i = 0; i < PER; ++i) s[(row0 + 4 * i) * 64 + e] = v[i];
+    for (int i = 0; i < PER; ++i) {
+      const int k = k0 + row0 + STEP * i;
+      v[i] = (k < chunks && c < C) ? __ldg(src + static_cast<size_t>(k) * 2 * C) : 0.f;
+    }
+    __syncthreads();                                     // the chains have read the chunks before
+#pragma unroll
+    for (int i = 0; i < PER; ++i) s[(row0 + STEP * i) * (2 * CF_COLS) + e] = v[i];
     __syncthreads();
-    if (k0 + CF_CHUNKS < chunks) fetch(k0 + CF_CHUNKS);
-    if (threadIdx.x < 64) {
+    if (threadIdx.x < 2 * CF_COLS) {
       const int n = min(CF_CHUNKS, chunks - k0);
 #pragma unroll 16
-      for (int k = 0; k < n; ++k) acc += s[k * 64 + e];
+      for (int k = 0; k < n; ++k) acc += s[k * (2 * CF_COLS) + e];
     }
   }
-  if (threadIdx.x < 64 && c < C) (e < 32 ? s1 : s2)[c] = acc;
+  if (threadIdx.x >= 32) return;                         // what is left is one warp's
+  const float other = __shfl_down_sync(0xffffffffu, acc, CF_COLS);
+  if (threadIdx.x >= CF_COLS || c >= C) return;
+  if (WHAT == FIN_SUMS) {
+    f.o1[c] = acc;
+    f.o2[c] = other;
+  } else if (WHAT == FIN_FORWARD) {
+    const float n = static_cast<float>(f.rows);
+    const float m = acc / n;
+    const float var = fmaxf(other / n - m * m, 0.f);
+    f.o1[c] = m;
+    f.o2[c] = rsqrtf(var + f.eps);
+    if (f.run_mean) {
+      f.run_mean[c] = (1.f - f.momentum) * f.run_mean[c] + f.momentum * m;
+      const float unbiased = f.rows > 1 ? var * n / (n - 1.f) : var;
+      f.run_var[c] = (1.f - f.momentum) * f.run_var[c] + f.momentum * unbiased;
+    }
+  } else {
+    f.o1[c] = acc;
+    f.o2[c] = (other - f.mean[c] * acc) * f.inv_std[c];
+  }
 }
 
-// BatchNorm forward (training): from column sums, mean/var (biased for normalisation), update
-// running stats (unbiased variance), y = (x-mean)*inv_std*gamma + beta, optional fused ReLU.
+// BatchNorm forward from sums taken elsewhere: mean and variance as in FIN_FORWARD above.
 __global__ void bn_prepare_kernel(const float* __restrict__ sum, const float* __restrict__ sumsq, int rows, int C,
                                   float eps, float momentum, float* __restrict__ mean, float* __restrict__ inv_std,
                                   float* __restrict__ run_mean, float* __restrict__ run_var) {
@@ -413,6 +454,7 @@ __global__ void bn_prepare_kernel(const float* __restrict__ sum, const float* __
     run_var[c] = (1.f - momentum) * run_var[c] + momentum * unbiased;
   }
 }
+// y = (x - mean) * inv_std * gamma + beta, optional ReLU
 __global__ void bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ mean,
                                 const float* __restrict__ inv_std, const float* __restrict__ gamma,
                                 const float* __restrict__ beta, __nv_bfloat16* __restrict__ y, size_t total, int C,
@@ -429,26 +471,55 @@ __device__ __forceinline__ void conv_load8(const float* __restrict__ p, float (&
   const float4 u = __ldg(reinterpret_cast<const float4*>(p)), v = __ldg(reinterpret_cast<const float4*>(p) + 1);
   f[0] = u.x; f[1] = u.y; f[2] = u.z; f[3] = u.w; f[4] = v.x; f[5] = v.y; f[6] = v.z; f[7] = v.w;
 }
+// U words of one thread lie 256 words apart: the same channels where a row's words divide 256, and the channels' values are then
+// loaded once. RES adds the shortcut of a residual block before the ReLU, with the roundings and the treatment of NaN that two torch
+// operators on the rounded output have. Us for 131072 x 64, one word a thread / four: 11.6 / 6.3, with a shortcut 7.9.
+template <int U, bool RES>
 __global__ void __launch_bounds__(256)
 bn_apply_vec8_kernel(const uint4* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ inv_std,
-                     const float* __restrict__ gamma, const float* __restrict__ beta, uint4* __restrict__ y,
-                     uint32_t total, FastDiv by_c8, int relu) {
-  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
-  if (i >= total) return;
+                     const float* __restrict__ gamma, const float* __restrict__ beta, const uint4* __restrict__ res,
+                     uint4* __restrict__ y, uint32_t total, FastDiv by_c8, int relu) {
+  const uint32_t i0 = blockIdx.x * (256u * U) + threadIdx.x;
+  if (i0 >= total) return;
   uint32_t c8;
-  by_c8.divmod(i, c8);
-  float v[8], m[8], s[8], g[8], b[8];
-  conv_unpack8(__ldg(x + i), v);
+  by_c8.divmod(i0, c8);
+  uint4 xw[U], rw[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t i = min(i0 + u * 256u, total - 1);
+    xw[u] = __ldg(x + i);
+    if (RES) rw[u] = __ldg(res + i);
+  }
+  float m[8], s[8], g[8], b[8];
   conv_load8(mean + c8 * 8, m);
   conv_load8(inv_std + c8 * 8, s);
   conv_load8(gamma + c8 * 8, g);
   conv_load8(beta + c8 * 8, b);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    v[j] = (v[j] - m[j]) * s[j] * g[j] + b[j];
-    if (relu) v[j] = fmaxf(v[j], 0.f);
+  for (int u = 0; u < U; ++u) {
+    const uint32_t i = i0 + u * 256u;
+    if (i >= total) break;
+    float v[8];
+    conv_unpack8(xw[u], v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = (v[j] - m[j]) * s[j] * g[j] + b[j];
+      if (!RES && relu) v[j] = fmaxf(v[j], 0.f);
+    }
+    uint4 o = conv_pack8(v);
+    if (RES) {
+      float r[8];
+      conv_unpack8(o, v);
+      conv_unpack8(rw[u], r);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] = __fadd_rn(v[j], r[j]);
+        if (relu && v[j] <= 0.f) v[j] = 0.f;
+      }
+      o = conv_pack8(v);
+    }
+    y[i] = o;
   }
-  y[i] = conv_pack8(v);
 }
 // BatchNorm backward. With xhat = (x-mean)*inv_std, g = dy (already masked by ReLU when fused):
 //   dbeta = sum g, dgamma = sum g*xhat, dx = gamma*inv_std/n * (n*g - dbeta - xhat*dgamma)
@@ -476,34 +547,50 @@ __global__ void bn_bwd_dx_kernel(const __nv_bfloat16* __restrict__ g, const __nv
   const float v = gamma[c] * inv_std[c] / n * (n * gi - dbeta[c] - xhat * dgamma[c]);
   dx[i] = __float2bfloat16_rn(v);
 }
-template <bool MASK>
+// U as in bn_apply_vec8_kernel; the quotient of a channel is taken once a thread. Us for 131072 x 64, one word a thread / four: 15.4 / 8.4, with
+// a mask 16.0 / 10.4.
+template <int U, int MASK>
 __global__ void __launch_bounds__(256)
 bn_bwd_dx_vec8_kernel(const uint4* __restrict__ g, const uint4* __restrict__ x, const float* __restrict__ mean,
                       const float* __restrict__ inv_std, const float* __restrict__ gamma,
                       const float* __restrict__ dgamma, const float* __restrict__ dbeta,
                       const uint4* __restrict__ mask, uint4* __restrict__ dx, uint32_t total, FastDiv by_c8, int rows) {
-  const uint32_t i = blockIdx.x * 256u + threadIdx.x;
-  if (i >= total) return;
+  const uint32_t i0 = blockIdx.x * (256u * U) + threadIdx.x;
+  if (i0 >= total) return;
   uint32_t c8;
-  by_c8.divmod(i, c8);
+  by_c8.divmod(i0, c8);
   const float n = static_cast<float>(rows);
-  uint4 gw = __ldg(g + i);
-  const uint4 xw = __ldg(x + i);
-  if (MASK) gw = conv_relu_mask8(gw, __ldg(mask + i));
-  float gi[8], xi[8], m[8], s[8], ga[8], dg[8], db[8];
-  conv_unpack8(gw, gi);
-  conv_unpack8(xw, xi);
+  uint4 gw[U], xw[U], mw[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t i = min(i0 + u * 256u, total - 1);
+    gw[u] = __ldg(g + i);
+    xw[u] = __ldg(x + i);
+    if (MASK) mw[u] = __ldg(mask + i);
+  }
+  float m[8], s[8], k[8], dg[8], db[8];
   conv_load8(mean + c8 * 8, m);
   conv_load8(inv_std + c8 * 8, s);
-  conv_load8(gamma + c8 * 8, ga);
+  conv_load8(gamma + c8 * 8, k);
   conv_load8(dgamma + c8 * 8, dg);
   conv_load8(dbeta + c8 * 8, db);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float xhat = (xi[j] - m[j]) * s[j];
-    gi[j] = ga[j] * s[j] / n * (n * gi[j] - db[j] - xhat * dg[j]);
+  for (int j = 0; j < 8; ++j) k[j] = k[j] * s[j] / n;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t i = i0 + u * 256u;
+    if (i >= total) break;
+    if (MASK) gw[u] = conv_relu_mask8<MASK>(gw[u], mw[u]);
+    float gi[8], xi[8];
+    conv_unpack8(gw[u], gi);
+    conv_unpack8(xw[u], xi);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float xhat = (xi[j] - m[j]) * s[j];
+      gi[j] = k[j] * (n * gi[j] - db[j] - xhat * dg[j]);
+    }
+    dx[i] = conv_pack8(gi);
   }
-  dx[i] = conv_pack8(gi);
 }
 // g = dy * (y > 0)
 __global__ void relu_mask_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ y,
@@ -582,29 +669,79 @@ extern "C" int sb_maxpool_bwd(const void* dy, const void* arg, void* dx, int B, 
                                                       static_cast<__nv_bfloat16*>(dx), B, H, W, C, k, stride, OH, OW);
   CHECK_LAUNCH();
 }
+// Whether the kernels of eight channels a thread take a [rows, C] matrix (addresses aside).
+static bool bn_vec8(size_t total, int C) { return (C & 7) == 0 && total / 8 <= 0x7fffff00u; }
+// Words of a thread: see bn_apply_vec8_kernel. A small matrix keeps one, so that its words reach all SMs (148 x 4 blocks of 256).
+static int bn_words(size_t total, int C) { return 256 % (C / 8) == 0 && total / 8 >= 4u * 148 * 4 * 256 ? 4 : 1; }
+
+// Column sums of a and of a * b into `partial` (2 * ceil(rows/256) * C floats) and what WHAT makes of them. g_out: see colstats_vec8_kernel.
+template <int WHAT>
+static int colstats(const void* a, const void* b, const void* mask, void* g_out, float* partial, const BnFinish& f, int rows, int C,
+                    cudaStream_t stream) {
+  const int chunks = (rows + 255) / 256;
+  const uint4 *a4 = static_cast<const uint4*>(a), *b4 = static_cast<const uint4*>(b), *m4 = static_cast<const uint4*>(mask);
+  const bool vec8 = (C & 7) == 0 && chunks <= 65535 && conv_al16(a, b, mask, g_out);
+  if (g_out && !vec8) return SB_ERR_ARG;
+  if (a == b && !mask && (C & 1) == 0 && (reinterpret_cast<uintptr_t>(a) & 3) == 0 && (chunks + 3) / 4 <= 65535) {
+    colstats_chain_kernel<<<dim3((C / 2 + 31) / 32, (chunks + 3) / 4), 128, 0, stream>>>(static_cast<const uint32_t*>(a),
+                                                                                        partial, rows, C / 2);
+  } else if (vec8) {
+    const dim3 grid((C / 8 + 7) / 8, chunks);
+    auto kern = g_out ? colstats_vec8_kernel<MASK_NOT_BELOW> : mask ? colstats_vec8_kernel<MASK_POSITIVE> : colstats_vec8_kernel<MASK_NONE>;
+    kern<<<grid, 256, 0, stream>>>(a4, b4, m4, static_cast<uint4*>(g_out), partial, rows, C / 8);
+  } else {
+    dim3 grid((C + 127) / 128, chunks);
+    auto kern = mask ? colstats_partial_kernel<true> : colstats_partial_kernel<false>;
+    kern<<<grid, 128, 0, stream>>>(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b),
+                                   static_cast<const __nv_bfloat16*>(mask), partial, rows, C);
+  }
+  if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
+  colstats_finish_kernel<WHAT><<<(C + CF_COLS - 1) / CF_COLS, CF_THREADS, 0, stream>>>(partial, chunks, C, f);
+  return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+}
+static int bn_apply(const void* x, const float* mean, const float* inv_std, const float* gamma, const float* beta,
+                    const void* res, void* y, int rows, int C, int relu, cudaStream_t stream) {
+  const size_t total = static_cast<size_t>(rows) * C;
+  if (bn_vec8(total, C) && conv_al16(x, y, res) && conv_al16(mean, inv_std, gamma, beta)) {
+    const int u = bn_words(total, C);
+    auto kern = u == 4 ? (res ? bn_apply_vec8_kernel<4, true> : bn_apply_vec8_kernel<4, false>)
+                       : (res ? bn_apply_vec8_kernel<1, true> : bn_apply_vec8_kernel<1, false>);
+    kern<<<nblk((total / 8 + u - 1) / u), 256, 0, stream>>>(static_cast<const uint4*>(x), mean, inv_std, gamma, beta,
+                                                            static_cast<const uint4*>(res), static_cast<uint4*>(y),
+                                                            static_cast<uint32_t>(total / 8), FastDiv(C / 8), relu);
+    CHECK_LAUNCH();
+  }
+  if (res) return SB_ERR_ARG;
+  bn_apply_kernel<<<nblk(total), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), mean, inv_std, gamma, beta,
+                                                   static_cast<__nv_bfloat16*>(y), total, C, relu);
+  CHECK_LAUNCH();
+}
+static int bn_bwd_dx(const void* g, const void* x, const float* mean, const float* inv_std, const float* gamma,
+                     const float* dgamma, const float* dbeta, const void* mask, void* dx, int rows, int C, cudaStream_t stream) {
+  const size_t total = static_cast<size_t>(rows) * C;
+  if (bn_vec8(total, C) && conv_al16(g, x, dx, mask) && conv_al16(mean, inv_std, gamma) && conv_al16(dgamma, dbeta)) {
+    const int u = bn_words(total, C);
+    auto kern = u == 4 ? (mask ? bn_bwd_dx_vec8_kernel<4, MASK_POSITIVE> : bn_bwd_dx_vec8_kernel<4, MASK_NONE>)
+                       : (mask ? bn_bwd_dx_vec8_kernel<1, MASK_POSITIVE> : bn_bwd_dx_vec8_kernel<1, MASK_NONE>);
+    kern<<<nblk((total / 8 + u - 1) / u), 256, 0, stream>>>(
+        static_cast<const uint4*>(g), static_cast<const uint4*>(x), mean, inv_std, gamma, dgamma, dbeta,
+        static_cast<const uint4*>(mask), static_cast<uint4*>(dx), static_cast<uint32_t>(total / 8), FastDiv(C / 8), rows);
+    CHECK_LAUNCH();
+  }
+  bn_bwd_dx_kernel<<<nblk(total), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(g),
+                                                    static_cast<const __nv_bfloat16*>(x), mean, inv_std, gamma,
+                                                    dgamma, dbeta, static_cast<const __nv_bfloat16*>(mask),
+                                                    static_cast<__nv_bfloat16*>(dx), total, C, rows);
+  CHECK_LAUNCH();
+}
 // s1 = column sums of a, s2 = of a * b; `mask` (optional, same shape): elements of a count where mask > 0.
 // partial: 2 * ceil(rows/256) * C floats
 extern "C" int sb_colstats_masked(const void* a, const void* b, const void* mask, float* partial, float* s1, float* s2,
                                   int rows, int C, void* stream) {
   if (rows <= 0 || C <= 0) return SB_ERR_ARG;
-  const int chunks = (rows + 255) / 256;
-  if (a == b && !mask && (C & 1) == 0 && (reinterpret_cast<uintptr_t>(a) & 3) == 0 && (chunks + 3) / 4 <= 65535) {
-    colstats_chain_kernel<<<dim3((C / 2 + 31) / 32, (chunks + 3) / 4), 128, 0, STREAM>>>(static_cast<const uint32_t*>(a),
-                                                                                        partial, rows, C / 2);
-  } else if ((C & 7) == 0 && chunks <= 65535 && conv_al16(a, b, mask)) {
-    const dim3 grid((C / 8 + 7) / 8, chunks);
-    auto kern = mask ? colstats_vec8_kernel<true> : colstats_vec8_kernel<false>;
-    kern<<<grid, 256, 0, STREAM>>>(static_cast<const uint4*>(a), static_cast<const uint4*>(b),
-                                   static_cast<const uint4*>(mask), partial, rows, C / 8);
-  } else {
-    dim3 grid((C + 127) / 128, chunks);
-    auto kern = mask ? colstats_partial_kernel<true> : colstats_partial_kernel<false>;
-    kern<<<grid, 128, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b),
-                                   static_cast<const __nv_bfloat16*>(mask), partial, rows, C);
-  }
-  if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
-  colstats_finish_kernel<<<(C + 31) / 32, 256, 0, STREAM>>>(partial, chunks, C, s1, s2);
-  CHECK_LAUNCH();
+  BnFinish f = {};
+  f.o1 = s1; f.o2 = s2;
+  return colstats<FIN_SUMS>(a, b, mask, nullptr, partial, f, rows, C, STREAM);
 }
 extern "C" int sb_bn_fwd(const void* x, const float* sum, const float* sumsq, const float* gamma, const float* beta,
                          float* mean, float* inv_std, float* run_mean, float* run_var, void* y, int rows, int C,
@@ -615,16 +752,37 @@ extern "C" int sb_bn_fwd(const void* x, const float* sum, const float* sumsq, co
                                                            run_mean, run_var);
     if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   }
-  const size_t total = static_cast<size_t>(rows) * C;
-  if ((C & 7) == 0 && total / 8 <= 0x7fffff00u && conv_al16(x, y) && conv_al16(mean, inv_std, gamma, beta)) {
-    bn_apply_vec8_kernel<<<nblk(total / 8), 256, 0, STREAM>>>(static_cast<const uint4*>(x), mean, inv_std, gamma, beta,
-                                                              static_cast<uint4*>(y), static_cast<uint32_t>(total / 8),
-                                                              FastDiv(C / 8), relu);
-    CHECK_LAUNCH();
+  return bn_apply(x, mean, inv_std, gamma, beta, nullptr, y, rows, C, relu, STREAM);
+}
+// The forward pass of a layer: with `partial` (2 * ceil(rows/256) * C floats) on the batch's own statistics, which are written to mean
+// and inv_std and into the running ones (optional); without it mean and inv_std are given. res (optional, C a multiple of 8, 16-byte
+// aligned like the other tensors, else SB_ERR_ARG): a shortcut that is added before the ReLU.
+extern "C" int sb_bn_layer_fwd(const void* x, float* partial, const float* gamma, const float* beta, float* mean, float* inv_std,
+                               float* run_mean, float* run_var, const void* res, void* y, int rows, int C, float eps,
+                               float momentum, int relu, void* stream) {
+  if (rows <= 0 || C <= 0) return SB_ERR_ARG;
+  if (res && !(bn_vec8(static_cast<size_t>(rows) * C, C) && conv_al16(x, y, res) && conv_al16(mean, inv_std, gamma, beta)))
+    return SB_ERR_ARG;
+  if (partial) {
+    BnFinish f = {};
+    f.o1 = mean; f.o2 = inv_std; f.run_mean = run_mean; f.run_var = run_var;
+    f.rows = rows; f.eps = eps; f.momentum = momentum;
+    const int rc = colstats<FIN_FORWARD>(x, x, nullptr, nullptr, partial, f, rows, C, STREAM);
+    if (rc) return rc;
   }
-  bn_apply_kernel<<<nblk(total), 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x), mean, inv_std, gamma, beta,
-                                                   static_cast<__nv_bfloat16*>(y), total, C, relu);
-  CHECK_LAUNCH();
+  return bn_apply(x, mean, inv_std, gamma, beta, res, y, rows, C, relu, STREAM);
+}
+// Its backward pass. mask (optional): the forward output after a fused ReLU; dy counts where it is positive. g_out (optional, with a
+// mask; C a multiple of 8 and all tensors 16-byte aligned, else SB_ERR_ARG): the masked dy, the gradient of an added shortcut.
+extern "C" int sb_bn_layer_bwd(const void* dy, const void* x, const void* mask, void* g_out, float* partial, const float* mean,
+                               const float* inv_std, const float* gamma, float* dgamma, float* dbeta, void* dx, int rows, int C,
+                               void* stream) {
+  if (rows <= 0 || C <= 0 || (g_out && !mask)) return SB_ERR_ARG;
+  BnFinish f = {};
+  f.o1 = dbeta; f.o2 = dgamma; f.mean = mean; f.inv_std = inv_std;
+  const int rc = colstats<FIN_BACKWARD>(dy, x, mask, g_out, partial, f, rows, C, STREAM);
+  if (rc) return rc;
+  return bn_bwd_dx(g_out ? g_out : dy, x, mean, inv_std, gamma, dgamma, dbeta, g_out ? nullptr : mask, dx, rows, C, STREAM);
 }
 // mask (optional): the forward output after a fused ReLU; g counts where it is positive (sum_g, sum_gx likewise).
 extern "C" int sb_bn_bwd_masked(const void* g, const void* x, const float* sum_g, const float* sum_gx,
@@ -633,21 +791,7 @@ extern "C" int sb_bn_bwd_masked(const void* g, const void* x, const float* sum_g
   if (rows <= 0 || C <= 0) return SB_ERR_ARG;
   bn_bwd_finish_kernel<<<(C + 127) / 128, 128, 0, STREAM>>>(sum_g, sum_gx, mean, inv_std, C, dgamma, dbeta);
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
-  const size_t total = static_cast<size_t>(rows) * C;
-  if ((C & 7) == 0 && total / 8 <= 0x7fffff00u && conv_al16(g, x, dx, mask) && conv_al16(mean, inv_std, gamma) &&
-      conv_al16(dgamma, dbeta)) {
-    auto kern = mask ? bn_bwd_dx_vec8_kernel<true> : bn_bwd_dx_vec8_kernel<false>;
-    kern<<<nblk(total / 8), 256, 0, STREAM>>>(static_cast<const uint4*>(g), static_cast<const uint4*>(x), mean, inv_std,
-                                              gamma, dgamma, dbeta, static_cast<const uint4*>(mask),
-                                              static_cast<uint4*>(dx), static_cast<uint32_t>(total / 8),
-                                              FastDiv(C / 8), rows);
-    CHECK_LAUNCH();
-  }
-  bn_bwd_dx_kernel<<<nblk(total), 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(g),
-                                                    static_cast<const __nv_bfloat16*>(x), mean, inv_std, gamma,
-                                                    dgamma, dbeta, static_cast<const __nv_bfloat16*>(mask),
-                                                    static_cast<__nv_bfloat16*>(dx), total, C, rows);
-  CHECK_LAUNCH();
+  return bn_bwd_dx(g, x, mean, inv_std, gamma, dgamma, dbeta, mask, dx, rows, C, STREAM);
 }
 // The forms without a mask: entry points of their own in the C ABI.
 extern "C" int sb_colstats(const void* a, const void* b, float* partial, float* s1, float* s2, int rows, int C,

@@ -28,7 +28,7 @@ class ConvLayer(nn.Module):
         self.bias = nn.Parameter(torch.zeros(out_c)) if bias else None
 
     def forward(self, x, geom):
-        y, og = C.conv2d(x, self.weight.to(BF), geom, self.k, self.stride, self.pad)
+        y, og = C.conv2d_master(x, self.weight, geom, self.k, self.stride, self.pad)
         if self.bias is not None:
             y = y + self.bias.to(BF)
         return y, og
@@ -45,9 +45,10 @@ class BNLayer(nn.Module):
         self.register_buffer("running_var", torch.ones(c))
         self.relu = relu
 
-    def forward(self, x):
-        return C.batchnorm(x, self.gamma, self.beta, self.running_mean, self.running_var, relu=self.relu,
-                           training=self.training)
+    def forward(self, x, shortcut=None):
+        """``shortcut``: added to the layer's output, before a ReLU that follows the sum."""
+        return C.batchnorm(x, self.gamma, self.beta, self.running_mean, self.running_var,
+                           relu=self.relu or shortcut is not None, training=self.training, shortcut=shortcut)
 
 
 class _DenseFn(torch.autograd.Function):
@@ -100,6 +101,14 @@ class MnistCNN(nn.Module):
         return self.f2(torch.relu(self.f1(y))).float()
 
 
+def _adds_shortcut(bn) -> bool:
+    """Whether a block's last norm may add the shortcut and apply the ReLU in its own pass: a ``BNLayer`` whose own output nothing
+    else sees (no hooks, no replaced ``forward``)."""
+    return (type(bn) is BNLayer and not bn.relu and "forward" not in bn.__dict__
+            and not (bn._forward_hooks or bn._forward_pre_hooks or bn._backward_hooks or bn._backward_pre_hooks)
+            and not torch.nn.modules.module._has_any_global_hook())
+
+
 class BasicBlock(nn.Module):
     def __init__(self, in_c, out_c, stride, gen):
         super().__init__()
@@ -112,6 +121,9 @@ class BasicBlock(nn.Module):
     def forward(self, x, g):
         y, g1 = self.conv1(x, g)
         y, g2 = self.conv2(self.bn1(y), g1)
+        if _adds_shortcut(self.bn2):
+            s = x if self.short is None else self.short_bn(self.short(x, g)[0])
+            return self.bn2(y, s), g2
         y = self.bn2(y)
         s = x if self.short is None else self.short_bn(self.short(x, g)[0])
         return torch.relu(y + s), g2

@@ -19,9 +19,8 @@ _lib.register("sb_im2col_nhwc", [vp, vp] + [i32] * 11 + [vp])
 _lib.register("sb_col2im_nhwc", [vp, vp] + [i32] * 11 + [vp])
 _lib.register("sb_maxpool_fwd", [vp, vp, vp] + [i32] * 8 + [vp])
 _lib.register("sb_maxpool_bwd", [vp, vp, vp] + [i32] * 8 + [vp])
-_lib.register("sb_colstats_masked", [vp, vp, vp, vp, vp, vp, i32, i32, vp])
-_lib.register("sb_bn_fwd", [vp] * 10 + [i32, i32, f32, f32, i32, i32, vp])
-_lib.register("sb_bn_bwd_masked", [vp] * 11 + [i32, i32, vp])
+_lib.register("sb_bn_layer_fwd", [vp] * 10 + [i32, i32, f32, f32, i32, vp])
+_lib.register("sb_bn_layer_bwd", [vp] * 11 + [i32, i32, vp])
 _lib.register("sb_bias_act", [vp, vp, vp, sz, i32, i32, vp])
 
 
@@ -67,7 +66,7 @@ def unpack_conv_weight(wp: torch.Tensor, in_c: int, k: int) -> torch.Tensor:
 
 _lib.register("sb_conv_gemm", [i32, vp, vp, vp] + [i32] * 11 + [vp, vp, vp])
 _lib.register("sb_conv_fprop_keep", [vp, vp, vp, vp] + [i32] * 11 + [vp, vp, vp])
-_FPROP, _WGRAD, _DGRAD = 1, 2, 3
+_FPROP, _WGRAD, _DGRAD, _WGRAD_F32 = 1, 2, 3, 4
 
 
 def _rows_tile(oh: int, ow: int, box: int) -> bool:
@@ -87,13 +86,17 @@ def implicit_ok(geom: ConvGeom, oc: int, k: int, stride: int, pad: int) -> bool:
             and (ow - 1) * stride < 256 and (128 // ow - 1) * stride < 256)
 
 
-def _conv_gemm(mode, a, b, geom, oc, k, stride, pad, OH, OW, keep=None):
+def _conv_gemm(mode, a, b, geom, oc, k, stride, pad, OH, OW, keep=None, f32=False):
     pix_o, pix_i, kp = geom.B * OH * OW, geom.rows, k * k * geom.C
-    M, N, K = {_FPROP: (pix_o, oc, kp), _WGRAD: (oc, kp, pix_o), _DGRAD: (pix_i, geom.C, k * k * oc)}[mode]
-    out = _lib.empty((M, N), BF, a.device)
+    M, N, K = ((pix_o, oc, kp) if mode == _FPROP else (oc, kp, pix_o) if mode == _WGRAD else (pix_i, geom.C, k * k * oc))
     # one wave of work items, at least eight 64-deep k-blocks each (a weight gradient has K = pixels and few tiles)
     tiles = ((M + 127) // 128) * ((N + 255) // 256)
     splits = max(1, min(G.num_sms(a.device) // tiles, (K + 63) // 64 // 8, 64))
+    if f32 and splits > 1:                              # the sum of the splits is written as it is
+        mode, dtype = _WGRAD_F32, torch.float32
+    else:
+        dtype = BF
+    out = _lib.empty((M, N), dtype, a.device)
     ws = G._workspace(splits * M * N, a.device) if splits > 1 else None
     rest = (geom.B, geom.H, geom.W, geom.C, oc, k, stride, pad, OH, OW, splits, _lib.ptr(ws),
             _lib.status_word(a.device).data_ptr(), _lib.stream())
@@ -102,13 +105,18 @@ def _conv_gemm(mode, a, b, geom, oc, k, stride, pad, OH, OW, keep=None):
     else:
         _lib.call("sb_conv_fprop_keep", a.data_ptr(), b.data_ptr(), out.data_ptr(), keep.data_ptr(), *rest)
     G.launch_count += 2 if splits > 1 else 1
-    return out
+    return out.float() if f32 and dtype == BF else out
 
 
 class _Conv(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, wp, geom, k, stride, pad, want_dw):
+    def forward(ctx, x, wp, geom, k, stride, pad, want_dw, master=False):
         B, H, W, C = geom.B, geom.H, geom.W, geom.C
+        ctx.master = master
+        if master:                                      # fp32 weights: rounded here, and their gradient is fp32 too
+            w32, wp = wp.contiguous(), _lib.empty(wp.shape, BF, wp.device)
+            _lib.call("sb_cast", w32.data_ptr(), wp.data_ptr(), wp.numel(), 1, 1.0, _lib.stream())
+            G.launch_count += 1
         OH, OW = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
         ctx.meta = (geom, k, stride, pad, OH, OW)
         ctx.implicit = implicit_ok(geom, wp.shape[0], k, stride, pad) and _tma_ok(x, wp, geom, k)
@@ -138,17 +146,21 @@ class _Conv(torch.autograd.Function):
             raise ValueError("conv2d: the output gradient must be bf16 and 16-byte aligned")
         dx = dw = None
         if ctx.needs_input_grad[1]:
-            dw = (_conv_gemm(_WGRAD, dy, col, geom, oc, k, stride, pad, OH, OW) if implicit
-                  else G.matmul_tn(dy, col))                  # [oc, Kp] = dy^T col
+            if implicit:
+                dw = _conv_gemm(_WGRAD, dy, col, geom, oc, k, stride, pad, OH, OW, f32=ctx.master)
+            else:
+                dw = G.matmul_tn(dy, col)                     # [oc, Kp] = dy^T col
+                if ctx.master:
+                    dw = dw.float()
         if ctx.needs_input_grad[0]:
             if implicit and stride == 1 and _rows_tile(geom.H, geom.W, 128):
-                return _conv_gemm(_DGRAD, dy, wp, geom, oc, k, stride, pad, OH, OW), dw, None, None, None, None, None
+                return _conv_gemm(_DGRAD, dy, wp, geom, oc, k, stride, pad, OH, OW), dw, None, None, None, None, None, None
             dcol = G.matmul_nn(dy, wp)                        # [M, Kp]
             dx = _lib.empty((geom.rows, geom.C), BF, dy.device)
             _lib.call("sb_col2im_nhwc", dcol.data_ptr(), dx.data_ptr(), geom.B, geom.H, geom.W, geom.C, k, k, stride,
                       pad, OH, OW, wp.shape[1], _lib.stream())
             G.launch_count += 1
-        return dx, dw, None, None, None, None, None
+        return dx, dw, None, None, None, None, None, None
 
 
 def _tma_ok(x, wp, geom, k) -> bool:
@@ -167,6 +179,16 @@ def conv2d(x, wp, geom: ConvGeom, k: int, stride: int = 1, pad: int = 0):
         return nchw_to_rows(y4.to(x.dtype))[0], og
     want_dw = torch.is_grad_enabled() and wp.requires_grad
     return _Conv.apply(x.contiguous(), wp, geom, k, stride, pad, want_dw), og
+
+
+def conv2d_master(x, w32, geom: ConvGeom, k: int, stride: int = 1, pad: int = 0):
+    """``conv2d(x, w32.to(bfloat16), ...)`` for fp32 master weights, as one node of the graph: the same y and dx to the bit, and a
+    weight gradient that is not rounded to bf16 where its sum is split."""
+    if not x.is_cuda or w32.dtype != torch.float32 or w32.device != x.device:
+        return conv2d(x, w32.to(BF), geom, k, stride, pad)
+    og = ConvGeom(geom.B, (geom.H + 2 * pad - k) // stride + 1, (geom.W + 2 * pad - k) // stride + 1, w32.shape[0])
+    want_dw = torch.is_grad_enabled() and w32.requires_grad
+    return _Conv.apply(x.contiguous(), w32, geom, k, stride, pad, want_dw, True), og
 
 
 class _MaxPool(torch.autograd.Function):
@@ -202,63 +224,74 @@ def maxpool2d(x, geom: ConvGeom, k: int, stride: int):
     return _MaxPool.apply(x.contiguous(), geom, k, stride), og
 
 
-def _colstats(a, b, mask=None):
-    """Column sums of ``a`` and of ``a * b``; with ``mask`` only the elements of ``a`` where it is positive count."""
-    rows, C = a.shape
-    part = torch.empty(2 * ((rows + 255) // 256) * C, dtype=torch.float32, device=a.device)
-    s1 = _lib.empty(C, torch.float32, a.device)
-    s2 = _lib.empty(C, torch.float32, a.device)
-    _lib.call("sb_colstats_masked", a.data_ptr(), b.data_ptr(), _lib.ptr(mask), part.data_ptr(), s1.data_ptr(), s2.data_ptr(), rows, C,
-              _lib.stream())
-    G.launch_count += 2
-    return s1, s2
-
-
 class _BatchNorm(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, gamma, beta, run_mean, run_var, eps, momentum, relu, training):
+    def forward(ctx, x, gamma, beta, run_mean, run_var, eps, momentum, relu, training, shortcut=None):
         rows, C = x.shape
-        mean = _lib.empty(C, torch.float32, x.device)
-        inv = _lib.empty(C, torch.float32, x.device)
+        stat = _lib.empty((2, C), torch.float32, x.device)          # mean, 1 / standard deviation
+        mean_p = stat.data_ptr()
+        inv_p = mean_p + 4 * C
+        part = None
         if training:
-            s1, s2 = _colstats(x, x)
+            part = torch.empty(2 * ((rows + 255) // 256) * C, dtype=torch.float32, device=x.device)
         else:
-            s1 = s2 = None
-            mean.copy_(run_mean)
-            inv.copy_(torch.rsqrt(run_var + eps))
+            stat[0].copy_(run_mean)
+            stat[1].copy_(torch.rsqrt(run_var + eps))
         y = torch.empty_like(x)
-        _lib.call("sb_bn_fwd", x.data_ptr(), _lib.ptr(s1), _lib.ptr(s2), gamma.data_ptr(), beta.data_ptr(),
-                  mean.data_ptr(), inv.data_ptr(), _lib.ptr(run_mean) if training else None,
-                  _lib.ptr(run_var) if training else None, y.data_ptr(), rows, C, float(eps), float(momentum),
-                  int(relu), int(training), _lib.stream())
-        G.launch_count += 2
-        ctx.save_for_backward(x, y, gamma, mean, inv)
-        ctx.relu = relu
+        _lib.call("sb_bn_layer_fwd", x.data_ptr(), _lib.ptr(part), gamma.data_ptr(), beta.data_ptr(), mean_p, inv_p,
+                  _lib.ptr(run_mean) if training else None, _lib.ptr(run_var) if training else None, _lib.ptr(shortcut),
+                  y.data_ptr(), rows, C, float(eps), float(momentum), int(relu), _lib.stream())
+        G.launch_count += 3 if training else 1
+        ctx.save_for_backward(x, y, gamma, stat)
+        ctx.relu, ctx.added = relu, shortcut is not None
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, y, gamma, mean, inv = ctx.saved_tensors
+        x, y, gamma, stat = ctx.saved_tensors
         rows, C = x.shape
         dy = dy.contiguous()
         mask = y if ctx.relu else None                  # the ReLU's mask is applied where dy is read
-        sg, sgx = _colstats(dy, x, mask)
+        ds = None
+        if ctx.added and not ctx.relu:
+            ds = dy
+        elif ctx.added:                                 # the masked dy, written by the kernel that reads dy first
+            ds = torch.empty_like(x)
+            if dy.data_ptr() % 16:
+                dy = dy.clone()
+        part = torch.empty(2 * ((rows + 255) // 256) * C, dtype=torch.float32, device=x.device)
         dgamma = _lib.empty(C, torch.float32, x.device)
         dbeta = _lib.empty(C, torch.float32, x.device)
         dx = torch.empty_like(x)
-        _lib.call("sb_bn_bwd_masked", dy.data_ptr(), x.data_ptr(), sg.data_ptr(), sgx.data_ptr(), mean.data_ptr(),
-                  inv.data_ptr(), gamma.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), _lib.ptr(mask), dx.data_ptr(),
+        mean_p = stat.data_ptr()
+        _lib.call("sb_bn_layer_bwd", dy.data_ptr(), x.data_ptr(), _lib.ptr(mask), _lib.ptr(ds) if ctx.relu else None,
+                  part.data_ptr(), mean_p, mean_p + 4 * C, gamma.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), dx.data_ptr(),
                   rows, C, _lib.stream())
-        G.launch_count += 2
-        return dx, dgamma, dbeta, None, None, None, None, None, None
+        G.launch_count += 3
+        return dx, dgamma, dbeta, None, None, None, None, None, None, ds
 
 
-def batchnorm(x, gamma, beta, run_mean, run_var, eps=1e-5, momentum=0.1, relu=False, training=True):
-    """Per-channel batch norm of [rows, C] (fp32 gamma/beta/running stats), optional fused ReLU."""
+def _adds_inside(x, gamma, beta, shortcut) -> bool:
+    """Whether the BatchNorm kernels add ``shortcut`` themselves: whole 16-byte words of eight channels everywhere, within the range of
+    their indexes (words) and grids (chunks of 256 rows). Else two torch operators do."""
+    return (x.dtype == BF and shortcut.dtype == BF and shortcut.shape == x.shape and x.shape[1] % 8 == 0
+            and x.numel() // 8 <= 0x7fffff00 and x.shape[0] <= 65535 * 256 and x.device == shortcut.device
+            and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, shortcut, gamma, beta)))
+
+
+def batchnorm(x, gamma, beta, run_mean, run_var, eps=1e-5, momentum=0.1, relu=False, training=True, shortcut=None):
+    """Per-channel batch norm of [rows, C] (fp32 gamma/beta/running stats), optional fused ReLU. ``shortcut`` is added to the
+    rounded result before the ReLU, with the results of ``relu(batchnorm(x) + shortcut)`` to the bit."""
     if not x.is_cuda:
         y = F.batch_norm(x.float().t().unsqueeze(0), run_mean, run_var, gamma, beta, training, momentum, eps)[0].t()
+        if shortcut is not None:
+            y = y.to(x.dtype) + shortcut
         return (torch.relu(y) if relu else y).to(x.dtype)
-    return _BatchNorm.apply(x.contiguous(), gamma, beta, run_mean, run_var, eps, momentum, relu, training)
+    x = x.contiguous()
+    if shortcut is not None and not _adds_inside(x, gamma, beta, shortcut):
+        y = _BatchNorm.apply(x, gamma, beta, run_mean, run_var, eps, momentum, False, training) + shortcut
+        return torch.relu(y) if relu else y
+    return _BatchNorm.apply(x, gamma, beta, run_mean, run_var, eps, momentum, relu, training, shortcut)
 
 
 def bias_act(x, bias, relu=False):

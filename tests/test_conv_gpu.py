@@ -175,3 +175,52 @@ def test_conv_input_may_be_written_before_the_backward_pass():
     y, _ = C.conv2d(x, frozen, geom, 3, 1, 1)
     x.data.fill_(float("nan"))
     assert torch.isfinite(torch.autograd.grad(y, x, dy)[0].float()).all()
+
+
+@pytest.mark.parametrize("rows,C_", [(1, 8), (255, 72), (2050, 520), (131072 + 3, 64), (40000, 256), (300, 12)])
+@pytest.mark.parametrize("relu,training", [(True, True), (False, True), (True, False)])
+def test_batchnorm_adds_a_shortcut(rows, C_, relu, training):
+    """The shortcut inside the norm's kernels against two torch operators behind them: one and four words a thread, last
+    blocks that end inside, more chunks than one round of the sums holds, channel counts that go the general way, NaN in x and
+    infinities in the shortcut. The same operations on the same roundings, so everything agrees to the bit."""
+    g = torch.Generator(device="cuda").manual_seed(rows + C_)
+    x = torch.randn(rows, C_, generator=g, device="cuda").to(BF)
+    s = torch.randn(rows, C_, generator=g, device="cuda").to(BF)
+    dy = torch.randn(rows, C_, generator=g, device="cuda").to(BF)
+    x[0, 3], s[0, 1], s[0, 2] = float("nan"), float("inf"), float("-inf")
+    gamma, beta = torch.rand(C_, generator=g, device="cuda") + 0.5, torch.randn(C_, generator=g, device="cuda")
+    got = []
+    for inside in (True, False):
+        xi, si, gi, bi = (t.clone().requires_grad_(True) for t in (x, s, gamma, beta))
+        rm, rv = torch.zeros(C_, device="cuda"), torch.ones(C_, device="cuda")
+        if inside:
+            y = C.batchnorm(xi, gi, bi, rm, rv, relu=relu, training=training, shortcut=si)
+        else:
+            y = C.batchnorm(xi, gi, bi, rm, rv, training=training) + si
+            y = torch.relu(y) if relu else y
+        got.append([y.detach(), rm, rv, *torch.autograd.grad(y, (xi, si, gi, bi), dy)])
+    for a, b in zip(*got):
+        assert torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0)) and torch.equal(a.isnan(), b.isnan())
+
+
+@pytest.mark.parametrize("B,Cin,H,W,Cout,k,stride,pad", [
+    (3, 64, 16, 16, 64, 3, 1, 1),       # three splits of the weight gradient
+    (1, 64, 8, 8, 128, 1, 1, 0),        # one: its sum is not split
+    (16, 64, 32, 32, 128, 3, 2, 1), (2, 3, 32, 32, 64, 3, 1, 1)])       # strided; a patch matrix
+def test_convolution_of_master_weights(B, Cin, H, W, Cout, k, stride, pad):
+    """fp32 weights as one node against a cast in front of the convolution: the same bits in y and dx, and a weight gradient that
+    is the other one before its rounding to bf16."""
+    geom = C.ConvGeom(B, H, W, Cin)
+    g = torch.Generator(device="cuda").manual_seed(B + Cin)
+    x = torch.randn(geom.rows, Cin, generator=g, device="cuda").to(BF)
+    w = C.pack_conv_weight(torch.randn(Cout, k * k * Cin, generator=g, device="cuda") * 0.1, Cin, k)
+    got = []
+    for master in (True, False):
+        xi, wi = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+        y, _ = C.conv2d_master(xi, wi, geom, k, stride, pad) if master else C.conv2d(xi, wi.to(BF), geom, k, stride, pad)
+        dy = torch.randn(y.shape, generator=torch.Generator(device="cuda").manual_seed(5), device="cuda").to(BF)
+        got.append([y.detach(), *torch.autograd.grad(y, (xi, wi), dy)])
+    _lib.check_status()
+    (y, dx, dw), want = got[0], got[1]
+    assert torch.equal(y, want[0]) and torch.equal(dx, want[1])
+    assert dw.dtype == torch.float32 and torch.equal(dw.to(BF).float(), want[2])
