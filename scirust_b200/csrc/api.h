@@ -113,6 +113,7 @@ int sb_swiglu_bwd(const void* gu, const void* dh, void* dgu, int rows, int ff, v
 int sb_add_bf16(const void* a, const void* b, void* out, size_t n, void* stream);
 int sb_embed_fwd(const void* table, const int64_t* tokens, void* out, int n, int d, int vocab, void* stream);
 int sb_embed_bwd(const void* dy, const int64_t* sorted_tok, const int64_t* perm, void* dtable, int n, int d, int vocab, int accumulate, void* stream);
+int sb_embed_bwd_tokens(const void* dy, const int64_t* tokens, int* scratch, void* dtable, int n, int d, int vocab, int accumulate, void* stream);
 int sb_ce_fwd_bwd(const void* logits, const int64_t* targets, float* loss_rows, void* dlogits, int rows, int cols, int ld, float grad_scale, void* stream);
 int sb_ce_shard_stats(const void* logits, const int64_t* targets, float* stats, int rows, int cols, int ld, int v0, void* stream);
 int sb_ce_shard_grad(const void* logits, const int64_t* targets, const float* lse, void* dlogits, int rows, int cols, int ld, int v0, float grad_scale, void* stream);

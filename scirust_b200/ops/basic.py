@@ -178,10 +178,11 @@ def embed_bwd(dy, tokens, dtable, accumulate=True):
         return dtable
     if not accumulate:
         dtable.zero_()
-    sorted_tok, perm = torch.sort(flat, stable=True)
-    _lib.call("sb_embed_bwd", dy.data_ptr(), sorted_tok.data_ptr(), perm.data_ptr(), dtable.data_ptr(), n, d,
-              vocab, 1, _lib.stream())
-    _count()
+    flat = flat.contiguous()
+    scratch = _lib.empty(vocab + n, torch.int32, dy.device)
+    _lib.call("sb_embed_bwd_tokens", dy.data_ptr(), flat.data_ptr(), scratch.data_ptr(), dtable.data_ptr(), n, d, vocab, 1,
+              _lib.stream())
+    _count(2)
     return dtable
 
 

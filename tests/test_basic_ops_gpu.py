@@ -81,6 +81,27 @@ def test_embedding_fwd_bwd_deterministic():
     _close(g1, ref, 2e-2)
 
 
+@pytest.mark.parametrize("n,V,d,repeat", [
+    (1, 1, 8, 0), (300, 7, 1032, 0),             # every chain longer than a warp ranks; a second slab of 8 columns
+    (2500, 4000, 64, 32), (2500, 4000, 64, 33),  # the longest ranked chain, the shortest that the tokens are read for
+    (2050, 50, 4096, 1500), (40, 1000, 2048, 2)])
+@pytest.mark.parametrize("accumulate", [True, False])
+def test_embedding_bwd_adds_in_ascending_order(n, V, d, repeat, accumulate):
+    """Rows of one token are added in fp32 in the order of their positions, whatever order the chains were built in: the same bits
+    as a loop. Ids outside the table count for its first and last row."""
+    tok = torch.randint(0, V, (n,), generator=torch.Generator().manual_seed(n))
+    if n > 4 and V > 7:
+        tok[tok == 3] = 4
+        tok[torch.randperm(n, generator=torch.Generator().manual_seed(1))[:repeat]] = 3
+        tok[1], tok[n - 1] = -5, V + 9
+    dy, base = _r((n, d), 11, 0.1), _r((V, d), 12, 0.1)
+    want = base.float() if accumulate else torch.zeros(V, d)
+    for i in range(n):
+        want[tok[i].clamp(0, V - 1)] += dy[i].float()
+    got = ops.embed_bwd(dy.cuda(), tok.cuda(), base.clone().cuda(), accumulate=accumulate)
+    assert torch.equal(got.cpu(), want.to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("rows,cols", [(64, 32000), (17, 1000), (9, 128256)])
 def test_cross_entropy(rows, cols):
     logits = _r((rows, cols), 13, 2.0)
