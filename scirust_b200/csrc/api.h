@@ -106,6 +106,7 @@ int sb_gemm_w8(const void* A, const void* Q, const float* scale, void* C, const 
 
 // kernels_basic.cu
 int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* inv_rms, int rows, int cols, int ldx, int ldy, float eps, void* stream);
+int sb_rmsnorm_bwd_both(const void* dy, const void* x, const void* w, const float* inv_rms, const void* dres, void* dx, float* partial, int parts, float* dw_f32, void* dw_bf16, int rows, int cols, void* stream);
 int sb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* inv_rms, const void* dres, void* dx, float* dw_partial, float* dw_f32, void* dw_bf16, int rows, int cols, void* stream);
 int sb_rope(void* x, int ld, int rows, int n_heads, int dh, int seq_len, int offset, const int* positions, const float* cos_t, const float* sin_t, int backward, void* stream);
 int sb_swiglu_fwd(const void* gu, void* h, int rows, int ff, void* stream);

@@ -295,6 +295,108 @@ __global__ void rmsnorm_bwd_dw_partial_kernel(const __nv_bfloat16* __restrict__ 
 }
 
 
+// Both gradients in one pass, for rows of NV * 256 columns (NV <= 4): dy and x are read once and not twice. A warp takes every
+// (warps of the grid)-th row, keeps the row in registers as above (the same dx bits) and adds its share of the gain's gradient to NV * 8
+// sums per lane; the warps of a CTA are added in warp order, the CTAs in stage 2. Two CTAs of eight warps per SM: 128 registers
+// hold the row and the sums, the gain lies in shared memory (with one CTA per SM this form lost to two passes). Bound by memory: 16384 x 1024
+// with a residual 21.4 + 14.4 + 4.3 us in two passes and their stage 2, 26.2 + 4.4 so; 999 x 1024 3.3 + 7.1 + 1.9 / 4.3 + 2.7.
+constexpr int RB_WARPS = 8;
+template <int NV, bool RES>
+__global__ void __launch_bounds__(RB_WARPS * 32, 2)
+rmsnorm_bwd_both_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ inv_rms,
+                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows) {
+  constexpr int cols = NV * 256;
+  __shared__ float red[RB_WARPS][cols];
+  __shared__ uint4 s_w[cols / 8];                        // the gain: in registers it would cost spills
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float acc[NV][8];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  }
+  if (threadIdx.x < cols / 8) s_w[threadIdx.x] = *reinterpret_cast<const uint4*>(w + threadIdx.x * 8);
+  __syncthreads();
+  for (int row = blockIdx.x * RB_WARPS + warp; row < rows; row += gridDim.x * RB_WARPS) {
+    const size_t off = static_cast<size_t>(row) * cols + lane * 8;
+    uint4 va[NV], vb[NV], vd[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      va[i] = *reinterpret_cast<const uint4*>(dy + off + i * 256);
+      vb[i] = *reinterpret_cast<const uint4*>(x + off + i * 256);
+      if (RES) vd[i] = *reinterpret_cast<const uint4*>(dres + off + i * 256);
+    }
+    const float r = inv_rms[row];
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      float a[8], b[8], g[8];
+      unpack8(va[i], a); unpack8(vb[i], b); unpack8(s_w[lane + i * 32], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        dot += a[j] * g[j] * b[j];
+        acc[i][j] += a[j] * b[j] * r;
+      }
+    }
+    dot = warp_sum(dot);
+    // the words are unpacked again below: kept as 64 floats across the sum they would spill
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      asm volatile("" : "+r"(va[i].x), "+r"(va[i].y), "+r"(va[i].z), "+r"(va[i].w));
+      asm volatile("" : "+r"(vb[i].x), "+r"(vb[i].y), "+r"(vb[i].z), "+r"(vb[i].w));
+    }
+    const float k = r * r * dot / static_cast<float>(cols);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      float a[8], b[8], g[8], o[8];
+      unpack8(va[i], a); unpack8(vb[i], b); unpack8(s_w[lane + i * 32], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = r * (a[j] * g[j] - b[j] * k);
+      if (RES) {
+        float d[8];
+        unpack8(vd[i], d);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] += d[j];
+      }
+      *reinterpret_cast<uint4*>(dx + off + i * 256) = pack8(o);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    *reinterpret_cast<float4*>(&red[warp][lane * 8 + i * 256]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    *reinterpret_cast<float4*>(&red[warp][lane * 8 + i * 256 + 4]) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < cols; c += RB_WARPS * 32) {
+    float s = red[0][c];
+#pragma unroll
+    for (int v = 1; v < RB_WARPS; ++v) s += red[v][c];
+    partial[static_cast<size_t>(blockIdx.x) * cols + c] = s;
+  }
+}
+
+// Stage 2 for many partial rows: 32 columns per CTA, 32 lanes of partials each (lane l adds l, l + 32, ... in order), lanes added in
+// order. A thread of colsum_finish_kernel walks all partials of its column: 64 x 1024 4.3 us, 296 x 1024 here 4.4.
+__global__ void __launch_bounds__(1024)
+colsum_finish_lanes_kernel(const float* __restrict__ partial, int parts, int cols, float* __restrict__ out_f32,
+                           __nv_bfloat16* __restrict__ out_bf16) {
+  __shared__ float s[32][33];
+  const int c = threadIdx.x & 31, l = threadIdx.x >> 5, col = blockIdx.x * 32 + c;
+  float v = 0.f;
+  if (col < cols) {
+#pragma unroll 10
+    for (int k = l; k < parts; k += 32) v += __ldg(partial + static_cast<size_t>(k) * cols + col);
+  }
+  s[l][c] = v;
+  __syncthreads();
+  if (l || col >= cols) return;
+#pragma unroll
+  for (int k = 1; k < 32; ++k) v += s[k][c];
+  if (out_f32) out_f32[col] = v;
+  if (out_bf16) out_bf16[col] = __float2bfloat16_rn(v);
+}
+
 // Generic fixed-order column sum finish: out[j] = sum_k partial[k][j] (k ascending);
 // writes fp32 and/or bf16.
 __global__ void colsum_finish_kernel(const float* __restrict__ partial, int chunks, int cols,
@@ -1075,10 +1177,25 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* inv_
   CHECK_LAUNCH();
 }
 
+// The two gradients in one pass: 512 or 1024 columns, `parts` CTAs (at most one per eight rows is used), partial of parts * cols floats.
+extern "C" int sb_rmsnorm_bwd_both(const void* dy, const void* x, const void* w, const float* inv_rms, const void* dres, void* dx,
+                                   float* partial, int parts, float* dw_f32, void* dw_bf16, int rows, int cols, void* stream) {
+  if (rows <= 0 || parts <= 0 || !partial || (cols != 512 && cols != 1024)) return SB_ERR_ARG;
+  if (!al16(dy) || !al16(x) || !al16(w) || !al16(dx) || (dres && !al16(dres))) return SB_ERR_ALIGN;
+  const int need = (rows + RB_WARPS - 1) / RB_WARPS;
+  if (parts > need) parts = need;
+  auto kern = cols == 1024 ? (dres ? rmsnorm_bwd_both_kernel<4, true> : rmsnorm_bwd_both_kernel<4, false>)
+                           : (dres ? rmsnorm_bwd_both_kernel<2, true> : rmsnorm_bwd_both_kernel<2, false>);
+  kern<<<parts, RB_WARPS * 32, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x),
+                                            static_cast<const __nv_bfloat16*>(w), inv_rms, static_cast<const __nv_bfloat16*>(dres),
+                                            static_cast<__nv_bfloat16*>(dx), partial, rows);
+  if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
+  colsum_finish_lanes_kernel<<<(cols + 31) / 32, 1024, 0, STREAM>>>(partial, parts, cols, dw_f32, static_cast<__nv_bfloat16*>(dw_bf16));
+  CHECK_LAUNCH();
+}
+
 // dw_partial: fp32 workspace of ceil(rows/rows_per_chunk)*cols floats; rows_per_chunk
-// is fixed at 256 so the summation tree depends only on (rows, cols). (A variant that produced dx and
-// the gain-gradient partials in one pass was measured slower: 83 + 20 us against 26 + 23 + 8 us at
-// 16384 x 1024, because its register footprint allowed one CTA per SM.)
+// is fixed at 256 so the summation tree depends only on (rows, cols).
 extern "C" int sb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* inv_rms, const void* dres,
                               void* dx, float* dw_partial, float* dw_f32, void* dw_bf16, int rows, int cols,
                               void* stream) {

@@ -33,6 +33,7 @@ _CUDA_SIGS = {
     "sb_gemm_pair_bf16": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp, i32, i32, vp, i32, vp, vp],
     "sb_rmsnorm_fwd": [vp, vp, vp, vp, i32, i32, i32, i32, f32, vp],
     "sb_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, vp],
+    "sb_rmsnorm_bwd_both": [vp, vp, vp, vp, vp, vp, vp, i32, vp, vp, i32, i32, vp],
     "sb_rope": [vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, i32, vp],
     "sb_swiglu_fwd": [vp, vp, i32, i32, vp],
     "sb_swiglu_bwd": [vp, vp, vp, i32, i32, vp],

@@ -62,8 +62,9 @@ def rmsnorm_bwd(dy, x, w, inv, dres=None, dw_out=None, want_dw=True):
     dy = dy.contiguous()
     dx = torch.empty_like(x)
     part = dwf = dwb = None
+    both = want_dw and cols in (512, 1024)      # one pass for both gradients, two CTAs per SM
     if want_dw:
-        chunks = (rows + 255) // 256
+        chunks = min((rows + 7) // 8, 2 * _g.num_sms(x.device)) if both else (rows + 255) // 256
         part = _lib.empty(chunks * cols, torch.float32, x.device)
         if dw_out is None:
             dw_out = _lib.empty(cols, torch.float32, x.device)
@@ -71,6 +72,11 @@ def rmsnorm_bwd(dy, x, w, inv, dres=None, dw_out=None, want_dw=True):
             dwf = dw_out
         else:
             dwb = dw_out
+    if both:
+        _lib.call("sb_rmsnorm_bwd_both", dy.data_ptr(), x.data_ptr(), w.data_ptr(), inv.data_ptr(), _lib.ptr(dres), dx.data_ptr(),
+                  part.data_ptr(), chunks, _lib.ptr(dwf), _lib.ptr(dwb), rows, cols, _lib.stream())
+        _count(2)
+        return dx, dw_out
     _lib.call("sb_rmsnorm_bwd", dy.data_ptr(), x.data_ptr(), w.data_ptr(), inv.data_ptr(), _lib.ptr(dres),
               dx.data_ptr(), _lib.ptr(part), _lib.ptr(dwf), _lib.ptr(dwb), rows, cols, _lib.stream())
     _count(3 if want_dw else 1)

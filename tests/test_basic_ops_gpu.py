@@ -36,6 +36,23 @@ def test_rmsnorm_fwd_bwd(rows, cols):
     assert torch.equal(dw, dw2) and torch.equal(dx, dx2)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 512), (9, 1024), (2368, 512), (2369, 1024), (5000, 1024)])
+@pytest.mark.parametrize("res,out", [(True, torch.float32), (False, torch.bfloat16), (True, torch.bfloat16)])
+def test_rmsnorm_bwd_in_one_pass(rows, cols, res, out):
+    """Both gradients from one pass (rows of 512 and 1024): a single row, a last CTA with one row, a grid that is exactly full and
+    one row more, several rows a warp. dx has one rounding to bf16 (2^-8) of terms of size one; dw sums rows fp32 terms."""
+    x, w, dy, dres = _r((rows, cols), 1), _r((cols,), 2), _r((rows, cols), 3), _r((rows, cols), 4)
+    inv = ops.rmsnorm_fwd(x, w)[1]
+    dx_ref, dw_ref = ops.rmsnorm_bwd(dy, x, w, inv, dres=dres if res else None)
+    dw_out = torch.full((cols,), float("nan"), dtype=out, device="cuda")
+    dx, dw = ops.rmsnorm_bwd(dy.cuda(), x.cuda(), w.cuda(), inv.cuda(), dres=dres.cuda() if res else None, dw_out=dw_out)
+    assert dw is dw_out
+    _close(dx, dx_ref, 2 ** -7)
+    terms = (dy.float() * x.float() * inv[:, None]).abs().sum(0).max().item()
+    lim = terms * (rows * 2.0 ** -24 if out == torch.float32 else 2.0 ** -8) + 1e-6
+    assert (dw.float().cpu() - dw_ref).abs().max().item() <= lim
+
+
 @pytest.mark.parametrize("dh", [64, 128])
 def test_rope_roundtrip_and_reference(dh):
     rows, heads, kv = 96, 4, 2
