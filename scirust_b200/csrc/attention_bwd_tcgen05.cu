@@ -85,33 +85,44 @@ __device__ __forceinline__ void bwd_chunk(uint32_t tm_S, uint32_t tm_dP, uint32_
   store_row32_sw128(ds_buf, r, c, dk);
 }
 
-// --------------------------------------------------------------------------- delta
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                  const float* __restrict__ lse, float2* __restrict__ stats, int B, int S, int H,
-                                  int dh, int ld_o, int ld_do) {
-  // a group of dh/8 lanes (8 or 16) owns one (token, head): 16-byte loads, then a butterfly inside the group
-  const int gl = dh >> 3;                       // lanes per group
-  const int gpw = 32 / gl;                      // groups per warp
-  const int lane = threadIdx.x & 31;
-  const int sub = lane % gl;
-  const long long w = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * gpw + lane / gl;
-  const bool live = w < static_cast<long long>(B) * S * H;
-  float acc = 0.f;
-  int row = 0, h = 0;
-  if (live) {
-    row = static_cast<int>(w / H);
-    h = static_cast<int>(w - static_cast<long long>(row) * H);
-    const uint4 a = *reinterpret_cast<const uint4*>(o + static_cast<size_t>(row) * ld_o + h * dh + sub * 8);
-    const uint4 g = *reinterpret_cast<const uint4*>(d_o + static_cast<size_t>(row) * ld_do + h * dh + sub * 8);
-    acc = bf16_lo(a.x) * bf16_lo(g.x) + bf16_hi(a.x) * bf16_hi(g.x) + bf16_lo(a.y) * bf16_lo(g.y) +
-          bf16_hi(a.y) * bf16_hi(g.y) + bf16_lo(a.z) * bf16_lo(g.z) + bf16_hi(a.z) * bf16_hi(g.z) +
-          bf16_lo(a.w) * bf16_lo(g.w) + bf16_hi(a.w) * bf16_hi(g.w);
+// Row statistics of the backward pass, (lse * log2(e), delta = rowsum(dO * O)) for every head and row. Bound by the bytes of O and dO: a
+// CTA takes eight rows x 512 columns, a row per warp; a group of dh/8 lanes (8 or 16) adds up its head in a butterfly, and
+// the results leave through shared memory, so that the statistics of a head, which lie S apart from the next head's, are read and
+// written eight rows at a time. With a group per (row, head), a 64-bit division each and scattered statistics 2 x 2048 x 32
+// heads of 128 took 19.7 us, 14.2 so (four rows a warp: 16.9); 8 x 2048 x 16 heads of 64 22.3 / 16.9.
+constexpr int DL_ROWS = 8, DL_COLS = 512;
+__global__ void __launch_bounds__(DL_ROWS * 32)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, const float* __restrict__ lse,
+                  float2* __restrict__ stats, int rows, int S, int H, int dh, int ld_o, int ld_do) {
+  __shared__ float s_delta[DL_COLS / 64][DL_ROWS + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gl = dh >> 3;
+  const int row0 = blockIdx.x * DL_ROWS, col0 = blockIdx.y * DL_COLS, cols = H * dh;
+  uint4 a[2], g[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int c = col0 + i * 256 + lane * 8;
+    a[i] = g[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (row0 + warp < rows && c < cols) {
+      a[i] = __ldg(reinterpret_cast<const uint4*>(o + static_cast<size_t>(row0 + warp) * ld_o + c));
+      g[i] = __ldg(reinterpret_cast<const uint4*>(d_o + static_cast<size_t>(row0 + warp) * ld_do + c));
+    }
   }
-  for (int o2 = gl >> 1; o2 > 0; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
-  if (live && sub == 0) {
-    const int b = row / S, s = row - b * S;
-    const size_t idx = (static_cast<size_t>(b) * H + h) * S + s;
-    stats[idx] = make_float2(lse[idx] * LOG2E, acc);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint4 x = a[i], y = g[i];
+    float acc = bf16_lo(x.x) * bf16_lo(y.x) + bf16_hi(x.x) * bf16_hi(y.x) + bf16_lo(x.y) * bf16_lo(y.y) +
+                bf16_hi(x.y) * bf16_hi(y.y) + bf16_lo(x.z) * bf16_lo(y.z) + bf16_hi(x.z) * bf16_hi(y.z) +
+                bf16_lo(x.w) * bf16_lo(y.w) + bf16_hi(x.w) * bf16_hi(y.w);
+    for (int off = gl >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (lane % gl == 0) s_delta[(i * 256 + lane * 8) / dh][warp] = acc;
+  }
+  __syncthreads();
+  const int hl = threadIdx.x / DL_ROWS, rl = threadIdx.x % DL_ROWS;     // head of this slab, row of this CTA
+  const int h = col0 / dh + hl, row = row0 + rl;
+  if (hl < DL_COLS / dh && h < H && row < rows) {
+    const int b = row / S;
+    const size_t idx = (static_cast<size_t>(b) * H + h) * S + (row - b * S);
+    stats[idx] = make_float2(lse[idx] * LOG2E, s_delta[hl][rl]);
   }
 }
 
@@ -1064,13 +1075,9 @@ extern "C" int sb_attention_bwd(const void* qkv, const void* O, const float* lse
   if (rc) return rc;
   if ((ld_o & 7) || (ld_do & 7) || (reinterpret_cast<uintptr_t>(O) & 15) || (reinterpret_cast<uintptr_t>(dO) & 15))
     return SB_ERR_ALIGN;
-  const long long groups = static_cast<long long>(B) * S * H;
-  const int gpw = 32 / (dh / 8);
-  const long long warps = (groups + gpw - 1) / gpw;
-  attn_delta_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(O),
-                                                         static_cast<const __nv_bfloat16*>(dO), lse,
-                                                         reinterpret_cast<float2*>(delta), B, S, H, dh, ld_o,
-                                                         ld_do);
+  attn_delta_kernel<<<dim3((B * S + DL_ROWS - 1) / DL_ROWS, (H * dh + DL_COLS - 1) / DL_COLS), DL_ROWS * 32, 0, stream>>>(
+      static_cast<const __nv_bfloat16*>(O), static_cast<const __nv_bfloat16*>(dO), lse, reinterpret_cast<float2*>(delta), B * S, S, H,
+      dh, ld_o, ld_do);
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   BwdParams p;
   p.B = B; p.S = S; p.H = H; p.Hkv = Hkv;

@@ -1,8 +1,7 @@
 // GQA flash-attention forward for sm_100a, head dimensions 64 and 128, two query tiles per CTA.
 //
 // One CTA owns 256 query rows of one (head, batch) as two 128-row tiles. Each tile has its own
-// score accumulator S_t and output accumulator O_t in tensor memory and its own group of four
-// softmax warps, so while the warps of one tile run their exponentials the tensor cores work on
+// output accumulator O_t in tensor memory and its own group of four softmax warps, so while the warps of one tile run their exponentials the tensor cores work on
 // the other tile's products. The output accumulator stays in tensor memory for the whole loop:
 // P V is accumulated there by the MMA itself, and a row is rescaled when its running maximum has grown
 // since the reference point used in the exponent: at head dimension 64 by more than 2^8 (bf16 P then
@@ -21,28 +20,30 @@
 //
 // A softmax thread holds its whole 128-column score row in registers (one pass over tensor memory),
 // scales it with packed fp32 pairs (fma.rn.f32x2, add.rn.f32x2: half the issue slots of scalar
-// code) and takes the row maximum with three-input max. What bounds the kernel is the chain inside a tile: scores, maximum,
-// exponentials, P, P V. Two softmax warps share a scheduler, so the special-function unit needs 1024 cycles for a block of
-// both tiles, and so does the tensor pipe at head dimension 128; a block takes about twice that, and each of the two is
-// busy half of the time (profiles/attention_issue_and_softmax.md). Nothing else may lengthen the chain:
-//  - Every tile has an issuing warp of its own, and the scores of block j+1 are issued as soon as those of block j
-//    are in registers, so they are there when block j is done. With one issuer for both tiles the waits of one
-//    tile held up the other.
-//  - An issuing warp walks through its loop as a whole and one lane issues: descriptors and addresses stay in uniform
+// code) and takes the row maximum with three-input max. What bounds the kernel is the chain inside a tile (scores, maximum, rescale,
+// exponentials, P, P V) and, in a long run, the power cap: 5000 tokens of 32 heads of 128 run at 1.96 GHz for a few
+// milliseconds and at 1.75 after that. Two softmax warps share a scheduler, so the special-function unit needs 2048 cycles for a
+// block of both tiles, and so does the tensor pipe at head dimension 128; a block takes about 3300 (2800 at 64; 3500 with P in
+// shared memory; profiles/attention_issue_and_softmax.md).
+//  - P goes to tensor memory, from where the tensor core takes it as its A operand. A product with both operands in shared memory reads
+//    8 KB in the 64 cycles that it runs, all that shared memory gives; with P there too, its stores, the products and the tiles
+//    that arrive asked shared memory for 3000 cycles a block. Its two halves of 64 columns are handed over one by one.
+//  - At head dimension 128 tensor memory is full with one score accumulator (128 columns), P (2 x 64) and O (2 x 128): the tiles take
+//    turns with the accumulator, which is free again when a tile has its scores in registers, and so run half a block
+//    apart, one in its exponentials while the other waits, loads and rescales. At 64 each has its own.
+//  - One warp issues for both tiles in the order S0(j) PV0(j-1) S1(j) PV1(j-1), in which they come up: the scores of a block are there
+//    when the block before is done.
+//  - The issuing warp walks through its loop as a whole and one lane issues: descriptors and addresses stay in uniform
 //    registers. As the loop of a single thread a product cost it 70 to 150 cycles to issue, more than to run.
-//  - The exponentials, their sum and their bf16 pairs come before the wait for the previous P V, which runs meanwhile.
 //  - The mask is applied to the scores of the blocks that need one; as a select beside every exponential it
 //    cost all blocks a third of their instructions.
 // The softmax warpgroups take the registers that the issuing one does not need (setmaxnreg), so rows stay unspilled.
-// us before all this / now, causal, 32 heads of 128, calls back to back on one input: 5000 tokens 262 / 206 (990 TFLOP/s; 237 and
-// 860 for a call among others on new inputs), 4096 185 / 154, 2 x 2048 112 / 96; 16 heads of 64: 8 x 2048 160 / 150.
+// us with P in shared memory and an issuing warp per tile / now, causal, calls back to back on one input, 32 heads of 128: 5000 tokens
+// 211 / 198 (1033 TFLOP/s; in a long run on new inputs 238 / 224), 4096 146 / 134, 2 x 2048 93 / 85; 16 heads of 64: 8 x 2048 140 / 128,
+// 2 x 2048 40.5 / 37.4; the same bits. Measured and dropped: the rescale in four warps of its own (5000 tokens 222: the softmax
+// warps wait longer for one another than for the rescale), two warps a row (212), exponentials of the tiles in strict turns (level).
 //
-// Head dimension 128: Q (64 KB), two P tiles (64 KB) and a K tile of 32 KB twice leave 32 KB for V. K gets two whole
-// stages; V is a ring of two half tiles of 64 kv rows, because the products consume V row by row: the first half is
-// free again before the second tile's P V ends, and its successor lands while the next scores run. With three
-// whole-tile slots for K and V together, every block would wait about a load latency for its K.
-//
-// Warps: 0 TMA producer, 1 and 2 MMA issuers of tiles 0 and 1, 3 idle, 4-7 softmax of tile 0, 8-11 softmax of tile 1.
+// Warps: 0 TMA producer, 1 MMA issuer, 2 and 3 idle, 4-7 softmax of tile 0, 8-11 softmax of tile 1.
 #include "sm100_ptx.cuh"
 #include "api.h"
 #include "per_device.h"
@@ -57,26 +58,26 @@ namespace attpp {
 constexpr int BM = 128;        // query rows per tile
 constexpr int BN = 128;        // kv rows per block
 constexpr int THREADS = 384;
-// Registers a thread: 168 at launch for all three warpgroups, shared out as 56 (producer, issuers) + 2 x 224 (softmax).
+// Registers a thread: 168 at launch for all three warpgroups, shared out as 56 (producer, issuer) + 2 x 224 (softmax).
 constexpr int REGS_ISSUE = 56, REGS_SOFTMAX = 224;
 static_assert(REGS_ISSUE + 2 * REGS_SOFTMAX <= 3 * 168, "the shares draw on the registers of the launch");
-constexpr int P_BYTES = BM * BN * 2;
-constexpr int TMEM_COLS = 512;  // S0 [0,128) S1 [128,256) O0 [256,256+DH) O1 [256+DH,256+2DH)
+constexpr int HALF = BN / 2;   // columns of P that are handed over at once
+constexpr int TMEM_COLS = 512;
 
 template <int DH>
 struct Cfg {
   static constexpr int NCH = DH / 64;                  // 64-column chunks per head
-  static constexpr int KS = DH == 64 ? 3 : 2;          // K ring stages (whole tiles)
-  static constexpr int VP = DH == 64 ? 1 : 2;          // pieces per V tile
-  static constexpr int VROWS = BN / VP;                // kv rows per piece
-  static constexpr int VS = DH == 64 ? 3 : 2;          // V ring stages (pieces)
+  static constexpr int KS = 3;                         // K ring stages
+  static constexpr int VS = DH == 64 ? 3 : 2;          // V ring stages
   static constexpr int Q_BYTES = BM * DH * 2;
-  static constexpr int K_BYTES = BN * DH * 2;
-  static constexpr int V_BYTES = VROWS * DH * 2;
-  static constexpr int TILE_BYTES = 2 * Q_BYTES + KS * K_BYTES + VS * V_BYTES + 2 * P_BYTES;
-  static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 256;
+  static constexpr int KV_BYTES = BN * DH * 2;
+  static constexpr int TILE_BYTES = 2 * Q_BYTES + (KS + VS) * KV_BYTES;
+  static constexpr int SMEM_BYTES = TILE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
-  static_assert(2 * BN + 2 * DH <= TMEM_COLS, "tensor memory");
+  // tensor memory: score accumulators (one that the tiles take turns with at 128, one each at 64), P as bf16 pairs, O
+  static constexpr int SB = DH == 64 ? 2 : 1;
+  static constexpr int COL_P = SB * BN, COL_O = COL_P + 2 * (BN / 2);
+  static_assert(COL_O + 2 * DH <= TMEM_COLS, "tensor memory");
   static constexpr float RESCALE_GAP = DH == 64 ? 8.f : 0.f;   // log2 of the growth that a reference may lag behind
 };
 
@@ -103,27 +104,25 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 
 template <int DH>
 __global__ void __launch_bounds__(THREADS, 1)
-attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_v,
-                        const Params p) {
+attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const Params p) {
   using C = Cfg<DH>;
   constexpr int KS = C::KS, VS = C::VS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + 2 * C::Q_BYTES;
-  uint8_t* sV = sK + KS * C::K_BYTES;
-  uint8_t* sP = sV + VS * C::V_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + 2 * P_BYTES);
+  uint8_t* sV = sK + KS * C::KV_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + VS * C::KV_BYTES);
   uint64_t* q_full = bars;               // [2]
   uint64_t* k_full = q_full + 2;         // [KS]
   uint64_t* k_empty = k_full + KS;
   uint64_t* v_full = k_empty + KS;       // [VS]
   uint64_t* v_empty = v_full + VS;
   uint64_t* s_full = v_empty + VS;       // [2] scores of tile t are in tensor memory
-  uint64_t* p_full = s_full + 2;         // [2] P of tile t is in shared memory (4 warp arrivals)
-  uint64_t* pv_done = p_full + 2;        // [2] P V of tile t has completed
-  uint64_t* s_free = pv_done + 2;        // [2] scores of tile t are in registers (4 warp arrivals)
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(s_free + 2);
+  uint64_t* s_free = s_full + 2;         // [SB] the scores that lay in this accumulator are in registers (4 warp arrivals)
+  uint64_t* p_full = s_free + 2;         // [2][2] a half of P of tile t is in tensor memory, O is rescaled (4 warp arrivals)
+  uint64_t* pv_done = p_full + 4;        // [2] P V of tile t has completed
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(pv_done + 2);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_pairs = (p.S + 2 * BM - 1) / (2 * BM);
@@ -148,16 +147,17 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
     for (int t = 0; t < 2; ++t) {
       mbar_init(&q_full[t], 1);
       mbar_init(&s_full[t], 1);
-      mbar_init(&p_full[t], 4);
-      mbar_init(&pv_done[t], 1);
       mbar_init(&s_free[t], 4);
+      mbar_init(&p_full[2 * t], 4);
+      mbar_init(&p_full[2 * t + 1], 4);
+      mbar_init(&pv_done[t], 1);
     }
-    for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 2); }   // one arrival per issuer
-    for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 2); }
+    for (int s = 0; s < KS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
+    for (int s = 0; s < VS; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
     fence_barrier_init();
     fence_proxy_async_smem();
   }
-  if (warp == 0 && lane == 0) { prefetch_tmap(&tmap); prefetch_tmap(&tmap_v); }
+  if (warp == 0 && lane == 0) prefetch_tmap(&tmap);
   if (warp == 1) {
     tmem_alloc(tmem_holder, TMEM_COLS);
     tmem_relinquish();
@@ -184,93 +184,92 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
       uint32_t kph = 0, vph = 0;
       auto load_k = [&](int j) -> bool {
         if (!mbar_wait(&k_empty[ks], kph ^ 1, p.status, ST_TIMEOUT_EMPTY)) return false;
-        mbar_arrive_expect_tx(&k_full[ks], C::K_BYTES);
+        mbar_arrive_expect_tx(&k_full[ks], C::KV_BYTES);
 #pragma unroll
         for (int c = 0; c < C::NCH; ++c)
-          tma_load_2d(sK + ks * C::K_BYTES + c * (BN * 128), &tmap, &k_full[ks], col_k + c * 64, row_base + j * BN);
+          tma_load_2d(sK + ks * C::KV_BYTES + c * (BN * 128), &tmap, &k_full[ks], col_k + c * 64, row_base + j * BN);
         if (++ks == KS) { ks = 0; kph ^= 1; }
         return true;
       };
       auto load_v = [&](int j) -> bool {
+        if (!mbar_wait(&v_empty[vs], vph ^ 1, p.status, ST_TIMEOUT_EMPTY)) return false;
+        mbar_arrive_expect_tx(&v_full[vs], C::KV_BYTES);
 #pragma unroll
-        for (int h = 0; h < C::VP; ++h) {
-          if (!mbar_wait(&v_empty[vs], vph ^ 1, p.status, ST_TIMEOUT_EMPTY)) return false;
-          mbar_arrive_expect_tx(&v_full[vs], C::V_BYTES);
-#pragma unroll
-          for (int c = 0; c < C::NCH; ++c)
-            tma_load_2d(sV + vs * C::V_BYTES + c * (C::VROWS * 128), &tmap_v, &v_full[vs], col_v + c * 64,
-                        row_base + j * BN + h * C::VROWS);
-          if (++vs == VS) { vs = 0; vph ^= 1; }
-        }
+        for (int c = 0; c < C::NCH; ++c)
+          tma_load_2d(sV + vs * C::KV_BYTES + c * (BN * 128), &tmap, &v_full[vs], col_v + c * 64, row_base + j * BN);
+        if (++vs == VS) { vs = 0; vph ^= 1; }
         return true;
       };
-      // two K stages: the consumer frees K of block j + 1 before V of block j (its scores come first), so loads go in that
-      // order; with three the first V need not wait for the second K
-      constexpr int AHEAD = KS == 2 ? 1 : 0;
-      bool ok = n_blocks == 0 || AHEAD == 0 || load_k(0);
+      // the consumer frees K of block j + 1 before V of block j (its scores come first), so loads go in that order
+      bool ok = n_blocks == 0 || load_k(0);
       for (int j = 0; j < n_blocks && ok; ++j) {
-        if (j + AHEAD < n_blocks) ok = load_k(j + AHEAD);
+        if (j + 1 < n_blocks) ok = load_k(j + 1);
         ok = ok && load_v(j);
       }
     }
-  } else if (warp == 1 || warp == 2) {
-    // ------------------------------------- MMA issuers -------------------------------------
-    {
-      // The whole warp walks through the loop, so that descriptors and addresses stay in uniform registers; one lane issues.
-      const bool leader = elect_one();
-      const int t = warp - 1;
-      const int n_t = nb[t];
-      constexpr uint32_t idesc_s = make_idesc_bf16(BM, BN, false, false);
-      constexpr uint32_t idesc_o = make_idesc_bf16(BM, DH, false, true);
-      const uint64_t dq = make_smem_desc(smem_u32(sQ + t * C::Q_BYTES), 16, 1024);
-      const uint64_t dp = make_smem_desc(smem_u32(sP + t * P_BYTES), 16, 1024);
-      int ks = 0, vs = 0;
-      uint32_t kph = 0, vph = 0;
-      bool ok = n_t == 0 || mbar_wait_warp(&q_full[t], 0, p.status, ST_TIMEOUT_FULL);
-      // Blocks that only the other tile sees are waited for and released all the same: a ring slot is free when both
-      // issuers have let go of it.
-      for (int j = 0; j <= n_blocks && ok; ++j) {
-        if (j < n_blocks) {                            // S = Q K^T of block j, as soon as the scores of j - 1 are in registers
-          if (!mbar_wait_warp(&k_full[ks], kph, p.status, ST_TIMEOUT_FULL)) break;
-          if (j < n_t) {
-            if (j > 0 && !mbar_wait_warp(&s_free[t], (j - 1) & 1, p.status, ST_TIMEOUT_TMEM_EMPTY)) break;
-            tc_fence_after();
-            const uint64_t dk = make_smem_desc(smem_u32(sK + ks * C::K_BYTES), 16, 1024);
+  } else if (warp == 1) {
+    // ------------------------------------- MMA issuer -------------------------------------
+    // The whole warp walks through the loop, so that descriptors and addresses stay in uniform registers; one lane issues. The
+    // order is S0(j) PV0(j-1) S1(j) PV1(j-1) S0(j+1) ..., which is the order in which the tiles, half a block apart, need them.
+    const bool leader = elect_one();
+    constexpr uint32_t idesc_s = make_idesc_bf16(BM, BN, false, false);
+    constexpr uint32_t idesc_o = make_idesc_bf16(BM, DH, false, true);
+    int ks = 0, vs = 0, n_scores = 0;
+    uint32_t kph = 0, vph = 0;
+    bool ok = true;
+    for (int t = 0; t < 2; ++t) ok = ok && (nb[t] == 0 || mbar_wait_warp(&q_full[t], 0, p.status, ST_TIMEOUT_FULL));
+    for (int j = 0; j <= n_blocks && ok; ++j) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (ok && j < nb[t]) {                         // S = Q K^T of block j
+          if (t == 0 || j >= nb[0]) ok = mbar_wait_warp(&k_full[ks], kph, p.status, ST_TIMEOUT_FULL);
+          // the scores before these in the same accumulator are in registers
+          if (C::SB == 2) ok = ok && (j == 0 || mbar_wait_warp(&s_free[t], (j - 1) & 1, p.status, ST_TIMEOUT_TMEM_EMPTY));
+          else ok = ok && (n_scores == 0 || mbar_wait_warp(&s_free[0], (n_scores - 1) & 1, p.status, ST_TIMEOUT_TMEM_EMPTY));
+          if (!ok) break;
+          ++n_scores;
+          tc_fence_after();
+          const uint64_t dq = make_smem_desc(smem_u32(sQ + t * C::Q_BYTES), 16, 1024);
+          const uint64_t dk = make_smem_desc(smem_u32(sK + ks * C::KV_BYTES), 16, 1024);
+          if (leader) {
 #pragma unroll
             for (int k = 0; k < DH / 16; ++k) {
               const uint32_t off = (k >> 2) * (BM * 128) + (k & 3) * 32;
-              if (leader) umma_bf16_ss(tmem_base + t * BN, smem_desc_at(dq, off), smem_desc_at(dk, off),
-                           idesc_s, k > 0 ? 1u : 0u);
+              umma_bf16_ss(tmem_base + (C::SB == 2 ? t * BN : 0), smem_desc_at(dq, off), smem_desc_at(dk, off), idesc_s,
+                           k > 0 ? 1u : 0u);
             }
-            if (leader) umma_commit(&s_full[t]);
-            if (leader) umma_commit(&k_empty[ks]);
-          } else {
-            if (leader) mbar_arrive(&k_empty[ks]);
+            umma_commit(&s_full[t]);
+            if (t == 1 || j >= nb[1]) umma_commit(&k_empty[ks]);
           }
-          if (++ks == KS) { ks = 0; kph ^= 1; }
+          if (t == 1 || j >= nb[1]) {
+            if (++ks == KS) { ks = 0; kph ^= 1; }
+          }
         }
-        if (j > 0) {                                   // O (+)= P V of block j - 1
+        if (ok && j > 0 && j - 1 < nb[t]) {            // O (+)= P V of block j - 1
           const int i = j - 1;
+          if (t == 0 || i >= nb[0]) ok = mbar_wait_warp(&v_full[vs], vph, p.status, ST_TIMEOUT_FULL);
 #pragma unroll
-          for (int h = 0; h < C::VP && ok; ++h) {
-            ok = mbar_wait_warp(&v_full[vs], vph, p.status, ST_TIMEOUT_FULL);
-            if (ok && i < n_t) {
-              if (h == 0) ok = mbar_wait_warp(&p_full[t], i & 1, p.status, ST_TIMEOUT_MISC);
-              if (!ok) break;
-              tc_fence_after();
-              const uint64_t dv = make_smem_desc(smem_u32(sV + vs * C::V_BYTES), C::VROWS * 128, 1024);
+          for (int h = 0; h < 2; ++h) {
+            ok = ok && mbar_wait_warp(&p_full[2 * t + h], i & 1, p.status, ST_TIMEOUT_MISC);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t dv = make_smem_desc(smem_u32(sV + vs * C::KV_BYTES), BN * 128, 1024);
+            if (leader) {
 #pragma unroll
-              for (int k2 = 0; k2 < C::VROWS / 16; ++k2) {
-                const int k = h * (C::VROWS / 16) + k2;
-                if (leader)
-                  umma_bf16_ss(tmem_base + 2 * BN + t * DH, smem_desc_at(dp, (k >> 2) * (BM * 128) + (k & 3) * 32),
-                               smem_desc_at(dv, k2 * (16 * 128)), idesc_o, (i > 0 || k > 0) ? 1u : 0u);
+              for (int k2 = 0; k2 < HALF / 16; ++k2) {
+                const int k = h * (HALF / 16) + k2;
+                umma_bf16_ts(tmem_base + C::COL_O + t * DH, tmem_base + C::COL_P + t * (BN / 2) + k * 8,
+                             smem_desc_at(dv, k * (16 * 128)), idesc_o, (i > 0 || k > 0) ? 1u : 0u);
               }
-              if (h == C::VP - 1 && leader) umma_commit(&pv_done[t]);
-              if (leader) umma_commit(&v_empty[vs]);
-            } else if (ok) {
-              if (leader) mbar_arrive(&v_empty[vs]);
             }
+          }
+          if (!ok) break;
+          const bool last = t == 1 || i >= nb[1];
+          if (leader) {
+            umma_commit(&pv_done[t]);
+            if (last) umma_commit(&v_empty[vs]);
+          }
+          if (last) {
             if (++vs == VS) { vs = 0; vph ^= 1; }
           }
         }
@@ -285,9 +284,9 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
     const int r = q * 32 + lane;       // row inside the tile == TMEM lane
     const int q_idx = q0 + t * BM + r; // position inside the sequence
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    const uint32_t tm_S = tmem_base + t * BN + lane_off;
-    const uint32_t tm_O = tmem_base + 2 * BN + t * DH + lane_off;
-    uint8_t* sPt = sP + t * P_BYTES;
+    const uint32_t tm_S = tmem_base + (C::SB == 2 ? t * BN : 0) + lane_off;
+    const uint32_t tm_P = tmem_base + C::COL_P + t * (BN / 2) + lane_off;
+    const uint32_t tm_O = tmem_base + C::COL_O + t * DH + lane_off;
     const float sl2 = p.scale_log2;
     constexpr float NEG = -1.0e30f;
     float m_ref = NEG, l = 0.f;
@@ -295,15 +294,16 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
     for (int j = 0; j < n_t; ++j) {
       // Waits in this loop may give up (the status word says so) but do not end it: lanes that left it one by one would be
       // missing at the warp barriers below. Leaving as a whole takes a vote for each wait: 5000 tokens of 32 heads 208 us, 214 with it.
-      mbar_wait(&s_full[t], j & 1, p.status, ST_TIMEOUT_TMEM_FULL);
+      mbar_wait_converged(&s_full[t], j & 1, p.status, ST_TIMEOUT_TMEM_FULL);
       tc_fence_after();
       uint32_t v[BN];
+      __syncwarp();
 #pragma unroll
       for (int c = 0; c < BN / 32; ++c) tmem_ld_32x32_converged(tm_S + c * 32, v + c * 32);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s_free[t]);
+      if (lane == 0) mbar_arrive(&s_free[C::SB == 2 ? t : 0]);
       const int kv0 = j * BN;
       const bool need_mask = (p.causal && j == n_t - 1) || (kv0 + BN > p.S);
       const int lim = (p.causal ? min(q_idx, p.S - 1) : (p.S - 1)) - kv0;   // last visible column
@@ -324,26 +324,12 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
       const bool grow = m_blk > m_ref + C::RESCALE_GAP;   // always true in the first block
       const float alpha = grow ? ex2(m_ref - m_blk) : 1.f;
       if (grow) m_ref = m_blk;
-      // exponentials and their bf16 pairs, all in registers: P V of the previous block runs meanwhile
       const float neg_m = -m_ref;
-      float sum4[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      uint32_t pk[BN / 2];
-#pragma unroll
-      for (int i = 0; i < BN; i += 2) {
-        fma2(v[i], v[i + 1], sl2, neg_m);
-        const float e0 = ex2(__uint_as_float(v[i]));
-        const float e1 = ex2(__uint_as_float(v[i + 1]));
-        add2(sum4[i & 6], sum4[(i & 6) + 1], __float_as_uint(e0), __float_as_uint(e1));
-        pk[i >> 1] = pack_bf16x2(e0, e1);
-      }
-      // Roundings are spelt out here and in the log-sum-exp: left to the compiler, what it contracts changes with the code around it.
-      const float row_sum = ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) + ((sum4[4] + sum4[5]) + (sum4[6] + sum4[7]));
-      l = __fadd_rn(__fmul_rn(l, alpha), row_sum);
       if (j > 0) {
-        // P V of the previous block has read the P tile and updated O
-        mbar_wait(&pv_done[t], (j - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL);
+        // P V of the previous block has read P and updated O
+        mbar_wait_converged(&pv_done[t], (j - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL);
+        tc_fence_after();
         if (__any_sync(0xffffffffu, grow)) {
-          tc_fence_after();
 #pragma unroll
           for (int c = 0; c < DH / 32; ++c) {
             uint32_t o[32];
@@ -353,18 +339,31 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
             for (int i = 0; i < 32; i += 2) mul2(o[i], o[i + 1], alpha, alpha);
             tmem_st_32x32_converged(tm_O + c * 32, o);
           }
-          tmem_st_wait();
         }
       }
+      float sum4[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int c = 0; c < BN / 8; ++c) {               // 16-byte units of the swizzled row
-        uint8_t* prow = sPt + (c >> 3) * (BM * 128) + r * 128;
-        *reinterpret_cast<uint4*>(prow + (((c & 7) ^ (r & 7)) * 16)) = make_uint4(pk[c * 4], pk[c * 4 + 1], pk[c * 4 + 2], pk[c * 4 + 3]);
+      for (int h = 0; h < 2; ++h) {
+        // exponentials of half a row and their bf16 pairs
+        uint32_t pk[HALF / 2];
+#pragma unroll
+        for (int i2 = 0; i2 < HALF; i2 += 2) {
+          const int i = h * HALF + i2;
+          fma2(v[i], v[i + 1], sl2, neg_m);
+          const float e0 = ex2(__uint_as_float(v[i]));
+          const float e1 = ex2(__uint_as_float(v[i + 1]));
+          add2(sum4[i & 6], sum4[(i & 6) + 1], __float_as_uint(e0), __float_as_uint(e1));
+          pk[i2 >> 1] = pack_bf16x2(e0, e1);
+        }
+        tmem_st_32x32(tm_P + h * (HALF / 2), pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[2 * t + h]);
       }
-      tc_fence_before();
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[t]);
+      // Roundings are spelt out here and in the log-sum-exp: left to the compiler, what it contracts changes with the code around it.
+      const float row_sum = ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3])) + ((sum4[4] + sum4[5]) + (sum4[6] + sum4[7]));
+      l = __fadd_rn(__fmul_rn(l, alpha), row_sum);
     }
     if (n_t > 0 && mbar_wait_warp(&pv_done[t], (n_t - 1) & 1, p.status, ST_TIMEOUT_TMEM_FULL)) {
       tc_fence_after();
@@ -404,12 +403,12 @@ attention_fwd_pp_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_c
 }
 
 template <int DH>
-static int launch(const CUtensorMap& tm, const CUtensorMap& tv, const Params& p, cudaStream_t stream) {
+static int launch(const CUtensorMap& tm, const Params& p, cudaStream_t stream) {
   auto kern = attention_fwd_pp_kernel<DH>;
   static PerDeviceOnce attr;
   if (allow_smem(attr, kern, Cfg<DH>::SMEM_BYTES, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
   dim3 grid(p.H, p.B, (p.S + 2 * BM - 1) / (2 * BM));
-  kern<<<grid, THREADS, Cfg<DH>::SMEM_BYTES, stream>>>(tm, tv, p);
+  kern<<<grid, THREADS, Cfg<DH>::SMEM_BYTES, stream>>>(tm, p);
   return cudaGetLastError() == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
@@ -428,15 +427,9 @@ extern "C" int sb_attention_fwd_pp(const void* qkv, void* O, float* lse, int B, 
   if (B <= 0 || S <= 0 || H <= 0 || Hkv <= 0 || (H % Hkv) || (dh != 64 && dh != 128)) return SB_ERR_ARG;
   if (B > 65535 || (S + 127) / 128 > 65535) return SB_ERR_TOO_LARGE;   // grid y / z limits
   if ((ld_o & 7) || (reinterpret_cast<uintptr_t>(O) & 15)) return SB_ERR_ALIGN;
-  CUtensorMap tm, tv;
+  CUtensorMap tm;
   int rc = make_tmap_2d_bf16(&tm, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(B) * S, ld, 64, 128);
   if (rc) return rc;
-  tv = tm;
-  if (dh == 128) {
-    rc = make_tmap_2d_bf16(&tv, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(B) * S, ld, 64,
-                           attpp::Cfg<128>::VROWS);
-    if (rc) return rc;
-  }
   attpp::Params p;
   p.B = B; p.S = S; p.H = H; p.Hkv = Hkv;
   p.ld_o = ld_o;
@@ -446,5 +439,5 @@ extern "C" int sb_attention_fwd_pp(const void* qkv, void* O, float* lse, int B, 
   p.lse = lse;
   p.status = status;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  return dh == 64 ? attpp::launch<64>(tm, tv, p, stream) : attpp::launch<128>(tm, tv, p, stream);
+  return dh == 64 ? attpp::launch<64>(tm, p, stream) : attpp::launch<128>(tm, p, stream);
 }
