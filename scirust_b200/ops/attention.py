@@ -28,30 +28,34 @@ FWD_TWO_TILES = os.environ.get("SB_ATT_FWD", "pair") != "single"
 
 
 def _two_tiles_win(B, S, H, dh, causal, device) -> bool:
-    """Which of the two kernels runs, by the CTAs that each of them starts.
+    """Which of the two kernels runs, by the CTAs that each of them starts (us below: one tile / two, in a graph on one input).
 
-    Head dimension 128 (one CTA per SM in both): a CTA of two tiles took about 1.7 times as long as one of a single
-    tile when these lines were drawn, so while its grid fits the GPU at once one tile runs, and beyond that two must save
-    waves: sequences of up to 256 rows need more than 1.5 times fewer, up to 384 (the second CTA of a head has one tile)
-    1.5 times, longer ones always do. The two-tile kernel has become the faster by more since, and the lines lie too far
-    out by up to a third. Causal, 32 heads, us, one tile / two: taken as two 1 x 1300 43.0 / 29.2, 2 x 1000 49.2 / 32.8,
-    9 x 256 28.9 / 20.8; as one 1 x 128 6.5 / 6.7, 2 x 256 8.9 / 10.3, 3 x 333 17.4 / 18.7, and, where two would be faster,
-    1 x 1000 25.1 / 23.4, 2 x 512 18.9 / 15.3, 4 x 256 15.0 / 11.0, 5 x 333 30.1 / 27.6, 12 x 333 63.1 / 53.3.
+    Head dimension 128, one CTA per SM in both: a CTA of two tiles takes little longer than one of a single tile, so two win
+    wherever they save a wave, and without the mask beyond seven tiles anyway. 32 heads, no mask: 1 x 333 11.0 / 12.3, 1 x 512
+    13.3 / 13.9, but 4 x 256 16.6 / 10.8, 2 x 512 25.4 / 14.5, 1 x 1000 42.1 / 22.6. Causal, up to 256 rows they need more than 1.5
+    times fewer waves, up to 384 (the second CTA of a head has one tile) 1.5 times: 2 x 256 9.2 / 10.4, 3 x 333 17.8 / 18.0, but 4 x
+    256 15.1 / 10.9, 2 x 333 15.0 / 10.9, 2 x 512 19.5 / 14.2; past 640 rows one tile runs while the two-tile grid fits the GPU at
+    once, a line that is older than the kernels (1 x 1000 25.8 / 21.2, with two 1 x 1300 43.6 / 27.5).
 
-    Head dimension 64 (two CTAs per SM with one tile, one with two), 16 heads: while the two-tile grid fits the GPU at
-    once one tile runs for causal sequences, but past 512 rows for an even number of tiles only (the longest tile
-    of an odd number runs alone in its CTA): 1 x 512 10.7 / 11.6, 1 x 1000 17.8 / 18.8, but 3 x 600 13.9 / 12.2; without
-    the mask up to 384 rows only: 3 x 333 9.6 / 11.6, but 2 x 1000 22.2 / 21.2. Off the faster side by now: causal 3 x 333
-    9.1 / 8.1 (one runs), 16 x 100 7.4 / 10.3 (two run), without the mask 1 x 512 10.6 / 12.8 (two run)."""
+    Head dimension 64, two CTAs per SM with one tile, one with two. Causal: up to three tiles a head, one (16 x 100 7.5 / 10.4, 12 x 256
+    13.5 / 15.6, 12 x 333 18.4 / 22.5), five tiles two while their grid fits (2 x 640 14.1 / 11.4, 16 x 640 47.9 / 51.1), other odd
+    numbers two (the longest tile would run alone on its SM), even numbers two past the GPU's SMs (16 x 512 level, 3 x 1000 23.8 / 19.4).
+    Without the mask two from four tiles on, with two or three where one-tile CTAs would share SMs (5 x 160
+    9.6 / 8.2, 4 x 333 12.0 / 10.2, but 4 x 256 7.4 / 8.0) and two take no more waves (8 x 333 19.2 / 16.8, 12 x 333 22.7 / 25.2)."""
     sms, tiles = _g.num_sms(device), (S + 127) // 128
     one, two = B * H * tiles, B * H * ((S + 255) // 256)
     if dh == 64:
-        fewer = (S <= 512 or tiles % 2 == 0) if causal else S <= 384
-        return two > sms or not fewer
-    if two <= sms or S <= 128:
+        if causal:
+            return tiles >= 4 and (two <= sms if tiles == 5 else two > sms or tiles % 2 == 1)
+        return tiles >= 4 or (tiles > 1 and one > sms and -(-two // sms) <= -(-one // (2 * sms)))
+    if tiles == 1:
         return False
-    one, two = -(-one // sms), -(-two // sms)          # waves
-    return S > 384 or (2 * one >= 3 * two if S > 256 else 2 * one > 3 * two)
+    waves, pair_waves = -(-one // sms), -(-two // sms)
+    if not causal:
+        return pair_waves < waves or tiles > 7
+    if S > 384:
+        return two > sms or (S <= 640 and pair_waves < waves)
+    return 2 * waves >= 3 * pair_waves if S > 256 else 2 * waves > 3 * pair_waves
 
 
 # The backward pass spills its dS tiles (bf16 [B*H, S, S]) to a scratch buffer so that dQ is a streamed

@@ -30,6 +30,20 @@ def test_attention_forward_tiles(B, S, H, dh, causal, two):
     assert A._two_tiles_win(B, S, H, dh, causal, None) is two
 
 
+@pytest.mark.parametrize("B,S,H,dh,causal,two", [
+    # two tiles that save a wave, on both sides of the line; without the mask, and past seven tiles without it
+    (1, 512, 32, 128, True, False), (2, 512, 32, 128, True, True), (1, 641, 32, 128, True, False), (2, 256, 32, 128, True, False),
+    (4, 256, 32, 128, True, True), (2, 256, 32, 128, False, False), (3, 256, 32, 128, False, True), (1, 896, 8, 128, False, False),
+    (1, 897, 8, 128, False, True),
+    # head dimension 64: short heads keep one tile, five tiles two while their grid fits; without the mask by waves
+    (16, 100, 16, 64, True, False), (24, 256, 16, 64, True, False), (12, 384, 16, 64, True, False), (3, 640, 16, 64, True, True),
+    (4, 640, 16, 64, True, False), (4, 256, 16, 64, False, False), (5, 256, 16, 64, False, True), (5, 384, 16, 64, False, False),
+    (8, 384, 16, 64, False, True), (1, 385, 16, 64, False, True),
+])
+def test_attention_forward_tiles_by_waves(B, S, H, dh, causal, two):
+    assert A._two_tiles_win(B, S, H, dh, causal, None) is two
+
+
 @pytest.mark.parametrize("B,L,H,Hkv,page,stream", [
     (1, 2048, 32, 8, 64, True), (4, 2048, 32, 8, 128, True), (16, 512, 32, 8, 64, True), (64, 256, 32, 8, 64, True),
     (64, 2048, 32, 8, 64, True), (16, 2304, 32, 2, 64, True), (1, 8192, 16, 2, 64, True),
