@@ -63,9 +63,9 @@ struct Params {
   float* partials;       // dense fp32 [256, 256] blocks, one per scratch slot
   // SwiGLU epilogue (ff > 0): B is a fused [gate | up] weight of 2*ff columns and N == 2*ff. A tile then
   // holds 128 gate columns (staged by the leader CTA) and the MATCHING 128 up columns (staged by the
-  // peer), so that after writing both to C the epilogue can also write act = silu(gate) * up.
+  // peer), so that the epilogue can write act = silu(gate) * up (tmap_rs.m[0]) behind gate (tmap_c) and up (tmap_rs.m[1]),
+  // or act alone (C == nullptr).
   int ff;
-  void* act; int ld_act;
   // SwiGLU-backward epilogue (gu != nullptr, ff == 0): the product is dh [M, N] (N = ff columns); instead
   // of storing it, the epilogue reads the saved [gate | up] row of the forward pass and writes
   // dgu = [dh * up * silu'(gate) | dh * silu(gate)] into C [M, 2N].
@@ -489,38 +489,51 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const int row = (m2 * 2 + static_cast<int>(rank)) * BM + q * 32 + lane;
       const uint32_t taddr_row = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
       if (p.ff) {
-        // SwiGLU tile: accumulator columns [0,128) are gate, [128,256) the matching up columns
-#pragma unroll 1
-        for (int gc = half * 2; gc < half * 2 + 2; ++gc) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_32x32(taddr_row + gc * 32, rg);
-          tmem_ld_32x32(taddr_row + BNH + gc * 32, ru);
+        // SwiGLU tile: accumulator columns [0,128) are gate, [128,256) the matching up columns. A warp takes 64 of each, hands the
+        // accumulator back as soon as it holds them as bf16, and sends gate, up (if C is wanted) and act through its
+        // staging buffer, 32 rows x 64 columns at a time.
+        uint8_t* stg = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
+        const int row0w = (m2 * 2 + static_cast<int>(rank)) * BM + q * 32, colw = n_idx * BNH + half * 64;
+        const bool issued = row0w < p.M && colw < p.ff;
+        uint32_t pg[32], pu[32];
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+          uint32_t r[32];
+          tmem_ld_32x32(taddr_row + (cc >> 1) * BNH + half * 64 + (cc & 1) * 32, r);
           tmem_ld_wait();
-          const int gcol = n_idx * BNH + gc * 32;
-          if (row < p.M && gcol < p.ff) {
-            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc;
-            __nv_bfloat16* arow = reinterpret_cast<__nv_bfloat16*>(p.act) + static_cast<size_t>(row) * p.ld_act;
+          uint32_t* to = (cc < 2 ? pg : pu) + (cc & 1) * 16;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              if (gcol + v * 8 < p.ff) {   // ff % 8 == 0 is enforced on the host
-                uint4 og, ou, oa;
-                uint32_t* pg = &og.x; uint32_t* pu = &ou.x; uint32_t* pa = &oa.x;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  pg[j] = pack_bf16x2(__uint_as_float(rg[v * 8 + 2 * j]), __uint_as_float(rg[v * 8 + 2 * j + 1]));
-                  pu[j] = pack_bf16x2(__uint_as_float(ru[v * 8 + 2 * j]), __uint_as_float(ru[v * 8 + 2 * j + 1]));
-                  // act from the bf16-rounded gate / up, exactly what the stand-alone kernel reads back
-                  const float g0 = bf16_lo(pg[j]), g1 = bf16_hi(pg[j]);
-                  const float u0 = bf16_lo(pu[j]), u1 = bf16_hi(pu[j]);
-                  pa[j] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1);
-                }
-                *reinterpret_cast<uint4*>(crow + gcol + v * 8) = og;
-                *reinterpret_cast<uint4*>(crow + p.ff + gcol + v * 8) = ou;
-                *reinterpret_cast<uint4*>(arow + gcol + v * 8) = oa;
-              }
-            }
-          }
+          for (int j = 0; j < 16; ++j) to[j] = pack_bf16x2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc ? leader_empty1 : leader_empty0);
+        auto send = [&](const uint32_t (&w)[32], const CUtensorMap* to) {
+          if (lane == 0) tma_store_wait_read<0>();      // the slab before has left the staging buffer
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(w[c * 4], w[c * 4 + 1], w[c * 4 + 2], w[c * 4 + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && issued) {
+            tma_store_2d(to, stg, colw, row0w);
+            tma_store_commit();
+          }
+        };
+        if (p.C) {
+          send(pg, &tmap_c);
+          send(pu, &tmap_rs.m[1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          // act from the bf16-rounded gate / up, exactly what the stand-alone kernel reads back
+          const float g0 = bf16_lo(pg[j]), g1 = bf16_hi(pg[j]);
+          const float u0 = bf16_lo(pu[j]), u1 = bf16_hi(pu[j]);
+          pg[j] = pack_bf16x2(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1);
+        }
+        send(pg, &tmap_rs.m[0]);
+        continue;
       } else if (!p.gu && sg.slot < 0 && p.use_tma_store) {
         // plain tile through shared memory and a TMA tensor store: two slabs of 64 columns per warp
         uint8_t* stg = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
@@ -772,8 +785,8 @@ using namespace sb;
 // `gu` (optional, with ff == 0): SwiGLU-backward epilogue. The product is dh [M, N]; C must be [M, 2N] and
 // receives dgu computed from the saved forward [gate | up] rows `gu` [M, ld_gu]; no residual.
 // `act` (optional, with ff > 0): SwiGLU epilogue. B then holds [gate | up] (N == 2*ff, ff % 8 == 0), C receives
-// the bf16 [gate | up] product as usual and `act` [M, ld_act] receives silu(gate) * up; no residual, no
-// balanced schedule on that path.
+// the bf16 [gate | up] product as usual (nullptr: it is not kept) and `act` [M, ld_act] receives silu(gate) * up; no
+// residual, no balanced schedule on that path.
 extern "C" size_t sb_gemm_pair_workspace_floats() { return static_cast<size_t>(num_sms() / 2) * 3 * 256 * 256; }
 
 extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda,
@@ -781,9 +794,10 @@ extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const vo
                                  int ff, const void* gu, int ld_gu, int* status, void* stream_) {
   using namespace sb::pair;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || (ldc & 7) || (R && (ldr & 7))) return SB_ERR_ARG;
+  if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || (ldc & 7) || (R && (ldr & 7)) || (!C && !ff)) return SB_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(C) & 15) || (R && (reinterpret_cast<uintptr_t>(R) & 15))) return SB_ERR_ALIGN;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, tc;
+  TmapSet swiglu_out;
   int rc;
   if (!a_mn) rc = make_tmap_2d_bf16(&ta, A, K, M, lda, BK, BM);
   else rc = make_tmap_2d_bf16(&ta, A, M, K, lda, 64, BK);
@@ -792,12 +806,18 @@ extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const vo
   else rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, BK);
   if (rc) return rc;
   if (ff) {
-    if (!act || N != 2 * ff || (ff & 7) || (ld_act & 7) || R || (reinterpret_cast<uintptr_t>(act) & 15)) return SB_ERR_ARG;
+    if (ff < 0 || !act || N != 2 * ff || (ff & 7) || (ld_act & 7) || R || (reinterpret_cast<uintptr_t>(act) & 15)) return SB_ERR_ARG;
     workspace = nullptr;
+    // gate and up have a map each, so that a slab that crosses the end of the gate columns does not write up columns
+    for (CUtensorMap& m : swiglu_out.m) m = ta;
+    rc = make_tmap_2d_bf16(&swiglu_out.m[0], act, ff, M, ld_act, 64, 32);
+    if (!rc && C) rc = make_tmap_2d_bf16(&tc, C, ff, M, ldc, 64, 32);
+    if (!rc && C) rc = make_tmap_2d_bf16(&swiglu_out.m[1], static_cast<__nv_bfloat16*>(C) + ff, ff, M, ldc, 64, 32);
+    if (rc) return rc;
   }
   Params p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.R = R; p.ldr = ldr; p.status = status;
-  p.ff = ff; p.act = act; p.ld_act = ld_act;
+  p.ff = ff;
   if (gu) {
     if (ff || R || (ld_gu & 7) || (reinterpret_cast<uintptr_t>(gu) & 15)) return SB_ERR_ARG;
     workspace = nullptr;
@@ -807,7 +827,6 @@ extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const vo
   p.rs.W = 0;
   // output through shared memory + TMA tensor store (SB_GEMM_TMA_STORE=0 keeps the register stores)
   static const bool tma_store = [] { const char* e = getenv("SB_GEMM_TMA_STORE"); return !(e && e[0] == '0'); }();
-  CUtensorMap tc;
   p.use_tma_store = 0;
   if (tma_store && !ff && !gu) {
     rc = make_tmap_2d_bf16(&tc, C, N, M, ldc, 64, 32);
@@ -828,11 +847,12 @@ extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const vo
     p.sched.dp_tiles = p.sched.sk_tiles = p.sched.sk_workers = p.sched.sk_slots = 0;
   }
   const int grid = 2 * pairs;
-  const CUtensorMap* tcp = p.use_tma_store ? &tc : nullptr;
-  if (!a_mn && !b_mn) rc = launch<false, false>(ta, tb, p, grid, stream, nullptr, tcp);
-  else if (!a_mn && b_mn) rc = launch<false, true>(ta, tb, p, grid, stream, nullptr, tcp);
-  else if (a_mn && !b_mn) rc = launch<true, false>(ta, tb, p, grid, stream, nullptr, tcp);
-  else rc = launch<true, true>(ta, tb, p, grid, stream, nullptr, tcp);
+  const CUtensorMap* tcp = p.use_tma_store || (ff && C) ? &tc : nullptr;
+  const TmapSet* outs = ff ? &swiglu_out : nullptr;
+  if (!a_mn && !b_mn) rc = launch<false, false>(ta, tb, p, grid, stream, nullptr, tcp, outs);
+  else if (!a_mn && b_mn) rc = launch<false, true>(ta, tb, p, grid, stream, nullptr, tcp, outs);
+  else if (a_mn && !b_mn) rc = launch<true, false>(ta, tb, p, grid, stream, nullptr, tcp, outs);
+  else rc = launch<true, true>(ta, tb, p, grid, stream, nullptr, tcp, outs);
   if (rc) return rc;
   if (fixup) {
     dim3 fg(p.sched.sk_tiles, 2 * BM * BN / (256 * 4));
@@ -871,7 +891,7 @@ extern "C" int sb_gemm_pair_ag_bf16(void* const* a_ptrs, const void* B, void* C,
   if (rc) return rc;
   Params p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.R = R; p.ldr = ldr; p.status = status;
-  p.ff = 0; p.act = nullptr; p.ld_act = 0; p.gu = nullptr; p.ld_gu = 0;
+  p.ff = 0; p.gu = nullptr; p.ld_gu = 0;
   p.partials = nullptr;
   p.use_tma_store = 0;
   p.sched.dp_tiles = p.sched.sk_tiles = p.sched.sk_workers = p.sched.sk_slots = 0;
@@ -938,7 +958,7 @@ extern "C" int sb_gemm_pair_rs_bf16(const void* A, const void* B, void* const* p
   }
   Params p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldp; p.R = nullptr; p.ldr = 0; p.status = status;
-  p.ff = 0; p.act = nullptr; p.ld_act = 0; p.gu = nullptr; p.ld_gu = 0;
+  p.ff = 0; p.gu = nullptr; p.ld_gu = 0;
   p.partials = nullptr;
   p.use_tma_store = 1;           // reduce-scatter tiles always leave by TMA store, into the owners' memory
   p.sched.dp_tiles = p.sched.sk_tiles = p.sched.sk_workers = p.sched.sk_slots = 0;

@@ -24,7 +24,7 @@ import torch
 from .. import ops
 from ..generate import SamplingParams
 from ..ops.sampling import DeviceSampler
-from ..ops import _lib, attention as att, decode as D
+from ..ops import _lib, attention as att, decode as D, gemm as G
 from .sciagent import BF, GQADecoder, SciAgentConfig
 
 
@@ -170,6 +170,18 @@ class InferenceEngine:
             w = w.dequantize()
         return ops.matmul_nn(x, w, residual=residual)
 
+    def _gated(self, x, w):
+        """silu(gate) * up of ``[gate | up] = x @ w`` in one launch, or None where that is not how ``_linear`` takes the product (by
+        1024 rows int8 weights are expanded whatever their shape)."""
+        M, (K, N) = x.shape[0], w.shape
+        if not x.is_cuda or M < 256 or not G.swiglu_in_epilogue(M, K, N // 2):
+            return None
+        if isinstance(w, D.QuantWeight):
+            if M < 1024 and N % 16 == 0:
+                return None
+            w = w.dequantize()
+        return ops.matmul_nn_swiglu_act(x, w)
+
     # ------------------------------------------------------------------ prefill
     def prefill(self, tokens: torch.Tensor):
         """tokens [B, P] (all prompts the same length). Fills the cache, leaves the greedy next
@@ -194,8 +206,12 @@ class InferenceEngine:
             a, _ = att.attention_fwd(qkv, B, P, H, Hkv, dh, causal=True, want_lse=False)
             x = self._proj_out(a, l["wo"], x, site="attn")
             h, _ = ops.rmsnorm_fwd(x, l["rms2"], cfg.eps, want_inv=False)
-            gu = self._linear(h, l["wgu"])
-            x = self._proj_out(gu, l["wd"], x, swiglu=True, site="mlp")
+            act = self._gated(h, l["wgu"])
+            if act is not None:
+                x = self._proj_out(act, l["wd"], x, site="mlp")
+            else:
+                gu = self._linear(h, l["wgu"])
+                x = self._proj_out(gu, l["wd"], x, swiglu=True, site="mlp")
         last = x.view(B, P, -1)[:, -1, :].contiguous()
         logits = self.logits[:B]
         self._head(last, logits, rms_weight=self.rms_final)

@@ -69,11 +69,10 @@ def _check2d(t: torch.Tensor, name: str) -> None:
 # products with at least one full wave of such tiles and no split-K; SB_GEMM_PAIR=0/1 forces it.
 PAIR_MODE = os.environ.get("SB_GEMM_PAIR", "auto")
 BALANCED = os.environ.get("SB_GEMM_BALANCED", "1") != "0"
-# SwiGLU forward / backward inside the GEMM epilogues (bit-identical to the separate kernels). Off by
-# default: measured on one box back to back, the training step took 30.9 ms with the fused epilogues and
-# 29.3 ms without - with K = 1024 a tile's main loop is too short to hide an epilogue that does exponentials,
-# divisions and (backward) global loads before it can hand the accumulator back to the tensor cores.
-FUSE_SWIGLU = os.environ.get("SB_FUSE_SWIGLU", "0") == "1"
+# SwiGLU forward inside the GEMM epilogue (bit-identical to the separate kernel): by the rule of ``swiglu_in_epilogue``, SB_FUSE_SWIGLU=0/1
+# forces it. 1 also puts the backward pass into the epilogue of its product, which is off otherwise: with K = 1024 a tile's main loop is too
+# short to hide an epilogue that reads gate and up from memory (training step 30.9 ms with both, 29.3 without, when measured).
+FUSE_SWIGLU = {"0": False, "1": True}.get(os.environ.get("SB_FUSE_SWIGLU"))
 
 
 # The balanced schedule pays a fix-up pass and fp32 scratch traffic (measured: about 20 us on 74 CTA pairs). Measured
@@ -201,34 +200,66 @@ def matmul_nn(x, w, residual=None, out=None, splits=None, bn=None, bias=None):
     return _gemm(x, w, M, N, K, False, True, out, residual, splits, bn, bias)
 
 
+def swiglu_in_epilogue(M: int, K: int, ff: int) -> bool:
+    """Whether the gate/up product of ``M`` rows writes ``silu(gate) * up`` itself. The epilogue takes as long as the main loop over about 1024
+    rows of k, and that of the last tile of every CTA pair is not hidden, so it wants long k and at least four waves of tiles (256 x 128
+    columns each of gate and up). Us, product and separate kernel / fused / fused without keeping [gate | up], M x K x ff: 16384 x 1024 x
+    2816 192 / 166 / 149, 4096 x 1024 x 2816 58.9 / 53.7 / 49.7, 2048 x 4096 x 14336 428 / 387 / 375, 1024 x 4096 x 11008 164 / 149 /
+    144; but 2048 x 1024 x 2816 37.4 / 37.2 / 33.1, 600 x 4096 x 11008 131 / 136 / 133, 999 x 1024 x 2816 28 / 37 / 35, 4096 x 512 x
+    1408 30 / 33 / 31."""
+    if PAIR_MODE == "0" or ff % 8 or FUSE_SWIGLU is False:
+        return False
+    if FUSE_SWIGLU:
+        return M >= 256
+    return K >= 1024 and ((M + 255) // 256) * ((ff + 127) // 128) >= 4 * (num_sms() // 2)
+
+
+def _swiglu_product(x, wgu, gu, act):
+    """One launch of the CTA-pair kernel: each CTA of a pair stages one half, gate columns and the matching up columns."""
+    global launch_count
+    M, K = x.shape
+    N = wgu.shape[1]
+    _check2d(x, "x")
+    _check2d(wgu, "wgu")
+    _lib.call("sb_gemm_pair_bf16", x.data_ptr(), wgu.data_ptr(), _lib.ptr(gu), None, M, N, K, x.stride(0), wgu.stride(0),
+              gu.stride(0) if gu is not None else 0, 0, 0, 1, None, act.data_ptr(), act.stride(0), N // 2, None, 0,
+              _lib.status_word(x.device).data_ptr(), _lib.stream())
+    launch_count += 1
+
+
 def matmul_nn_swiglu(x, wgu, out=None, act=None):
     """Gate/up projection with the SwiGLU fused into the GEMM epilogue: returns ``(gu, act)`` with
     ``gu = x @ wgu`` (bf16 ``[M, 2*ff]`` = [gate | up], kept for the backward pass) and
-    ``act = silu(gate) * up`` (bf16 ``[M, ff]``), bit-identical to ``swiglu_fwd(matmul_nn(x, wgu))``.
-    Runs on the CTA-pair kernel (each CTA of a pair stages one half: gate columns / matching up columns)."""
-    global launch_count
+    ``act = silu(gate) * up`` (bf16 ``[M, ff]``), bit-identical to ``swiglu_fwd(matmul_nn(x, wgu))``."""
     M, K = x.shape
     K2, N = wgu.shape
     ff = N // 2
     if K != K2 or N % 2:
         raise ValueError("matmul_nn_swiglu: shape mismatch")
-    fused = x.is_cuda and PAIR_MODE != "0" and FUSE_SWIGLU and ff % 8 == 0 and M >= 256
-    if not fused:
+    if not (x.is_cuda and swiglu_in_epilogue(M, K, ff)):
         from . import basic
         gu = matmul_nn(x, wgu, out=out)
         return gu, basic.swiglu_fwd(gu, out=act)
-    _check2d(x, "x")
-    _check2d(wgu, "wgu")
     if out is None:
         out = _lib.empty((M, N), torch.bfloat16, x.device)
     if act is None:
         act = _lib.empty((M, ff), torch.bfloat16, x.device)
-    st = _lib.status_word(x.device)
-    _lib.call("sb_gemm_pair_bf16", x.data_ptr(), wgu.data_ptr(), out.data_ptr(), None, M, N, K, x.stride(0),
-              wgu.stride(0), out.stride(0), 0, 0, 1, None, act.data_ptr(), act.stride(0), ff, None, 0, st.data_ptr(),
-              _lib.stream())
-    launch_count += 1
+    _swiglu_product(x, wgu, out, act)
     return out, act
+
+
+def matmul_nn_swiglu_act(x, wgu):
+    """``matmul_nn_swiglu`` without the gate/up product: ``act`` alone, the same bits, for passes without a backward."""
+    M, K = x.shape
+    K2, N = wgu.shape
+    if K != K2 or N % 2:
+        raise ValueError("matmul_nn_swiglu_act: shape mismatch")
+    if not (x.is_cuda and swiglu_in_epilogue(M, K, N // 2)):
+        from . import basic
+        return basic.swiglu_fwd(matmul_nn(x, wgu))
+    act = _lib.empty((M, N // 2), torch.bfloat16, x.device)
+    _swiglu_product(x, wgu, None, act)
+    return act
 
 
 def matmul_nt_swiglu_bwd(dy, wd, gu, out=None):

@@ -209,6 +209,40 @@ def test_swiglu_epilogue_is_bitwise_the_unfused_path(M, K, ff, monkeypatch):
     _check(gu, x.float() @ wgu.float(), K)
 
 
+@pytest.mark.parametrize("M,K,ff", [(256, 64, 8), (257, 128, 72), (1000, 512, 264), (2048, 1024, 4736)])
+def test_swiglu_epilogue_without_the_product(M, K, ff, monkeypatch):
+    """act alone, the same bits as with the product kept: one row past a tile, slabs of 64 columns that end inside (and would
+    reach into the up columns), more tiles than CTA pairs. The product keeps its gate and up columns apart."""
+    from scirust_b200.ops import gemm
+    monkeypatch.setattr(gemm, "FUSE_SWIGLU", True)
+    x, wgu = _mk((M, K), 1), _mk((K, 2 * ff), 2)
+    gu, act = ops.matmul_nn_swiglu(x, wgu)
+    only = ops.matmul_nn_swiglu_act(x, wgu)
+    _lib.check_status()
+    assert torch.equal(act, only)
+    assert torch.equal(act, ops.swiglu_fwd(gu))
+    _check(gu, x.float() @ wgu.float(), K)
+
+
+@pytest.mark.parametrize("quant", [None, "int8"])
+def test_prefill_with_the_swiglu_in_the_product(quant, monkeypatch):
+    """The engine's feed-forward with and without it: the same logits and cache to the bit."""
+    from scirust_b200.models.infer import InferenceEngine
+    from scirust_b200.models.sciagent import GQADecoder, SciAgentConfig
+    from scirust_b200.ops import gemm
+    cfg = SciAgentConfig(512, 256, 2, 4, 2, 512, 2048, 1e4)
+    model = GQADecoder(cfg, device="cuda", seed=3)
+    tokens = torch.randint(0, 512, (2, 600), generator=torch.Generator().manual_seed(1)).cuda()
+    got = []
+    for fuse in (True, False):
+        monkeypatch.setattr(gemm, "FUSE_SWIGLU", fuse)
+        eng = InferenceEngine(model, quant=quant, max_batch=2, max_seq=640)
+        got.append((eng.prefill(tokens).clone(), *eng.cache.pools))
+    _lib.check_status()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("M,d,ff", [(512, 256, 128), (4096, 1024, 2816), (1000, 512, 264)])
 def test_swiglu_backward_epilogue_is_bitwise_the_unfused_path(M, d, ff, monkeypatch):
     from scirust_b200.ops import basic, gemm
