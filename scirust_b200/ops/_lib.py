@@ -162,10 +162,15 @@ def check_canaries() -> None:
     _fenced[:] = live
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)   # without the test for an initialised CUDA
+
+
 def stream() -> int:
     """Handle of the current stream of the current device, without building a ``torch.cuda.Stream`` object (an op asks
-    for it two or three times: the launch and the keys of its workspaces)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    for it two or three times: the launch and the keys of its workspaces), and without ``torch.cuda.current_device()``, whose
+    test for an initialised CUDA costs more than both answers (0.37 us, 0.15 without): callers hold a CUDA tensor."""
+    return _raw_stream(current_device())
 
 
 def check(rc: int, what: str) -> None:

@@ -31,8 +31,8 @@ _GEMV_FMA = os.environ.get("SB_GEMV_FMA") == "1"      # as csrc/decode.cu, read 
 _ws: dict = {}
 
 
-def _workspace(n, device):
-    key = (device, _lib.stream())             # per stream: concurrent calls on two streams must not share scratch
+def _workspace(n, device, stream=None):
+    key = (device, _lib.stream() if stream is None else stream)     # per stream: concurrent calls on two streams must not share scratch
     w = _ws.get(key)
     if w is None or w.numel() < n:
         w = _lib.empty(max(n, 1 << 22), torch.float32, device)
@@ -46,10 +46,10 @@ _lib.register("sb_set_pdl", [i32])
 _gemv_ws: dict = {}
 
 
-def _gemv_workspace(n, device):
+def _gemv_workspace(n, device, stream=None):
     """Workspace of the GEMV: 4096 counter words (kept zero by the kernel) + split partials; one per (device,
     stream), so that GEMVs issued on two streams share neither counters nor partial sums."""
-    key = (device, _lib.stream())
+    key = (device, _lib.stream() if stream is None else stream)
     w = _gemv_ws.get(key)
     if w is None or w.numel() < n:
         w = torch.zeros(max(n, 1 << 22), dtype=torch.float32, device=device)
@@ -194,25 +194,36 @@ def gemv(x, w, residual=None, out=None, out_f32=None, splits=None, rms_weight=No
             out.copy_(y.to(BF))
             return out
         return y.to(BF) if out_f32 is None else out_f32
-    if out is None and out_f32 is None:
-        out = _lib.empty((M, N), BF, x.device)
+    device, stream = x.device, _lib.stream()
+    os_ = 0
+    if out is not None:
+        os_ = out.stride(0)
+    elif out_f32 is None:
+        out, os_ = _lib.empty((M, N), BF, device), N
     grp = 8                                   # rows per call
+    rows = M if M < grp else grp
     if splits is None:
-        splits = _gemv_splits(N, K, 512 if quant else 256, min(M, grp), quant)
-    splits = max(splits, (K + 4095) // 4096)
-    ws = _gemv_workspace(4096 + splits * min(M, grp) * N, x.device)
-    st = _lib.status_word(x.device)
+        splits = _gemv_splits(N, K, 512 if quant else 256, rows, quant)
+    if K > 4096 * splits:
+        splits = (K + 4095) // 4096
+    ws = _gemv_workspace(4096 + splits * rows * N, device, stream).data_ptr()
+    st = _lib.status_word(device).data_ptr()
     # row groups are addressed by offsets: a decode step is one group, and slicing its tensors costs more than the launch
     xp, xs = x.data_ptr(), x.stride(0)
     rp, rs = (residual.data_ptr(), residual.stride(0)) if residual is not None else (None, 0)
-    op, os_ = (out.data_ptr(), out.stride(0)) if out is not None else (None, 0)
+    op = out.data_ptr() if out is not None else None
     fp, fs = (out_f32.data_ptr(), out_f32.stride(0)) if out_f32 is not None else (None, 0)
-    pro = 1 if rms_weight is not None else (2 if swiglu else 0)
+    wp, ws0, sp = wm.data_ptr(), wm.stride(0), w.scale.data_ptr() if quant else None
+    pro, gain = (1, rms_weight.data_ptr()) if rms_weight is not None else (2 if swiglu else 0, None)
+    if M <= grp:
+        _lib.call("sb_gemv", xp, xs, wp, ws0, sp, rp, rs, op, os_, fp, M, N, K, int(quant), splits, ws, pro, gain, float(eps), st,
+                  stream)
+        _g.launch_count += 1
+        return out if out is not None else out_f32
     for m0 in range(0, M, grp):
-        _lib.call("sb_gemv", xp + m0 * xs * 2, xs, wm.data_ptr(), wm.stride(0), w.scale.data_ptr() if quant else None,
-                  rp + m0 * rs * 2 if rp else None, rs, op + m0 * os_ * 2 if op else None, os_,
-                  fp + m0 * fs * 4 if fp else None, min(grp, M - m0), N, K, int(quant), splits, ws.data_ptr(), pro,
-                  _lib.ptr(rms_weight), float(eps), st.data_ptr(), _lib.stream())
+        _lib.call("sb_gemv", xp + m0 * xs * 2, xs, wp, ws0, sp, rp + m0 * rs * 2 if rp else None, rs,
+                  op + m0 * os_ * 2 if op else None, os_, fp + m0 * fs * 4 if fp else None, min(grp, M - m0), N, K, int(quant),
+                  splits, ws, pro, gain, float(eps), st, stream)
         _g.launch_count += 1
     return out if out is not None else out_f32
 
@@ -536,34 +547,36 @@ def decode_attention(q, pool, block_table, page, seq_len, H, Hkv, dh, scale=None
     B = q.shape[0]
     if not q.is_cuda:
         return decode_attention_ref(q, pool, block_table, page, seq_len, H, Hkv, dh, scale).to(BF)
-    L = max_len if max_len is not None else block_table.shape[1] * page
+    device, on = q.device, _lib.stream()
+    max_blocks = block_table.shape[1]
+    L = max_len if max_len is not None else max_blocks * page
     tiles = B * Hkv * max(1, (L + 63) // 64)
     if stream is None:
-        stream = max_len is not None and _stream_wins(L, B * Hkv, H // Hkv, page, q.device)
+        stream = max_len is not None and _stream_wins(L, B * Hkv, H // Hkv, page, device)
     if n_splits is None and stream and _stream_ok(pool, page, B, H, Hkv, dh):
         # the tiles of the whole batch dealt out evenly over the SMs
-        part = _workspace(2 * _g.num_sms(q.device) * 16 * (dh + 2), q.device)
-        ctr = _gemv_workspace(4096, q.device)
-        out = _lib.empty((B, H * dh), BF, q.device)
+        part = _workspace(2 * _g.num_sms(device) * 16 * (dh + 2), device, on)
+        ctr = _gemv_workspace(4096, device, on)
+        out = _lib.empty((B, H * dh), BF, device)
         _lib.call("sb_decode_attention_stream", q.data_ptr(), q.stride(0), pool.data_ptr(), pool.shape[0],
-                  block_table.data_ptr(), block_table.shape[1], page, seq_len.data_ptr(), B, H, Hkv, dh,
+                  block_table.data_ptr(), max_blocks, page, seq_len.data_ptr(), B, H, Hkv, dh,
                   tiles, float(scale), part.data_ptr(), ctr.data_ptr() + 2048 * 4,
-                  out.data_ptr(), out.stride(0), _lib.status_word(q.device).data_ptr(), _lib.stream())
+                  out.data_ptr(), out.stride(0), _lib.status_word(device).data_ptr(), on)
         _g.launch_count += 1
         return out
     if n_splits is None:
         # about four 128-thread CTAs per SM, at least two 64-position tiles per split
         n_splits = max(1, min(64, (148 * 4 + B * Hkv - 1) // max(1, B * Hkv), (L + 127) // 128))
-    ws = _workspace(B * H * n_splits * (dh + 2), q.device)
-    ctr = _gemv_workspace(4096, q.device) if B * Hkv <= 2048 else None
+    ws = _workspace(B * H * n_splits * (dh + 2), device, on)
+    ctr = _gemv_workspace(4096, device, on) if B * Hkv <= 2048 else None
     if ctr is None:
         raise ValueError("decode_attention: batch * kv_heads above 2048 is not supported")
     part_o = ws.data_ptr()                       # by offset: a slice costs as much as the launch
-    out = _lib.empty((B, H * dh), BF, q.device)
+    out = _lib.empty((B, H * dh), BF, device)
     _lib.call("sb_decode_attention", q.data_ptr(), q.stride(0), pool.data_ptr(), block_table.data_ptr(),
-              block_table.shape[1], page, seq_len.data_ptr(), B, H, Hkv, dh, n_splits, float(scale),
+              max_blocks, page, seq_len.data_ptr(), B, H, Hkv, dh, n_splits, float(scale),
               part_o, part_o + B * H * n_splits * dh * 4, ctr.data_ptr() + 2048 * 4, out.data_ptr(), out.stride(0),
-              _lib.stream())
+              on)
     _g.launch_count += 1
     return out
 

@@ -25,7 +25,9 @@ _workspaces: dict = {}
 
 def num_sms(device=None) -> int:
     """Streaming multiprocessors of the device (148 on a B200), asked of the driver once per device."""
-    idx = torch.cuda.current_device() if device is None or device.index is None else device.index
+    idx = None if device is None else device.index
+    if idx is None:
+        idx = _lib.current_device()
     n = _sm_count.get(idx)
     if n is None:
         n = torch.cuda.get_device_properties(idx).multi_processor_count
