@@ -19,6 +19,7 @@
 #include "sm100_ptx.cuh"
 #include "peer_sync.cuh"
 #include "dependent.cuh"
+#include "rope_rows.cuh"
 #include <atomic>
 
 namespace sb {
@@ -2343,6 +2344,18 @@ extern "C" int sb_rope_kv_append(void* qkv, int ld, int H, int Hkv, int dh, cons
                                  void* pool, const int* block_table, int max_blocks, int page, const int* seq_of,
                                  const int* pos, int n_tok, void* stream) {
   if (n_tok <= 0 || (dh & 7)) return SB_ERR_ARG;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(pool) | reinterpret_cast<uintptr_t>(cos_t) |
+                       reinterpret_cast<uintptr_t>(sin_t);
+  if (n_tok > 128 && (ld & 7) == 0 && (at & 15) == 0) {     // a prompt: by rows; below that a CTA per token and head starts sooner
+    RopeRows p = {};
+    p.x = static_cast<__nv_bfloat16*>(qkv);
+    p.ld = ld; p.rows = n_tok; p.rot_heads = H + Hkv; p.heads = H + 2 * Hkv; p.dh = dh;
+    p.seq_len = 1; p.positions = pos;
+    p.cos_t = cos_t; p.sin_t = sin_t; p.sign = 1.f;
+    p.q_heads = H; p.kv_heads = Hkv; p.page = page; p.max_blocks = max_blocks;
+    p.pool = static_cast<__nv_bfloat16*>(pool); p.block_table = block_table; p.seq_of = seq_of;
+    return launch_rope_rows<true>(p, STREAM) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
+  }
   return launch_dep(rope_kv_append_kernel, dim3(n_tok, H + 2 * Hkv), dim3(dh / 2), 0, STREAM, static_cast<__nv_bfloat16*>(qkv), ld, H,
                     Hkv, dh, cos_t, sin_t, static_cast<__nv_bfloat16*>(pool), block_table, max_blocks, page, seq_of,
                     pos, n_tok) == cudaSuccess ? 0 : SB_ERR_LAUNCH;

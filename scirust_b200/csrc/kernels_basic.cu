@@ -16,6 +16,7 @@
 #include "api.h"
 
 #include "dependent.cuh"
+#include "rope_rows.cuh"
 
 namespace sb {
 
@@ -407,39 +408,6 @@ __global__ void colsum_finish_kernel(const float* __restrict__ partial, int chun
   for (int k = 0; k < chunks; ++k) s += partial[static_cast<size_t>(k) * cols + j];
   if (out_f32) out_f32[j] = s;
   if (out_bf16) out_bf16[j] = __float2bfloat16_rn(s);
-}
-
-// ---------------------------------------------------------------------------
-// RoPE on interleaved pairs, head-local frequency, rotate in place. `x` points at a
-// [rows, ld] matrix whose first n_heads*dh columns are rotated (q heads then k heads
-// of a fused qkv buffer). Table: cos/sin fp32 [max_pos, dh/2]. sign=+1 forward,
-// -1 backward (the transpose of a rotation is the rotation by the negative angle).
-// pos = positions[r] if given, else (r % seq_len) + offset.
-// ---------------------------------------------------------------------------
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ x, int ld, int rows, int n_heads, int dh, int seq_len,
-                            int offset, const int* __restrict__ positions, const float* __restrict__ cos_t,
-                            const float* __restrict__ sin_t, float sign) {
-  const int half = dh >> 1;
-  const int quads_per_row = n_heads * (half >> 2);  // 4 pairs (8 bf16 = 16 B) per thread
-  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= static_cast<size_t>(rows) * quads_per_row) return;
-  const int r = static_cast<int>(idx / quads_per_row);
-  const int qd = static_cast<int>(idx - static_cast<size_t>(r) * quads_per_row);
-  const int head = qd / (half >> 2);
-  const int p0 = (qd - head * (half >> 2)) * 4;  // first pair index inside the head
-  const int pos = positions ? positions[r] : (r % seq_len) + offset;
-  __nv_bfloat16* ptr = x + static_cast<size_t>(r) * ld + head * dh + p0 * 2;
-  float f[8];
-  unpack8(*reinterpret_cast<const uint4*>(ptr), f);
-  const float4 c = *reinterpret_cast<const float4*>(cos_t + static_cast<size_t>(pos) * half + p0);
-  float4 s = *reinterpret_cast<const float4*>(sin_t + static_cast<size_t>(pos) * half + p0);
-  s.x *= sign; s.y *= sign; s.z *= sign; s.w *= sign;
-  float o[8];
-  o[0] = f[0] * c.x - f[1] * s.x; o[1] = f[0] * s.x + f[1] * c.x;
-  o[2] = f[2] * c.y - f[3] * s.y; o[3] = f[2] * s.y + f[3] * c.y;
-  o[4] = f[4] * c.z - f[5] * s.z; o[5] = f[4] * s.z + f[5] * c.z;
-  o[6] = f[6] * c.w - f[7] * s.w; o[7] = f[6] * s.w + f[7] * c.w;
-  *reinterpret_cast<uint4*>(ptr) = pack8(o);
 }
 
 // ---------------------------------------------------------------------------
@@ -1233,11 +1201,12 @@ extern "C" int sb_rope(void* x, int ld, int rows, int n_heads, int dh, int seq_l
                        const int* positions, const float* cos_t, const float* sin_t, int backward, void* stream) {
   if (rows <= 0 || n_heads <= 0 || (dh & 7) || (ld & 7) || seq_len <= 0) return SB_ERR_ARG;
   if (!al16(x) || !al16(cos_t) || !al16(sin_t)) return SB_ERR_ALIGN;
-  const size_t total = static_cast<size_t>(rows) * n_heads * (dh >> 3);
-  rope_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, STREAM>>>(
-      static_cast<__nv_bfloat16*>(x), ld, rows, n_heads, dh, seq_len, offset, positions, cos_t, sin_t,
-      backward ? -1.f : 1.f);
-  CHECK_LAUNCH();
+  RopeRows p = {};
+  p.x = static_cast<__nv_bfloat16*>(x);
+  p.ld = ld; p.rows = rows; p.rot_heads = p.heads = n_heads; p.dh = dh;
+  p.seq_len = seq_len; p.offset = offset; p.positions = positions;
+  p.cos_t = cos_t; p.sin_t = sin_t; p.sign = backward ? -1.f : 1.f;
+  return launch_rope_rows<false>(p, STREAM) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
 extern "C" int sb_swiglu_fwd(const void* gu, void* h, int rows, int ff, void* stream) {

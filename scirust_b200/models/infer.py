@@ -201,8 +201,7 @@ class InferenceEngine:
         for li, l in enumerate(self.layers):
             h, _ = ops.rmsnorm_fwd(x, l["rms1"], cfg.eps, want_inv=False)
             qkv = self._linear(h, l["wqkv"])
-            ops.rope_(qkv, H + Hkv, dh, P, self.cos, self.sin)
-            D.kv_append(qkv, H, Hkv, dh, cache.pools[li], cache.block_table, cache.page, seq_of, pos)
+            D.rope_kv_append(qkv, H, Hkv, dh, self.cos, self.sin, cache.pools[li], cache.block_table, cache.page, seq_of, pos)
             a, _ = att.attention_fwd(qkv, B, P, H, Hkv, dh, causal=True, want_lse=False)
             x = self._proj_out(a, l["wo"], x, site="attn")
             h, _ = ops.rmsnorm_fwd(x, l["rms2"], cfg.eps, want_inv=False)

@@ -276,3 +276,28 @@ def test_cross_entropy_of_large_logits(cols):
     assert (loss[n:] == 0).all() and (d[n:] == 0).all()
     _check_cross_entropy(lg[:n], tg[:n], 0.25, loss[:n], d[:n])
     assert torch.equal(loss, ops.ce_loss_only(lg, tg))
+
+
+@pytest.mark.parametrize("rows,H,Hkv,dh,page", [(129, 3, 1, 64, 16), (300, 4, 2, 128, 64), (257, 5, 1, 24, 8), (1000, 2, 2, 8, 64)])
+def test_rope_by_rows_fills_the_cache(rows, H, Hkv, dh, page):
+    """A prompt's rotation with the copy to the cache (by rows, past 128 tokens) against the rotation and the copy by themselves: heads
+    that do not fill a thread's four, rows that do not fill a block, head dimensions that do not divide it. The same bits; and the
+    rotation against its fp32 statement."""
+    from scirust_b200.ops import decode as D
+    ld = (H + 2 * Hkv) * dh
+    x = _r((rows, ld), 21).cuda()
+    cos_t, sin_t = ops.rope_table(rows, dh, 10000.0, "cuda")
+    blocks = (rows + page - 1) // page
+    table = torch.randperm(blocks, generator=torch.Generator().manual_seed(2)).int().reshape(1, blocks).cuda()
+    pos = torch.arange(rows, dtype=torch.int32, device="cuda")
+    seq_of = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    pools = [torch.zeros(blocks, 2, Hkv, page, dh, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    one, two = x.clone(), x.clone()
+    D.rope_kv_append(one, H, Hkv, dh, cos_t, sin_t, pools[0], table, page, seq_of, pos)
+    ops.rope_(two, H + Hkv, dh, rows, cos_t, sin_t)
+    D.kv_append(two, H, Hkv, dh, pools[1], table, page, seq_of, pos)
+    assert torch.equal(one, two) and torch.equal(pools[0], pools[1])
+    ref = ops.rope_(x.cpu(), H + Hkv, dh, rows, *(t.cpu() for t in (cos_t, sin_t)))
+    _close(two, ref, 2 ** -8)
+    back = ops.rope_(two.clone(), H + Hkv, dh, rows, cos_t, sin_t, backward=True)
+    _close(back, x, 2 ** -7)
