@@ -13,7 +13,7 @@
 //
 // What bounds it: a row is read once (0.5 MB at a vocabulary of 128 k) and then walked about ten times, so with one
 // CTA per row the passes over global memory set the pace, whatever the number of rows. A row is spread over the
-// shared memory of a cluster instead: eight CTAs hold 64 KB each, a pass takes 16 words per thread, and the CTAs
+// shared memory of a cluster instead: of eight CTAs each holds 64 KB, a pass takes 16 words per thread, and the CTAs
 // exchange only their 256-bin histograms (distributed shared memory, one cluster barrier per radix level, two
 // histogram buffers in turn). The bin scan runs in one warp by shuffles instead of in one thread, the number of
 // ties falls out of the last level, and the second walk starts from the first walk's top-level histogram. 16 rows of
@@ -23,9 +23,12 @@
 // Each of the ten levels that are left costs a barrier, an exchange and a scan, about 6 us, and mostly sorts out a few
 // dozen words. So when the first level, whose histogram is made by the pass that makes the weights, leaves no more than
 // SAMP_LIST words at or above the digit that the cut falls into, these go to one CTA, which ranks them and finishes alone.
-// Ranks, sums and ties are those of the walks. The same 16 rows, normal logits of deviation 2.5: 27 us. Not taken where the cut
+// Ranks, sums and ties are those of the walks. The same 16 rows, normal logits of deviation 2.5: 26.5 us, of which half was a second
+// wave for the sixteenth cluster of eight; 17.8 in clusters of four (sample_cluster). Not taken where the cut
 // falls among the words below 1/256 of the largest, whose first digit is 0 (top-k without top-p on a confident row: deviation
-// 8, top-k 50 73 us, with top-p 0.95 24), nor where more words than SAMP_LIST share the digit (a nucleus of 0.9 alone 79).
+// 8, top-k 50 73 us, with top-p 0.95 24), nor where more words than SAMP_LIST share the digit (a nucleus of 0.9 alone 79; these
+// three in clusters of eight).
+#include <atomic>
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -339,6 +342,7 @@ sample_rows_kernel(const SampleParams p) {
   row.n = max(0, min(p.slice, V - row.base));
   row.w = SMEM ? slice_smem : p.work + static_cast<size_t>(row_id) * V + min(row.base, V);
   float* wf = reinterpret_cast<float*>(row.w);
+  uint64_t st = p.rng_state[row_id];          // on its way long before the draw
 
   // ---- penalised copy of the slice ----
   const float* xs = x + min(row.base, V);
@@ -407,8 +411,11 @@ sample_rows_kernel(const SampleParams p) {
     if (lane == 0) s.vmax = mx;
   }
   cl.sync();
-  mx = s.vmax;
-  for (int r = 0; r < nr; ++r) mx = fmaxf(mx, *cl.map_shared_rank(&s.vmax, r));
+  // a lane per CTA: one trip to the others' memory instead of eight in a row
+  mx = *cl.map_shared_rank(&s.vmax, lane < nr ? lane : rank);
+#pragma unroll
+  for (int o = SAMP_CLUSTER / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  mx = __shfl_sync(0xffffffffu, mx, 0);
   // fixed-point weights, their total and the first level's histogram
   unsigned long long local = 0;
   const float inv_t = 1.0f / p.temperature;
@@ -448,15 +455,16 @@ sample_rows_kernel(const SampleParams p) {
   }
   combine<SMEM>(cl, s, 0);
   int buf = 1;
-  unsigned long long z = 0;
-  for (int r = 0; r < nr; ++r) z += *cl.map_shared_rank(&s.total, r);
+  unsigned long long z = lane < nr ? *cl.map_shared_rank(&s.total, lane) : 0;
+#pragma unroll
+  for (int o = SAMP_CLUSTER / 2; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+  z = __shfl_sync(0xffffffffu, z, 0);
   if (t < SAMP_BINS) { s.top_cnt[t] = s.tot_cnt[t]; s.top_sum[t] = s.tot_sum[t]; }
   // kept set: first min(top_k, V) ranks, cut where the cumulative probability reaches top_p
   const unsigned long long n_all = static_cast<unsigned long long>(V);
   const unsigned long long limit = (p.top_k > 0 && p.top_k < V) ? static_cast<unsigned long long>(p.top_k) : n_all;
   const bool cut = limit < n_all || p.top_p < 1.0f;
   const unsigned long long tp = p.top_p < 1.0f ? nucleus_target(p.top_p, z) : ~0ull;   // ~0: only the count stops the walk
-  uint64_t st = p.rng_state[row_id];
   {
     // the first level of the first walk: the cut's, or the draw's when everything is kept
     uint64_t peek = st;
@@ -694,6 +702,54 @@ static int launch_greedy(SampleParams p, int rows, cudaStream_t stream) {
   return launch_clusters(greedy_rows_kernel<SAMP_THREADS>, p, rows, cluster, SAMP_THREADS, 0, stream);
 }
 
+// Clusters of `c` CTAs of the sampler that the current device holds at once; asked for once per device and size.
+static int sample_clusters(int c) {
+  static std::atomic<int> known[64][SAMP_CLUSTER + 1] = {};
+  int device = 0;
+  const bool keep = cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < 64;
+  if (keep) {
+    const int k = known[device][c].load(std::memory_order_relaxed);
+    if (k > 0) return k;
+  }
+  auto kern = sample_rows_kernel<true>;
+  int n = num_sms() / c;
+  if (c > 1) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c);
+    cfg.blockDim = dim3(SAMP_THREADS);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = c;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = num_sms() * 3 / 4 / c; }
+  }
+  if (n < 1) n = 1;
+  if (keep) known[device][c].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// CTAs of a row. Eight while the clusters of all rows run at once; a cluster lies in one part of the GPU, which holds 15 of eight, 33
+// of four, 74 of two. Beyond that the size whose waves take least: a wave is about FIXED + the words of a slice, in half cycles.
+// 128256 logits, us, clusters of eight / four: 15 rows 16.5 / 18.5, 16 rows 25.9 / 18.5, 64 rows 73.8 / 55.5; 32000, 64 rows, eight / four
+// / two / one: 47.2 / 22.6 / 14.4 / 16.4.
+static int sample_cluster(int V, int rows) {
+  if (V <= SAMP_SINGLE_MAX_V) return 1;
+  int best = SAMP_CLUSTER;
+  if (rows <= sample_clusters(SAMP_CLUSTER)) return best;
+  constexpr long long FIXED[4] = {20000, 25000, 27000, 28000};       // of one, two, four and eight CTAs
+  long long least = 0;
+  for (int k = 3, c = SAMP_CLUSTER; k >= 0; --k, c >>= 1) {
+    const int words = (V + c - 1) / c, held = sample_clusters(c);
+    if (c < SAMP_CLUSTER && (words + 3) / 4 * 4 > SAMP_SLICE_WORDS) break;
+    const long long cost = static_cast<long long>((rows + held - 1) / held) * (FIXED[k] + words);
+    if (c == SAMP_CLUSTER || cost < least) { least = cost; best = c; }
+  }
+  return best;
+}
+
 template <bool SMEM>
 static int launch_sample(const SampleParams& p, int rows, int cluster, cudaStream_t stream) {
   auto kern = sample_rows_kernel<SMEM>;
@@ -722,7 +778,7 @@ extern "C" int sb_sample_rows(const float* logits, int ld, int rows, int V, floa
   p.gen_stride = gen_stride; p.step = step; p.work = work;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (temperature <= 0.f) return launch_greedy(p, rows, st);
-  const int cluster = V <= SAMP_SINGLE_MAX_V ? 1 : SAMP_CLUSTER;
+  const int cluster = sample_cluster(V, rows);
   p.slice = ((V + cluster - 1) / cluster + 3) / 4 * 4;
   return p.slice <= SAMP_SLICE_WORDS ? launch_sample<true>(p, rows, cluster, st) : launch_sample<false>(p, rows, cluster, st);
 }

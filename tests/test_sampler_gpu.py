@@ -216,3 +216,23 @@ def test_short_lists_and_walks_take_the_same_element(vocab, ties, top_k, top_p):
         z = kept * w
         t = min(int(SamplerRng(7 + b).next_uniform() * float(z)), z - 1)
         assert got[b] == int(ids[b, t // w])
+
+
+@pytest.mark.parametrize("vocab", [8193, 32000, 100003, 128256])
+@pytest.mark.parametrize("rows", [16, 34, 64, 150])
+@pytest.mark.parametrize("params", [SamplingParams(temperature=0.8, top_k=50, top_p=0.95), SamplingParams(temperature=1.1),
+                                    SamplingParams(temperature=0.7, top_k=700, top_p=0.9, repetition_penalty=1.3)])
+def test_batches_draw_what_their_rows_draw_alone(vocab, rows, params):
+    """A row's CTAs are fewer in a batch whose clusters of eight do not all run at once. Sums are of integers, so a row of the batch
+    draws the same token, and leaves the same generator, as alone on a cluster of eight."""
+    lg = _logits(rows, vocab, vocab + rows).cuda()
+    hist = torch.randint(0, vocab, (rows, 40), generator=torch.Generator().manual_seed(rows))
+    seeds = list(range(50, 50 + rows))
+    batch = DeviceSampler(params, rows, vocab, seeds, "cuda", history_len=64)
+    batch.set_history(hist)
+    got = batch.sample(lg).tolist()
+    for b in range(0, rows, 7):
+        one = DeviceSampler(params, 1, vocab, seeds[b:b + 1], "cuda", history_len=64)
+        one.set_history(hist[b:b + 1])
+        assert one.sample(lg[b:b + 1]).tolist() == got[b:b + 1]
+        assert torch.equal(one.state, batch.state[b:b + 1])
