@@ -9,10 +9,10 @@
 //
 //   warp 0   TMA producer (both CTAs; bytes of both are counted on the leader's "full" barrier)
 //   warp 1   MMA issuer (leader CTA only); the same warp allocates TMEM in both CTAs
-//   warp 2-9 epilogue (both CTAs; "accumulator drained" arrives on the leader's barrier). The plain epilogue
-//            (no SwiGLU, no split parts) does not store from registers: a warp converts 32 rows x 64 columns, lays
-//            them out as 128-byte swizzled rows in its own 4 KB of shared memory and hands them to a TMA tensor
+//   warp 2-9 epilogue (both CTAs; "accumulator drained" arrives on the leader's barrier). The plain and the SwiGLU
+//            forward epilogue do not store from registers: a warp converts 32 rows x 64 columns, lays them out as 128-byte swizzled rows in its own 4 KB of shared memory and hands them to a TMA tensor
 //            store, so the output leaves the SM as full 128-byte lines and edge tiles are clipped by the hardware
+//   warp 10-13 copiers (both CTAs): shards of a distributed product, or int8 matrices of later products to bf16
 // Stage release and "accumulator ready" are tcgen05.commit arrivals delivered to both CTAs.
 // No TMA multicast is used.
 #include <cstdlib>
@@ -34,7 +34,7 @@ constexpr int BN = 256;        // columns of the pair's tile
 constexpr int BNH = BN / 2;    // columns of B staged per CTA
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int THREADS = 448;        // warp 0 TMA, 1 MMA, 2-9 epilogue, 10-13 all-gather copiers (idle otherwise)
+constexpr int THREADS = 448;        // warp 0 TMA, 1 MMA, 2-9 epilogue, 10-13 copiers
 constexpr int COPY_WARPS = 4;
 constexpr int CP_UNROLL = 8;   // 16-byte peer loads in flight per copier thread
 constexpr int GROUP_M = 8;           // row tiles (of 256 rows) per raster group
@@ -48,6 +48,20 @@ constexpr int TMEM_COLS = 2 * BN;                // two accumulators
 constexpr int EPI_WARPS = 8;
 constexpr int EPI_STAGE_BYTES = 32 * 128;        // one warp's 32 rows x 64 bf16 columns, 128-byte swizzled rows
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * EPI_STAGE_BYTES + 1024 + 256;
+
+// An int8 matrix [K, N] with column scales that the copier warps write as bf16 beside the product; N % 16 == 0. The expansion is bound
+// by memory (3 bytes a code, 56 us for 117 M codes alone) and the product by the tensor cores, so the two hide each other: the four
+// warps of an SM keep 16 KB of codes in flight, about 3 TB/s with what they write. 2048 x 4096 x 28672 with 101 M codes: 365 us in turn,
+// 350 beside, at the power cap in both; 2048 x 14336 x 4096 with 117 M 224 / 199. Nothing waits for a copier but the launch's end.
+constexpr int MAX_WIDEN = 3;
+constexpr int WIDEN_FLY = 8;       // 16-byte loads in flight per thread
+struct Widen {
+  const uint4* q;
+  const float* scale;
+  uint4* w;
+  int K, N;
+  int rows;                        // of a unit: 512 columns wide
+};
 
 struct TmapSet {
   CUtensorMap m[MAXW];   // reduce-scatter: the slot of this rank in every owner's receive buffer
@@ -117,6 +131,8 @@ struct Params {
     uint64_t wait_ns;
     int team;        // CTAs that share one row block; teams reduce different blocks at the same time
   } rs;
+  int n_widen;
+  Widen widen[MAX_WIDEN];
 };
 
 __device__ __forceinline__ void p_st_release_sys(uint32_t* ptr, uint32_t v) {
@@ -146,6 +162,39 @@ __device__ bool p_wait_flag(const uint32_t* flag, uint32_t epoch, uint64_t limit
     }
   }
   return true;
+}
+
+// Rows [k0, k0 + job.rows) of sixteen columns: the arithmetic of dequant_vec8_kernel (decode.cu), the same bits.
+__device__ __forceinline__ void widen_unit(const Widen& job, int k0, int c, int n16) {
+  float s[16];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 f = __ldg(reinterpret_cast<const float4*>(job.scale) + c * 4 + i);
+    s[4 * i] = f.x; s[4 * i + 1] = f.y; s[4 * i + 2] = f.z; s[4 * i + 3] = f.w;
+  }
+  const int k1 = min(job.K, k0 + job.rows);
+  for (; k0 < k1; k0 += WIDEN_FLY) {
+    uint4 q[WIDEN_FLY];
+#pragma unroll
+    for (int r = 0; r < WIDEN_FLY; ++r)
+      if (k0 + r < k1) q[r] = __ldcs(job.q + static_cast<size_t>(k0 + r) * n16 + c);
+#pragma unroll
+    for (int r = 0; r < WIDEN_FLY; ++r) {
+      if (k0 + r >= k1) break;
+      const uint32_t b[4] = {q[r].x ^ 0x80808080u, q[r].y ^ 0x80808080u, q[r].z ^ 0x80808080u, q[r].w ^ 0x80808080u};
+      uint32_t o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t word = b[i >> 1];
+        const int e = (i & 1) * 2;
+        o[i] = pack_bf16x2((__uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540 + e)) - 8388736.0f) * s[2 * i],
+                           (__uint_as_float(__byte_perm(word, 0x4B000000u, 0x7541 + e)) - 8388736.0f) * s[2 * i + 1]);
+      }
+      uint4* w = job.w + (static_cast<size_t>(k0 + r) * n16 + c) * 2;
+      w[0] = make_uint4(o[0], o[1], o[2], o[3]);
+      w[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+  }
 }
 
 template <bool A_MN, bool B_MN>
@@ -307,6 +356,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else if (warp >= 10) {
     // -------------------------------- copiers (both CTAs) ---------------------------------
+    // The matrices of later products: units of job.rows x 512 columns, dealt to the copier warps of the grid in turn.
+    long long u = static_cast<long long>(blockIdx.x) * COPY_WARPS + warp - 10;
+    for (int j = 0; j < p.n_widen; ++j) {
+      const Widen& job = p.widen[j];
+      const int n16 = job.N >> 4, cols = (n16 + 31) >> 5;
+      const long long units = static_cast<long long>(cols) * ((job.K + job.rows - 1) / job.rows);
+      for (; u < units; u += gridDim.x * COPY_WARPS) {
+        const int rb = static_cast<int>(u / cols), c = static_cast<int>(u - static_cast<long long>(rb) * cols) * 32 + lane;
+        if (c < n16) widen_unit(job, rb * job.rows, c, n16);
+      }
+      u -= units;
+    }
     if (ag && !A_MN && (p.ag.W > 1 || p.ag.copy_own)) {
       // Push my shard to every peer, one destination after the other (rank-1 first: it needs my rows first), all
       // CTAs sharing each destination's copy. One system fence per warp and destination; the warp that completes a
@@ -789,9 +850,12 @@ using namespace sb;
 // residual, no balanced schedule on that path.
 extern "C" size_t sb_gemm_pair_workspace_floats() { return static_cast<size_t>(num_sms() / 2) * 3 * 256 * 256; }
 
-extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda,
-                                 int ldb, int ldc, int ldr, int a_mn, int b_mn, void* workspace, void* act, int ld_act,
-                                 int ff, const void* gu, int ld_gu, int* status, void* stream_) {
+// `n_widen` up to 3 (0: none): int8 matrices q[i] [K, N] with fp32 column scales, contiguous, that the launch also writes as
+// bf16 to w[i]; kn: K and N of each, N % 16 == 0, q, scale and w 16-byte aligned.
+extern "C" int sb_gemm_pair_widen_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda,
+                                       int ldb, int ldc, int ldr, int a_mn, int b_mn, void* workspace, void* act, int ld_act,
+                                       int ff, const void* gu, int ld_gu, int n_widen, const void* const* q,
+                                       const void* const* scale, void* const* w, const int* kn, int* status, void* stream_) {
   using namespace sb::pair;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || (ldc & 7) || (R && (ldr & 7)) || (!C && !ff)) return SB_ERR_ARG;
@@ -816,6 +880,19 @@ extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const vo
     if (rc) return rc;
   }
   Params p;
+  p.n_widen = n_widen;
+  if (n_widen < 0 || n_widen > MAX_WIDEN) return SB_ERR_ARG;
+  for (int i = 0; i < n_widen; ++i) {
+    if (!q[i] || !scale[i] || !w[i] || kn[2 * i] <= 0 || kn[2 * i + 1] <= 0 || (kn[2 * i + 1] & 15)) return SB_ERR_ARG;
+    if ((reinterpret_cast<uintptr_t>(q[i]) | reinterpret_cast<uintptr_t>(scale[i]) | reinterpret_cast<uintptr_t>(w[i])) & 15)
+      return SB_ERR_ALIGN;
+    p.widen[i] = {static_cast<const uint4*>(q[i]), static_cast<const float*>(scale[i]), static_cast<uint4*>(w[i]), kn[2 * i],
+                  kn[2 * i + 1], 64};
+    // enough units that the last round of the warps is a small part, unless that takes fewer rows than a thread has in flight
+    const long long cols = (kn[2 * i + 1] + 511) / 512;
+    while (p.widen[i].rows > WIDEN_FLY && cols * ((kn[2 * i] + p.widen[i].rows - 1) / p.widen[i].rows) < 8ll * num_sms() * COPY_WARPS)
+      p.widen[i].rows /= 2;
+  }
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.R = R; p.ldr = ldr; p.status = status;
   p.ff = ff;
   if (gu) {
@@ -864,6 +941,13 @@ extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const vo
   return 0;
 }
 
+extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda,
+                                 int ldb, int ldc, int ldr, int a_mn, int b_mn, void* workspace, void* act, int ld_act,
+                                 int ff, const void* gu, int ld_gu, int* status, void* stream_) {
+  return sb_gemm_pair_widen_bf16(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, workspace, act, ld_act, ff, gu, ld_gu, 0,
+                                 nullptr, nullptr, nullptr, nullptr, status, stream_);
+}
+
 // All-gather -> GEMM on CTA pairs: C[M,N] = gather(A shards)[M,K] * op(B) (+ R). a_ptrs[s]: rank s's shard
 // [M/W, lda] (only entry `rank`, the local one, is read); stage_ptrs[r]: rank r's landing buffer [M, ld_stage]
 // (peer-mapped: every rank pushes its shard into every peer's); flag_ptrs[r]: this call site's flag slot on rank r;
@@ -890,6 +974,7 @@ extern "C" int sb_gemm_pair_ag_bf16(void* const* a_ptrs, const void* B, void* C,
   else rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, BK);
   if (rc) return rc;
   Params p;
+  p.n_widen = 0;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.R = R; p.ldr = ldr; p.status = status;
   p.ff = 0; p.gu = nullptr; p.ld_gu = 0;
   p.partials = nullptr;
@@ -957,6 +1042,7 @@ extern "C" int sb_gemm_pair_rs_bf16(const void* A, const void* B, void* const* p
     if (rc) return rc;
   }
   Params p;
+  p.n_widen = 0;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldp; p.R = nullptr; p.ldr = 0; p.status = status;
   p.ff = 0; p.gu = nullptr; p.ld_gu = 0;
   p.partials = nullptr;

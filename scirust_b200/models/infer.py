@@ -105,6 +105,50 @@ class PagedKVCache:
         self.table_host[seq].zero_()
 
 
+class _WidenAhead:
+    """The int8 matrices of one prefill in the order of their use. A long prompt's products take them as bf16, and expanding each before
+    its product leaves the tensor cores idle for as long as memory takes. Instead the launch of a product also expands the next matrices,
+    in warps that it has to spare, up to two codes for each of its own weights: the down product takes the next layer's gate/up
+    matrix, the gate/up product down and the next qkv and output matrices. Us at 2048 rows, d 4096, ff 14336, expanded before / beside:
+    gate/up with down 383 / 336, down with the next gate/up 224 / 199, qkv with the output matrix 82.8 / 78.4; more gains less than the
+    next product would with it (qkv with down, 2.3 codes for one, 12 us, gate/up 47) or loses (output product with gate/up, 7 codes, 108
+    / 114). At 1024 rows gate/up with three 219 / 202, down with gate/up 139 / 129; d 1024 at 2048 rows gate/up with three 43.5 / 34.4.
+    Up to three matrices more than before are in memory; one that does not fit there is expanded before its product."""
+
+    AHEAD = 3
+
+    def __init__(self, layers, rows):
+        self.rows = rows
+        self.order = [l[k] for l in layers for k in ("wqkv", "wo", "wgu", "wd")] if rows >= 1024 else []
+        self.at = 0
+        self.wide = {}                 # position in the order -> bf16 matrix
+
+    def product(self, w):
+        """The next product's matrix (expanded, or as it is) and what its launch is to expand, as keyword arguments."""
+        if not self.order:
+            return w, {}
+        w = self.wide.pop(self.at, w)
+        self.at += 1
+        K, N = w.shape
+        if not G.widens_beside(self.rows, N, K):
+            return w, {}
+        room, jobs = 2 * K * N, []
+        for i in range(self.at, min(self.at + self.AHEAD, len(self.order))):
+            q = self.order[i]
+            if i in self.wide:
+                continue
+            if not isinstance(q, D.QuantWeight) or not q.widenable() or q.q.numel() > room:
+                break
+            try:
+                out = torch.empty(q.shape, dtype=torch.bfloat16, device=q.q.device)
+            except torch.OutOfMemoryError:
+                break
+            room -= q.q.numel()
+            self.wide[i] = out
+            jobs.append((q.q, q.scale, out))
+        return w, {"widen": jobs} if jobs else {}
+
+
 class InferenceEngine:
     def __init__(self, model: GQADecoder, quant: str | None = None, max_batch: int = 1, max_seq: int = 4096,
                  page: int = 64, use_graph: bool = True):
@@ -144,16 +188,17 @@ class InferenceEngine:
         self.head_t = prep(model.head_weight().detach().t().contiguous())
 
     # ------------------------------------------------------------------ linear dispatch
-    def _proj_out(self, a, w, x, swiglu=False, site="attn"):
+    def _proj_out(self, a, w, x, swiglu=False, site="attn", widen=()):
         """x + f(a) @ w: the attention-output and MLP-down products (row-parallel under tensor
-        parallelism, where a subclass adds the all-reduce). ``swiglu``: a is a fused [gate | up]."""
+        parallelism, where a subclass adds the all-reduce). ``swiglu``: a is a fused [gate | up]. ``widen``: as in ``_linear``."""
         if a.shape[0] <= D.gemv_max_rows(w):
             return D.gemv(a, w, residual=x, swiglu=swiglu)
         if swiglu:
             a = ops.swiglu_fwd(a)
-        return self._linear(a, w, residual=x)
+        return self._linear(a, w, residual=x, widen=widen)
 
-    def _linear(self, x, w, residual=None):
+    def _linear(self, x, w, residual=None, widen=()):
+        """``widen``: int8 matrices of later products that this one's launch expands (``_WidenAhead``)."""
         M = x.shape[0]
         if M <= D.gemv_max_rows(w):
             return D.gemv(x, w, residual=residual)
@@ -168,9 +213,9 @@ class InferenceEngine:
             if M < 1024 and w.q.shape[1] % 16 == 0:
                 return D.matmul_int8(x, w, residual=residual)
             w = w.dequantize()
-        return ops.matmul_nn(x, w, residual=residual)
+        return G.matmul_nn_beside(x, w, residual, widen) if widen else ops.matmul_nn(x, w, residual=residual)
 
-    def _gated(self, x, w):
+    def _gated(self, x, w, widen=()):
         """silu(gate) * up of ``[gate | up] = x @ w`` in one launch, or None where that is not how ``_linear`` takes the product (by
         1024 rows int8 weights are expanded whatever their shape)."""
         M, (K, N) = x.shape[0], w.shape
@@ -180,7 +225,7 @@ class InferenceEngine:
             if M < 1024 and N % 16 == 0:
                 return None
             w = w.dequantize()
-        return ops.matmul_nn_swiglu_act(x, w)
+        return ops.matmul_nn_swiglu_act(x, w, widen)
 
     # ------------------------------------------------------------------ prefill
     def prefill(self, tokens: torch.Tensor):
@@ -198,19 +243,26 @@ class InferenceEngine:
         seq_of = torch.arange(B, dtype=torch.int32, device=self.dev).repeat_interleave(P)
         pos = torch.arange(P, dtype=torch.int32, device=self.dev).repeat(B)
         x = ops.embed_fwd(self.embed, tok.reshape(-1))
+        cls = type(self)                 # a subclass with products of its own (tensor parallelism) expands before each
+        own = (cls._linear, cls._proj_out, cls._gated) == (InferenceEngine._linear, InferenceEngine._proj_out, InferenceEngine._gated)
+        product = _WidenAhead(self.layers if own and x.is_cuda else [], B * P).product
         for li, l in enumerate(self.layers):
             h, _ = ops.rmsnorm_fwd(x, l["rms1"], cfg.eps, want_inv=False)
-            qkv = self._linear(h, l["wqkv"])
+            w, kw = product(l["wqkv"])
+            qkv = self._linear(h, w, **kw)
             D.rope_kv_append(qkv, H, Hkv, dh, self.cos, self.sin, cache.pools[li], cache.block_table, cache.page, seq_of, pos)
             a, _ = att.attention_fwd(qkv, B, P, H, Hkv, dh, causal=True, want_lse=False)
-            x = self._proj_out(a, l["wo"], x, site="attn")
+            w, kw = product(l["wo"])
+            x = self._proj_out(a, w, x, site="attn", **kw)
             h, _ = ops.rmsnorm_fwd(x, l["rms2"], cfg.eps, want_inv=False)
-            act = self._gated(h, l["wgu"])
-            if act is not None:
-                x = self._proj_out(act, l["wd"], x, site="mlp")
-            else:
-                gu = self._linear(h, l["wgu"])
-                x = self._proj_out(gu, l["wd"], x, swiglu=True, site="mlp")
+            w, kw = product(l["wgu"])
+            gu = self._gated(h, w, **kw)             # silu(gate) * up
+            fused = gu is not None
+            if not fused:
+                gu = self._linear(h, w, **kw)
+            w, kw = product(l["wd"])
+            x = self._proj_out(gu, w, x, swiglu=not fused, site="mlp", **kw)
+        w = None
         last = x.view(B, P, -1)[:, -1, :].contiguous()
         logits = self.logits[:B]
         self._head(last, logits, rms_weight=self.rms_final)

@@ -79,6 +79,11 @@ class QuantWeight:
     def shape(self):
         return self.q.shape
 
+    def widenable(self) -> bool:
+        """Whether a product's launch can expand it (``ops.gemm.matmul_nn_beside``)."""
+        return (self.q.is_cuda and self.q.shape[1] % 16 == 0 and self.q.is_contiguous() and self.scale.is_contiguous()
+                and self.q.data_ptr() % 16 == 0 and self.scale.data_ptr() % 16 == 0)
+
     def dequantize(self) -> torch.Tensor:
         if not self.q.is_cuda:
             return (self.q.float() * self.scale[None, :]).to(BF)

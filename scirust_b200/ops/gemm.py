@@ -13,6 +13,7 @@ be tested without a GPU; CUDA tensors always run the native kernel.
 """
 from __future__ import annotations
 
+import ctypes
 import os
 
 import torch
@@ -132,7 +133,14 @@ class _Bias:
         return 0
 
 
-def _gemm(a, b, M, N, K, a_mn, b_mn, out, residual, splits, bn, bias=None):
+def _widen_args(widen):
+    """``[(q, scale, w), ...]`` as the arguments of ``sb_gemm_pair_widen_bf16``: count, three tables of pointers, sizes."""
+    ptrs = ctypes.c_void_p * len(widen)
+    sizes = [n for q, _, _ in widen for n in q.shape]
+    return (len(widen), *(ptrs(*(job[i].data_ptr() for job in widen)) for i in range(3)), (ctypes.c_int * len(sizes))(*sizes))
+
+
+def _gemm(a, b, M, N, K, a_mn, b_mn, out, residual, splits, bn, bias=None, widen=()):
     global launch_count
     if bias is not None:
         if residual is not None:
@@ -155,9 +163,13 @@ def _gemm(a, b, M, N, K, a_mn, b_mn, out, residual, splits, bn, bias=None):
         pair_tiles = ((M + 255) // 256) * ((N + 255) // 256)
         pairs = num_sms(a.device) // 2
         ws = _workspace(pairs * 3 * 256 * 256, a.device) if _use_balanced(pair_tiles, pairs, K) else None
-        _lib.call("sb_gemm_pair_bf16", a.data_ptr(), b.data_ptr(), out.data_ptr(), residual.data_ptr() if residual is not None else None, M, N, K,
-                  a.stride(0), b.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
-                  int(a_mn), int(b_mn), _lib.ptr(ws), None, 0, 0, None, 0, st.data_ptr(), _lib.stream())
+        args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), residual.data_ptr() if residual is not None else None, M, N, K,
+                a.stride(0), b.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
+                int(a_mn), int(b_mn), _lib.ptr(ws), None, 0, 0, None, 0)
+        if widen:
+            _lib.call("sb_gemm_pair_widen_bf16", *args, *_widen_args(widen), st.data_ptr(), _lib.stream())
+        else:
+            _lib.call("sb_gemm_pair_bf16", *args, st.data_ptr(), _lib.stream())
         launch_count += 1
         return out
     if bn is None:
@@ -202,6 +214,22 @@ def matmul_nn(x, w, residual=None, out=None, splits=None, bn=None, bias=None):
     return _gemm(x, w, M, N, K, False, True, out, residual, splits, bn, bias)
 
 
+def widens_beside(M: int, N: int, K: int) -> bool:
+    """Whether ``matmul_nn_beside`` and ``matmul_nn_swiglu_act`` of these sizes take int8 matrices to widen (the CTA-pair kernel)."""
+    return _use_pair(M, N, K, None, None)
+
+
+def matmul_nn_beside(x, w, residual=None, widen=()):
+    """``matmul_nn``, and in the same launch the bf16 form of int8 matrices that later products need: ``widen`` holds up to three
+    ``(q int8 [K, N], scale fp32 [N], out bf16 [K, N])``, contiguous, with N a multiple of 16. Only where ``widens_beside``."""
+    M, K = x.shape
+    if K != w.shape[0]:
+        raise ValueError(f"matmul_nn_beside: inner dims differ ({K} vs {w.shape[0]})")
+    if widen and not widens_beside(M, w.shape[1], K):
+        raise ValueError("matmul_nn_beside: a product of this size widens nothing")
+    return _gemm(x, w, M, w.shape[1], K, False, True, None, residual, None, None, widen=widen)
+
+
 def swiglu_in_epilogue(M: int, K: int, ff: int) -> bool:
     """Whether the gate/up product of ``M`` rows writes ``silu(gate) * up`` itself. The epilogue takes as long as the main loop over about 1024
     rows of k, and that of the last tile of every CTA pair is not hidden, so it wants long k and at least four waves of tiles (256 x 128
@@ -216,16 +244,20 @@ def swiglu_in_epilogue(M: int, K: int, ff: int) -> bool:
     return K >= 1024 and ((M + 255) // 256) * ((ff + 127) // 128) >= 4 * (num_sms() // 2)
 
 
-def _swiglu_product(x, wgu, gu, act):
+def _swiglu_product(x, wgu, gu, act, widen=()):
     """One launch of the CTA-pair kernel: each CTA of a pair stages one half, gate columns and the matching up columns."""
     global launch_count
     M, K = x.shape
     N = wgu.shape[1]
     _check2d(x, "x")
     _check2d(wgu, "wgu")
-    _lib.call("sb_gemm_pair_bf16", x.data_ptr(), wgu.data_ptr(), _lib.ptr(gu), None, M, N, K, x.stride(0), wgu.stride(0),
-              gu.stride(0) if gu is not None else 0, 0, 0, 1, None, act.data_ptr(), act.stride(0), N // 2, None, 0,
-              _lib.status_word(x.device).data_ptr(), _lib.stream())
+    args = (x.data_ptr(), wgu.data_ptr(), _lib.ptr(gu), None, M, N, K, x.stride(0), wgu.stride(0),
+            gu.stride(0) if gu is not None else 0, 0, 0, 1, None, act.data_ptr(), act.stride(0), N // 2, None, 0)
+    st = _lib.status_word(x.device).data_ptr()
+    if widen:
+        _lib.call("sb_gemm_pair_widen_bf16", *args, *_widen_args(widen), st, _lib.stream())
+    else:
+        _lib.call("sb_gemm_pair_bf16", *args, st, _lib.stream())
     launch_count += 1
 
 
@@ -250,17 +282,18 @@ def matmul_nn_swiglu(x, wgu, out=None, act=None):
     return out, act
 
 
-def matmul_nn_swiglu_act(x, wgu):
-    """``matmul_nn_swiglu`` without the gate/up product: ``act`` alone, the same bits, for passes without a backward."""
+def matmul_nn_swiglu_act(x, wgu, widen=()):
+    """``matmul_nn_swiglu`` without the gate/up product: ``act`` alone, the same bits, for passes without a backward. ``widen`` as in
+    ``matmul_nn_beside``, where ``swiglu_in_epilogue``."""
     M, K = x.shape
     K2, N = wgu.shape
     if K != K2 or N % 2:
         raise ValueError("matmul_nn_swiglu_act: shape mismatch")
     if not (x.is_cuda and swiglu_in_epilogue(M, K, N // 2)):
         from . import basic
-        return basic.swiglu_fwd(matmul_nn(x, wgu))
+        return basic.swiglu_fwd(matmul_nn_beside(x, wgu, widen=widen) if widen else matmul_nn(x, wgu))
     act = _lib.empty((M, N // 2), torch.bfloat16, x.device)
-    _swiglu_product(x, wgu, None, act)
+    _swiglu_product(x, wgu, None, act, widen)
     return act
 
 

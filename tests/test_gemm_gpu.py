@@ -254,3 +254,65 @@ def test_swiglu_backward_epilogue_is_bitwise_the_unfused_path(M, d, ff, monkeypa
     monkeypatch.setattr(gemm, "BALANCED", False)
     ref = basic.swiglu_bwd(gu, ops.matmul_nt(dy, wd))
     assert torch.equal(dgu, ref)
+
+
+@pytest.mark.parametrize("M,N,K,form", [(300, 520, 128, "plain"), (1100, 2816, 1024, "residual"), (2560, 2304, 4096, "balanced"),
+                                        (1100, 5632, 1024, "swiglu")])
+def test_product_widens_int8_matrices_beside_itself(M, N, K, form, monkeypatch):
+    """The product's bits are those without the expansion, the matrices' those of ``dequantize``; ragged units of rows and columns, few
+    CTAs and all of them, and nothing is written behind a matrix."""
+    from scirust_b200.ops import decode as D, gemm
+    monkeypatch.setattr(gemm, "PAIR_MODE", "1")
+    monkeypatch.setattr(gemm, "FUSE_SWIGLU", form == "swiglu")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    sizes = [(13, 16), (2056, 1040), (70, 528)]
+    jobs, want, tails = [], [], []
+    for k, n in sizes:
+        q = torch.randint(-128, 128, (k, n), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+        scale = torch.rand(n, generator=g, device="cuda") * 0.1
+        buf = torch.full((k * n + 512,), 7.0, dtype=torch.bfloat16, device="cuda")
+        jobs.append((q, scale, buf[:k * n].view(k, n)))
+        want.append(D.QuantWeight(q, scale).dequantize())
+        tails.append(buf[k * n:])
+    x, w = _mk((M, K), 1), _mk((K, N), 2)
+    res = _mk((M, N), 3) if form == "residual" else None
+    if form == "swiglu":
+        alone, y = ops.matmul_nn_swiglu_act(x, w), ops.matmul_nn_swiglu_act(x, w, widen=jobs)
+    else:
+        alone, y = ops.matmul_nn(x, w, residual=res), gemm.matmul_nn_beside(x, w, res, jobs)
+    _lib.check_status()
+    assert torch.equal(alone, y)
+    for (_, _, got), right, tail in zip(jobs, want, tails):
+        assert torch.equal(got, right)
+        assert bool((tail == 7.0).all())
+    with pytest.raises((ValueError, RuntimeError)):            # a width that the expansion does not take
+        gemm.matmul_nn_beside(x, w, None, [(jobs[0][0].view(16, 13), jobs[0][1][:13].clone(), jobs[0][2].view(16, 13))])
+
+
+@pytest.mark.parametrize("batch,seq,ff", [(1, 1100, 2816), (3, 683, 2824)])
+def test_prefill_that_widens_ahead(batch, seq, ff):
+    """Logits and cache as from an engine that expands each matrix before its product (ff 2824: two matrices are not wide enough by
+    whole 16-byte words and are left to that)."""
+    from scirust_b200.models.infer import InferenceEngine, _WidenAhead
+    from scirust_b200.models.sciagent import GQADecoder, SciAgentConfig
+
+    class Before(InferenceEngine):
+        def _linear(self, x, w, residual=None):
+            return InferenceEngine._linear(self, x, w, residual)
+
+        def _proj_out(self, a, w, x, swiglu=False, site="attn"):
+            return InferenceEngine._linear(self, ops.swiglu_fwd(a) if swiglu else a, w, residual=x)
+
+    cfg = SciAgentConfig(512, 1024, 3, 16, 4, ff, 2048, 1e4)
+    model = GQADecoder(cfg, device="cuda", seed=3)
+    tokens = torch.randint(0, 512, (batch, seq), generator=torch.Generator().manual_seed(1)).cuda()
+    got = []
+    for cls in (InferenceEngine, Before):
+        eng = cls(model, quant="int8", max_batch=batch, max_seq=seq + 20)
+        got.append((eng.prefill(tokens).clone(), *eng.cache.pools))
+    _lib.check_status()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    plan = _WidenAhead(eng.layers, batch * seq)
+    taken = [len(plan.product(l[k])[1].get("widen", ())) for l in eng.layers for k in ("wqkv", "wo", "wgu", "wd")]
+    assert sum(taken) >= 3 and max(taken) <= 3
