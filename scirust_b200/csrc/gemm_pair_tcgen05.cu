@@ -10,8 +10,9 @@
 //   warp 0   TMA producer (both CTAs; bytes of both are counted on the leader's "full" barrier)
 //   warp 1   MMA issuer (leader CTA only); the same warp allocates TMEM in both CTAs
 //   warp 2-9 epilogue (both CTAs; "accumulator drained" arrives on the leader's barrier). The plain and the SwiGLU
-//            forward epilogue do not store from registers: a warp converts 32 rows x 64 columns, lays them out as 128-byte swizzled rows in its own 4 KB of shared memory and hands them to a TMA tensor
-//            store, so the output leaves the SM as full 128-byte lines and edge tiles are clipped by the hardware
+//            forward epilogue do not store from registers: a warp converts 32 rows x 64 columns, lays them out as
+//            128-byte swizzled rows in its own 4 KB of shared memory and hands them to a TMA tensor store, so the
+//            output leaves the SM as full 128-byte lines and edge tiles are clipped by the hardware
 //   warp 10-13 copiers (both CTAs): shards of a distributed product, or int8 matrices of later products to bf16
 // Stage release and "accumulator ready" are tcgen05.commit arrivals delivered to both CTAs.
 // No TMA multicast is used.
