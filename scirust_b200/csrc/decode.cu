@@ -1536,14 +1536,15 @@ decode_attn_kernel(const __grid_constant__ DecodeAttnParams p) {
 // producer warp fills with 128-byte-swizzled TMA boxes, and the 64-position tiles of all (sequence, kv head) jobs, laid
 // end to end, are dealt out in equal contiguous ranges, so lengths may be as ragged as they like. A job that ends up in
 // several CTAs is merged by the last of them to finish, pieces in tile order (a counter, no data atomics): the
-// summation tree depends on the lengths and the grid only.
+// summation tree depends on the lengths and the grid only. Three warps do all merging beside the stream.
 // Two groups of four consumer warps take the tiles of a piece in turn (one group alone needs 1650 cycles for a tile that
 // memory delivers in 1400); warp w of a group owns positions [16w, 16w + 16), as above.
 // Head dimension 128 only: at 64 the tiles are half the bytes for the same consumer work, and the kernel above is as fast
 // or faster up to 64 x 2048 positions (36.9 us against 37.1). Where the line lies at 128, with figures: ops/decode.py,
 // _stream_wins. 64 sequences of 1536-2048 positions, 8 kv heads: 108.5 us above (4.3 TB/s), 87.5 us here (5.4 TB/s).
 // ---------------------------------------------------------------------------
-constexpr int DST_THREADS = 288;         // warps 0-7 consume (two groups of four, every other tile each), warp 8 produces
+constexpr int DST_THREADS = 384;         // warps 0-7 consume (two groups of four, every other tile each), 8 produces, 9-11 finish
+constexpr int DST_FINISHERS = 96;        // a CTA's registers are given to warps by the four, so these three cost none
 constexpr int DST_STAGES_MAX = 6;        // one query head per kv head; sixteen leave room for four
 constexpr int DST_MAX_B = 1024;          // sequences whose tile offsets fit the shared prefix table
 
@@ -1566,7 +1567,7 @@ struct DstCfg {
   static constexpr int TILE_BYTES = DEC_TK * DH * 2;         // K or V of one tile
   // eight warps' partial results of the G live rows; what is left of shared memory holds stages
   static constexpr int merge_floats(int G) { return 8 * G * (DH + 2); }
-  static constexpr int fixed_bytes(int G) { return merge_floats(G) * 4 + (DST_MAX_B + 1) * 4 + 2 * DST_STAGES_MAX * 8 + 1024 + 64; }
+  static constexpr int fixed_bytes(int G) { return merge_floats(G) * 4 + (2 * DST_MAX_B + 1) * 4 + 2 * DST_STAGES_MAX * 8 + 1024 + 64; }
   static constexpr int stages(int G) {
     const int n = (226 * 1024 - fixed_bytes(G)) / (2 * TILE_BYTES);
     return n < DST_STAGES_MAX ? n : DST_STAGES_MAX;
@@ -1592,6 +1593,7 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
   float* sm_o = reinterpret_cast<float*>(empty + DST_STAGES_MAX);                   // [8 warps][G rows][DH]
   float* sm_ml = sm_o + 8 * G * DH;                                                 // [8 warps][G rows][2]
   int* prefix = reinterpret_cast<int*>(sm_ml + 8 * G * 2);                          // [B + 1] tiles before sequence b
+  int* lens = prefix + DST_MAX_B + 1;                                               // [B]
   __shared__ int s_last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -1605,14 +1607,15 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
   if (warp == 0) {
     int base = 0;
     for (int b0 = 0; b0 < p.B; b0 += 32) {
-      const int n = b0 + lane < p.B ? dst_tiles(p.seq_len[b0 + lane]) : 0;
+      const int len = b0 + lane < p.B ? p.seq_len[b0 + lane] : 0;
+      const int n = b0 + lane < p.B ? dst_tiles(len) : 0;
       int inc = n;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += v;
       }
-      if (b0 + lane < p.B) prefix[b0 + lane] = base + inc - n;
+      if (b0 + lane < p.B) { prefix[b0 + lane] = base + inc - n; lens[b0 + lane] = len; }
       base += __shfl_sync(0xffffffffu, inc, 31);
     }
     if (lane == 0) prefix[p.B] = base;
@@ -1633,75 +1636,74 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
     b_first = lo;
   }
 
+  // A piece: the tiles [t_beg, t_end) of a job that lie in this CTA's range. Consumers and finishers walk over the same pieces.
+  int b = b_first, len = 0, nt = 0, kvh = 0, t_beg = 0, t_end = 0;
+  long long s_job = 0;
+  auto locate = [&](long long u) {
+    long long s_b = 0;
+    for (;; ++b) {
+      len = lens[b];
+      nt = dst_tiles(len);
+      s_b = static_cast<long long>(prefix[b]) * Hkv;
+      if (u < s_b + static_cast<long long>(nt) * Hkv) break;
+    }
+    const int off = static_cast<int>(u - s_b);           // below nt * Hkv
+    kvh = off / nt;
+    s_job = s_b + static_cast<long long>(kvh) * nt;
+    t_beg = off - kvh * nt;
+    t_end = static_cast<int>(min(static_cast<long long>(nt), t_beg + (u1 - u)));
+  };
+
   if (warp == 8) {
     // ------------------------------ producer ------------------------------
     const int box = min(p.page, DEC_TK), nbx = DEC_TK / box;    // positions per TMA box, boxes per tile
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    int b = b_first;
-    for (long long u = u0; u < u1 && ok; ++b) {
-      const int len = p.seq_len[b], nt = dst_tiles(len);
-      const long long s_b = static_cast<long long>(prefix[b]) * Hkv;
-      const long long e_b = min(u1, s_b + static_cast<long long>(nt) * Hkv);
+    for (long long u = u0; u < u1; u += t_end - t_beg) {
+      locate(u);
       const int* table = p.block_table + static_cast<size_t>(b) * p.max_blocks;
-      for (; u < e_b && ok;) {
-        const int kvh = static_cast<int>((u - s_b) / nt);
-        const int t_beg = static_cast<int>((u - s_b) - static_cast<long long>(kvh) * nt);
-        const int t_end = static_cast<int>(min(static_cast<long long>(nt), t_beg + (e_b - u)));
-        int blk_of_lane = 0;                   // block of box (fetched + lane) of this job
-        int fetched = -1000000;
-        for (int t = t_beg; t < t_end && ok; ++t) {
-          if (!mbar_wait_warp(&empty[stage], phase ^ 1, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-          const int bx0 = t * nbx;
-          if (bx0 + nbx > fetched + 32) {      // nbx divides 32: a tile's boxes are fetched together
-            fetched = bx0;
-            const int pos = (fetched + lane) * box;
-            blk_of_lane = pos < len ? table[pos / p.page] : 0;
-          }
-          const int live = max(0, min(nbx, (len - t * DEC_TK + box - 1) / box));   // boxes with a position < len
-          uint8_t* kt = ring + stage * 2 * C::TILE_BYTES;
-          if (lane == 0) mbar_arrive_expect_tx(&full[stage], live * box * DH * 2 * 2);
-          for (int x = 0; x < live; ++x) {
-            const int blk = __shfl_sync(0xffffffffu, blk_of_lane, bx0 + x - fetched);
-            if (lane == 0) {
-              const int row = (blk * 2 * Hkv + kvh) * p.page + (bx0 + x) * box % p.page;
-              const int vrow = row + Hkv * p.page;
+      int blk_of_lane = 0;                   // block of box (fetched + lane) of this job
+      int fetched = -1000000;
+      for (int t = t_beg; t < t_end && ok; ++t) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1, p.status, ST_TIMEOUT_EMPTY)) { ok = false; break; }
+        const int bx0 = t * nbx;
+        if (bx0 + nbx > fetched + 32) {      // nbx divides 32: a tile's boxes are fetched together
+          fetched = bx0;
+          const int pos = (fetched + lane) * box;
+          blk_of_lane = pos < len ? table[pos / p.page] : 0;
+        }
+        const int live = max(0, min(nbx, (len - t * DEC_TK + box - 1) / box));   // boxes with a position < len
+        uint8_t* kt = ring + stage * 2 * C::TILE_BYTES;
+        if (lane == 0) mbar_arrive_expect_tx(&full[stage], live * box * DH * 2 * 2);
+        for (int x = 0; x < live; ++x) {
+          const int blk = __shfl_sync(0xffffffffu, blk_of_lane, bx0 + x - fetched);
+          if (lane == 0) {
+            const int row = (blk * 2 * Hkv + kvh) * p.page + (bx0 + x) * box % p.page;
+            const int vrow = row + Hkv * p.page;
 #pragma unroll
-              for (int c = 0; c < C::NCH; ++c) {
-                tma_load_2d(kt + c * (DEC_TK * 128) + x * box * 128, &tmap, &full[stage], c * 64, row);
-                tma_load_2d(kt + C::TILE_BYTES + c * (DEC_TK * 128) + x * box * 128, &tmap, &full[stage], c * 64, vrow);
-              }
+            for (int c = 0; c < C::NCH; ++c) {
+              tma_load_2d(kt + c * (DEC_TK * 128) + x * box * 128, &tmap, &full[stage], c * 64, row);
+              tma_load_2d(kt + C::TILE_BYTES + c * (DEC_TK * 128) + x * box * 128, &tmap, &full[stage], c * 64, vrow);
             }
           }
-          __syncwarp();
-          if (++stage == stages) { stage = 0; phase ^= 1; }
         }
-        u += t_end - t_beg;
+        __syncwarp();
+        if (++stage == stages) { stage = 0; phase ^= 1; }
       }
     }
-    return;
   }
 
-  // ------------------------------ consumers -----------------------------
-  const int quad = lane >> 2, tq = lane & 3, mi = lane >> 3;
-  const int group = warp >> 2, pw = warp & 3;      // group 0 takes the even tiles of a piece, group 1 the odd ones
-  int stage = 0;
-  uint32_t phase = 0;
-  bool ok = true;
-  int b = b_first;
-  for (long long u = u0; u < u1;) {
-    const int len = p.seq_len[b], nt = dst_tiles(len);
-    const long long s_b = static_cast<long long>(prefix[b]) * Hkv;
-    if (u >= s_b + static_cast<long long>(nt) * Hkv) { ++b; continue; }
-    const int kvh = static_cast<int>((u - s_b) / nt);
-    const long long s_job = s_b + static_cast<long long>(kvh) * nt;
-    const int t_beg = static_cast<int>(u - s_job);
-    const int t_end = static_cast<int>(min(static_cast<long long>(nt), t_beg + (u1 - u)));
-
+  if (warp < 8) {
+    // ------------------------------ consumers -----------------------------
+    const int quad = lane >> 2, tq = lane & 3, mi = lane >> 3;
+    const int group = warp >> 2, pw = warp & 3;      // group 0 takes the even tiles of a piece, group 1 the odd ones
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
     // Q as A fragments: row `quad` (and quad + 8) of the 16-row operand is query head kvh * G + row
     uint32_t qa[KS][4];
-    {
+    auto load_q = [&] {
       const __nv_bfloat16* q_lo = p.q + static_cast<size_t>(b) * p.ldq + static_cast<size_t>(kvh * G + quad) * DH;
       const __nv_bfloat16* q_hi = q_lo + 8 * DH;
       const bool lo = quad < G, hi = quad + 8 < G;
@@ -1713,168 +1715,215 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
         qa[ks][2] = lo ? *reinterpret_cast<const uint32_t*>(q_lo + c + 8) : 0u;
         qa[ks][3] = hi ? *reinterpret_cast<const uint32_t*>(q_hi + c + 8) : 0u;
       }
-    }
-    float m_lo = -1.0e30f, m_hi = -1.0e30f, l_lo = 0.f, l_hi = 0.f;
-    float o[NB][4];
+    };
+    locate(u0);
+    load_q();
+    for (long long u = u0; u < u1;) {
+      float m_lo = -1.0e30f, m_hi = -1.0e30f, l_lo = 0.f, l_hi = 0.f;
+      float o[NB][4];
 #pragma unroll
-    for (int j = 0; j < NB; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
+      for (int j = 0; j < NB; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
 
-    for (int t = t_beg; t < t_end; ++t) {
-      const int st = stage;
-      const uint32_t ph = phase;
-      if (++stage == stages) { stage = 0; phase ^= 1; }
-      // All eight warps wait for and release every tile, the other group's too: a parity wait tells one fill of a stage from
-      // the next only while no warp is a whole fill ahead (it would pass on the previous fill) or behind (it would wait
-      // for the fill after next, which in turn waits for it).
-      if (ok && !mbar_wait_warp(&full[st], ph, p.status, ST_TIMEOUT_FULL)) ok = false;
-      if (!ok) continue;
-      if (((t - t_beg) & 1) != group) {
-        if (lane == 0) mbar_arrive(&empty[st]);
-        continue;
-      }
-      uint8_t* kp = ring + st * 2 * C::TILE_BYTES;
-      uint8_t* vp = kp + C::TILE_BYTES;
-      const uint32_t kt = smem_u32(kp), vt = smem_u32(vp);
-      const int valid = len - t * DEC_TK - pw * 16;        // positions of this warp's 16 that exist
-      if (valid < 16) {
-        // value rows past the end hold whatever the page holds (or an older tile): 0 * x must not meet NaN
-        for (int i = lane; i < 16 * C::NCH * 8; i += 32) {
-          const int r = i / (C::NCH * 8), x = i - r * (C::NCH * 8);
-          if (r >= valid)
-            *reinterpret_cast<uint4*>(vp + (x >> 3) * (DEC_TK * 128) + (pw * 16 + r) * 128 + (x & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+      for (int t = t_beg; t < t_end; ++t) {
+        const int st = stage;
+        const uint32_t ph = phase;
+        if (++stage == stages) { stage = 0; phase ^= 1; }
+        // All eight warps wait for and release every tile, the other group's too: a parity wait tells one fill of a stage from
+        // the next only while no warp is a whole fill ahead (it would pass on the previous fill) or behind (it would wait
+        // for the fill after next, which in turn waits for it).
+        if (ok && !mbar_wait_warp(&full[st], ph, p.status, ST_TIMEOUT_FULL)) ok = false;
+        if (!ok) continue;
+        if (((t - t_beg) & 1) != group) {
+          if (lane == 0) mbar_arrive(&empty[st]);
+          continue;
         }
-        fence_proxy_async_smem();              // the stage is refilled by TMA later
-        __syncwarp();
-      }
-      // ---- S = Q K^T for this warp's 16 positions (two 16x8 blocks) ----
-      float sacc[2][4];
-#pragma unroll
-      for (int nb = 0; nb < 2; ++nb) { sacc[nb][0] = sacc[nb][1] = sacc[nb][2] = sacc[nb][3] = 0.f; }
-      {
-        const int r = pw * 16 + (mi >> 1) * 8 + (lane & 7);
-#pragma unroll
-        for (int ks = 0; ks < KS; ++ks) {
-          const int unit = ks * 2 + (mi & 1);
-          uint32_t r0, r1, r2, r3;
-          ldsm_x4(kt + (unit >> 3) * (DEC_TK * 128) + r * 128 + (((unit & 7) ^ (r & 7)) << 4), r0, r1, r2, r3);
-          mma_16816(sacc[0], qa[ks], r0, r1);
-          mma_16816(sacc[1], qa[ks], r2, r3);
+        uint8_t* kp = ring + st * 2 * C::TILE_BYTES;
+        uint8_t* vp = kp + C::TILE_BYTES;
+        const uint32_t kt = smem_u32(kp), vt = smem_u32(vp);
+        const int valid = len - t * DEC_TK - pw * 16;        // positions of this warp's 16 that exist
+        if (valid < 16) {
+          // value rows past the end hold whatever the page holds (or an older tile): 0 * x must not meet NaN
+          for (int i = lane; i < 16 * C::NCH * 8; i += 32) {
+            const int r = i / (C::NCH * 8), x = i - r * (C::NCH * 8);
+            if (r >= valid)
+              *reinterpret_cast<uint4*>(vp + (x >> 3) * (DEC_TK * 128) + (pw * 16 + r) * 128 + (x & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+          }
+          fence_proxy_async_smem();              // the stage is refilled by TMA later
+          __syncwarp();
         }
-      }
-      // ---- online softmax on the fragments ----
-      float mx_lo = -1.0e30f, mx_hi = -1.0e30f;
+        // ---- S = Q K^T for this warp's 16 positions (two 16x8 blocks) ----
+        float sacc[2][4];
 #pragma unroll
-      for (int nb = 0; nb < 2; ++nb) {
-        const int pos = nb * 8 + tq * 2;
+        for (int nb = 0; nb < 2; ++nb) { sacc[nb][0] = sacc[nb][1] = sacc[nb][2] = sacc[nb][3] = 0.f; }
+        {
+          const int r = pw * 16 + (mi >> 1) * 8 + (lane & 7);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const bool in = pos + e < valid;
-          sacc[nb][e] = in ? sacc[nb][e] * p.scale_log2 : -1.0e30f;
-          sacc[nb][2 + e] = in ? sacc[nb][2 + e] * p.scale_log2 : -1.0e30f;
-          mx_lo = fmaxf(mx_lo, sacc[nb][e]);
-          mx_hi = fmaxf(mx_hi, sacc[nb][2 + e]);
-        }
-      }
-      mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
-      mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
-      mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
-      mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-      const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
-      const float al_lo = exp2f(m_lo - mn_lo), al_hi = exp2f(m_hi - mn_hi);
-      m_lo = mn_lo; m_hi = mn_hi;
-      uint32_t pa[4];
-      {
-        float pr[2][4];
-        float sum_lo = 0.f, sum_hi = 0.f;
-#pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            // a masked score stays at -1e30: exp2 of (-1e30 - m) is 0 unless the row is empty so far,
-            // in which case m is -1e30 too and the position must still contribute nothing
-            pr[nb][e] = sacc[nb][e] > -1.0e29f ? exp2f(sacc[nb][e] - mn_lo) : 0.f;
-            pr[nb][2 + e] = sacc[nb][2 + e] > -1.0e29f ? exp2f(sacc[nb][2 + e] - mn_hi) : 0.f;
-            sum_lo += pr[nb][e];
-            sum_hi += pr[nb][2 + e];
+          for (int ks = 0; ks < KS; ++ks) {
+            const int unit = ks * 2 + (mi & 1);
+            uint32_t r0, r1, r2, r3;
+            ldsm_x4(kt + (unit >> 3) * (DEC_TK * 128) + r * 128 + (((unit & 7) ^ (r & 7)) << 4), r0, r1, r2, r3);
+            mma_16816(sacc[0], qa[ks], r0, r1);
+            mma_16816(sacc[1], qa[ks], r2, r3);
           }
         }
-        l_lo = l_lo * al_lo + sum_lo;
-        l_hi = l_hi * al_hi + sum_hi;
-        pa[0] = dpack(pr[0][0], pr[0][1]);
-        pa[1] = dpack(pr[0][2], pr[0][3]);
-        pa[2] = dpack(pr[1][0], pr[1][1]);
-        pa[3] = dpack(pr[1][2], pr[1][3]);
-      }
+        // ---- online softmax on the fragments ----
+        float mx_lo = -1.0e30f, mx_hi = -1.0e30f;
 #pragma unroll
-      for (int j = 0; j < NB; ++j) { o[j][0] *= al_lo; o[j][1] *= al_lo; o[j][2] *= al_hi; o[j][3] *= al_hi; }
-      // ---- O += P V over this warp's 16 positions ----
-      {
-        const int r = pw * 16 + (mi & 1) * 8 + (lane & 7);
+        for (int nb = 0; nb < 2; ++nb) {
+          const int pos = nb * 8 + tq * 2;
 #pragma unroll
-        for (int j = 0; j < NB; j += 2) {
-          const int unit = j + (mi >> 1);
-          uint32_t r0, r1, r2, r3;
-          ldsm_x4_t(vt + (unit >> 3) * (DEC_TK * 128) + r * 128 + (((unit & 7) ^ (r & 7)) << 4), r0, r1, r2, r3);
-          mma_16816(o[j], pa, r0, r1);
-          mma_16816(o[j + 1], pa, r2, r3);
+          for (int e = 0; e < 2; ++e) {
+            const bool in = pos + e < valid;
+            sacc[nb][e] = in ? sacc[nb][e] * p.scale_log2 : -1.0e30f;
+            sacc[nb][2 + e] = in ? sacc[nb][2 + e] * p.scale_log2 : -1.0e30f;
+            mx_lo = fmaxf(mx_lo, sacc[nb][e]);
+            mx_hi = fmaxf(mx_hi, sacc[nb][2 + e]);
+          }
         }
+        mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
+        mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
+        mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
+        mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
+        const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
+        const float al_lo = exp2f(m_lo - mn_lo), al_hi = exp2f(m_hi - mn_hi);
+        m_lo = mn_lo; m_hi = mn_hi;
+        uint32_t pa[4];
+        {
+          float pr[2][4];
+          float sum_lo = 0.f, sum_hi = 0.f;
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              // a masked score stays at -1e30: exp2 of (-1e30 - m) is 0 unless the row is empty so far,
+              // in which case m is -1e30 too and the position must still contribute nothing
+              pr[nb][e] = sacc[nb][e] > -1.0e29f ? exp2f(sacc[nb][e] - mn_lo) : 0.f;
+              pr[nb][2 + e] = sacc[nb][2 + e] > -1.0e29f ? exp2f(sacc[nb][2 + e] - mn_hi) : 0.f;
+              sum_lo += pr[nb][e];
+              sum_hi += pr[nb][2 + e];
+            }
+          }
+          l_lo = l_lo * al_lo + sum_lo;
+          l_hi = l_hi * al_hi + sum_hi;
+          pa[0] = dpack(pr[0][0], pr[0][1]);
+          pa[1] = dpack(pr[0][2], pr[0][3]);
+          pa[2] = dpack(pr[1][0], pr[1][1]);
+          pa[3] = dpack(pr[1][2], pr[1][3]);
+        }
+#pragma unroll
+        for (int j = 0; j < NB; ++j) { o[j][0] *= al_lo; o[j][1] *= al_lo; o[j][2] *= al_hi; o[j][3] *= al_hi; }
+        // ---- O += P V over this warp's 16 positions ----
+        {
+          const int r = pw * 16 + (mi & 1) * 8 + (lane & 7);
+#pragma unroll
+          for (int j = 0; j < NB; j += 2) {
+            const int unit = j + (mi >> 1);
+            uint32_t r0, r1, r2, r3;
+            ldsm_x4_t(vt + (unit >> 3) * (DEC_TK * 128) + r * 128 + (((unit & 7) ^ (r & 7)) << 4), r0, r1, r2, r3);
+            mma_16816(o[j], pa, r0, r1);
+            mma_16816(o[j + 1], pa, r2, r3);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[st]);
+      }
+
+      const bool first = u == u0;
+      u += t_end - t_beg;
+      if (u < u1) {                                  // the next piece's Q comes while this one is handed over
+        locate(u);
+        load_q();
+      }
+      // ---- to the finishers, once they have read the piece before ----
+      l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
+      l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
+      l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
+      l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+      if (!first) asm volatile("bar.sync 2, %0;" ::"n"(256 + DST_FINISHERS) : "memory");
+#pragma unroll
+      for (int j = 0; j < NB; ++j) {
+        float* r_lo = sm_o + (warp * G + quad) * DH + j * 8 + tq * 2;
+        if (quad < G) *reinterpret_cast<float2*>(r_lo) = make_float2(o[j][0], o[j][1]);
+        if (quad + 8 < G) *reinterpret_cast<float2*>(r_lo + 8 * DH) = make_float2(o[j][2], o[j][3]);
+      }
+      if (tq == 0) {
+        if (quad < G) { sm_ml[(warp * G + quad) * 2] = m_lo; sm_ml[(warp * G + quad) * 2 + 1] = l_lo; }
+        if (quad + 8 < G) { sm_ml[(warp * G + quad + 8) * 2] = m_hi; sm_ml[(warp * G + quad + 8) * 2 + 1] = l_hi; }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[st]);
+      if (u < u1) asm volatile("bar.arrive 1, %0;" ::"n"(256 + DST_FINISHERS) : "memory");
+      else asm volatile("bar.arrive 4, %0;" ::"n"(256 + DST_FINISHERS + 32) : "memory");
     }
+    return;
+  }
 
-    // ---- merge the eight warps in warp order ----
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      float* r_lo = sm_o + (warp * G + quad) * DH + j * 8 + tq * 2;
-      if (quad < G) *reinterpret_cast<float2*>(r_lo) = make_float2(o[j][0], o[j][1]);
-      if (quad + 8 < G) *reinterpret_cast<float2*>(r_lo + 8 * DH) = make_float2(o[j][2], o[j][3]);
-    }
-    if (tq == 0) {
-      if (quad < G) { sm_ml[(warp * G + quad) * 2] = m_lo; sm_ml[(warp * G + quad) * 2 + 1] = l_lo; }
-      if (quad + 8 < G) { sm_ml[(warp * G + quad + 8) * 2] = m_hi; sm_ml[(warp * G + quad + 8) * 2 + 1] = l_hi; }
-    }
-    asm volatile("bar.sync 1, 256;" ::: "memory");
+  // ------------------------------ finishers -----------------------------
+  // They merge the eight warps in warp order and then the pieces of a job while the consumers are at the next piece, whose Q has been
+  // fetched meanwhile; at the CTA's last piece the producer helps. Consumers that did this themselves, the ring full behind them, took
+  // about 2 us a piece: 64 x 2048 positions 94 -> 85 us, 64 x 256 32.4 -> 25, 32 x 2048 54.5 -> 49, 1 x 2048 11.6 -> 11.2.
+  const int fw = (warp + 3) & 3, ft = fw * 32 + lane;      // warps 9, 10, 11 and 8
+  for (long long u = warp == 8 ? s_job + t_beg : u0; u < u1;) {
+    locate(u);
+    const bool last = u + (t_end - t_beg) >= u1;
+    const int nf = DST_FINISHERS + (last ? 32 : 0);
+    // the last piece has barriers of its own: the producer comes to them while the others are still at pieces before it
+    if (last) asm volatile("bar.sync 4, %0;" ::"n"(256 + DST_FINISHERS + 32) : "memory");
+    else asm volatile("bar.sync 1, %0;" ::"n"(256 + DST_FINISHERS) : "memory");
+    auto meet = [&] {
+      __syncwarp();
+      if (last) asm volatile("bar.sync 5, %0;" ::"n"(DST_FINISHERS + 32) : "memory");
+      else asm volatile("bar.sync 3, %0;" ::"n"(DST_FINISHERS) : "memory");
+    };
     const bool direct = t_beg == 0 && t_end == nt;
     const int job = b * Hkv + kvh;
+    auto store_out = [&](int g, int d, float lt, const float4& ot) {
+      uint2 pk = make_uint2(0u, 0u);             // no weight: zeros, whatever the values held
+      if (lt > 0.f) pk = make_uint2(dpack(ot.x / lt, ot.y / lt), dpack(ot.z / lt, ot.w / lt));
+      __nv_bfloat16* dst = p.out + static_cast<size_t>(b) * p.ldo + (kvh * G + g) * DH + d;
+      if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) *reinterpret_cast<uint2*>(dst) = pk;
+      else {
+        uint16_t* d16 = reinterpret_cast<uint16_t*>(dst);
+        d16[0] = static_cast<uint16_t>(pk.x); d16[1] = static_cast<uint16_t>(pk.x >> 16);
+        d16[2] = static_cast<uint16_t>(pk.y); d16[3] = static_cast<uint16_t>(pk.y >> 16);
+      }
+    };
     // CTAs that share this job: c is the owner of unit v when c * T / grid <= v < (c + 1) * T / grid
     const int c_first = static_cast<int>(((s_job + 1) * grid - 1) / T);
     const int c_last = static_cast<int>(((s_job + nt) * grid - 1) / T);
     constexpr int SLOT = 16 * (DH + 2);
     // a CTA's first piece goes to slot 2c, a later one (a job that starts inside its range) to 2c + 1
     float* slot = p.part + static_cast<size_t>(2 * blockIdx.x + (u == u0 ? 0 : 1)) * SLOT;
-    for (int i = threadIdx.x; i < G * DH; i += 256) {
-      const int g = i / DH, d = i - g * DH;
+    for (int i = ft; i < G * (DH / 4); i += nf) {
+      const int g = i / (DH / 4), d = (i - g * (DH / 4)) * 4;
       float mt = -1.0e30f;
 #pragma unroll
       for (int w = 0; w < 8; ++w) mt = fmaxf(mt, sm_ml[(w * G + g) * 2]);
-      float lt = 0.f, ot = 0.f;
+      float lt = 0.f;
+      float4 ot = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int w = 0; w < 8; ++w) {
         const float wgt = exp2f(sm_ml[(w * G + g) * 2] - mt);
+        const float4 v = *reinterpret_cast<const float4*>(sm_o + (w * G + g) * DH + d);
         lt += sm_ml[(w * G + g) * 2 + 1] * wgt;
-        ot += sm_o[(w * G + g) * DH + d] * wgt;
+        ot.x += v.x * wgt; ot.y += v.y * wgt; ot.z += v.z * wgt; ot.w += v.w * wgt;
       }
       if (direct) {
-        p.out[static_cast<size_t>(b) * p.ldo + (kvh * G + g) * DH + d] = __float2bfloat16_rn(lt > 0.f ? ot / lt : 0.f);
+        store_out(g, d, lt, ot);
       } else {
-        slot[g * DH + d] = ot;
+        *reinterpret_cast<float4*>(slot + g * DH + d) = ot;
         if (d == 0) { slot[16 * DH + g * 2] = mt; slot[16 * DH + g * 2 + 1] = lt; }
       }
     }
+    __syncwarp();
     if (!direct) {
       __threadfence();
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (threadIdx.x == 0) {
+      meet();
+      if (ft == 0) {
         const unsigned int prev = atomicAdd(p.counters + job, 1u);
         s_last = (prev == static_cast<unsigned int>(c_last - c_first)) ? 1 : 0;
         if (s_last) p.counters[job] = 0;
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      meet();
       if (s_last) {
         __threadfence();
         const int np = c_last - c_first + 1;
@@ -1886,14 +1935,23 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
         // sums take 16-byte loads (a job of 1 x 2048 positions has 16 pieces: 14.0 -> 10.7 us for the whole kernel)
         float* w_m = sm_o;                             // [np][G] maxima, then weights
         float* w_l = sm_o + np * G;                    // [np][G] sums; row g's total ends up in w_l[g]
-        for (int i = threadIdx.x; i < np * G; i += 256) {
+        // sixteen pieces' values of a thread's columns in flight, the first of them while the weights are made
+        float4 vo[16];
+        auto fetch = [&](int i, int s0) {
+          const int g = i / (DH / 4), d = (i - g * (DH / 4)) * 4;
+#pragma unroll
+          for (int x = 0; x < 16; ++x)
+            if (s0 + x < np) vo[x] = __ldcg(reinterpret_cast<const float4*>(piece(s0 + x) + g * DH + d));
+        };
+        if (ft < G * (DH / 4)) fetch(ft, 0);
+        for (int i = ft; i < np * G; i += nf) {
           const int s = i / G, g = i - s * G;
           const float2 ml = __ldcg(reinterpret_cast<const float2*>(piece(s) + 16 * DH + g * 2));
           w_m[i] = ml.x;
           w_l[i] = ml.y;
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        for (int g = warp; g < G; g += 8) {
+        meet();
+        for (int g = fw; g < G; g += nf / 32) {
           float mt = -1.0e30f, lt = 0.f;
           for (int s = lane; s < np; s += 32) mt = fmaxf(mt, w_m[s * G + g]);
 #pragma unroll
@@ -1908,38 +1966,27 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
           __syncwarp();
           if (lane == 0) w_l[g] = lt;                  // row g of piece 0, read by this warp only
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        for (int i = threadIdx.x; i < G * (DH / 4); i += 256) {
+        meet();
+        for (int i = ft; i < G * (DH / 4); i += nf) {
           const int g = i / (DH / 4), d = (i - g * (DH / 4)) * 4;
           float4 ot = make_float4(0.f, 0.f, 0.f, 0.f);
-          for (int s0 = 0; s0 < np; s0 += 4) {   // four pieces' loads in flight, added in piece order
-            float4 vo[4];
+          for (int s0 = 0; s0 < np; s0 += 16) {                       // added in piece order
+            if (i != ft || s0 > 0) fetch(i, s0);
 #pragma unroll
-            for (int x = 0; x < 4; ++x)
-              if (s0 + x < np) vo[x] = __ldcg(reinterpret_cast<const float4*>(piece(s0 + x) + g * DH + d));
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
+            for (int x = 0; x < 16; ++x) {
               if (s0 + x < np) {
                 const float wgt = w_m[(s0 + x) * G + g];
                 ot.x += vo[x].x * wgt; ot.y += vo[x].y * wgt; ot.z += vo[x].z * wgt; ot.w += vo[x].w * wgt;
               }
             }
           }
-          const float lt = w_l[g];
-          uint2 pk = make_uint2(0u, 0u);             // no weight: zeros, whatever the values held
-          if (lt > 0.f) pk = make_uint2(dpack(ot.x / lt, ot.y / lt), dpack(ot.z / lt, ot.w / lt));
-          __nv_bfloat16* dst = p.out + static_cast<size_t>(b) * p.ldo + (kvh * G + g) * DH + d;
-          if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) *reinterpret_cast<uint2*>(dst) = pk;
-          else {
-            uint16_t* d16 = reinterpret_cast<uint16_t*>(dst);
-            d16[0] = static_cast<uint16_t>(pk.x); d16[1] = static_cast<uint16_t>(pk.x >> 16);
-            d16[2] = static_cast<uint16_t>(pk.y); d16[3] = static_cast<uint16_t>(pk.y >> 16);
-          }
+          store_out(g, d, w_l[g], ot);
         }
       }
     }
-    asm volatile("bar.sync 1, 256;" ::: "memory");   // the merge buffers and s_last are free again
     u += t_end - t_beg;
+    __syncwarp();
+    if (!last) asm volatile("bar.arrive 2, %0;" ::"n"(256 + DST_FINISHERS) : "memory");   // the merge buffers are free again
   }
 }
 
