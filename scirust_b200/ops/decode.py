@@ -518,21 +518,23 @@ def _stream_wins(L, jobs, G, page, device) -> bool:
     """Where the balanced stream beats the split kernel, for ``jobs`` (sequence, kv head) pairs that hold about ``L`` positions,
     ``G`` query heads per kv head. us, split against stream.
 
-    Four query heads and more, pages of 64 and more (32 / 8 heads): 1 x 2048 14.1 / 10.1, 1 x 8192 43.8 / 16.7, 4 x 2048
-    22.4 / 16.5, 16 x 512 18.9 / 16.6, 16 x 2304 40.2 / 32.3, 64 x 256 31.3 / 29.5, 64 x 2048 107.0 / 88.6; but 4 x 1024
-    13.3 / 14.3, 16 x 256 11.9 / 14.2, 64 x 128 13.0 / 21.0: its start and the merge of many short pieces need six tiles of
-    64 positions per SM, or long sequences (where the split kernel's 64 splits and its last wave bind), to pay.
-    Smaller pages make smaller copies, one thread issues them: 32 positions win by less (64 x 2048 105.7 / 106.6), 16 only
-    while a batch is small (1 x 8192 43.5 / 20.0, 4 x 2048 23.7 / 22.3; 16 x 2304 41.5 / 49.8), 8 lose (64 x 2048 110 / 250).
+    Four query heads and more, pages of 64 and more (32 / 8 heads): 1 x 2048 17.5 / 9.8, 2 x 1024 14.4 / 13.5, 4 x 1536 18.2 / 17.1,
+    4 x 2048 26.2 / 18.1, 16 x 512 21.8 / 16.3, 16 x 2304 43.1 / 33.5, 64 x 192 31.3 / 22.3, 64 x 256 34.3 / 23.4, 64 x 2048 111 / 83.5;
+    but 4 x 1024 15.1 / 16.0, 8 x 768 15.2 / 16.9, 16 x 256 13.7 / 15.9, 64 x 128 14.7 / 17.9: its start and the merge of many short
+    pieces need six tiles of 64 positions per SM, or long sequences (where the split kernel's 64 splits and its last wave bind), to pay.
+    Smaller pages make smaller copies, one thread issues them: 32 positions win by less (64 x 2048 111.7 / 105.6), 16 only
+    while a batch is small (1 x 8192 47.3 / 18.9, 4 x 2048 25.9 / 19.4; 16 x 2304 43.5 / 51.4), 8 lose.
     With fewer query heads per kv head the split kernel is bound by memory sooner and the merge weighs more: two and three want
-    512 positions (16 / 8 heads, 32 x 256 17.1 / 17.7, 16 x 512 16.4 / 15.5), one long sequences and few jobs (32 / 32 heads
-    16 x 2304 105.5 / 89.6, 4 x 512 14.5 / 15.2, 64 x 1024 156.9 / 166.4)."""
+    512 positions (16 / 8 heads 16 x 384 12.0 / 14.1, 16 x 512 18.9 / 15.3), one longer sequences and few jobs (32 / 32 heads 16 x 1024
+    59.2 / 48.3, 16 x 2304 111.4 / 89.0, 64 x 256 55.2 / 57.2; 64 x 1024 would win by little, 162 / 154)."""
     per_sm = jobs * max(1, (L + 63) // 64) / _g.num_sms(device)
     if G < 4:
-        return page >= 64 and per_sm >= 6.0 and (L >= 512 if G > 1 else L >= 2048 and jobs <= 512)
+        return page >= 64 and per_sm >= 6.0 and (L >= 512 if G > 1 else L >= 1024 and jobs <= 512)
     if page < 32:
         return page == 16 and L >= 2048 and 1.5 <= per_sm <= 7.0
-    return L >= 256 and per_sm >= (1.5 if L >= 2048 else 6.0) and (page >= 64 or per_sm <= 60.0)
+    if page < 64:
+        return L >= 256 and (1.5 if L >= 2048 else 6.0) <= per_sm <= 60.0
+    return L >= 192 and per_sm >= (1.5 if L >= 1536 or L >= 1024 and jobs <= 16 else 6.0)
 
 
 def _stream_ok(pool, page, B, H, Hkv, dh) -> bool:

@@ -60,6 +60,16 @@ def test_streamed_decode_attention(B, L, H, Hkv, page, stream):
     assert D._stream_wins(L, B * Hkv, H // Hkv, page, None) is stream
 
 
+@pytest.mark.parametrize("B,L,H,Hkv,page,stream", [
+    # lines that lie lower since pieces are merged beside the stream, on both sides
+    (64, 192, 32, 8, 64, True), (64, 191, 32, 8, 64, False), (64, 192, 32, 8, 32, False), (2, 1024, 32, 8, 64, True),
+    (2, 1023, 32, 8, 64, False), (4, 1536, 32, 8, 64, True), (4, 1535, 32, 8, 64, False), (4, 1536, 32, 8, 32, False),
+    (16, 1024, 32, 32, 64, True), (16, 1023, 32, 32, 64, False), (32, 1024, 32, 32, 64, False),
+])
+def test_streamed_decode_attention_of_shorter_sequences(B, L, H, Hkv, page, stream):
+    assert D._stream_wins(L, B * Hkv, H // Hkv, page, None) is stream
+
+
 def test_kernel_attributes_are_set_for_every_device(tmp_path):
     """The helper of the launchers, with a counting stand-in for the CUDA call: once per device, again after a failure, and
     every time for device numbers beyond its mask."""
