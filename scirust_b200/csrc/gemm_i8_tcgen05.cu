@@ -252,9 +252,11 @@ __global__ void quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int ld
 
 // The same quantiser, one CTA per row, eight elements (16 bytes) per thread and step: the row is read once from memory,
 // the maximum is combined through shared memory. KEEP words a thread stay in registers, all loads in flight; what lies
-// beyond them is read again from L1 / L2. Rows of 8192 and more are bound by those loads (16 rows of 14336: 5.6 us with
-// 256 threads and nothing kept, 4.5 with 512 threads and four words); for shorter ones and for many rows the
-// unrolled words only cost the threads that have none (1024 rows of 1024: 3.2 and 7.0 us, 4096 of 8192: 42.7 and 47.5).
+// beyond them is read again from L1 / L2. A few rows are bound by the latency of those loads: up to 4096 elements a word for each of 512
+// threads, from 8192 on four (us, 256 threads and nothing kept / so: 16 x 1024 2.3 / 2.1, 16 x 4096 3.0 / 2.5, 64 x 4096 3.1 / 2.6,
+// 16 x 14336 5.6 / 4.5). Many rows are bound by instructions, where the words that a thread does not have cost (1024 x 1024 3.4 and
+// 4.3 with one, 4096 x 4096 15.9 and 18.7), and so does the division: with it 1024 x 4096 8.2 us, 4096 x 4096 23.5, 1024 x 14336 21.0,
+// with a product that settles all but the halfway cases 6.3, 15.8, 16.6.
 template <int THREADS, int KEEP>
 __global__ void __launch_bounds__(THREADS)
 quantize_rows_vec8_kernel(const __nv_bfloat16* x, int ldx, int8_t* q, int ldq, float* sx, int K) {
@@ -288,10 +290,26 @@ quantize_rows_vec8_kernel(const __nv_bfloat16* x, int ldx, int8_t* q, int ldq, f
   const float s = amax == 0.f ? 1.f : amax / 127.f;
   if (threadIdx.x == 0) sx[row] = s;
   uint2* qr = reinterpret_cast<uint2*>(q + static_cast<size_t>(row) * ldq);
+  const float inv = __frcp_rn(s);
   auto quantise = [&](int i, const uint4& v) {
     const float f[8] = {bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y),
                         bf16_lo(v.z), bf16_hi(v.z), bf16_lo(v.w), bf16_hi(v.w)};
     uint32_t w[2] = {0u, 0u};
+    // x * (1 / s) is within 127 * 2^-23 of x / s, and t + 0.5f below rounds by at most 2^-18, so the nearest whole number is the same
+    // but where the product lies within 1e-4 of halfway (or is no number): those words take the divisions.
+    bool near_half = false;
+    uint32_t m[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float r = __fmaf_rn(f[j], inv, 12582912.f);           // 1.5 * 2^23: the sum's last bit is one
+      near_half |= !(fabsf(__fmaf_rn(f[j], inv, __fsub_rn(12582912.f, r))) <= 0.4999f);
+      m[j] = __float_as_uint(r);
+    }
+    if (!near_half) {
+      qr[i] = make_uint2(__byte_perm(__byte_perm(m[0], m[1], 0x0040), __byte_perm(m[2], m[3], 0x0040), 0x5410),
+                         __byte_perm(__byte_perm(m[4], m[5], 0x0040), __byte_perm(m[6], m[7], 0x0040), 0x5410));
+      return;
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float t = __fdiv_rn(f[j], s);
@@ -321,8 +339,9 @@ extern "C" int sb_quantize_rows(const void* x, int ldx, void* xq, int ldq, float
   if ((K & 7) == 0 && (ldx & 7) == 0 && (ldq & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(xq) & 7) == 0) {
     const bool keep = K >= 8192 && M <= 1024;
-    auto kern = keep ? quantize_rows_vec8_kernel<512, 4> : quantize_rows_vec8_kernel<256, 0>;
-    return launch_dep(kern, dim3(M), dim3(keep ? 512 : 256), 0, STREAM, static_cast<const __nv_bfloat16*>(x), ldx,
+    const bool one = K <= 4096 && M <= num_sms();
+    auto kern = keep ? quantize_rows_vec8_kernel<512, 4> : one ? quantize_rows_vec8_kernel<512, 1> : quantize_rows_vec8_kernel<256, 0>;
+    return launch_dep(kern, dim3(M), dim3(keep || one ? 512 : 256), 0, STREAM, static_cast<const __nv_bfloat16*>(x), ldx,
                       static_cast<int8_t*>(xq), ldq, sx, K) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
   }
   quantize_rows_kernel<<<(M + 7) / 8, 256, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(x), ldx,

@@ -506,3 +506,21 @@ def test_launches_of_the_weight_streaming_gemm_are_counted_as_they_are(quant, M,
     D.matmul_skinny(x, w, splits=splits)
     counted = _g.launch_count - before - (1 if quant else 0)   # the row quantiser is one
     assert counted == (1 if ws.isnan().all() else 2)
+
+
+@pytest.mark.parametrize("M,K", [(3, 8), (16, 1000), (16, 4096), (149, 4096), (9, 4104), (2, 8192), (16, 14336)])
+def test_row_quantiser_is_the_division_rounded(M, K):
+    """Bit for bit the host statement on rows of halfway values, of one size, tiny, huge, denormal and with no number in them: the
+    product by 1 / scale decides only where the division would decide the same."""
+    g = torch.Generator().manual_seed(K)
+    for size in (1.0, 1e-30, 1e-38, 3e-39, 1e-40, 3e38):
+        x = (torch.randn((M, K), generator=g).clamp(-1, 1) * size).to(BF)
+        x[0] = (torch.arange(K) % 255 - 127).to(BF) * 0.5 * (size if size < 1e30 else 1e30)
+        x[0, 0] = 127.0 * (size if size < 1e30 else 1e30)
+        x[1] = x[1].abs().max()
+        q, s = D.quantize_rows(x.cuda())
+        qr, sr = D.quantize_rows(x)
+        assert torch.equal(q.cpu(), qr) and torch.equal(s.cpu(), sr)
+    x[0], x[1, 0] = float("nan"), float("inf")            # as the division has it: -128 where there is no number
+    q, s = D.quantize_rows(x.cuda())
+    assert bool((q[0] == -128).all()) and int(q[1, 0]) == -128 and bool((q[1, 1:] == 0).all())
