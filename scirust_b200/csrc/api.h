@@ -87,7 +87,7 @@ int sb_gemm_i8(const void* xq, int ldq, const float* sx, const void* wq_t, int l
 
 // gemm_pair_tcgen05.cu
 size_t sb_gemm_pair_workspace_floats();
-int sb_gemm_pair_widen_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, void* workspace, void* act, int ld_act, int ff, const void* gu, int ld_gu, int n_widen, const void* const* q, const void* const* scale, void* const* w, const int* kn, int* status, void* stream_);
+int sb_gemm_pair_widen_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, void* workspace, void* act, int ld_act, int ff, const void* gu, int ld_gu, int n_widen, const int64_t* widen, int* status, void* stream_);
 int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc, int ldr, int a_mn, int b_mn, void* workspace, void* act, int ld_act, int ff, const void* gu, int ld_gu, int* status, void* stream_);
 int sb_gemm_pair_ag_bf16(void* const* a_ptrs, const void* B, void* C, const void* R, int M, int N, int K, int lda, int ldb, int ldc, int ldr, int b_mn, void* const* stage_ptrs, int ld_stage, void* const* flag_ptrs, void* const* chunk_flag_ptrs, unsigned int* chunk_ctr, unsigned int* cta_ctr, int rank, int W, uint32_t epoch, int wait_ms, int copy_own, int* status, void* stream_);
 int sb_gemm_pair_rs_bf16(const void* A, const void* B, void* const* part_ptrs, int ldp, void* out, int ld_out, const void* res, int ld_res, int M, int N, int K, int lda, int ldb, int b_mn, void* const* ready_ptrs, void* const* flag_ptrs, unsigned int* block_ctr, unsigned int* cta_ctr, int rank, int W, uint32_t epoch, int wait_ms, int* status, void* stream_);

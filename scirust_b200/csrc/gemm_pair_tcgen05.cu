@@ -16,6 +16,7 @@
 //   warp 10-13 copiers (both CTAs): shards of a distributed product, or int8 matrices of later products to bf16
 // Stage release and "accumulator ready" are tcgen05.commit arrivals delivered to both CTAs.
 // No TMA multicast is used.
+#include <climits>
 #include <cstdlib>
 #include "sm100_ptx.cuh"
 #include "api.h"
@@ -851,12 +852,12 @@ using namespace sb;
 // residual, no balanced schedule on that path.
 extern "C" size_t sb_gemm_pair_workspace_floats() { return static_cast<size_t>(num_sms() / 2) * 3 * 256 * 256; }
 
-// `n_widen` up to 3 (0: none): int8 matrices q[i] [K, N] with fp32 column scales, contiguous, that the launch also writes as
-// bf16 to w[i]; kn: K and N of each, N % 16 == 0, q, scale and w 16-byte aligned.
+// `n_widen` up to 3 (0: none): int8 matrices [K, N] with fp32 column scales, contiguous, that the launch also writes as bf16;
+// widen: for each the addresses of codes, scales and output, all 16-byte aligned, K and N, N % 16 == 0.
 extern "C" int sb_gemm_pair_widen_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K, int lda,
                                        int ldb, int ldc, int ldr, int a_mn, int b_mn, void* workspace, void* act, int ld_act,
-                                       int ff, const void* gu, int ld_gu, int n_widen, const void* const* q,
-                                       const void* const* scale, void* const* w, const int* kn, int* status, void* stream_) {
+                                       int ff, const void* gu, int ld_gu, int n_widen, const int64_t* widen,
+                                       int* status, void* stream_) {
   using namespace sb::pair;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || (ldc & 7) || (R && (ldr & 7)) || (!C && !ff)) return SB_ERR_ARG;
@@ -884,15 +885,15 @@ extern "C" int sb_gemm_pair_widen_bf16(const void* A, const void* B, void* C, co
   p.n_widen = n_widen;
   if (n_widen < 0 || n_widen > MAX_WIDEN) return SB_ERR_ARG;
   for (int i = 0; i < n_widen; ++i) {
-    if (!q[i] || !scale[i] || !w[i] || kn[2 * i] <= 0 || kn[2 * i + 1] <= 0 || (kn[2 * i + 1] & 15)) return SB_ERR_ARG;
-    if ((reinterpret_cast<uintptr_t>(q[i]) | reinterpret_cast<uintptr_t>(scale[i]) | reinterpret_cast<uintptr_t>(w[i])) & 15)
-      return SB_ERR_ALIGN;
-    p.widen[i] = {static_cast<const uint4*>(q[i]), static_cast<const float*>(scale[i]), static_cast<uint4*>(w[i]), kn[2 * i],
-                  kn[2 * i + 1], 64};
+    const int64_t* j = widen + 5 * i;
+    if (!j[0] || !j[1] || !j[2] || j[3] <= 0 || j[3] > INT_MAX || j[4] <= 0 || j[4] > INT_MAX || (j[4] & 15)) return SB_ERR_ARG;
+    if ((j[0] | j[1] | j[2]) & 15) return SB_ERR_ALIGN;
+    Widen& to = p.widen[i];
+    to = {reinterpret_cast<const uint4*>(j[0]), reinterpret_cast<const float*>(j[1]), reinterpret_cast<uint4*>(j[2]),
+          static_cast<int>(j[3]), static_cast<int>(j[4]), 64};
     // enough units that the last round of the warps is a small part, unless that takes fewer rows than a thread has in flight
-    const long long cols = (kn[2 * i + 1] + 511) / 512;
-    while (p.widen[i].rows > WIDEN_FLY && cols * ((kn[2 * i] + p.widen[i].rows - 1) / p.widen[i].rows) < 8ll * num_sms() * COPY_WARPS)
-      p.widen[i].rows /= 2;
+    const long long cols = (j[4] + 511) / 512;
+    while (to.rows > WIDEN_FLY && cols * ((to.K + to.rows - 1) / to.rows) < 8ll * num_sms() * COPY_WARPS) to.rows /= 2;
   }
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.R = R; p.ldr = ldr; p.status = status;
   p.ff = ff;
@@ -946,7 +947,7 @@ extern "C" int sb_gemm_pair_bf16(const void* A, const void* B, void* C, const vo
                                  int ldb, int ldc, int ldr, int a_mn, int b_mn, void* workspace, void* act, int ld_act,
                                  int ff, const void* gu, int ld_gu, int* status, void* stream_) {
   return sb_gemm_pair_widen_bf16(A, B, C, R, M, N, K, lda, ldb, ldc, ldr, a_mn, b_mn, workspace, act, ld_act, ff, gu, ld_gu, 0,
-                                 nullptr, nullptr, nullptr, nullptr, status, stream_);
+                                 nullptr, status, stream_);
 }
 
 // All-gather -> GEMM on CTA pairs: C[M,N] = gather(A shards)[M,K] * op(B) (+ R). a_ptrs[s]: rank s's shard

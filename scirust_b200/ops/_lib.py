@@ -32,7 +32,7 @@ _CUDA_SIGS = {
     "sb_gemm_bf16": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, i32, vp, vp],
     "sb_gemm_pair_bf16": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp, i32, i32, vp, i32, vp, vp],
     "sb_gemm_pair_widen_bf16": [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp, i32, i32, vp, i32,
-                                i32, vp, vp, vp, vp, vp, vp],
+                                i32, vp, vp, vp],
     "sb_rmsnorm_fwd": [vp, vp, vp, vp, i32, i32, i32, i32, f32, vp],
     "sb_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, vp],
     "sb_rmsnorm_bwd_both": [vp, vp, vp, vp, vp, vp, vp, i32, vp, vp, i32, i32, vp],

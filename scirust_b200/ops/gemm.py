@@ -13,7 +13,7 @@ be tested without a GPU; CUDA tensors always run the native kernel.
 """
 from __future__ import annotations
 
-import ctypes
+import array
 import os
 
 import torch
@@ -133,11 +133,12 @@ class _Bias:
         return 0
 
 
-def _widen_args(widen):
-    """``[(q, scale, w), ...]`` as the arguments of ``sb_gemm_pair_widen_bf16``: count, three tables of pointers, sizes."""
-    ptrs = ctypes.c_void_p * len(widen)
-    sizes = [n for q, _, _ in widen for n in q.shape]
-    return (len(widen), *(ptrs(*(job[i].data_ptr() for job in widen)) for i in range(3)), (ctypes.c_int * len(sizes))(*sizes))
+def _widen_table(widen):
+    """``[(q, scale, w), ...]`` as ``sb_gemm_pair_widen_bf16`` takes it; read before the call returns."""
+    table = array.array("q")
+    for q, scale, w in widen:
+        table.extend((q.data_ptr(), scale.data_ptr(), w.data_ptr(), *q.shape))
+    return table
 
 
 def _gemm(a, b, M, N, K, a_mn, b_mn, out, residual, splits, bn, bias=None, widen=()):
@@ -167,7 +168,8 @@ def _gemm(a, b, M, N, K, a_mn, b_mn, out, residual, splits, bn, bias=None, widen
                 a.stride(0), b.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
                 int(a_mn), int(b_mn), _lib.ptr(ws), None, 0, 0, None, 0)
         if widen:
-            _lib.call("sb_gemm_pair_widen_bf16", *args, *_widen_args(widen), st.data_ptr(), _lib.stream())
+            table = _widen_table(widen)
+            _lib.call("sb_gemm_pair_widen_bf16", *args, len(widen), table.buffer_info()[0], st.data_ptr(), _lib.stream())
         else:
             _lib.call("sb_gemm_pair_bf16", *args, st.data_ptr(), _lib.stream())
         launch_count += 1
@@ -255,7 +257,8 @@ def _swiglu_product(x, wgu, gu, act, widen=()):
             gu.stride(0) if gu is not None else 0, 0, 0, 1, None, act.data_ptr(), act.stride(0), N // 2, None, 0)
     st = _lib.status_word(x.device).data_ptr()
     if widen:
-        _lib.call("sb_gemm_pair_widen_bf16", *args, *_widen_args(widen), st, _lib.stream())
+        table = _widen_table(widen)
+        _lib.call("sb_gemm_pair_widen_bf16", *args, len(widen), table.buffer_info()[0], st, _lib.stream())
     else:
         _lib.call("sb_gemm_pair_bf16", *args, st, _lib.stream())
     launch_count += 1

@@ -290,7 +290,7 @@ def test_product_widens_int8_matrices_beside_itself(M, N, K, form, monkeypatch):
 
 
 @pytest.mark.parametrize("batch,seq,ff", [(1, 1100, 2816), (3, 683, 2824)])
-def test_prefill_that_widens_ahead(batch, seq, ff):
+def test_prefill_that_widens_ahead(batch, seq, ff, monkeypatch):
     """Logits and cache as from an engine that expands each matrix before its product (ff 2824: two matrices are not wide enough by
     whole 16-byte words and are left to that)."""
     from scirust_b200.models.infer import InferenceEngine, _WidenAhead
@@ -303,6 +303,7 @@ def test_prefill_that_widens_ahead(batch, seq, ff):
         def _proj_out(self, a, w, x, swiglu=False, site="attn"):
             return InferenceEngine._linear(self, ops.swiglu_fwd(a) if swiglu else a, w, residual=x)
 
+    monkeypatch.setattr(_WidenAhead, "WORK", 0)
     cfg = SciAgentConfig(512, 1024, 3, 16, 4, ff, 2048, 1e4)
     model = GQADecoder(cfg, device="cuda", seed=3)
     tokens = torch.randint(0, 512, (batch, seq), generator=torch.Generator().manual_seed(1)).cuda()
@@ -316,3 +317,6 @@ def test_prefill_that_widens_ahead(batch, seq, ff):
     plan = _WidenAhead(eng.layers, batch * seq)
     taken = [len(plan.product(l[k])[1].get("widen", ())) for l in eng.layers for k in ("wqkv", "wo", "wgu", "wd")]
     assert sum(taken) >= 3 and max(taken) <= 3
+    monkeypatch.undo()
+    plan = _WidenAhead(eng.layers, batch * seq)            # too little work for the host to plan
+    assert all(plan.product(l[k]) == (l[k], {}) for l in eng.layers for k in ("wqkv", "wo", "wgu", "wd"))
