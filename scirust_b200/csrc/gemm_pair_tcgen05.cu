@@ -883,7 +883,7 @@ extern "C" int sb_gemm_pair_widen_bf16(const void* A, const void* B, void* C, co
   }
   Params p;
   p.n_widen = n_widen;
-  if (n_widen < 0 || n_widen > MAX_WIDEN) return SB_ERR_ARG;
+  if (n_widen < 0 || n_widen > MAX_WIDEN || (n_widen && !widen)) return SB_ERR_ARG;
   for (int i = 0; i < n_widen; ++i) {
     const int64_t* j = widen + 5 * i;
     if (!j[0] || !j[1] || !j[2] || j[3] <= 0 || j[3] > INT_MAX || j[4] <= 0 || j[4] > INT_MAX || (j[4] & 15)) return SB_ERR_ARG;
