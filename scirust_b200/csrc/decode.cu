@@ -1540,8 +1540,8 @@ decode_attn_kernel(const __grid_constant__ DecodeAttnParams p) {
 // Two groups of four consumer warps take the tiles of a piece in turn (one group alone needs 1650 cycles for a tile that
 // memory delivers in 1400); warp w of a group owns positions [16w, 16w + 16), as above.
 // Head dimension 128 only: at 64 the tiles are half the bytes for the same consumer work, and the kernel above is as fast
-// or faster up to 64 x 2048 positions (36.9 us against 37.1). Where the line lies at 128, with figures: ops/decode.py,
-// _stream_wins. 64 sequences of 1536-2048 positions, 8 kv heads: 108.5 us above (4.3 TB/s), 87.5 us here (5.4 TB/s).
+// or faster up to 64 x 2048 positions (38.8 us against 39.3, with four groups of consumers 42.5). Where the line lies at 128, with
+// figures: ops/decode.py, _stream_wins. 64 sequences of 1536-2048 positions, 8 kv heads: 111 us above, 83.5 us here (5.7 TB/s).
 // ---------------------------------------------------------------------------
 constexpr int DST_THREADS = 384;         // warps 0-7 consume (two groups of four, every other tile each), 8 produces, 9-11 finish
 constexpr int DST_FINISHERS = 96;        // a CTA's registers are given to warps by the four, so these three cost none
