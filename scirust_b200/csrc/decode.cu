@@ -1625,7 +1625,13 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
   const long long T = static_cast<long long>(prefix[p.B]) * Hkv;
   const long long grid = min(static_cast<long long>(gridDim.x), T);     // every CTA of the deal has a unit
   if (blockIdx.x >= grid) return;
-  const long long u0 = blockIdx.x * T / grid, u1 = (blockIdx.x + 1) * T / grid;
+  // Divisions of whole 64-bit numbers take hundreds of cycles, and several stand before the first copy and behind the last tile; up to
+  // 29 million tiles on 148 CTAs 32 bits hold every dividend. 1 x 2048 positions 9.8 -> 9.5 us, 16 x 512 16.3 -> 15.8.
+  const bool narrow = (T + 1) * grid <= 0xffffffffll;
+  auto quotient = [&](long long a, long long d) -> long long {
+    return narrow ? static_cast<long long>(static_cast<uint32_t>(a) / static_cast<uint32_t>(d)) : a / d;
+  };
+  const long long u0 = quotient(blockIdx.x * T, grid), u1 = quotient((blockIdx.x + 1) * T, grid);
   int b_first = 0;
   {
     int lo = 0, hi = p.B - 1;                  // last sequence whose first unit is <= u0
@@ -1866,6 +1872,11 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
     locate(u);
     const bool last = u + (t_end - t_beg) >= u1;
     const int nf = DST_FINISHERS + (last ? 32 : 0);
+    // CTAs that share this job: c is the owner of unit v when c * T / grid <= v < (c + 1) * T / grid
+    const int c_first = static_cast<int>(quotient((s_job + 1) * grid - 1, T));
+    const int c_last = static_cast<int>(quotient((s_job + nt) * grid - 1, T));
+    // the first sharing CTA's piece is its second slot unless its range starts with this job
+    const int first_odd = quotient(c_first * T, grid) < s_job ? 1 : 0;
     // the last piece has barriers of its own: the producer comes to them while the others are still at pieces before it
     if (last) asm volatile("bar.sync 4, %0;" ::"n"(256 + DST_FINISHERS + 32) : "memory");
     else asm volatile("bar.sync 1, %0;" ::"n"(256 + DST_FINISHERS) : "memory");
@@ -1887,9 +1898,6 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
         d16[2] = static_cast<uint16_t>(pk.y); d16[3] = static_cast<uint16_t>(pk.y >> 16);
       }
     };
-    // CTAs that share this job: c is the owner of unit v when c * T / grid <= v < (c + 1) * T / grid
-    const int c_first = static_cast<int>(((s_job + 1) * grid - 1) / T);
-    const int c_last = static_cast<int>(((s_job + nt) * grid - 1) / T);
     constexpr int SLOT = 16 * (DH + 2);
     // a CTA's first piece goes to slot 2c, a later one (a job that starts inside its range) to 2c + 1
     float* slot = p.part + static_cast<size_t>(2 * blockIdx.x + (u == u0 ? 0 : 1)) * SLOT;
@@ -1927,8 +1935,6 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
       if (s_last) {
         __threadfence();
         const int np = c_last - c_first + 1;
-        // the first sharing CTA's piece is its second slot unless its range starts with this job
-        const int first_odd = c_first * T / grid < s_job ? 1 : 0;
         const float* base = p.part + static_cast<size_t>(2 * c_first) * SLOT;
         auto piece = [&](int s) { return base + static_cast<size_t>(2 * s + (s == 0 ? first_odd : 0)) * SLOT; };
         // a piece's (max, sum) of every row first, all loads at once; a warp then turns a row's maxima into weights, and the
