@@ -160,6 +160,13 @@ rmsnorm_fwd_row_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bflo
 
 // RMSNorm backward, input gradient. With g = dy*w and r = inv_rms:
 //   dx = r * (g - x * r^2 * mean(g*x))   (+ optional residual-stream gradient `dres`)
+// Every rounding is spelt out: left to the compiler, which product of a sum it contracts changes with the code around it, and a dx that
+// rounds otherwise in a few places moves every gradient below it by its last bits. g = a * w is exact (two bf16 values).
+__device__ __forceinline__ float rms_dot(float dot, float a, float g, float b) { return __fmaf_rn(__fmul_rn(a, g), b, dot); }
+// Rows that stay in registers (512, 1024 and 2048 columns): r * (g - b k), one rounding in the bracket, and then d.
+__device__ __forceinline__ float rms_dx_reg(float r, float k, float a, float g, float b) {
+  return __fmul_rn(r, __fmaf_rn(-b, k, __fmul_rn(a, g)));
+}
 __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                       const __nv_bfloat16* __restrict__ w, const float* __restrict__ inv_rms,
                                       const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
@@ -175,7 +182,7 @@ __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, cons
     unpack8(*reinterpret_cast<const uint4*>(x + off + c), b);
     unpack8(*reinterpret_cast<const uint4*>(w + c), g);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dot += a[j] * g[j] * b[j];
+    for (int j = 0; j < 8; ++j) dot = rms_dot(dot, a[j], g[j], b[j]);
   }
   dot = warp_sum(dot);
   const float r = inv_rms[row];
@@ -185,20 +192,24 @@ __global__ void rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, cons
     unpack8(*reinterpret_cast<const uint4*>(dy + off + c), a);
     unpack8(*reinterpret_cast<const uint4*>(x + off + c), b);
     unpack8(*reinterpret_cast<const uint4*>(w + c), g);
+    // here b k is rounded before it is subtracted, and d is added in the rounding of the product
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = r * (a[j] * g[j] - b[j] * k);
+    for (int j = 0; j < 8; ++j) o[j] = __fmaf_rn(a[j], g[j], -__fmul_rn(b[j], k));
     if (dres) {
       float d[8];
       unpack8(*reinterpret_cast<const uint4*>(dres + off + c), d);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] += d[j];
+      for (int j = 0; j < 8; ++j) o[j] = __fmaf_rn(r, o[j], d[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = __fmul_rn(r, o[j]);
     }
     *reinterpret_cast<uint4*>(dx + off + c) = pack8(o);
   }
 }
 
 // The same for rows of NV * 256 columns (NV <= 8): dy and x of the row stay in registers, all loads are issued
-// before the first use, and the sums run in the order of the general kernel (same bits).
+// before the first use, and the sum runs in the order of the general kernel.
 template <int NV>
 __global__ void rmsnorm_bwd_dx_reg_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                           const __nv_bfloat16* __restrict__ w, const float* __restrict__ inv_rms,
@@ -224,7 +235,7 @@ __global__ void rmsnorm_bwd_dx_reg_kernel(const __nv_bfloat16* __restrict__ dy, 
     float a[8], b[8], g[8];
     unpack8(va[i], a); unpack8(vb[i], b); unpack8(vg[i], g);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dot += a[j] * g[j] * b[j];
+    for (int j = 0; j < 8; ++j) dot = rms_dot(dot, a[j], g[j], b[j]);
   }
   dot = warp_sum(dot);
   const float r = inv_rms[row];
@@ -234,12 +245,12 @@ __global__ void rmsnorm_bwd_dx_reg_kernel(const __nv_bfloat16* __restrict__ dy, 
     float a[8], b[8], g[8], o[8];
     unpack8(va[i], a); unpack8(vb[i], b); unpack8(vg[i], g);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = r * (a[j] * g[j] - b[j] * k);
+    for (int j = 0; j < 8; ++j) o[j] = rms_dx_reg(r, k, a[j], g[j], b[j]);
     if (dres) {
       float d[8];
       unpack8(vd[i], d);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] += d[j];
+      for (int j = 0; j < 8; ++j) o[j] = __fadd_rn(o[j], d[j]);
     }
     *reinterpret_cast<uint4*>(dx + off + lane * 8 + i * 256) = pack8(o);
   }
@@ -297,10 +308,10 @@ __global__ void rmsnorm_bwd_dw_partial_kernel(const __nv_bfloat16* __restrict__ 
 
 
 // Both gradients in one pass, for rows of NV * 256 columns (NV <= 4): dy and x are read once and not twice. A warp takes every
-// (warps of the grid)-th row, keeps the row in registers as above (the same dx bits) and adds its share of the gain's gradient to NV * 8
+// (warps of the grid)-th row, keeps the row in registers as above (the same dx to the bit) and adds its share of the gain's gradient to NV * 8
 // sums per lane; the warps of a CTA are added in warp order, the CTAs in stage 2. Two CTAs of eight warps per SM: 128 registers
 // hold the row and the sums, the gain lies in shared memory (with one CTA per SM this form lost to two passes). Bound by memory: 16384 x 1024
-// with a residual 21.4 + 14.4 + 4.3 us in two passes and their stage 2, 26.2 + 4.4 so; 999 x 1024 3.3 + 7.1 + 1.9 / 4.3 + 2.7.
+// with a residual 21.4 + 14.4 + 4.3 us in two passes and their stage 2, 26.7 + 4.4 so; 999 x 1024 3.3 + 7.1 + 1.9 / 4.3 + 2.7.
 constexpr int RB_WARPS = 8;
 template <int NV, bool RES>
 __global__ void __launch_bounds__(RB_WARPS * 32, 2)
@@ -336,7 +347,7 @@ rmsnorm_bwd_both_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
       unpack8(va[i], a); unpack8(vb[i], b); unpack8(s_w[lane + i * 32], g);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        dot += a[j] * g[j] * b[j];
+        dot = rms_dot(dot, a[j], g[j], b[j]);
         acc[i][j] += a[j] * b[j] * r;
       }
     }
@@ -353,12 +364,12 @@ rmsnorm_bwd_both_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
       float a[8], b[8], g[8], o[8];
       unpack8(va[i], a); unpack8(vb[i], b); unpack8(s_w[lane + i * 32], g);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = r * (a[j] * g[j] - b[j] * k);
+      for (int j = 0; j < 8; ++j) o[j] = rms_dx_reg(r, k, a[j], g[j], b[j]);
       if (RES) {
         float d[8];
         unpack8(vd[i], d);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += d[j];
+        for (int j = 0; j < 8; ++j) o[j] = __fadd_rn(o[j], d[j]);
       }
       *reinterpret_cast<uint4*>(dx + off + i * 256) = pack8(o);
     }

@@ -53,6 +53,17 @@ def test_rmsnorm_bwd_in_one_pass(rows, cols, res, out):
     assert (dw.float().cpu() - dw_ref).abs().max().item() <= lim
 
 
+@pytest.mark.parametrize("rows,cols", [(999, 512), (16384, 1024)])
+@pytest.mark.parametrize("res", [True, False])
+def test_rmsnorm_bwd_rounds_alike_with_and_without_the_gain(rows, cols, res):
+    """dx of the pass that takes both gradients against the kernel of dx alone: the same operations on the same roundings, so the same
+    bits. Enough elements that another contraction of r (g - x k) + d shows in a few of them."""
+    x, w, dy, dres = (_r(s, i).cuda() for i, s in enumerate([(rows, cols), (cols,), (rows, cols), (rows, cols)], 1))
+    inv = ops.rmsnorm_fwd(x, w)[1]
+    one, two = (ops.rmsnorm_bwd(dy, x, w, inv, dres=dres if res else None, want_dw=want)[0] for want in (True, False))
+    assert torch.equal(one, two)
+
+
 @pytest.mark.parametrize("dh", [64, 128])
 def test_rope_roundtrip_and_reference(dh):
     rows, heads, kv = 96, 4, 2
