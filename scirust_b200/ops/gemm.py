@@ -68,6 +68,12 @@ def _check2d(t: torch.Tensor, name: str) -> None:
                          f"{tuple(t.shape)} {t.dtype} strides {t.stride()}")
 
 
+def _check_out(out: torch.Tensor, M: int, N: int) -> None:
+    _check2d(out, "out")
+    if tuple(out.shape) != (M, N):
+        raise ValueError(f"out has shape {tuple(out.shape)}, expected {(M, N)}")
+
+
 # CTA-pair kernel (csrc/gemm_pair_tcgen05.cu): 256 x 256 tiles on two SMs. "auto" uses it for
 # products with at least one full wave of such tiles and no split-K; SB_GEMM_PAIR=0/1 forces it.
 PAIR_MODE = os.environ.get("SB_GEMM_PAIR", "auto")
@@ -152,9 +158,7 @@ def _gemm(a, b, M, N, K, a_mn, b_mn, out, residual, splits, bn, bias=None, widen
     if out is None:
         out = _lib.empty((M, N), torch.bfloat16, a.device)
     else:
-        _check2d(out, "out")
-        if tuple(out.shape) != (M, N):
-            raise ValueError(f"out has shape {tuple(out.shape)}, expected {(M, N)}")
+        _check_out(out, M, N)
     if residual is not None and not isinstance(residual, _Bias):
         _check2d(residual, "residual")
         if tuple(residual.shape) != (M, N):
@@ -246,7 +250,7 @@ def swiglu_in_epilogue(M: int, K: int, ff: int) -> bool:
     return K >= 1024 and ((M + 255) // 256) * ((ff + 127) // 128) >= 4 * (num_sms() // 2)
 
 
-def _swiglu_product(x, wgu, gu, act, widen=()):
+def _swiglu_product(x, wgu, gu, act, ld_act, widen=()):
     """One launch of the CTA-pair kernel: each CTA of a pair stages one half, gate columns and the matching up columns."""
     global launch_count
     M, K = x.shape
@@ -254,7 +258,7 @@ def _swiglu_product(x, wgu, gu, act, widen=()):
     _check2d(x, "x")
     _check2d(wgu, "wgu")
     args = (x.data_ptr(), wgu.data_ptr(), _lib.ptr(gu), None, M, N, K, x.stride(0), wgu.stride(0),
-            gu.stride(0) if gu is not None else 0, 0, 0, 1, None, act.data_ptr(), act.stride(0), N // 2, None, 0)
+            gu.stride(0) if gu is not None else 0, 0, 0, 1, None, act.data_ptr(), ld_act, N // 2, None, 0)
     st = _lib.status_word(x.device).data_ptr()
     if widen:
         table = _widen_table(widen)
@@ -264,24 +268,46 @@ def _swiglu_product(x, wgu, gu, act, widen=()):
     launch_count += 1
 
 
+def _act_pitch(act: torch.Tensor, M: int, ff: int) -> int:
+    """Row pitch of the [M, ff] result in a buffer that a caller has brought: a matrix of that shape with rows of its own pitch, or
+    whatever holds M * ff elements in one piece."""
+    if act.dtype != torch.bfloat16:
+        raise ValueError(f"act: expected bf16, got {act.dtype}")
+    if tuple(act.shape) == (M, ff) and act.stride(1) == 1 and (act.stride(0) >= ff or M == 1):
+        return max(act.stride(0), ff)
+    if act.is_contiguous() and act.numel() >= M * ff:
+        return ff
+    raise ValueError(f"act has shape {tuple(act.shape)} and strides {act.stride()}, expected {(M, ff)} or a buffer of as many elements")
+
+
 def matmul_nn_swiglu(x, wgu, out=None, act=None):
     """Gate/up projection with the SwiGLU fused into the GEMM epilogue: returns ``(gu, act)`` with
     ``gu = x @ wgu`` (bf16 ``[M, 2*ff]`` = [gate | up], kept for the backward pass) and
-    ``act = silu(gate) * up`` (bf16 ``[M, ff]``), bit-identical to ``swiglu_fwd(matmul_nn(x, wgu))``."""
+    ``act = silu(gate) * up`` (bf16 ``[M, ff]``), bit-identical to ``swiglu_fwd(matmul_nn(x, wgu))``. What is refused of ``out`` and
+    ``act`` does not depend on which kernels run."""
     M, K = x.shape
     K2, N = wgu.shape
     ff = N // 2
     if K != K2 or N % 2:
         raise ValueError("matmul_nn_swiglu: shape mismatch")
+    ld_act = ff
+    if x.is_cuda:
+        if out is not None:
+            _check_out(out, M, N)
+        if act is not None:
+            ld_act = _act_pitch(act, M, ff)
     if not (x.is_cuda and swiglu_in_epilogue(M, K, ff)):
         from . import basic
         gu = matmul_nn(x, wgu, out=out)
-        return gu, basic.swiglu_fwd(gu, out=act)
+        dense = gu if gu.is_contiguous() else gu.contiguous()      # that kernel takes and gives rows one behind the other
+        if ld_act == ff:
+            return gu, basic.swiglu_fwd(dense, out=act)
+        return gu, act.copy_(basic.swiglu_fwd(dense))
     if out is None:
         out = _lib.empty((M, N), torch.bfloat16, x.device)
     if act is None:
         act = _lib.empty((M, ff), torch.bfloat16, x.device)
-    _swiglu_product(x, wgu, out, act)
+    _swiglu_product(x, wgu, out, act, ld_act)
     return out, act
 
 
@@ -296,7 +322,7 @@ def matmul_nn_swiglu_act(x, wgu, widen=()):
         from . import basic
         return basic.swiglu_fwd(matmul_nn_beside(x, wgu, widen=widen) if widen else matmul_nn(x, wgu))
     act = _lib.empty((M, N // 2), torch.bfloat16, x.device)
-    _swiglu_product(x, wgu, None, act, widen)
+    _swiglu_product(x, wgu, None, act, N // 2, widen)
     return act
 
 

@@ -224,6 +224,38 @@ def test_swiglu_epilogue_without_the_product(M, K, ff, monkeypatch):
     _check(gu, x.float() @ wgu.float(), K)
 
 
+@pytest.mark.parametrize("fuse", [True, False])
+def test_swiglu_product_looks_at_the_buffers_it_is_given(fuse, monkeypatch):
+    """What does not hold the result is refused before anything is launched, whichever kernels would run; a matrix with rows of its
+    own pitch and a buffer of as many elements are filled, and nothing beside them."""
+    from scirust_b200.ops import gemm
+    monkeypatch.setattr(gemm, "FUSE_SWIGLU", fuse)
+    M, K, ff = 300, 128, 264
+    x, wgu = _mk((M, K), 1), _mk((K, 2 * ff), 2)
+    gu, act = ops.matmul_nn_swiglu(x, wgu)
+
+    def buf(*shape, dtype=torch.bfloat16):
+        return torch.full(shape, 7.0, dtype=dtype, device="cuda")
+
+    launched = gemm.launch_count
+    for out in (buf(M - 1, 2 * ff), buf(M, ff), buf(M, 2 * ff, dtype=torch.float32), buf(2 * ff, M).t(), buf(M * 2 * ff)):
+        with pytest.raises(ValueError):
+            ops.matmul_nn_swiglu(x, wgu, out=out)
+    for a in (buf(M - 1, ff), buf(M, ff, dtype=torch.float32), buf(ff, M).t(), buf(M, 2 * ff)[:, ::2], buf(1, ff).expand(M, ff)):
+        with pytest.raises(ValueError):
+            ops.matmul_nn_swiglu(x, wgu, act=a)
+    assert gemm.launch_count == launched
+    wide_out, wide_act = buf(M, 2 * ff + 8), buf(M, ff + 16)
+    got, a = ops.matmul_nn_swiglu(x, wgu, out=wide_out[:, :2 * ff], act=wide_act[:, :ff])
+    assert torch.equal(got, gu) and torch.equal(a, act)
+    assert bool((wide_out[:, 2 * ff:] == 7.0).all()) and bool((wide_act[:, ff:] == 7.0).all())
+    for shape in ((M * ff,), (3, M // 3, ff), (M + 1, ff)):
+        a = buf(*shape)
+        assert ops.matmul_nn_swiglu(x, wgu, act=a)[1] is a
+        assert torch.equal(a.view(-1)[:M * ff].view(M, ff), act) and bool((a.view(-1)[M * ff:] == 7.0).all())
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("quant", [None, "int8"])
 def test_prefill_with_the_swiglu_in_the_product(quant, monkeypatch):
     """The engine's feed-forward with and without it: the same logits and cache to the bit."""
