@@ -139,10 +139,14 @@ class _Bias:
         return 0
 
 
-def _widen_table(widen):
+def _widen_table(widen, device):
     """``[(q, scale, w), ...]`` as ``sb_gemm_pair_widen_bf16`` takes it; read before the call returns."""
     table = array.array("q")
     for q, scale, w in widen:
+        if not (q.dim() == 2 and q.dtype == torch.int8 and w.dtype == torch.bfloat16 and w.shape == q.shape
+                and scale.dtype == torch.float32 and scale.numel() == q.shape[1] and q.device == scale.device == w.device == device
+                and q.is_contiguous() and scale.is_contiguous() and w.is_contiguous()):
+            raise ValueError("widen: expected contiguous int8 [K, N], fp32 [N] and bf16 [K, N] on the device of the product")
         table.extend((q.data_ptr(), scale.data_ptr(), w.data_ptr(), *q.shape))
     return table
 
@@ -172,7 +176,7 @@ def _gemm(a, b, M, N, K, a_mn, b_mn, out, residual, splits, bn, bias=None, widen
                 a.stride(0), b.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
                 int(a_mn), int(b_mn), _lib.ptr(ws), None, 0, 0, None, 0)
         if widen:
-            table = _widen_table(widen)
+            table = _widen_table(widen, a.device)
             _lib.call("sb_gemm_pair_widen_bf16", *args, len(widen), table.buffer_info()[0], st.data_ptr(), _lib.stream())
         else:
             _lib.call("sb_gemm_pair_bf16", *args, st.data_ptr(), _lib.stream())
@@ -261,7 +265,7 @@ def _swiglu_product(x, wgu, gu, act, ld_act, widen=()):
             gu.stride(0) if gu is not None else 0, 0, 0, 1, None, act.data_ptr(), ld_act, N // 2, None, 0)
     st = _lib.status_word(x.device).data_ptr()
     if widen:
-        table = _widen_table(widen)
+        table = _widen_table(widen, x.device)
         _lib.call("sb_gemm_pair_widen_bf16", *args, len(widen), table.buffer_info()[0], st, _lib.stream())
     else:
         _lib.call("sb_gemm_pair_bf16", *args, st, _lib.stream())

@@ -319,6 +319,12 @@ def test_product_widens_int8_matrices_beside_itself(M, N, K, form, monkeypatch):
         assert bool((tail == 7.0).all())
     with pytest.raises((ValueError, RuntimeError)):            # a width that the expansion does not take
         gemm.matmul_nn_beside(x, w, None, [(jobs[0][0].view(16, 13), jobs[0][1][:13].clone(), jobs[0][2].view(16, 13))])
+    (q, scale, out), launched = jobs[0], gemm.launch_count
+    for bad in ((q, scale, out[:12]), (q, scale, out.float()), (q, scale[:8], out), (q, scale.double(), out), (q.int(), scale, out),
+                (q, scale, torch.empty(16, 13, dtype=torch.bfloat16, device="cuda").t()), (q.cpu(), scale, out), (q, scale, out.view(-1))):
+        with pytest.raises(ValueError):                        # buffers that would be read or written past their ends
+            gemm.matmul_nn_beside(x, w, None, [bad])
+    assert gemm.launch_count == launched
 
 
 @pytest.mark.parametrize("batch,seq,ff", [(1, 1100, 2816), (3, 683, 2824)])
