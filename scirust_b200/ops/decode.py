@@ -220,7 +220,7 @@ def gemv(x, w, residual=None, out=None, out_f32=None, splits=None, rms_weight=No
     fp, fs = (out_f32.data_ptr(), out_f32.stride(0)) if out_f32 is not None else (None, 0)
     wp, ws0, sp = wm.data_ptr(), wm.stride(0), w.scale.data_ptr() if quant else None
     pro, gain = (1, rms_weight.data_ptr()) if rms_weight is not None else (2 if swiglu else 0, None)
-    if M <= grp:
+    if 0 < M <= grp:                          # no rows: no launch below either
         _lib.call("sb_gemv", xp, xs, wp, ws0, sp, rp, rs, op, os_, fp, M, N, K, int(quant), splits, ws, pro, gain, float(eps), st,
                   stream)
         _g.launch_count += 1

@@ -43,6 +43,19 @@ def test_gemv_int8_and_quantize(M, K, N):
     assert (qw.dequantize().float() - qw.q.float() * qw.scale[None, :]).abs().max().item() <= 1e-2
 
 
+@pytest.mark.parametrize("quant", [False, True])
+def test_gemv_of_no_rows_is_empty(quant):
+    """As on the CPU: an empty result and no launch."""
+    w = _r((256, 512), 2)
+    w = D.quantize_per_channel(w) if quant else w
+    launched = _g.launch_count
+    assert tuple(D.gemv(_r((0, 256), 1), w, residual=_r((0, 512), 3)).shape) == (0, 512)
+    assert tuple(D.gemv(_r((0, 512), 1), w, swiglu=True).shape) == (0, 512)
+    f = torch.empty((0, 512), device="cuda")
+    assert D.gemv(_r((0, 256), 1), w, out_f32=f, rms_weight=_r((256,), 4)) is f
+    assert _g.launch_count == launched
+
+
 @pytest.mark.parametrize("dh,H,Hkv", [(64, 16, 4), (128, 32, 8), (128, 4, 4), (64, 16, 2), (128, 16, 1)])
 def test_paged_decode_attention(dh, H, Hkv):
     B, page, max_seq = 3, 16, 700
