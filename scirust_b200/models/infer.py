@@ -200,7 +200,7 @@ class InferenceEngine:
             return D.gemv(a, w, residual=x, swiglu=swiglu)
         if swiglu:
             a = ops.swiglu_fwd(a)
-        return self._linear(a, w, residual=x, widen=widen)
+        return self._linear(a, w, residual=x, **({"widen": widen} if widen else {}))     # a subclass's may not know of it
 
     def _linear(self, x, w, residual=None, widen=()):
         """``widen``: int8 matrices of later products that this one's launch expands (``_WidenAhead``)."""

@@ -114,6 +114,18 @@ def test_cached_paged_generation_equals_full_recompute():
         eng.generate(p, 100)
 
 
+def test_engine_with_a_product_of_its_own():
+    """A subclass whose ``_linear`` takes the activations, the matrix and a residual, and nothing else."""
+    class Adapted(InferenceEngine):
+        def _linear(self, x, w, residual=None):
+            return InferenceEngine._linear(self, x, w, residual)
+
+    m = GQADecoder(CFG, seed=1, init_std=0.2)
+    p = torch.randint(1, 256, (10, 9), generator=torch.Generator().manual_seed(0))
+    a, b = (cls(m, max_batch=10, max_seq=32, page=8).generate(p, 4) for cls in (Adapted, InferenceEngine))
+    assert torch.equal(a, b)
+
+
 def test_warmup_cosine_schedule():
     s = WarmupCosineSchedule(1.0, 0.1, 10, 110)
     assert s.lr_at(0) == 0.0 and s.lr_at(5) == pytest.approx(0.5) and s.lr_at(10) == pytest.approx(1.0)
