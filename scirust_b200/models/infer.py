@@ -220,6 +220,11 @@ class InferenceEngine:
             w = w.dequantize()
         return G.matmul_nn_beside(x, w, residual, widen) if widen else ops.matmul_nn(x, w, residual=residual)
 
+    def _products(self):
+        """The functions behind this engine's products. What is done across them (gate/up without ``_linear``, expanding one's matrix in
+        another's launch) is done only where they are known to go together: an override of one of them sees every product of its own."""
+        return tuple(getattr(getattr(self, name), "__func__", None) for name in ("_linear", "_proj_out", "_gated"))
+
     def _gated(self, x, w, widen=()):
         """silu(gate) * up of ``[gate | up] = x @ w`` in one launch, or None where that is not how ``_linear`` takes the product (by
         1024 rows int8 weights are expanded whatever their shape)."""
@@ -248,9 +253,9 @@ class InferenceEngine:
         seq_of = torch.arange(B, dtype=torch.int32, device=self.dev).repeat_interleave(P)
         pos = torch.arange(P, dtype=torch.int32, device=self.dev).repeat(B)
         x = ops.embed_fwd(self.embed, tok.reshape(-1))
-        cls = type(self)                 # a subclass with products of its own (tensor parallelism) expands before each
-        own = (cls._linear, cls._proj_out, cls._gated) == (InferenceEngine._linear, InferenceEngine._proj_out, InferenceEngine._gated)
-        product = _WidenAhead(self.layers if own and x.is_cuda else [], B * P).product
+        products = self._products()
+        product = _WidenAhead(self.layers if products == _OWN_PRODUCTS and x.is_cuda else [], B * P).product
+        gates = products in GATED_PRODUCTS
         for li, l in enumerate(self.layers):
             h, _ = ops.rmsnorm_fwd(x, l["rms1"], cfg.eps, want_inv=False)
             w, kw = product(l["wqkv"])
@@ -261,7 +266,7 @@ class InferenceEngine:
             x = self._proj_out(a, w, x, site="attn", **kw)
             h, _ = ops.rmsnorm_fwd(x, l["rms2"], cfg.eps, want_inv=False)
             w, kw = product(l["wgu"])
-            gu = self._gated(h, w, **kw)             # silu(gate) * up
+            gu = self._gated(h, w, **kw) if gates else None          # silu(gate) * up
             fused = gu is not None
             if not fused:
                 gu = self._linear(h, w, **kw)
@@ -436,6 +441,11 @@ class InferenceEngine:
                 out[:, i] = self.tokens[:B]
         _lib.check_status(self.dev) if self.dev.type == "cuda" else None
         return out
+
+
+_OWN_PRODUCTS = (InferenceEngine._linear, InferenceEngine._proj_out, InferenceEngine._gated)
+# Products whose feed-forward may take gate/up through ``_gated``: a class that replaces one of them enters its own here.
+GATED_PRODUCTS = {_OWN_PRODUCTS}
 
 
 def teacher_forced_logits(engine: "InferenceEngine", prompts: torch.Tensor, tokens: torch.Tensor) -> torch.Tensor:

@@ -24,7 +24,7 @@ import torch.distributed as dist
 from .. import ops
 from ..ops import decode as D
 from ..parallel.small_collectives import SmallCollectives
-from .infer import InferenceEngine
+from .infer import GATED_PRODUCTS, InferenceEngine
 from .sciagent import BF, GQADecoder
 
 SMALL_BYTES = 1 << 20      # partials up to this size (summed over ranks) take the latency path
@@ -171,3 +171,6 @@ class TPInferenceEngine(InferenceEngine):
         if self.region is not None:
             self.region.close()
             self.region = None
+
+
+GATED_PRODUCTS.add((TPInferenceEngine._linear, TPInferenceEngine._proj_out, TPInferenceEngine._gated))

@@ -275,6 +275,46 @@ def test_prefill_with_the_swiglu_in_the_product(quant, monkeypatch):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("how", ["_linear", "_proj_out", "instance"])
+def test_prefill_takes_every_product_of_a_subclass(how, monkeypatch):
+    """An engine with products of its own (an adapter, another quantisation) has all of them taken in a prefill, gate/up among
+    them, at sizes where the base class takes that one through its epilogue."""
+    from scirust_b200.models.infer import InferenceEngine
+    from scirust_b200.models.sciagent import GQADecoder, SciAgentConfig
+    from scirust_b200.ops import gemm
+
+    class Adapted(InferenceEngine):
+        pass
+
+    def linear(self, x, w, residual=None):
+        seen.append(tuple(w.shape))
+        return InferenceEngine._linear(self, x, w, residual) * 1.5
+
+    def proj_out(self, a, w, x, swiglu=False, site="attn"):
+        seen.append((site, swiglu))
+        return InferenceEngine._proj_out(self, a, w, x, swiglu, site)
+
+    if how != "instance":
+        setattr(Adapted, how, {"_linear": linear, "_proj_out": proj_out}[how])
+    cfg = SciAgentConfig(512, 256, 2, 4, 2, 512, 2048, 1e4)
+    model = GQADecoder(cfg, device="cuda", seed=3)
+    tokens = torch.randint(0, 512, (2, 600), generator=torch.Generator().manual_seed(1)).cuda()
+    got = []
+    for fuse in (True, False):
+        monkeypatch.setattr(gemm, "FUSE_SWIGLU", fuse)
+        seen = []
+        eng = Adapted(model, max_batch=2, max_seq=640)
+        if how == "instance":
+            eng._linear = lambda x, w, residual=None: linear(eng, x, w, residual)
+        got.append((eng.prefill(tokens).clone(), *eng.cache.pools))
+        want = ([("attn", False), ("mlp", True)] if how == "_proj_out" else
+                [(256, 512), (256, 256), (256, 1024), (512, 256)])
+        assert [s for s in seen if s in want] == want * 2
+    _lib.check_status()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("M,d,ff", [(512, 256, 128), (4096, 1024, 2816), (1000, 512, 264)])
 def test_swiglu_backward_epilogue_is_bitwise_the_unfused_path(M, d, ff, monkeypatch):
     from scirust_b200.ops import basic, gemm
