@@ -113,7 +113,8 @@ class _WidenAhead:
     gate/up with down 383 / 336, down with the next gate/up 224 / 199, qkv with the output matrix 82.8 / 78.4; more gains less than the
     next product would with it (qkv with down, 2.3 codes for one, 12 us, gate/up 47) or loses (output product with gate/up, 7 codes, 108
     / 114). At 1024 rows gate/up with three 219 / 202, down with gate/up 139 / 129; d 1024 at 2048 rows gate/up with three 43.5 / 34.4.
-    Up to three matrices more than before are in memory; one that does not fit there is expanded before its product."""
+    Up to three matrices more than without it are in memory; where memory runs out, for one of them or for what a layer needs beside
+    them (``run``), those expanded ahead are given back and every matrix is expanded before its product again."""
 
     AHEAD = 3
     # Rows times the elements of gate/up. Below it a layer waits for the host, whom planning costs more (12 us) than the launches that it
@@ -127,6 +128,8 @@ class _WidenAhead:
             self.order = [l[k] for l in layers for k in ("wqkv", "wo", "wgu", "wd")]
         self.at = 0
         self.wide = {}                 # position in the order -> bf16 matrix
+        self.taken = 0                 # matrices expanded ahead so far
+        self.ran_out = False
 
     def product(self, w):
         """The next product's matrix (expanded, or as it is) and what its launch is to expand, as keyword arguments."""
@@ -150,8 +153,21 @@ class _WidenAhead:
                 break
             room -= q.q.numel()
             self.wide[i] = out
+            self.taken += 1
             jobs.append((q.q, q.scale, out))
         return w, {"widen": jobs} if jobs else {}
+
+    def run(self, part, *args):
+        """``part(*args)``, a piece of a layer that can be run again; if memory runs out in it, once more with nothing expanded ahead. The
+        second run is outside the handler, whose exception holds on to what the first one had allocated."""
+        try:
+            return part(*args)
+        except torch.OutOfMemoryError:
+            if not self.taken:
+                raise
+            self.order, self.wide, self.taken = [], {}, 0
+            self.ran_out = True
+        return part(*args)
 
 
 class InferenceEngine:
@@ -238,6 +254,8 @@ class InferenceEngine:
         return ops.matmul_nn_swiglu_act(x, w, widen)
 
     # ------------------------------------------------------------------ prefill
+    _ahead_below = math.inf              # rows of a prefill in which memory ran out for matrices expanded ahead: fewer may still have them
+
     def prefill(self, tokens: torch.Tensor):
         """tokens [B, P] (all prompts the same length). Fills the cache, leaves the greedy next
         token of every sequence in ``self.tokens`` and returns the last-position logits [B, V]."""
@@ -254,25 +272,34 @@ class InferenceEngine:
         pos = torch.arange(P, dtype=torch.int32, device=self.dev).repeat(B)
         x = ops.embed_fwd(self.embed, tok.reshape(-1))
         products = self._products()
-        product = _WidenAhead(self.layers if products == _OWN_PRODUCTS and x.is_cuda else [], B * P).product
         gates = products in GATED_PRODUCTS
-        for li, l in enumerate(self.layers):
+        ahead = products == _OWN_PRODUCTS and x.is_cuda and B * P < self._ahead_below
+        plan = _WidenAhead(self.layers if ahead else [], B * P)
+
+        def attention(li, l, x):
             h, _ = ops.rmsnorm_fwd(x, l["rms1"], cfg.eps, want_inv=False)
-            w, kw = product(l["wqkv"])
+            w, kw = plan.product(l["wqkv"])
             qkv = self._linear(h, w, **kw)
             D.rope_kv_append(qkv, H, Hkv, dh, self.cos, self.sin, cache.pools[li], cache.block_table, cache.page, seq_of, pos)
             a, _ = att.attention_fwd(qkv, B, P, H, Hkv, dh, causal=True, want_lse=False)
-            w, kw = product(l["wo"])
-            x = self._proj_out(a, w, x, site="attn", **kw)
+            w, kw = plan.product(l["wo"])
+            return self._proj_out(a, w, x, site="attn", **kw)
+
+        def feed_forward(l, x):
             h, _ = ops.rmsnorm_fwd(x, l["rms2"], cfg.eps, want_inv=False)
-            w, kw = product(l["wgu"])
+            w, kw = plan.product(l["wgu"])
             gu = self._gated(h, w, **kw) if gates else None          # silu(gate) * up
             fused = gu is not None
             if not fused:
                 gu = self._linear(h, w, **kw)
-            w, kw = product(l["wd"])
-            x = self._proj_out(gu, w, x, swiglu=not fused, site="mlp", **kw)
-        w = None
+            w, kw = plan.product(l["wd"])
+            return self._proj_out(gu, w, x, swiglu=not fused, site="mlp", **kw)
+
+        for li, l in enumerate(self.layers):
+            x = plan.run(attention, li, l, x)
+            x = plan.run(feed_forward, l, x)
+        if plan.ran_out:
+            self._ahead_below = B * P
         last = x.view(B, P, -1)[:, -1, :].contiguous()
         logits = self.logits[:B]
         self._head(last, logits, rms_weight=self.rms_final)

@@ -2,6 +2,7 @@
 round trip with exact resume, cached generation vs full recompute, reference checkpoint."""
 import math
 import os
+import weakref
 
 import pytest
 import torch
@@ -124,6 +125,46 @@ def test_engine_with_a_product_of_its_own():
     p = torch.randint(1, 256, (10, 9), generator=torch.Generator().manual_seed(0))
     a, b = (cls(m, max_batch=10, max_seq=32, page=8).generate(p, 4) for cls in (Adapted, InferenceEngine))
     assert torch.equal(a, b)
+
+
+def test_memory_that_runs_out_beside_matrices_expanded_ahead():
+    """A piece of a layer is run again with those matrices given back, and with nothing left of what the first run had allocated;
+    where none had been expanded the error is the caller's."""
+    from scirust_b200.models.infer import _WidenAhead
+
+    class Block:
+        pass
+
+    alive = []
+
+    def part(runs):
+        mine = Block()
+        alive.append(weakref.ref(mine))
+        if len(alive) <= runs:
+            raise torch.OutOfMemoryError("no memory")
+        assert alive[0]() is None
+        return 7
+
+    def plan(taken):
+        alive.clear()
+        p = _WidenAhead([], 0)
+        p.order, p.wide, p.taken = ["a", "b"], {1: early} if taken else {}, taken
+        return p
+
+    early = Block()
+    p = plan(1)
+    gone = weakref.ref(early)
+    del early
+    assert p.run(part, 1) == 7 and p.ran_out and len(alive) == 2 and gone() is None
+    assert p.product("c") == ("c", {})
+    with pytest.raises(torch.OutOfMemoryError):       # once per plan
+        p.run(lambda: part(99))
+    early = Block()
+    for taken in (1, 0):                              # both runs fail; nothing was expanded ahead
+        p = plan(taken)
+        with pytest.raises(torch.OutOfMemoryError):
+            p.run(part, 99)
+        assert len(alive) == 1 + taken and p.ran_out is bool(taken)
 
 
 def test_warmup_cosine_schedule():

@@ -398,3 +398,53 @@ def test_prefill_that_widens_ahead(batch, seq, ff, monkeypatch):
     monkeypatch.undo()
     plan = _WidenAhead(eng.layers, batch * seq)            # too little work for the host to plan
     assert all(plan.product(l[k]) == (l[k], {}) for l in eng.layers for k in ("wqkv", "wo", "wgu", "wd"))
+
+
+@pytest.mark.parametrize("where", ["attention_fwd", "swiglu_fwd", "rmsnorm_fwd"])
+def test_prefill_gives_matrices_back_when_memory_runs_out(where, monkeypatch):
+    """An allocation that fails while matrices expanded ahead are held (here by exception, on the host): the piece of the layer is run
+    again without them, with the same logits and cache, and prompts of as many rows expand nothing ahead from then on."""
+    from scirust_b200.models import infer
+    from scirust_b200.models.sciagent import GQADecoder, SciAgentConfig
+    from scirust_b200.ops import gemm
+    monkeypatch.setattr(infer._WidenAhead, "WORK", 0)
+    monkeypatch.setattr(gemm, "FUSE_SWIGLU", False)
+    cfg = SciAgentConfig(512, 1024, 3, 16, 4, 2816, 2048, 1e4)
+    model = GQADecoder(cfg, device="cuda", seed=3)
+    tokens = torch.randint(0, 512, (1, 1100), generator=torch.Generator().manual_seed(1)).cuda()
+    plans, product = [], infer._WidenAhead.product
+
+    def watched(self, w):
+        if self not in plans:
+            plans.append(self)
+        return product(self, w)
+
+    monkeypatch.setattr(infer._WidenAhead, "product", watched)
+    eng = infer.InferenceEngine(model, quant="int8", max_batch=1, max_seq=1200)
+
+    def prefill():                                             # logits, and the cache in the order of the sequence
+        for p in eng.cache.pools:
+            p.zero_()
+        logits = eng.prefill(tokens).clone()
+        _lib.check_status()
+        return [logits, *(p[eng.cache.block_table[0, :18].long()] for p in eng.cache.pools)]
+
+    want = prefill()
+    assert plans[0].taken > 3 and not plans[0].ran_out
+    module = infer.att if where == "attention_fwd" else infer.ops
+    real, failed = getattr(module, where), []
+
+    def short_of_memory(*args, **kw):
+        if plans[-1].wide and len(plans) == 2 and not failed:
+            failed.append(1)
+            raise torch.OutOfMemoryError("no memory")
+        return real(*args, **kw)
+
+    monkeypatch.setattr(module, where, short_of_memory)
+    for _ in range(2):
+        for a, b in zip(want, prefill()):
+            assert torch.equal(a, b)
+    assert failed and plans[1].ran_out and not plans[1].order and not plans[2].taken and not plans[2].ran_out
+    monkeypatch.setattr(module, where, real)
+    eng.prefill(tokens[:, :1050])                              # fewer rows may again
+    assert plans[3].taken > 3
