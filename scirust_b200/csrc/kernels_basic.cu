@@ -1160,7 +1160,8 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* w, void* y, float* inv_
   CHECK_LAUNCH();
 }
 
-// The two gradients in one pass: 512 or 1024 columns, `parts` CTAs (at most one per eight rows is used), partial of parts * cols floats.
+// The two gradients in one pass: 512 or 1024 columns, partial of parts * cols floats. `parts` CTAs, at most one per eight rows: the order
+// of the gain gradient's sum follows from (rows, cols, parts).
 extern "C" int sb_rmsnorm_bwd_both(const void* dy, const void* x, const void* w, const float* inv_rms, const void* dres, void* dx,
                                    float* partial, int parts, float* dw_f32, void* dw_bf16, int rows, int cols, void* stream) {
   if (rows <= 0 || parts <= 0 || !partial || (cols != 512 && cols != 1024)) return SB_ERR_ARG;

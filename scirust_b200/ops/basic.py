@@ -44,6 +44,11 @@ def rmsnorm_fwd(x, w, eps=1e-5, out=None, want_inv=True):
     return out, inv
 
 
+# CTAs of the pass for both gradients: two on each of the 148 SMs of a B200, and a fixed number, so that the order of the gain gradient's
+# sum follows from (rows, cols) alone on every device, as in the two-pass form.
+_RMS_BOTH_CTAS = 296
+
+
 def rmsnorm_bwd(dy, x, w, inv, dres=None, dw_out=None, want_dw=True):
     """Returns (dx [+ dres], dw). dw is written into ``dw_out`` (bf16 or fp32 [cols]) if given."""
     rows, cols = x.shape
@@ -62,9 +67,9 @@ def rmsnorm_bwd(dy, x, w, inv, dres=None, dw_out=None, want_dw=True):
     dy = dy.contiguous()
     dx = torch.empty_like(x)
     part = dwf = dwb = None
-    both = want_dw and cols in (512, 1024)      # one pass for both gradients, two CTAs per SM
+    both = want_dw and cols in (512, 1024)      # one pass for both gradients
     if want_dw:
-        chunks = min((rows + 7) // 8, 2 * _g.num_sms(x.device)) if both else (rows + 255) // 256
+        chunks = min((rows + 7) // 8, _RMS_BOTH_CTAS) if both else (rows + 255) // 256
         part = _lib.empty(chunks * cols, torch.float32, x.device)
         if dw_out is None:
             dw_out = _lib.empty(cols, torch.float32, x.device)

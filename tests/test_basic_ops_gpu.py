@@ -64,6 +64,19 @@ def test_rmsnorm_bwd_rounds_alike_with_and_without_the_gain(rows, cols, res):
     assert torch.equal(one, two)
 
 
+@pytest.mark.parametrize("rows,cols", [(999, 512), (5000, 1024)])
+def test_rmsnorm_gain_gradient_does_not_depend_on_the_device(rows, cols, monkeypatch):
+    """The order of its sum follows from rows and columns: the same bits where the device says that it has other numbers of SMs."""
+    from scirust_b200.ops import basic
+    x, w, dy = (_r(s, i).cuda() for i, s in enumerate([(rows, cols), (cols,), (rows, cols)], 1))
+    inv = ops.rmsnorm_fwd(x, w)[1]
+    got = []
+    for sms in (148, 132, 20):
+        monkeypatch.setattr(basic._g, "num_sms", lambda device=None: sms)
+        got.append(ops.rmsnorm_bwd(dy, x, w, inv)[1])
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 @pytest.mark.parametrize("dh", [64, 128])
 def test_rope_roundtrip_and_reference(dh):
     rows, heads, kv = 96, 4, 2
