@@ -588,6 +588,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           send(pg, &tmap_c);
           send(pu, &tmap_rs.m[1]);
         }
+        // Past the last row and column the accumulator holds zeros, which the division below takes its slow path for, and a warp waits
+        // for all of its lanes: ones there instead, of which nothing is stored (us, 255 x 1024 x 37888 79.9 / 55.3, as 256 rows).
+        if (row >= p.M || colw + 64 > p.ff) {
+          const int live = row < p.M ? p.ff - colw : 0;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) pg[j] = 2 * j < live ? pg[j] : 0x3f803f80u;
+        }
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           // act from the bf16-rounded gate / up, exactly what the stand-alone kernel reads back
