@@ -245,7 +245,7 @@ class InferenceEngine:
         """silu(gate) * up of ``[gate | up] = x @ w`` in one launch, or None where that is not how ``_linear`` takes the product (by
         1024 rows int8 weights are expanded whatever their shape)."""
         M, (K, N) = x.shape[0], w.shape
-        if not x.is_cuda or M < 256 or not G.swiglu_in_epilogue(M, K, N // 2):
+        if not x.is_cuda or not G.swiglu_in_epilogue(M, K, N // 2):
             return None
         if isinstance(w, D.QuantWeight):
             if M < 1024 and N % 16 == 0:

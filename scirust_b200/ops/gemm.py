@@ -244,13 +244,15 @@ def swiglu_in_epilogue(M: int, K: int, ff: int) -> bool:
     """Whether the gate/up product of ``M`` rows writes ``silu(gate) * up`` itself. The epilogue takes as long as the main loop over about 1024
     rows of k, and that of the last tile of every CTA pair is not hidden, so it wants long k and at least four waves of tiles (256 x 128
     columns each of gate and up). Us, product and separate kernel / fused / fused without keeping [gate | up], M x K x ff: 16384 x 1024 x
-    2816 192 / 166 / 149, 4096 x 1024 x 2816 58.9 / 53.7 / 49.7, 2048 x 4096 x 14336 428 / 387 / 375, 1024 x 4096 x 11008 164 / 149 /
-    144; but 2048 x 1024 x 2816 37.4 / 37.2 / 33.1, 600 x 4096 x 11008 131 / 136 / 133, 999 x 1024 x 2816 28 / 37 / 35, 4096 x 512 x
-    1408 30 / 33 / 31."""
-    if PAIR_MODE == "0" or ff % 8 or FUSE_SWIGLU is False:
+    2816 184 / 161 / 147, 4096 x 1024 x 2816 51.4 / 47.4 / 42.3, 4000 rows 54.5 / 50.3 / 45.2, 2048 x 4096 x 14336 412 / 370 / 353, 1024 x
+    4096 x 11008 143 / 137 / 133; but 4096 x 512 x 1408 31.7 / 35.8 / 33.8. From one to four waves it is level or ahead as well (2048 x 1024 x
+    2816 38.9 / 34.2 / 30.9, 999 x 1024 x 2816 31.6 / 31.4 / 29.3, 600 x 4096 x 11008 105.7 / 101 / 98): the line dates from when ragged tiles
+    were slow, and has not been moved. Less than a tile of rows leaves most of the epilogue's warps without any: 8 x 1024 x 37888 44.2 /
+    50.3 / 49.9, 64 rows 39.1 / 42.5 / 40."""
+    if PAIR_MODE == "0" or ff % 8 or FUSE_SWIGLU is False or M < 256:
         return False
     if FUSE_SWIGLU:
-        return M >= 256
+        return True
     return K >= 1024 and ((M + 255) // 256) * ((ff + 127) // 128) >= 4 * (num_sms() // 2)
 
 

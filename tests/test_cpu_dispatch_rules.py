@@ -5,7 +5,9 @@ import subprocess
 from pathlib import Path
 
 import pytest
+import torch
 
+from scirust_b200.models.infer import _WidenAhead
 from scirust_b200.ops import attention as A, conv as C, decode as D, gemm as G
 
 
@@ -127,3 +129,33 @@ def test_splits_of_the_weight_stream(K, N, M, quant, splits):
 ])
 def test_splits_that_finish_in_a_cluster(K, N, M, quant, splits):
     assert D._gemv_splits(N, K, 512 if quant else 256, M, quant) == splits
+
+
+@pytest.mark.parametrize("M,K,ff,fused", [
+    # four waves of 256 x 128 tiles on 74 pairs, k of 1024, one whole tile of rows, columns by the eight
+    (16384, 1024, 2816, True), (4096, 1024, 2816, True), (4000, 1024, 2816, True), (1024, 4096, 11008, True), (2048, 4096, 14336, True),
+    (2048, 1024, 2816, False), (600, 4096, 11008, False), (4096, 512, 1408, False), (16384, 1023, 2816, False), (16384, 1024, 2820, False),
+    (512, 1024, 148 * 128, True), (512, 1024, 147 * 128, False),
+    (256, 1024, 296 * 128, True), (256, 1024, 295 * 128, False), (255, 1024, 296 * 128, False), (8, 1024, 65536, False),
+])
+def test_swiglu_in_the_epilogue(M, K, ff, fused, monkeypatch):
+    monkeypatch.setattr(G, "FUSE_SWIGLU", None)
+    monkeypatch.setattr(G, "PAIR_MODE", "auto")
+    assert G.swiglu_in_epilogue(M, K, ff) is fused
+    monkeypatch.setattr(G, "FUSE_SWIGLU", True)                     # forced: wherever the kernel takes the call
+    assert G.swiglu_in_epilogue(M, K, ff) is (M >= 256 and ff % 8 == 0)
+    for name, value in (("PAIR_MODE", "0"), ("FUSE_SWIGLU", False)):
+        monkeypatch.setattr(G, name, value)
+        assert not G.swiglu_in_epilogue(M, K, ff)
+
+
+@pytest.mark.parametrize("rows,d,ff,ahead", [
+    # 1024 rows, and 2^35 products of rows and elements of gate/up
+    (2048, 4096, 14336, True), (1024, 4096, 14336, True), (1023, 4096, 14336, False), (1024, 4096, 4096, True), (1023, 4096, 4096, False),
+    (1024, 4096, 4095, False), (8192, 1024, 2816, True), (5958, 1024, 2816, True), (5957, 1024, 2816, False), (2000, 1024, 2816, False),
+])
+def test_prefill_plans_expansions_for_long_prompts(rows, d, ff, ahead):
+    shapes = {"wqkv": (d, 3 * d // 2), "wo": (d, d), "wgu": (d, 2 * ff), "wd": (ff, d)}
+    layer = {k: torch.empty(s, dtype=torch.int8, device="meta") for k, s in shapes.items()}
+    assert bool(_WidenAhead([layer, layer], rows).order) is ahead
+    assert not _WidenAhead([], rows).order
