@@ -109,10 +109,14 @@ class OnnxGraph:
     """Parsed ONNX-JSON document."""
 
     def __init__(self, doc: dict):
+        if not isinstance(doc, dict):
+            raise ValueError(f"ONNX-JSON: expected an object, got {type(doc).__name__}")
         for k in ("name", "ir_version", "graph"):
             if k not in doc:
                 raise ValueError(f"ONNX-JSON: missing field {k!r}")
         g = doc["graph"]
+        if not isinstance(g, dict):
+            raise ValueError(f"ONNX-JSON: graph is {type(g).__name__}, expected an object")
         for k in ("inputs", "outputs", "nodes", "initializers"):
             if k not in g:
                 raise ValueError(f"ONNX-JSON: graph is missing {k!r}")

@@ -223,3 +223,12 @@ def test_cross_process_determinism_gate():
         assert r.returncode == 0, r.stderr[-2000:]
         sigs.append(r.stdout.strip().splitlines()[-1])
     assert sigs[0] == sigs[1] and len(sigs[0]) == 64
+
+
+@pytest.mark.parametrize("text", ["0", "null", "[]", '"name ir_version graph"', '["name", "ir_version", "graph"]',
+                                  '{"name": "m", "ir_version": 7, "graph": 3}',
+                                  '{"name": "m", "ir_version": 7, "graph": ["inputs", "outputs", "nodes", "initializers"]}'])
+def test_onnx_json_that_is_no_object_is_refused(text):
+    from scirust_b200.io import onnx_json as O
+    with pytest.raises(ValueError, match="ONNX-JSON"):
+        O.import_onnx_json(text)
