@@ -69,7 +69,7 @@ class BpeTokenizer:
                 a, b, c = m.split() if isinstance(m, str) else m
                 merges.append((int(a), int(b), int(c)))
             vocab = {str(k): int(v) for k, v in d["vocab"].items()}
-        except (KeyError, ValueError, TypeError, json.JSONDecodeError) as e:
+        except (KeyError, ValueError, TypeError, AttributeError, OverflowError) as e:
             raise ValueError(f"malformed tokenizer json: {e}") from None
         return BpeTokenizer(vocab, merges)
 

@@ -232,3 +232,10 @@ def test_onnx_json_that_is_no_object_is_refused(text):
     from scirust_b200.io import onnx_json as O
     with pytest.raises(ValueError, match="ONNX-JSON"):
         O.import_onnx_json(text)
+
+
+@pytest.mark.parametrize("text", ['{"merges": [], "vocab": []}', '{"merges": [], "vocab": {"a": Infinity}}', '{"merges": [[0, 1, Infinity]], "vocab": {}}'])
+def test_tokenizer_json_of_other_types_is_refused(text):
+    from scirust_b200.tokenizer import BpeTokenizer
+    with pytest.raises(ValueError, match="malformed"):
+        BpeTokenizer.from_json_str(text)
