@@ -387,6 +387,24 @@ struct BnFinish {
   int rows;
   float eps, momentum;
 };
+// of a column's sums of x and x*x
+__device__ __forceinline__ void bn_statistics(const BnFinish& f, int c, float sum, float sumsq) {
+  const float n = static_cast<float>(f.rows);
+  const float m = sum / n;
+  const float var = fmaxf(sumsq / n - m * m, 0.f);
+  f.o1[c] = m;
+  f.o2[c] = rsqrtf(var + f.eps);
+  if (f.run_mean) {
+    f.run_mean[c] = (1.f - f.momentum) * f.run_mean[c] + f.momentum * m;
+    const float unbiased = f.rows > 1 ? var * n / (n - 1.f) : var;
+    f.run_var[c] = (1.f - f.momentum) * f.run_var[c] + f.momentum * unbiased;
+  }
+}
+// of a column's sums of g and g*x
+__device__ __forceinline__ void bn_gradients(const BnFinish& f, int c, float sum_g, float sum_gx) {
+  f.o1[c] = sum_g;
+  f.o2[c] = (sum_gx - f.mean[c] * sum_g) * f.inv_std[c];
+}
 constexpr int CF_COLS = 8, CF_CHUNKS = 512, CF_THREADS = 256;
 template <int WHAT>
 __global__ void __launch_bounds__(CF_THREADS)
@@ -421,38 +439,19 @@ colstats_finish_kernel(const float* __restrict__ partial, int chunks, int C, con
     f.o1[c] = acc;
     f.o2[c] = other;
   } else if (WHAT == FIN_FORWARD) {
-    const float n = static_cast<float>(f.rows);
-    const float m = acc / n;
-    const float var = fmaxf(other / n - m * m, 0.f);
-    f.o1[c] = m;
-    f.o2[c] = rsqrtf(var + f.eps);
-    if (f.run_mean) {
-      f.run_mean[c] = (1.f - f.momentum) * f.run_mean[c] + f.momentum * m;
-      const float unbiased = f.rows > 1 ? var * n / (n - 1.f) : var;
-      f.run_var[c] = (1.f - f.momentum) * f.run_var[c] + f.momentum * unbiased;
-    }
+    bn_statistics(f, c, acc, other);
   } else {
-    f.o1[c] = acc;
-    f.o2[c] = (other - f.mean[c] * acc) * f.inv_std[c];
+    bn_gradients(f, c, acc, other);
   }
 }
 
-// BatchNorm forward from sums taken elsewhere: mean and variance as in FIN_FORWARD above.
-__global__ void bn_prepare_kernel(const float* __restrict__ sum, const float* __restrict__ sumsq, int rows, int C,
-                                  float eps, float momentum, float* __restrict__ mean, float* __restrict__ inv_std,
-                                  float* __restrict__ run_mean, float* __restrict__ run_var) {
+// The same from sums taken elsewhere (the C entries that begin with a layer's sums).
+template <int WHAT>
+__global__ void bn_from_sums_kernel(const float* __restrict__ s1, const float* __restrict__ s2, int C, const BnFinish f) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
-  const float n = static_cast<float>(rows);
-  const float m = sum[c] / n;
-  const float var = fmaxf(sumsq[c] / n - m * m, 0.f);
-  mean[c] = m;
-  inv_std[c] = rsqrtf(var + eps);
-  if (run_mean) {
-    run_mean[c] = (1.f - momentum) * run_mean[c] + momentum * m;
-    const float unbiased = rows > 1 ? var * n / (n - 1.f) : var;
-    run_var[c] = (1.f - momentum) * run_var[c] + momentum * unbiased;
-  }
+  if (WHAT == FIN_FORWARD) bn_statistics(f, c, s1[c], s2[c]);
+  else bn_gradients(f, c, s1[c], s2[c]);
 }
 // y = (x - mean) * inv_std * gamma + beta, optional ReLU
 __global__ void bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ mean,
@@ -523,15 +522,6 @@ bn_apply_vec8_kernel(const uint4* __restrict__ x, const float* __restrict__ mean
 }
 // BatchNorm backward. With xhat = (x-mean)*inv_std, g = dy (already masked by ReLU when fused):
 //   dbeta = sum g, dgamma = sum g*xhat, dx = gamma*inv_std/n * (n*g - dbeta - xhat*dgamma)
-// sums come from colstats (a = g, b = x): sum g and sum g*x; dgamma = (sum g*x - mean*sum g)*inv_std.
-__global__ void bn_bwd_finish_kernel(const float* __restrict__ sum_g, const float* __restrict__ sum_gx,
-                                     const float* __restrict__ mean, const float* __restrict__ inv_std, int C,
-                                     float* __restrict__ dgamma, float* __restrict__ dbeta) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  dbeta[c] = sum_g[c];
-  dgamma[c] = (sum_gx[c] - mean[c] * sum_g[c]) * inv_std[c];
-}
 __global__ void bn_bwd_dx_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ x,
                                  const float* __restrict__ mean, const float* __restrict__ inv_std,
                                  const float* __restrict__ gamma, const float* __restrict__ dgamma,
@@ -748,8 +738,10 @@ extern "C" int sb_bn_fwd(const void* x, const float* sum, const float* sumsq, co
                          float eps, float momentum, int relu, int training, void* stream) {
   if (rows <= 0 || C <= 0) return SB_ERR_ARG;
   if (training) {
-    bn_prepare_kernel<<<(C + 127) / 128, 128, 0, STREAM>>>(sum, sumsq, rows, C, eps, momentum, mean, inv_std,
-                                                           run_mean, run_var);
+    BnFinish f = {};
+    f.o1 = mean; f.o2 = inv_std; f.run_mean = run_mean; f.run_var = run_var;
+    f.rows = rows; f.eps = eps; f.momentum = momentum;
+    bn_from_sums_kernel<FIN_FORWARD><<<(C + 127) / 128, 128, 0, STREAM>>>(sum, sumsq, C, f);
     if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   }
   return bn_apply(x, mean, inv_std, gamma, beta, nullptr, y, rows, C, relu, STREAM);
@@ -789,11 +781,14 @@ extern "C" int sb_bn_bwd_masked(const void* g, const void* x, const float* sum_g
                                 const float* mean, const float* inv_std, const float* gamma, float* dgamma,
                                 float* dbeta, const void* mask, void* dx, int rows, int C, void* stream) {
   if (rows <= 0 || C <= 0) return SB_ERR_ARG;
-  bn_bwd_finish_kernel<<<(C + 127) / 128, 128, 0, STREAM>>>(sum_g, sum_gx, mean, inv_std, C, dgamma, dbeta);
+  BnFinish f = {};
+  f.o1 = dbeta; f.o2 = dgamma; f.mean = mean; f.inv_std = inv_std;
+  bn_from_sums_kernel<FIN_BACKWARD><<<(C + 127) / 128, 128, 0, STREAM>>>(sum_g, sum_gx, C, f);
   if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   return bn_bwd_dx(g, x, mean, inv_std, gamma, dgamma, dbeta, mask, dx, rows, C, STREAM);
 }
-// The forms without a mask: entry points of their own in the C ABI.
+// The forms without a mask: entry points of their own in the C ABI. The layers above begin with sb_bn_layer_fwd / _bwd, hosts of the C ABI
+// that take the sums themselves (synchronised over ranks, say) with these.
 extern "C" int sb_colstats(const void* a, const void* b, float* partial, float* s1, float* s2, int rows, int C,
                            void* stream) {
   return sb_colstats_masked(a, b, nullptr, partial, s1, s2, rows, C, stream);

@@ -302,6 +302,21 @@ def test_cross_entropy_of_large_logits(cols):
     assert torch.equal(loss, ops.ce_loss_only(lg, tg))
 
 
+@pytest.mark.parametrize("n,V,d", [(1, 1, 8), (300, 7, 1032), (2500, 4000, 64)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_embedding_bwd_of_sorted_tokens_by_the_c_abi(n, V, d, accumulate):
+    """The entry that takes tokens sorted by the caller, which the Python side no longer calls: rows of a token in the order of their
+    positions, the same bits as the form that takes tokens as they are."""
+    from scirust_b200.ops import _lib
+    _lib.register("sb_embed_bwd", [_lib.vp] * 4 + [_lib.i32] * 4 + [_lib.vp])
+    tok = torch.randint(0, V, (n,), generator=torch.Generator().manual_seed(n)).cuda()
+    dy, base = _r((n, d), 11, 0.1).cuda(), _r((V, d), 12, 0.1).cuda()
+    order, perm = torch.sort(tok, stable=True)
+    got = base.clone() if accumulate else torch.zeros_like(base)
+    _lib.call("sb_embed_bwd", dy.data_ptr(), order.data_ptr(), perm.data_ptr(), got.data_ptr(), n, d, V, accumulate, _lib.stream())
+    assert torch.equal(got, ops.embed_bwd(dy, tok, base.clone(), accumulate=bool(accumulate)))
+
+
 @pytest.mark.parametrize("rows,H,Hkv,dh,page", [(129, 3, 1, 64, 16), (300, 4, 2, 128, 64), (257, 5, 1, 24, 8), (1000, 2, 2, 8, 64)])
 def test_rope_by_rows_fills_the_cache(rows, H, Hkv, dh, page):
     """A prompt's rotation with the copy to the cache (by rows, past 128 tokens) against the rotation and the copy by themselves: heads

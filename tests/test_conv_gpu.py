@@ -224,3 +224,56 @@ def test_convolution_of_master_weights(B, Cin, H, W, Cout, k, stride, pad):
     (y, dx, dw), want = got[0], got[1]
     assert torch.equal(y, want[0]) and torch.equal(dx, want[1])
     assert dw.dtype == torch.float32 and torch.equal(dw.to(BF).float(), want[2])
+
+
+@pytest.mark.parametrize("rows,C_", [(1, 8), (300, 12), (2050, 520), (1000, 7)])
+@pytest.mark.parametrize("relu", [True, False])
+def test_batchnorm_from_sums_by_the_c_abi(rows, C_, relu):
+    """The entries that take the sums apart from what is made of them, which the layer of the Python side no longer calls: the sums
+    against 64 bits (rows fp32 additions), and with them the results of the layer's entries to the bit, the statistics being the
+    same code."""
+    vp, i32, f32 = _lib.vp, _lib.i32, _lib.f32
+    _lib.register("sb_colstats_masked", [vp] * 6 + [i32, i32, vp])
+    _lib.register("sb_colstats", [vp] * 5 + [i32, i32, vp])
+    _lib.register("sb_bn_fwd", [vp] * 10 + [i32, i32, f32, f32, i32, i32, vp])
+    _lib.register("sb_bn_bwd_masked", [vp] * 11 + [i32, i32, vp])
+    _lib.register("sb_bn_bwd", [vp] * 10 + [i32, i32, vp])
+    g = torch.Generator(device="cuda").manual_seed(rows + C_)
+    x, dy = (torch.randn(rows, C_, generator=g, device="cuda").to(BF) for _ in range(2))
+    gamma, beta = torch.rand(C_, generator=g, device="cuda") + 0.5, torch.randn(C_, generator=g, device="cuda")
+    st = _lib.stream()
+
+    def new(*shape, dtype=torch.float32):
+        return torch.empty(shape, dtype=dtype, device="cuda")
+
+    def sums(a, b, mask):
+        part, s1, s2 = new(2 * ((rows + 255) // 256) * C_), new(C_), new(C_)
+        args = (part.data_ptr(), s1.data_ptr(), s2.data_ptr(), rows, C_, st)
+        if mask is None:
+            _lib.call("sb_colstats", a.data_ptr(), b.data_ptr(), *args)
+        else:
+            _lib.call("sb_colstats_masked", a.data_ptr(), b.data_ptr(), mask.data_ptr(), *args)
+        a64 = a.double() if mask is None else torch.where(mask > 0, a.double(), 0.0)
+        for got, terms in ((s1, a64), (s2, a64 * b.double())):
+            assert bool(((got.double() - terms.sum(0)).abs() <= terms.abs().sum(0) * rows * 2.0 ** -24 + 1e-30).all())
+        return s1, s2
+
+    s1, s2 = sums(x, x, None)
+    mean, inv, y = new(C_), new(C_), new(rows, C_, dtype=BF)
+    rm, rv = torch.zeros(C_, device="cuda"), torch.ones(C_, device="cuda")
+    _lib.call("sb_bn_fwd", x.data_ptr(), s1.data_ptr(), s2.data_ptr(), gamma.data_ptr(), beta.data_ptr(), mean.data_ptr(), inv.data_ptr(),
+              rm.data_ptr(), rv.data_ptr(), y.data_ptr(), rows, C_, 1e-5, 0.1, int(relu), 1, st)
+    xi, gi, bi = (t.clone().requires_grad_(True) for t in (x, gamma, beta))
+    rm2, rv2 = torch.zeros(C_, device="cuda"), torch.ones(C_, device="cuda")
+    y2 = C.batchnorm(xi, gi, bi, rm2, rv2, relu=relu)
+    assert torch.equal(y, y2.detach()) and torch.equal(rm, rm2) and torch.equal(rv, rv2)
+    mask = y if relu else None
+    s1, s2 = sums(dy, x, mask)
+    dgamma, dbeta, dx = new(C_), new(C_), new(rows, C_, dtype=BF)
+    args = [x.data_ptr(), s1.data_ptr(), s2.data_ptr(), mean.data_ptr(), inv.data_ptr(), gamma.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr()]
+    if relu:
+        _lib.call("sb_bn_bwd_masked", dy.data_ptr(), *args, mask.data_ptr(), dx.data_ptr(), rows, C_, st)
+    else:
+        _lib.call("sb_bn_bwd", dy.data_ptr(), *args, dx.data_ptr(), rows, C_, st)
+    for a, b in zip((dx, dgamma, dbeta), torch.autograd.grad(y2, (xi, gi, bi), dy)):
+        assert torch.equal(a, b)
