@@ -19,6 +19,8 @@
 
 namespace sb {
 
+int num_sms();   // gemm_tcgen05.cu
+
 // col[(b,oh,ow), (kh,kw,c)] = x[b, oh*s - pad + kh, ow*s - pad + kw, c] (0 outside); Kp = padded width
 __global__ void im2col_nhwc_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ col, int B,
                                    int H, int W, int C, int KH, int KW, int stride, int pad, int OH, int OW,
@@ -661,8 +663,10 @@ extern "C" int sb_maxpool_bwd(const void* dy, const void* arg, void* dx, int B, 
 }
 // Whether the kernels of eight channels a thread take a [rows, C] matrix (addresses aside).
 static bool bn_vec8(size_t total, int C) { return (C & 7) == 0 && total / 8 <= 0x7fffff00u; }
-// Words of a thread: see bn_apply_vec8_kernel. A small matrix keeps one, so that its words reach all SMs (148 x 4 blocks of 256).
-static int bn_words(size_t total, int C) { return 256 % (C / 8) == 0 && total / 8 >= 4u * 148 * 4 * 256 ? 4 : 1; }
+// Words of a thread: see bn_apply_vec8_kernel. A small matrix keeps one, so that its words reach all SMs (four blocks of 256 on each).
+static int bn_words(size_t total, int C) {
+  return 256 % (C / 8) == 0 && total / 8 >= 4u * num_sms() * 4 * 256 ? 4 : 1;
+}
 
 // Column sums of a and of a * b into `partial` (2 * ceil(rows/256) * C floats) and what WHAT makes of them. g_out: see colstats_vec8_kernel.
 template <int WHAT>
