@@ -309,14 +309,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 }
 
 // Adds split-K partials in split order 0..S-1 (fixed order => bitwise repeatable),
-// optionally adds a bf16 residual, rounds to bf16 (F32: leaves the sums as they are). Eight partials are on their way at once: a
-// weight gradient of a convolution has up to 64 and few elements (49 splits of 64 x 576: 8.3 us with one at a time, 6.1 so).
-template <bool F32>
+// optionally adds a bf16 residual, rounds to bf16 (F32: leaves the sums as they are). U partials are on their way at once: eight
+// from four splits on (a weight gradient of a convolution has up to 64 and few elements: 49 splits of 64 x 576 8.3 us with one at a
+// time, 6.1 with eight), one for fewer, where the unused places of eight cost (product and sum, us, one / eight: two splits, 999 x 1536 x
+// 1024 18.0 / 19.0; three, 300 x 4096 x 4096 19.25 / 19.35).
+template <bool F32, int U>
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, size_t mn, int N, void* __restrict__ C_, int ldc,
                                      const __nv_bfloat16* __restrict__ R, int ldr) {
   const size_t i4 = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (i4 >= mn) return;
-  constexpr int U = 8;
   float4 acc = __ldg(reinterpret_cast<const float4*>(part + i4));
   for (int s0 = 1; s0 < splits; s0 += U) {
     float4 v[U];
@@ -343,6 +344,9 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
     *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(C_) + row * ldc + col) = o;
   }
 }
+
+template <bool F32>
+static auto splitk_reduce(int splits) { return splits < 4 ? splitk_reduce_kernel<F32, 1> : splitk_reduce_kernel<F32, 8>; }
 
 // ------------------------------ host side ------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -562,8 +566,9 @@ extern "C" int sb_gemm_bf16(const void* A, const void* B, void* C, const void* R
     const size_t mn = static_cast<size_t>(M) * N;
     const int threads = 256;
     const unsigned blocks = static_cast<unsigned>((mn / 4 + threads - 1) / threads);
-    splitk_reduce_kernel<false><<<blocks, threads, 0, stream>>>(static_cast<const float*>(workspace), splits, mn, N, C, ldc,
-                                                                static_cast<const __nv_bfloat16*>(R), ldr);
+    auto kern = splitk_reduce<false>(splits);
+    kern<<<blocks, threads, 0, stream>>>(static_cast<const float*>(workspace), splits, mn, N, C, ldc,
+                                         static_cast<const __nv_bfloat16*>(R), ldr);
     if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
   }
   return 0;
@@ -656,7 +661,7 @@ static int conv_gemm(int mode, const void* a, const void* b, void* out, void* ke
   if (rc) return rc;
   if (splits > 1) {
     const size_t mn = static_cast<size_t>(p.M) * p.N;
-    auto kern = f32 ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>;
+    auto kern = f32 ? splitk_reduce<true>(splits) : splitk_reduce<false>(splits);
     kern<<<static_cast<unsigned>((mn / 4 + 255) / 256), 256, 0, stream>>>(static_cast<const float*>(workspace), splits, mn, p.N, out,
                                                                           p.N, nullptr, 0);
     if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;

@@ -91,6 +91,18 @@ def test_splitk_fixed_order_is_repeatable():
     _check(y3, ref, 8192)
 
 
+@pytest.mark.parametrize("splits", [2, 3, 4, 8, 9, 10])
+def test_splitk_adds_every_part_once(splits):
+    """Numbers of parts around what the sum has on its way at once. Operands in {-2..2} over 640 of k: sums are integers, exact in fp32,
+    and in bf16 up to 256, which they stay below by ten deviations."""
+    x, w, r = _ints((136, 640), 1), _ints((640, 264), 2), _ints((136, 264), 3)
+    want = x.float() @ w.float()
+    assert want.abs().max() < 250
+    assert torch.equal(ops.matmul_nn(x, w, splits=splits).float(), want)
+    assert torch.equal(ops.matmul_nn(x, w, residual=r, splits=splits).float(), want + r.float())
+    _lib.check_status()
+
+
 def test_strided_views():
     big = _mk((512, 3072), 11)
     x = big[:, 1024:2048]  # pitch 3072, offset 2048 bytes
