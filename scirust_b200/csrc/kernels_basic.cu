@@ -494,39 +494,96 @@ __global__ void embed_fwd_kernel(const __nv_bfloat16* __restrict__ table, const 
   for (int c = threadIdx.x; c < (d >> 3); c += blockDim.x) dst[c] = src[c];
 }
 
-__global__ void embed_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __restrict__ sorted_tok,
-                                 const int64_t* __restrict__ perm, __nv_bfloat16* __restrict__ dtable, int n, int d,
-                                 int vocab, int accumulate) {
-  const int i = blockIdx.x;
-  if (i >= n) return;
-  const int64_t tok = sorted_tok[i];
-  if (i > 0 && sorted_tok[i - 1] == tok) return;  // not a segment head
-  int64_t t = tok < 0 ? 0 : (tok >= vocab ? vocab - 1 : tok);
-  for (int c = threadIdx.x; c < (d >> 3); c += blockDim.x) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    uint4* dst = reinterpret_cast<uint4*>(dtable + static_cast<size_t>(t) * d) + c;
-    if (accumulate) unpack8(*dst, acc);
-    for (int j = i; j < n && sorted_tok[j] == tok; ++j) {
-      float f[8];
-      unpack8(reinterpret_cast<const uint4*>(dy + static_cast<size_t>(perm[j]) * d)[c], f);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] += f[k];
-    }
-    *dst = pack8(acc);
-  }
-}
-
-// The same gradient from the tokens as they are, without sorting them: three launches (a memset among them) instead of a radix sort's
-// ten. The positions of a token are chained through `next` from `head` by atomic exchanges, in whatever order those happen; a CTA
-// per position (and 1024, 2048 or 4096 columns, as the rows are long) looks whether its position heads the chain, puts the chain's positions in ascending order and adds
-// their rows in that order, so the sums do not depend on the chain's. Up to EB_SHORT positions are ranked in a warp; a longer
-// chain (padding, spaces) is not followed: the CTA reads the tokens from the front, 1024 at a time, and keeps those that are its own.
-// Bound by the rows of dy and of the table. 16384 tokens of 32000, d 1024: 110 us with the sort before it, 20 so; one token
-// in four the same 1370 / 380; 65536 of 128256, d 4096: 317 / 267 (408 with 1024 columns a CTA).
+// The embedding's gradient: rows of dy added to the table's row of their token, in fp32 and in the order of their positions.
 constexpr int EB_THREADS = 128, EB_SHORT = 32, EB_SCAN = 8;
 __device__ __forceinline__ int eb_token(int64_t t, int vocab) {
   return t < 0 ? 0 : t >= vocab ? vocab - 1 : static_cast<int>(t);
 }
+// A thread's columns: eight from c + w * EB_STEP, w < W, of a row; a CTA takes EB_THREADS * W words of 16 bytes of it.
+constexpr int EB_STEP = EB_THREADS * 8;
+__device__ __forceinline__ void eb_add(const uint4& v, float (&to)[8]) {
+  float f[8];
+  unpack8(v, f);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) to[k] += f[k];
+}
+// Rows at(0) .. at(m - 1) one after the other, the words of R rows on their way at once. The whole warp comes here.
+template <int W, int R, class At>
+__device__ __forceinline__ void eb_add_rows(const __nv_bfloat16* col, const At& at, int m, int c, int d, float (&acc)[W][8]) {
+  for (int j0 = 0; j0 < m; j0 += R) {
+    uint4 v[R][W];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const size_t row = static_cast<size_t>(at(j0 + u)) * d;
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        if (j0 + u < m && c + w * EB_STEP < d) v[u][w] = __ldg(reinterpret_cast<const uint4*>(col + row + w * EB_STEP));
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u)
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        if (j0 + u < m && c + w * EB_STEP < d) eb_add(v[u][w], acc[w]);
+  }
+}
+
+// From sorted tokens (stable, so the positions of a token ascend), in two launches. Runs of up to EB_SHORT places: a CTA per place looks
+// whether it heads one and adds its rows, one load of a thread at a time in 32 registers, so that all threads of an SM have one; where tokens
+// are spread this is what counts (131072 of 128256, d 1024: 133 us, with four rows in flight and fewer CTAs 220).
+__global__ void __launch_bounds__(EB_THREADS, 2048 / EB_THREADS)
+embed_bwd_short_runs_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __restrict__ sorted_tok, const int64_t* __restrict__ perm,
+                            __nv_bfloat16* __restrict__ dtable, int n, int d, int vocab, int accumulate) {
+  const int i = blockIdx.x;
+  const int64_t here = sorted_tok[i], before = sorted_tok[max(i - 1, 0)], far = sorted_tok[min(i + EB_SHORT, n - 1)];
+  const int t = eb_token(here, vocab);
+  if ((i > 0 && eb_token(before, vocab) == t) || (i + EB_SHORT < n && eb_token(far, vocab) == t)) return;
+  for (int c = threadIdx.x; c < (d >> 3); c += EB_THREADS) {
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint4* dst = reinterpret_cast<uint4*>(dtable + static_cast<size_t>(t) * d) + c;
+    if (accumulate) unpack8(*dst, acc);
+    for (int j = i; j < n && eb_token(sorted_tok[j], vocab) == t; ++j)
+      eb_add(reinterpret_cast<const uint4*>(dy + static_cast<size_t>(perm[j]) * d)[c], acc);
+    *dst = pack8(acc);
+  }
+}
+// Longer runs, whose rows are one chain of additions: eight on their way at once. A run of more than EB_SHORT places holds a place that is a
+// multiple of EB_SHORT; the CTA of the first of these takes it. Each warp reads the places by itself, 32 at a time and the next 32 while
+// the rows of these come, and passes positions by shuffles. 65536 tokens of 32000 with frequencies 1 / rank, d 1024: 3735 us one row at a
+// time, 956 so, d 4096 from 131072 29170 / 2108.
+static_assert(EB_SHORT == 32, "a warp looks back over the places before its own");
+__global__ void __launch_bounds__(EB_THREADS)
+embed_bwd_long_runs_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __restrict__ sorted_tok, const int64_t* __restrict__ perm,
+                           __nv_bfloat16* __restrict__ dtable, int n, int d, int vocab, int accumulate) {
+  const int place = blockIdx.x * EB_SHORT, lane = threadIdx.x & 31, c = (blockIdx.y * EB_THREADS + threadIdx.x) * 8;
+  if (c - lane * 8 >= d) return;                          // no column for this warp
+  const int t = eb_token(sorted_tok[place], vocab);
+  const int back = place - 1 - lane;
+  const uint32_t same = __ballot_sync(0xffffffffu, back >= 0 && eb_token(sorted_tok[back], vocab) == t);
+  if (same == 0xffffffffu) return;                        // the place EB_SHORT before is of the run too
+  const int first = place - __popc(same);
+  if (first + EB_SHORT >= n || eb_token(sorted_tok[first + EB_SHORT], vocab) != t) return;
+  uint4* dst = reinterpret_cast<uint4*>(dtable + static_cast<size_t>(t) * d + c);
+  float acc[1][8] = {};
+  if (accumulate && c < d) unpack8(*dst, acc[0]);
+  auto read = [&](int p) { return p < n && eb_token(sorted_tok[p], vocab) == t ? static_cast<int>(perm[p]) : -1; };
+  int mine = read(first + lane);
+  for (int base = first + 32;; base += 32) {
+    const int m = __popc(__ballot_sync(0xffffffffu, mine >= 0));        // a run is in one piece
+    const int next = m == 32 ? read(base + lane) : -1;
+    eb_add_rows<1, 8>(dy + c, [&](int j) { return __shfl_sync(0xffffffffu, mine, j & 31); }, m, c, d, acc);
+    if (m < 32) break;
+    mine = next;
+  }
+  if (c < d) *dst = pack8(acc[0]);
+}
+
+// From the tokens as they are, without sorting them: three launches (a memset among them) instead of a radix sort's
+// ten. The positions of a token are chained through `next` from `head` by atomic exchanges, in whatever order those happen; a CTA
+// per position (and 1024, 2048 or 4096 columns, as the rows are long) looks whether its position heads the chain, puts the chain's positions in ascending order and adds
+// their rows in that order, so the sums do not depend on the chain's. Up to EB_SHORT positions are ranked in a warp; a longer
+// chain (padding, spaces) is not followed: the CTA reads the tokens from the front, 1024 at a time, and keeps those that are its own,
+// which is why the tokens may not be too many (ops/basic.py).
+// Bound by the rows of dy and of the table. 16384 tokens of 32000, d 1024: 110 us with the sort before it, 20 so.
 __global__ void __launch_bounds__(256)
 embed_chain_kernel(const int64_t* __restrict__ tokens, int* __restrict__ head, int* __restrict__ next, int n, int vocab) {
   const int i = blockIdx.x * 256 + threadIdx.x;
@@ -540,8 +597,7 @@ embed_bwd_chain_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __re
   __shared__ int s_count[EB_SCAN * (EB_THREADS / 32)];
   __shared__ int s_n;
   const int i = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = (blockIdx.y * (EB_THREADS * W) + threadIdx.x) * 8;   // this thread's columns: eight from c + w * STEP, w < W
-  constexpr int STEP = EB_THREADS * 8;
+  const int c = (blockIdx.y * (EB_THREADS * W) + threadIdx.x) * 8;
   const int t = eb_token(tokens[i], vocab);
   // all that a token of a single position needs is asked for before the first answer is used
   const int first = head[t], after = next[i];
@@ -551,41 +607,19 @@ embed_bwd_chain_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __re
 #pragma unroll
   for (int w = 0; w < W; ++w) {
     own[w] = old[w] = make_uint4(0u, 0u, 0u, 0u);
-    if (c + w * STEP < d) {
-      own[w] = __ldg(reinterpret_cast<const uint4*>(col + static_cast<size_t>(i) * d + w * STEP));
-      if (accumulate && first == i) old[w] = *reinterpret_cast<const uint4*>(dst + w * STEP);
+    if (c + w * EB_STEP < d) {
+      own[w] = __ldg(reinterpret_cast<const uint4*>(col + static_cast<size_t>(i) * d + w * EB_STEP));
+      if (accumulate && first == i) old[w] = *reinterpret_cast<const uint4*>(dst + w * EB_STEP);
     }
   }
   if (first != i) return;                                // the same for the whole CTA
   float acc[W][8];
 #pragma unroll
   for (int w = 0; w < W; ++w) unpack8(old[w], acc[w]);
-  auto add_word = [&](const uint4& v, float (&to)[8]) {
-    float f[8];
-    unpack8(v, f);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) to[k] += f[k];
-  };
-  auto add_rows = [&](int m) {                           // rows s_list[0..m), four words on their way at once
-    constexpr int R = 4 / W;
-    for (int j0 = 0; j0 < m; j0 += R) {
-      uint4 v[R][W];
-#pragma unroll
-      for (int u = 0; u < R; ++u)
-#pragma unroll
-        for (int w = 0; w < W; ++w)
-          if (j0 + u < m && c + w * STEP < d)
-            v[u][w] = __ldg(reinterpret_cast<const uint4*>(col + static_cast<size_t>(s_list[j0 + u]) * d + w * STEP));
-#pragma unroll
-      for (int u = 0; u < R; ++u)
-#pragma unroll
-        for (int w = 0; w < W; ++w)
-          if (j0 + u < m && c + w * STEP < d) add_word(v[u][w], acc[w]);
-    }
-  };
+  auto add_rows = [&](int m) { eb_add_rows<W, 4 / W>(col, [&](int j) { return s_list[min(j, m - 1)]; }, m, c, d, acc); };
   if (after < 0) {
 #pragma unroll
-    for (int w = 0; w < W; ++w) add_word(own[w], acc[w]);
+    for (int w = 0; w < W; ++w) eb_add(own[w], acc[w]);
   } else {
     if (warp == 0) {
       int m = 0, at = i, mine = 0x7fffffff;              // the whole warp follows the chain; lane j keeps its j-th position
@@ -641,7 +675,7 @@ embed_bwd_chain_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __re
   }
 #pragma unroll
   for (int w = 0; w < W; ++w)
-    if (c + w * STEP < d) *reinterpret_cast<uint4*>(dst + w * STEP) = pack8(acc[w]);
+    if (c + w * EB_STEP < d) *reinterpret_cast<uint4*>(dst + w * EB_STEP) = pack8(acc[w]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1252,11 +1286,18 @@ extern "C" int sb_embed_fwd(const void* table, const int64_t* tokens, void* out,
                                           static_cast<__nv_bfloat16*>(out), n, d, vocab);
   CHECK_LAUNCH();
 }
+// From tokens sorted by the caller and the positions that they had.
 extern "C" int sb_embed_bwd(const void* dy, const int64_t* sorted_tok, const int64_t* perm, void* dtable, int n,
                             int d, int vocab, int accumulate, void* stream) {
-  if (n <= 0 || (d & 7) || !al16(dy) || !al16(dtable)) return SB_ERR_ARG;
-  embed_bwd_kernel<<<n, 128, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(dy), sorted_tok, perm,
-                                          static_cast<__nv_bfloat16*>(dtable), n, d, vocab, accumulate);
+  if (n <= 0 || d <= 0 || vocab <= 0 || (d & 7) || !al16(dy) || !al16(dtable)) return SB_ERR_ARG;
+  const int slabs = (d / 8 + EB_THREADS - 1) / EB_THREADS;
+  if (slabs > 65535) return SB_ERR_TOO_LARGE;
+  const __nv_bfloat16* from = static_cast<const __nv_bfloat16*>(dy);
+  __nv_bfloat16* to = static_cast<__nv_bfloat16*>(dtable);
+  embed_bwd_short_runs_kernel<<<n, EB_THREADS, 0, STREAM>>>(from, sorted_tok, perm, to, n, d, vocab, accumulate);
+  if (cudaGetLastError() != cudaSuccess) return SB_ERR_LAUNCH;
+  if (n > EB_SHORT)
+    embed_bwd_long_runs_kernel<<<dim3((n - 1) / EB_SHORT + 1, slabs), EB_THREADS, 0, STREAM>>>(from, sorted_tok, perm, to, n, d, vocab, accumulate);
   CHECK_LAUNCH();
 }
 

@@ -41,6 +41,7 @@ _CUDA_SIGS = {
     "sb_swiglu_bwd": [vp, vp, vp, i32, i32, vp],
     "sb_add_bf16": [vp, vp, vp, sz, vp],
     "sb_embed_fwd": [vp, vp, vp, i32, i32, i32, vp],
+    "sb_embed_bwd": [vp, vp, vp, vp, i32, i32, i32, i32, vp],
     "sb_embed_bwd_tokens": [vp, vp, vp, vp, i32, i32, i32, i32, vp],
     "sb_ce_fwd_bwd": [vp, vp, vp, vp, i32, i32, i32, f32, vp],
     "sb_ce_shard_stats": [vp, vp, vp, i32, i32, i32, i32, vp],

@@ -302,13 +302,35 @@ def test_cross_entropy_of_large_logits(cols):
     assert torch.equal(loss, ops.ce_loss_only(lg, tg))
 
 
+@pytest.mark.parametrize("n,V,d", [(1, 1, 8), (32, 1, 1032), (33, 1, 2056), (97, 1, 64), (1000, 7, 4096), (2500, 4000, 1024), (32769, 3000, 64)])
+@pytest.mark.parametrize("accumulate", [True, False])
+def test_embedding_bwd_of_many_tokens(n, V, d, accumulate, monkeypatch):
+    """Sorted tokens, which many take, against tokens as they are: rows in ascending order either way, so the same bits. Runs of 32
+    places and of one more, runs that begin on a multiple of 32 and beside one, several slabs of columns. Ids outside the table come
+    before and behind the others in the order: its first and last row, summed in another order."""
+    from scirust_b200.ops import basic
+    tok = torch.randint(0, V, (n,), generator=torch.Generator().manual_seed(n))
+    outside = n > 1000
+    if outside:
+        tok[::5] = 3
+        tok[torch.randperm(n)[:64]] = 2                       # with one id below, runs of 63 to 65 from the second place on
+        tok[1], tok[n - 1] = -5, V + 9
+    dy, base = _r((n, d), 11, 0.1).cuda(), _r((V, d), 12, 0.1).cuda()
+    got = []
+    for line in (n, n - 1):
+        monkeypatch.setattr(basic, "EMBED_CHAIN_TOKENS", line)
+        got.append(ops.embed_bwd(dy, tok.cuda(), base.clone(), accumulate=accumulate))
+    one, two = (g[1:-1] if outside else g for g in got)
+    assert torch.equal(one, two)
+    _close(*got, tol=2 ** -7)
+
+
 @pytest.mark.parametrize("n,V,d", [(1, 1, 8), (300, 7, 1032), (2500, 4000, 64)])
 @pytest.mark.parametrize("accumulate", [0, 1])
 def test_embedding_bwd_of_sorted_tokens_by_the_c_abi(n, V, d, accumulate):
-    """The entry that takes tokens sorted by the caller, which the Python side no longer calls: rows of a token in the order of their
-    positions, the same bits as the form that takes tokens as they are."""
+    """The entry that takes tokens sorted by the caller: rows of a token in the order of their positions, the same bits as the form
+    that takes tokens as they are."""
     from scirust_b200.ops import _lib
-    _lib.register("sb_embed_bwd", [_lib.vp] * 4 + [_lib.i32] * 4 + [_lib.vp])
     tok = torch.randint(0, V, (n,), generator=torch.Generator().manual_seed(n)).cuda()
     dy, base = _r((n, d), 11, 0.1).cuda(), _r((V, d), 12, 0.1).cuda()
     order, perm = torch.sort(tok, stable=True)
