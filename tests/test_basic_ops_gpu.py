@@ -339,6 +339,22 @@ def test_embedding_bwd_of_sorted_tokens_by_the_c_abi(n, V, d, accumulate):
     assert torch.equal(got, ops.embed_bwd(dy, tok, base.clone(), accumulate=bool(accumulate)))
 
 
+@pytest.mark.parametrize("rows,heads,dh", [(1, 1, 8), (33, 3, 24), (4736, 8, 64), (4737, 8, 64), (40000, 1, 64), (20000, 5, 24), (2400, 5, 256)])
+@pytest.mark.parametrize("backward", [False, True])
+def test_rope_by_words_and_by_heads(rows, heads, dh, backward):
+    """Both kernels around the line between them (a thread of the GPU's 148 x 2048 for each word of 16 bytes), one head, narrow heads. The rows
+    of a call one by one are its bits: rotations have no sums over rows."""
+    cos_t, sin_t = ops.rope_table(256, dh, 10000.0, "cuda")
+    x = _r((rows, (heads + 1) * dh), 5).cuda()
+    got = ops.rope_(x.clone(), heads, dh, 100, cos_t, sin_t, offset=7, backward=backward)
+    _close(got, ops.rope_(x.cpu(), heads, dh, 100, cos_t.cpu(), sin_t.cpu(), offset=7, backward=backward), 2 ** -8)
+    assert torch.equal(got[:, heads * dh:], x[:, heads * dh:])
+    part = x[rows // 2:][:50].clone()
+    pos = (torch.arange(rows)[rows // 2:][:50] % 100 + 7).int().cuda()
+    ops.rope_(part, heads, dh, 100, cos_t, sin_t, positions=pos, backward=backward)
+    assert torch.equal(part, got[rows // 2:][:50])
+
+
 @pytest.mark.parametrize("rows,H,Hkv,dh,page", [(129, 3, 1, 64, 16), (300, 4, 2, 128, 64), (257, 5, 1, 24, 8), (1000, 2, 2, 8, 64)])
 def test_rope_by_rows_fills_the_cache(rows, H, Hkv, dh, page):
     """A prompt's rotation with the copy to the cache (by rows, past 128 tokens) against the rotation and the copy by themselves: heads
