@@ -1536,7 +1536,7 @@ decode_attn_kernel(const __grid_constant__ DecodeAttnParams p) {
 // producer warp fills with 128-byte-swizzled TMA boxes, and the 64-position tiles of all (sequence, kv head) jobs, laid
 // end to end, are dealt out in equal contiguous ranges, so lengths may be as ragged as they like. A job that ends up in
 // several CTAs is merged by the last of them to finish, pieces in tile order (a counter, no data atomics): the
-// summation tree depends on the lengths and the grid only. Three warps do all merging beside the stream.
+// summation tree depends on the lengths and the grid only. Three warps do the merging beside the stream.
 // Two groups of four consumer warps take the tiles of a piece in turn (one group alone needs 1650 cycles for a tile that
 // memory delivers in 1400); warp w of a group owns positions [16w, 16w + 16), as above.
 // Head dimension 128 only: at 64 the tiles are half the bytes for the same consumer work, and the kernel above is as fast
@@ -1574,11 +1574,13 @@ struct DstCfg {
   }
   static constexpr int smem_bytes(int G) { return stages(G) * 2 * TILE_BYTES + fixed_bytes(G); }
 };
+static_assert(DST_THREADS == 256 + DST_FINISHERS + 32, "consumers, finishers, producer");
 static_assert(DstCfg::stages(16) >= 4 && DstCfg::stages(1) == DST_STAGES_MAX, "a ring of four to six stages");
 
 // Tiles of one sequence: an empty one keeps a tile without positions, whose job writes zeros.
 __device__ __forceinline__ int dst_tiles(int len) { return len > 0 ? (len + DEC_TK - 1) / DEC_TK : 1; }
 
+template <bool JOIN>
 __global__ void __launch_bounds__(DST_THREADS, 1)
 decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ DecodeStreamParams p) {
   using C = DstCfg;
@@ -1594,11 +1596,12 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
   float* sm_ml = sm_o + 8 * G * DH;                                                 // [8 warps][G rows][2]
   int* prefix = reinterpret_cast<int*>(sm_ml + 8 * G * 2);                          // [B + 1] tiles before sequence b
   int* lens = prefix + DST_MAX_B + 1;                                               // [B]
-  __shared__ int s_last;
+  __shared__ int s_last, s_pend;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap);
+    s_pend = 0;
     for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 8); }
     fence_barrier_init();
   }
@@ -1858,35 +1861,43 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
       }
       __syncwarp();
       if (u < u1) asm volatile("bar.arrive 1, %0;" ::"n"(256 + DST_FINISHERS) : "memory");
-      else asm volatile("bar.arrive 4, %0;" ::"n"(256 + DST_FINISHERS + 32) : "memory");
+      else if (!JOIN) asm volatile("bar.arrive 4, %0;" ::"n"(DST_THREADS) : "memory");
     }
-    return;
+    if (!JOIN) return;
   }
 
   // ------------------------------ finishers -----------------------------
   // They merge the eight warps in warp order and then the pieces of a job while the consumers are at the next piece, whose Q has been
-  // fetched meanwhile; at the CTA's last piece the producer helps. Consumers that did this themselves, the ring full behind them, took
-  // about 2 us a piece: 64 x 2048 positions 94 -> 85 us, 64 x 256 32.4 -> 25, 32 x 2048 54.5 -> 49, 1 x 2048 11.6 -> 11.2.
-  const int fw = (warp + 3) & 3, ft = fw * 32 + lane;      // warps 9, 10, 11 and 8
-  for (long long u = warp == 8 ? s_job + t_beg : u0; u < u1;) {
+  // fetched meanwhile; at the CTA's last piece the producer helps, and with JOIN (more rows than those four warps take at once) the
+  // consumers. Consumers that did all this themselves, the ring full behind them, took about 2 us a piece: 64 x 2048 positions 94 -> 85 us,
+  // 64 x 256 32.4 -> 25, 32 x 2048 54.5 -> 49, 1 x 2048 11.6 -> 11.2. Without their help at the end and without what is put off below,
+  // with it (us): 16 query heads per kv head 1 x 4096 18.6 / 15.9, 8 x 2048 of mixed lengths 31.5 / 23.7, seven 2 x 2048 20.6 / 17.2.
+  const int fw = warp < 8 ? 4 + warp : (warp + 3) & 3, ft = fw * 32 + lane;      // warps 9, 10, 11, 8 and then the consumers
+  for (long long u = warp <= 8 ? s_job + t_beg : u0; u < u1;) {
     locate(u);
     const bool last = u + (t_end - t_beg) >= u1;
-    const int nf = DST_FINISHERS + (last ? 32 : 0);
+    const int nf = DST_FINISHERS + (last ? (JOIN ? DST_THREADS - DST_FINISHERS : 32) : 0);
     // CTAs that share this job: c is the owner of unit v when c * T / grid <= v < (c + 1) * T / grid
-    const int c_first = static_cast<int>(quotient((s_job + 1) * grid - 1, T));
-    const int c_last = static_cast<int>(quotient((s_job + nt) * grid - 1, T));
-    // the first sharing CTA's piece is its second slot unless its range starts with this job
-    const int first_odd = quotient(c_first * T, grid) < s_job ? 1 : 0;
-    // the last piece has barriers of its own: the producer comes to them while the others are still at pieces before it
-    if (last) asm volatile("bar.sync 4, %0;" ::"n"(256 + DST_FINISHERS + 32) : "memory");
+    int c_first = 0, c_last = 0, first_odd = 0;
+    auto sharers = [&] {
+      c_first = static_cast<int>(quotient((s_job + 1) * grid - 1, T));
+      c_last = static_cast<int>(quotient((s_job + nt) * grid - 1, T));
+      // the first sharing CTA's piece is its second slot unless its range starts with this job
+      first_odd = quotient(c_first * T, grid) < s_job ? 1 : 0;
+    };
+    sharers();
+    // the last piece has barriers of its own: the producer comes to them while the others are still at pieces before it. The consumers
+    // are counted at the first of them in any case, having arrived or waiting here.
+    if (last) asm volatile("bar.sync 4, %0;" ::"n"(DST_THREADS) : "memory");
     else asm volatile("bar.sync 1, %0;" ::"n"(256 + DST_FINISHERS) : "memory");
     auto meet = [&] {
       __syncwarp();
-      if (last) asm volatile("bar.sync 5, %0;" ::"n"(DST_FINISHERS + 32) : "memory");
+      if (last && JOIN) asm volatile("bar.sync 5, %0;" ::"n"(DST_THREADS) : "memory");
+      else if (last) asm volatile("bar.sync 5, %0;" ::"n"(DST_FINISHERS + 32) : "memory");
       else asm volatile("bar.sync 3, %0;" ::"n"(DST_FINISHERS) : "memory");
     };
     const bool direct = t_beg == 0 && t_end == nt;
-    const int job = b * Hkv + kvh;
+    const long long after = u + (t_end - t_beg);
     auto store_out = [&](int g, int d, float lt, const float4& ot) {
       uint2 pk = make_uint2(0u, 0u);             // no weight: zeros, whatever the values held
       if (lt > 0.f) pk = make_uint2(dpack(ot.x / lt, ot.y / lt), dpack(ot.z / lt, ot.w / lt));
@@ -1927,70 +1938,83 @@ decode_attn_stream_kernel(const __grid_constant__ CUtensorMap tmap, const __grid
       __threadfence();
       meet();
       if (ft == 0) {
-        const unsigned int prev = atomicAdd(p.counters + job, 1u);
+        unsigned int* counter = p.counters + b * Hkv + kvh;
+        const unsigned int prev = atomicAdd(counter, 1u);
         s_last = (prev == static_cast<unsigned int>(c_last - c_first)) ? 1 : 0;
-        if (s_last) p.counters[job] = 0;
+        if (s_last) *counter = 0;
       }
       meet();
-      if (s_last) {
-        __threadfence();
-        const int np = c_last - c_first + 1;
-        const float* base = p.part + static_cast<size_t>(2 * c_first) * SLOT;
-        auto piece = [&](int s) { return base + static_cast<size_t>(2 * s + (s == 0 ? first_odd : 0)) * SLOT; };
-        // a piece's (max, sum) of every row first, all loads at once; a warp then turns a row's maxima into weights, and the
-        // sums take 16-byte loads (a job of 1 x 2048 positions has 16 pieces: 14.0 -> 10.7 us for the whole kernel)
-        float* w_m = sm_o;                             // [np][G] maxima, then weights
-        float* w_l = sm_o + np * G;                    // [np][G] sums; row g's total ends up in w_l[g]
-        // sixteen pieces' values of a thread's columns in flight, the first of them while the weights are made
-        float4 vo[16];
-        auto fetch = [&](int i, int s0) {
-          const int g = i / (DH / 4), d = (i - g * (DH / 4)) * 4;
+    }
+    // What is left of a job whose pieces have all come. With JOIN that of the CTA's first piece is put off to its end if few tiles are left
+    // by then (for the time that its rows take): the four warps would be at it when the last piece comes, which others may wait for. With
+    // fewer rows what this gains in such calls (four query heads, 2 x 2048 of mixed lengths, 4 kv heads 15.4 / 14.5) the code costs in all
+    // (2 x 2048, 8 kv heads 11.1 / 11.6).
+    const bool mine = !direct && s_last, put_off = JOIN && mine && !last && 4 * (u1 - after) <= G;
+    if (put_off && ft == 0) s_pend = 1;
+    for (int turn = mine && !put_off ? 0 : 1; turn < (JOIN && last && s_pend ? 2 : 1); ++turn) {
+      if (turn) {
+        meet();                                        // the merge buffers have been read
+        b = b_first;
+        locate(u0);
+        sharers();
+      }
+      __threadfence();
+      const int np = c_last - c_first + 1;
+      const float* base = p.part + static_cast<size_t>(2 * c_first) * SLOT;
+      auto piece = [&](int s) { return base + static_cast<size_t>(2 * s + (s == 0 ? first_odd : 0)) * SLOT; };
+      // a piece's (max, sum) of every row first, all loads at once; a warp then turns a row's maxima into weights, and the
+      // sums take 16-byte loads (a job of 1 x 2048 positions has 16 pieces: 14.0 -> 10.7 us for the whole kernel)
+      float* w_m = sm_o;                             // [np][G] maxima, then weights
+      float* w_l = sm_o + np * G;                    // [np][G] sums; row g's total ends up in w_l[g]
+      // sixteen pieces' values of a thread's columns in flight, the first of them while the weights are made
+      float4 vo[16];
+      auto fetch = [&](int i, int s0) {
+        const int g = i / (DH / 4), d = (i - g * (DH / 4)) * 4;
 #pragma unroll
-          for (int x = 0; x < 16; ++x)
-            if (s0 + x < np) vo[x] = __ldcg(reinterpret_cast<const float4*>(piece(s0 + x) + g * DH + d));
-        };
-        if (ft < G * (DH / 4)) fetch(ft, 0);
-        for (int i = ft; i < np * G; i += nf) {
-          const int s = i / G, g = i - s * G;
-          const float2 ml = __ldcg(reinterpret_cast<const float2*>(piece(s) + 16 * DH + g * 2));
-          w_m[i] = ml.x;
-          w_l[i] = ml.y;
+        for (int x = 0; x < 16; ++x)
+          if (s0 + x < np) vo[x] = __ldcg(reinterpret_cast<const float4*>(piece(s0 + x) + g * DH + d));
+      };
+      if (ft < G * (DH / 4)) fetch(ft, 0);
+      for (int i = ft; i < np * G; i += nf) {
+        const int s = i / G, g = i - s * G;
+        const float2 ml = __ldcg(reinterpret_cast<const float2*>(piece(s) + 16 * DH + g * 2));
+        w_m[i] = ml.x;
+        w_l[i] = ml.y;
+      }
+      meet();
+      for (int g = fw; g < G; g += nf / 32) {
+        float mt = -1.0e30f, lt = 0.f;
+        for (int s = lane; s < np; s += 32) mt = fmaxf(mt, w_m[s * G + g]);
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o2));
+        for (int s = lane; s < np; s += 32) {
+          const float wgt = exp2f(w_m[s * G + g] - mt);
+          w_m[s * G + g] = wgt;
+          lt += w_l[s * G + g] * wgt;
         }
-        meet();
-        for (int g = fw; g < G; g += nf / 32) {
-          float mt = -1.0e30f, lt = 0.f;
-          for (int s = lane; s < np; s += 32) mt = fmaxf(mt, w_m[s * G + g]);
 #pragma unroll
-          for (int o2 = 16; o2 > 0; o2 >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o2));
-          for (int s = lane; s < np; s += 32) {
-            const float wgt = exp2f(w_m[s * G + g] - mt);
-            w_m[s * G + g] = wgt;
-            lt += w_l[s * G + g] * wgt;
-          }
+        for (int o2 = 16; o2 > 0; o2 >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o2);
+        __syncwarp();
+        if (lane == 0) w_l[g] = lt;                  // row g of piece 0, read by this warp only
+      }
+      meet();
+      for (int i = ft; i < G * (DH / 4); i += nf) {
+        const int g = i / (DH / 4), d = (i - g * (DH / 4)) * 4;
+        float4 ot = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s0 = 0; s0 < np; s0 += 16) {                       // added in piece order
+          if (i != ft || s0 > 0) fetch(i, s0);
 #pragma unroll
-          for (int o2 = 16; o2 > 0; o2 >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o2);
-          __syncwarp();
-          if (lane == 0) w_l[g] = lt;                  // row g of piece 0, read by this warp only
-        }
-        meet();
-        for (int i = ft; i < G * (DH / 4); i += nf) {
-          const int g = i / (DH / 4), d = (i - g * (DH / 4)) * 4;
-          float4 ot = make_float4(0.f, 0.f, 0.f, 0.f);
-          for (int s0 = 0; s0 < np; s0 += 16) {                       // added in piece order
-            if (i != ft || s0 > 0) fetch(i, s0);
-#pragma unroll
-            for (int x = 0; x < 16; ++x) {
-              if (s0 + x < np) {
-                const float wgt = w_m[(s0 + x) * G + g];
-                ot.x += vo[x].x * wgt; ot.y += vo[x].y * wgt; ot.z += vo[x].z * wgt; ot.w += vo[x].w * wgt;
-              }
+          for (int x = 0; x < 16; ++x) {
+            if (s0 + x < np) {
+              const float wgt = w_m[(s0 + x) * G + g];
+              ot.x += vo[x].x * wgt; ot.y += vo[x].y * wgt; ot.z += vo[x].z * wgt; ot.w += vo[x].w * wgt;
             }
           }
-          store_out(g, d, w_l[g], ot);
         }
+        store_out(g, d, w_l[g], ot);
       }
     }
-    u += t_end - t_beg;
+    u = after;
     __syncwarp();
     if (!last) asm volatile("bar.arrive 2, %0;" ::"n"(256 + DST_FINISHERS) : "memory");   // the merge buffers are free again
   }
@@ -2450,13 +2474,11 @@ extern "C" int sb_decode_attention(const void* q, int ldq, const void* pool, con
   return dh == 64 ? launch_decode_attn<64>(p, grid, STREAM) : launch_decode_attn<128>(p, grid, STREAM);
 }
 
-static int launch_decode_stream(const CUtensorMap& tm, DecodeStreamParams p, int grid, cudaStream_t s) {
+template <bool JOIN>
+static int launch_decode_stream(const CUtensorMap& tm, const DecodeStreamParams& p, int grid, int smem, cudaStream_t s) {
   static PerDeviceOnce attr;
-  if (allow_smem(attr, decode_attn_stream_kernel, 227 * 1024 - 1024, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
-  const int G = p.H / p.Hkv;
-  p.stages = DstCfg::stages(G);
-  return launch_dep(decode_attn_stream_kernel, dim3(grid), dim3(DST_THREADS), DstCfg::smem_bytes(G), s, tm, p) == cudaSuccess
-             ? 0 : SB_ERR_LAUNCH;
+  if (allow_smem(attr, decode_attn_stream_kernel<JOIN>, 227 * 1024 - 1024, SB_ERR_LAUNCH)) return SB_ERR_LAUNCH;
+  return launch_dep(decode_attn_stream_kernel<JOIN>, dim3(grid), dim3(DST_THREADS), smem, s, tm, p) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
 }
 
 // The same attention as one balanced stream of KV tiles. pool: n_blocks pages (n_blocks * 2 * Hkv * page < 2^31, base
@@ -2485,7 +2507,11 @@ extern "C" int sb_decode_attention_stream(const void* q, int ldq, const void* po
   // a CTA with less than two tiles has nothing to overlap; more CTAs than that only add pieces to merge
   int grid = (max_tiles + 1) / 2;
   if (grid > num_sms()) grid = num_sms();
-  return launch_decode_stream(tm, p, grid, STREAM);
+  const int G = H / Hkv, smem = DstCfg::smem_bytes(G);
+  p.stages = DstCfg::stages(G);
+  // more rows than the four warps take at once
+  return G * (DstCfg::DH / 4) > DST_FINISHERS + 32 ? launch_decode_stream<true>(tm, p, grid, smem, STREAM)
+                                                   : launch_decode_stream<false>(tm, p, grid, smem, STREAM);
 }
 
 // logits: fp32 [rows, V]. pval/pidx: rows * ceil(V/4096) scratch. out_tokens: int64 [rows].

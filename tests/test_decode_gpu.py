@@ -276,6 +276,26 @@ def test_paged_decode_attention_stream(dh, H, Hkv, page, monkeypatch):
     _lib.check_status(torch.device("cuda"))
 
 
+@pytest.mark.parametrize("H,Hkv", [(4, 1), (5, 1), (14, 2), (16, 1)])
+def test_decode_attention_stream_of_jobs_that_share_a_cta(H, Hkv):
+    """Two tiles to a CTA and lengths that differ, so that CTAs end one job and begin the next: with more than four query heads the
+    consumers help to merge the last piece, and the job of the first may be put off behind it. Whichever CTA comes last, the sums are the same."""
+    dh, page = 128, 64
+    g = torch.Generator().manual_seed(H)
+    for B, longest in ((2, 2048), (3, 1500), (9, 300), (2, 700)):
+        max_blocks = (longest + page - 1) // page
+        pool = _r((B * max_blocks, 2, Hkv, page, dh), 3)
+        table = torch.randperm(B * max_blocks, generator=g).int().reshape(B, max_blocks).cuda()
+        q = _r((B, (H + 2 * Hkv) * dh), 20)
+        for _ in range(4):
+            lens = torch.randint(1, longest + 1, (B,), generator=g).int().cuda()
+            out, *again = (D.decode_attention(q, pool, table, page, lens, H, Hkv, dh, max_len=longest, stream=True) for _ in range(6))
+            assert all(torch.equal(out, o) for o in again)
+            ref = D.decode_attention_ref(q, pool, table, page, lens, H, Hkv, dh)
+            assert (out.float() - ref).abs().max().item() < 2e-2
+    _lib.check_status(torch.device("cuda"))
+
+
 def test_decode_attention_stream_repeats_under_load(monkeypatch):
     """The ring of the streamed attention refills a stage only after all eight consumer warps have passed its fill: many
     repetitions over long sequences give the same bits, and no bounded wait runs out."""
