@@ -253,11 +253,14 @@ __global__ void quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int ld
 // The same quantiser, one CTA per row, eight elements (16 bytes) per thread and step: the row is read once from memory,
 // the maximum is combined through shared memory. KEEP words a thread stay in registers, all loads in flight; what lies
 // beyond them is read again from L1 / L2. A few rows are bound by the latency of those loads: up to 4096 elements a word for each of 512
-// threads, from 8192 on four (us, 256 threads and nothing kept / so: 16 x 1024 2.3 / 2.1, 16 x 4096 3.0 / 2.5, 64 x 4096 3.1 / 2.6,
+// threads, from 8192 on four (us, 256 threads and nothing kept / so: 16 x 1024 2.2 / 2.05, 16 x 4096 2.8 / 2.4, 64 x 4096 2.8 / 2.5,
 // 16 x 14336 5.6 / 4.5). Many rows are bound by instructions, where the words that a thread does not have cost (1024 x 1024 3.4 and
-// 4.3 with one, 4096 x 4096 15.9 and 18.7), and so does the division: with it 1024 x 4096 8.2 us, 4096 x 4096 23.5, 1024 x 14336 21.0,
-// with a product that settles all but the halfway cases 6.3, 15.8, 16.6.
-template <int THREADS, int KEEP>
+// 4.3 with one, 4096 x 4096 15.9 and 18.7), and so does the division: with it 1024 x 4096 7.4 us, 4096 x 4096 22.5, 1024 x 14336 19.8,
+// with a product that settles all but the halfway cases (PRODUCT) 5.75, 14.5, 14.7. A word that has one takes both, about one in 600, and
+// what is bound by latency waits for the CTA that has most of them: up to one row per SM the product pays for a few long rows only (us,
+// product / division, eight draws: 16 x 14336 4.0 / 4.5, 32 4.5 / 4.55, 64 4.7 / 4.55, 148 4.9 / 4.75, 64 x 4096 2.53 / 2.48, 64 x 1024 2.21
+// / 2.11), beyond that from about a million elements on (512 x 2048 3.36 / 3.49, 256 x 2048 2.77 / 2.67, 1024 x 1024 3.48 / 3.38).
+template <int THREADS, int KEEP, bool PRODUCT>
 __global__ void __launch_bounds__(THREADS)
 quantize_rows_vec8_kernel(const __nv_bfloat16* x, int ldx, int8_t* q, int ldq, float* sx, int K) {
   pdl_trigger();
@@ -305,7 +308,7 @@ quantize_rows_vec8_kernel(const __nv_bfloat16* x, int ldx, int8_t* q, int ldq, f
       near_half |= !(fabsf(__fmaf_rn(f[j], inv, __fsub_rn(12582912.f, r))) <= 0.4999f);
       m[j] = __float_as_uint(r);
     }
-    if (!near_half) {
+    if (PRODUCT && !near_half) {
       qr[i] = make_uint2(__byte_perm(__byte_perm(m[0], m[1], 0x0040), __byte_perm(m[2], m[3], 0x0040), 0x5410),
                          __byte_perm(__byte_perm(m[4], m[5], 0x0040), __byte_perm(m[6], m[7], 0x0040), 0x5410));
       return;
@@ -340,7 +343,11 @@ extern "C" int sb_quantize_rows(const void* x, int ldx, void* xq, int ldq, float
       (reinterpret_cast<uintptr_t>(xq) & 7) == 0) {
     const bool keep = K >= 8192 && M <= 1024;
     const bool one = K <= 4096 && M <= num_sms();
-    auto kern = keep ? quantize_rows_vec8_kernel<512, 4> : one ? quantize_rows_vec8_kernel<512, 1> : quantize_rows_vec8_kernel<256, 0>;
+    const bool product = M <= num_sms() ? K >= 8192 && M <= 32
+                                        : K >= 4096 || static_cast<long long>(M) * K >= (K >= 2048 ? 1 << 20 : 1 << 21);
+    auto kern = keep ? (product ? quantize_rows_vec8_kernel<512, 4, true> : quantize_rows_vec8_kernel<512, 4, false>)
+                : one ? quantize_rows_vec8_kernel<512, 1, false>
+                : product ? quantize_rows_vec8_kernel<256, 0, true> : quantize_rows_vec8_kernel<256, 0, false>;
     return launch_dep(kern, dim3(M), dim3(keep || one ? 512 : 256), 0, STREAM, static_cast<const __nv_bfloat16*>(x), ldx,
                       static_cast<int8_t*>(xq), ldq, sx, K) == cudaSuccess ? 0 : SB_ERR_LAUNCH;
   }

@@ -541,7 +541,8 @@ def test_launches_of_the_weight_streaming_gemm_are_counted_as_they_are(quant, M,
     assert counted == (1 if ws.isnan().all() else 2)
 
 
-@pytest.mark.parametrize("M,K", [(3, 8), (16, 1000), (16, 4096), (149, 4096), (9, 4104), (2, 8192), (16, 14336)])
+@pytest.mark.parametrize("M,K", [(3, 8), (16, 1000), (16, 4096), (149, 4096), (9, 4104), (2, 8192), (16, 14336), (148, 4096), (32, 8192),
+                                 (33, 8192), (512, 2048), (511, 2048), (1025, 8192)])
 def test_row_quantiser_is_the_division_rounded(M, K):
     """Bit for bit the host statement on rows of halfway values, of one size, tiny, huge, denormal and with no number in them: the
     product by 1 / scale decides only where the division would decide the same."""
