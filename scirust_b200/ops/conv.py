@@ -257,8 +257,8 @@ class _BatchNorm(torch.autograd.Function):
             ds = dy
         elif ctx.added:                                 # the masked dy, written by the kernel that reads dy first
             ds = torch.empty_like(x)
-            if dy.data_ptr() % 16:
-                dy = dy.clone()
+            # which takes whole words only; the saved tensors may come from a hook
+            dy, x, mask = (t if t.data_ptr() % 16 == 0 else t.clone() for t in (dy, x, mask))
         part = torch.empty(2 * ((rows + 255) // 256) * C, dtype=torch.float32, device=x.device)
         dgamma = _lib.empty(C, torch.float32, x.device)
         dbeta = _lib.empty(C, torch.float32, x.device)

@@ -203,6 +203,27 @@ def test_batchnorm_adds_a_shortcut(rows, C_, relu, training):
         assert torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0)) and torch.equal(a.isnan(), b.isnan())
 
 
+@pytest.mark.parametrize("relu", [True, False])
+def test_batchnorm_with_a_shortcut_takes_what_saved_tensor_hooks_give(relu):
+    """Saved tensors that come back two bytes off a word: the gradients of those that do not."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, s, dy = (torch.randn(300, 64, generator=g, device="cuda").to(BF) for _ in range(3))
+    gamma, beta = torch.rand(64, generator=g, device="cuda") + 0.5, torch.randn(64, generator=g, device="cuda")
+
+    def beside(t):
+        buf = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+        return buf[1:1 + t.numel()].view(t.shape).copy_(t) if t.dtype == BF else t
+
+    got = []
+    for unpack in (beside, lambda t: t):
+        leaves = [t.clone().requires_grad_(True) for t in (x, gamma, beta, s)]
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            y = C.batchnorm(*leaves[:3], torch.zeros(64, device="cuda"), torch.ones(64, device="cuda"), relu=relu, shortcut=leaves[3])
+            got.append(torch.autograd.grad(y, leaves, dy))
+    for a, b in zip(*got):
+        assert (a.float() - b.float()).abs().max().item() <= 2 ** -7 * b.float().abs().max().item()
+
+
 @pytest.mark.parametrize("B,Cin,H,W,Cout,k,stride,pad", [
     (3, 64, 16, 16, 64, 3, 1, 1),       # three splits of the weight gradient
     (1, 64, 8, 8, 128, 1, 1, 0),        # one: its sum is not split
