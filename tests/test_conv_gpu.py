@@ -298,3 +298,23 @@ def test_batchnorm_from_sums_by_the_c_abi(rows, C_, relu):
         _lib.call("sb_bn_bwd", dy.data_ptr(), *args, dx.data_ptr(), rows, C_, st)
     for a, b in zip((dx, dgamma, dbeta), torch.autograd.grad(y2, (xi, gi, bi), dy)):
         assert torch.equal(a, b)
+
+
+def test_block_with_a_replaced_norm(monkeypatch):
+    """A norm whose ``forward`` somebody has replaced, in the class or on the instance, is called with what it takes."""
+    from scirust_b200.models import cnn
+    block = cnn.BasicBlock(64, 64, 1, torch.Generator().manual_seed(1)).cuda()
+    geom = C.ConvGeom(2, 8, 8, 64)
+    x = torch.relu(torch.randn(geom.rows, 64, generator=torch.Generator().manual_seed(2))).to(BF).cuda()
+    want = block(x, geom)[0]
+    forward, calls = cnn.BNLayer.forward, []
+
+    def watched(self, x):
+        calls.append(self)
+        return forward(self, x)
+
+    block.bn2.forward = lambda x: watched(block.bn2, x)
+    assert torch.equal(block(x, geom)[0], want) and calls == [block.bn2]
+    del block.bn2.forward
+    monkeypatch.setattr(cnn.BNLayer, "forward", watched)
+    assert torch.equal(block(x, geom)[0], want) and calls == [block.bn2, block.bn1, block.bn2]
