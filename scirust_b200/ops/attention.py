@@ -151,7 +151,10 @@ def attention_bwd(qkv, o, lse, do, B, S, H, Hkv, dh, causal=True, scale=None):
     scale = 1.0 / math.sqrt(dh) if scale is None else scale
     if not qkv.is_cuda:
         return attention_bwd_flash_ref(qkv, o, lse, do, B, S, H, Hkv, dh, causal, scale).to(qkv.dtype)
-    dqkv = torch.empty_like(qkv)
+    if qkv.dim() != 2 or qkv.stride(1) != 1 or qkv.dtype != torch.bfloat16:
+        raise ValueError("qkv must be a 2-D bf16 matrix with unit inner stride")
+    # the kernels write the gradient with the row pitch of qkv
+    dqkv = torch.empty((qkv.shape[0], qkv.stride(0)), dtype=qkv.dtype, device=qkv.device)[:, :qkv.shape[1]]
     delta = _lib.empty((B, H, S, 2), torch.float32, qkv.device)
     ds = _scratch(B, S, H, qkv.device)
     _lib.call("sb_attention_bwd", qkv.data_ptr(), o.data_ptr(), lse.data_ptr(), do.data_ptr(), dqkv.data_ptr(),

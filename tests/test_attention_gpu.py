@@ -153,3 +153,19 @@ def test_two_tiles_at_128_are_as_exact_as_one(causal, scale, monkeypatch):
         err.append(((o.double() - ref).norm() / ref.norm()).item())
     _lib.check_status()
     assert err[1] <= err[0] * 1.001, err
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,dh", [(2, 200, 4, 2, 64), (1, 333, 2, 1, 128)])
+def test_backward_of_rows_with_a_pitch(B, S, H, Hkv, dh):
+    """qkv as columns of a wider matrix: the gradient has that row pitch too, of memory that is its own, and the bits of the dense one."""
+    ld = (H + 2 * Hkv) * dh
+    g = torch.Generator(device="cuda").manual_seed(1)
+    wide = torch.randn(B * S, ld + 64, generator=g, device="cuda").to(torch.bfloat16)
+    do = torch.randn(B * S, H * dh, generator=g, device="cuda").to(torch.bfloat16)
+    qkv, dense = wide[:, :ld], wide[:, :ld].contiguous()
+    o, lse = A.attention_fwd(dense, B, S, H, Hkv, dh)
+    want = A.attention_bwd(dense, o, lse, do, B, S, H, Hkv, dh)
+    got = A.attention_bwd(qkv, o, lse, do, B, S, H, Hkv, dh)
+    _lib.check_status()
+    assert want.is_contiguous() and got.stride() == qkv.stride() and torch.equal(got, want)
+    assert got.untyped_storage().nbytes() >= B * S * (ld + 64) * 2
