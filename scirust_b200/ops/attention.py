@@ -68,7 +68,7 @@ def _scratch(B, S, H, device):
     n = B * H * S * ((S + 63) // 64 * 64)
     if n * 2 > DS_SCRATCH_LIMIT_BYTES:
         return None
-    key = str(device)
+    key = (str(device), _lib.stream())        # per stream: passes on two streams must not share it
     t = _ds_scratch.get(key)
     if t is None or t.numel() < n:
         t = _lib.empty(n, torch.bfloat16, device)

@@ -169,3 +169,13 @@ def test_backward_of_rows_with_a_pitch(B, S, H, Hkv, dh):
     _lib.check_status()
     assert want.is_contiguous() and got.stride() == qkv.stride() and torch.equal(got, want)
     assert got.untyped_storage().nbytes() >= B * S * (ld + 64) * 2
+
+
+def test_backward_scratch_belongs_to_a_stream():
+    """The dS tiles of two passes that may run at once lie in buffers of their own; a pass after another on its stream takes the same."""
+    device = torch.device("cuda", torch.cuda.current_device())
+    first = A._scratch(1, 64, 2, device)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        other = A._scratch(1, 64, 2, device)
+        assert A._scratch(1, 64, 2, device) is other
+    assert A._scratch(1, 64, 2, device) is first and other.data_ptr() != first.data_ptr()
