@@ -307,7 +307,8 @@ __global__ void rmsnorm_bwd_dw_partial_kernel(const __nv_bfloat16* __restrict__ 
 }
 
 
-// Both gradients in one pass, for rows of NV * 256 columns (NV <= 4): dy and x are read once and not twice. A warp takes every
+// Both gradients in one pass, for rows of NV * 256 columns (NV <= 4 by its registers; 512 and 1024 are the widths that the models here
+// have, 256 and 768 keep two passes and have not been timed): dy and x are read once and not twice. A warp takes every
 // (warps of the grid)-th row, keeps the row in registers as above (the same dx to the bit) and adds its share of the gain's gradient to NV * 8
 // sums per lane; the warps of a CTA are added in warp order, the CTAs in stage 2. Two CTAs of eight warps per SM: 128 registers
 // hold the row and the sums, the gain lies in shared memory (with one CTA per SM this form lost to two passes). Bound by memory: 16384 x 1024
