@@ -147,7 +147,7 @@ class _WidenAhead:
             q = self.order[i]
             if i in self.wide:
                 continue
-            if not isinstance(q, D.QuantWeight) or not q.widenable() or q.q.numel() > room:
+            if type(q) is not D.QuantWeight or not q.widenable() or q.q.numel() > room:      # a subclass may expand in its own way
                 break
             try:
                 out = torch.empty(q.shape, dtype=torch.bfloat16, device=q.q.device)

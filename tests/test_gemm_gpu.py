@@ -412,6 +412,31 @@ def test_prefill_that_widens_ahead(batch, seq, ff, monkeypatch):
     assert all(plan.product(l[k]) == (l[k], {}) for l in eng.layers for k in ("wqkv", "wo", "wgu", "wd"))
 
 
+def test_prefill_expands_a_kind_of_weight_of_its_own_by_its_own_method(monkeypatch):
+    """A subclass of the int8 weight with another meaning of its codes is not expanded beside a product."""
+    from scirust_b200.models import infer
+    from scirust_b200.models.sciagent import GQADecoder, SciAgentConfig
+    from scirust_b200.ops import decode as D
+
+    class Doubled(D.QuantWeight):
+        def dequantize(self):
+            return super().dequantize() * 2
+
+    cfg = SciAgentConfig(512, 1024, 2, 16, 4, 2816, 2048, 1e4)
+    model = GQADecoder(cfg, device="cuda", seed=3)
+    tokens = torch.randint(0, 512, (1, 1100), generator=torch.Generator().manual_seed(1)).cuda()
+    got = []
+    for work in (0, 1 << 60):
+        monkeypatch.setattr(infer._WidenAhead, "WORK", work)
+        eng = infer.InferenceEngine(model, quant="int8", max_batch=1, max_seq=1200)
+        for l in eng.layers:
+            l["wd"] = Doubled(l["wd"].q, l["wd"].scale)
+        got.append((eng.prefill(tokens).clone(), *eng.cache.pools))
+    _lib.check_status()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("where", ["attention_fwd", "swiglu_fwd", "rmsnorm_fwd"])
 def test_prefill_gives_matrices_back_when_memory_runs_out(where, monkeypatch):
     """An allocation that fails while matrices expanded ahead are held (here by exception, on the host): the piece of the layer is run
